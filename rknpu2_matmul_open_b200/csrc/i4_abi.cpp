@@ -3,7 +3,7 @@
 // The original packs A into int4 device tiles (directly or through a caller-supplied producer), runs int4 x int4 ->
 // INT16 waves on its NPU and widens / sums the partials on the CPU (src/rk_npu_matmul_i4.cpp:8-71,
 // src/rk_npu_i4_executor.cpp:54-126, src/rk_npu_i4_plan.cpp:126-242).  Here the int4 codes of A ride as int8 codes
-// through the same tcgen05 per-tile kernel the W4A8 path uses (int4 weights unpacked into tensor memory, exact int32
+// through the same persistent tcgen05 kernel the W4A8 path uses (int4 weights unpacked into tensor memory, exact int32
 // accumulation, the int32 epilogue), so there are no INT16 partials to saturate.  The producer protocol is kept: the
 // callback is invoked serially on the calling thread, K wave by K wave and M panel by M panel, with a zeroed
 // [padded_k / 32][rows][32] int4 tile (even element in the HIGH nibble) that the library then decodes.
@@ -44,11 +44,13 @@ struct rk_npu_i4_workspace {
     cudaStream_t stream = nullptr;
     int T = 0, KB = 0;
     uint8_t* codes = nullptr;
+    int* partials = nullptr;         // partial sums of tiles whose K is cut between CTA pairs
+    unsigned* counts = nullptr;      // and how far each such tile is
     float* scales = nullptr;
     Status* status = nullptr;
     int8_t* stage_in = nullptr;
     int32_t* stage_out = nullptr;
-    size_t codes_bytes = 0, stage_in_bytes = 0, stage_out_bytes = 0;
+    size_t codes_bytes = 0, partials_bytes = 0, counts_bytes = 0, stage_in_bytes = 0, stage_out_bytes = 0;
     Status* host_status = nullptr;
     std::vector<int8_t> host_a;      // the decoded activations of a producer run
     std::vector<uint8_t> host_tile;  // one producer tile
@@ -82,6 +84,8 @@ void workspace_destroy(rk_npu_i4_workspace* ws)
     if (d) cudaSetDevice(d->ctx->device);
     if (ws->stream) cudaStreamSynchronize(ws->stream);
     if (ws->codes) device_free(d, ws->codes, ws->codes_bytes);
+    if (ws->partials) device_free(d, ws->partials, ws->partials_bytes);
+    if (ws->counts) device_free(d, ws->counts, ws->counts_bytes);
     if (ws->scales) device_free(d, ws->scales, sizeof(float) * ws->config.M);
     if (ws->status) device_free(d, ws->status, sizeof(Status));
     if (ws->stage_in) device_free(d, ws->stage_in, ws->stage_in_bytes);
@@ -125,12 +129,13 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     g.KB = ws->KB; g.NG = w->NG; g.T = ws->T;
     g.epi = EPI_I32;
     g.split = 1;
-    g.pair = cfg.M > 128 ? 1 : 0;              // beyond 128 tokens: 128-token tiles, two per CTA pair of the persistent kernel
+    g.pair = 1;
+    g.partials = ws->partials;
+    g.counts = ws->counts;
+    g.max_clusters = ws->domain->ctx->sm_count / 2;
     g.timeout_ns = (unsigned long long)cfg.timeout_ms * 1000000ull;
     const auto t0 = Clock::now();
-    const bool persistent = g.pair && gemm_tc_persist_supported(g);
-    if (launch_w8_quantize(q, s) != cudaSuccess ||
-        (persistent ? launch_gemm_tc_persist(g, s, false) : launch_gemm_tc(g, s, false)) != cudaSuccess) {
+    if (launch_w8_quantize(q, s) != cudaSuccess || launch_gemm_tc_persist(g, s, false) != cudaSuccess) {
         cudaGetLastError();
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
@@ -141,6 +146,7 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     times.submit_us += since(t0);
     if (ws->host_status->device_error) {
         cudaMemsetAsync(&ws->status->device_error, 0, sizeof(int), s);
+        cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
     }
@@ -235,19 +241,25 @@ extern "C" rk_npu_i4_workspace* rk_npu_i4_workspace_create(rk_npu_iommu_domain* 
         ws->ctx_id = ctx->id;
         ws->domain_id = domain->id;
         domain_retain(domain);
-        ws->T = cfg->M > 128 ? 128 : align_up(cfg->M, 16);
         ws->KB = (cfg->K + KBLOCK - 1) / KBLOCK;
-        ws->codes_bytes = size_t(align_up(cfg->M, cfg->M > 128 ? 256 : ws->T)) * size_t(ws->KB) * KBLOCK;
+        const int tok = gemm_tc_persist_tok(cfg->N, cfg->M, ws->KB, ctx->sm_count);   // the code buffer covers whole pairs of token tiles
+        ws->T = tok / 2;
+        ws->codes_bytes = size_t(align_up(cfg->M, tok)) * size_t(ws->KB) * KBLOCK;
+        ws->partials_bytes = gemm_tc_persist_slot_bytes(ctx->sm_count, tok);
+        ws->counts_bytes = gemm_tc_persist_count_bytes(cfg->N, cfg->M, tok);
         ws->stage_in_bytes = size_t(cfg->M) * cfg->K;
         ws->stage_out_bytes = size_t(cfg->M) * cfg->N * sizeof(int32_t);
         bool ok = cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaMallocHost(reinterpret_cast<void**>(&ws->host_status), sizeof(Status)) == cudaSuccess;
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes) &&
+             !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
+             !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), sizeof(float) * cfg->M) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status)) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->stage_in), ws->stage_in_bytes) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->stage_out), ws->stage_out_bytes);
         ok = ok && cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
+             cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess &&
              cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess && cudaStreamSynchronize(ws->stream) == cudaSuccess;
         if (!ok) { cudaGetLastError(); return nullptr; }
         return ws.release();

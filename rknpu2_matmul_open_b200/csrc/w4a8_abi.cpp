@@ -484,7 +484,10 @@ int enqueue(const Call& c)
         // parking pays where finishing a chunk is expensive, i.e. for the SwiGLU epilogue (measured: the plain epilogues gain
         // nothing, the extra L2 traffic lengthens their MMA phase as much as the earlier hand-back saves);
         // RK_NPU_B200_PARK_ALL=1 parks for every epilogue (experiments)
-        if (c.epi == EPI_SWIGLU || env_flag("RK_NPU_B200_PARK_ALL", false)) g.partials = ws.partials;
+        if (c.epi == EPI_SWIGLU || env_flag("RK_NPU_B200_PARK_ALL", false)) g.park = ws.park;
+        g.partials = ws.partials;
+        g.counts = ws.counts;
+        g.max_clusters = ws.domain->ctx->sm_count / 2;
         if (gemm_tc_persist_supported(g) && !env_flag("RK_NPU_B200_NO_PERSIST", false)) err = launch_gemm_tc_persist(g, c.stream, pdl);
         else err = launch_gemm_tc(g, c.stream, pdl);
     } else if (ws.variant == 4) {
@@ -516,8 +519,7 @@ int status_to_rc(rk_npu_w4a8_workspace& ws, cudaStream_t stream)
     const Status s = *ws.host_status;
     if (s.device_error) {
         cudaMemsetAsync(&ws.status->device_error, 0, sizeof(int), stream);
-        // a streaming launch that gave up may have left partial sums behind
-        if (ws.partials) cudaMemsetAsync(ws.partials, 0, ws.partials_bytes, stream);
+        // a launch that gave up may have left tiles unfinished
         if (ws.counts) cudaMemsetAsync(ws.counts, 0, ws.counts_bytes, stream);
         cudaStreamSynchronize(stream);
         return RK_NPU_ERR_SUBMIT;
@@ -653,6 +655,7 @@ void workspace_destroy(rk_npu_w4a8_workspace* ws)
     if (ws->trace) device_free(d, ws->trace, ws->trace_bytes);
     if (ws->partials) device_free(d, ws->partials, ws->partials_bytes);
     if (ws->counts) device_free(d, ws->counts, ws->counts_bytes);
+    if (ws->park) device_free(d, ws->park, ws->park_bytes);
     if (ws->gather) device_free(d, ws->gather, ws->gather_bytes);
     if (ws->code_gather) device_free(d, ws->code_gather, ws->code_gather_bytes);
     if (ws->host_status) cudaFreeHost(ws->host_status);
@@ -1080,7 +1083,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         int pair_min = 33;
         if (const char* e = std::getenv("RK_NPU_B200_PAIR_MIN")) pair_min = std::max(1, std::atoi(e));   // experiments
         ws->pair = cfg->M >= pair_min && !env_flag("RK_NPU_B200_NO_PAIR", false);
-        ws->T = ws->pair ? 128 : (cfg->M >= 256 ? 256 : align_up(cfg->M, 16));
+        ws->T = ws->pair ? gemm_tc_persist_tok(local_N, cfg->M, ws->KB, ctx->sm_count) / 2 : (cfg->M >= 256 ? 256 : align_up(cfg->M, 16));
     } else if (variant == 4) {
         ws->TC = ws->T = cfg->M <= 16 ? 16 : cfg->M <= 32 ? 32 : cfg->M <= 64 ? 64 : 128;   // tcgen05 N
     } else {
@@ -1095,7 +1098,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (schedule.cluster && (variant == 1 || variant == 5 || (variant == 3 && (ws->KB + schedule.cluster - 1) / schedule.cluster <= FUSED_MAX_STAGES)) &&
         (variant == 5 || ws->KB >= schedule.cluster))
         ws->split_override = schedule.cluster;
-    const size_t Mp = size_t(align_up(cfg->M, ws->pair ? 256 : ws->T));
+    const size_t Mp = size_t(align_up(cfg->M, ws->pair ? 2 * ws->T : ws->T));
     ws->codes_bytes = Mp * size_t(ws->KB) * KBLOCK;
     const int out_cols = cfg->N;
     ws->stage_in_bytes = size_t(cfg->M) * cfg->K * 4;
@@ -1111,10 +1114,17 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes);
     }
-    if (variant == 2 && ws->pair && env_flag("RK_NPU_B200_PARK", true)) {
-        // the persistent kernel parks accumulator chunks here between reading them out of tensor memory and finishing them
-        ws->partials_bytes = gemm_tc_persist_park_bytes(ctx->sm_count);
+    if (variant == 2 && ws->pair) {
+        // partial sums of tiles whose K is cut between CTA pairs, and their stage counters
+        ws->partials_bytes = gemm_tc_persist_slot_bytes(ctx->sm_count, 2 * ws->T);
+        ws->counts_bytes = gemm_tc_persist_count_bytes(local_N, cfg->M, 2 * ws->T);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes);
+        ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes);
+        if (ws->T == 128 && env_flag("RK_NPU_B200_PARK", true)) {
+            // accumulator chunks between being read out of tensor memory and being finished
+            ws->park_bytes = gemm_tc_persist_park_bytes(ctx->sm_count);
+            ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->park), ws->park_bytes);
+        }
     }
     if (ctx->world > 1) {
         ws->gather_slot = size_t(cfg->M) * size_t(shard_plan(cfg->N, ctx->world, 0).columns()) * 4;   // rank 0's share is the widest
@@ -1137,7 +1147,6 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         ok = cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
              cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess &&
              cudaMemsetAsync(ws->rowmax, 0, sizeof(uint32_t) * cfg->M, ws->stream) == cudaSuccess &&
-             (!ws->partials || cudaMemsetAsync(ws->partials, 0, ws->partials_bytes, ws->stream) == cudaSuccess) &&
              (!ws->counts || cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess) &&
              cudaStreamSynchronize(ws->stream) == cudaSuccess;
         std::memset(ws->host_status, 0, sizeof(Status));

@@ -109,8 +109,12 @@ struct GemmParams {
     int w8;                 // tcgen05 per-tile kernel: Wp holds int8 codes in the W8 layout (w8a8_kernels.cu), sums are not scaled by 16
     unsigned long long timeout_ns;
     unsigned long long* trace;  // optional cycle stamps of CTA (0,0): [role 0..2][k-block 0..63][2] (nullable)
-    int* partials;              // streaming kernel: [2 x CTAs][T / 4][128][4] int32 partial sums (two slots per CTA, never cleared)
-    unsigned int* counts;       // streaming kernel: [tiles] stages accumulated so far, zero between launches
+    // streaming and persistent kernels: [2 x CTAs][tokens of the tile / 4][128][4] int32 partial sums (two slots per CTA,
+    // never cleared) and [tiles] ([tiles][2 CTAs] in the persistent kernel) stages accumulated so far, zero between launches
+    int* partials;
+    unsigned int* counts;
+    int* park;                  // persistent kernel, SwiGLU: where accumulator chunks wait to be finished (nullable)
+    int max_clusters;           // persistent kernel: CTA pairs the slots are sized for
 };
 
 // Single-kernel linear for small batches: quantisation fused in front of the GEMM.
@@ -239,11 +243,19 @@ cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, 
 // tcgen05 path: p.T is the token tile of the code layout (multiple of 16, <= 256; 128 when p.pair)
 cudaError_t launch_gemm_tc(const GemmParams& p, cudaStream_t stream, bool pdl);
 bool gemm_tc_supported(const GemmParams& p);
-// persistent two-CTA form (binary16 output or fused SwiGLU); p.pair and p.T == 128 required
+// persistent two-CTA form: p.pair, p.T (tokens of one CTA's activation tile: 32, 64 or 128), p.partials, p.counts and
+// p.max_clusters required
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
 bool gemm_tc_persist_supported(const GemmParams& p);
-// Bytes of GemmParams.partials the persistent kernel uses to park accumulator chunks (NULL: chunks are finished one by
-// one before the accumulator is handed back).  No initial contents needed.
+// Tokens of the MMA tile (64, 128 or 256) for a problem, and the CTA pairs of a launch (columns: all accumulator rows,
+// i.e. gate and up together for SwiGLU; tok = 2 T)
+int gemm_tc_persist_tok(int columns, int M, int KB, int sm_count);
+int gemm_tc_persist_clusters(int columns, int M, int KB, int tok, int max_clusters);
+// Bytes of GemmParams.partials and .counts (the latter zero before the first launch)
+size_t gemm_tc_persist_slot_bytes(int sm_count, int tok);
+size_t gemm_tc_persist_count_bytes(int columns, int M, int tok);
+// Bytes of GemmParams.park (NULL: chunks are finished one by one before the accumulator is handed back).  No initial
+// contents needed.
 size_t gemm_tc_persist_park_bytes(int sm_count);
 
 } // namespace rkb200

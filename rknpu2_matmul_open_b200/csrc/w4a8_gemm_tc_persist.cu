@@ -27,90 +27,129 @@
 #include "w4a8_math.cuh"
 #include "w4a8_ptx.cuh"
 #include "w4a8_tc.cuh"
+#include <algorithm>
+#include <cstdlib>
 
 namespace rkb200 {
 
-// activation ring: stages of 2 k-blocks (2 x 16 KB); five deep for int4 weights, three where int8 weights (the
-// W8A8 operators) take twice the room in the weight ring
-__host__ __device__ constexpr int ps_xa(bool w8) { return w8 ? 3 : 5; }
-constexpr int PS_XW = 4;                     // weight ring: stages of 2 k-blocks (4 groups x 2 x 2 KB, or x 4 KB for int8 weights)
-constexpr int PS_ABUF = 4;                   // weight buffers in tensor memory, one stage (2 k-blocks, 64 columns) each
+constexpr int PS_ROLE_WARPS = 4;             // warp 0: activation producer, 1: MMA issuer, 2: weight producer, 3: activation voucher
 constexpr int PS_UNPACK_WARPS = 8;
 constexpr int PS_EPI_WARPS = 8;              // two per tensor-memory lane quarter, alternating 32-token chunks
-constexpr int PS_UNPACK_WARP0 = 3;           // warp 0: activation producer, 1: MMA issuer, 2: weight producer
+constexpr int PS_UNPACK_WARP0 = PS_ROLE_WARPS;
 constexpr int PS_EPI_WARP0 = PS_UNPACK_WARP0 + PS_UNPACK_WARPS;
-constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 608
-constexpr int PS_T = 128;                    // tokens of one CTA's activation tile
-constexpr int PS_TOK = 256;                  // tokens of the MMA tile (accumulator columns)
-constexpr int PS_A_COL0 = 256;
+constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 640
 constexpr int PS_TMEM_COLS = 512;
-constexpr size_t PS_XA_BYTES = 2 * (size_t)PS_T * 128;   // 32768
-__host__ __device__ constexpr size_t ps_group_bytes(bool w8) { return w8 ? 4096 : 2048; }   // one k-block of one 32-channel group
-__host__ __device__ constexpr size_t ps_xw_bytes(bool w8) { return 2 * 4 * ps_group_bytes(w8); }   // 16384 / 32768
-__host__ __device__ constexpr int ps_barriers(bool w8) { return 2 * ps_xa(w8) + 2 * PS_XW + 2 * PS_ABUF + 2; }
-__host__ __device__ constexpr size_t ps_smem_bytes(bool w8)
-{
-    return ps_xa(w8) * PS_XA_BYTES + PS_XW * ps_xw_bytes(w8) + 2 * PS_TOK * 4 + ps_barriers(w8) * 8 + 32;
-}
 constexpr int PS_PARK_INTS = 3 * 32 * 32 * PS_EPI_WARPS;   // per CTA: three parked chunks of 32 sums per epilogue thread (96 KB)
-static_assert(ps_smem_bytes(false) <= 232448 && ps_smem_bytes(true) <= 232448, "exceeds the shared memory of one CTA");
-static_assert(PS_XW == PS_ABUF, "a weight stage and its tensor-memory buffer share one index");
+
+// One instantiation's resources.  TOK = tokens of the MMA tile (accumulator columns), half of them in each CTA.
+// Stages are 2 k-blocks.  Tensor memory holds the accumulator (two of them where they fit, so that the epilogue of a
+// segment overlaps the MMAs of the next) and the unpacked weights, 64 columns per stage.
+template <bool W8, int TOK>
+struct PsShape {
+    static constexpr int T = TOK / 2;                                            // tokens of one CTA's activation tile
+    static constexpr int XA = TOK == 256 ? (W8 ? 3 : 5) : TOK == 128 && W8 ? 4 : 6;   // activation ring
+    static constexpr int XW = TOK == 256 ? 4 : W8 ? 4 : TOK == 128 ? 6 : 8;     // weight ring
+    static constexpr int ACC = TOK == 256 ? 1 : 2;                               // accumulators
+    static constexpr int ABUF = TOK == 64 ? 6 : 4;                               // unpacked weight stages
+    static constexpr int A_COL0 = ACC * TOK;
+    static constexpr size_t XA_BYTES = 2 * (size_t)T * 128;
+    static constexpr uint32_t GB = W8 ? 4096 : 2048;                             // one k-block of one 32-channel group
+    static constexpr size_t XW_BYTES = 2 * 4 * (size_t)GB;
+    static constexpr int BARRIERS = 3 * XA + 2 * XW + 2 * ABUF + 2 * ACC;
+    static constexpr size_t SMEM = XA * XA_BYTES + XW * XW_BYTES + 2 * TOK * 4 + BARRIERS * 8 + 32;
+    static constexpr size_t SLOT_INTS = 128 * (size_t)TOK;                       // one CTA's partial sums of a segment
+    static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
+    static_assert(A_COL0 + 64 * ABUF <= PS_TMEM_COLS, "exceeds tensor memory");
+    // The two unpack sets take alternate stages, so with an even ring every slot belongs to one set, which sees all of its
+    // phases.  (With an odd one a set could ask for a slot's second phase while the first, the other set's, is still open;
+    // a parity wait takes that for completed.)
+    static_assert(XW % 2 == 0 && ABUF % 2 == 0, "a ring slot would change between the unpack sets");
+};
+
+// A position in a ring of N barriers: slot and phase parity.
+template <int N>
+struct RingPos {
+    int slot = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next() { if (++slot == N) { slot = 0; phase ^= 1u; } }
+};
+
+// Barrier of the eight epilogue warps that also tells every one of them whether `ok` holds in all.
+__device__ __forceinline__ bool epilogue_all(bool ok)
+{
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %1, 0;\n\t"
+        "bar.red.and.pred p, 1, 256, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(all)
+        : "r"(ok ? 1u : 0u)
+        : "memory");
+    return all != 0;
+}
 
 // W8: the weights are int8 codes in the W8 layout (w8a8_kernels.cu): "unpacking" is a copy into tensor memory and the sums
 // are not scaled by 16.
-template <bool W8>
+template <bool W8, int TOK>
 __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const GemmParams p, int num_clusters)
 {
-    constexpr int PS_XA = ps_xa(W8);
-    constexpr size_t PS_XW_BYTES = ps_xw_bytes(W8);
-    constexpr uint32_t GB = (uint32_t)ps_group_bytes(W8);
+    using S = PsShape<W8, TOK>;
+    constexpr uint32_t GB = S::GB;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* const acts = smem;
-    uint8_t* const wts = acts + PS_XA * PS_XA_BYTES;
-    float* const s_sx = reinterpret_cast<float*>(wts + PS_XW * PS_XW_BYTES);   // token scales of the tile being finished
-    uint32_t* const s_tilemax = reinterpret_cast<uint32_t*>(s_sx + PS_TOK);      // SwiGLU: the CTA's row maxima of that tile
-    uint64_t* const xfull = reinterpret_cast<uint64_t*>(s_tilemax + PS_TOK);
-    uint64_t* const xempty = xfull + PS_XA;
-    uint64_t* const wfull = xempty + PS_XA;
-    uint64_t* const wempty = wfull + PS_XW;
-    uint64_t* const a_ready = wempty + PS_XW;
-    uint64_t* const a_free = a_ready + PS_ABUF;
-    uint64_t* const acc_full = a_free + PS_ABUF;
-    uint64_t* const acc_empty = acc_full + 1;
-    uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 1);
+    uint8_t* const wts = acts + S::XA * S::XA_BYTES;
+    float* const s_sx = reinterpret_cast<float*>(wts + S::XW * S::XW_BYTES);     // token scales of the tile being finished
+    uint32_t* const s_tilemax = reinterpret_cast<uint32_t*>(s_sx + TOK);         // SwiGLU: the CTA's row maxima of that tile
+    uint64_t* const xfull = reinterpret_cast<uint64_t*>(s_tilemax + TOK);
+    uint64_t* const xempty = xfull + S::XA;
+    uint64_t* const x_ready = xempty + S::XA;    // leader: both CTAs' activations of the stage have landed
+    uint64_t* const wfull = x_ready + S::XA;
+    uint64_t* const wempty = wfull + S::XW;
+    uint64_t* const a_ready = wempty + S::XW;    // leader: both CTAs' weights of the stage are in tensor memory
+    uint64_t* const a_free = a_ready + S::ABUF;
+    uint64_t* const acc_full = a_free + S::ABUF;
+    uint64_t* const acc_empty = acc_full + S::ACC;
+    uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(acc_empty + S::ACC);
     int* const s_error = reinterpret_cast<int*>(s_tmem + 1);
+    int* const s_finish = s_error + 1;           // this CTA completed the tile whose partial sums it just stored
 
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();
     const int cluster_id = blockIdx.x >> 1;
     const bool swiglu = p.epi == EPI_SWIGLU;
-    const int KB = p.KB, KC = KB * 4;
+    const int KB = p.KB;
     const int nst = (KB + 1) / 2;                                      // stage iterations per tile
     const int tiles_n = swiglu ? (p.F + 63) / 64 : (p.N + TILE_N - 1) / TILE_N;
     const int pairs_n = (tiles_n + 1) / 2;
-    const int pairs_m = (p.M + PS_TOK - 1) / PS_TOK;
-    const int total = pairs_n * pairs_m;
+    const int pairs_m = (p.M + TOK - 1) / TOK;
+    // The work is the flat list of (tile, stage) items; every cluster takes one contiguous share of it.  The launcher
+    // picks a cluster count that divides the tile count where cutting tiles along K would not pay.
+    const long long total = (long long)pairs_n * pairs_m * nst;
+    const long long b0 = total * cluster_id / num_clusters, b1 = total * (cluster_id + 1) / num_clusters;
+    const int n_items = (int)(b1 - b0);
+    const int tile0 = (int)(b0 / nst), it0 = (int)(b0 - (long long)tile0 * nst);
     const unsigned long long deadline = global_ns() + p.timeout_ns;
-    // optional cycle stamps of cluster 0's leader: [tile j < 16][8] = MMA wait-begin, MMA first issue,
+    // optional cycle stamps of cluster 0's leader: [segment j < 16][8] = MMA wait-begin, MMA first issue,
     // MMA last commit, epilogue acc_full seen, tensor memory handed back, stored, [6] cycles the MMA
-    // issuer waited for operands; [128 + 2j] / [129 + 2j] cycles unpack warp 0 waited for weights /
-    // for a free tensor-memory buffer, [160 + j] for activations; [200] = clusters in the grid
+    // issuer waited for operands; [128] / [129] cycles unpack warp 0 waited for weights / for a free
+    // tensor-memory buffer, [160] cycles for activations; [200] = clusters in the grid
     unsigned long long* const trace = (p.trace && blockIdx.x == 0) ? p.trace : nullptr;
     const long long c0 = clock64();
 #define PS_STAMP(j, slot) do { if (trace && (j) < 16) trace[(j) * 8 + (slot)] = (unsigned long long)(clock64() - c0); } while (0)
     if (trace && tid == 0) trace[200] = (unsigned long long)num_clusters;
 
     if (tid == 0) {
-        for (int s = 0; s < PS_XA; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); }
-        for (int s = 0; s < PS_XW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 4); }
-        for (int b = 0; b < PS_ABUF; ++b) { mbar_init(&a_ready[b], 8); mbar_init(&a_free[b], 1); }
-        mbar_init(acc_full, 1);
-        mbar_init(acc_empty, 2 * PS_EPI_WARPS);   // every epilogue warp of both CTAs
+        for (int s = 0; s < S::XA; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); mbar_init(&x_ready[s], 2); }
+        for (int s = 0; s < S::XW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 4); }
+        for (int b = 0; b < S::ABUF; ++b) { mbar_init(&a_ready[b], 8); mbar_init(&a_free[b], 1); }
+        for (int b = 0; b < S::ACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * PS_EPI_WARPS); }   // every epilogue warp of both CTAs
         mbar_fence_init();
         *s_error = 0;
+        *s_finish = 0;
     }
-    if (tid < PS_TOK) s_tilemax[tid] = 0u;
+    if (tid < TOK) s_tilemax[tid] = 0u;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(PS_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -122,103 +161,152 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem;
 
-    // ---------------------------------------------------------------- weight producer (warp 2)
-    // Weights never change, so the ring is filled before the dependency wait below; the
-    // producer's position (tile, stage iteration, count) carries over to the loop after it.
-    int wp_t = cluster_id, wp_it = 0, wp_gi = 0;
-    auto produce_weights = [&](int limit) -> bool {
-        const int w = lane & 3;
-        bool ok = true;
-        while (wp_t < total && wp_gi < limit) {
-            const int tile = 2 * (wp_t % pairs_n) + (int)rank;
-            const int group = swiglu ? (w < 2 ? tile * 2 + w : p.F / GROUP + tile * 2 + (w - 2)) : tile * 4 + w;
-            const uint8_t* wsrc = p.Wp + (size_t)group * KB * GB;
-            const int s = wp_gi % PS_XW;
-            const int kbs = min(2, KB - 2 * wp_it);
-            if (lane == 0) {
-                if (wp_gi >= PS_XW) ok = mbar_wait(&wempty[s], ((wp_gi / PS_XW) - 1) & 1, deadline);
-                if (ok) mbar_arrive_expect_tx(&wfull[s], (uint32_t)kbs * 4u * GB);
-            }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) { *s_error = 1; return false; }
-            if (lane < 4) bulk_g2s(wts + (size_t)s * PS_XW_BYTES + w * 2 * GB, wsrc + (size_t)wp_it * 2 * GB, (uint32_t)kbs * GB, &wfull[s]);
-            ++wp_gi;
-            if (++wp_it == nst) { wp_it = 0; wp_t += num_clusters; }
-        }
-        return true;
+    // What does not depend on the kernel in front -- requesting weights, unpacking the first of them into tensor
+    // memory -- starts before the dependency wait; every other warp waits here.
+    auto dependency_met = [&]() -> bool {   // false: the quantiser rejected the input, nothing is to be written
+        pdl_wait();
+        return *reinterpret_cast<volatile const int*>(&p.status->bad_input) == 0;
     };
-    if (warp == 2) produce_weights(PS_XW);   // the first ring-full needs no free slot
-    pdl_wait();       // activation codes, scales and the status word come from the kernel in front
-    const bool skip = *reinterpret_cast<volatile const int*>(&p.status->bad_input) != 0;
 
     if (warp == 2) {
-        if (!skip) produce_weights(0x7fffffff);
-        else if (lane == 0)   // nobody will consume: let the copies already requested land before leaving
-            for (int s = 0; s < wp_gi; ++s)
+        // ---------------------------------------------------------------- weight producer
+        // (the whole warp walks the loop and one elected lane issues, as in the MMA issuer below: copy requests take their
+        // operands from uniform registers, and four lanes issuing one request each took 1000 cycles per stage)
+        RingPos<S::XW> r;
+        int it = it0;
+        bool ok = true, live = true;
+        const uint8_t* src = nullptr;                              // group 0 of this CTA's channel tile, stage `it`
+        const size_t group_bytes = (size_t)KB * GB;
+        const size_t upper = swiglu ? (size_t)(p.F / GROUP) * group_bytes : 2 * group_bytes;   // groups 2, 3 behind groups 0, 1
+        for (int gi = 0, tile = tile0; gi < n_items; ++gi, r.next()) {
+            if (gi == S::XW) {
+                live = dependency_met();
+                if (!live) break;
+            }
+            if (src == nullptr) {
+                const int ct = 2 * (tile % pairs_n) + (int)rank;
+                src = p.Wp + (size_t)(swiglu ? ct * 2 : ct * 4) * group_bytes + (size_t)it * 2 * GB;
+            }
+            const uint32_t bytes = (uint32_t)min(2, KB - 2 * it) * GB;
+            if (gi >= S::XW) ok = __all_sync(0xffffffffu, mbar_wait(&wempty[r.slot], r.phase ^ 1u, deadline));
+            if (!ok) { *s_error = 1; break; }
+            uint8_t* const dst = wts + (size_t)r.slot * S::XW_BYTES;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(&wfull[r.slot], 4u * bytes);
+                bulk_g2s(dst, src, bytes, &wfull[r.slot]);
+                bulk_g2s(dst + 2 * GB, src + group_bytes, bytes, &wfull[r.slot]);
+                bulk_g2s(dst + 4 * GB, src + upper, bytes, &wfull[r.slot]);
+                bulk_g2s(dst + 6 * GB, src + upper + group_bytes, bytes, &wfull[r.slot]);
+            }
+            __syncwarp();
+            src += 2 * GB;
+            if (++it == nst) { it = 0; ++tile; src = nullptr; }
+        }
+        if (n_items <= S::XW) live = dependency_met();
+        if (!live && lane == 0)   // nobody will consume: let the copies already requested land before leaving
+            for (int s = 0; s < min(n_items, S::XW); ++s)
                 if (!mbar_wait(&wfull[s], 0, deadline)) { *s_error = 1; break; }
     } else if (warp == 0) {
         // ---------------------------------------------------------------- activation producer
-        bool ok = !skip;
-        int gi = 0;
-        if (lane == 0) {
-            for (int t = cluster_id; t < total && ok; t += num_clusters) {
-                const int mt = 2 * (t / pairs_n) + (int)rank;
-                const uint8_t* xtile = p.Xq + (size_t)mt * ((size_t)KB * 8) * PS_T * 16;
-                for (int it = 0; it < nst && ok; ++it, ++gi) {
-                    const int s = gi % PS_XA;
-                    const int kbs = min(2, KB - 2 * it);
-                    if (gi >= PS_XA) ok = mbar_wait_cluster(&xempty[s], ((gi / PS_XA) - 1) & 1, deadline);
-                    if (!ok) { *s_error = 1; break; }
-                    mbar_arrive_expect_tx(&xfull[s], (uint32_t)kbs * PS_T * 128u);
-                    bulk_g2s(acts + (size_t)s * PS_XA_BYTES, xtile + (size_t)it * PS_XA_BYTES, (uint32_t)kbs * PS_T * 128u, &xfull[s]);
+        if (dependency_met()) {
+            RingPos<S::XA> r;
+            int it = it0;
+            const uint8_t* src = nullptr;
+            for (int gi = 0, tile = tile0; gi < n_items; ++gi, r.next()) {
+                if (src == nullptr) src = p.Xq + ((size_t)(2 * (tile / pairs_n) + (int)rank) * KB + (size_t)it * 2) * (S::T * 128);
+                const uint32_t bytes = (uint32_t)min(2, KB - 2 * it) * S::T * 128u;
+                bool ok = true;
+                if (gi >= S::XA) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xempty[r.slot], r.phase ^ 1u, deadline));
+                if (!ok) { *s_error = 1; break; }
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&xfull[r.slot], bytes);
+                    bulk_g2s(acts + (size_t)r.slot * S::XA_BYTES, src, bytes, &xfull[r.slot]);
                 }
+                __syncwarp();
+                src += S::XA_BYTES;
+                if (++it == nst) { it = 0; ++tile; src = nullptr; }
             }
+            // The MMAs' commits arrive on this CTA's barriers asynchronously, the peer's among them: the CTA may not leave
+            // (and its shared memory change hands) before the last of them is here.
+            for (int gi = n_items; gi < n_items + S::XA && !*reinterpret_cast<volatile int*>(s_error); ++gi, r.next())
+                if (gi >= S::XA && !mbar_wait_cluster(&xempty[r.slot], r.phase ^ 1u, deadline)) *s_error = 1;
+        }
+    } else if (warp == 3) {
+        // ---------------------------------------------------------------- activation voucher
+        // The leader's MMAs read both CTAs' activations: this warp passes on that this CTA's copy has landed.  It runs
+        // ahead of the MMAs by the depth of the ring.  (When the unpack warps vouched for it, with a release at cluster
+        // scope, that release bounded the whole loop: 730 cycles per k-block at K = 11008 against 525 now.)
+        if (dependency_met() && lane == 0) {
+            RingPos<S::XA> r;
+            long long waited = 0;
+            for (int gi = 0; gi < n_items; ++gi, r.next()) {
+                const long long w0 = trace ? clock64() : 0;
+                if (!mbar_wait(&xfull[r.slot], r.phase, deadline)) { *s_error = 1; break; }
+                if (trace) waited += clock64() - w0;
+                if (rank != 0) mbar_arrive_remote(&x_ready[r.slot], 0); else mbar_arrive(&x_ready[r.slot]);
+            }
+            if (trace) trace[160] = (unsigned long long)waited;
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (leader CTA)
-        if (lane == 0 && rank == 0 && !skip) {
-            const uint32_t idesc = tc_idesc_s8(256, PS_TOK);
+        // The whole warp walks the loop, so that descriptors and addresses are warp-uniform values, and one elected lane
+        // issues.  (A loop that only lane 0 enters moves every operand of every MMA into uniform registers first: 85
+        // cycles per MMA, which bounded a stage at 1190 cycles whatever the token tile; 1050 now at 256 tokens, of 1024.)
+        if (dependency_met() && rank == 0) {
+            const uint32_t idesc = tc_idesc_s8(256, TOK);
             bool ok = true;
-            int gi = 0, j = 0;
-            for (int t = cluster_id; t < total && ok; t += num_clusters, ++j) {
-                PS_STAMP(j, 0);
-                if (j > 0) {   // the epilogue warps of both CTAs have read the previous tile out of tensor memory
-                    ok = mbar_wait_cluster(acc_empty, (j - 1) & 1, deadline);
+            RingPos<S::XA> rx;
+            RingPos<S::ABUF> ra;
+            RingPos<S::ACC> rc;
+            int it = it0;
+            for (int gi = 0, j = 0; gi < n_items && ok; ++j, rc.next()) {
+                const int n = min(nst - it, n_items - gi);
+                if (lane == 0) PS_STAMP(j, 0);
+                if (j >= S::ACC) {   // the epilogue warps of both CTAs have read this accumulator's previous segment
+                    ok = __all_sync(0xffffffffu, mbar_wait_cluster(&acc_empty[rc.slot], rc.phase ^ 1u, deadline));
                     if (!ok) { *s_error = 1; break; }
                     tc_fence_after();
                 }
+                const uint32_t d_tmem = tmem_base + rc.slot * TOK;
                 long long waited = 0;
-                for (int it = 0; it < nst && ok; ++it) {
-                    const int g = gi + it, s = g % PS_XA, b = g % PS_ABUF;
+                for (int i = 0; i < n; ++i, ++it, rx.next(), ra.next()) {
                     const int kbs = min(2, KB - 2 * it);
                     const long long w0 = trace ? clock64() : 0;
-                    ok = mbar_wait_cluster(&a_ready[b], (g / PS_ABUF) & 1, deadline);
+                    ok = mbar_wait_cluster(&x_ready[rx.slot], rx.phase, deadline) && mbar_wait_cluster(&a_ready[ra.slot], ra.phase, deadline);
+                    ok = __all_sync(0xffffffffu, ok);
                     if (trace) waited += clock64() - w0;
                     if (!ok) { *s_error = 1; break; }
-                    if (it == 0) PS_STAMP(j, 1);
+                    if (i == 0 && lane == 0) PS_STAMP(j, 1);
                     tc_fence_after();
-                    const uint32_t xaddr = smem_u32(acts + (size_t)s * PS_XA_BYTES);
-                    const uint32_t a_tmem = tmem_base + PS_A_COL0 + b * 64;
+                    const uint32_t xaddr = smem_u32(acts + (size_t)rx.slot * S::XA_BYTES);
+                    const uint32_t a_tmem = tmem_base + S::A_COL0 + ra.slot * 64;
                     // k-step q: k-block q / 4 of the stage, 32 k = two 16-byte chunks per token: the descriptor's
-                    // address field advances by 2 * PS_T (16-byte units) per step
-                    const uint64_t desc0 = tc_smem_desc(xaddr, PS_T * 16u, 128u);
-                    tc_mma_i8_ts_pair(tmem_base, a_tmem, desc0, idesc, it > 0 ? 1u : 0u);
+                    // address field advances by 2 * T (16-byte units) per step
+                    const uint64_t desc0 = tc_smem_desc(xaddr, S::T * 16u, 128u);
+                    if (elect_one()) {
+                        tc_mma_i8_ts_pair(d_tmem, a_tmem, desc0, idesc, i > 0 ? 1u : 0u);
 #pragma unroll
-                    for (int q = 1; q < 4; ++q) tc_mma_i8_ts_pair_acc(tmem_base, a_tmem + q * 8, desc0 + (uint64_t)(q * 2 * PS_T), idesc);
-                    if (kbs == 2) {
+                        for (int q = 1; q < 4; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_tmem + q * 8, desc0 + (uint64_t)(q * 2 * S::T), idesc);
+                        if (kbs == 2) {
 #pragma unroll
-                        for (int q = 4; q < 8; ++q) tc_mma_i8_ts_pair_acc(tmem_base, a_tmem + q * 8, desc0 + (uint64_t)(q * 2 * PS_T), idesc);
+                            for (int q = 4; q < 8; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_tmem + q * 8, desc0 + (uint64_t)(q * 2 * S::T), idesc);
+                        }
+                        tc_commit_pair(&xempty[rx.slot]);   // the activation stage may be refilled once these MMAs retire
+                        tc_commit_pair(&a_free[ra.slot]);   // and the weight buffer rewritten, in both CTAs
+                        if (i == n - 1) tc_commit_pair(&acc_full[rc.slot]);
                     }
-                    tc_commit_pair(&xempty[s]);   // the activation stage may be refilled once these MMAs retire
-                    tc_commit_pair(&a_free[b]);   // and the weight buffer rewritten, in both CTAs
+                    __syncwarp();
                 }
-                gi += nst;
-                tc_commit_pair(acc_full);
-                PS_STAMP(j, 2);
-                if (trace && j < 16) trace[j * 8 + 6] = (unsigned long long)waited;
+                if (!ok) break;
+                if (lane == 0) {
+                    PS_STAMP(j, 2);
+                    if (trace && j < 16) trace[j * 8 + 6] = (unsigned long long)waited;
+                }
+                gi += n;
+                if (it == nst) it = 0;
             }
         }
-    } else if (warp >= PS_UNPACK_WARP0 && warp < PS_EPI_WARP0) {
+    } else if (warp < PS_EPI_WARP0) {
         // ---------------------------------------------------------------- weight unpack -> TMEM
         const int q = warp & 3;
         const int set = (warp - PS_UNPACK_WARP0) >> 2;
@@ -228,87 +316,87 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         // up rows (staged groups 0,1 = gate, 2,3 = up of the same 64 features).
         const int src_group = swiglu ? (q >> 1) + (lane >= 16 ? 2 : 0) : q;
         const int src_row = swiglu ? (q & 1) * 16 + (lane & 15) : lane;
-        bool ok = !skip;
-        int gi0 = 0, tj = 0;
         const bool tr = trace && warp == PS_UNPACK_WARP0 && lane == 0;
-        for (int t = cluster_id; t < total && ok; t += num_clusters, ++tj) {
-            long long wait_full = 0, wait_free = 0, wait_x = 0;
-            for (int it = 0; it < nst && ok; ++it) {
-                const int g = gi0 + it;
-                if ((g & 1) != set) continue;                      // the two sets take alternate stages
-                const int s = g % PS_XW, b = s, sa = g % PS_XA;
-                const int kbs = min(2, KB - 2 * it);
-                const long long w0 = tr ? clock64() : 0;
-                ok = mbar_wait(&wfull[s], (g / PS_XW) & 1, deadline);
-                const long long w1 = tr ? clock64() : 0;
-                if (ok && g >= PS_ABUF) ok = mbar_wait_cluster(&a_free[b], ((g / PS_ABUF) - 1) & 1, deadline);
-                if (tr) { wait_full += w1 - w0; wait_free += clock64() - w1; }
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) { *s_error = 1; break; }
-                tc_fence_after();
-                const uint4* src = reinterpret_cast<const uint4*>(wts + (size_t)s * PS_XW_BYTES + src_group * 2 * GB) + src_row;
-                if constexpr (W8) {
-                    // int8 codes: a lane's sixteen 16-byte pieces of the stage are the words of its tensor-memory row in order
+        long long wait_full = 0, wait_free = 0;
+        RingPos<S::XW> rw;
+        RingPos<S::ABUF> ra;
+        // The two sets take alternate stages.  A stage's packed words are read from shared memory while the previous
+        // stage's stores to tensor memory are still on their way, so that the two latencies overlap.
+        constexpr int NV = W8 ? 16 : 8;                        // 16-byte pieces a lane takes from a stage
+        uint4 w[NV];
+        bool ok = true;
+        auto fetch = [&](int it) {
+            const int kbs = min(2, KB - 2 * it);
+            const long long w0 = tr ? clock64() : 0;
+            ok = __all_sync(0xffffffffu, mbar_wait(&wfull[rw.slot], rw.phase, deadline));
+            if (tr) wait_full += clock64() - w0;
+            const uint4* src = reinterpret_cast<const uint4*>(wts + (size_t)rw.slot * S::XW_BYTES + src_group * 2 * GB) + src_row;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        if (h < kbs) {
-                            uint32_t r[32];
+            for (int c = 0; c < NV; ++c) w[c] = (c < NV / 2 * kbs) ? src[c * 32] : make_uint4(0u, 0u, 0u, 0u);
+        };
+        int it = it0;
+        auto advance = [&]() { rw.next(); ra.next(); if (++it == nst) it = 0; };
+        if (set == 1) advance();
+        if (set < n_items) fetch(it);
+        for (int g = set; g < n_items && ok; g += 2) {
+            const int kbs = min(2, KB - 2 * it), b = ra.slot;
+            // (before the first buffer comes back from the MMAs, which need the activations)
+            if ((g == S::ABUF || g == S::ABUF + 1) && !dependency_met()) break;
+            const long long w0 = tr ? clock64() : 0;
+            if (g >= S::ABUF) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&a_free[b], ra.phase ^ 1u, deadline));
+            if (tr) wait_free += clock64() - w0;
+            if (!ok) break;
+            tc_fence_after();
 #pragma unroll
-                            for (int c = 0; c < 8; ++c) {
-                                const uint4 v = src[(8 * h + c) * 32];
-                                r[4 * c] = v.x; r[4 * c + 1] = v.y; r[4 * c + 2] = v.z; r[4 * c + 3] = v.w;
-                            }
-                            if (h == kbs - 1) {
-                                __syncwarp();
-                                if (lane == 0) mbar_arrive(&wempty[s]);    // the stage has been read into registers
-                            }
-                            tc_st32(lane_addr + PS_A_COL0 + b * 64 + h * 32, r);
+            for (int h = 0; h < 2; ++h) {
+                if (h < kbs) {
+                    uint32_t r[32];
+                    if constexpr (W8) {
+                        // int8 codes: a lane's sixteen 16-byte pieces of the stage are the words of its tensor-memory row in order
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            const uint4 v = w[8 * h + c];
+                            r[4 * c] = v.x; r[4 * c + 1] = v.y; r[4 * c + 2] = v.z; r[4 * c + 3] = v.w;
                         }
-                    }
-                } else {
-                uint4 w[8];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) w[c] = (c < 4 * kbs) ? src[c * 32] : make_uint4(0u, 0u, 0u, 0u);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&wempty[s]);            // the packed copy is in registers
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (h < kbs) {
-                        uint32_t r[32];
+                    } else {
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
-                            const uint32_t ww[4] = {w[4 * h + c].x, w[4 * h + c].y, w[4 * h + c].z, w[4 * h + c].w};
+                            const uint4 v = w[4 * h + c];
+                            const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                             for (int jj = 0; jj < 4; ++jj) {
                                 r[c * 8 + jj] = (ww[jj] << 4) & 0xF0F0F0F0u;
                                 r[c * 8 + 4 + jj] = ww[jj] & 0xF0F0F0F0u;
                             }
                         }
-                        tc_st32(lane_addr + PS_A_COL0 + b * 64 + h * 32, r);
                     }
+                    tc_st32(lane_addr + S::A_COL0 + b * 64 + h * 32, r);
                 }
-                }
-                tc_wait_st();
-                tc_fence_before();
-                // the MMA also reads this stage's activations from both CTAs: vouch for this CTA's copy
-                const long long w2 = tr ? clock64() : 0;
-                ok = mbar_wait(&xfull[sa], (g / PS_XA) & 1, deadline);
-                if (tr) wait_x += clock64() - w2;
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) { *s_error = 1; break; }
-                if (lane == 0) { if (rank != 0) mbar_arrive_remote(&a_ready[b], 0); else mbar_arrive(&a_ready[b]); }
             }
-            gi0 += nst;
-            if (tr && tj < 16) {
-                trace[128 + tj * 2] = (unsigned long long)wait_full;
-                trace[128 + tj * 2 + 1] = (unsigned long long)wait_free;
-                trace[160 + tj] = (unsigned long long)wait_x;
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&wempty[rw.slot]);      // the packed copy has been read
+            advance();
+            advance();
+            if (g + 2 < n_items) fetch(it);
+            tc_wait_st();
+            tc_fence_before();
+            // Tensor-memory writes are ordered by the wait and the fences; the arrival itself carries nothing, so it is
+            // relaxed (see mbar_arrive_remote for what a release at cluster scope costs).
+            __syncwarp();
+            if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(&a_ready[b], 0); else mbar_arrive_relaxed(&a_ready[b]); }
         }
-    } else if (warp >= PS_EPI_WARP0) {
+        if (!ok) *s_error = 1;
+        // (the commits on the buffers have to be here before the CTA leaves, as for the activation ring; none come where
+        // the input was rejected)
+        if (ok && dependency_met())
+            for (int g = n_items + ((n_items ^ set) & 1); g < n_items + S::ABUF; g += 2, ra.next(), ra.next())
+                if (g >= S::ABUF && !mbar_wait_cluster(&a_free[ra.slot], ra.phase ^ 1u, deadline)) { *s_error = 1; break; }
+        if (tr) { trace[128] = (unsigned long long)wait_full; trace[129] = (unsigned long long)wait_free; }
+    } else {
         // ---------------------------------------------------------------- epilogue warps
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes 32-token chunks eset, eset + 2, ...
+        constexpr int CHUNKS = TOK / 64;
         const int sid = (warp - PS_EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const int out_cols = swiglu ? p.F : p.N;
@@ -319,40 +407,89 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         const bool quad_ok = (out_cols % 4 == 0) && (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
         constexpr int SHIFT = W8 ? 0 : 4;             // int4 records enter the MMA times 16
         const bool small_sums = (long long)KB * KBLOCK * (W8 ? 127 : 7) * 127 < (1ll << 22);
-        bool ok = !skip;
-        int j = 0;
-        for (int t = cluster_id; t < total && ok; t += num_clusters, ++j) {
-            const int tile = 2 * (t % pairs_n) + (int)rank;
-            const int tok_base = (t / pairs_n) * PS_TOK;
-            const int col0 = swiglu ? tile * 64 : tile * TILE_N;
+        bool ok = dependency_met();
+        RingPos<S::ACC> rc;
+        int tile = tile0, it = it0;
+        for (int gi = 0, j = 0; gi < n_items && ok; ++j, rc.next()) {
+            const int n_seg = min(nst - it, n_items - gi);
+            const bool whole = n_seg == nst;                 // this segment covers its tile's whole K
+            const bool last_seg = gi + n_seg >= n_items;
+            const int ct = 2 * (tile % pairs_n) + (int)rank;
+            const int tok_base = (tile / pairs_n) * TOK;
+            const int col0 = swiglu ? ct * 64 : ct * TILE_N;
             const int n = col0 + col;
             const bool n_ok = n < out_cols;
             const float sw = n_ok ? p.sw[(up_lane ? p.F : 0) + n] : 0.f;
             float* const sx = s_sx;
-            {
+            if (sid < TOK) {
                 const int m = tok_base + sid;
                 sx[sid] = m < p.M ? p.sx[m] : 0.f;
             }
             asm volatile("bar.sync 1, 256;" ::: "memory");   // scales staged (the barrier at the end of a tile keeps stragglers out)
-            ok = mbar_wait_cluster(acc_full, j & 1, deadline);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // one verdict for all eight warps
             if (!ok) { *s_error = 1; break; }
             if (sid == 0) PS_STAMP(j, 3);
             tc_fence_after();
+            const uint32_t acc_addr = lane_addr + rc.slot * TOK;
+            auto hand_back = [&]() {   // this warp is done with the accumulator: another segment's MMAs may overwrite it
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(&acc_empty[rc.slot], 0); else mbar_arrive_relaxed(&acc_empty[rc.slot]); }
+                if (sid == 0) PS_STAMP(j, 4);
+            };
+            // ---- a part of a tile's K: the raw sums go to this CTA's slot, the tile's stage counter is advanced, and the
+            // CTA that completes it adds the contributors' slots (integer addition: exact in any order) and finishes the
+            // tile.  Nobody waits for anybody, and no slot needs clearing.  A cluster's run begins and ends with at most
+            // one partial segment each, so two slots per CTA suffice.
+            int part_lo = 0, part_hi = -1;                   // contributing clusters when the sums come from slots
+            if (!whole) {
+                int4* const slot = reinterpret_cast<int4*>(p.partials) + ((size_t)(2 * cluster_id + (gi == 0 ? 0 : 1)) * 2 + rank) * (S::SLOT_INTS / 4);
+#pragma unroll 1
+                for (int c = 0; c < CHUNKS; ++c) {
+                    const int t0 = eset * 32 + 64 * c;
+                    if (tok_base + t0 < p.M) {
+                        uint32_t r[32];
+                        tc_ld32(acc_addr + t0, r);
+                        tc_wait_ld();
+                        int4* const dst = slot + (size_t)(t0 / 4) * 128 + q * 32 + lane;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) dst[(size_t)i * 128] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
+                    }
+                }
+                hand_back();
+                __threadfence();
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if (sid == 0) {
+                    // (a tile with a segment whose wait ran out is never completed; the launch reports the error and the host
+                    // clears the counters)
+                    unsigned* const count = p.counts + 2 * tile + (int)rank;
+                    const bool done = atomicAdd(count, (unsigned)n_seg) + (unsigned)n_seg == (unsigned)nst;
+                    if (done) *count = 0u;
+                    *s_finish = done ? 1 : 0;
+                    __threadfence();
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if (*reinterpret_cast<volatile int*>(s_finish)) {
+                    const long long s0 = (long long)tile * nst;
+                    part_lo = (int)(((s0 + 1) * num_clusters - 1) / total);
+                    part_hi = (int)(((s0 + nst) * num_clusters - 1) / total);
+                }
+            }
+            const bool finish = whole || part_hi >= part_lo;
             // The tensor pipe stands still until the accumulator is handed back.  Where finishing a chunk is expensive
             // (`park`: the SwiGLU epilogue, fp32 / int32 stores) the first three chunks are only moved: tensor memory ->
             // registers -> this thread's own slots of a scratch in global memory (it stays in L2); the fourth stays in
             // registers, the accumulator goes back, and then the four chunks are finished, the parked ones read back
             // by the thread that wrote them.
-            const bool park = p.partials != nullptr && t + num_clusters < total;   // (nothing waits behind a cluster's last tile)
-            int* const park_at = park ? p.partials + (size_t)blockIdx.x * PS_PARK_INTS + sid : nullptr;
+            const bool park = S::ACC == 1 && whole && p.park != nullptr && !last_seg;   // (nothing waits behind a cluster's last tile)
+            int* const park_at = park ? p.park + (size_t)blockIdx.x * PS_PARK_INTS + sid : nullptr;
             if (park) {
 #pragma unroll 1
                 for (int c = 0; c < 3; ++c) {
                     const int t0 = eset * 32 + 64 * c;
                     if (tok_base + t0 >= p.M) continue;
                     uint32_t r[32];
-                    tc_ld32(lane_addr + t0, r);
+                    tc_ld32(acc_addr + t0, r);
                     tc_wait_ld();
 #pragma unroll
                     for (int i = 0; i < 32; ++i) __stcg(park_at + (c * 32 + i) * 256, (int)r[i]);
@@ -366,27 +503,37 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                 if (trace && sid == 0) { const long long now = clock64(); trace[176 + which] += (unsigned long long)(now - phase_t); phase_t = now; }
             };
 #pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                const int c = park ? (k + 3) & 3 : k;
+            for (int k = 0; k < (finish ? CHUNKS : 0); ++k) {
+                const int c = park ? (k + CHUNKS - 1) % CHUNKS : k;
                 const int t0 = eset * 32 + 64 * c;
                 const bool live_chunk = tok_base + t0 < p.M;
                 uint32_t r[32];
                 if (live_chunk) {
-                    if (!park || k == 0) {
-                        tc_ld32(lane_addr + t0, r);
+                    if (!whole) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[i] = 0u;
+#pragma unroll 1
+                        for (int cc = part_lo; cc <= part_hi; ++cc) {
+                            // a cluster whose run starts inside the tile contributed its first segment, another one its last
+                            const int which = total * cc / num_clusters >= (long long)tile * nst ? 0 : 1;
+                            const int4* const src = reinterpret_cast<const int4*>(p.partials) + ((size_t)(2 * cc + which) * 2 + rank) * (S::SLOT_INTS / 4) + (size_t)(t0 / 4) * 128 + q * 32 + lane;
+                            int4 v[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) v[i] = __ldcg(src + (size_t)i * 128);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) {
+                                r[4 * i] += (uint32_t)v[i].x; r[4 * i + 1] += (uint32_t)v[i].y; r[4 * i + 2] += (uint32_t)v[i].z; r[4 * i + 3] += (uint32_t)v[i].w;
+                            }
+                        }
+                    } else if (!park || k == 0) {
+                        tc_ld32(acc_addr + t0, r);
                         tc_wait_ld();
                     } else {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) r[i] = (uint32_t)__ldcg(park_at + (c * 32 + i) * 256);
                     }
                 }
-                if (k == (park ? 0 : 3)) {
-                    // ---- this warp is done with tensor memory: the next tile's MMAs may overwrite it
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(acc_empty, 0); else mbar_arrive_relaxed(acc_empty); }
-                    if (sid == 0) PS_STAMP(j, 4);
-                }
+                if (whole && k == (park ? 0 : CHUNKS - 1)) hand_back();
                 if (!live_chunk) continue;
                 phase(0);
                 // All loads of a chunk come first, then the arithmetic, then the stores: the compiler
@@ -535,13 +682,16 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
             if (sid == 0) PS_STAMP(j, 5);
             asm volatile("bar.sync 1, 256;" ::: "memory");   // every epilogue warp is done with this tile's scales and maxima
             phase(3);
-            if (swiglu && p.rowmax) {
+            if (swiglu && p.rowmax && sid < TOK) {
                 const uint32_t m = s_tilemax[sid];
                 if (m) {
                     atomicMax(&p.rowmax[tok_base + sid], m);
                     s_tilemax[sid] = 0u;
                 }
             }
+            gi += n_seg;
+            it += n_seg;
+            if (it == nst) { it = 0; ++tile; }
         }
     }
 
@@ -557,17 +707,14 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     }
 }
 
-bool gemm_tc_persist_supported(const GemmParams& p)
-{
-    return p.pair && p.T == PS_T && (long long)p.KB * KBLOCK <= 131072;
-}
+namespace {
+constexpr long long PS_MAX_K = 131072;
 
-size_t gemm_tc_persist_park_bytes(int sm_count) { return size_t(sm_count) * PS_PARK_INTS * sizeof(int); }
-
-template <bool W8>
-static cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool pdl)
+template <bool W8, int TOK>
+cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
-    auto kernel = gemm_tc_persist_kernel<W8>;
+    using S = PsShape<W8, TOK>;
+    auto kernel = gemm_tc_persist_kernel<W8, TOK>;
     static PerDeviceOnce configured;
     static int clusters_of_device[64] = {};   // resident CTA pairs, per CUDA ordinal
     int device = -1;
@@ -576,7 +723,7 @@ static cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream,
     if (!setup) max_clusters = clusters_of_device[device];
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(PS_THREADS);
-    cfg.dynamicSmemBytes = ps_smem_bytes(W8);
+    cfg.dynamicSmemBytes = S::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -584,9 +731,9 @@ static cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream,
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     if (setup || !max_clusters) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps_smem_bytes(W8));
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
         if (e != cudaSuccess) return e;
-        // how many CTA pairs can be resident at once: the grid is exactly that many
+        // how many CTA pairs can be resident at once: the grid is at most that many
         cfg.gridDim = dim3(2, 1, 1);
         cfg.attrs = attr;
         cfg.numAttrs = 1;
@@ -596,9 +743,8 @@ static cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream,
         max_clusters = n;
         if (device >= 0 && device < 64) { clusters_of_device[device] = n; configured.mark(device); }
     }
-    const int tiles_n = p.epi == EPI_SWIGLU ? (p.F + 63) / 64 : (p.N + TILE_N - 1) / TILE_N;
-    const int total = ((tiles_n + 1) / 2) * ((p.M + PS_TOK - 1) / PS_TOK);
-    const int clusters = total < max_clusters ? total : max_clusters;
+    if (max_clusters > p.max_clusters) max_clusters = p.max_clusters;      // what the slots in p.partials were sized for
+    const int clusters = gemm_tc_persist_clusters(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, p.KB, TOK, max_clusters);
     cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
     int n = 1;
     if (pdl) {
@@ -610,11 +756,43 @@ static cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream,
     cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, p, clusters);
 }
+} // namespace
+
+bool gemm_tc_persist_supported(const GemmParams& p)
+{
+    return p.pair && (p.T == 128 || p.T == 64 || p.T == 32) && (long long)p.KB * KBLOCK <= PS_MAX_K && p.partials && p.counts;
+}
+
+// CTA pairs of a launch: all resident ones, but no more than `split_cap` per tile.
+int gemm_tc_persist_clusters(int columns, int M, int KB, int tok, int max_clusters)
+{
+    const long long tiles = (long long)((columns + 255) / 256) * ((M + tok - 1) / tok);
+    const long long stages = tiles * ((KB + 1) / 2);
+    static const int cap = std::getenv("RK_PS_CAP") ? std::atoi(std::getenv("RK_PS_CAP")) : 1;
+    long long n = std::min<long long>(max_clusters, tiles * cap);
+    n = std::min(n, std::max<long long>(stages / 2, 1));
+    return (int)n;
+}
+
+int gemm_tc_persist_tok(int columns, int M, int KB, int sm_count)
+{
+    static const int forced = std::getenv("RK_PS_TOK") ? std::atoi(std::getenv("RK_PS_TOK")) : 0;
+    if (forced) return forced;
+    return M <= 64 ? 64 : M <= 128 ? 128 : 256;
+}
+
+size_t gemm_tc_persist_park_bytes(int sm_count) { return size_t(sm_count) * PS_PARK_INTS * sizeof(int); }
+size_t gemm_tc_persist_slot_bytes(int sm_count, int tok) { return 2 * size_t(sm_count) * 128 * size_t(tok) * sizeof(int); }
+size_t gemm_tc_persist_count_bytes(int columns, int M, int tok) { return 2 * size_t((columns + 255) / 256) * size_t((M + tok - 1) / tok) * sizeof(unsigned); }
 
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
     if (!gemm_tc_persist_supported(p)) return cudaErrorInvalidValue;
-    return p.w8 ? launch_persist_inst<true>(p, stream, pdl) : launch_persist_inst<false>(p, stream, pdl);
+    switch (p.T) {
+    case 32: return p.w8 ? launch_persist_inst<true, 64>(p, stream, pdl) : launch_persist_inst<false, 64>(p, stream, pdl);
+    case 64: return p.w8 ? launch_persist_inst<true, 128>(p, stream, pdl) : launch_persist_inst<false, 128>(p, stream, pdl);
+    default: return p.w8 ? launch_persist_inst<true, 256>(p, stream, pdl) : launch_persist_inst<false, 256>(p, stream, pdl);
+    }
 }
 
 } // namespace rkb200

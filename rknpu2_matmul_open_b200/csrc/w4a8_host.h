@@ -123,7 +123,8 @@ struct rk_npu_w4a8_workspace {
     uint32_t* rowmax = nullptr;
     int* partials = nullptr;          // variant 4: per-tile partial sums and k-block counters
     unsigned int* counts = nullptr;
-    size_t partials_bytes = 0, counts_bytes = 0;
+    int* park = nullptr;              // variant 2: accumulator chunks of the SwiGLU epilogue
+    size_t partials_bytes = 0, counts_bytes = 0, park_bytes = 0;
     rkb200::Status* status = nullptr;
     void* stage_in = nullptr;   // device copy of host activations
     void* stage_out = nullptr;  // device copy of host outputs

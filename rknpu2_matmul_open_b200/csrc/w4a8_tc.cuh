@@ -12,13 +12,21 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// One lane of a converged warp, the same one every time.  Code behind it may keep its operands in uniform registers,
+// which is where MMA and bulk-copy instructions want them.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ void tc_mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // Accumulating forms (D += A * B) without the predicate set-up.  The issuing thread is a single
@@ -29,8 +37,8 @@ __device__ __forceinline__ void tc_mma_i8_ts_acc(uint32_t d_tmem, uint32_t a_tme
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.eq.u32 p, 1, 1;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, {%4, %4, %4, %4}, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(0u)
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc)
         : "memory");
 }
 __device__ __forceinline__ void tc_mma_i8_ts_pair_acc(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc)
@@ -38,8 +46,8 @@ __device__ __forceinline__ void tc_mma_i8_ts_pair_acc(uint32_t d_tmem, uint32_t 
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.eq.u32 p, 1, 1;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, {%4, %4, %4, %4, %4, %4, %4, %4}, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(0u)
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc)
         : "memory");
 }
 // paired forms: the MMA spans both CTAs of the cluster; the commit arrives on the barrier at
@@ -54,17 +62,20 @@ __device__ __forceinline__ void tc_mma_i8_ts_pair(uint32_t d_tmem, uint32_t a_tm
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// arrive on the barrier at the same offset in CTA `rank` of the cluster
+// Arrive on the barrier at the same offset in CTA `rank` of the cluster, for signals whose data the tensor core reads:
+// bulk copies whose completion this thread has observed on its own barrier.  (The release is at CTA scope: at cluster
+// scope the arrival waits one to three thousand cycles for this SM's outstanding traffic, and what it would order --
+// this thread's own stores -- is not what the receiver reads.)
 __device__ __forceinline__ void mbar_arrive_remote(uint64_t* bar, uint32_t rank)
 {
     asm volatile(
         "{\n\t.reg .b32 ra;\n\t"
         "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-        "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
+        "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
         ::"r"(smem_u32(bar)), "r"(rank)
         : "memory");
 }

@@ -20,6 +20,7 @@ using namespace rkb200;
 
 namespace {
 constexpr int W8_N_TILE_MAX = 3072, W8_CHANNEL_TILE = 32;   // src/rk_npu_quant_matmul.cpp:50, src/rk_npu_internal.h:123
+constexpr int QUERY_SMS = 148;                               // the memory query has no device to ask: this GPU's SM count
 constexpr uint32_t W8_TIMEOUT_MS = 500;                      // the original's fixed plan timeout (src/rk_npu_quant_matmul.cpp:1709)
 
 struct W8Weights {
@@ -46,11 +47,13 @@ struct rk_npu_matmul_workspace {
     cudaStream_t stream = nullptr;
     int T = 0, KB = 0;
     uint8_t* codes = nullptr;
+    int* partials = nullptr;          // partial sums of tiles whose K is cut between CTA pairs
+    unsigned* counts = nullptr;       // and how far each such tile is
     float* scales = nullptr;          // [M] used scales, then [M] the caller's static scales
     Status* status = nullptr;
     void* stage_in = nullptr;
     void* stage_out = nullptr;
-    size_t codes_bytes = 0, scale_bytes = 0, stage_in_bytes = 0, stage_out_bytes = 0;
+    size_t codes_bytes = 0, partials_bytes = 0, counts_bytes = 0, scale_bytes = 0, stage_in_bytes = 0, stage_out_bytes = 0;
     Status* host_status = nullptr;    // pinned
     std::atomic<uint64_t> launches{0};
 };
@@ -89,22 +92,20 @@ bool valid_strategy(const rk_npu_matmul_strategy* s)
 }
 // what the kernels need on top: K within the contraction kernel's range, sizes that fit
 bool runnable_shape(int M, int N, int K) { return K <= 131072 && (int64_t)M * K <= INT32_MAX && (int64_t)M * N <= INT32_MAX; }
-// Up to 128 tokens: one token tile per CTA of the per-tile kernel.  Beyond: 128-token tiles, two per CTA pair of the
-// persistent kernel (the code buffer then covers whole pairs of tiles).
-int token_tile(int M) { return M > 128 ? 128 : align_up(M, 16); }
-int token_span(int M) { return M > 128 ? 256 : token_tile(M); }
-
 struct Sizes {
     int T, KB, NG;
-    size_t codes, scales, stage_in, stage_out, packed, wscales;
+    size_t codes, partials, counts, scales, stage_in, stage_out, packed, wscales;
 };
-Sizes sizes_of(int M, int N, int K, int kind)
+Sizes sizes_of(int M, int N, int K, int kind, int sm_count)
 {
     Sizes z{};
-    z.T = token_tile(M);
     z.KB = (K + KBLOCK - 1) / KBLOCK;
+    const int tok = gemm_tc_persist_tok(N, M, z.KB, sm_count);   // the code buffer covers whole pairs of token tiles
+    z.T = tok / 2;
     z.NG = align_up((N + GROUP - 1) / GROUP, 8) + 8;   // zero groups behind the last tile, as for the int4 weights
-    z.codes = size_t(align_up(M, token_span(M))) * size_t(z.KB) * KBLOCK;
+    z.codes = size_t(align_up(M, tok)) * size_t(z.KB) * KBLOCK;
+    z.partials = gemm_tc_persist_slot_bytes(sm_count, tok);
+    z.counts = gemm_tc_persist_count_bytes(N, M, tok);
     z.scales = sizeof(float) * 2 * size_t(M);
     const int in_elem = kind == RK_NPU_MATMUL_I8I8I32 ? 1 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? 2 : 4);
     const int out_elem = kind == RK_NPU_MATMUL_I8I8I32 ? 4 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? 2 : 4);
@@ -140,7 +141,7 @@ int weights_prepare(W8Weights& w, rk_npu_iommu_domain* domain, const rk_npu_matm
     rk_npu_ctx* ctx = domain->ctx;
     if (ctx->world > 1 || !runnable_shape(1, config->N, config->K)) return RK_NPU_ERR_PARAM;
     if (cudaSetDevice(ctx->device) != cudaSuccess) return RK_NPU_ERR_SUBMIT;
-    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32);
+    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32, ctx->sm_count);
     w.config = *config;
     w.KB = z.KB;
     w.NG = z.NG;
@@ -204,6 +205,8 @@ void workspace_destroy(rk_npu_matmul_workspace* ws)
     if (d) cudaSetDevice(d->ctx->device);
     if (ws->stream) cudaStreamSynchronize(ws->stream);
     if (ws->codes) device_free(d, ws->codes, ws->codes_bytes);
+    if (ws->partials) device_free(d, ws->partials, ws->partials_bytes);
+    if (ws->counts) device_free(d, ws->counts, ws->counts_bytes);
     if (ws->scales) device_free(d, ws->scales, ws->scale_bytes);
     if (ws->status) device_free(d, ws->status, sizeof(Status));
     if (ws->stage_in) device_free(d, ws->stage_in, ws->stage_in_bytes);
@@ -267,11 +270,12 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     g.epi = kind == RK_NPU_MATMUL_I8I8I32 ? EPI_I32 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? EPI_F16 : EPI_F32);
     g.split = 1;
     g.w8 = 1;
-    g.pair = st.M > 128 ? 1 : 0;
+    g.pair = 1;
+    g.partials = ws->partials;
+    g.counts = ws->counts;
+    g.max_clusters = ws->domain->ctx->sm_count / 2;
     g.timeout_ns = (unsigned long long)W8_TIMEOUT_MS * 1000000ull;
-    const bool persistent = g.pair && gemm_tc_persist_supported(g);
-    if (launch_w8_quantize(q, s) != cudaSuccess ||
-        (persistent ? launch_gemm_tc_persist(g, s, false) : launch_gemm_tc(g, s, false)) != cudaSuccess) {
+    if (launch_w8_quantize(q, s) != cudaSuccess || launch_gemm_tc_persist(g, s, false) != cudaSuccess) {
         cudaGetLastError();
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
@@ -282,6 +286,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
     if (ws->host_status->device_error) {       // a bounded wait inside the kernel ran out: report, clear, stay usable
         cudaMemsetAsync(&ws->status->device_error, 0, sizeof(int), s);
+        cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
     }
@@ -291,7 +296,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
 int weights_memory_query(const rk_npu_matmul_weight_config* config, bool with_scale, rk_npu_matmul_weight_requirements* out)
 {
     if (!valid_weight_config(config) || !out || !runnable_shape(1, config->N, config->K)) return RK_NPU_ERR_PARAM;
-    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32);
+    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32, QUERY_SMS);
     std::memset(out, 0, sizeof(*out));
     out->packed_b_bytes = z.packed;
     out->scale_bytes = with_scale ? uint64_t(config->N) * sizeof(float) : 0;   // the logical payload, as the original counts it
@@ -317,14 +322,14 @@ extern "C" int rk_npu_matmul_k_partition_query(int M, int K, int k_tile)
 extern "C" int rk_npu_matmul_workspace_memory_query(const rk_npu_matmul_strategy* strategy, rk_npu_matmul_workspace_requirements* out)
 {
     if (!strategy || !out || !valid_strategy(strategy) || !runnable_shape(strategy->M, strategy->N, strategy->K)) return RK_NPU_ERR_PARAM;
-    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind));
+    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind), QUERY_SMS);
     std::memset(out, 0, sizeof(*out));
     out->input_bytes = z.codes + z.stage_in;
-    out->output_bytes = z.stage_out;
-    out->control_bytes = z.scales + sizeof(Status);
+    out->output_bytes = z.stage_out + z.partials;
+    out->control_bytes = z.scales + z.counts + sizeof(Status);
     out->bytes = out->input_bytes + out->output_bytes + out->control_bytes;
     out->wave_count = uint32_t((strategy->K + strategy->k_tile - 1) / strategy->k_tile);
-    out->buffer_count = 5;
+    out->buffer_count = 7;
     return RK_NPU_OK;
 }
 extern "C" int rk_npu_i8i8i32_weights_memory_query(const rk_npu_matmul_weight_config* c, rk_npu_matmul_weight_requirements* out) { return weights_memory_query(c, false, out); }
@@ -340,7 +345,7 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     if (cudaSetDevice(ctx->device) != cudaSuccess) return nullptr;
     rk_npu_matmul_workspace* ws = new (std::nothrow) rk_npu_matmul_workspace();
     if (!ws) return nullptr;
-    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind));
+    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind), ctx->sm_count);
     ws->strategy = *strategy;
     ws->domain = domain;
     ws->ctx_id = ctx->id;
@@ -348,6 +353,8 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     ws->T = z.T;
     ws->KB = z.KB;
     ws->codes_bytes = z.codes;
+    ws->partials_bytes = z.partials;
+    ws->counts_bytes = z.counts;
     ws->scale_bytes = z.scales;
     ws->stage_in_bytes = z.stage_in;
     ws->stage_out_bytes = z.stage_out;
@@ -355,11 +362,14 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     bool ok = cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMallocHost(reinterpret_cast<void**>(&ws->host_status), sizeof(Status)) == cudaSuccess;
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes) &&
+         !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
+         !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), ws->scale_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status)) &&
          !device_alloc(domain, &ws->stage_in, ws->stage_in_bytes) && !device_alloc(domain, &ws->stage_out, ws->stage_out_bytes);
     // codes of the tokens that pad the last tile stay zero for the life of the workspace
     ok = ok && cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
+         cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess &&
          cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess && cudaStreamSynchronize(ws->stream) == cudaSuccess;
     if (!ok) { cudaGetLastError(); workspace_destroy(ws); return nullptr; }
     return ws;
