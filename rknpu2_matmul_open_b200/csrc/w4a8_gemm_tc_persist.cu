@@ -394,9 +394,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         if (tr) { trace[128] = (unsigned long long)wait_full; trace[129] = (unsigned long long)wait_free; }
     } else {
         // ---------------------------------------------------------------- epilogue warps
+        // A warp finishes sixteen tokens (of its 32 accumulator rows) per turn of a rolled loop.  What bounds it is the
+        // number of instructions: eight warps share the issue slots with the unpack warps, so the arithmetic works on pairs
+        // of tokens (one instruction per two operations).
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes 32-token chunks eset, eset + 2, ...
-        constexpr int CHUNKS = TOK / 64;
         const int sid = (warp - PS_EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const int out_cols = swiglu ? p.F : p.N;
@@ -406,31 +408,31 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         const int odd = lane & 1;
         const bool quad_ok = (out_cols % 4 == 0) && (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
         constexpr int SHIFT = W8 ? 0 : 4;             // int4 records enter the MMA times 16
-        const bool small_sums = (long long)KB * KBLOCK * (W8 ? 127 : 7) * 127 < (1ll << 22);
         bool ok = dependency_met();
         RingPos<S::ACC> rc;
         int tile = tile0, it = it0;
         for (int gi = 0, j = 0; gi < n_items && ok; ++j, rc.next()) {
             const int n_seg = min(nst - it, n_items - gi);
             const bool whole = n_seg == nst;                 // this segment covers its tile's whole K
-            const bool last_seg = gi + n_seg >= n_items;
             const int ct = 2 * (tile % pairs_n) + (int)rank;
             const int tok_base = (tile / pairs_n) * TOK;
             const int col0 = swiglu ? ct * 64 : ct * TILE_N;
             const int n = col0 + col;
             const bool n_ok = n < out_cols;
             const float sw = n_ok ? p.sw[(up_lane ? p.F : 0) + n] : 0.f;
-            float* const sx = s_sx;
+            // 32-token chunks of this warp that hold live tokens: those at 32 eset + 64 c, c < chunks
+            const int chunks = max(0, min(TOK / 64, (p.M - tok_base - 32 * eset + 63) / 64));
             if (sid < TOK) {
                 const int m = tok_base + sid;
-                sx[sid] = m < p.M ? p.sx[m] : 0.f;
+                s_sx[sid] = m < p.M ? p.sx[m] : 0.f;
             }
             asm volatile("bar.sync 1, 256;" ::: "memory");   // scales staged (the barrier at the end of a tile keeps stragglers out)
             ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // one verdict for all eight warps
             if (!ok) { *s_error = 1; break; }
             if (sid == 0) PS_STAMP(j, 3);
             tc_fence_after();
-            const uint32_t acc_addr = lane_addr + rc.slot * TOK;
+            const uint32_t acc_addr = lane_addr + rc.slot * TOK + 32 * eset;
+            const int row = q * 32 + lane;
             auto hand_back = [&]() {   // this warp is done with the accumulator: another segment's MMAs may overwrite it
                 tc_fence_before();
                 __syncwarp();
@@ -443,18 +445,15 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
             // one partial segment each, so two slots per CTA suffice.
             int part_lo = 0, part_hi = -1;                   // contributing clusters when the sums come from slots
             if (!whole) {
-                int4* const slot = reinterpret_cast<int4*>(p.partials) + ((size_t)(2 * cluster_id + (gi == 0 ? 0 : 1)) * 2 + rank) * (S::SLOT_INTS / 4);
+                int4* const slot = reinterpret_cast<int4*>(p.partials) + ((size_t)(2 * cluster_id + (gi == 0 ? 0 : 1)) * 2 + rank) * (S::SLOT_INTS / 4) + (size_t)(8 * eset) * 128 + row;   // [token / 4][row][4 tokens]
 #pragma unroll 1
-                for (int c = 0; c < CHUNKS; ++c) {
-                    const int t0 = eset * 32 + 64 * c;
-                    if (tok_base + t0 < p.M) {
-                        uint32_t r[32];
-                        tc_ld32(acc_addr + t0, r);
-                        tc_wait_ld();
-                        int4* const dst = slot + (size_t)(t0 / 4) * 128 + q * 32 + lane;
+                for (int c = 0; c < chunks; ++c) {
+                    uint32_t r[32];
+                    tc_ld32(acc_addr + 64 * c, r);
+                    tc_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) dst[(size_t)i * 128] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
-                    }
+                    for (int i = 0; i < 8; ++i)
+                        slot[(size_t)(16 * c + i) * 128] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
                 }
                 hand_back();
                 __threadfence();
@@ -475,213 +474,163 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                     part_hi = (int)(((s0 + nst) * num_clusters - 1) / total);
                 }
             }
-            const bool finish = whole || part_hi >= part_lo;
-            // The tensor pipe stands still until the accumulator is handed back.  Where finishing a chunk is expensive
-            // (`park`: the SwiGLU epilogue, fp32 / int32 stores) the first three chunks are only moved: tensor memory ->
-            // registers -> this thread's own slots of a scratch in global memory (it stays in L2); the fourth stays in
-            // registers, the accumulator goes back, and then the four chunks are finished, the parked ones read back
-            // by the thread that wrote them.
-            const bool park = S::ACC == 1 && whole && p.park != nullptr && !last_seg;   // (nothing waits behind a cluster's last tile)
-            int* const park_at = park ? p.park + (size_t)blockIdx.x * PS_PARK_INTS + sid : nullptr;
-            if (park) {
+            if (whole && chunks == 0) hand_back();
+            const int turns = whole || part_hi >= part_lo ? 2 * chunks : 0;
 #pragma unroll 1
-                for (int c = 0; c < 3; ++c) {
-                    const int t0 = eset * 32 + 64 * c;
-                    if (tok_base + t0 >= p.M) continue;
-                    uint32_t r[32];
-                    tc_ld32(acc_addr + t0, r);
+            for (int k = 0; k < turns; ++k) {
+                const int t0 = 32 * eset + 64 * (k >> 1) + 16 * (k & 1), m0 = tok_base + t0;
+                uint32_t r[16];
+                if (whole) {
+                    tc_ld16(lane_addr + rc.slot * TOK + t0, r);
                     tc_wait_ld();
+                    if (k + 1 == turns) hand_back();
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) __stcg(park_at + (c * 32 + i) * 256, (int)r[i]);
-                }
-            }
-            long long phase_t = (trace && sid == 0) ? clock64() : 0;
-            // (diagnostics) cycles the first epilogue thread spends per phase of finishing, summed over the launch:
-            // [176] getting a chunk into registers, [177] scales and conversion, [178] the epilogue proper and its stores
-            // (SwiGLU: [180] dequantisation, [181] pairing and SiLU, [182] stores, and [178] what is left: the row maxima)
-            auto phase = [&](int which) {
-                if (trace && sid == 0) { const long long now = clock64(); trace[176 + which] += (unsigned long long)(now - phase_t); phase_t = now; }
-            };
+                    for (int i = 0; i < 16; ++i) r[i] = 0u;
 #pragma unroll 1
-            for (int k = 0; k < (finish ? CHUNKS : 0); ++k) {
-                const int c = park ? (k + CHUNKS - 1) % CHUNKS : k;
-                const int t0 = eset * 32 + 64 * c;
-                const bool live_chunk = tok_base + t0 < p.M;
-                uint32_t r[32];
-                if (live_chunk) {
-                    if (!whole) {
+                    for (int cc = part_lo; cc <= part_hi; cc += 2) {       // two contributors' loads in flight at a time
+                        int4 v[2][4];
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = 0u;
-#pragma unroll 1
-                        for (int cc = part_lo; cc <= part_hi; ++cc) {
-                            // a cluster whose run starts inside the tile contributed its first segment, another one its last
-                            const int which = total * cc / num_clusters >= (long long)tile * nst ? 0 : 1;
-                            const int4* const src = reinterpret_cast<const int4*>(p.partials) + ((size_t)(2 * cc + which) * 2 + rank) * (S::SLOT_INTS / 4) + (size_t)(t0 / 4) * 128 + q * 32 + lane;
-                            int4 v[8];
+                        for (int c = 0; c < 2; ++c)
+                            if (cc + c <= part_hi) {
+                                // a cluster whose run starts inside the tile contributed its first segment, another one its last
+                                const int which = total * (cc + c) / num_clusters >= (long long)tile * nst ? 0 : 1;
+                                const int4* const src = reinterpret_cast<const int4*>(p.partials) + ((size_t)(2 * (cc + c) + which) * 2 + rank) * (S::SLOT_INTS / 4) + (size_t)(t0 / 4) * 128 + row;
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) v[i] = __ldcg(src + (size_t)i * 128);
+                                for (int h = 0; h < 4; ++h) v[c][h] = __ldcg(src + (size_t)h * 128);
+                            } else {
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) {
-                                r[4 * i] += (uint32_t)v[i].x; r[4 * i + 1] += (uint32_t)v[i].y; r[4 * i + 2] += (uint32_t)v[i].z; r[4 * i + 3] += (uint32_t)v[i].w;
+                                for (int h = 0; h < 4; ++h) v[c][h] = make_int4(0, 0, 0, 0);
                             }
-                        }
-                    } else if (!park || k == 0) {
-                        tc_ld32(acc_addr + t0, r);
-                        tc_wait_ld();
-                    } else {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = (uint32_t)__ldcg(park_at + (c * 32 + i) * 256);
+                        for (int c = 0; c < 2; ++c)
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) {
+                                r[4 * h] += (uint32_t)v[c][h].x; r[4 * h + 1] += (uint32_t)v[c][h].y; r[4 * h + 2] += (uint32_t)v[c][h].z; r[4 * h + 3] += (uint32_t)v[c][h].w;
+                            }
                     }
                 }
-                if (whole && k == (park ? 0 : CHUNKS - 1)) hand_back();
-                if (!live_chunk) continue;
-                phase(0);
-                // All loads of a chunk come first, then the arithmetic, then the stores: the compiler
-                // may not move a load across a store it cannot prove unrelated, and one store per
-                // loop iteration would serialise the whole chunk on the latency of each iteration.
-                const int m0 = tok_base + t0;
-                float sxr[32];
+                if (m0 >= p.M) continue;
+                if (p.epi == EPI_I32) {
+                    int* const row0 = reinterpret_cast<int*>(p.out) + (size_t)m0 * out_cols + n;
+                    if (n_ok) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (m0 + i < p.M) row0[(size_t)i * out_cols] = (int)r[i] >> SHIFT;
+                    }
+                    continue;
+                }
+                // y[i]: tokens m0 + 2i and m0 + 2i + 1.  (float)(16 s) / 16 is (float)s, exactly.
+                F2 y[8];
                 {
-                    const float4* sx4 = reinterpret_cast<const float4*>(sx + t0);
+                    const ulonglong2* const sx2 = reinterpret_cast<const ulonglong2*>(s_sx + t0);
+                    const F2 sw2 = f2_all(sw);
 #pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        const float4 f = sx4[v];
-                        sxr[4 * v] = f.x; sxr[4 * v + 1] = f.y; sxr[4 * v + 2] = f.z; sxr[4 * v + 3] = f.w;
+                    for (int i = 0; i < 4; ++i) {
+                        const ulonglong2 sx = sx2[i];
+                        y[2 * i] = f2_pack(__int2float_rn((int)r[4 * i]), __int2float_rn((int)r[4 * i + 1]));
+                        y[2 * i + 1] = f2_pack(__int2float_rn((int)r[4 * i + 2]), __int2float_rn((int)r[4 * i + 3]));
+                        if constexpr (!W8) { y[2 * i] = f2_mul(y[2 * i], f2_all(0.0625f)); y[2 * i + 1] = f2_mul(y[2 * i + 1], f2_all(0.0625f)); }
+                        y[2 * i] = f2_mul(f2_mul(y[2 * i], sx.x), sw2);
+                        y[2 * i + 1] = f2_mul(f2_mul(y[2 * i + 1], sx.y), sw2);
                     }
                 }
-                // int32 sum (a multiple of 16) -> float, rounded to nearest like the conversion instruction.
-                // The conversion unit is an eighth as wide as the FP32 pipe and would bound the whole
-                // drain, so when the bound K * 7 * 127 keeps every sum below 2^22 the exact
-                // magic-number form is used: bits(1.5 * 2^23) + v read as a float is 1.5 * 2^23 + v.
-                if (p.epi != EPI_I32) {
-                    if (small_sums) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__fsub_rn(__uint_as_float(0x4B400000u + (uint32_t)((int)r[i] >> SHIFT)), 12582912.f));
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__int2float_rn((int)r[i] >> SHIFT));
-                    }
-                }
-                phase(1);
                 if (p.epi == EPI_F16) {
-                    // a lane holds one channel of 32 tokens; neighbouring lanes swap halves so that
-                    // every lane stores two neighbouring channels of one token as one 32-bit word
-                    __half* const out = reinterpret_cast<__half*>(p.out);
-                    uint32_t word[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const float y0 = __fmul_rn(__fmul_rn(__uint_as_float(r[2 * i]), sxr[2 * i]), sw);
-                        const float y1 = __fmul_rn(__fmul_rn(__uint_as_float(r[2 * i + 1]), sxr[2 * i + 1]), sw);
-                        const __half2 h = __floats2half2_rn(y0, y1);
-                        word[i] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                    // two exchange rounds turn (one channel, 32 tokens) per lane into (four neighbouring
-                    // channels, 8 tokens) per lane: lanes 4g..4g+3 end up with tokens 4i + (lane & 3)
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const uint32_t other = __shfl_xor_sync(0xffffffffu, word[i], 1);
-                        word[i] = odd ? __byte_perm(other, word[i], 0x7632) : __byte_perm(word[i], other, 0x5410);
-                    }
-                    const bool upper = (lane & 2) != 0;
+                    // a lane holds one channel of sixteen tokens; two exchange rounds turn that into four neighbouring
+                    // channels of four tokens: lanes 4g..4g+3 end up with tokens 4i + (lane & 3)
+                    uint32_t word[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
+                        float lo, hi;
+                        f2_unpack(y[i], lo, hi);
+                        const __half2 h = __floats2half2_rn(lo, hi);
+                        word[i] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                    const uint32_t selector = odd ? 0x3276u : 0x5410u;     // even lanes: low halves (own, peer's); odd lanes: high halves (peer's, own)
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) word[i] = __byte_perm(word[i], __shfl_xor_sync(0xffffffffu, word[i], 1), selector);
+                    const bool upper = (lane & 2) != 0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
                         const uint32_t recv = __shfl_xor_sync(0xffffffffu, upper ? word[2 * i] : word[2 * i + 1], 2);
                         if (upper) word[2 * i] = recv; else word[2 * i + 1] = recv;
                         // now (word[2i], word[2i+1]) = channels n4 .. n4+3 of token m0 + 4i + (lane & 3)
                     }
                     const int n4 = n - (lane & 3);
-                    const int mrow = m0 + 2 * (int)upper + odd;
-                    __half* const row0 = out + (size_t)mrow * out_cols + n4;
-                    if (quad_ok && n4 + 3 < out_cols) {
+                    const int mrow = m0 + (lane & 3);
+                    __half* dst = reinterpret_cast<__half*>(p.out) + (size_t)mrow * out_cols + n4;
+                    const size_t step = 4 * (size_t)out_cols;
 #pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (mrow + 4 * i < p.M) *reinterpret_cast<uint2*>(row0 + (size_t)(4 * i) * out_cols) = make_uint2(word[2 * i], word[2 * i + 1]);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (mrow + 4 * i < p.M) {
-                                __half* dst = row0 + (size_t)(4 * i) * out_cols;
+                    for (int i = 0; i < 4; ++i, dst += step)
+                        if (mrow + 4 * i < p.M) {
+                            if (quad_ok && n4 + 3 < out_cols) *reinterpret_cast<uint2*>(dst) = make_uint2(word[2 * i], word[2 * i + 1]);
+                            else {
                                 const uint32_t ww[2] = {word[2 * i], word[2 * i + 1]};
 #pragma unroll
                                 for (int e = 0; e < 4; ++e)
                                     if (n4 + e < out_cols) dst[e] = __ushort_as_half((unsigned short)((ww[e >> 1] >> (16 * (e & 1))) & 0xffffu));
                             }
-                    }
-                } else if (p.epi == EPI_F32 || p.epi == EPI_I32) {
-                    const bool f32 = p.epi == EPI_F32;
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        r[i] = f32 ? __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[i]), sxr[i]), sw)) : (uint32_t)((int)r[i] >> SHIFT);
-                    }
-                    uint32_t* const row0 = reinterpret_cast<uint32_t*>(p.out) + (size_t)m0 * out_cols + n;
+                        }
+                } else if (p.epi == EPI_F32) {
+                    float* dst = reinterpret_cast<float*>(p.out) + (size_t)m0 * out_cols + n;
                     if (n_ok) {
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (m0 + i < p.M) row0[(size_t)i * out_cols] = r[i];
+                        for (int i = 0; i < 8; ++i, dst += 2 * (size_t)out_cols) {
+                            float lo, hi;
+                            f2_unpack(y[i], lo, hi);
+                            if (m0 + 2 * i < p.M) dst[0] = lo;
+                            if (m0 + 2 * i + 1 < p.M) dst[out_cols] = hi;
+                        }
                     }
                 } else {
-                    // Lanes 0-15 hold the gate rows g, lanes 16-31 the matching up rows u of 16 features.  For
-                    // every token pair the halves swap what the other needs, so that the gate lanes finish the
-                    // even token and the up lanes the odd one: each lane evaluates 16 SiLUs instead of 32.
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__fmul_rn(__fmul_rn(__uint_as_float(r[i]), sxr[i]), sw));
-                    float y[16];
-                    uint32_t mx[16];
+                    // Lanes 0-15 hold the gate rows g, lanes 16-31 the matching up rows u of 16 features.  The gate lanes
+                    // finish the even token of every pair and the up lanes the odd one: each sends the half of the pair
+                    // that the other finishes and evaluates eight SiLUs.
+                    uint32_t mx[8];
                     const int mine_row = m0 + (up_lane ? 1 : 0);
-                    phase(4);
+                    float* dst = reinterpret_cast<float*>(p.out) + (size_t)mine_row * out_cols + n;
 #pragma unroll
-                    for (int i0 = 0; i0 < 16; i0 += 4) {     // four tokens in lock step (see silu_poly4)
-                        float g4[4], u4[4], s4[4];
+                    for (int i = 0; i < 8; i += 2) {
+                        float g[2], u[2], v[2];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int i = i0 + k;
-                            const float a0 = __uint_as_float(r[2 * i]), a1 = __uint_as_float(r[2 * i + 1]);
-                            const float o0 = __shfl_xor_sync(0xffffffffu, a0, 16);   // gate lanes: u of token 2i; up lanes: g of token 2i
-                            const float o1 = __shfl_xor_sync(0xffffffffu, a1, 16);   // gate lanes: u of token 2i+1; up lanes: g of token 2i+1
-                            g4[k] = up_lane ? o1 : a0;
-                            u4[k] = up_lane ? a1 : o0;
+                        for (int e = 0; e < 2; ++e) {
+                            float even_token, odd_token;
+                            f2_unpack(y[i + e], even_token, odd_token);
+                            const float recv = __shfl_xor_sync(0xffffffffu, up_lane ? even_token : odd_token, 16);
+                            g[e] = up_lane ? recv : even_token;
+                            u[e] = up_lane ? odd_token : recv;
                         }
-                        silu_poly4(g4, s4);
+                        silu_poly2(g[0], g[1], v[0], v[1]);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const int i = i0 + k;
-                            y[i] = __fmul_rn(s4[k], u4[k]);
-                            const bool live = n_ok && mine_row + 2 * i < p.M;
-                            mx[i] = live ? (__float_as_uint(y[i]) & 0x7fffffffu) : 0u;
+                        for (int e = 0; e < 2; ++e, dst += 2 * (size_t)out_cols) {
+                            v[e] = __fmul_rn(v[e], u[e]);
+                            const bool live = n_ok && mine_row + 2 * (i + e) < p.M;
+                            if (live) *dst = v[e];
+                            mx[i + e] = live ? (__float_as_uint(v[e]) & 0x7fffffffu) : 0u;
                         }
                     }
-                    phase(5);
-                    float* const row0 = reinterpret_cast<float*>(p.out) + (size_t)mine_row * out_cols + n;
-                    if (n_ok) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (mine_row + 2 * i < p.M) row0[(size_t)(2 * i) * out_cols] = y[i];
-                    }
-                    phase(6);
                     if (p.rowmax) {
-                        // Maxima over the 16 lanes of each half, one token per value: a folding exchange that halves
-                        // the values a lane holds at every step (8 + 4 + 2 + 1 shuffles instead of 16 x 4); lane l of
-                        // a half ends up with the maximum of token l & 15 and issues that token's one atomic.
+                        // Maxima over the 16 lanes of each half, one token per value: three folding steps that halve the
+                        // values a lane holds and a plain one; lanes 2i of a half end up with the maximum of their token.
 #pragma unroll
-                        for (int width = 8; width > 0; width >>= 1) {
+                        for (int width = 8; width > 1; width >>= 1) {
                             const bool upper = (lane & width) != 0;
 #pragma unroll
-                            for (int k = 0; k < width; ++k) {
-                                const uint32_t keep = upper ? mx[k + width] : mx[k];
-                                const uint32_t give = upper ? mx[k] : mx[k + width];
-                                mx[k] = max(keep, __shfl_xor_sync(0xffffffffu, give, width));
+                            for (int i = 0; i < width / 2; ++i) {
+                                const uint32_t keep = upper ? mx[i + width / 2] : mx[i];
+                                const uint32_t give = upper ? mx[i] : mx[i + width / 2];
+                                mx[i] = max(keep, __shfl_xor_sync(0xffffffffu, give, width));
                             }
                         }
+                        mx[0] = max(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], 1));
                         // collected per CTA and tile in shared memory first: one global atomic per token and tile
                         // instead of one per token, tile and 16 features
-                        if (mx[0]) atomicMax(&s_tilemax[t0 + (up_lane ? 1 : 0) + 2 * (lane & 15)], mx[0]);
+                        if (!odd && mx[0]) atomicMax(&s_tilemax[t0 + (up_lane ? 1 : 0) + 2 * ((lane >> 1) & 7)], mx[0]);
                     }
                 }
-                phase(2);
             }
             if (sid == 0) PS_STAMP(j, 5);
             asm volatile("bar.sync 1, 256;" ::: "memory");   // every epilogue warp is done with this tile's scales and maxima
-            phase(3);
             if (swiglu && p.rowmax && sid < TOK) {
                 const uint32_t m = s_tilemax[sid];
                 if (m) {

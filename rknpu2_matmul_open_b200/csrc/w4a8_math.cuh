@@ -99,60 +99,63 @@ __device__ __forceinline__ void load16(const typename ActType<HALF>::type* row, 
     raw_to_float<HALF>(r, v);
 }
 
+// Pairs of floats in one 64-bit register pair: one instruction per two operations, each rounded on its own exactly like
+// the scalar instruction.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) { F2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi)); return d; }
+__device__ __forceinline__ void f2_unpack(F2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ F2 f2_add_rm(F2 a, F2 b) { F2 d; asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ F2 f2_all(float v) { return f2_pack(v, v); }
+
 // Degree-7 polynomial SiLU of the reference's production target, every rounding kept:
-// src/rk_npu_swiglu_fp32_neon.h:17-41.
+// src/rk_npu_swiglu_fp32_neon.h:17-41.  Two arguments at a time.
+//   * floor(y) for |y| < 2^22: adding 1.5 * 2^23 with rounding towards minus infinity leaves floor(y) in the low bits,
+//     from where the subtraction brings it back as a float and a shift puts it into the exponent of 2^n.
+//   * g / d, correctly rounded: a reciprocal within an ulp refined by one Newton step, a quotient from it, its remainder
+//     by fused multiply-add (exact) and one correction (P. Markstein, "Computation of elementary functions on the IBM
+//     RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  Magnitudes for which a step could leave the normal range
+//     take the division instruction sequence.
+// Equal bit for bit to the scalar statement of the reference's routine for every one of the 2^32 arguments (checked).
+__device__ __forceinline__ void silu_poly2(float g0, float g1, float& y0, float& y1)
+{
+    const F2 g = f2_pack(g0, g1);
+    const F2 x = f2_pack(fminf(fmaxf(-g0, -80.f), 80.f), fminf(fmaxf(-g1, -80.f), 80.f));
+    const F2 shifted = f2_add_rm(f2_fma(x, f2_all(1.4426950408889634f), f2_all(0.5f)), f2_all(12582912.f));
+    const F2 n = f2_add(shifted, f2_all(-12582912.f));
+    F2 r = f2_fma(n, f2_all(-0.693145751953125f), x);
+    r = f2_fma(n, f2_all(-1.428606765330187e-6f), r);
+    F2 q = f2_fma(f2_all(1.f / 5040.f), r, f2_all(1.f / 720.f));
+    q = f2_fma(q, r, f2_all(1.f / 120.f));
+    q = f2_fma(q, r, f2_all(1.f / 24.f));
+    q = f2_fma(q, r, f2_all(1.f / 6.f));
+    q = f2_fma(q, r, f2_all(0.5f));
+    q = f2_fma(q, r, f2_all(1.f));
+    q = f2_fma(q, r, f2_all(1.f));
+    float s0, s1;
+    f2_unpack(shifted, s0, s1);
+    const F2 power = f2_pack(__int_as_float((__float_as_int(s0) << 23) + (127 << 23)), __int_as_float((__float_as_int(s1) << 23) + (127 << 23)));
+    const F2 d = f2_add(f2_all(1.f), f2_mul(q, power));
+    float d0, d1, r0, r1;
+    f2_unpack(d, d0, d1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
+    const F2 minus_d = f2_pack(-d0, -d1), rough = f2_pack(r0, r1);
+    const F2 inv = f2_fma(rough, f2_fma(minus_d, rough, f2_all(1.f)), rough);
+    const F2 quo = f2_mul(g, inv);
+    f2_unpack(f2_fma(f2_fma(minus_d, quo, g), inv, quo), y0, y1);
+    // |g| in [2^-40, 80]: d < 2^116, so quotient and remainder are normal numbers (or the remainder is zero)
+    const bool plain0 = fabsf(g0) >= 9.094947017729282e-13f && fabsf(g0) <= 80.f, plain1 = fabsf(g1) >= 9.094947017729282e-13f && fabsf(g1) <= 80.f;
+    if (!plain0) y0 = g0 < -80.f ? -0.f : __fdiv_rn(g0, d0);
+    if (!plain1) y1 = g1 < -80.f ? -0.f : __fdiv_rn(g1, d1);
+}
 __device__ __forceinline__ float silu_poly(float g)
 {
-    float x = fminf(fmaxf(-g, -80.f), 80.f);
-    const float n = floorf(fmaf(x, 1.4426950408889634f, 0.5f));
-    float r = fmaf(-n, 0.693145751953125f, x);
-    r = fmaf(-n, 1.428606765330187e-6f, r);
-    float q = 1.f / 5040.f;
-    q = fmaf(q, r, 1.f / 720.f);
-    q = fmaf(q, r, 1.f / 120.f);
-    q = fmaf(q, r, 1.f / 24.f);
-    q = fmaf(q, r, 1.f / 6.f);
-    q = fmaf(q, r, 0.5f);
-    q = fmaf(q, r, 1.f);
-    q = fmaf(q, r, 1.f);
-    const float power = __int_as_float(((int)n + 127) << 23);
-    const float d = __fadd_rn(1.f, __fmul_rn(q, power));
-    return g < -80.f ? -0.f : __fdiv_rn(g, d);
-}
-// The same function for four arguments in lock step: every statement is applied to all four values before the next
-// one.  Each value goes through exactly the operations of silu_poly (same bits); what changes is that the four
-// dependent chains are interleaved in program order -- written one value after the other, sixteen evaluations took
-// 2190 cycles per warp, in lock step 1420 (the divisions sit in separate basic blocks and are not interleaved by
-// the compiler on its own).
-__device__ __forceinline__ void silu_poly4(const float (&g)[4], float (&y)[4])
-{
-    float x[4], n[4], r[4], q[4], d[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) x[j] = fminf(fmaxf(-g[j], -80.f), 80.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) n[j] = floorf(fmaf(x[j], 1.4426950408889634f, 0.5f));
-#pragma unroll
-    for (int j = 0; j < 4; ++j) r[j] = fmaf(-n[j], 0.693145751953125f, x[j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) r[j] = fmaf(-n[j], 1.428606765330187e-6f, r[j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(1.f / 5040.f, r[j], 1.f / 720.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(q[j], r[j], 1.f / 120.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(q[j], r[j], 1.f / 24.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(q[j], r[j], 1.f / 6.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(q[j], r[j], 0.5f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(q[j], r[j], 1.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = fmaf(q[j], r[j], 1.f);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) d[j] = __fadd_rn(1.f, __fmul_rn(q[j], __int_as_float(((int)n[j] + 127) << 23)));
-#pragma unroll
-    for (int j = 0; j < 4; ++j) y[j] = g[j] < -80.f ? -0.f : __fdiv_rn(g[j], d[j]);
+    float y, unused;
+    silu_poly2(g, g, y, unused);
+    return y;
 }
 __device__ __forceinline__ float dequant(int acc, float sx, float sw)
 {
