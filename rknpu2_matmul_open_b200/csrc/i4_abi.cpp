@@ -42,7 +42,7 @@ struct rk_npu_i4_workspace {
     uint32_t domain_id = 0;
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
     cudaStream_t stream = nullptr;
-    int T = 0, KB = 0;
+    int T = 0, KB = 0, parts = 1;
     uint8_t* codes = nullptr;
     int* partials = nullptr;         // partial sums of tiles whose K is cut between CTA pairs
     unsigned* counts = nullptr;      // and how far each such tile is
@@ -128,11 +128,9 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     g.M = cfg.M; g.N = cfg.N; g.K = cfg.K;
     g.KB = ws->KB; g.NG = w->NG; g.T = ws->T;
     g.epi = EPI_I32;
-    g.split = 1;
-    g.pair = 1;
+    g.split = ws->parts;
     g.partials = ws->partials;
     g.counts = ws->counts;
-    g.max_clusters = ws->domain->ctx->sm_count / 2;
     g.timeout_ns = (unsigned long long)cfg.timeout_ms * 1000000ull;
     const auto t0 = Clock::now();
     if (launch_w8_quantize(q, s) != cudaSuccess || launch_gemm_tc_persist(g, s, false) != cudaSuccess) {
@@ -146,7 +144,7 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     times.submit_us += since(t0);
     if (ws->host_status->device_error) {
         cudaMemsetAsync(&ws->status->device_error, 0, sizeof(int), s);
-        cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
+        if (ws->counts) cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
     }
@@ -242,24 +240,25 @@ extern "C" rk_npu_i4_workspace* rk_npu_i4_workspace_create(rk_npu_iommu_domain* 
         ws->domain_id = domain->id;
         domain_retain(domain);
         ws->KB = (cfg->K + KBLOCK - 1) / KBLOCK;
-        const int tok = gemm_tc_persist_tok(cfg->N, cfg->M, ws->KB, ctx->sm_count);   // the code buffer covers whole pairs of token tiles
-        ws->T = tok / 2;
-        ws->codes_bytes = size_t(align_up(cfg->M, tok)) * size_t(ws->KB) * KBLOCK;
-        ws->partials_bytes = gemm_tc_persist_slot_bytes(ctx->sm_count, tok);
-        ws->counts_bytes = gemm_tc_persist_count_bytes(cfg->N, cfg->M, tok);
+        const PersistPlan plan = gemm_tc_persist_plan(cfg->N, cfg->M, ws->KB, false, ctx->sm_count);
+        ws->T = plan.tok / 2;
+        ws->parts = plan.split;
+        ws->codes_bytes = size_t(align_up(cfg->M, plan.tok)) * size_t(ws->KB) * KBLOCK;
+        ws->partials_bytes = gemm_tc_persist_slot_bytes(cfg->N, cfg->M, plan);
+        ws->counts_bytes = gemm_tc_persist_count_bytes(cfg->N, cfg->M, plan);
         ws->stage_in_bytes = size_t(cfg->M) * cfg->K;
         ws->stage_out_bytes = size_t(cfg->M) * cfg->N * sizeof(int32_t);
         bool ok = cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaMallocHost(reinterpret_cast<void**>(&ws->host_status), sizeof(Status)) == cudaSuccess;
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes) &&
-             !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
-             !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes) &&
+             (!ws->partials_bytes || (!device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
+                                      !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes))) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), sizeof(float) * cfg->M) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status)) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->stage_in), ws->stage_in_bytes) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->stage_out), ws->stage_out_bytes);
         ok = ok && cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
-             cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess &&
+             (!ws->counts || cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess) &&
              cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess && cudaStreamSynchronize(ws->stream) == cudaSuccess;
         if (!ok) { cudaGetLastError(); return nullptr; }
         return ws.release();

@@ -1,7 +1,7 @@
 // w4a8_abi.cpp -- the C ABI of the W4A8 path: context and domains, geometry
 // validation and memory accounting, weight preparation, workspaces and the run entry
 // points.  Host C++ only; every tensor operation is a CUDA kernel (w4a8_kernels.cu,
-// w4a8_gemm_tc.cu).  There is no CPU compute path: without a GPU rk_npu_open fails.
+// w4a8_gemm_tc_persist.cu, w4a8_decode.cu, ...).  There is no CPU compute path: without a GPU rk_npu_open fails.
 //
 // Behaviour mirrors the reference operator front-end src/rk_npu_w4a8.cpp (validation
 // order :83-94, BUSY guard :70-81, run :98-159, accounting :169-207, FFN :354-380) and
@@ -479,17 +479,10 @@ int enqueue(const Call& c)
     g.trace = ws.trace;
     cudaError_t err;
     if (ws.variant == 2) {
-        g.split = 1;
-        g.pair = ws.pair ? 1 : 0;
-        // parking pays where finishing a chunk is expensive, i.e. for the SwiGLU epilogue (measured: the plain epilogues gain
-        // nothing, the extra L2 traffic lengthens their MMA phase as much as the earlier hand-back saves);
-        // RK_NPU_B200_PARK_ALL=1 parks for every epilogue (experiments)
-        if (c.epi == EPI_SWIGLU || env_flag("RK_NPU_B200_PARK_ALL", false)) g.park = ws.park;
         g.partials = ws.partials;
         g.counts = ws.counts;
-        g.max_clusters = ws.domain->ctx->sm_count / 2;
-        if (gemm_tc_persist_supported(g) && !env_flag("RK_NPU_B200_NO_PERSIST", false)) err = launch_gemm_tc_persist(g, c.stream, pdl);
-        else err = launch_gemm_tc(g, c.stream, pdl);
+        g.split = ws.parts;
+        err = launch_gemm_tc_persist(g, c.stream, pdl);
     } else if (ws.variant == 4) {
         g.split = 1;
         g.partials = ws.partials;
@@ -655,7 +648,6 @@ void workspace_destroy(rk_npu_w4a8_workspace* ws)
     if (ws->trace) device_free(d, ws->trace, ws->trace_bytes);
     if (ws->partials) device_free(d, ws->partials, ws->partials_bytes);
     if (ws->counts) device_free(d, ws->counts, ws->counts_bytes);
-    if (ws->park) device_free(d, ws->park, ws->park_bytes);
     if (ws->gather) device_free(d, ws->gather, ws->gather_bytes);
     if (ws->code_gather) device_free(d, ws->code_gather, ws->code_gather_bytes);
     if (ws->host_status) cudaFreeHost(ws->host_status);
@@ -1034,15 +1026,11 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     ws->shard_N = ws->shard.columns();
     if (ws->shard_N < 1) { workspace_destroy(ws); return nullptr; }   // fewer 64-column blocks than GPUs in the group
     const int local_N = ws->shard_N;      // what this GPU's kernels compute; schedules are chosen for it
-    // Schedule: the mma.sync kernel serves up to 32 tokens per CTA pass; larger batches
-    // go to the tcgen05 kernel when it can run this geometry.
-    GemmParams probe{};
-    probe.M = cfg->M; probe.N = local_N; probe.K = cfg->K; probe.KB = ws->KB;
     // an explicit schedule (a tuned strategy) wins over the environment override, which wins over the rules below
     const int forced = schedule.family ? schedule.family : std::getenv("RK_NPU_B200_VARIANT") ? std::atoi(std::getenv("RK_NPU_B200_VARIANT")) : 0;
-    const bool tc_ok = gemm_tc_supported(probe);
+    const bool tc_ok = (long long)ws->KB * KBLOCK <= 131072;
     const bool fused_ok = cfg->M <= 32 && ws->KB <= 8 * FUSED_MAX_STAGES;
-    const bool stream_ok = cfg->M <= 128 && (long long)ws->KB * KBLOCK <= 131072;
+    const bool stream_ok = cfg->M <= 128 && tc_ok;
     // Small batches: the single-kernel path wins while all of the weights fit in the SMs' shared
     // memory at once (one wave, up to about 24 MB) and the batch is a single 8-token MMA column
     // block; beyond that the two-kernel ring (quantise + mma.sync GEMM) streams better.  Up to 32
@@ -1058,16 +1046,15 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     // and partial sums (8 tokens: 1479 against 1669 GB/s), so the split-K kernel keeps those where it applies.
     const bool decode_ok = gemm_decode_supported(cfg->M, cfg->K);
     const bool decode_best = decode_ok && (cfg->M <= 4 || !fused_best);
-    // 33..128 tokens: the per-tile tcgen05 kernel has one CTA per 128 output channels; when that is less than
-    // half the SMs and K is long, the streaming kernel (all SMs, K split between CTAs) is faster.
-    const bool stream_best = stream_ok && cfg->M > 32 && cfg->K >= 8192 &&
-                             (local_N + TILE_N - 1) / TILE_N * 2 <= ctx->sm_count;
-    // 33..128 tokens with so few tiles that tiles x 32-token chunks fit the SMs in one wave (N = 4096: 32 x 4): the
-    // mma.sync ring, one CTA per (tile, chunk, K split), fills the GPU where the tcgen05 kernels leave SMs idle or
-    // pay for combining partial tiles (11008 -> 4096 at 128 tokens: 33 us against 44 and 47 us).
-    const bool ring_best = cfg->M > 32 && cfg->M <= 128 &&
-                           (long long)((local_N + TILE_N - 1) / TILE_N) * ((cfg->M + 31) / 32) <= ctx->sm_count;
-    int variant = decode_best ? 5 : ring_best ? 1 : (cfg->M > 32 && stream_best) ? 4 : (cfg->M > 32 && tc_ok) ? 2 : fused_best ? 3 : 1;
+    // 9..16 tokens: one launch (the split-K kernel) beats two (the ring) while the weights are small (16 tokens, 4096 ->
+    // 4096 9.6 against 10.0 us, 8192 -> 1024 8.5 against 10.6, 11008 -> 4096 17.2 against 14.1).
+    const bool fused_mid = fused_ok && cfg->M > 8 && cfg->M <= 16 && (long long)cfg->K * local_N / 2 <= (8ll << 20);
+    // From 17 tokens on the persistent tcgen05 kernel, whose time hardly depends on the batch up to 64 (4096 -> 4096 13 us,
+    // 11008 -> 4096 19, 4096 -> 14336 14.5), unless its 256-channel tiles are so few that the ring's small CTAs cover more
+    // of the GPU (24 tokens: 2048 -> 2048 9.3 us, the ring's 16.4 / 24 / 17.1 us on the three shapes above).
+    const int channel_tiles = (local_N + 255) / 256;
+    const bool pair_best = tc_ok && (cfg->M > 96 || (cfg->M > 32 && channel_tiles > 4) || (cfg->M > 16 && channel_tiles > 12));
+    int variant = decode_best ? 5 : pair_best ? 2 : (fused_best || fused_mid) ? 3 : 1;
     if (forced == 1 || (forced == 2 && tc_ok) || (forced == 3 && fused_ok) || (forced == 4 && stream_ok) || (forced == 5 && decode_ok))
         variant = forced;
     ws->variant = variant;
@@ -1076,14 +1063,10 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         ws->tiles_per_cta_override = (v == 1 || v == 2) ? v : 0;
     }
     if (variant == 2) {
-        // Two-CTA tiles (128-token code tiles, two per MMA tile) on the persistent kernel.  Also for 33..128 tokens,
-        // where half of every MMA multiplies zero tokens: its resident CTA pairs still beat one launch-and-leave CTA
-        // per tile (FFN 4096 -> 2 x 14336 -> 4096 at 128 tokens 129 -> 104 us, the 128 x 4096 x 28672 linear 49 -> 41 us).
         ws->TC = 0;
-        int pair_min = 33;
-        if (const char* e = std::getenv("RK_NPU_B200_PAIR_MIN")) pair_min = std::max(1, std::atoi(e));   // experiments
-        ws->pair = cfg->M >= pair_min && !env_flag("RK_NPU_B200_NO_PAIR", false);
-        ws->T = ws->pair ? gemm_tc_persist_tok(local_N, cfg->M, ws->KB, ctx->sm_count) / 2 : (cfg->M >= 256 ? 256 : align_up(cfg->M, 16));
+        const PersistPlan plan = gemm_tc_persist_plan(local_N, cfg->M, ws->KB, false, ctx->sm_count);
+        ws->T = plan.tok / 2;
+        ws->parts = plan.split;
     } else if (variant == 4) {
         ws->TC = ws->T = cfg->M <= 16 ? 16 : cfg->M <= 32 ? 32 : cfg->M <= 64 ? 64 : 128;   // tcgen05 N
     } else {
@@ -1098,7 +1081,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (schedule.cluster && (variant == 1 || variant == 5 || (variant == 3 && (ws->KB + schedule.cluster - 1) / schedule.cluster <= FUSED_MAX_STAGES)) &&
         (variant == 5 || ws->KB >= schedule.cluster))
         ws->split_override = schedule.cluster;
-    const size_t Mp = size_t(align_up(cfg->M, ws->pair ? 2 * ws->T : ws->T));
+    const size_t Mp = size_t(align_up(cfg->M, variant == 2 ? 2 * ws->T : ws->T));
     ws->codes_bytes = Mp * size_t(ws->KB) * KBLOCK;
     const int out_cols = cfg->N;
     ws->stage_in_bytes = size_t(cfg->M) * cfg->K * 4;
@@ -1114,17 +1097,13 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes);
     }
-    if (variant == 2 && ws->pair) {
-        // partial sums of tiles whose K is cut between CTA pairs, and their stage counters
-        ws->partials_bytes = gemm_tc_persist_slot_bytes(ctx->sm_count, 2 * ws->T);
-        ws->counts_bytes = gemm_tc_persist_count_bytes(local_N, cfg->M, 2 * ws->T);
+    if (variant == 2 && ws->parts > 1) {
+        // partial sums of tiles whose K is cut between CTA pairs, and how many parts of each are done
+        const PersistPlan plan{2 * ws->T, ws->parts};
+        ws->partials_bytes = gemm_tc_persist_slot_bytes(local_N, cfg->M, plan);
+        ws->counts_bytes = gemm_tc_persist_count_bytes(local_N, cfg->M, plan);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes);
-        if (ws->T == 128 && env_flag("RK_NPU_B200_PARK", true)) {
-            // accumulator chunks between being read out of tensor memory and being finished
-            ws->park_bytes = gemm_tc_persist_park_bytes(ctx->sm_count);
-            ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->park), ws->park_bytes);
-        }
     }
     if (ctx->world > 1) {
         ws->gather_slot = size_t(cfg->M) * size_t(shard_plan(cfg->N, ctx->world, 0).columns()) * 4;   // rank 0's share is the widest

@@ -105,16 +105,14 @@ struct GemmParams {
     int F;                  // SwiGLU: N/2, else 0
     int epi;
     int split;              // split-K factor == cluster size along y (1, 2, 4, 8)
-    int pair;               // tcgen05 path: 1 = two-CTA tiles (cta_group::2), T must be 128
-    int w8;                 // tcgen05 per-tile kernel: Wp holds int8 codes in the W8 layout (w8a8_kernels.cu), sums are not scaled by 16
+    int w8;                 // persistent kernel: Wp holds int8 codes in the W8 layout (w8a8_kernels.cu), sums are not scaled by 16
     unsigned long long timeout_ns;
     unsigned long long* trace;  // optional cycle stamps of CTA (0,0): [role 0..2][k-block 0..63][2] (nullable)
-    // streaming and persistent kernels: [2 x CTAs][tokens of the tile / 4][128][4] int32 partial sums (two slots per CTA,
-    // never cleared) and [tiles] ([tiles][2 CTAs] in the persistent kernel) stages accumulated so far, zero between launches
+    // streaming kernel: [2 x CTAs][T / 4][128][4] int32 partial sums (two slots per CTA, never cleared) and [tiles] stages
+    // accumulated so far, zero between launches; persistent kernel with split > 1: [tiles][split][2 CTAs][tokens of the
+    // tile / 4][128][4] and [tiles][2 CTAs] parts done
     int* partials;
     unsigned int* counts;
-    int* park;                  // persistent kernel, SwiGLU: where accumulator chunks wait to be finished (nullable)
-    int max_clusters;           // persistent kernel: CTA pairs the slots are sized for
 };
 
 // Single-kernel linear for small batches: quantisation fused in front of the GEMM.
@@ -215,7 +213,7 @@ struct W8QuantParams {
 cudaError_t launch_w8_pack_weights(const W8PackParams& p, cudaStream_t stream);
 cudaError_t launch_w8_quantize(const W8QuantParams& p, cudaStream_t stream);
 
-// Launch wrappers (w4a8_kernels.cu / w4a8_gemm_tc.cu). All return the launch error.
+// Launch wrappers (w4a8_kernels.cu and the files named below). All return the launch error.
 cudaError_t launch_pack_weights(const PackParams& p, cudaStream_t stream);
 cudaError_t launch_quantize(const QuantParams& p, cudaStream_t stream, bool pdl);
 cudaError_t launch_quantize_slice(const SliceQuantParams& p, cudaStream_t stream);
@@ -240,22 +238,19 @@ int gemm_decode_ctas(int items, int cluster, int cap);
 int gemm_decode_resident_ctas(int cluster, size_t smem, int sm_count);
 cudaError_t launch_gemm_decode(const DecodeParams& p, cudaStream_t stream, bool pdl);
 cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, bool pdl);
-// tcgen05 path: p.T is the token tile of the code layout (multiple of 16, <= 256; 128 when p.pair)
-cudaError_t launch_gemm_tc(const GemmParams& p, cudaStream_t stream, bool pdl);
-bool gemm_tc_supported(const GemmParams& p);
-// persistent two-CTA form: p.pair, p.T (tokens of one CTA's activation tile: 32, 64 or 128), p.partials, p.counts and
-// p.max_clusters required
+// persistent two-CTA tcgen05 kernel (K <= 131072): p.T (tokens of one CTA's activation tile: 32, 64 or 128) and p.split
+// required, p.partials and p.counts where split > 1
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
 bool gemm_tc_persist_supported(const GemmParams& p);
-// Tokens of the MMA tile (64, 128 or 256) for a problem, and the CTA pairs of a launch (columns: all accumulator rows,
-// i.e. gate and up together for SwiGLU; tok = 2 T)
-int gemm_tc_persist_tok(int columns, int M, int KB, int sm_count);
-int gemm_tc_persist_clusters(int columns, int M, int KB, int tok, int max_clusters);
-// Bytes of GemmParams.partials and .counts (the latter zero before the first launch)
-size_t gemm_tc_persist_slot_bytes(int sm_count, int tok);
-size_t gemm_tc_persist_count_bytes(int columns, int M, int tok);
-// Bytes of GemmParams.park (NULL: chunks are finished one by one before the accumulator is handed back).  No initial
-// contents needed.
-size_t gemm_tc_persist_park_bytes(int sm_count);
+// How the persistent kernel cuts a problem (columns: all accumulator rows, i.e. gate and up together for SwiGLU)
+struct PersistPlan {
+    int tok;      // tokens of the MMA tile (64, 128 or 256): p.T = tok / 2, the code buffer holds whole multiples of tok
+    int split;    // parts a tile's K is cut into (p.split)
+};
+PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, int sm_count);
+int gemm_tc_persist_tiles(int columns, int M, int tok);
+// Bytes of GemmParams.partials and .counts (the latter zero before the first launch); 0 where nothing is split
+size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan);
+size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan);
 
 } // namespace rkb200

@@ -1,23 +1,18 @@
-// w4a8_gemm_tc_persist.cu -- persistent two-CTA tcgen05 W4A8 GEMM for large batches (sm_100a).
+// w4a8_gemm_tc_persist.cu -- persistent two-CTA tcgen05 W4A8 GEMM from 17 tokens on (sm_100a).
 //
-// Same data path as w4a8_gemm_tc.cu (packed int4 weights -> tensor memory as the A operand,
-// int8 activation codes as shared-memory B operand, kind::i8 MMA over a CTA pair with
-// cta_group::2, int32 accumulators in tensor memory), organised so that nothing but the
+// Packed int4 weights -> tensor memory as the A operand, int8 activation codes as shared-memory B operand, kind::i8
+// MMA over a CTA pair with cta_group::2, int32 accumulators in tensor memory, organised so that nothing but the
 // tensor pipe sits on the critical path:
-//   * one cluster of two CTAs per SM pair stays resident and walks a list of 256-channel x
-//     256-token tiles; barriers, tensor memory and descriptors are set up once;
+//   * one cluster of two CTAs per SM pair stays resident and walks a run of 256-channel x (64, 128 or 256)-token
+//     tiles; barriers, tensor memory and descriptors are set up once.  Where the tiles are few, K is cut into parts;
 //   * weights and activations travel through SEPARATE rings of bulk copies.  A weight slot is
 //     free again as soon as the unpack warps have read it (the unpacked copy lives in tensor
-//     memory), an activation slot when the MMAs that read it retire.  Together the rings hold
-//     ten k-blocks of activations and eight of weights per CTA -- all of shared memory -- because
-//     the copies (L2 hits) take several MMA-stage times to arrive and the pipe starves on a
+//     memory), an activation slot when the MMAs that read it retire.  Together the rings take all of shared memory,
+//     because the copies (L2 hits) take several MMA-stage times to arrive and the pipe starves on a
 //     shallower ring;
 //   * eight dedicated epilogue warps read the accumulator out of tensor memory, hand it back
 //     after the last read and store straight from registers: the 32 lanes of a warp hold 32
-//     neighbouring channels of one token, i.e. 64..128 contiguous bytes per store.  For the
-//     SwiGLU epilogue, where finishing a chunk costs far more than reading it, three of the four
-//     chunks are parked in an L2-resident scratch so that the tensor pipe gets the accumulator
-//     back after four reads;
+//     neighbouring channels of one token, i.e. 64..128 contiguous bytes per store;
 //   * for SwiGLU the unpack warps place gate channels in lanes 0-15 and the matching up
 //     channels in lanes 16-31 of every tensor-memory lane quarter, so the epilogue pairs them
 //     with one warp shuffle.
@@ -28,7 +23,6 @@
 #include "w4a8_ptx.cuh"
 #include "w4a8_tc.cuh"
 #include <algorithm>
-#include <cstdlib>
 
 namespace rkb200 {
 
@@ -39,7 +33,7 @@ constexpr int PS_UNPACK_WARP0 = PS_ROLE_WARPS;
 constexpr int PS_EPI_WARP0 = PS_UNPACK_WARP0 + PS_UNPACK_WARPS;
 constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 640
 constexpr int PS_TMEM_COLS = 512;
-constexpr int PS_PARK_INTS = 3 * 32 * 32 * PS_EPI_WARPS;   // per CTA: three parked chunks of 32 sums per epilogue thread (96 KB)
+
 
 // One instantiation's resources.  TOK = tokens of the MMA tile (accumulator columns), half of them in each CTA.
 // Stages are 2 k-blocks.  Tensor memory holds the accumulator (two of them where they fit, so that the epilogue of a
@@ -124,12 +118,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     const int tiles_n = swiglu ? (p.F + 63) / 64 : (p.N + TILE_N - 1) / TILE_N;
     const int pairs_n = (tiles_n + 1) / 2;
     const int pairs_m = (p.M + TOK - 1) / TOK;
-    // The work is the flat list of (tile, stage) items; every cluster takes one contiguous share of it.  The launcher
-    // picks a cluster count that divides the tile count where cutting tiles along K would not pay.
-    const long long total = (long long)pairs_n * pairs_m * nst;
-    const long long b0 = total * cluster_id / num_clusters, b1 = total * (cluster_id + 1) / num_clusters;
-    const int n_items = (int)(b1 - b0);
-    const int tile0 = (int)(b0 / nst), it0 = (int)(b0 - (long long)tile0 * nst);
+    // Every cluster takes a run of whole tiles, or (split > 1) one of the `split` parts of one tile's stages.
+    const int tiles = pairs_n * pairs_m, split = p.split;
+    const int part = cluster_id % split;
+    const int tile0 = split > 1 ? cluster_id / split : (int)((long long)tiles * cluster_id / num_clusters);
+    const int it0 = nst * part / split;
+    const int n_items = split > 1 ? nst * (part + 1) / split - it0 : ((int)((long long)tiles * (cluster_id + 1) / num_clusters) - tile0) * nst;
     const unsigned long long deadline = global_ns() + p.timeout_ns;
     // optional cycle stamps of cluster 0's leader: [segment j < 16][8] = MMA wait-begin, MMA first issue,
     // MMA last commit, epilogue acc_full seen, tensor memory handed back, stored, [6] cycles the MMA
@@ -413,7 +407,6 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         int tile = tile0, it = it0;
         for (int gi = 0, j = 0; gi < n_items && ok; ++j, rc.next()) {
             const int n_seg = min(nst - it, n_items - gi);
-            const bool whole = n_seg == nst;                 // this segment covers its tile's whole K
             const int ct = 2 * (tile % pairs_n) + (int)rank;
             const int tok_base = (tile / pairs_n) * TOK;
             const int col0 = swiglu ? ct * 64 : ct * TILE_N;
@@ -439,13 +432,14 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                 if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(&acc_empty[rc.slot], 0); else mbar_arrive_relaxed(&acc_empty[rc.slot]); }
                 if (sid == 0) PS_STAMP(j, 4);
             };
-            // ---- a part of a tile's K: the raw sums go to this CTA's slot, the tile's stage counter is advanced, and the
-            // CTA that completes it adds the contributors' slots (integer addition: exact in any order) and finishes the
-            // tile.  Nobody waits for anybody, and no slot needs clearing.  A cluster's run begins and ends with at most
-            // one partial segment each, so two slots per CTA suffice.
-            int part_lo = 0, part_hi = -1;                   // contributing clusters when the sums come from slots
-            if (!whole) {
-                int4* const slot = reinterpret_cast<int4*>(p.partials) + ((size_t)(2 * cluster_id + (gi == 0 ? 0 : 1)) * 2 + rank) * (S::SLOT_INTS / 4) + (size_t)(8 * eset) * 128 + row;   // [token / 4][row][4 tokens]
+            // ---- a part of a tile's K: the raw sums go to this CTA's slot, the tile's part counter is advanced, and the CTA
+            // that completes it adds the other parts' slots to its own sums, which are still in tensor memory (integer
+            // addition: exact in any order), and finishes the tile.  Nobody waits for anybody, and no slot needs clearing.
+            const size_t part_stride = 2 * (S::SLOT_INTS / 4);            // from one part's slot to the next one's
+            const int4* const slots = reinterpret_cast<const int4*>(p.partials) + (size_t)(2 * split * tile + (int)rank) * (S::SLOT_INTS / 4) + (size_t)(8 * eset) * 128 + row;   // [token / 4][row][4 tokens]
+            bool finish = true;
+            if (split > 1) {
+                int4* const slot = const_cast<int4*>(slots) + part * part_stride;
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t r[32];
@@ -453,62 +447,56 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                     tc_wait_ld();
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        slot[(size_t)(16 * c + i) * 128] = make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]);
+                        __stcg(slot + (size_t)(16 * c + i) * 128, make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]));
                 }
-                hand_back();
                 __threadfence();
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 if (sid == 0) {
-                    // (a tile with a segment whose wait ran out is never completed; the launch reports the error and the host
+                    // (a tile with a part whose wait ran out is never completed; the launch reports the error and the host
                     // clears the counters)
                     unsigned* const count = p.counts + 2 * tile + (int)rank;
-                    const bool done = atomicAdd(count, (unsigned)n_seg) + (unsigned)n_seg == (unsigned)nst;
+                    const bool done = atomicAdd(count, 1u) == (unsigned)split - 1u;
                     if (done) *count = 0u;
                     *s_finish = done ? 1 : 0;
                     __threadfence();
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (*reinterpret_cast<volatile int*>(s_finish)) {
-                    const long long s0 = (long long)tile * nst;
-                    part_lo = (int)(((s0 + 1) * num_clusters - 1) / total);
-                    part_hi = (int)(((s0 + nst) * num_clusters - 1) / total);
-                }
+                finish = *reinterpret_cast<volatile int*>(s_finish) != 0;
             }
-            if (whole && chunks == 0) hand_back();
-            const int turns = whole || part_hi >= part_lo ? 2 * chunks : 0;
+            const int turns = finish ? 2 * chunks : 0;
+            const int other = part == 0 ? 1 : 0;                          // the first of the other parts
+            int4 ahead[4];                                                // its sums of the next turn, on their way
+            auto fetch_part = [&](int4 (&v)[4], int which, int k) {
+                const int4* const src = slots + which * part_stride + (size_t)(16 * (k >> 1) + 4 * (k & 1)) * 128;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) v[h] = __ldcg(src + (size_t)h * 128);
+            };
+            if (split > 1 && turns) fetch_part(ahead, other, 0);
+            if (split == 1 && chunks == 0) hand_back();
 #pragma unroll 1
             for (int k = 0; k < turns; ++k) {
                 const int t0 = 32 * eset + 64 * (k >> 1) + 16 * (k & 1), m0 = tok_base + t0;
                 uint32_t r[16];
-                if (whole) {
-                    tc_ld16(lane_addr + rc.slot * TOK + t0, r);
-                    tc_wait_ld();
+                tc_ld16(lane_addr + rc.slot * TOK + t0, r);
+                tc_wait_ld();
+                if (split == 1) {
                     if (k + 1 == turns) hand_back();
                 } else {
+                    auto add = [&](const int4 (&v)[4]) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) r[i] = 0u;
+                        for (int h = 0; h < 4; ++h) {
+                            r[4 * h] += (uint32_t)v[h].x; r[4 * h + 1] += (uint32_t)v[h].y; r[4 * h + 2] += (uint32_t)v[h].z; r[4 * h + 3] += (uint32_t)v[h].w;
+                        }
+                    };
+                    add(ahead);
 #pragma unroll 1
-                    for (int cc = part_lo; cc <= part_hi; cc += 2) {       // two contributors' loads in flight at a time
-                        int4 v[2][4];
-#pragma unroll
-                        for (int c = 0; c < 2; ++c)
-                            if (cc + c <= part_hi) {
-                                // a cluster whose run starts inside the tile contributed its first segment, another one its last
-                                const int which = total * (cc + c) / num_clusters >= (long long)tile * nst ? 0 : 1;
-                                const int4* const src = reinterpret_cast<const int4*>(p.partials) + ((size_t)(2 * (cc + c) + which) * 2 + rank) * (S::SLOT_INTS / 4) + (size_t)(t0 / 4) * 128 + row;
-#pragma unroll
-                                for (int h = 0; h < 4; ++h) v[c][h] = __ldcg(src + (size_t)h * 128);
-                            } else {
-#pragma unroll
-                                for (int h = 0; h < 4; ++h) v[c][h] = make_int4(0, 0, 0, 0);
-                            }
-#pragma unroll
-                        for (int c = 0; c < 2; ++c)
-#pragma unroll
-                            for (int h = 0; h < 4; ++h) {
-                                r[4 * h] += (uint32_t)v[c][h].x; r[4 * h + 1] += (uint32_t)v[c][h].y; r[4 * h + 2] += (uint32_t)v[c][h].z; r[4 * h + 3] += (uint32_t)v[c][h].w;
-                            }
-                    }
+                    for (int which = other + 1; which < split; ++which)
+                        if (which != part) {
+                            int4 v[4];
+                            fetch_part(v, which, k);
+                            add(v);
+                        }
+                    if (k + 1 < turns) fetch_part(ahead, other, k + 1);
                 }
                 if (m0 >= p.M) continue;
                 if (p.epi == EPI_I32) {
@@ -692,8 +680,9 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
         max_clusters = n;
         if (device >= 0 && device < 64) { clusters_of_device[device] = n; configured.mark(device); }
     }
-    if (max_clusters > p.max_clusters) max_clusters = p.max_clusters;      // what the slots in p.partials were sized for
-    const int clusters = gemm_tc_persist_clusters(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, p.KB, TOK, max_clusters);
+    const int tiles = gemm_tc_persist_tiles(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, TOK);
+    if (p.split > 1 && tiles * p.split > max_clusters) return cudaErrorInvalidValue;
+    const int clusters = p.split > 1 ? tiles * p.split : std::min(tiles, max_clusters);
     cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
     int n = 1;
     if (pdl) {
@@ -709,30 +698,52 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
 
 bool gemm_tc_persist_supported(const GemmParams& p)
 {
-    return p.pair && (p.T == 128 || p.T == 64 || p.T == 32) && (long long)p.KB * KBLOCK <= PS_MAX_K && p.partials && p.counts;
+    return (p.T == 128 || p.T == 64 || p.T == 32) && (long long)p.KB * KBLOCK <= PS_MAX_K && p.split >= 1 && (p.split == 1 || (p.partials && p.counts));
 }
 
-// CTA pairs of a launch: all resident ones, but no more than `split_cap` per tile.
-int gemm_tc_persist_clusters(int columns, int M, int KB, int tok, int max_clusters)
+int gemm_tc_persist_tiles(int columns, int M, int tok) { return (columns + 255) / 256 * ((M + tok - 1) / tok); }
+
+// The token tile and the number of parts a tile's K is cut into: the cheapest by a model of the kernel's time in cycles,
+// from what it measured on 60 shapes (M 33..4096, K 2048..14336, N 1024..28672, both epilogues; within 1 % of the best
+// choice on average, 15 % at worst):
+//   * a k-block takes 270 to 390 cycles at 64 tokens and 310 to 370 at 128, more with more SMs busy (the operands come
+//     out of L2 at about 45 bytes per SM and cycle when all SMs ask), and 530 at 256, where the MMAs bound it; int8
+//     weights are delivery-bound at every width;
+//   * finishing a tile takes 33 cycles per token, 1500 at least (90 with SwiGLU, which changes no choice); two accumulators hide it behind the next
+//     tile's MMAs up to 128 tokens, at 256 there is room for one and nothing is hidden;
+//   * K in parts costs an exchange through L2: so much per part and pair, more for wide token tiles;
+//   * a launch on more than half of the SMs leaves the one behind it no room to set itself up meanwhile.
+PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, int sm_count)
 {
-    const long long tiles = (long long)((columns + 255) / 256) * ((M + tok - 1) / tok);
-    const long long stages = tiles * ((KB + 1) / 2);
-    static const int cap = std::getenv("RK_PS_CAP") ? std::atoi(std::getenv("RK_PS_CAP")) : 1;
-    long long n = std::min<long long>(max_clusters, tiles * cap);
-    n = std::min(n, std::max<long long>(stages / 2, 1));
-    return (int)n;
+    PersistPlan best{256, 1};
+    double best_time = 0;
+    const int pairs = std::max(1, sm_count / 2);
+    for (const int tok : {64, 128, 256}) {
+        if (tok > 64 && M <= 64) break;                        // half of the tile would be padding
+        const long long tiles = (long long)((columns + 255) / 256) * ((M + tok - 1) / tok);
+        for (const int split : {1, 2, 3, 4, 6, 8}) {
+            if (split > 1 && (tok == 256 || tiles * split > pairs || KB < 4 * split)) break;
+            const long long clusters = std::min<long long>(tiles * split, pairs), rounds = (tiles + pairs - 1) / pairs;
+            const double busy = double(clusters) / pairs;
+            double block = tok == 64 ? 270 + 120 * busy : tok == 128 ? 310 + 60 * busy : 530;
+            if (w8) block = std::max(block, (16384 + 64 * tok) / 45.0);
+            const double mma = KB * block / split, live = std::min(tok, M), finish = 1500 + 33 * live;
+            double time = tok == 256 ? rounds * (mma + finish) : rounds * std::max(mma, finish) + finish;
+            if (split > 1) time += (1500 + 1000 * (split - 1) + 30 * clusters) * (1 + 1.5 * std::max(0.0, live - 64) / 64);
+            if (2 * clusters > pairs) time += 3000;
+            if (best_time == 0 || time < best_time) { best_time = time; best = {tok, split}; }
+        }
+    }
+    return best;
 }
-
-int gemm_tc_persist_tok(int columns, int M, int KB, int sm_count)
+size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan)
 {
-    static const int forced = std::getenv("RK_PS_TOK") ? std::atoi(std::getenv("RK_PS_TOK")) : 0;
-    if (forced) return forced;
-    return M <= 64 ? 64 : M <= 128 ? 128 : 256;
+    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_tiles(columns, M, plan.tok)) * size_t(plan.split) * 128 * size_t(plan.tok) * sizeof(int) : 0;
 }
-
-size_t gemm_tc_persist_park_bytes(int sm_count) { return size_t(sm_count) * PS_PARK_INTS * sizeof(int); }
-size_t gemm_tc_persist_slot_bytes(int sm_count, int tok) { return 2 * size_t(sm_count) * 128 * size_t(tok) * sizeof(int); }
-size_t gemm_tc_persist_count_bytes(int columns, int M, int tok) { return 2 * size_t((columns + 255) / 256) * size_t((M + tok - 1) / tok) * sizeof(unsigned); }
+size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan)
+{
+    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_tiles(columns, M, plan.tok)) * sizeof(unsigned) : 0;
+}
 
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl)
 {

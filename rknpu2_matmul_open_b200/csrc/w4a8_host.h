@@ -106,7 +106,6 @@ struct rk_npu_w4a8_workspace {
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
     cudaStream_t stream = nullptr;
     // geometry
-    bool pair = false; // tcgen05 path runs two-CTA tiles
     int T = 0;        // token tile of the code layout
     int TC = 0;       // tokens per CTA of the mma.sync kernel (0 when the tcgen05 kernel is used)
     int KB = 0;       // k-blocks
@@ -121,10 +120,10 @@ struct rk_npu_w4a8_workspace {
     float* scales = nullptr;
     float* inverse = nullptr;
     uint32_t* rowmax = nullptr;
-    int* partials = nullptr;          // variant 4: per-tile partial sums and k-block counters
+    int parts = 1;                    // variant 2: parts a tile's K is cut into
+    int* partials = nullptr;          // variants 2, 4: partial sums of tiles and progress counters
     unsigned int* counts = nullptr;
-    int* park = nullptr;              // variant 2: accumulator chunks of the SwiGLU epilogue
-    size_t partials_bytes = 0, counts_bytes = 0, park_bytes = 0;
+    size_t partials_bytes = 0, counts_bytes = 0;
     rkb200::Status* status = nullptr;
     void* stage_in = nullptr;   // device copy of host activations
     void* stage_out = nullptr;  // device copy of host outputs

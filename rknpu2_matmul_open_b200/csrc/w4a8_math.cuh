@@ -111,14 +111,33 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 d; asm("fma.rn.f32x2
 __device__ __forceinline__ F2 f2_all(float v) { return f2_pack(v, v); }
 
 // Degree-7 polynomial SiLU of the reference's production target, every rounding kept:
-// src/rk_npu_swiglu_fp32_neon.h:17-41.  Two arguments at a time.
+// src/rk_npu_swiglu_fp32_neon.h:17-41.  (The small-batch kernels evaluate it once per thread: the shortest code is best.)
+__device__ __forceinline__ float silu_poly(float g)
+{
+    float x = fminf(fmaxf(-g, -80.f), 80.f);
+    const float n = floorf(fmaf(x, 1.4426950408889634f, 0.5f));
+    float r = fmaf(-n, 0.693145751953125f, x);
+    r = fmaf(-n, 1.428606765330187e-6f, r);
+    float q = 1.f / 5040.f;
+    q = fmaf(q, r, 1.f / 720.f);
+    q = fmaf(q, r, 1.f / 120.f);
+    q = fmaf(q, r, 1.f / 24.f);
+    q = fmaf(q, r, 1.f / 6.f);
+    q = fmaf(q, r, 0.5f);
+    q = fmaf(q, r, 1.f);
+    q = fmaf(q, r, 1.f);
+    const float power = __int_as_float(((int)n + 127) << 23);
+    const float d = __fadd_rn(1.f, __fmul_rn(q, power));
+    return g < -80.f ? -0.f : __fdiv_rn(g, d);
+}
+// The same function, two arguments at a time, for the kernels that evaluate it over and over.
 //   * floor(y) for |y| < 2^22: adding 1.5 * 2^23 with rounding towards minus infinity leaves floor(y) in the low bits,
 //     from where the subtraction brings it back as a float and a shift puts it into the exponent of 2^n.
 //   * g / d, correctly rounded: a reciprocal within an ulp refined by one Newton step, a quotient from it, its remainder
 //     by fused multiply-add (exact) and one correction (P. Markstein, "Computation of elementary functions on the IBM
 //     RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  Magnitudes for which a step could leave the normal range
 //     take the division instruction sequence.
-// Equal bit for bit to the scalar statement of the reference's routine for every one of the 2^32 arguments (checked).
+// Equal bit for bit to silu_poly for every one of the 2^32 arguments (checked).
 __device__ __forceinline__ void silu_poly2(float g0, float g1, float& y0, float& y1)
 {
     const F2 g = f2_pack(g0, g1);
@@ -150,12 +169,6 @@ __device__ __forceinline__ void silu_poly2(float g0, float g1, float& y0, float&
     const bool plain0 = fabsf(g0) >= 9.094947017729282e-13f && fabsf(g0) <= 80.f, plain1 = fabsf(g1) >= 9.094947017729282e-13f && fabsf(g1) <= 80.f;
     if (!plain0) y0 = g0 < -80.f ? -0.f : __fdiv_rn(g0, d0);
     if (!plain1) y1 = g1 < -80.f ? -0.f : __fdiv_rn(g1, d1);
-}
-__device__ __forceinline__ float silu_poly(float g)
-{
-    float y, unused;
-    silu_poly2(g, g, y, unused);
-    return y;
 }
 __device__ __forceinline__ float dequant(int acc, float sx, float sw)
 {

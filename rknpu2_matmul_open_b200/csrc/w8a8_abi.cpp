@@ -45,7 +45,7 @@ struct rk_npu_matmul_workspace {
     uint32_t domain_id = 0;
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
     cudaStream_t stream = nullptr;
-    int T = 0, KB = 0;
+    int T = 0, KB = 0, parts = 1;
     uint8_t* codes = nullptr;
     int* partials = nullptr;          // partial sums of tiles whose K is cut between CTA pairs
     unsigned* counts = nullptr;       // and how far each such tile is
@@ -93,19 +93,20 @@ bool valid_strategy(const rk_npu_matmul_strategy* s)
 // what the kernels need on top: K within the contraction kernel's range, sizes that fit
 bool runnable_shape(int M, int N, int K) { return K <= 131072 && (int64_t)M * K <= INT32_MAX && (int64_t)M * N <= INT32_MAX; }
 struct Sizes {
-    int T, KB, NG;
+    int T, KB, NG, parts;
     size_t codes, partials, counts, scales, stage_in, stage_out, packed, wscales;
 };
 Sizes sizes_of(int M, int N, int K, int kind, int sm_count)
 {
     Sizes z{};
     z.KB = (K + KBLOCK - 1) / KBLOCK;
-    const int tok = gemm_tc_persist_tok(N, M, z.KB, sm_count);   // the code buffer covers whole pairs of token tiles
-    z.T = tok / 2;
+    const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, sm_count);
+    z.T = plan.tok / 2;
+    z.parts = plan.split;
     z.NG = align_up((N + GROUP - 1) / GROUP, 8) + 8;   // zero groups behind the last tile, as for the int4 weights
-    z.codes = size_t(align_up(M, tok)) * size_t(z.KB) * KBLOCK;
-    z.partials = gemm_tc_persist_slot_bytes(sm_count, tok);
-    z.counts = gemm_tc_persist_count_bytes(N, M, tok);
+    z.codes = size_t(align_up(M, plan.tok)) * size_t(z.KB) * KBLOCK;
+    z.partials = gemm_tc_persist_slot_bytes(N, M, plan);
+    z.counts = gemm_tc_persist_count_bytes(N, M, plan);
     z.scales = sizeof(float) * 2 * size_t(M);
     const int in_elem = kind == RK_NPU_MATMUL_I8I8I32 ? 1 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? 2 : 4);
     const int out_elem = kind == RK_NPU_MATMUL_I8I8I32 ? 4 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? 2 : 4);
@@ -268,12 +269,10 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     g.M = st.M; g.N = st.N; g.K = st.K;
     g.KB = ws->KB; g.NG = w->NG; g.T = ws->T;
     g.epi = kind == RK_NPU_MATMUL_I8I8I32 ? EPI_I32 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? EPI_F16 : EPI_F32);
-    g.split = 1;
+    g.split = ws->parts;
     g.w8 = 1;
-    g.pair = 1;
     g.partials = ws->partials;
     g.counts = ws->counts;
-    g.max_clusters = ws->domain->ctx->sm_count / 2;
     g.timeout_ns = (unsigned long long)W8_TIMEOUT_MS * 1000000ull;
     if (launch_w8_quantize(q, s) != cudaSuccess || launch_gemm_tc_persist(g, s, false) != cudaSuccess) {
         cudaGetLastError();
@@ -286,7 +285,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
     if (ws->host_status->device_error) {       // a bounded wait inside the kernel ran out: report, clear, stay usable
         cudaMemsetAsync(&ws->status->device_error, 0, sizeof(int), s);
-        cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
+        if (ws->counts) cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
     }
@@ -351,6 +350,7 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     ws->ctx_id = ctx->id;
     ws->domain_id = domain->id;
     ws->T = z.T;
+    ws->parts = z.parts;
     ws->KB = z.KB;
     ws->codes_bytes = z.codes;
     ws->partials_bytes = z.partials;
@@ -362,14 +362,14 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     bool ok = cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMallocHost(reinterpret_cast<void**>(&ws->host_status), sizeof(Status)) == cudaSuccess;
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes) &&
-         !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
-         !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes) &&
+         (!ws->partials_bytes || (!device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
+                                  !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes))) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), ws->scale_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status)) &&
          !device_alloc(domain, &ws->stage_in, ws->stage_in_bytes) && !device_alloc(domain, &ws->stage_out, ws->stage_out_bytes);
     // codes of the tokens that pad the last tile stay zero for the life of the workspace
     ok = ok && cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
-         cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess &&
+         (!ws->counts || cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess) &&
          cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess && cudaStreamSynchronize(ws->stream) == cudaSuccess;
     if (!ok) { cudaGetLastError(); workspace_destroy(ws); return nullptr; }
     return ws;

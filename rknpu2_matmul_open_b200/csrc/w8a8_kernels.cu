@@ -7,7 +7,7 @@
 //   codes           : :126-131: q = clamp(round_half_away(x * (1 / s)), -127, 127), NaN -> 127; a row whose scale is
 //                     not positive quantises to zeros (:598-606)
 //   int8 A as given : include/rk_npu_quant_matmul.h:335-340 (no quantisation at all)
-// The contraction itself runs on the tcgen05 kernel of w4a8_gemm_tc.cu with int8 weights (GemmParams::w8).
+// The contraction itself runs on the tcgen05 kernel of w4a8_gemm_tc_persist.cu with int8 weights (GemmParams::w8).
 //
 // Weight layout  W8p[g][kb][c][r][16 B]: g = group of 32 output channels, kb = 128-element k-block, c = 16-element
 // chunk of the k-block (8 of them), r = channel of the group; the 16 bytes are the int8 codes k = 128kb + 16c .. +15.
