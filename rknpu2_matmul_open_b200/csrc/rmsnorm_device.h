@@ -14,6 +14,7 @@ struct AddRmsNormParams {
     int M, D;
     float eps;
     int row_major;           // 0: block-8 (D/8, M, 8); 1: [M, D]
+    int over_bus;            // the tensors are host memory the GPU reads and writes over the bus
     int tile_tokens;         // set by the launcher
 };
 

@@ -8,7 +8,8 @@
 // would be the busiest pipe of this kernel, so the second pass proves per value that single precision
 // gives the same fp16 bits and falls back to the defining expression where it cannot (scale_one).
 //
-// HBM-bound: 4 tensors of 2 M D bytes cross DRAM once each.  A tile of TM tokens is shared by a CLUSTER of CS CTAs,
+// HBM-bound: 4 tensors of 2 M D bytes cross DRAM once each.  Two forms.  Rows that fit a CTA's registers take
+// add_rmsnorm_row_kernel; longer block-8 rows take add_rmsnorm_kernel, where a tile of TM tokens is shared by a CLUSTER of CS CTAs,
 // each taking a slice of D: the sums stay in that CTA's shared memory between the two passes (both outputs are stored
 // in the second one, so that no global store is in flight at the cluster barrier), the per-token sums of squares are exchanged through distributed shared memory and added in rank
 // order by every CTA, so that the result does not depend on the schedule.  Both tensor layouts move 16-byte chunks
@@ -16,6 +17,8 @@
 // [M, D] consecutive CHUNKS of one token are; the thread index is split accordingly so that a warp touches 512
 // contiguous bytes either way.
 #include "rmsnorm_device.h"
+#include "w4a8_math.cuh"
+#include "w4a8_ptx.cuh"
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <atomic>
@@ -58,31 +61,31 @@ __device__ __forceinline__ uint32_t add_pair(uint32_t a, uint32_t b, double& acc
 }
 // One output: fp16(float(double(v) * inv * double(g))), the defining expression, evaluated in double only when needed.
 // y = fl32(fl32(v * inv_f) * g) with inv_f = fl32(inv) differs from the exact product x by at most 3 * 2^-24 |x|, and
-// the float the defining expression rounds to fp16 by at most (2^-24 + 2^-52) |x|: the two are less than 4.000001
-// float ulps apart.  fp16 rounding of a float in the normal fp16 range is decided by its low 13 mantissa bits L
-// against the midpoint 0x1000; when |L - 0x1000| >= 8 no midpoint lies between the two floats (or on one of them), so
-// fp16(y) IS the defined result.  About 0.2 % of the values, everything outside the normal fp16 range, and rows whose
-// inv is not a normal float are not proven and are evaluated in double.
+// the float the defining expression rounds to fp16 by at most (2^-24 + 2^-52) |x|: that float lies between
+// y (1 - 2^-21) and y (1 + 2^-21) (for the magnitudes |v| < 2^16, 2^-16 < inv, |g| < 2^16 nothing leaves the normal float
+// range).  Rounding is monotone, so when both ends -- taken at 2^-20, which covers their own rounding -- round to the same
+// fp16, that IS the defined result.  About 0.4 % of the values, and rows whose inv is not a normal float, are evaluated
+// in double.
 
-// The defining expression.  A real call, so that this rare path is branched around instead of being evaluated for
-// every value (checking per value and not per chunk keeps the double-precision conversions, the slowest instructions
-// here, to the values that need them).
-__device__ __noinline__ float scale_defined(float v, float g, double inv) { return __double2float_rn(double(v) * inv * double(g)); }
-__device__ __forceinline__ float scale_one(float v, float g, double inv, float inv_f, bool fast)
+// The defining expression, for a pair.  A real call, so that this rare path is branched around instead of being
+// evaluated for every value.
+__device__ __noinline__ uint32_t scale_defined(float2 v, float2 g, double inv)
 {
-    float y = __fmul_rn(__fmul_rn(v, inv_f), g);
-    const uint32_t u = __float_as_uint(y);
-    const bool proven = fast && fabsf(y) >= 6.103515625e-05f && fabsf(y) < 65536.f      // 2^-14 <= |y| < 2^16 (false for NaN)
-                        && ((u - (0x1000u - 7u)) & 0x1fffu) > 14u;                      // |L - 0x1000| >= 8
-    if (!proven) y = scale_defined(v, g, inv);
-    return y;
+    const __half2 o = __floats2half2_rn(__double2float_rn(double(v.x) * inv * double(g.x)), __double2float_rn(double(v.y) * inv * double(g.y)));
+    return *reinterpret_cast<const uint32_t*>(&o);
 }
 __device__ __forceinline__ uint32_t scale_pair(uint32_t v, uint32_t g, double inv, float inv_f, bool fast)
 {
     const float2 fv = __half22float2(*reinterpret_cast<const __half2*>(&v));
     const float2 fg = __half22float2(*reinterpret_cast<const __half2*>(&g));
-    const __half2 o = __floats2half2_rn(scale_one(fv.x, fg.x, inv, inv_f, fast), scale_one(fv.y, fg.y, inv, inv_f, fast));
-    return *reinterpret_cast<const uint32_t*>(&o);
+    const F2 y = f2_mul(f2_mul(f2_pack(fv.x, fv.y), f2_all(inv_f)), f2_pack(fg.x, fg.y));
+    float a0, a1, b0, b1;
+    f2_unpack(f2_mul(y, f2_all(1.f - 9.5367431640625e-07f)), a0, a1);
+    f2_unpack(f2_mul(y, f2_all(1.f + 9.5367431640625e-07f)), b0, b1);
+    const __half2 lower = __floats2half2_rn(a0, a1), upper = __floats2half2_rn(b0, b1);
+    uint32_t o = *reinterpret_cast<const uint32_t*>(&lower);
+    if (!fast || o != *reinterpret_cast<const uint32_t*>(&upper)) o = scale_defined(fv, fg, inv);
+    return o;
 }
 
 // ROWS: row-major [M, D]; else block-8 (D/8, M, 8).  grid = tiles * CS CTAs in clusters of CS.
@@ -174,6 +177,78 @@ __global__ void __launch_bounds__(RN_THREADS, RN_CTAS) add_rmsnorm_kernel(AddRms
     }
 }
 
+
+// The form for rows that fit a CTA's registers.  A row's JL threads keep its sums in registers (CPL chunks each) between
+// the passes: no shared-memory round trip of the sums, no cluster, one barrier.  What bounds the operator is how many
+// loads an SM has in flight and how long a CTA lives behind them, so the CTAs are small (their phases interleave) and
+// every thread requests all of its chunks before it uses the first.  4096 x 4096 row-major: 36.9 -> 25.6 us
+// (134 MB; the copy rate of this GPU gives 20.5), 8192 x 8192 118 -> 89 us (82), 16 x 4096 3.9 -> 2.6 us.
+template <bool ROWS, int CPL>
+__global__ void __launch_bounds__(RN_THREADS) add_rmsnorm_row_kernel(AddRmsNormParams p)
+{
+    pdl_launch_dependents();
+    pdl_wait();                                               // x or the residual may come from the kernel in front
+    __shared__ double s_part[RN_THREADS / 32 * 8];
+    const int TM = p.tile_tokens, JL = int(blockDim.x) / TM;  // tokens of the CTA x threads per token
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int dm = ROWS ? tid / JL : tid % TM, jl = ROWS ? tid % JL : tid / TM;
+    const int m = int(blockIdx.x) * TM + dm;
+    const int chunks = p.D / 8;
+    const bool live = m < p.M;
+    auto global_at = [&](int j) { return ROWS ? size_t(m) * chunks + j : size_t(j) * p.M + m; };
+    uint4 sum[CPL];
+    double acc = 0.0;
+    {
+        uint4 b[CPL];
+#pragma unroll
+        for (int u = 0; u < CPL; ++u) {
+            sum[u] = b[u] = make_uint4(0u, 0u, 0u, 0u);
+            const int j = jl + u * JL;
+            if (live && j < chunks) {
+                const size_t at = global_at(j);
+                sum[u] = ld_stream(p.x + at);
+                b[u] = ld_stream(p.residual + at);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < CPL; ++u) {
+            sum[u].x = add_pair(sum[u].x, b[u].x, acc);
+            sum[u].y = add_pair(sum[u].y, b[u].y, acc);
+            sum[u].z = add_pair(sum[u].z, b[u].z, acc);
+            sum[u].w = add_pair(sum[u].w, b[u].w, acc);
+        }
+    }
+    // a fixed tree over the lanes of a token inside each warp, then the warps in order
+    for (int step = ROWS ? 1 : TM; step < 32; step <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, step);
+    if (ROWS ? lane == 0 : lane < TM) s_part[ROWS ? warp : warp * TM + lane] = acc;
+    __syncthreads();
+    double total = 0.0;
+    if (ROWS) {
+        const int per = JL / 32;
+        for (int w = 0; w < per; ++w) total += s_part[dm * per + w];
+    } else {
+        for (int w = 0; w < int(blockDim.x) / 32; ++w) total += s_part[w * TM + dm];
+    }
+    const double inv = 1.0 / sqrt(total / double(p.D) + double(p.eps));
+    const float inv_f = __double2float_rn(inv);
+    const bool fast = inv_f >= 1.17549435e-38f && inv_f <= 3.402823466e38f;       // a normal float (false for NaN)
+    if (!live) return;
+#pragma unroll
+    for (int u = 0; u < CPL; ++u) {
+        const int j = jl + u * JL;
+        if (j < chunks) {
+            const uint4 s = sum[u], g = __ldg(p.gamma + j);
+            st_stream(p.residual_out + global_at(j), s);
+            uint4 o;
+            o.x = scale_pair(s.x, g.x, inv, inv_f, fast);
+            o.y = scale_pair(s.y, g.y, inv, inv_f, fast);
+            o.z = scale_pair(s.z, g.z, inv, inv_f, fast);
+            o.w = scale_pair(s.w, g.w, inv, inv_f, fast);
+            st_stream(p.norm_out + global_at(j), o);
+        }
+    }
+}
+
 } // namespace
 
 // Tile and cluster.  Candidates: tokens per tile a power of two up to 32 and up to the batch (in the block-8 layout
@@ -216,9 +291,64 @@ void add_rmsnorm_geometry(int M, int D, int row_major, int& tile_tokens, int& cl
             }
 }
 
+// Threads of a CTA, its tokens and the chunks per thread of the register form; false where the cluster form is taken:
+// block-8 rows too long for the registers of a CTA that covers four tokens (whose chunks of one column are the two
+// sectors a warp should touch at least), and tensors across the bus, which wants 128 contiguous bytes and more (128 x
+// 4096: 93 us against 180).  Measured on shapes from 1 x 1024 to 8192 x 8192: large tensors want many loads
+// per thread in small CTAs (4096 x 4096 row-major, 128 threads: four chunks 25.6 us, two 27.9, eight 30; block-8, four
+// tokens and eight chunks 33.3, two tokens 34.1), small ones want the whole GPU and short chains (16 x 4096: one chunk 2.6,
+// two 2.8 us; block-8 128 x 4096: two tokens 4.0, four 4.9 us, 16 x 4096: one token 3.2 us, two 3.7).
+static bool row_geometry(const AddRmsNormParams& p, int& threads, int& tokens, int& cpl)
+{
+    const int M = p.M, D = p.D, row_major = p.row_major;
+    if (p.over_bus && M > 1) return false;
+    const int chunks = D / 8;
+    const long long work = (long long)M * chunks;
+    auto power = [](int least, int x) { while (least < x) least <<= 1; return least; };
+    if (row_major) {
+        cpl = work >= (1 << 20) ? 4 : work >= (1 << 15) ? 2 : 1;
+        while (power(32, (chunks + cpl - 1) / cpl) > RN_THREADS) cpl <<= 1;          // (D <= 32768: eight at most)
+        const int lanes = power(32, (chunks + cpl - 1) / cpl);
+        threads = lanes < 128 ? 128 : lanes;
+        tokens = threads / lanes;
+        return true;
+    }
+    tokens = work >= (1 << 18) ? 4 : work >= (1 << 15) ? 2 : 1;
+    while (tokens > 1 && tokens / 2 >= M) tokens >>= 1;
+    cpl = tokens == 4 ? 8 : 1;
+    while (cpl < 8 && RN_THREADS / tokens * cpl < chunks) cpl <<= 1;
+    if (RN_THREADS / tokens * cpl < chunks && work >= (1 << 15)) return false;
+    while (RN_THREADS / tokens * cpl < chunks) tokens >>= 1;                          // (a few long rows: D <= 32768 fits one token)
+    threads = power(64, tokens * ((chunks + cpl - 1) / cpl));
+    return true;
+}
+
+template <bool ROWS>
+static cudaError_t launch_rows(const AddRmsNormParams& p, int threads, int cpl, cudaStream_t stream)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned((p.M + p.tile_tokens - 1) / p.tile_tokens));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    switch (cpl) {
+    case 1: return cudaLaunchKernelEx(&cfg, add_rmsnorm_row_kernel<ROWS, 1>, p);
+    case 2: return cudaLaunchKernelEx(&cfg, add_rmsnorm_row_kernel<ROWS, 2>, p);
+    case 4: return cudaLaunchKernelEx(&cfg, add_rmsnorm_row_kernel<ROWS, 4>, p);
+    default: return cudaLaunchKernelEx(&cfg, add_rmsnorm_row_kernel<ROWS, 8>, p);
+    }
+}
+
 cudaError_t launch_add_rmsnorm(const AddRmsNormParams& q, cudaStream_t stream)
 {
     AddRmsNormParams p = q;
+    int threads = 0, cpl = 0;
+    if (row_geometry(p, threads, p.tile_tokens, cpl))
+        return p.row_major ? launch_rows<true>(p, threads, cpl, stream) : launch_rows<false>(p, threads, cpl, stream);
     int cs = 1;
     add_rmsnorm_geometry(p.M, p.D, p.row_major, p.tile_tokens, cs);
     const int per = (p.D / 8 + cs - 1) / cs;
