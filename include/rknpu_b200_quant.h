@@ -126,7 +126,7 @@ typedef struct rk_npu_matmul_workspace_requirements {
     uint64_t bytes;           /* all device memory of the workspace */
     uint64_t input_bytes;     /* activation codes and the staged copy of A */
     uint64_t output_bytes;    /* the staged copy of C */
-    uint64_t control_bytes;   /* scales and the status block */
+    uint64_t control_bytes;   /* scales, sums of K parts, the status block */
     uint32_t wave_count;      /* ceil(K / k_tile), as the original reports it */
     uint32_t buffer_count;
 } rk_npu_matmul_workspace_requirements;

@@ -313,7 +313,7 @@ struct Call {
     bool keep_codes = false;   // fused kernel: also store the activation codes (diagnostic entry only)
     const int8_t* codes_in = nullptr;   // activations arrive as int8 codes [parts][M][K/parts]; scales from rowmax_in
     int parts = 1;
-    Status* status = nullptr;   // single-kernel families: where the launch reports (default: the workspace's device block)
+    Status* status = nullptr;   // page-locked block the call's verdict goes to (default: the workspace's device block)
 };
 
 // Split-K factor (= cluster size) of the single-kernel path: the largest split whose CTAs
@@ -370,7 +370,8 @@ void decode_params(const Call& c, DecodeParams& d, int cluster_override = 0)
     d.rowmax_in = c.rowmax_in;
     d.scales_out = ws.scales;
     d.codes_out = c.keep_codes ? ws.codes : nullptr;
-    d.status = c.status ? c.status : ws.status;
+    d.status = ws.status;
+    d.report = c.status ? c.status : ws.status;
     d.M = cfg.M; d.N = N; d.K = cfg.K;
     d.KB = ws.KB; d.NG = c.w->NG; d.F = F; d.epi = c.epi;
     d.half = c.half ? 1 : 0;
@@ -414,7 +415,8 @@ int enqueue(const Call& c)
         f.rowmax_in = c.rowmax_in;
         f.scales_out = ws.scales;
         f.codes_out = c.keep_codes ? ws.codes : nullptr;
-        f.status = c.status ? c.status : ws.status;
+        f.status = ws.status;
+        f.report = c.status ? c.status : ws.status;
         f.M = cfg.M; f.N = N; f.K = cfg.K;
         f.KB = ws.KB; f.NG = c.w->NG; f.F = F; f.epi = c.epi;
         f.split = fused_split(ws, tiles);
@@ -449,7 +451,7 @@ int enqueue(const Call& c)
     q.rowmax_zero = nullptr;
     q.rowmax = c.rowmax_in;
     q.status = ws.status;
-    q.host_flag = nullptr;
+    q.host_flag = c.status ? &c.status->bad_input : nullptr;
     q.M = cfg.M;
     q.K = cfg.K;
     q.Kp = ws.KB * KBLOCK;
@@ -467,6 +469,7 @@ int enqueue(const Call& c)
     g.out = c.dOut;
     g.rowmax = c.rowmax_out;
     g.status = ws.status;
+    g.report = c.status ? &c.status->device_error : nullptr;
     g.M = cfg.M;
     g.N = N;
     g.K = cfg.K;
@@ -558,6 +561,47 @@ int enqueue_linear(Call call, void* dOut)
     return rc;
 }
 
+// ---- ordinary (pageable) host tensors of the blocking calls
+// Small ones pass through the workspace's page-locked pieces: a host copy and a copy engine transfer beat the staging the
+// driver does for pageable memory (64 KB to the device 11 against 16 us, 256 KB back 23 against 33).  Larger ones go
+// directly: the host copy then runs out of the caches and is no faster (1 MB either way: the same within the noise).
+constexpr size_t BOUNCE_IN = size_t(256) << 10, BOUNCE_OUT = size_t(512) << 10;
+
+bool upload(rk_npu_w4a8_workspace& ws, void* device, const void* host, size_t bytes, bool locked, cudaStream_t s)
+{
+    if (!locked && bytes <= BOUNCE_IN && bytes <= ws.bounce_in.bytes) host = std::memcpy(ws.bounce_in.ptr, host, bytes);
+    return cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
+}
+
+struct Download {
+    void* host;
+    const void* device;
+    size_t bytes;
+    bool locked;      // the host tensor is page-locked
+};
+// Brings results to the caller's tensors and waits for the stream.  What passes through the workspace's piece is handed to
+// the caller only if verdict() returns RK_NPU_OK (a direct copy of a rejected call brings back what the device buffer held,
+// as it always did).
+template <class Verdict>
+int download(rk_npu_w4a8_workspace& ws, const Download* list, int count, cudaStream_t s, Verdict verdict)
+{
+    uint8_t* const piece = static_cast<uint8_t*>(ws.bounce_out.ptr);
+    const size_t room = std::min(BOUNCE_OUT, ws.bounce_out.bytes);
+    size_t used = 0, place[2] = {};
+    bool staged[2] = {}, ok = true;
+    for (int i = 0; i < count; ++i) {
+        const Download& d = list[i];
+        staged[i] = !d.locked && used + d.bytes <= room;
+        if (staged[i]) { place[i] = used; used += (d.bytes + 63) / 64 * 64; }
+        ok = ok && cudaMemcpyAsync(staged[i] ? piece + place[i] : d.host, d.device, d.bytes, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+    }
+    if (cudaStreamSynchronize(s) != cudaSuccess || !ok) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+    const int rc = verdict();
+    for (int i = 0; i < count && !rc; ++i)
+        if (staged[i]) std::memcpy(list[i].host, piece + place[i], list[i].bytes);
+    return rc;
+}
+
 // One blocking projection; the caller holds the workspace.
 int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const void* A, void* C, bool half, int epi,
                rk_npu_w4a8_timings* metrics)
@@ -576,27 +620,25 @@ int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const vo
     void* dC = C;
     auto copy_start = Clock::now();
     if (!a_dev) {
-        // ordinary (pageable) host memory: a small tensor is copied into the workspace's page-locked piece first -- the
-        // host copy is cheaper than the staging the driver does for pageable memory
-        const void* from = A;
-        if (!a_at.alias && ws->bounce_in && in_bytes <= ws->bounce_bytes) { std::memcpy(ws->bounce_in, A, in_bytes); from = ws->bounce_in; }
-        if (cudaMemcpyAsync(ws->stage_in, from, in_bytes, cudaMemcpyHostToDevice, s) != cudaSuccess) return RK_NPU_ERR_SUBMIT;
+        if (!upload(*ws, ws->stage_in, A, in_bytes, a_at.alias != nullptr, s)) return RK_NPU_ERR_SUBMIT;
         dA = ws->stage_in;
     }
-    // A small batch through one of the single-kernel families writes every output element once and reports through two
-    // plain stores, so a host caller is served without the two copies behind the kernel: the kernel stores straight
-    // into the caller's tensor when that is page-locked memory the GPU can address, and reports into the workspace's
-    // own page-locked status block.  (The activations are still copied in: every CTA reads them.)
+    // The verdict of a call lands in page-locked memory by itself (plain stores of the kernels), and so does a small
+    // result: straight in the caller's tensor when that is page-locked, else in the workspace's piece, from where the host
+    // copies it out.  (The activations are still copied in: every CTA reads them.)  The single-kernel families write
+    // every element once, in rows as long as a warp; the others in pieces of 64 bytes, which the bus takes more slowly, so
+    // that from 128 KB on the copy engine is as fast.
     // (Not when the caller asks for stage timings: the device part of a call must not contain stores that cross the bus,
     // or the figures of different kernel families -- which the search tuner ranks -- stop being comparable.)
-    const bool single_kernel = (ws->variant == 3 || ws->variant == 5) && !grouped(*ws) && epi != EPI_SWIGLU && !metrics;
-    void* c_alias = (!c_dev && single_kernel && out_bytes <= (size_t(1) << 20)) ? c_at.alias : nullptr;
-    // ... and an ordinary host result of a small batch lands in the workspace's page-locked piece and is copied out by the host
-    const bool bounce_out = !c_dev && !c_alias && single_kernel && ws->bounce_out_alias && out_bytes <= ws->bounce_bytes;
-    if (bounce_out) c_alias = ws->bounce_out_alias;
+    const bool own_report = !grouped(*ws) && !metrics && ws->host_status_alias;
+    const bool single_kernel = ws->variant == 3 || ws->variant == 5;
+    const bool bus_result = !c_dev && own_report && epi != EPI_SWIGLU && out_bytes <= (single_kernel ? size_t(512) << 10 : size_t(128) << 10);
+    void* c_alias = bus_result ? c_at.alias : nullptr;
+    const bool bounce_out = bus_result && !c_alias && ws->bounce_out.alias && out_bytes <= ws->bounce_out.bytes;
+    if (bounce_out) c_alias = ws->bounce_out.alias;
     if (c_alias) dC = c_alias;
     else if (!c_dev) dC = ws->stage_out;
-    Status* status_alias = single_kernel ? ws->host_status_alias : nullptr;
+    Status* status_alias = own_report ? ws->host_status_alias : nullptr;
     if (status_alias) *ws->host_status = Status{};
     t.sync_us += elapsed_us(copy_start);
     Call call{ws, w, dA, dC, half, epi, nullptr, nullptr, s, metrics ? ws->events : nullptr, epi == EPI_I32};
@@ -604,12 +646,10 @@ int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const vo
     int rc = enqueue_linear(call, dC);
     if (rc) { cudaStreamSynchronize(s); return rc; }
     copy_start = Clock::now();
-    // Other host tensors are copied straight from and to the caller's memory.
-    if (!c_dev && !c_alias) cudaMemcpyAsync(C, dC, out_bytes, cudaMemcpyDeviceToHost, s);
     if (!status_alias) cudaMemcpyAsync(ws->host_status, ws->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
-    rc = status_to_rc(*ws, s);
-    if (bounce_out && rc == RK_NPU_OK) std::memcpy(C, ws->bounce_out, out_bytes);
+    const Download down[1] = {{C, dC, out_bytes, c_at.alias != nullptr}};
+    rc = download(*ws, down, !c_dev && !c_alias ? 1 : 0, s, [&] { return status_to_rc(*ws, s); });
+    if (bounce_out && rc == RK_NPU_OK) std::memcpy(C, ws->bounce_out.ptr, out_bytes);
     t.sync_us += elapsed_us(copy_start);
     if (metrics) {
         t.activation_scan_us = event_us(ws->events[0], ws->events[1]);
@@ -643,8 +683,10 @@ void workspace_destroy(rk_npu_w4a8_workspace* ws)
     if (ws->status) device_free(d, ws->status, sizeof(Status));
     if (ws->stage_in) device_free(d, ws->stage_in, ws->stage_in_bytes);
     if (ws->stage_out) device_free(d, ws->stage_out, ws->stage_out_bytes);
-    if (ws->bounce_in) cudaFreeHost(ws->bounce_in);
-    if (ws->bounce_out) cudaFreeHost(ws->bounce_out);
+    if (d) {
+        host_piece_release(d->ctx, ws->bounce_in);
+        host_piece_release(d->ctx, ws->bounce_out);
+    }
     if (ws->trace) device_free(d, ws->trace, ws->trace_bytes);
     if (ws->partials) device_free(d, ws->partials, ws->partials_bytes);
     if (ws->counts) device_free(d, ws->counts, ws->counts_bytes);
@@ -660,6 +702,47 @@ void workspace_destroy(rk_npu_w4a8_workspace* ws)
 
 // ================================================================== domains, context
 namespace rkb200 {
+rk_npu_ctx::HostPiece host_piece_acquire(rk_npu_ctx* ctx, size_t bytes)
+{
+    size_t size = size_t(64) << 10;
+    while (size < bytes) size <<= 1;
+    {
+        std::lock_guard<std::mutex> g(ctx->host_lock);
+        for (size_t i = 0; i < ctx->host_free.size(); ++i)
+            if (ctx->host_free[i].bytes == size) {
+                const rk_npu_ctx::HostPiece piece = ctx->host_free[i];
+                ctx->host_free.erase(ctx->host_free.begin() + long(i));
+                ctx->host_free_bytes -= size;
+                return piece;
+            }
+    }
+    rk_npu_ctx::HostPiece piece{nullptr, nullptr, size};
+    if (cudaHostAlloc(&piece.ptr, size, cudaHostAllocMapped) != cudaSuccess) { cudaGetLastError(); return {}; }
+    if (cudaHostGetDevicePointer(&piece.alias, piece.ptr, 0) != cudaSuccess) { cudaGetLastError(); piece.alias = nullptr; }
+    return piece;
+}
+// The caller has synchronised whatever used the piece.
+void host_piece_release(rk_npu_ctx* ctx, rk_npu_ctx::HostPiece& piece)
+{
+    if (!piece.ptr) return;
+    bool keep = false;
+    {
+        std::lock_guard<std::mutex> g(ctx->host_lock);
+        keep = ctx->host_free_bytes + piece.bytes <= HOST_PIECES_KEPT;
+        if (keep) {
+            try { ctx->host_free.push_back(piece); ctx->host_free_bytes += piece.bytes; } catch (...) { keep = false; }
+        }
+    }
+    if (!keep) cudaFreeHost(piece.ptr);
+    piece = {};
+}
+void host_pieces_drop(rk_npu_ctx* ctx)
+{
+    std::lock_guard<std::mutex> g(ctx->host_lock);
+    for (auto& piece : ctx->host_free) cudaFreeHost(piece.ptr);
+    ctx->host_free.clear();
+    ctx->host_free_bytes = 0;
+}
 void domain_retain(rk_npu_iommu_domain* d) { if (d) d->refs.fetch_add(1, std::memory_order_relaxed); }
 void domain_release(rk_npu_iommu_domain* d)
 {
@@ -754,6 +837,7 @@ extern "C" void rk_npu_close(rk_npu_ctx* ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) { cudaStreamSynchronize(ctx->stream); cudaStreamDestroy(ctx->stream); }
     group_close(ctx);
+    host_pieces_drop(ctx);
     delete ctx;
 }
 
@@ -1130,19 +1214,11 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
              cudaStreamSynchronize(ws->stream) == cudaSuccess;
         std::memset(ws->host_status, 0, sizeof(Status));
         ws->host_status_alias = static_cast<Status*>(mapped_alias(ws->host_status));
-        // page-locked pieces for small host tensors of the blocking calls (optional: without them the calls copy directly)
-        const size_t most = std::max(ws->stage_in_bytes, ws->stage_out_bytes);
-        if ((variant == 3 || variant == 5) && ctx->world == 1 && most <= (size_t(1) << 20)) {
-            if (cudaHostAlloc(&ws->bounce_in, most, cudaHostAllocDefault) == cudaSuccess &&
-                cudaHostAlloc(&ws->bounce_out, most, cudaHostAllocMapped) == cudaSuccess) {
-                ws->bounce_bytes = most;
-                ws->bounce_out_alias = mapped_alias(ws->bounce_out);
-            } else {
-                cudaGetLastError();
-                if (ws->bounce_in) cudaFreeHost(ws->bounce_in);
-                if (ws->bounce_out) cudaFreeHost(ws->bounce_out);
-                ws->bounce_in = ws->bounce_out = nullptr;
-            }
+        // page-locked pieces for ordinary host tensors of the blocking calls (optional: without them the calls copy directly)
+        const size_t in_most = size_t(cfg->M) * cfg->K * 4, out_most = size_t(cfg->M) * cfg->N * 4;
+        if (cfg->M <= 128) {
+            ws->bounce_in = host_piece_acquire(ctx, std::min(in_most, BOUNCE_IN));
+            ws->bounce_out = host_piece_acquire(ctx, std::min(out_most, BOUNCE_OUT));
         }
     }
     if (!ok) { cudaGetLastError(); workspace_destroy(ws); return nullptr; }
@@ -1203,19 +1279,23 @@ extern "C" int rk_npu_w4a8_run_ffn_f32(rk_npu_w4a8_workspace* gate_up, const rk_
         const int M = gate_up->config.M, K = gate_up->config.K, F = gate_up->config.N / 2, N = down->config.N;
         if (cudaSetDevice(gate_up->domain->ctx->device) != cudaSuccess) return RK_NPU_ERR_SUBMIT;
         cudaStream_t s = gate_up->stream;
-        const bool a_dev = on_device(A), m_dev = on_device(middle), c_dev = on_device(C);
+        const Placement a_at = placement(A), m_at = placement(middle), c_at = placement(C);
+        const bool a_dev = a_at.device, m_dev = m_at.device, c_dev = c_at.device;
         const void* dA = A;
         float* dMiddle = m_dev ? middle : static_cast<float*>(gate_up->stage_out);
         float* dC = c_dev ? C : static_cast<float*>(down->stage_out);
         auto mark = Clock::now();
         if (!a_dev) {
-            if (cudaMemcpyAsync(gate_up->stage_in, A, size_t(M) * K * 4, cudaMemcpyHostToDevice, s) != cudaSuccess)
-                return RK_NPU_ERR_SUBMIT;
+            if (!upload(*gate_up, gate_up->stage_in, A, size_t(M) * K * 4, a_at.alias != nullptr, s)) return RK_NPU_ERR_SUBMIT;
             dA = gate_up->stage_in;
         }
+        // (the verdicts land in page-locked memory by themselves, as in a single projection)
+        const bool own_report = !grouped(*gate_up) && !metrics && gate_up->host_status_alias && down->host_status_alias;
+        if (own_report) *gate_up->host_status = *down->host_status = Status{};
         t.gate_up.sync_us += elapsed_us(mark);
         cudaEvent_t* ev = metrics ? gate_up->events : nullptr;
         Call first{gate_up, gate_up_weights, dA, dMiddle, false, EPI_SWIGLU, gate_up->rowmax, nullptr, s, ev};
+        if (own_report) first.status = gate_up->host_status_alias;
         rc = enqueue_linear(first, dMiddle);
         // in a group every GPU has collected the maxima of its feature slice: the row maximum is their maximum
         if (!rc && grouped(*gate_up)) rc = group_all_reduce_max_u32(gate_up->domain->ctx, gate_up->rowmax, size_t(M), s);
@@ -1224,19 +1304,26 @@ extern "C" int rk_npu_w4a8_run_ffn_f32(rk_npu_w4a8_workspace* gate_up, const rk_
             // no rescan (src/rk_npu_w4a8.cpp:112-121,376); a non-finite maximum makes the
             // down kernels return without work.
             Call second{down, down_weights, dMiddle, dC, false, EPI_F32, nullptr, gate_up->rowmax, s, metrics ? down->events : nullptr};
+            if (own_report) second.status = down->host_status_alias;
             rc = enqueue_linear(second, dC);
         }
         if (rc) { cudaStreamSynchronize(s); return rc; }
         mark = Clock::now();
-        if (!m_dev) cudaMemcpyAsync(middle, dMiddle, size_t(M) * F * 4, cudaMemcpyDeviceToHost, s);
-        if (!c_dev) cudaMemcpyAsync(C, dC, size_t(M) * N * 4, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(gate_up->host_status, gate_up->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(down->host_status, down->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        if (!own_report) {
+            cudaMemcpyAsync(gate_up->host_status, gate_up->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(down->host_status, down->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
+        }
+        Download results[2];
+        int count = 0;
+        if (!c_dev) results[count++] = {C, dC, size_t(M) * N * 4, c_at.alias != nullptr};
+        if (!m_dev) results[count++] = {middle, dMiddle, size_t(M) * F * 4, m_at.alias != nullptr};
+        int rc_down = RK_NPU_OK;
+        rc = download(*gate_up, results, count, s, [&] {
+            const int rc_gate = status_to_rc(*gate_up, s);
+            rc_down = status_to_rc(*down, s);
+            return rc_gate ? rc_gate : rc_down;
+        });
         t.down.sync_us += elapsed_us(mark);
-        rc = status_to_rc(*gate_up, s);
-        const int rc_down = status_to_rc(*down, s);
-        if (!rc) rc = rc_down;
         if (metrics) {
             t.gate_up.activation_scan_us = event_us(gate_up->events[0], gate_up->events[1]);
             t.gate_up.submit_us = event_us(gate_up->events[1], gate_up->events[2]);

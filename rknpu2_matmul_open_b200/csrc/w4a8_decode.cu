@@ -194,7 +194,7 @@ __device__ __forceinline__ void decode_cta(const DecodeParams& p, const unsigned
                                 deadline = global_ns() + p.timeout_ns;
                             }
                             if (!mbar_wait(&empty[slot], (turn - 1u) & 1u, deadline)) {
-                                *reinterpret_cast<volatile int*>(&p.status->device_error) = 1;   // (a plain store: the block may be page-locked host memory)
+                                *reinterpret_cast<volatile int*>(&p.report->device_error) = 1;   // (a plain store: the block may be page-locked host memory)
                                 return;
                             }
                         }
@@ -482,10 +482,10 @@ __device__ __forceinline__ void decode_cta(const DecodeParams& p, const unsigned
     }
 
     // ---- bookkeeping
-    if (failed && lane == 0) *reinterpret_cast<volatile int*>(&p.status->device_error) = 1;   // (a plain store: the block may be page-locked host memory)
+    if (failed && lane == 0) *reinterpret_cast<volatile int*>(&p.report->device_error) = 1;   // (a plain store: the block may be page-locked host memory)
     if (TRACE && trace) trace[7] = global_ns();
     if (tid == 0) {
-        if (cta == 0) p.status->bad_input = verdict;
+        if (cta == 0) p.report->bad_input = verdict;
         if (no_scan) {
             // Every CTA has read the collected maxima by now; the last one to get here clears them
             // for the next SwiGLU epilogue.  The ticket counter wraps by itself.

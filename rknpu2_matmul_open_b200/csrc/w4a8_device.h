@@ -90,6 +90,12 @@ struct CodesInParams {
     int parts;
 };
 
+// A bounded wait ran out (a plain store: the word may be page-locked host memory).
+__device__ __forceinline__ void report_device_error(Status* status, int* report)
+{
+    *reinterpret_cast<volatile int*>(report ? report : &status->device_error) = 1;
+}
+
 struct GemmParams {
     const uint8_t* Wp;
     const uint8_t* Xq;
@@ -98,6 +104,7 @@ struct GemmParams {
     void* out;              // [M,N] fp32 / fp16 / int32, or middle [M,F] fp32
     uint32_t* rowmax;       // SwiGLU: per-row max |middle| bit pattern (nullable)
     Status* status;
+    int* report;            // where a wait that ran out is recorded: a word of page-locked host memory, or NULL for status->device_error
     int M, N, K;
     int KB;                 // k-blocks (Kp / 128)
     int NG;                 // weight groups (padded)
@@ -125,7 +132,8 @@ struct FusedParams {
     uint32_t* rowmax_in;        // non-null: row scales come from these bits (no scan); cleared after use
     float* scales_out;          // [M] per-token scales, written by the first CTA
     uint8_t* codes_out;         // activation codes in the Xq layout with T = tokens per CTA (nullable)
-    Status* status;
+    Status* status;             // the workspace's block (its ticket counter)
+    Status* report;             // where the verdict goes: the same block or one in page-locked host memory
     int M, N, K;
     int KB, NG, F, epi;
     int split;                  // cluster size along y == split-K factor
@@ -147,7 +155,8 @@ struct DecodeParams {
     uint32_t* rowmax_in;        // non-null: row scales come from these bits (no scan); cleared after use
     float* scales_out;          // [M] per-token scales, written by the first cluster
     uint8_t* codes_out;         // activation codes in the Xq layout with T = 8 (nullable)
-    Status* status;
+    Status* status;             // the workspace's block (its ticket counter)
+    Status* report;             // where the verdict goes: the same block or one in page-locked host memory
     int M, N, K;
     int KB, NG, F, epi;
     int half;                   // activations are binary16

@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     __syncthreads();
     cluster_arrive();
     cluster_wait();   // neither CTA frees tensor memory or leaves while the other may still use it
-    if (tid == 0 && *s_error) atomicExch(&p.status->device_error, 1);
+    if (tid == 0 && *s_error) report_device_error(p.status, p.report);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PS_TMEM_COLS) : "memory");

@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <mutex>
 #include <string>
+#include <vector>
 
 struct rk_npu_ctx {
     int device = 0;
@@ -13,6 +14,12 @@ struct rk_npu_ctx {
     uint32_t driver_version = 0;  // CUDA driver version; part of the tuning-cache key
     int sm_count = 0;
     cudaStream_t stream = nullptr;  // weight uploads
+    // Page-locked pieces that workspaces borrow for their lifetime (host_piece_acquire / _release): creating one takes
+    // the driver a good part of a millisecond.  Free pieces are kept up to HOST_PIECES_KEPT bytes, the rest go back.
+    struct HostPiece { void* ptr; void* alias; size_t bytes; };
+    std::mutex host_lock;
+    std::vector<HostPiece> host_free;
+    size_t host_free_bytes = 0;
     // group of GPUs (rk_npu_b200_open_group): this context is `rank` of `world`; comm is the NCCL communicator
     int rank = 0, world = 1;
     void* comm = nullptr;
@@ -57,6 +64,12 @@ void domain_release(rk_npu_iommu_domain* d);
 // Device allocations are accounted to the owning domain.
 int device_alloc(rk_npu_iommu_domain* d, void** ptr, size_t bytes);
 void device_free(rk_npu_iommu_domain* d, void* ptr, size_t bytes);
+
+// A page-locked piece of at least `bytes` that the GPU can address, borrowed from the context; ptr is NULL on failure.
+constexpr size_t HOST_PIECES_KEPT = size_t(16) << 20;
+rk_npu_ctx::HostPiece host_piece_acquire(rk_npu_ctx* ctx, size_t bytes);
+void host_piece_release(rk_npu_ctx* ctx, rk_npu_ctx::HostPiece& piece);
+void host_pieces_drop(rk_npu_ctx* ctx);
 
 // ---- group of GPUs (w4a8_group.cpp)
 void group_close(rk_npu_ctx* ctx);
@@ -130,9 +143,8 @@ struct rk_npu_w4a8_workspace {
     size_t codes_bytes = 0, stage_in_bytes = 0, stage_out_bytes = 0;
     rkb200::Status* host_status = nullptr;  // pinned
     rkb200::Status* host_status_alias = nullptr;   // its device address (NULL if the GPU cannot address it)
-    void* bounce_in = nullptr;        // page-locked pieces the blocking calls copy small ordinary host tensors through
-    void* bounce_out = nullptr, *bounce_out_alias = nullptr;
-    size_t bounce_bytes = 0;
+    // page-locked pieces the blocking calls copy small ordinary host tensors through (ptr NULL: copied directly)
+    rk_npu_ctx::HostPiece bounce_in{}, bounce_out{};
     cudaEvent_t events[8]{};
     std::atomic<uint64_t> launches{0};
     unsigned long long* trace = nullptr;   // device stamps, allocated by rk_npu_b200_w4a8_trace_enable

@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
                 for (int it = pre; it < nkb; ++it) {
                     const int s = it % MMA_STAGES;
                     if (!mbar_wait(&empty[s], ((it / MMA_STAGES) - 1) & 1, deadline)) {
-                        atomicExch(&p.status->device_error, 1);
+                        report_device_error(p.status, p.report);
                         break;
                     }
                     mbar_arrive_expect_tx(&full[s], STAGE);
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
         for (int it = 0; it < iters; ++it) {
             const int s = it % MMA_STAGES;
             if (!mbar_wait(&full[s], (it / MMA_STAGES) & 1, deadline)) {
-                if (lane == 0) atomicExch(&p.status->device_error, 1);
+                if (lane == 0) report_device_error(p.status, p.report);
                 break;
             }
             if (!skip) {

@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_tc_stream_kernel(const Gem
     // ------------------------------------------------------------------------ teardown
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && s_flag[1]) atomicExch(&p.status->device_error, 1);
+    if (tid == 0 && s_flag[1]) report_device_error(p.status, p.report);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TS_TMEM_COLS) : "memory");

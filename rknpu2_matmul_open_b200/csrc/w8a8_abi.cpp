@@ -54,7 +54,8 @@ struct rk_npu_matmul_workspace {
     void* stage_in = nullptr;
     void* stage_out = nullptr;
     size_t codes_bytes = 0, partials_bytes = 0, counts_bytes = 0, scale_bytes = 0, stage_in_bytes = 0, stage_out_bytes = 0;
-    Status* host_status = nullptr;    // pinned
+    Status* host_status = nullptr;    // pinned; a wait that ran out is recorded there through its device alias
+    Status* host_status_alias = nullptr;
     std::atomic<uint64_t> launches{0};
 };
 
@@ -266,6 +267,8 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     g.sw = w->scales;
     g.out = dC;
     g.status = ws->status;
+    g.report = &ws->host_status_alias->device_error;
+    *ws->host_status = Status{};
     g.M = st.M; g.N = st.N; g.K = st.K;
     g.KB = ws->KB; g.NG = w->NG; g.T = ws->T;
     g.epi = kind == RK_NPU_MATMUL_I8I8I32 ? EPI_I32 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? EPI_F16 : EPI_F32);
@@ -274,17 +277,15 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     g.partials = ws->partials;
     g.counts = ws->counts;
     g.timeout_ns = (unsigned long long)W8_TIMEOUT_MS * 1000000ull;
-    if (launch_w8_quantize(q, s) != cudaSuccess || launch_gemm_tc_persist(g, s, false) != cudaSuccess) {
+    if (launch_w8_quantize(q, s) != cudaSuccess || launch_gemm_tc_persist(g, s, true) != cudaSuccess) {
         cudaGetLastError();
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
     }
     ws->launches.fetch_add(2, std::memory_order_relaxed);
     if (!c_dev) cudaMemcpyAsync(C, dC, ws->stage_out_bytes, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(ws->host_status, ws->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
     if (ws->host_status->device_error) {       // a bounded wait inside the kernel ran out: report, clear, stay usable
-        cudaMemsetAsync(&ws->status->device_error, 0, sizeof(int), s);
         if (ws->counts) cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;
@@ -324,8 +325,8 @@ extern "C" int rk_npu_matmul_workspace_memory_query(const rk_npu_matmul_strategy
     const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind), QUERY_SMS);
     std::memset(out, 0, sizeof(*out));
     out->input_bytes = z.codes + z.stage_in;
-    out->output_bytes = z.stage_out + z.partials;
-    out->control_bytes = z.scales + z.counts + sizeof(Status);
+    out->output_bytes = z.stage_out;
+    out->control_bytes = z.scales + z.partials + z.counts + sizeof(Status);
     out->bytes = out->input_bytes + out->output_bytes + out->control_bytes;
     out->wave_count = uint32_t((strategy->K + strategy->k_tile - 1) / strategy->k_tile);
     out->buffer_count = 7;
@@ -360,7 +361,8 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     ws->stage_out_bytes = z.stage_out;
     domain_retain(domain);
     bool ok = cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaMallocHost(reinterpret_cast<void**>(&ws->host_status), sizeof(Status)) == cudaSuccess;
+              cudaHostAlloc(reinterpret_cast<void**>(&ws->host_status), sizeof(Status), cudaHostAllocMapped) == cudaSuccess &&
+              cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws->host_status_alias), ws->host_status, 0) == cudaSuccess;
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes) &&
          (!ws->partials_bytes || (!device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes) &&
                                   !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes))) &&

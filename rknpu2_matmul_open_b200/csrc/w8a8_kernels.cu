@@ -62,6 +62,7 @@ template <bool HALF>
 __global__ void __launch_bounds__(256) w8_quantize_kernel(const W8QuantParams p)
 {
     using T = typename ActType<HALF>::type;
+    pdl_launch_dependents();   // the GEMM behind this kernel may set itself up and request its weights
     const int m = blockIdx.x, tid = threadIdx.x;
     const T* row = reinterpret_cast<const T*>(p.A) + (size_t)m * p.K;
     const bool vec = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(256) w8_quantize_kernel(const W8QuantParams p)
 // int8 activations as given -> the Xq layout; every token's scale is 1
 __global__ void __launch_bounds__(256) w8_codes_kernel(const W8QuantParams p)
 {
+    pdl_launch_dependents();
     const int m = blockIdx.x, tid = threadIdx.x;
     const int8_t* row = reinterpret_cast<const int8_t*>(p.A) + (size_t)m * p.K;
     const int chunks = p.Kp / 16;

@@ -27,17 +27,18 @@ class W4A8Error(RuntimeError):
 
 
 def _ptr(t):
-    """Raw address of a numpy array or a torch tensor (host or device)."""
+    """Raw address of a numpy array or a torch tensor (host or device), as the integer the C prototypes take."""
     if t is None:
         return None
-    if isinstance(t, np.ndarray):
-        if not t.flags["C_CONTIGUOUS"]:
-            raise ValueError("tensor must be compact row-major")
-        return C.c_void_p(t.ctypes.data)
-    if hasattr(t, "data_ptr"):
+    data_ptr = getattr(t, "data_ptr", None)
+    if data_ptr is not None:
         if not t.is_contiguous():
             raise ValueError("tensor must be compact row-major")
-        return C.c_void_p(t.data_ptr())
+        return data_ptr()
+    if isinstance(t, np.ndarray):
+        if not t.flags.c_contiguous:
+            raise ValueError("tensor must be compact row-major")
+        return t.__array_interface__["data"][0]
     raise TypeError(f"unsupported tensor type {type(t)}")
 
 
@@ -68,7 +69,7 @@ class Context:
 
     def all_gather(self, dBuffer, bytes_per_rank: int, stream: int = 0) -> int:
         """rk_npu_b200_group_all_gather: in-place all-gather of the group (every rank's piece at its slot)."""
-        return self.lib.rk_npu_b200_group_all_gather(self.handle, _ptr(dBuffer), bytes_per_rank, C.c_void_p(stream))
+        return self.lib.rk_npu_b200_group_all_gather(self.handle, _ptr(dBuffer), bytes_per_rank, stream)
 
     def domain(self, domain_id: int = 0) -> "Domain":
         return Domain(self, domain_id)
@@ -179,27 +180,25 @@ class Workspace:
 
     # ---- enqueue forms (device tensors, caller's stream)
     def enqueue_f16(self, weights: Weights, dA, dC, stream: int = 0) -> int:
-        return self.lib.rk_npu_b200_w4a8_enqueue_f16(self.handle, weights.handle, _ptr(dA), _ptr(dC), C.c_void_p(stream))
+        return self.lib.rk_npu_b200_w4a8_enqueue_f16(self.handle, weights.handle, _ptr(dA), _ptr(dC), stream)
 
     def enqueue_f32(self, weights: Weights, dA, dC, stream: int = 0) -> int:
-        return self.lib.rk_npu_b200_w4a8_enqueue_f32(self.handle, weights.handle, _ptr(dA), _ptr(dC), C.c_void_p(stream))
+        return self.lib.rk_npu_b200_w4a8_enqueue_f32(self.handle, weights.handle, _ptr(dA), _ptr(dC), stream)
 
     def enqueue_swiglu_f32(self, weights: Weights, dA, dMiddle, stream: int = 0) -> int:
-        return self.lib.rk_npu_b200_w4a8_enqueue_swiglu_f32(self.handle, weights.handle, _ptr(dA), _ptr(dMiddle),
-                                                            C.c_void_p(stream))
+        return self.lib.rk_npu_b200_w4a8_enqueue_swiglu_f32(self.handle, weights.handle, _ptr(dA), _ptr(dMiddle), stream)
 
     # ---- column-sharded FFN: the pieces around the exchange between GPUs (rknpu_b200_ext.h)
     def enqueue_swiglu_collect_f32(self, weights: Weights, dA, dMiddle, dRowMaxima, stream: int = 0) -> int:
         return self.lib.rk_npu_b200_w4a8_enqueue_swiglu_collect_f32(self.handle, weights.handle, _ptr(dA), _ptr(dMiddle),
-                                                                    _ptr(dRowMaxima), C.c_void_p(stream))
+                                                                    _ptr(dRowMaxima), stream)
 
     def enqueue_quantize_slice(self, dMiddle, dRowMaxima, dCodes, stream: int = 0) -> int:
-        return self.lib.rk_npu_b200_w4a8_enqueue_quantize_slice(self.handle, _ptr(dMiddle), _ptr(dRowMaxima), _ptr(dCodes),
-                                                                C.c_void_p(stream))
+        return self.lib.rk_npu_b200_w4a8_enqueue_quantize_slice(self.handle, _ptr(dMiddle), _ptr(dRowMaxima), _ptr(dCodes), stream)
 
     def enqueue_codes_f32(self, weights: Weights, dCodes, parts: int, dRowMaxima, dC, stream: int = 0) -> int:
         return self.lib.rk_npu_b200_w4a8_enqueue_codes_f32(self.handle, weights.handle, _ptr(dCodes), int(parts),
-                                                           _ptr(dRowMaxima), _ptr(dC), C.c_void_p(stream))
+                                                           _ptr(dRowMaxima), _ptr(dC), stream)
 
     # ---- group of GPUs: this rank's columns only, no exchange
     def shard(self):
@@ -209,10 +208,10 @@ class Workspace:
         return bool(v[0].value), v[1].value, v[2].value, v[3].value
 
     def enqueue_local_f16(self, weights: Weights, dA, dLocal, stream: int = 0) -> int:
-        return self.lib.rk_npu_b200_w4a8_enqueue_local_f16(self.handle, weights.handle, _ptr(dA), _ptr(dLocal), C.c_void_p(stream))
+        return self.lib.rk_npu_b200_w4a8_enqueue_local_f16(self.handle, weights.handle, _ptr(dA), _ptr(dLocal), stream)
 
     def enqueue_local_f32(self, weights: Weights, dA, dLocal, stream: int = 0) -> int:
-        return self.lib.rk_npu_b200_w4a8_enqueue_local_f32(self.handle, weights.handle, _ptr(dA), _ptr(dLocal), C.c_void_p(stream))
+        return self.lib.rk_npu_b200_w4a8_enqueue_local_f32(self.handle, weights.handle, _ptr(dA), _ptr(dLocal), stream)
 
     def finish(self) -> int:
         return self.lib.rk_npu_b200_w4a8_finish(self.handle)
@@ -243,20 +242,22 @@ def run_ffn_f32(gate_up: Workspace, gate_up_weights: Weights, down: Workspace, d
                                                C.byref(timings) if timings is not None else None)
 
 
+_POINTERS = [C.c_void_p * n for n in range(5)]     # the array types of up to four linears, made once
+
+
 def enqueue_batch_f16(workspaces, weights, dAs, dLocals, stream: int = 0) -> int:
     """rk_npu_b200_w4a8_enqueue_batch_f16: up to four independent decode linears (same token count) in one launch."""
     n = len(workspaces)
-    arr = lambda items: (C.c_void_p * n)(*[x if isinstance(x, C.c_void_p) else C.c_void_p(x) for x in items])
+    pointers = _POINTERS[n] if n < len(_POINTERS) else C.c_void_p * n
     return workspaces[0].lib.rk_npu_b200_w4a8_enqueue_batch_f16(
-        n, arr([w.handle for w in workspaces]), arr([w.handle for w in weights]), arr([_ptr(a) for a in dAs]),
-        arr([_ptr(c) for c in dLocals]), C.c_void_p(stream))
+        n, pointers(*[w.handle for w in workspaces]), pointers(*[w.handle for w in weights]), pointers(*[_ptr(a) for a in dAs]),
+        pointers(*[_ptr(c) for c in dLocals]), stream)
 
 
 def enqueue_ffn_f32(gate_up: Workspace, gate_up_weights: Weights, down: Workspace, down_weights: Weights, dA, dMiddle,
                     dC, stream: int = 0) -> int:
     return gate_up.lib.rk_npu_b200_w4a8_enqueue_ffn_f32(gate_up.handle, gate_up_weights.handle, down.handle,
-                                                        down_weights.handle, _ptr(dA), _ptr(dMiddle), _ptr(dC),
-                                                        C.c_void_p(stream))
+                                                        down_weights.handle, _ptr(dA), _ptr(dMiddle), _ptr(dC), stream)
 
 
 __all__ = ["Context", "Domain", "Weights", "Workspace", "W4A8Error", "default_config", "memory_query", "run_ffn_f32",
