@@ -12,6 +12,9 @@
 #include "moe_device.h"
 #include "../../include/rknpu_b200_moe.h"
 #include <algorithm>
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -25,6 +28,12 @@ using namespace rkb200;
 namespace {
 using Clock = std::chrono::steady_clock;
 double since_us(Clock::time_point t) { return std::chrono::duration<double, std::micro>(Clock::now() - t).count(); }
+// Rows up to this size are staged in page-locked memory and read from there by the intake kernel; larger ones are copied
+// from the caller's array by the driver (one token: the copy engine would cost another call and its own start, 4 + 2 us of
+// about 30; 512 KB: 40 us against 44; 2 MB: 148 against 136).
+constexpr size_t MOE_PULL_MOST = size_t(512) << 10;
+// Results up to this size are stored by the combine kernel straight into page-locked host memory.
+constexpr size_t MOE_DIRECT_MOST = size_t(512) << 10;
 constexpr int MOE_HIDDEN_MAX = 8192;   // 16 gathered rows of codes must fit one CTA's shared memory
 
 bool valid_weights(const rk_npu_moe_w8_weight_config& c)   // src/rk_npu_moe_w8.cpp:293-298
@@ -135,23 +144,39 @@ struct rk_npu_moe_w8_workspace {
     int8_t* codes = nullptr;       // [max_rows][H] codes made by the quantise kernel (run_f32)
     float* in_scales = nullptr;    // [max_rows] and their scales
     float* middle = nullptr;       // [assignments][I]
-    uint32_t* row_max = nullptr;   // [assignments]
+    uint32_t* row_max = nullptr;   // [assignments], and behind them the two projections' item counters
     float* expert_out = nullptr;   // [assignments][H]
     float* out = nullptr;          // [max_rows][H]
-    uint8_t* upload = nullptr;     // one run's host arrays in one piece (see Upload)
-    Status* status = nullptr;
+    uint8_t* upload = nullptr;     // one run's piece (see MoeRun)
     size_t codes_bytes = 0, in_scale_bytes = 0, middle_bytes = 0, row_max_bytes = 0, expert_out_bytes = 0, out_bytes = 0,
            upload_bytes = 0;
-    uint8_t* host_upload = nullptr;   // pinned mirror of `upload`
-    Status* host_status = nullptr; // pinned; the quantise kernel reports into it through its device alias
+    uint8_t* host_upload = nullptr;   // page-locked mirror of `upload`, and its device alias
+    uint8_t* host_upload_alias = nullptr;
+    uint32_t input_at = 0;            // of the input rows in it
+    // Page-locked, written by the kernels through the device alias: the verdict, then a flag for each 16 output rows.
+    Status* host_status = nullptr;
     Status* host_status_alias = nullptr;
-    float* host_out = nullptr;     // pinned landing place of small results, written by the combine kernel through its alias
-    float* host_out_alias = nullptr;
-    size_t host_out_bytes = 0;
+    unsigned* arrived = nullptr;   // [chunks] device counters behind the flags
+    size_t arrived_bytes = 0;
+    uint32_t serial = 0;           // of the last run that raised flags
+    // The launches of a run, kept as graphs: their parameters depend on the workspace, on the kind of rows, on how they
+    // arrive and on the grid's rows (a power of two, or max_rows) alone, so that any weights and routes can use them.  A
+    // graph is made at the second run of its kind: a state that runs once does not pay for it.
+    struct Kept { bool seen = false, failed = false; cudaGraphExec_t exec = nullptr; };
+    Kept kept[2][2][9];            // [fp32 rows][read from host memory][log2 of the grid's rows]
+    unsigned* tickets() const { return row_max + assignments_max; }
+    uint32_t* flags() const { return reinterpret_cast<uint32_t*>(host_status + 1); }
+    rk_npu_ctx::HostPiece host_out{};   // page-locked landing place of results
     std::vector<std::vector<int>> groups;   // per expert: token * slots + slot of its assignments
 };
 
 namespace {
+void cpu_relax()
+{
+#if defined(__x86_64__)
+    _mm_pause();
+#endif
+}
 void weights_destroy(rk_npu_moe_w8_weights* w)
 {
     if (!w) return;
@@ -183,10 +208,12 @@ void workspace_destroy(rk_npu_moe_w8_workspace* ws)
     if (ws->expert_out) device_free(d, ws->expert_out, ws->expert_out_bytes);
     if (ws->out) device_free(d, ws->out, ws->out_bytes);
     if (ws->upload) device_free(d, ws->upload, ws->upload_bytes);
-    if (ws->status) device_free(d, ws->status, sizeof(Status));
+    for (auto& a : ws->kept) for (auto& b : a) for (auto& k : b)
+        if (k.exec) cudaGraphExecDestroy(k.exec);
+    if (ws->arrived) device_free(d, ws->arrived, ws->arrived_bytes);
     if (ws->host_upload) cudaFreeHost(ws->host_upload);
     if (ws->host_status) cudaFreeHost(ws->host_status);
-    if (ws->host_out) cudaFreeHost(ws->host_out);
+    if (d) host_piece_release(d->ctx, ws->host_out);
     for (auto& e : ws->events)
         if (e) cudaEventDestroy(e);
     if (ws->stream) cudaStreamDestroy(ws->stream);
@@ -201,21 +228,35 @@ struct Lock {
     bool held;
 };
 
-// What one run sends to the device, packed into one page-locked piece so that it travels as ONE copy: the
-// schedule (jobs and assignments, grouped by expert), each token's slots, the coefficients, and the input rows
-// (int8 codes with their scales, or fp32 rows).  Offsets in bytes from the start of the piece.
-struct Upload {
-    size_t job_expert, job_first, job_rows, assign_token, slot_assign, coefficients, scales, rows_data, bytes;
-    int jobs, assignments;
-};
-size_t upload_capacity(int max_rows, int slots, int H, int experts)
+// What one run hands to the device, packed into one page-locked piece: the MoeRun header, the schedule (jobs and assignments,
+// grouped by expert), each token's slots, the coefficients, the codes' scales, where a slot bank's experts live; then, at a
+// place of its own, the input rows (int8 codes or fp32).
+uint32_t input_place(int max_rows, int slots, int experts)
 {
     const size_t A = size_t(max_rows) * slots;
-    return (4 * A + 2 * A + size_t(max_rows)) * 4 + 16 + size_t(max_rows) * H * 4 + 16 + 4 * sizeof(void*) * size_t(experts);   // + a slot bank's tables
+    return uint32_t((sizeof(MoeRun) + 16 + (4 * A + 2 * A + size_t(max_rows)) * 4 + 16 + 4 * sizeof(void*) * size_t(experts) + 15) / 16 * 16);
+}
+// The rows are read once, by the device, soon after: past the cache they come back from memory without a snoop (384 KB
+// staged and pulled: 33 us instead of 35; 512 KB: 40 instead of 46).
+void stage_rows(uint8_t* to, const void* from, size_t bytes)
+{
+#if defined(__x86_64__)
+    if (bytes >= (size_t(64) << 10)) {
+        const __m128i* src = static_cast<const __m128i*>(from);
+        __m128i* dst = reinterpret_cast<__m128i*>(to);
+        for (size_t i = 0; i < bytes / 16; i += 2) {       // rows are multiples of 32 bytes
+            _mm_stream_si128(dst + i, _mm_loadu_si128(src + i));
+            _mm_stream_si128(dst + i + 1, _mm_loadu_si128(src + i + 1));
+        }
+        _mm_sfence();
+        return;
+    }
+#endif
+    std::memcpy(to, from, bytes);
 }
 
 // Groups the assignments by expert, cuts the groups into jobs of at most 16 and writes everything into the mirror.
-Upload build_upload(rk_npu_moe_w8_workspace& ws, int rows, const void* input, bool f32, const float* scales, const int32_t* ids,
+MoeRun& build_upload(rk_npu_moe_w8_workspace& ws, const rk_npu_moe_w8_weights& w, int rows, const void* input, bool f32, const float* scales, const int32_t* ids,
                     const float* routes)
 {
     const auto& c = ws.config;
@@ -228,18 +269,39 @@ Upload build_upload(rk_npu_moe_w8_workspace& ws, int rows, const void* input, bo
         if (c.weights.shared_expert) ws.groups[R].push_back(r * S + top);
     }
     for (const auto& g : ws.groups) { assignments += int(g.size()); jobs += int((g.size() + MOE_JOB_ROWS - 1) / MOE_JOB_ROWS); }
-    Upload u{};
+    MoeRun& u = *reinterpret_cast<MoeRun*>(ws.host_upload);
+    u = MoeRun{};
+    u.rows = rows;
     u.jobs = jobs;
     u.assignments = assignments;
-    u.job_expert = 0;
-    u.job_first = u.job_expert + size_t(jobs) * 4;
-    u.job_rows = u.job_first + size_t(jobs) * 4;
-    u.assign_token = u.job_rows + size_t(jobs) * 4;
-    u.slot_assign = u.assign_token + size_t(assignments) * 4;
-    u.coefficients = u.slot_assign + size_t(rows) * S * 4;
-    u.scales = u.coefficients + size_t(rows) * S * 4;
-    u.rows_data = (u.scales + size_t(rows) * 4 + 15) / 16 * 16;
-    u.bytes = u.rows_data + size_t(rows) * H * (f32 ? 4 : 1);
+    u.f32 = f32;
+    u.job_expert = uint32_t((sizeof(MoeRun) + 15) / 16 * 16);
+    u.job_first = u.job_expert + uint32_t(jobs) * 4;
+    u.job_rows = u.job_first + uint32_t(jobs) * 4;
+    u.assign_token = u.job_rows + uint32_t(jobs) * 4;
+    u.slot_assign = u.assign_token + uint32_t(assignments) * 4;
+    u.coefficients = u.slot_assign + uint32_t(rows * S) * 4;
+    u.scales = u.coefficients + uint32_t(rows * S) * 4;
+    u.used = u.scales + uint32_t(rows) * 4;
+    u.gate_up = MoeMatrix{w.gate_up_bank(), w.gate_up_scales};
+    u.down = MoeMatrix{w.down_bank(), w.down_scales};
+    if (w.slotted) {       // where every expert lives right now travels with the run: records and scales of both projections
+        const uint32_t E = uint32_t(w.experts()), tables = (u.used + 15) / 16 * 16;
+        const void** host = reinterpret_cast<const void**>(ws.host_upload + tables);
+        for (uint32_t e = 0; e < E; ++e) {
+            host[e] = w.gate_up_at(int(e));
+            host[E + e] = w.down_at(int(e));
+            host[2 * E + e] = w.gate_up_scales_at(int(e));
+            host[3 * E + e] = w.down_scales_at(int(e));
+        }
+        const uint8_t* const at = ws.upload + tables;      // as the kernels find them
+        u.gate_up.bank.table = reinterpret_cast<const uint8_t* const*>(at);
+        u.down.bank.table = reinterpret_cast<const uint8_t* const*>(at) + E;
+        u.gate_up.bank.scale_table = reinterpret_cast<const float* const*>(at) + 2 * E;
+        u.down.bank.scale_table = reinterpret_cast<const float* const*>(at) + 3 * E;
+        u.used = tables + 4 * uint32_t(sizeof(void*)) * E;
+    }
+    u.used = (u.used + 15) / 16 * 16;
     uint8_t* base = ws.host_upload;
     int* job_expert = reinterpret_cast<int*>(base + u.job_expert), *job_first = reinterpret_cast<int*>(base + u.job_first);
     int* job_rows = reinterpret_cast<int*>(base + u.job_rows), *assign_token = reinterpret_cast<int*>(base + u.assign_token);
@@ -264,8 +326,64 @@ Upload build_upload(rk_npu_moe_w8_workspace& ws, int rows, const void* input, bo
     for (int r = 0; r < rows; ++r)
         for (int slot = 0; slot < S; ++slot) coefficients[r * S + slot] = slot < top ? routes[r * top + slot] : 1.0f;
     if (!f32) std::memcpy(base + u.scales, scales, size_t(rows) * 4);
-    std::memcpy(base + u.rows_data, input, size_t(rows) * H * (f32 ? 4 : 1));
     return u;
+}
+
+// The launches of a run in stream order; `events` (may be null) are recorded between them.
+bool launch_run(rk_npu_moe_w8_workspace& ws, bool f32, bool pull, int grid_rows, bool project, cudaEvent_t* events)
+{
+    const auto& c = ws.config;
+    const int H = c.weights.hidden, I = c.weights.intermediate, sms = ws.domain->ctx->sm_count;
+    const unsigned long long timeout_ns = (unsigned long long)c.timeout_ms * 1000000ull;
+    cudaStream_t s = ws.stream;
+    bool ok = true;
+    if (f32 || pull) ok = launch_moe_intake(MoeIntakeParams{pull ? ws.host_upload_alias : nullptr, ws.upload, ws.codes, ws.in_scales, ws.host_status_alias, ws.input_at, H, f32}, grid_rows, s) == cudaSuccess;
+    if (!project) return ok;
+    if (events) cudaEventRecord(events[1], s);
+    MoeProjectParams p{ws.upload, ws.codes, ws.in_scales, ws.middle, ws.row_max, ws.expert_out, ws.tickets(), ws.host_status_alias, ws.input_at, H, I, timeout_ns};
+    ok = ok && launch_moe_gate_up(p, sms, s) == cudaSuccess;
+    if (events) cudaEventRecord(events[2], s);
+    ok = ok && launch_moe_down(p, sms, s) == cudaSuccess;
+    if (events) cudaEventRecord(events[3], s);
+    uint32_t* const flags = reinterpret_cast<uint32_t*>(ws.host_status_alias + 1);
+    ok = ok && launch_moe_combine(MoeCombineParams{ws.upload, ws.expert_out, ws.row_max, ws.tickets(), ws.arrived, flags, ws.slots, H}, grid_rows, s) == cudaSuccess;
+    if (events) cudaEventRecord(events[4], s);
+    return ok;
+}
+
+// The same launches as one graph, from the second run of their kind on; false: not available.
+bool launch_kept(rk_npu_moe_w8_workspace& ws, bool f32, bool pull, int grid_rows, int level)
+{
+    auto& k = ws.kept[f32][pull][level];
+    if (k.failed) return false;
+    if (!k.exec) {
+        if (!k.seen) { k.seen = true; return false; }
+        cudaGraph_t graph = nullptr;
+        bool ok = cudaStreamBeginCapture(ws.stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+        if (ok) {
+            const bool launched = launch_run(ws, f32, pull, grid_rows, true, nullptr);
+            ok = cudaStreamEndCapture(ws.stream, &graph) == cudaSuccess && launched && cudaGraphInstantiate(&k.exec, graph, 0) == cudaSuccess;
+        }
+        if (graph) cudaGraphDestroy(graph);
+        if (!ok) { cudaGetLastError(); k.exec = nullptr; k.failed = true; return false; }
+    }
+    return cudaGraphLaunch(k.exec, ws.stream) == cudaSuccess;
+}
+
+// Waits until the rows of a chunk have arrived: its flag is raised by the combine kernel, whose stores precede it.  The
+// stream is asked now and then, so that a failed launch or a fault ends the wait (every wait inside the kernels is bounded).
+bool wait_chunk(rk_npu_moe_w8_workspace& ws, int chunk)
+{
+    const uint32_t* const flag = ws.flags() + chunk;
+    for (unsigned spin = 1;; ++spin) {
+        if (__atomic_load_n(flag, __ATOMIC_ACQUIRE) == ws.serial) return true;
+        if (spin % 8192 == 0) {
+            const cudaError_t e = cudaStreamQuery(ws.stream);
+            if (e == cudaSuccess) return __atomic_load_n(flag, __ATOMIC_ACQUIRE) == ws.serial;
+            if (e != cudaErrorNotReady) return false;
+        }
+        cpu_relax();
+    }
 }
 
 int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int rows, const void* input, bool f32, const float* scales,
@@ -294,50 +412,37 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
     cudaStream_t s = ws->stream;
     rk_npu_moe_w8_timings t{};
     try {
-        // ---- the routes grouped by expert, the input rows: one piece, one copy
+        // ---- the routes grouped by expert, the input rows: one piece
         auto at = Clock::now();
-        Upload u = build_upload(*ws, rows, input, f32, scales, ids, routes);
+        MoeRun& u = build_upload(*ws, *w, rows, input, f32, scales, ids, routes);
         const int assignments = u.assignments, jobs = u.jobs;
-        MoeBank gate_up_bank = w->gate_up_bank(), down_bank = w->down_bank();
-        if (w->slotted) {      // where every expert lives right now travels with the run: records and scales of both projections
-            const int E = w->experts();
-            const size_t tables = (u.bytes + 15) / 16 * 16;
-            const void** host = reinterpret_cast<const void**>(ws->host_upload + tables);
-            for (int e = 0; e < E; ++e) {
-                host[e] = w->gate_up_at(e);
-                host[E + e] = w->down_at(e);
-                host[2 * E + e] = w->gate_up_scales_at(e);
-                host[3 * E + e] = w->down_scales_at(e);
-            }
-            const uint8_t* device = ws->upload + tables;
-            gate_up_bank.table = reinterpret_cast<const uint8_t* const*>(device);
-            down_bank.table = reinterpret_cast<const uint8_t* const*>(device + sizeof(void*) * E);
-            gate_up_bank.scale_table = reinterpret_cast<const float* const*>(device + 2 * sizeof(void*) * E);
-            down_bank.scale_table = reinterpret_cast<const float* const*>(device + 3 * sizeof(void*) * E);
-            u.bytes = tables + 4 * sizeof(void*) * E;
+        // The combine kernel stores a small result straight into page-locked host memory, from where the host copies it to the
+        // caller's array; a larger one is copied by the driver.  Either once the verdict is known (a rejected call must not
+        // touch that array).
+        const bool direct = ws->host_out.alias && values * 4 <= ws->host_out.bytes;
+        u.out = direct ? static_cast<float*>(ws->host_out.alias) : ws->out;
+        if (direct && !timings) {
+            if (++ws->serial == 0) ws->serial = 1;
+            u.serial = ws->serial;
         }
+        const size_t row_bytes = values * (f32 ? 4 : 1);
+        const bool pull = row_bytes <= MOE_PULL_MOST;
+        if (pull) stage_rows(ws->host_upload + ws->input_at, input, row_bytes);
         t.schedule_us = since_us(at);
         at = Clock::now();
         if (timings) cudaEventRecord(ws->events[0], s);
+        *ws->host_status = Status{};          // the kernels' verdict lands in page-locked memory by itself
         bool ok = true;
-        if (assignments || f32) ok = cudaMemcpyAsync(ws->upload, ws->host_upload, u.bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
-        const int8_t* codes = reinterpret_cast<const int8_t*>(ws->upload + u.rows_data);
-        const float* in_scales = reinterpret_cast<const float*>(ws->upload + u.scales);
-        if (f32) {
-            // the kernel's verdict lands in page-locked memory by itself: no copy, no second wait
-            *ws->host_status = Status{};
-            const MoeQuantParams q{reinterpret_cast<const float*>(ws->upload + u.rows_data), ws->codes, ws->in_scales, ws->host_status_alias, rows, H};
-            ok = ok && launch_moe_quantize(q, s) == cudaSuccess;
-            codes = ws->codes;
-            in_scales = ws->in_scales;
-        }
-        if (!ok) { cudaGetLastError(); cudaStreamSynchronize(s); return RK_NPU_ERR_SUBMIT; }
-        t.input_us = since_us(at);
+        if (!pull && (assignments || f32))
+            ok = cudaMemcpyAsync(ws->upload, ws->host_upload, u.used, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+                 cudaMemcpyAsync(ws->upload + ws->input_at, input, row_bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
         if (!assignments) {                    // nothing routed: the output is zero and no device work is issued for it
             if (f32) {                         // (the rows are still judged)
-                if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+                ok = ok && launch_run(*ws, f32, pull, rows, false, nullptr);
+                if (cudaStreamSynchronize(s) != cudaSuccess || !ok) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
                 if (ws->host_status->bad_input) return RK_NPU_ERR_PARAM;
             }
+            t.input_us = since_us(at);
             at = Clock::now();
             std::fill_n(output, values, 0.0f);
             t.combine_us = since_us(at);
@@ -345,39 +450,33 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
             if (timings) *timings = t;
             return RK_NPU_OK;
         }
-        if (timings) cudaEventRecord(ws->events[1], s);
-        // A small result is stored by the combine kernel straight into page-locked host memory and copied to the caller's
-        // array by the host after the wait (a rejected call must not touch that array); a large one takes the copy engine.
-        const bool direct = values * 4 <= ws->host_out_bytes;
-        float* const landing = direct ? ws->host_out_alias : ws->out;
-        const MoeSchedule sched{reinterpret_cast<const int*>(ws->upload + u.job_expert), reinterpret_cast<const int*>(ws->upload + u.job_first),
-                                reinterpret_cast<const int*>(ws->upload + u.job_rows), reinterpret_cast<const int*>(ws->upload + u.assign_token), jobs};
-        const MoeGateUpParams gu{sched, gate_up_bank, w->gate_up_scales, codes, in_scales, ws->middle, ws->row_max, H, I};
-        ok = launch_moe_gate_up(gu, s) == cudaSuccess;
-        if (timings) cudaEventRecord(ws->events[2], s);
-        const MoeDownParams dn{sched, down_bank, w->down_scales, ws->middle, ws->row_max, ws->expert_out, H, I};
-        ok = ok && launch_moe_down(dn, s) == cudaSuccess;
-        if (timings) cudaEventRecord(ws->events[3], s);
-        const MoeCombineParams cb{ws->expert_out, reinterpret_cast<const int*>(ws->upload + u.slot_assign),
-                                  reinterpret_cast<const float*>(ws->upload + u.coefficients), landing, ws->row_max, rows, S, H};
-        ok = ok && launch_moe_combine(cb, s) == cudaSuccess;
-        if (timings) cudaEventRecord(ws->events[4], s);
+        int level = 0;
+        while ((1 << level) < rows) ++level;
+        const int grid_rows = std::min(1 << level, c.max_rows);
+        ok = ok && ((!timings && launch_kept(*ws, f32, pull, grid_rows, level)) || launch_run(*ws, f32, pull, grid_rows, true, timings ? ws->events : nullptr));
+        at = Clock::now();
         if (!ok) {      // a launch failed part-way: the row maxima may be left behind
             cudaGetLastError();
             cudaMemsetAsync(ws->row_max, 0, ws->row_max_bytes, s);
             cudaStreamSynchronize(s);
             return RK_NPU_ERR_SUBMIT;
         }
-        at = Clock::now();
-        if (!direct && !f32 && cudaMemcpyAsync(output, ws->out, values * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) ok = false;
-        if (!ok || cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
-        if (f32 && ws->host_status->bad_input) return RK_NPU_ERR_PARAM;      // a rejected row: the output is not written
-        if (direct) std::memcpy(output, ws->host_out, values * 4);
-        else if (f32 && (cudaMemcpyAsync(output, ws->out, values * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-                         cudaStreamSynchronize(s) != cudaSuccess)) {
-            cudaGetLastError();
+        if (u.serial) {
+            for (int r = 0; r < rows; r += MOE_CHUNK_ROWS) {
+                if (!wait_chunk(*ws, r / MOE_CHUNK_ROWS)) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+                if (ws->host_status->device_error || ws->host_status->bad_input) break;     // final before the first flag
+                const size_t first = size_t(r) * H, some = size_t(std::min(MOE_CHUNK_ROWS, rows - r)) * H;
+                std::memcpy(output + first, static_cast<const float*>(ws->host_out.ptr) + first, some * 4);
+            }
+        } else if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        if (ws->host_status->device_error) {                                  // a bounded wait ran out: the row maxima may be left behind
+            cudaMemsetAsync(ws->row_max, 0, ws->row_max_bytes, s);
+            cudaStreamSynchronize(s);
             return RK_NPU_ERR_SUBMIT;
         }
+        if (ws->host_status->bad_input) return RK_NPU_ERR_PARAM;              // a rejected row: the output is not written
+        if (!u.serial && direct) std::memcpy(output, ws->host_out.ptr, values * 4);
+        else if (!u.serial && cudaMemcpy(output, ws->out, values * 4, cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
         t.sync_us = since_us(at);
         if (timings) {
             t.input_us = event_us(ws->events[0], ws->events[1]);
@@ -540,10 +639,12 @@ rk_npu_moe_w8_workspace* workspace_create(rk_npu_iommu_domain* domain, const rk_
     ws->codes_bytes = size_t(rows) * H;
     ws->in_scale_bytes = size_t(rows) * 4;
     ws->middle_bytes = A * I * 4;
-    ws->row_max_bytes = A * 4;
+    ws->row_max_bytes = (A + 2) * 4;
+    ws->arrived_bytes = size_t((rows + MOE_CHUNK_ROWS - 1) / MOE_CHUNK_ROWS) * sizeof(unsigned);
     ws->expert_out_bytes = A * H * 4;
     ws->out_bytes = size_t(rows) * H * 4;
-    ws->upload_bytes = upload_capacity(rows, ws->slots, H, config->weights.routed_experts + config->weights.shared_expert);
+    ws->input_at = input_place(rows, ws->slots, config->weights.routed_experts + config->weights.shared_expert);
+    ws->upload_bytes = ws->input_at + size_t(rows) * H * 4;
     bool ok = true;
     try { ws->groups.resize(size_t(config->weights.routed_experts + config->weights.shared_expert)); } catch (...) { ok = false; }
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes) &&
@@ -553,16 +654,16 @@ rk_npu_moe_w8_workspace* workspace_create(rk_npu_iommu_domain* domain, const rk_
          !device_alloc(domain, reinterpret_cast<void**>(&ws->expert_out), ws->expert_out_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->out), ws->out_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->upload), ws->upload_bytes) &&
-         !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status));
+         !device_alloc(domain, reinterpret_cast<void**>(&ws->arrived), ws->arrived_bytes);
     ok = ok && cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
-         cudaMallocHost(reinterpret_cast<void**>(&ws->host_upload), ws->upload_bytes) == cudaSuccess &&
-         cudaHostAlloc(reinterpret_cast<void**>(&ws->host_status), sizeof(Status), cudaHostAllocMapped) == cudaSuccess &&
+         cudaHostAlloc(reinterpret_cast<void**>(&ws->host_upload), ws->input_at + std::min(size_t(rows) * H * 4, std::max(MOE_PULL_MOST, size_t(H) * 4)), cudaHostAllocMapped) == cudaSuccess &&
+         cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws->host_upload_alias), ws->host_upload, 0) == cudaSuccess &&
+         cudaHostAlloc(reinterpret_cast<void**>(&ws->host_status), sizeof(Status) + ws->arrived_bytes, cudaHostAllocMapped) == cudaSuccess &&
          cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws->host_status_alias), ws->host_status, 0) == cudaSuccess;
-    ws->host_out_bytes = std::min<size_t>(ws->out_bytes, size_t(256) << 10);
-    ok = ok && cudaHostAlloc(reinterpret_cast<void**>(&ws->host_out), ws->host_out_bytes, cudaHostAllocMapped) == cudaSuccess &&
-         cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws->host_out_alias), ws->host_out, 0) == cudaSuccess;
+    if (ok) ws->host_out = host_piece_acquire(ctx, std::min(ws->out_bytes, MOE_DIRECT_MOST));     // (without it results are copied directly)
     for (auto& e : ws->events) ok = ok && cudaEventCreate(&e) == cudaSuccess;
-    ok = ok && cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess &&
+    if (ok) std::memset(static_cast<void*>(ws->host_status), 0, sizeof(Status) + ws->arrived_bytes);
+    ok = ok && cudaMemsetAsync(ws->arrived, 0, ws->arrived_bytes, ws->stream) == cudaSuccess &&
          cudaMemsetAsync(ws->row_max, 0, ws->row_max_bytes, ws->stream) == cudaSuccess &&     // every run leaves them zero again
          cudaStreamSynchronize(ws->stream) == cudaSuccess;
     if (!ok) { cudaGetLastError(); workspace_destroy(ws); return nullptr; }
@@ -586,7 +687,7 @@ extern "C" uint64_t rk_npu_moe_w8_weights_device_bytes(const rk_npu_moe_w8_weigh
 extern "C" uint64_t rk_npu_moe_w8_workspace_device_bytes(const rk_npu_moe_w8_workspace* ws)
 {
     return ws ? uint64_t(ws->codes_bytes + ws->in_scale_bytes + ws->middle_bytes + ws->row_max_bytes + ws->expert_out_bytes +
-                         ws->out_bytes + ws->upload_bytes + sizeof(Status))
+                         ws->out_bytes + ws->upload_bytes + ws->arrived_bytes)
               : 0;
 }
 

@@ -1,7 +1,7 @@
 // moe_device.h -- device side of the routed-experts operator (rk_npu_moe_w8.h): parameter blocks and launchers.
 //
-// A run is a list of JOBS: up to 16 (token, slot) assignments that use the same expert.  Three launches work
-// on the list: gate/up projection + SwiGLU (fp32 middle rows and their maxima), down projection (re-quantises
+// A run is a list of JOBS: up to 16 (token, slot) assignments that use the same expert.  After the intake of the rows
+// three launches work on the list: gate/up projection + SwiGLU (fp32 middle rows and their maxima), down projection (re-quantises
 // the middle rows on the way into shared memory), and the weighted sum over each token's slots.
 #pragma once
 #include "w4a8_device.h"
@@ -52,56 +52,73 @@ struct MoePackParams {
     int nibbles;          // 1: int4 codes, two per byte
 };
 
-struct MoeQuantParams {
-    const float* X;       // [rows][H]
+// One projection's weights: the experts' records and their scales.
+struct MoeMatrix {
+    MoeBank bank;
+    const float* scales;       // [E][channels] (immutable banks)
+};
+// What one run hands to the device, in one piece, begins with this: what there is and where it lies (bytes from the start
+// of the piece).  The kernels of a run read everything that changes from call to call from here, so that their parameters,
+// and with them a kept graph of the launches, depend on the workspace alone.
+struct MoeRun {
+    int rows, jobs, assignments;
+    int f32;                   // the rows are fp32 and the intake kernel quantises them; else int8 codes
+    uint32_t job_expert;       // [jobs]
+    uint32_t job_first;        // [jobs] first assignment of the job (a job's assignments are consecutive)
+    uint32_t job_rows;         // [jobs] 1..16
+    uint32_t assign_token;     // [assignments] source row of each assignment
+    uint32_t slot_assign;      // [rows][slots] assignment index, -1: the slot takes no part
+    uint32_t coefficients;     // [rows][slots]
+    uint32_t scales;           // [rows] (int8 rows)
+    uint32_t used;             // bytes of header, schedule and tables: a multiple of 16
+    MoeMatrix gate_up, down;
+    float* out;                // [rows][H], on the device or the device alias of page-locked host memory
+    uint32_t serial;           // not 0: the combine kernel stores this number into a chunk's flag when its rows are complete
+    uint32_t pad;
+};
+constexpr int MOE_CHUNK_ROWS = 16;                                   // output rows per flag
+template <class T> __host__ __device__ inline const T* moe_piece(const uint8_t* upload, uint32_t offset) { return reinterpret_cast<const T*>(upload + offset); }
+
+struct MoeIntakeParams {
+    const uint8_t* from;  // device alias of the piece in page-locked host memory, or NULL: it has been copied to `upload` already
+    uint8_t* upload;
     int8_t* codes;        // [rows][H]
     float* scales;        // [rows]
     Status* status;       // bad_input: a non-finite element, or a scale whose reciprocal is not finite
-    int rows, H;
+    uint32_t input_at;    // where the input rows [rows][H] begin: behind all that header, schedule and tables can take
+    int H, f32;
 };
 
-struct MoeSchedule {
-    const int* job_expert;     // [jobs]
-    const int* job_first;      // [jobs] first assignment of the job
-    const int* job_rows;       // [jobs] 1..16
-    const int* assign_token;   // [assignments] source row of each assignment (assignments of a job are consecutive)
-    int jobs;
-};
-
-struct MoeGateUpParams {
-    MoeSchedule sched;
-    MoeBank bank;                // experts' gate/up matrices
-    const float* w_scales;       // [E][2I] (immutable banks; a slot bank's come from its table)
-    const int8_t* codes;         // [rows][H]
-    const float* in_scales;      // [rows]
+// One projection of every job: gate/up with SwiGLU, or down.
+struct MoeProjectParams {
+    const uint8_t* upload;
+    const int8_t* codes;         // gate/up: [rows][H] and
+    const float* in_scales;      // [rows], where the run's rows are fp32
     float* middle;               // [assignments][I]
-    uint32_t* row_max;           // [assignments] bit patterns of max |middle|, zero before the launch
+    uint32_t* row_max;           // [assignments] bit patterns of max |middle|, zero before the first launch
+    float* expert_out;           // down: [assignments][H]
+    unsigned* tickets;           // [2] items handed out by gate/up and by down; zero before the first launch
+    Status* status;              // device_error: a bounded wait ran out
+    uint32_t input_at;
     int H, I;
-};
-
-struct MoeDownParams {
-    MoeSchedule sched;
-    MoeBank bank;                // experts' down matrices
-    const float* w_scales;       // [E][H] (immutable banks)
-    const float* middle;         // [assignments][I]
-    const uint32_t* row_max;     // [assignments]
-    float* expert_out;           // [assignments][H]
-    int H, I;
+    unsigned long long timeout_ns;
 };
 
 struct MoeCombineParams {
+    const uint8_t* upload;
     const float* expert_out;     // [assignments][H]
-    const int* slot_assign;      // [rows][slots] assignment index, -1: the slot takes no part
-    const float* coefficients;   // [rows][slots]
-    float* out;                  // [rows][H]
     uint32_t* row_max;           // [assignments] cleared here for the next run
-    int rows, slots, H;
+    unsigned* tickets;           // [2] cleared here as well
+    unsigned* arrived;           // [chunks] blocks that have stored their part; zero between runs
+    uint32_t* flags;             // [chunks] in page-locked host memory
+    int slots, H;
 };
 
 cudaError_t launch_moe_pack(const MoePackParams& p, cudaStream_t stream);
-cudaError_t launch_moe_quantize(const MoeQuantParams& p, cudaStream_t stream);
-cudaError_t launch_moe_gate_up(const MoeGateUpParams& p, cudaStream_t stream);
-cudaError_t launch_moe_down(const MoeDownParams& p, cudaStream_t stream);
-cudaError_t launch_moe_combine(const MoeCombineParams& p, cudaStream_t stream);
+// max_rows: the rows a grid has to be able to cover (the run's own count is read on the device)
+cudaError_t launch_moe_intake(const MoeIntakeParams& p, int max_rows, cudaStream_t stream);
+cudaError_t launch_moe_gate_up(const MoeProjectParams& p, int sm_count, cudaStream_t stream);
+cudaError_t launch_moe_down(const MoeProjectParams& p, int sm_count, cudaStream_t stream);
+cudaError_t launch_moe_combine(const MoeCombineParams& p, int max_rows, cudaStream_t stream);
 
 } // namespace rkb200

@@ -7,92 +7,79 @@
 // register order of mma.sync.m16n8k32 so that every warp load is 512 contiguous bytes; the gathered activation
 // rows sit in shared memory; sums are exact int32.
 //
-//   moe_quantize_kernel   fp32 rows -> int8 codes + scales, nearest-even, scale = max/127 (1 for a zero row)
-//   moe_gate_up_kernel    per (job, 64 features): gate and up sums of the same feature in the same thread (two warps
-//                         per 16 features, half of K each, summed through shared memory),
-//                         (float(sum) * s_in) * s_w, y = silu(gate) * up (degree-7 polynomial shared with the dense
-//                         path), fp32 middle rows + atomicMax of |y| bit patterns per assignment
-//   moe_down_kernel       per (job, 256 columns): re-quantises the job's middle rows into shared memory with the
-//                         row scale max/127 (nearest-even), int8 GEMM over I, (float(sum) * s_mid) * s_w
+//   moe_intake_kernel     a small run's piece from page-locked host memory to the device; fp32 rows -> int8 codes + scales,
+//                         nearest-even, scale = max/127 (1 for a zero row)
+//   moe_project_kernel    gate/up: (float(sum) * s_in) * s_w, y = silu(gate) * up (degree-7 polynomial shared with the dense
+//                         path), fp32 middle rows + atomicMax of |y| bit patterns per assignment;
+//                         down: re-quantised middle rows, int8 GEMM over I, (float(sum) * s_mid) * s_w
 //   moe_combine_kernel    out[token] = sum over the token's slots, in slot order, one fused multiply-add each
 #include "moe_device.h"
 #include "w4a8_math.cuh"
 #include "w4a8_ptx.cuh"
+#include "w4a8_tc.cuh"
 #include <algorithm>
 
 namespace rkb200 {
 
 namespace {
-constexpr int MOE_FEATURE_BLOCKS = 4;    // gate/up kernel: blocks of 16 features per CTA; two warps share one, half of K each
-constexpr int MOE_WARPS = 2 * MOE_FEATURE_BLOCKS;
-constexpr int MOE_THREADS = 32 * MOE_WARPS;
-constexpr int MOE_DOWN_BLOCKS = 2;       // 16-channel blocks per warp of the down kernel (a CTA covers 256 columns)
-constexpr int MOE_ROW_PAD = 16;          // bytes between activation rows in shared memory beyond K: conflict-free fragment loads
+constexpr int MOE_WARPS = 8;                 // contraction warps of a group
+constexpr int MOE_GROUP = 32 * MOE_WARPS;    // and its threads; one more warp of the CTA streams the weights
+constexpr int MOE_STAGE_RECORDS = 16;        // 16-channel x 128-k records in a stage
+constexpr int MOE_STAGE_BYTES = MOE_STAGE_RECORDS * 2048;            // 32 KB (half of it for int4 records)
+constexpr int MOE_RING_MOST = 5;
+constexpr int MOE_TURNS = 16;                // announced items: more than the ring can hold, with the closing ones
+constexpr int MOE_PARTIAL = MOE_WARPS * 8 * 32;                      // int32 sums of an item
+constexpr int MOE_ROW_PAD = 16;              // bytes between activation rows in shared memory beyond K: conflict-free fragment loads
+constexpr size_t MOE_SMEM_MOST = 218 * 1024;     // (scales, barriers and announced items are static shared memory)
+
+__host__ __device__ constexpr int moe_row_bytes(int K) { return (K + MOE_KQ - 1) / MOE_KQ * MOE_KQ + MOE_ROW_PAD; }
+__host__ __device__ constexpr size_t moe_group_bytes(int K) { return size_t(MOE_JOB_ROWS) * moe_row_bytes(K) + 2 * MOE_PARTIAL * 4; }
+// Two groups of warps wherever two stages fit beside their rows; one for the longest rows.
+__host__ __device__ constexpr int moe_groups(int K) { return 2 * moe_group_bytes(K) + 2 * MOE_STAGE_BYTES <= MOE_SMEM_MOST ? 2 : 1; }
+__host__ __device__ constexpr int moe_ring(int K)
+{
+    const int fit = int((MOE_SMEM_MOST - moe_groups(K) * moe_group_bytes(K)) / MOE_STAGE_BYTES);
+    return fit < MOE_RING_MOST ? fit : MOE_RING_MOST;
+}
+static_assert(moe_ring(8192) >= 2, "two stages fit beside the longest rows");
 
 __device__ __forceinline__ int8_t nearest_even_code(float v)
 {
     return (int8_t)__float2int_rn(fminf(fmaxf(v, -127.f), 127.f));
 }
 
-// NB 16-channel blocks (their records at w[0..NB)) against up to 16 activation rows in shared memory:
-// c[b][half] += W_b(16 x K) * X^T.  Fragment mapping of m16n8k32 (g = lane / 4, t = lane % 4): A regs = channels g / g + 8
-// at k = 4t.. and 16 + 4t..; B regs = token g at the same k; C regs = channels g, g + 8 x tokens 2t, 2t + 1.
-// The records of 128 k are double-buffered in registers: while one is multiplied the next is on its way.
-// NIB: int4 records (two 16-byte pieces per 128 k instead of four); the sums come out times 16.
-template <bool TWO, int NB, bool NIB>
-__device__ __forceinline__ void block_mma(const uint4* const (&w)[NB], const uint8_t* xs, int row_bytes, int kq_begin, int kq_count,
-                                          int lane, int (&c)[NB][2][4])
+// `kqs` 128-k records of one 16-channel block in shared memory against up to 16 activation rows: c[half] += W(16 x k) * X^T.
+// Fragment mapping of m16n8k32 (g = lane / 4, t = lane % 4): A regs = channels g / g + 8 at k = 4t.. and 16 + 4t..; B regs
+// = token g at the same k; C regs = channels g, g + 8 x tokens 2t, 2t + 1.  NIB: int4 records (two 16-byte pieces per 128 k
+// instead of four); the sums come out times 16.
+template <bool TWO, bool NIB>
+__device__ __forceinline__ void block_mma(const uint4* w, const uint8_t* x0, int row_bytes, int kqs, int lane, int (&c)[2][4])
 {
-    constexpr int PIECES = NIB ? 2 : 4;
-    const int g = lane >> 2, t = lane & 3;
-    const uint8_t* x0 = xs + (size_t)g * row_bytes + 4 * t;
     const uint8_t* x1 = x0 + (size_t)8 * row_bytes;
-    uint4 even[NB][PIECES], odd[NB][PIECES];
-    auto fetch = [&](uint4 (&a)[NB][PIECES], int kq) {
+#pragma unroll 2
+    for (int kq = 0; kq < kqs; ++kq, w += NIB ? 64 : 128, x0 += MOE_KQ, x1 += MOE_KQ) {
+        uint4 a[NIB ? 2 : 4];
 #pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int s = 0; s < PIECES; ++s) a[b][s] = __ldg(w[b] + (size_t)(kq * PIECES + s) * 32 + lane);
-    };
-    auto multiply = [&](const uint4 (&a)[NB][PIECES], int kq) {
+        for (int s = 0; s < (NIB ? 2 : 4); ++s) a[s] = w[s * 32 + lane];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const int k = kq * MOE_KQ + s * 32;
-            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(x0 + k), b1 = *reinterpret_cast<const uint32_t*>(x0 + k + 16);
+            const uint32_t b0 = *reinterpret_cast<const uint32_t*>(x0 + s * 32), b1 = *reinterpret_cast<const uint32_t*>(x0 + s * 32 + 16);
             uint32_t d0 = 0, d1 = 0;
-            if (TWO) { d0 = *reinterpret_cast<const uint32_t*>(x1 + k); d1 = *reinterpret_cast<const uint32_t*>(x1 + k + 16); }
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                uint32_t a0, a1, a2, a3;
-                if (NIB) {
-                    const uint4 v = a[b][s >> 1];
-                    const uint32_t wx = (s & 1) ? v.z : v.x, wy = (s & 1) ? v.w : v.y;
-                    a0 = (wx << 4) & 0xF0F0F0F0u; a2 = wx & 0xF0F0F0F0u;
-                    a1 = (wy << 4) & 0xF0F0F0F0u; a3 = wy & 0xF0F0F0F0u;
-                } else {
-                    const uint4 v = a[b][NIB ? 0 : s];
-                    a0 = v.x; a1 = v.y; a2 = v.z; a3 = v.w;
-                }
-                mma_s8(c[b][0], a0, a1, a2, a3, b0, b1);
-                if (TWO) mma_s8(c[b][1], a0, a1, a2, a3, d0, d1);
+            if (TWO) { d0 = *reinterpret_cast<const uint32_t*>(x1 + s * 32); d1 = *reinterpret_cast<const uint32_t*>(x1 + s * 32 + 16); }
+            uint32_t a0, a1, a2, a3;
+            if (NIB) {
+                const uint4 v = a[s >> 1];
+                const uint32_t wx = (s & 1) ? v.z : v.x, wy = (s & 1) ? v.w : v.y;
+                a0 = (wx << 4) & 0xF0F0F0F0u; a2 = wx & 0xF0F0F0F0u;
+                a1 = (wy << 4) & 0xF0F0F0F0u; a3 = wy & 0xF0F0F0F0u;
+            } else {
+                const uint4 v = a[NIB ? 0 : s];
+                a0 = v.x; a1 = v.y; a2 = v.z; a3 = v.w;
             }
+            mma_s8(c[TWO ? 0 : s & 1], a0, a1, a2, a3, b0, b1);      // (one half of tokens: two chains of sums instead)
+            if (TWO) mma_s8(c[1], a0, a1, a2, a3, d0, d1);
         }
-    };
-    if (kq_begin >= kq_count) return;
-    fetch(even, kq_begin);
-    for (int kq = kq_begin; kq < kq_count; kq += 2) {
-        if (kq + 1 < kq_count) fetch(odd, kq + 1);
-        multiply(even, kq);
-        if (kq + 2 < kq_count) fetch(even, kq + 2);
-        if (kq + 1 < kq_count) multiply(odd, kq + 1);
     }
-}
-
-// Pulls `bytes` starting at p towards L2, one 128-byte line per lane and step (no data dependence: a hint only).
-__device__ __forceinline__ void warp_prefetch_l2(const void* p, size_t bytes, int lane)
-{
-    const char* c = reinterpret_cast<const char*>(p);
-    for (size_t off = (size_t)lane * 128; off < bytes; off += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(c + off));
 }
 } // namespace
 
@@ -134,229 +121,417 @@ __global__ void __launch_bounds__(256) moe_pack_kernel(const MoePackParams p)
     }
 }
 
-// ------------------------------------------------------------------ fp32 rows -> codes (src/rk_npu_moe_w8.cpp:317-343)
-__global__ void __launch_bounds__(128) moe_quantize_kernel(const MoeQuantParams p)
+// ------------------------------------------------------------------ intake (fp32 rows -> codes: src/rk_npu_moe_w8.cpp:317-343)
+// Blocks below row_blocks take a row each; the others carry the rest of a piece that is still in host memory (header and
+// schedule) to the device.  Nothing is asked of the header where that can be avoided: a row is requested before the header is known to name it (a piece always has room for every row
+// of the grid) and stays in registers between its maximum and its codes: one trip over the bus, not three.
+constexpr int MOE_INTAKE_THREADS = 256, MOE_INTAKE_MOVERS = 8;
+constexpr int MOE_INTAKE_BLIND = MOE_INTAKE_MOVERS * MOE_INTAKE_THREADS * 16;    // moved without asking how much of it is in use
+__global__ void __launch_bounds__(MOE_INTAKE_THREADS) moe_intake_kernel(const MoeIntakeParams p)
 {
-    __shared__ uint32_t s_max[4];
-    __shared__ int s_bad[4];
-    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float* x = p.X + (size_t)row * p.H;
-    uint32_t m = 0;
-    int bad = 0;
-    for (int i = tid; i < p.H; i += 128) {
-        const uint32_t bits = __float_as_uint(x[i]) & 0x7fffffffu;
-        bad |= bits >= 0x7f800000u;
-        m = max(m, bits);
+    __shared__ uint32_t s_max[MOE_INTAKE_THREADS / 32];
+    pdl_launch_dependents();
+    const uint8_t* const piece = p.from ? p.from : p.upload;
+    const MoeRun* const run = moe_piece<MoeRun>(piece, 0);
+    const int row_blocks = gridDim.x - (p.from ? MOE_INTAKE_MOVERS : 0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if ((int)blockIdx.x >= row_blocks) {
+        const int step = MOE_INTAKE_MOVERS * MOE_INTAKE_THREADS;
+        const uint4* const src = reinterpret_cast<const uint4*>(piece);
+        uint4* const dst = reinterpret_cast<uint4*>(p.upload);
+        const int end = (int)((p.input_at <= MOE_INTAKE_BLIND ? p.input_at : run->used) / 16);
+#pragma unroll 4
+        for (int i = ((int)blockIdx.x - row_blocks) * MOE_INTAKE_THREADS + tid; i < end; i += step) dst[i] = src[i];
+        return;
     }
+    const int row = blockIdx.x;
+    if (!p.f32) {
+        const uint4* const src = reinterpret_cast<const uint4*>(piece + p.input_at + (size_t)row * p.H);       // H is a multiple of 32
+        uint4* const dst = reinterpret_cast<uint4*>(p.upload + p.input_at + (size_t)row * p.H);
+        if (row < run->rows)
+            for (int i = tid; i < p.H / 16; i += MOE_INTAKE_THREADS) dst[i] = src[i];
+        return;
+    }
+    constexpr int MOST = 8192 / 4 / MOE_INTAKE_THREADS;
+    const float4* const x = reinterpret_cast<const float4*>(piece + p.input_at) + (size_t)row * (p.H / 4);
+    const int quads = p.H / 4;
+    float4 v[MOST];
+#pragma unroll
+    for (int k = 0; k < MOST; ++k) {
+        const int i = k * MOE_INTAKE_THREADS + tid;
+        v[k] = i < quads ? x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (row >= run->rows) return;
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < MOST; ++k)
+        m = max(m, max(max(__float_as_uint(v[k].x) & 0x7fffffffu, __float_as_uint(v[k].y) & 0x7fffffffu),
+                       max(__float_as_uint(v[k].z) & 0x7fffffffu, __float_as_uint(v[k].w) & 0x7fffffffu)));
     m = __reduce_max_sync(0xffffffffu, m);
-    bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) { s_max[warp] = m; s_bad[warp] = bad; }
+    if (lane == 0) s_max[warp] = m;
     __syncthreads();
-    m = max(max(s_max[0], s_max[1]), max(s_max[2], s_max[3]));
-    bad = s_bad[0] | s_bad[1] | s_bad[2] | s_bad[3];
+#pragma unroll
+    for (int i = 0; i < MOE_INTAKE_THREADS / 32; ++i) m = max(m, s_max[i]);
     const float scale = m ? __fdiv_rn(__uint_as_float(m), 127.f) : 1.f;
     const float inverse = __frcp_rn(scale);
-    if (bad || !(scale > 0.f) || (__float_as_uint(inverse) & 0x7fffffffu) >= 0x7f800000u) {
+    if (m >= 0x7f800000u || !(scale > 0.f) || (__float_as_uint(inverse) & 0x7fffffffu) >= 0x7f800000u) {     // an infinite or NaN element is the largest pattern
         if (tid == 0) p.status->bad_input = 1;
         return;
     }
     if (tid == 0) p.scales[row] = scale;
-    int8_t* q = p.codes + (size_t)row * p.H;
-    for (int i = tid; i < p.H; i += 128) q[i] = nearest_even_code(__fmul_rn(x[i], inverse));
-}
-
-// ------------------------------------------------------------------ gate/up + SwiGLU
-__global__ void __launch_bounds__(MOE_THREADS) moe_gate_up_kernel(const MoeGateUpParams p)
-{
-    extern __shared__ __align__(16) uint8_t xs[];
-    __shared__ float s_scale[MOE_JOB_ROWS];
-    __shared__ int s_token[MOE_JOB_ROWS];
-    __shared__ int s_partial[MOE_FEATURE_BLOCKS][16][32];
-    pdl_launch_dependents();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int job = blockIdx.y;
-    // the schedule was uploaded before any kernel of this run started; the weights never change
-    const int expert = p.sched.job_expert[job], first = p.sched.job_first[job], rows = p.sched.job_rows[job];
-    const int kq_count = (p.H + MOE_KQ - 1) / MOE_KQ;
-    const int row_bytes = kq_count * MOE_KQ + MOE_ROW_PAD;
-    const int fbi = warp % MOE_FEATURE_BLOCKS, k_half = warp / MOE_FEATURE_BLOCKS;
-    const int fb = blockIdx.x * MOE_FEATURE_BLOCKS + fbi;     // block of 16 features
-    const bool live = fb * 16 < p.I;
-    const int kq_mid = (kq_count + 1) / 2;
-    const int kq_begin = k_half ? kq_mid : 0, kq_end = k_half ? kq_count : kq_mid;
-    const uint4* base = reinterpret_cast<const uint4*>(p.bank.expert(expert));
-    const bool nib = p.bank.nibbles(expert);
-    const size_t kq_vecs = nib ? 64 : 128;            // 16-byte pieces of one block per 128 k
-    const size_t block_vecs = (size_t)kq_count * kq_vecs;
-    const uint4* const w[2] = {base + (size_t)fb * block_vecs, base + (size_t)(p.I / 16 + fb) * block_vecs};
-    if (live && kq_end > kq_begin) {
-        warp_prefetch_l2(w[0] + (size_t)kq_begin * kq_vecs, (size_t)(kq_end - kq_begin) * kq_vecs * 16, lane);
-        warp_prefetch_l2(w[1] + (size_t)kq_begin * kq_vecs, (size_t)(kq_end - kq_begin) * kq_vecs * 16, lane);
-    }
-    pdl_wait();                                       // fp32 entry: the codes and scales come from the quantise kernel
-    if (tid < MOE_JOB_ROWS) {
-        const int token = tid < rows ? p.sched.assign_token[first + tid] : -1;
-        s_token[tid] = token;
-        s_scale[tid] = token >= 0 ? p.in_scales[token] : 0.f;
-    }
-    __syncthreads();
-    // the job's activation rows, 16 bytes per thread and step; rows beyond the job and k beyond H are zero
-    {
-        const int vec_per_row = row_bytes / 16, h_vec = p.H / 16;   // H is a multiple of 32
-        for (int i = tid; i < MOE_JOB_ROWS * vec_per_row; i += MOE_THREADS) {
-            const int r = i / vec_per_row, v = i - r * vec_per_row;
-            const int token = s_token[r];
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (token >= 0 && v < h_vec) val = *(reinterpret_cast<const uint4*>(p.codes + (size_t)token * p.H) + v);
-            *reinterpret_cast<uint4*>(xs + (size_t)r * row_bytes + 16 * v) = val;
-        }
-    }
-    __syncthreads();
-    int c[2][2][4] = {};                              // [gate | up][token half][fragment]
-    if (live) {
-        if (nib) {
-            if (rows > 8) block_mma<true, 2, true>(w, xs, row_bytes, kq_begin, kq_end, lane, c);
-            else block_mma<false, 2, true>(w, xs, row_bytes, kq_begin, kq_end, lane, c);
-        } else {
-            if (rows > 8) block_mma<true, 2, false>(w, xs, row_bytes, kq_begin, kq_end, lane, c);
-            else block_mma<false, 2, false>(w, xs, row_bytes, kq_begin, kq_end, lane, c);
-        }
-    }
-    // the warp with the upper half of K hands its sums to its partner
-    if (k_half == 1) {
+    uint32_t* const q = reinterpret_cast<uint32_t*>(p.codes + (size_t)row * p.H);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) s_partial[fbi][i][lane] = c[i >> 3][(i >> 2) & 1][i & 3];
-    }
-    __syncthreads();
-    if (k_half == 1 || !live) return;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int sum = c[i >> 3][(i >> 2) & 1][i & 3] + s_partial[fbi][i][lane];
-        c[i >> 3][(i >> 2) & 1][i & 3] = nib ? sum >> 4 : sum;     // int4 records: every code entered times 16
-    }
-    const int g = lane >> 2, t = lane & 3;
-    const float* ws = p.bank.scales(expert, p.w_scales, 2 * p.I);
-    float wg[2], wu[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) { wg[h] = __ldg(ws + fb * 16 + g + 8 * h); wu[h] = __ldg(ws + p.I + fb * 16 + g + 8 * h); }
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        if (half == 1 && rows <= 8) break;
-        uint32_t mx[2] = {0u, 0u};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = half * 8 + 2 * t + (i & 1), h = i >> 1;
-            if (r < rows) {
-                const float sc = s_scale[r];
-                const float y = __fmul_rn(silu_poly(dequant(c[0][half][i], sc, wg[h])), dequant(c[1][half][i], sc, wu[h]));
-                p.middle[(size_t)(first + r) * p.I + fb * 16 + g + 8 * h] = y;
-                mx[i & 1] = max(mx[i & 1], __float_as_uint(y) & 0x7fffffffu);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            uint32_t m = mx[e];
-            m = max(m, __shfl_xor_sync(0xffffffffu, m, 4));
-            m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
-            m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-            const int r = half * 8 + 2 * t + e;
-            if (g == 0 && r < rows && m) atomicMax(&p.row_max[first + r], m);
-        }
+    for (int k = 0; k < MOST; ++k) {
+        const int i = k * MOE_INTAKE_THREADS + tid;
+        if (i < quads)
+            q[i] = (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v[k].x, inverse)) | (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v[k].y, inverse)) << 8 |
+                   (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v[k].z, inverse)) << 16 | (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v[k].w, inverse)) << 24;
     }
 }
 
-// ------------------------------------------------------------------ down projection
-__global__ void __launch_bounds__(MOE_THREADS) moe_down_kernel(const MoeDownParams p)
+// ------------------------------------------------------------------ the two projections
+// Byte work: every expert's weights cross HBM once per job of up to 16 assignments.  The work is a flat list of items for one
+// persistent CTA per SM: a job and two 16-channel gate blocks with their two up blocks, or a job and eight 16-column blocks of
+// the down projection.  One warp streams the items' records and scales through a ring of 32 KB stages with bulk copies, ahead
+// of the contraction, so that 64 to 160 KB per SM are on their way whatever the other warps do.  Two groups of eight warps
+// take the items in turn, each with activation rows of its own, so that one finishes or gathers while the other contracts
+// (one group alone cannot keep up with the memory).  Down: a warp has a block and all of K (at most 512), and its sums never
+// leave its registers.  Gate/up: a warp has a block and half of each stage's K; the sums of an item meet in shared memory.
+// A job's activation rows are brought into shared memory when a group's job changes: the int8 codes, or, for the down
+// projection, the middle rows re-quantised with their row scale max/127 (nearest-even; src/rk_npu_moe_cpu.cpp:78-80).
+// SMs do not get equal shares of the memory: with the list cut evenly the first CTA was done after 26 us and the last after
+// 38.  So a CTA owns a contiguous share of three quarters of a long list and takes the rest from a common counter, item by
+// item; a list of fewer than eight items per CTA is cut evenly (a turn at the counter costs a microsecond).
+// 64 rows over 128 + 1 int8 experts of 1536 x 512, 305 MB of weights, with an event on either side of each launch: gate/up
+// 53 -> 43 us, down 39 -> 33 us (before: a CTA per item with register double buffering, a quarter as much in flight, and a
+// CTA's start and its gather paid per item).  The whole call 190 -> 150 us, one token over int4 experts 36 -> 29 us, of which
+// the launch takes 11 us, and the trips over the bus at either end 16 + 20 us at 64 rows.
+template <bool DOWN>
+__global__ void __launch_bounds__(2 * MOE_GROUP + 32, 1) moe_project_kernel(const MoeProjectParams p)
 {
-    extern __shared__ __align__(16) uint8_t xs[];
-    __shared__ float s_scale[MOE_JOB_ROWS], s_inverse[MOE_JOB_ROWS];
+    extern __shared__ __align__(128) uint8_t smem[];
+    // A stage's full barrier belongs to the group that reads it: a group waits on a parity only after it has seen the phase
+    // before (copies land out of order, and a slot's last stage may be the other group's and still on its way).
+    __shared__ __align__(8) uint64_t full[2][MOE_RING_MOST], empty[MOE_RING_MOST], told[MOE_TURNS];
+    __shared__ int4 s_turn[MOE_TURNS];                                     // item (-1: no more), first assignment, rows, int4 records
+    __shared__ __align__(16) float s_w[MOE_TURNS][(DOWN ? 8 : 4) * 16];        // and the scales of its channels
+    __shared__ float s_scales[2][MOE_JOB_ROWS];
+    const int K = DOWN ? p.I : p.H;
+    const int kq_count = (K + MOE_KQ - 1) / MOE_KQ, row_bytes = moe_row_bytes(K);
+    const int R = moe_ring(K), groups = moe_groups(K);
+    constexpr int BLOCKS = DOWN ? 8 : 4, STAGE_KQ = MOE_STAGE_RECORDS / BLOCKS;    // of a stage: its blocks, and 128-k records of each
+    constexpr int PER_ITEM = DOWN ? BLOCKS : BLOCKS / 2, BLOCK_STAGE = STAGE_KQ * 2048;
+    const int stages = (kq_count + STAGE_KQ - 1) / STAGE_KQ;               // of an item
+    uint8_t* const ring = smem;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < R; ++i) { mbar_init(&full[0][i], 1); mbar_init(&full[1][i], 1); mbar_init(&empty[i], MOE_WARPS); }
+        for (int i = 0; i < MOE_TURNS; ++i) mbar_init(&told[i], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+    // The schedule is the intake's work: gate/up waits for it before it lets the down projection's CTAs in, which can then
+    // read the schedule and request weights (these never change) while gate/up still runs.
+    if (!DOWN) pdl_wait();
     pdl_launch_dependents();
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int job = blockIdx.y;
-    const int expert = p.sched.job_expert[job], first = p.sched.job_first[job], rows = p.sched.job_rows[job];
-    const int kq_count = (p.I + MOE_KQ - 1) / MOE_KQ;
-    const int row_bytes = kq_count * MOE_KQ + MOE_ROW_PAD;
-    const uint4* base = reinterpret_cast<const uint4*>(p.bank.expert(expert));
-    const bool nib = p.bank.nibbles(expert);
-    const size_t block_vecs = (size_t)kq_count * (nib ? 64 : 128);
-    const int cb0 = (blockIdx.x * MOE_WARPS + warp) * MOE_DOWN_BLOCKS;
-    {   // this warp's weights on their way to L2 while the gate/up launch still runs
-        const int blocks = min(MOE_DOWN_BLOCKS, p.H / 16 - cb0);
-        if (blocks > 0) warp_prefetch_l2(base + (size_t)cb0 * block_vecs, (size_t)blocks * block_vecs * 16, lane);
-    }
-    pdl_wait();                                       // the middle rows and their maxima come from the launch in front
-    if (tid < MOE_JOB_ROWS) {
-        // src/rk_npu_moe_cpu.cpp:78-80: scale = max/127, 1 for an all-zero row; inverse = 1/scale
-        const uint32_t m = tid < rows ? p.row_max[first + tid] : 0u;
-        const float scale = m ? __fdiv_rn(__uint_as_float(m), 127.f) : 1.f;
-        s_scale[tid] = scale;
-        s_inverse[tid] = __frcp_rn(scale);
-    }
-    __syncthreads();
-    {
-        const int words_per_row = row_bytes / 4;
-        for (int i = tid; i < MOE_JOB_ROWS * words_per_row; i += MOE_THREADS) {
-            const int r = i / words_per_row, w = i - r * words_per_row;
-            uint32_t packed = 0;
-            if (r < rows && 4 * w < p.I) {       // I is a multiple of 32
-                const float4 v = *reinterpret_cast<const float4*>(p.middle + (size_t)(first + r) * p.I + 4 * w);
-                const float inv = s_inverse[r];
-                packed = (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.x, inv)) | (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.y, inv)) << 8 |
-                         (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.z, inv)) << 16 | (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.w, inv)) << 24;
+    const MoeRun* const run = moe_piece<MoeRun>(p.upload, 0);
+    const int* const job_expert = moe_piece<int>(p.upload, run->job_expert), *const job_first = moe_piece<int>(p.upload, run->job_first);
+    const int* const job_rows = moe_piece<int>(p.upload, run->job_rows);
+    const MoeBank bank = DOWN ? run->down.bank : run->gate_up.bank;
+    const float* const all_scales = DOWN ? run->down.scales : run->gate_up.scales;
+    const int blocks = DOWN ? p.H / 16 : p.I / 16;                       // 16-channel blocks to cover per job (gate blocks)
+    const int per_job = (blocks + PER_ITEM - 1) / PER_ITEM;
+    const int total = run->jobs * per_job;
+
+    if (tid >= groups * MOE_GROUP) {
+        // ---------------------------------------------------------------- the copy warp
+        const int owned = total >= 8 * (int)gridDim.x ? total - total / 4 : total;
+        int item = (int)((long long)owned * blockIdx.x / gridDim.x), last = (int)((long long)owned * (blockIdx.x + 1) / gridDim.x);
+        int slot = 0, issued = 0, turn = 0;
+        uint32_t phase = 0;
+        unsigned long long deadline = 0;
+        int job = -1, first = 0, rows = 0;
+        bool nib = false, failed = false;
+        const uint8_t* base = nullptr;
+        const float* ws = nullptr;
+        uint32_t armed[2] = {}, used[2] = {};                            // per group: the phase each slot is armed in, and whether it ever was
+        size_t block_bytes = 0;
+        for (;;) {
+            if (item == last) {
+                if (owned == total) break;
+                if (lane == 0) item = owned + (int)atomicAdd(p.tickets + DOWN, 1u);
+                item = __shfl_sync(0xffffffffu, item, 0);
+                if (item >= total) break;
+                last = item + 1;
             }
-            *reinterpret_cast<uint32_t*>(xs + (size_t)r * row_bytes + 4 * w) = packed;
+            if (item / per_job != job) {
+                job = item / per_job;
+                const int expert = job_expert[job];
+                first = job_first[job];
+                rows = job_rows[job];
+                base = bank.expert(expert);
+                nib = bank.nibbles(expert);
+                ws = bank.scales(expert, all_scales, DOWN ? p.H : 2 * p.I);
+                block_bytes = (size_t)kq_count * (nib ? 1024 : 2048);
+            }
+            const int b0 = (item - job * per_job) * PER_ITEM, live = min(PER_ITEM, blocks - b0);
+            for (int kq = 0; kq < kq_count; kq += STAGE_KQ, ++issued) {
+                const uint32_t bytes = (uint32_t)min(STAGE_KQ, kq_count - kq) * (nib ? 1024u : 2048u);
+                if (issued >= R) {
+                    if (deadline == 0) { if (DOWN) pdl_wait(); deadline = global_ns() + p.timeout_ns; }   // slots come back once the activations exist
+                    if (!__all_sync(0xffffffffu, mbar_wait(&empty[slot], phase ^ 1u, deadline))) {
+                        if (lane == 0) *reinterpret_cast<volatile int*>(&p.status->device_error) = 1;
+                        failed = true;
+                        break;
+                    }
+                }
+                uint8_t* const dst = ring + (size_t)slot * MOE_STAGE_BYTES;
+                const uint8_t* const src = base + (size_t)b0 * block_bytes + (size_t)kq * (nib ? 1024 : 2048);
+                const int reader = turn % groups, entry = turn % MOE_TURNS;
+                uint64_t* const bar = &full[reader][slot];
+                if (used[reader] >> slot & 1u) armed[reader] ^= 1u << slot;
+                used[reader] |= 1u << slot;
+                if (elect_one()) {
+                    const uint32_t scale_bytes = kq == 0 ? (uint32_t)live * 64u : 0u;
+                    mbar_arrive_expect_tx(bar, (bytes * (uint32_t)live + scale_bytes) * (DOWN ? 1u : 2u));
+                    if (kq == 0) {       // (an entry is used again 16 turns later: its readers have freed a later stage since)
+                        s_turn[entry] = make_int4(item, first, rows, nib);
+                        mbar_arrive(&told[entry]);
+                        bulk_g2s(s_w[entry], ws + b0 * 16, scale_bytes, bar);
+                        if (!DOWN) bulk_g2s(s_w[entry] + PER_ITEM * 16, ws + p.I + b0 * 16, scale_bytes, bar);
+                    }
+                    for (int b = 0; b < live; ++b) bulk_g2s(dst + b * BLOCK_STAGE, src + (size_t)b * block_bytes, bytes, bar);
+                    if (!DOWN)
+                        for (int b = 0; b < live; ++b)
+                            bulk_g2s(dst + (PER_ITEM + b) * BLOCK_STAGE, src + (size_t)(blocks + b) * block_bytes, bytes, bar);
+                }
+                __syncwarp();
+                if (++slot == R) { slot = 0; phase ^= 1u; }
+            }
+            if (failed) break;
+            ++item;
+            ++turn;
         }
+        if (!failed && elect_one())
+            for (int i = 0; i < groups; ++i, ++turn) {                   // no more
+                s_turn[turn % MOE_TURNS] = make_int4(-1, 0, 0, 0);
+                mbar_arrive(&told[turn % MOE_TURNS]);
+            }
+        __syncwarp();
+        // the CTA stays until its copies have landed, whoever still waits for them
+        if (deadline == 0 || failed) deadline = global_ns() + p.timeout_ns;
+        for (int g = 0; g < groups; ++g)
+            for (int i = 0; i < R; ++i)
+                if (used[g] >> i & 1u) mbar_wait(&full[g][i], armed[g] >> i & 1u, deadline);
+        return;
     }
-    __syncthreads();
-    const float* ws = p.bank.scales(expert, p.w_scales, p.H);
+
+    // ------------------------------------------------------------------ contraction warps
+    const int group = tid / MOE_GROUP, gtid = tid - group * MOE_GROUP, warp = gtid >> 5;
+    uint8_t* const xs = ring + (size_t)R * MOE_STAGE_BYTES + (size_t)group * moe_group_bytes(K);
+    int* const partials = reinterpret_cast<int*>(xs + (size_t)MOE_JOB_ROWS * row_bytes);      // two buffers
+    float* const s_scale = s_scales[group];
+    const int8_t* const codes = run->f32 ? p.codes : moe_piece<int8_t>(p.upload, p.input_at);
+    const float* const in_scales = run->f32 ? p.in_scales : moe_piece<float>(p.upload, run->scales);
+    const int* const assign_token = moe_piece<int>(p.upload, run->assign_token);
     const int g = lane >> 2, t = lane & 3;
-#pragma unroll 1
-    for (int b = 0; b < MOE_DOWN_BLOCKS; ++b) {
-        const int cb = cb0 + b;
-        if (cb * 16 >= p.H) break;
-        int c[1][2][4] = {};
-        const uint4* const w[1] = {base + (size_t)cb * block_vecs};
-        if (nib) {
-            if (rows > 8) block_mma<true, 1, true>(w, xs, row_bytes, 0, kq_count, lane, c);
-            else block_mma<false, 1, true>(w, xs, row_bytes, 0, kq_count, lane, c);
-        } else {
-            if (rows > 8) block_mma<true, 1, false>(w, xs, row_bytes, 0, kq_count, lane, c);
-            else block_mma<false, 1, false>(w, xs, row_bytes, 0, kq_count, lane, c);
+    const int block = DOWN ? warp : warp & 3, k_half = DOWN ? 0 : warp >> 2;
+    const uint8_t* const x0 = xs + (size_t)g * row_bytes + 4 * t;
+    unsigned long long deadline = 0;
+    bool waited = !DOWN;
+    auto wait = [&](uint64_t* bar, uint32_t parity) {        // false: it ran out
+        if (mbar_test(bar, parity)) return true;
+        if (deadline == 0) deadline = global_ns() + p.timeout_ns;
+        if (mbar_wait(bar, parity, deadline)) return true;
+        *reinterpret_cast<volatile int*>(&p.status->device_error) = 1;
+        return false;
+    };
+    // The group's eight warps meet; true: one of them could not wait any longer, and all of them leave (a warp that gives up
+    // takes part in one more meeting, whichever the others come to next, so that none is left waiting for it).
+    auto meet = [&](bool failed) {
+        uint32_t any;
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %3, 0;\n\tbarrier.cta.red.or.pred p, %1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(any) : "r"(1 + group), "n"(MOE_GROUP), "r"((uint32_t)failed) : "memory");
+        return any != 0;
+    };
+    int job = -1;
+    uint32_t phases = 0;                                     // of the group's full barriers, one bit per slot
+    for (int turn = group;; turn += groups) {
+        const bool knows = __all_sync(0xffffffffu, wait(&told[turn % MOE_TURNS], (uint32_t)(turn / MOE_TURNS) & 1u));
+        const int4 told_item = s_turn[turn % MOE_TURNS];
+        const int item = told_item.x, first = told_item.y, rows = told_item.z;
+        const bool nib = told_item.w;
+        if (!knows || item < 0) {
+            meet(!knows);
+            break;
         }
-        const int shift = nib ? 4 : 0;
-        const float w0 = __ldg(ws + cb * 16 + g), w1 = __ldg(ws + cb * 16 + g + 8);
+        if (item / per_job != job) {
+            job = item / per_job;
+            if (!waited) { pdl_wait(); waited = true; }      // middle rows and their maxima come from the gate/up launch
+            if (meet(false)) break;                          // the rows of the job before are no longer read
+            // rows beyond the job are not read (their columns of the sums are not used); k beyond K meets zero weights
+            const int live_rows = rows > 8 ? 16 : 8;
+            auto row_scale = [&](int r) {
+                const uint32_t m = __ldcg(p.row_max + first + r);
+                return m ? __fdiv_rn(__uint_as_float(m), 127.f) : 1.f;
+            };
+            if (gtid < MOE_JOB_ROWS) s_scale[gtid] = gtid >= rows ? 0.f : DOWN ? row_scale(gtid) : in_scales[assign_token[first + gtid]];
+            if (DOWN) {
+                const int quads = p.I / 4;                   // I is a multiple of 32
+#pragma unroll 4
+                for (int i = gtid; i < live_rows * quads; i += MOE_GROUP) {
+                    const int r = i / quads, w = i - r * quads;
+                    uint32_t packed = 0;
+                    if (r < rows) {
+                        const float4 v = __ldcg(reinterpret_cast<const float4*>(p.middle + (size_t)(first + r) * p.I + 4 * w));
+                        const float inv = __frcp_rn(row_scale(r));
+                        packed = (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.x, inv)) | (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.y, inv)) << 8 |
+                                 (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.z, inv)) << 16 | (uint32_t)(uint8_t)nearest_even_code(__fmul_rn(v.w, inv)) << 24;
+                    }
+                    *reinterpret_cast<uint32_t*>(xs + (size_t)r * row_bytes + 4 * w) = packed;
+                }
+            } else {
+                const int vecs = p.H / 16;                   // H is a multiple of 32
+#pragma unroll 4
+                for (int i = gtid; i < live_rows * vecs; i += MOE_GROUP) {
+                    const int r = i / vecs, v = i - r * vecs;
+                    uint4 val = make_uint4(0u, 0u, 0u, 0u);
+                    if (r < rows) val = *(reinterpret_cast<const uint4*>(codes + (size_t)assign_token[first + r] * p.H) + v);
+                    *reinterpret_cast<uint4*>(xs + (size_t)r * row_bytes + 16 * v) = val;
+                }
+            }
+            if (meet(false)) break;
+        }
+        const int b0 = (item - job * per_job) * PER_ITEM, live = min(PER_ITEM, blocks - b0);
+        const bool mine = DOWN ? block < live : (block & 1) < live;      // this warp's block exists
+        int c[2][4] = {};
+        int slot = turn * stages % R;
+        bool failed = false;
+        for (int kq = 0; kq < kq_count; kq += STAGE_KQ) {
+            const int n = min(STAGE_KQ, kq_count - kq), lead = DOWN ? n : (n + 1) / 2;
+            if (!__all_sync(0xffffffffu, wait(&full[group][slot], phases >> slot & 1u))) failed = true;
+            const int from = k_half ? lead : 0, count = k_half ? n - lead : lead;
+            if (mine && count > 0) {
+                const uint4* const w = reinterpret_cast<const uint4*>(ring + (size_t)slot * MOE_STAGE_BYTES + block * BLOCK_STAGE) + from * (nib ? 64 : 128);
+                const uint8_t* const x = x0 + (kq + from) * MOE_KQ;
+                if (nib) {
+                    if (rows > 8) block_mma<true, true>(w, x, row_bytes, count, lane, c);
+                    else block_mma<false, true>(w, x, row_bytes, count, lane, c);
+                } else {
+                    if (rows > 8) block_mma<true, false>(w, x, row_bytes, count, lane, c);
+                    else block_mma<false, false>(w, x, row_bytes, count, lane, c);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[slot]);
+            phases ^= 1u << slot;
+            if (++slot == R) slot = 0;
+        }
+        if (rows <= 8) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            if (half == 1 && rows <= 8) break;
+            for (int i = 0; i < 4; ++i) c[0][i] += c[1][i];
+        }
+        const int shift = nib ? 4 : 0;                       // int4 records: every code entered times 16
+        const float* const scales = s_w[turn % MOE_TURNS];
+        if (DOWN) {
+            if (failed) { meet(true); break; }
+            if (!mine) continue;
+            const int column = (b0 + block) * 16 + g;
+            const float w0 = scales[block * 16 + g], w1 = scales[block * 16 + g + 8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = half * 8 + 2 * t + (i & 1), h = i >> 1;
-                if (r < rows) p.expert_out[(size_t)(first + r) * p.H + cb * 16 + g + 8 * h] = dequant(c[0][half][i] >> shift, s_scale[r], h ? w1 : w0);
+            for (int i = 0; i < 8; ++i) {
+                const int r = (i >> 2) * 8 + 2 * t + (i & 1);
+                if (r < rows) p.expert_out[(size_t)(first + r) * p.H + column + (i & 2 ? 8 : 0)] = dequant(c[i >> 2][i & 3] >> shift, s_scale[r], i & 2 ? w1 : w0);
+            }
+        } else {
+            // the halves of K meet in shared memory; a warp finishes feature block fbi, features g + 8 h, tokens 8 half ..
+            int* const partial = partials + (turn / groups & 1) * MOE_PARTIAL;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) partial[(warp * 8 + i) * 32 + lane] = c[i >> 2][i & 3];
+            if (meet(failed)) break;
+            const int half = (warp >> 1) & 1, fbi = warp & 1, h = warp >> 2;
+            if (fbi >= live || (half == 1 && rows <= 8)) continue;
+            const int feature = (b0 + fbi) * 16 + g + 8 * h;
+            const float w0 = scales[fbi * 16 + g + 8 * h], w1 = scales[(PER_ITEM + fbi) * 16 + g + 8 * h];
+            auto sum = [&](int b, int i) { return (partial[(b * 8 + i) * 32 + lane] + partial[((b + 4) * 8 + i) * 32 + lane]) >> shift; };
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = half * 8 + 2 * t + e;
+                uint32_t m = 0;
+                if (r < rows) {
+                    const int i = half * 4 + 2 * h + e;
+                    const float sc = s_scale[r];
+                    const float y = __fmul_rn(silu_poly(dequant(sum(fbi, i), sc, w0)), dequant(sum(2 + fbi, i), sc, w1));
+                    p.middle[(size_t)(first + r) * p.I + feature] = y;
+                    m = __float_as_uint(y) & 0x7fffffffu;
+                }
+                m = max(m, __shfl_xor_sync(0xffffffffu, m, 4));
+                m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
+                m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+                if (g == 0 && r < rows && m) atomicMax(&p.row_max[first + r], m);
             }
         }
     }
+    if (!waited) pdl_wait();        // (the next kernel relies on this one to have waited)
 }
 
 // ------------------------------------------------------------------ weighted sum over a token's slots (src/rk_npu_moe_w8.cpp:786-816)
-__global__ void __launch_bounds__(256) moe_combine_kernel(const MoeCombineParams p)
+// Four columns per thread.  Where the result goes to host memory, the last block of every 16 rows to have stored its part
+// raises these rows' flag, and the host carries them on while later rows still cross the bus.
+constexpr int MOE_COMBINE_THREADS = 128;
+__global__ void __launch_bounds__(MOE_COMBINE_THREADS) moe_combine_kernel(const MoeCombineParams p)
 {
-    pdl_launch_dependents();
-    const int token = blockIdx.y;
-    const int n = blockIdx.x * 256 + threadIdx.x;
+    const MoeRun* const run = moe_piece<MoeRun>(p.upload, 0);
+    const int token = blockIdx.y, rows = run->rows;
+    const int n = (blockIdx.x * MOE_COMBINE_THREADS + threadIdx.x) * 4;
+    if (token >= rows) return;
+    const int* const assign = moe_piece<int>(p.upload, run->slot_assign) + token * p.slots;
+    const float* const coefficients = moe_piece<float>(p.upload, run->coefficients) + token * p.slots;
+    constexpr int MOST = 9;                           // top-8 and the shared expert
+    int at[MOST];
+    float c[MOST];
+#pragma unroll
+    for (int slot = 0; slot < MOST; ++slot) {
+        at[slot] = slot < p.slots ? assign[slot] : -1;
+        c[slot] = slot < p.slots ? coefficients[slot] : 0.f;
+    }
+    float* const out = run->out;
+    const uint32_t serial = run->serial;
     pdl_wait();
     // the row maxima have been consumed by the down projection: leave them zero for the next run
     if (blockIdx.x == 0 && threadIdx.x < p.slots) {
-        const int a = p.slot_assign[token * p.slots + threadIdx.x];
+        const int a = assign[threadIdx.x];
         if (a >= 0) p.row_max[a] = 0u;
     }
-    if (n >= p.H) return;
-    float sum = 0.f;
-    for (int slot = 0; slot < p.slots; ++slot) {
-        const int a = p.slot_assign[token * p.slots + slot];
-        if (a < 0) continue;
-        sum = __fmaf_rn(p.expert_out[(size_t)a * p.H + n], p.coefficients[token * p.slots + slot], sum);
+    if (blockIdx.x == 0 && token == 0 && threadIdx.x < 2) p.tickets[threadIdx.x] = 0u;
+    if (n < p.H) {
+        float4 v[MOST];
+#pragma unroll
+        for (int slot = 0; slot < MOST; ++slot)
+            v[slot] = at[slot] >= 0 ? *reinterpret_cast<const float4*>(p.expert_out + (size_t)at[slot] * p.H + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int slot = 0; slot < MOST; ++slot)
+            if (at[slot] >= 0) {                          // slot order, one fused multiply-add each
+                sum.x = __fmaf_rn(v[slot].x, c[slot], sum.x);
+                sum.y = __fmaf_rn(v[slot].y, c[slot], sum.y);
+                sum.z = __fmaf_rn(v[slot].z, c[slot], sum.z);
+                sum.w = __fmaf_rn(v[slot].w, c[slot], sum.w);
+            }
+        *reinterpret_cast<float4*>(out + (size_t)token * p.H + n) = sum;
     }
-    p.out[(size_t)token * p.H + n] = sum;
+    if (!serial) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const int chunk = token / MOE_CHUNK_ROWS;
+        const unsigned all = gridDim.x * (unsigned)min(MOE_CHUNK_ROWS, rows - chunk * MOE_CHUNK_ROWS);
+        __threadfence_system();                       // the block's rows are in host memory: the one trip over the bus that is waited for
+        if (atomicAdd(&p.arrived[chunk], 1u) + 1 == all) {
+            p.arrived[chunk] = 0u;
+            __threadfence();
+            *reinterpret_cast<volatile uint32_t*>(&p.flags[chunk]) = serial;
+        }
+    }
 }
 
 // ------------------------------------------------------------------ launchers
@@ -366,26 +541,6 @@ cudaError_t launch_moe_pack(const MoePackParams& p, cudaStream_t stream)
     const unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, 148 * 8);
     moe_pack_kernel<<<blocks, 256, 0, stream>>>(p);
     return cudaGetLastError();
-}
-
-cudaError_t launch_moe_quantize(const MoeQuantParams& p, cudaStream_t stream)
-{
-    moe_quantize_kernel<<<p.rows, 128, 0, stream>>>(p);
-    return cudaGetLastError();
-}
-
-static cudaError_t allow_shared(const void* kernel, size_t bytes, PerDeviceOnce& once, size_t& allowed)
-{
-    int device = -1;
-    const bool setup = once.needed(device);
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    if (setup || bytes > allowed) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return e;
-        allowed = 200 * 1024;
-        once.mark(device);
-    }
-    return bytes <= 200 * 1024 ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // one launch that may start while the kernel in front of it on the stream still runs (each kernel above waits
@@ -406,28 +561,32 @@ static cudaError_t launch_dependent(void (*kernel)(const Params), dim3 grid, uns
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-cudaError_t launch_moe_gate_up(const MoeGateUpParams& p, cudaStream_t stream)
+cudaError_t launch_moe_intake(const MoeIntakeParams& p, int max_rows, cudaStream_t stream)
+{
+    moe_intake_kernel<<<unsigned(max_rows + (p.from ? MOE_INTAKE_MOVERS : 0)), MOE_INTAKE_THREADS, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
+template <bool DOWN>
+static cudaError_t launch_project(const MoeProjectParams& p, int sm_count, cudaStream_t stream)
 {
     static PerDeviceOnce once;
-    static size_t allowed = 0;
-    const size_t smem = size_t(MOE_JOB_ROWS) * ((p.H + MOE_KQ - 1) / MOE_KQ * MOE_KQ + MOE_ROW_PAD);
-    if (const cudaError_t e = allow_shared(reinterpret_cast<const void*>(moe_gate_up_kernel), smem, once, allowed)) return e;
-    const dim3 grid((p.I / 16 + MOE_FEATURE_BLOCKS - 1) / MOE_FEATURE_BLOCKS, p.sched.jobs);
-    return launch_dependent(moe_gate_up_kernel, grid, MOE_THREADS, smem, stream, p);
+    int device = -1;
+    if (once.needed(device)) {
+        const cudaError_t e = cudaFuncSetAttribute(moe_project_kernel<DOWN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(MOE_SMEM_MOST));
+        if (e != cudaSuccess) return e;
+        once.mark(device);
+    }
+    const int K = DOWN ? p.I : p.H, groups = moe_groups(K);
+    return launch_dependent(moe_project_kernel<DOWN>, dim3(unsigned(sm_count)), unsigned(groups * MOE_GROUP + 32),
+                            groups * moe_group_bytes(K) + size_t(moe_ring(K)) * MOE_STAGE_BYTES, stream, p);
 }
+cudaError_t launch_moe_gate_up(const MoeProjectParams& p, int sm_count, cudaStream_t stream) { return launch_project<false>(p, sm_count, stream); }
+cudaError_t launch_moe_down(const MoeProjectParams& p, int sm_count, cudaStream_t stream) { return launch_project<true>(p, sm_count, stream); }
 
-cudaError_t launch_moe_down(const MoeDownParams& p, cudaStream_t stream)
+cudaError_t launch_moe_combine(const MoeCombineParams& p, int max_rows, cudaStream_t stream)
 {
-    const size_t smem = size_t(MOE_JOB_ROWS) * ((p.I + MOE_KQ - 1) / MOE_KQ * MOE_KQ + MOE_ROW_PAD);   // I <= 512: 8.4 KB
-    const int per_cta = 16 * MOE_WARPS * MOE_DOWN_BLOCKS;
-    const dim3 grid((p.H + per_cta - 1) / per_cta, p.sched.jobs);
-    return launch_dependent(moe_down_kernel, grid, MOE_THREADS, smem, stream, p);
-}
-
-cudaError_t launch_moe_combine(const MoeCombineParams& p, cudaStream_t stream)
-{
-    const dim3 grid((p.H + 255) / 256, p.rows);
-    return launch_dependent(moe_combine_kernel, grid, 256, 0, stream, p);
+    return launch_dependent(moe_combine_kernel, dim3(unsigned((p.H / 4 + MOE_COMBINE_THREADS - 1) / MOE_COMBINE_THREADS), unsigned(max_rows)), MOE_COMBINE_THREADS, 0, stream, p);
 }
 
 } // namespace rkb200
