@@ -11,6 +11,7 @@
 #include "w4a8_host.h"
 #include "w4a8_ptx.cuh"
 #include "w4a8_math.cuh"
+#include "w4a8_quantize.cuh"
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <float.h>
@@ -61,13 +62,79 @@ cudaError_t launch_pack_weights(const PackParams& p, cudaStream_t stream)
 }
 
 // =============================================================== activation quantisation
-// One CTA per token.  Pass 1: max |x| over the full row on the raw bit patterns (for
-// binary16 and fp32 alike the magnitude bits order like the magnitudes, and anything
-// at or above the infinity pattern is NaN/Inf).  Pass 2: q = clamp(round_half_away(
-// x * inverse), -127, 127), written as 16-byte units of the Xq layout.
-template <bool HALF, int BS>
-__global__ void __launch_bounds__(BS, 2048 / BS) quantize_kernel(const QuantParams p)
+// Pass 1: max |x| over the full row on the raw bit patterns (for binary16 and fp32 alike the
+// magnitude bits order like the magnitudes, and anything at or above the infinity pattern is
+// NaN/Inf).  Pass 2: q = clamp(round_half_away(x * inverse), -127, 127), written as 16-byte units of
+// the Xq layout.  Rows that allow 16-byte loads: quantize_rows (w4a8_quantize.cuh).
+template <bool HALF>
+struct RowQuant {
+    const QuantParams& p;
+    int bad = 0;                 // of the tokens this thread began
+    unsigned ticket = 0;
+    static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r)
+    {
+        if constexpr (HALF) {
+            // pairs of magnitudes in one word: both halves order like unsigned 16-bit numbers
+            uint32_t m = __vmaxu2(__vmaxu2(r.x & 0x7fff7fffu, r.y & 0x7fff7fffu), __vmaxu2(r.z & 0x7fff7fffu, r.w & 0x7fff7fffu));
+            return max(best, max(m & 0xffffu, m >> 16));
+        }
+        return max(max(best, max(r.x & 0x7fffffffu, r.y & 0x7fffffffu)), max(r.z & 0x7fffffffu, r.w & 0x7fffffffu));
+    }
+    __device__ __forceinline__ float begin(int m, uint32_t bits)
+    {
+        if (p.rowmax) {
+            bits = p.rowmax[m];
+            p.rowmax[m] = 0u;    // consumed: the next SwiGLU epilogue maxes into a clean word
+        }
+        float maximum;
+        if (HALF && !p.rowmax) {
+            bad = bits >= 0x7c00u ? 1 : 0;
+            maximum = __half2float(__ushort_as_half((uint16_t)bits));
+        } else {
+            bad = bits >= 0x7f800000u ? (p.rowmax ? 2 : 1) : 0;
+            maximum = __uint_as_float(bits);
+        }
+        const float s = (maximum == 0.f || bad) ? 1.0f : fmaxf(__fdiv_rn(maximum, 127.0f), FLT_MIN);
+        const float inv = __fdiv_rn(1.0f, s);
+        p.scales[m] = s;
+        p.inverse[m] = inv;
+        if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
+        // "any row bad" without a reset pass, see finish(): the ticket is drawn here, its answer is needed at the end
+        if (bad) { atomicOr(&p.status->bad_accum, bad); __threadfence(); }
+        ticket = atomicInc(&p.status->done, (unsigned)p.M - 1u);
+        return inv;
+    }
+    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
+    {
+        return quantize4(__fmul_rn(a, inv), __fmul_rn(b, inv), __fmul_rn(c, inv), __fmul_rn(d, inv));
+    }
+    // the last token to have drawn its ticket publishes the accumulated verdict and clears the scratch word; the counter
+    // wraps to zero by itself (atomicInc with limit M - 1)
+    __device__ __forceinline__ void finish(bool began)
+    {
+        if (began && ticket == (unsigned)p.M - 1u) {
+            __threadfence();
+            const int any = atomicExch(&p.status->bad_accum, 0);
+            p.status->bad_input = any;
+            if (p.host_flag) *p.host_flag = any;
+        }
+    }
+};
+template <bool HALF, int TG, bool SCAN, int BS, int UN>
+__global__ void __launch_bounds__(BS, (UN == 4 ? 2048 : 1024) / BS) quantize_rows_kernel(const QuantParams p)
 {
+    pdl_launch_dependents();   // the GEMM behind this kernel may start prefetching weights
+    pdl_wait();                // A may be the output of the kernel in front of this one
+    RowQuant<HALF> op{p};
+    quantize_rows<HALF, TG, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, op);
+    op.finish(threadIdx.x < TG && (int)(blockIdx.x * TG + threadIdx.x) < p.M);
+}
+
+// Any row: one CTA per token, a thread per 16-element unit, element by element where 16-byte loads are not possible.
+template <bool HALF>
+__global__ void __launch_bounds__(256, 8) quantize_kernel(const QuantParams p)
+{
+    constexpr int BS = 256;
     using T = typename ActType<HALF>::type;
     pdl_launch_dependents();   // the GEMM behind this kernel may start prefetching weights
     pdl_wait();                // A may be the output of the kernel in front of this one
@@ -123,8 +190,6 @@ __global__ void __launch_bounds__(BS, 2048 / BS) quantize_kernel(const QuantPara
     const float inv = s_inverse;
     const int mt = m / p.T, t = m - mt * p.T;
     uint4* dst = reinterpret_cast<uint4*>(p.Xq) + ((size_t)mt * chunks) * p.T + t;
-    // (the row is read a second time here, from L2: keeping it in registers between the passes needs more than the 32
-    // registers per thread that let sixteen 128-thread CTAs share an SM -- the compiler spilled it)
     for (int kc = tid; kc < chunks; kc += BS) {
         uint4 q = make_uint4(0u, 0u, 0u, 0u);
         if (kc < live_chunks) {
@@ -160,6 +225,17 @@ __global__ void __launch_bounds__(BS, 2048 / BS) quantize_kernel(const QuantPara
     }
 }
 
+template <bool HALF, bool SCAN>
+static cudaError_t launch_quantize_rows(const QuantParams& p, cudaLaunchConfig_t& cfg)
+{
+    return with_quantize_rows_shape<HALF, SCAN>(p.M, p.K, [&](auto tg, auto bs, auto un) {
+        constexpr int TG = decltype(tg)::value, BS = decltype(bs)::value, UN = decltype(un)::value;
+        cfg.gridDim = dim3((unsigned)((p.M + TG - 1) / TG));
+        cfg.blockDim = dim3((unsigned)BS);
+        return cudaLaunchKernelEx(&cfg, quantize_rows_kernel<HALF, TG, SCAN, BS, UN>, p);
+    });
+}
+
 cudaError_t launch_quantize(const QuantParams& p, cudaStream_t stream, bool pdl)
 {
     cudaLaunchConfig_t cfg = {};
@@ -169,14 +245,15 @@ cudaError_t launch_quantize(const QuantParams& p, cudaStream_t stream, bool pdl)
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    // One CTA per token.  With many tokens the kernel is bound by how many rows are in flight, so
-    // rows of up to 4096 elements get 128-thread CTAs (16 resident per SM instead of 8).
-    const bool narrow = p.M >= 512 && p.K <= 4096;
-    cfg.gridDim = dim3((unsigned)p.M);
-    cfg.blockDim = dim3(narrow ? 128 : 256);
     cfg.dynamicSmemBytes = 0;
-    if (narrow) return p.half ? cudaLaunchKernelEx(&cfg, quantize_kernel<true, 128>, p) : cudaLaunchKernelEx(&cfg, quantize_kernel<false, 128>, p);
-    return p.half ? cudaLaunchKernelEx(&cfg, quantize_kernel<true, 256>, p) : cudaLaunchKernelEx(&cfg, quantize_kernel<false, 256>, p);
+    const bool scan = p.rowmax == nullptr;      // (collected maxima come with an fp32 middle)
+    if (!(p.half ? scan && quantize_rows_ok<true>(p.A, p.K, p.T) : quantize_rows_ok<false>(p.A, p.K, p.T))) {
+        cfg.gridDim = dim3((unsigned)p.M);
+        cfg.blockDim = dim3(256);
+        return p.half ? cudaLaunchKernelEx(&cfg, quantize_kernel<true>, p) : cudaLaunchKernelEx(&cfg, quantize_kernel<false>, p);
+    }
+    if (p.half) return launch_quantize_rows<true, true>(p, cfg);
+    return scan ? launch_quantize_rows<false, true>(p, cfg) : launch_quantize_rows<false, false>(p, cfg);
 }
 
 // =============================================================== mma.sync GEMM

@@ -16,6 +16,7 @@
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
 #include "w4a8_ptx.cuh"
+#include "w4a8_quantize.cuh"
 
 namespace rkb200 {
 
@@ -57,7 +58,51 @@ __device__ __forceinline__ int w8_code(float x, float inv)
     return (y != y) ? 127 : round_clamp(y);
 }
 
-// One CTA per token: scale (dynamic scan or the caller's), then codes in the Xq layout.  MODE 0 dynamic, 1 static.
+// Scale (dynamic scan or the caller's), then codes in the Xq layout, for rows that allow 16-byte loads.
+template <bool HALF>
+struct W8RowQuant {
+    const W8QuantParams& p;
+    static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r)
+    {
+        // magnitude bits order like magnitudes; a NaN pattern (above infinity) never raises the maximum
+        constexpr uint32_t INF = HALF ? 0x7c00u : 0x7f800000u;
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t a = w[i] & (HALF ? 0x7fffu : 0x7fffffffu), b = HALF ? (w[i] >> 16) & 0x7fffu : 0u;
+            if (a <= INF) best = max(best, a);
+            if (HALF && b <= INF) best = max(best, b);
+        }
+        return best;
+    }
+    // (a negative inverse marks a row whose scale is not positive -- an underflowed maximum: its codes are zeros)
+    __device__ __forceinline__ float begin(int m, uint32_t bits)
+    {
+        float s;
+        if (p.static_scale) s = p.static_scale[m];
+        else {
+            const float maximum = HALF ? __half2float(__ushort_as_half((uint16_t)bits)) : __uint_as_float(bits);
+            s = maximum > 0.f ? __fdiv_rn(maximum, 127.0f) : 1.0f;
+        }
+        p.scales[m] = s;
+        return s > 0.f ? __fdiv_rn(1.0f, s) : -1.f;
+    }
+    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
+    {
+        if (inv < 0.f) return 0u;
+        return __byte_perm(__byte_perm((uint32_t)w8_code(a, inv), (uint32_t)w8_code(b, inv), 0x0040),
+                           __byte_perm((uint32_t)w8_code(c, inv), (uint32_t)w8_code(d, inv), 0x0040), 0x5410);
+    }
+};
+template <bool HALF, int TG, bool SCAN, int BS, int UN>
+__global__ void __launch_bounds__(BS, (UN == 4 ? 2048 : 1024) / BS) w8_quantize_rows_kernel(const W8QuantParams p)
+{
+    pdl_launch_dependents();   // the GEMM behind this kernel may set itself up and request its weights
+    W8RowQuant<HALF> op{p};
+    quantize_rows<HALF, TG, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, op);
+}
+
+// The same for any row: one CTA per token, a thread per 16-element unit.
 template <bool HALF>
 __global__ void __launch_bounds__(256) w8_quantize_kernel(const W8QuantParams p)
 {
@@ -161,12 +206,25 @@ __global__ void __launch_bounds__(256) w8_codes_kernel(const W8QuantParams p)
     }
 }
 
+template <bool HALF, bool SCAN>
+static void launch_w8_rows(const W8QuantParams& p, cudaStream_t stream)
+{
+    if (!quantize_rows_ok<HALF>(p.A, p.K, p.T)) {
+        w8_quantize_kernel<HALF><<<(unsigned)p.M, 256, 0, stream>>>(p);
+        return;
+    }
+    with_quantize_rows_shape<HALF, SCAN>(p.M, p.K, [&](auto tg, auto bs, auto un) {
+        constexpr int TG = decltype(tg)::value, BS = decltype(bs)::value, UN = decltype(un)::value;
+        w8_quantize_rows_kernel<HALF, TG, SCAN, BS, UN><<<(unsigned)((p.M + TG - 1) / TG), BS, 0, stream>>>(p);
+    });
+}
+
 cudaError_t launch_w8_quantize(const W8QuantParams& p, cudaStream_t stream)
 {
     if (p.M < 1 || p.T < 1) return cudaErrorInvalidValue;
     if (p.kind == 2) w8_codes_kernel<<<(unsigned)p.M, 256, 0, stream>>>(p);
-    else if (p.kind == 1) w8_quantize_kernel<true><<<(unsigned)p.M, 256, 0, stream>>>(p);
-    else w8_quantize_kernel<false><<<(unsigned)p.M, 256, 0, stream>>>(p);
+    else if (p.kind == 1) p.static_scale ? launch_w8_rows<true, false>(p, stream) : launch_w8_rows<true, true>(p, stream);
+    else p.static_scale ? launch_w8_rows<false, false>(p, stream) : launch_w8_rows<false, true>(p, stream);
     return cudaGetLastError();
 }
 
