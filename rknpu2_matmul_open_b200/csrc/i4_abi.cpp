@@ -240,7 +240,7 @@ extern "C" rk_npu_i4_workspace* rk_npu_i4_workspace_create(rk_npu_iommu_domain* 
         ws->domain_id = domain->id;
         domain_retain(domain);
         ws->KB = (cfg->K + KBLOCK - 1) / KBLOCK;
-        const PersistPlan plan = gemm_tc_persist_plan(cfg->N, cfg->M, ws->KB, false, ctx->sm_count);
+        const PersistPlan plan = gemm_tc_persist_plan(cfg->N, cfg->M, ws->KB, false, false, ctx->sm_count);
         ws->T = plan.tok / 2;
         ws->parts = plan.split;
         ws->codes_bytes = size_t(align_up(cfg->M, plan.tok)) * size_t(ws->KB) * KBLOCK;

@@ -431,6 +431,7 @@ int enqueue(const Call& c)
         ws.launches.fetch_add(1, std::memory_order_relaxed);
         return RK_NPU_OK;
     }
+    if (ws.variant == 2) ws.T = ws.plan[c.epi == EPI_SWIGLU].tok / 2;      // the layout of the codes follows the launch that reads them
     if (c.codes_in) {
         CodesInParams ci{};
         ci.codes = c.codes_in;
@@ -484,7 +485,7 @@ int enqueue(const Call& c)
     if (ws.variant == 2) {
         g.partials = ws.partials;
         g.counts = ws.counts;
-        g.split = ws.parts;
+        g.split = ws.plan[c.epi == EPI_SWIGLU].split;
         err = launch_gemm_tc_persist(g, c.stream, pdl);
     } else if (ws.variant == 4) {
         g.split = 1;
@@ -1148,9 +1149,8 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     }
     if (variant == 2) {
         ws->TC = 0;
-        const PersistPlan plan = gemm_tc_persist_plan(local_N, cfg->M, ws->KB, false, ctx->sm_count);
-        ws->T = plan.tok / 2;
-        ws->parts = plan.split;
+        for (int swiglu = 0; swiglu < 2; ++swiglu) ws->plan[swiglu] = gemm_tc_persist_plan(local_N, cfg->M, ws->KB, false, swiglu != 0, ctx->sm_count);
+        ws->T = ws->plan[0].tok / 2;
     } else if (variant == 4) {
         ws->TC = ws->T = cfg->M <= 16 ? 16 : cfg->M <= 32 ? 32 : cfg->M <= 64 ? 64 : 128;   // tcgen05 N
     } else {
@@ -1165,7 +1165,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (schedule.cluster && (variant == 1 || variant == 5 || (variant == 3 && (ws->KB + schedule.cluster - 1) / schedule.cluster <= FUSED_MAX_STAGES)) &&
         (variant == 5 || ws->KB >= schedule.cluster))
         ws->split_override = schedule.cluster;
-    const size_t Mp = size_t(align_up(cfg->M, variant == 2 ? 2 * ws->T : ws->T));
+    const size_t Mp = variant == 2 ? size_t(std::max(align_up(cfg->M, ws->plan[0].tok), align_up(cfg->M, ws->plan[1].tok))) : size_t(align_up(cfg->M, ws->T));
     ws->codes_bytes = Mp * size_t(ws->KB) * KBLOCK;
     const int out_cols = cfg->N;
     ws->stage_in_bytes = size_t(cfg->M) * cfg->K * 4;
@@ -1181,11 +1181,12 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes);
     }
-    if (variant == 2 && ws->parts > 1) {
+    if (variant == 2 && (ws->plan[0].split > 1 || ws->plan[1].split > 1)) {
         // partial sums of tiles whose K is cut between CTA pairs, and how many parts of each are done
-        const PersistPlan plan{2 * ws->T, ws->parts};
-        ws->partials_bytes = gemm_tc_persist_slot_bytes(local_N, cfg->M, plan);
-        ws->counts_bytes = gemm_tc_persist_count_bytes(local_N, cfg->M, plan);
+        for (const PersistPlan& plan : ws->plan) {
+            ws->partials_bytes = std::max(ws->partials_bytes, gemm_tc_persist_slot_bytes(local_N, cfg->M, plan));
+            ws->counts_bytes = std::max(ws->counts_bytes, gemm_tc_persist_count_bytes(local_N, cfg->M, plan));
+        }
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->partials), ws->partials_bytes);
         ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->counts), ws->counts_bytes);
     }

@@ -247,16 +247,16 @@ int gemm_decode_ctas(int items, int cluster, int cap);
 int gemm_decode_resident_ctas(int cluster, size_t smem, int sm_count);
 cudaError_t launch_gemm_decode(const DecodeParams& p, cudaStream_t stream, bool pdl);
 cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, bool pdl);
-// persistent two-CTA tcgen05 kernel (K <= 131072): p.T (tokens of one CTA's activation tile: 32, 64 or 128) and p.split
+// persistent two-CTA tcgen05 kernel (K <= 131072): p.T (tokens of one CTA's activation tile: 32, 64, 96, 112 or 128) and p.split
 // required, p.partials and p.counts where split > 1
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
 bool gemm_tc_persist_supported(const GemmParams& p);
 // How the persistent kernel cuts a problem (columns: all accumulator rows, i.e. gate and up together for SwiGLU)
 struct PersistPlan {
-    int tok;      // tokens of the MMA tile (64, 128 or 256): p.T = tok / 2, the code buffer holds whole multiples of tok
+    int tok;      // tokens of the MMA tile (64, 128, 192, 224 or 256): p.T = tok / 2, the code buffer holds whole multiples of tok
     int split;    // parts a tile's K is cut into (p.split)
 };
-PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, int sm_count);
+PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count);
 int gemm_tc_persist_tiles(int columns, int M, int tok);
 // Bytes of GemmParams.partials and .counts (the latter zero before the first launch); 0 where nothing is split
 size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan);

@@ -3,8 +3,8 @@
 // Packed int4 weights -> tensor memory as the A operand, int8 activation codes as shared-memory B operand, kind::i8
 // MMA over a CTA pair with cta_group::2, int32 accumulators in tensor memory, organised so that nothing but the
 // tensor pipe sits on the critical path:
-//   * one cluster of two CTAs per SM pair stays resident and walks a run of 256-channel x (64, 128 or 256)-token
-//     tiles; barriers, tensor memory and descriptors are set up once.  Where the tiles are few, K is cut into parts;
+//   * one cluster of two CTAs per SM pair stays resident and walks a run of 256-channel x (64, 128, 192, 224 or
+//     256)-token tiles; barriers, tensor memory and descriptors are set up once.  Where the tiles are few, K is cut into parts;
 //   * weights and activations travel through SEPARATE rings of bulk copies.  A weight slot is
 //     free again as soon as the unpack warps have read it (the unpacked copy lives in tensor
 //     memory), an activation slot when the MMAs that read it retire.  Together the rings take all of shared memory,
@@ -28,7 +28,10 @@ namespace rkb200 {
 
 constexpr int PS_ROLE_WARPS = 4;             // warp 0: activation producer, 1: MMA issuer, 2: weight producer, 3: activation voucher
 constexpr int PS_UNPACK_WARPS = 8;
-constexpr int PS_EPI_WARPS = 8;              // two per tensor-memory lane quarter, alternating 32-token chunks
+// (With twelve or sixteen, at 80 and 72 registers a thread, the finishing gets the issue slots that the unpacking and the MMA
+// issuer need: SwiGLU at 192 tokens 426 -> 458 and 558 us.)
+constexpr int PS_EPI_WARPS = 8;
+constexpr int PS_EPI_SETS = PS_EPI_WARPS / 4;  // per tensor-memory lane quarter, taking 32-token chunks in turn
 constexpr int PS_UNPACK_WARP0 = PS_ROLE_WARPS;
 constexpr int PS_EPI_WARP0 = PS_UNPACK_WARP0 + PS_UNPACK_WARPS;
 constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 640
@@ -41,10 +44,10 @@ constexpr int PS_TMEM_COLS = 512;
 template <bool W8, int TOK>
 struct PsShape {
     static constexpr int T = TOK / 2;                                            // tokens of one CTA's activation tile
-    static constexpr int XA = TOK == 256 ? (W8 ? 3 : 5) : TOK == 128 && W8 ? 4 : 6;   // activation ring
-    static constexpr int XW = TOK == 256 ? 4 : W8 ? 4 : TOK == 128 ? 6 : 8;     // weight ring
-    static constexpr int ACC = TOK == 256 ? 1 : 2;                               // accumulators
-    static constexpr int ABUF = TOK == 64 ? 6 : 4;                               // unpacked weight stages
+    static constexpr int XA = TOK == 256 ? (W8 ? 3 : 5) : TOK == 224 ? (W8 ? 3 : 4) : TOK == 192 ? (W8 ? 4 : 5) : TOK == 128 && W8 ? 4 : 6;   // activation ring
+    static constexpr int XW = TOK == 256 || W8 ? 4 : TOK >= 128 ? 6 : 8;        // weight ring
+    static constexpr int ACC = TOK > 192 ? 1 : 2;                                // accumulators
+    static constexpr int ABUF = TOK == 64 ? 6 : TOK == 192 ? 2 : 4;              // unpacked weight stages
     static constexpr int A_COL0 = ACC * TOK;
     static constexpr size_t XA_BYTES = 2 * (size_t)T * 128;
     static constexpr uint32_t GB = W8 ? 4096 : 2048;                             // one k-block of one 32-channel group
@@ -75,10 +78,10 @@ __device__ __forceinline__ bool epilogue_all(bool ok)
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 q, %1, 0;\n\t"
-        "bar.red.and.pred p, 1, 256, q;\n\t"
+        "bar.red.and.pred p, 1, %2, q;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(all)
-        : "r"(ok ? 1u : 0u)
+        : "r"(ok ? 1u : 0u), "n"(32 * PS_EPI_WARPS)
         : "memory");
     return all != 0;
 }
@@ -392,7 +395,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         // number of instructions: eight warps share the issue slots with the unpack warps, so the arithmetic works on pairs
         // of tokens (one instruction per two operations).
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
-        const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes 32-token chunks eset, eset + 2, ...
+        const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes 32-token chunks eset, eset + PS_EPI_SETS, ...
         const int sid = (warp - PS_EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const int out_cols = swiglu ? p.F : p.N;
@@ -401,6 +404,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         const bool up_lane = swiglu && lane >= 16;
         const int odd = lane & 1;
         const bool quad_ok = (out_cols % 4 == 0) && (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
+        constexpr int STEP = 32 * PS_EPI_SETS;
         constexpr int SHIFT = W8 ? 0 : 4;             // int4 records enter the MMA times 16
         bool ok = dependency_met();
         RingPos<S::ACC> rc;
@@ -413,13 +417,13 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
             const int n = col0 + col;
             const bool n_ok = n < out_cols;
             const float sw = n_ok ? p.sw[(up_lane ? p.F : 0) + n] : 0.f;
-            // 32-token chunks of this warp that hold live tokens: those at 32 eset + 64 c, c < chunks
-            const int chunks = max(0, min(TOK / 64, (p.M - tok_base - 32 * eset + 63) / 64));
+            // 32-token chunks of this warp that hold live tokens: those at 32 eset + STEP c, c < chunks
+            const int chunks = max(0, (min(TOK, p.M - tok_base) - 32 * eset + STEP - 1) / STEP);
             if (sid < TOK) {
                 const int m = tok_base + sid;
                 s_sx[sid] = m < p.M ? p.sx[m] : 0.f;
             }
-            asm volatile("bar.sync 1, 256;" ::: "memory");   // scales staged (the barrier at the end of a tile keeps stragglers out)
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");   // scales staged (the barrier at the end of a tile keeps stragglers out)
             ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // one verdict for all eight warps
             if (!ok) { *s_error = 1; break; }
             if (sid == 0) PS_STAMP(j, 3);
@@ -443,14 +447,14 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
 #pragma unroll 1
                 for (int c = 0; c < chunks; ++c) {
                     uint32_t r[32];
-                    tc_ld32(acc_addr + 64 * c, r);
+                    tc_ld32(acc_addr + STEP * c, r);
                     tc_wait_ld();
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        __stcg(slot + (size_t)(16 * c + i) * 128, make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]));
+                        __stcg(slot + (size_t)(STEP / 4 * c + i) * 128, make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]));
                 }
                 __threadfence();
-                asm volatile("bar.sync 1, 256;" ::: "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
                 if (sid == 0) {
                     // (a tile with a part whose wait ran out is never completed; the launch reports the error and the host
                     // clears the counters)
@@ -460,14 +464,14 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                     *s_finish = done ? 1 : 0;
                     __threadfence();
                 }
-                asm volatile("bar.sync 1, 256;" ::: "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
                 finish = *reinterpret_cast<volatile int*>(s_finish) != 0;
             }
             const int turns = finish ? 2 * chunks : 0;
             const int other = part == 0 ? 1 : 0;                          // the first of the other parts
             int4 ahead[4];                                                // its sums of the next turn, on their way
             auto fetch_part = [&](int4 (&v)[4], int which, int k) {
-                const int4* const src = slots + which * part_stride + (size_t)(16 * (k >> 1) + 4 * (k & 1)) * 128;
+                const int4* const src = slots + which * part_stride + (size_t)(STEP / 4 * (k >> 1) + 4 * (k & 1)) * 128;
 #pragma unroll
                 for (int h = 0; h < 4; ++h) v[h] = __ldcg(src + (size_t)h * 128);
             };
@@ -475,7 +479,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
             if (split == 1 && chunks == 0) hand_back();
 #pragma unroll 1
             for (int k = 0; k < turns; ++k) {
-                const int t0 = 32 * eset + 64 * (k >> 1) + 16 * (k & 1), m0 = tok_base + t0;
+                const int t0 = 32 * eset + STEP * (k >> 1) + 16 * (k & 1), m0 = tok_base + t0;
                 uint32_t r[16];
                 tc_ld16(lane_addr + rc.slot * TOK + t0, r);
                 tc_wait_ld();
@@ -618,7 +622,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                 }
             }
             if (sid == 0) PS_STAMP(j, 5);
-            asm volatile("bar.sync 1, 256;" ::: "memory");   // every epilogue warp is done with this tile's scales and maxima
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");   // every epilogue warp is done with this tile's scales and maxima
             if (swiglu && p.rowmax && sid < TOK) {
                 const uint32_t m = s_tilemax[sid];
                 if (m) {
@@ -694,41 +698,50 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
     cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, p, clusters);
 }
+template <int TOK>
+cudaError_t launch_persist_tok(const GemmParams& p, cudaStream_t stream, bool pdl)
+{
+    return p.w8 ? launch_persist_inst<true, TOK>(p, stream, pdl) : launch_persist_inst<false, TOK>(p, stream, pdl);
+}
 } // namespace
 
 bool gemm_tc_persist_supported(const GemmParams& p)
 {
-    return (p.T == 128 || p.T == 64 || p.T == 32) && (long long)p.KB * KBLOCK <= PS_MAX_K && p.split >= 1 && (p.split == 1 || (p.partials && p.counts));
+    return (p.T == 32 || p.T == 64 || p.T == 96 || p.T == 112 || p.T == 128) && (long long)p.KB * KBLOCK <= PS_MAX_K && p.split >= 1 && (p.split == 1 || (p.partials && p.counts));
 }
 
 int gemm_tc_persist_tiles(int columns, int M, int tok) { return (columns + 255) / 256 * ((M + tok - 1) / tok); }
 
 // The token tile and the number of parts a tile's K is cut into: the cheapest by a model of the kernel's time in cycles,
-// from what it measured on 60 shapes (M 33..4096, K 2048..14336, N 1024..28672, both epilogues; within 1 % of the best
+// from what it measured on 80 shapes (M 33..4096, K 2048..14336, N 1024..28672, both epilogues; within 1 % of the best
 // choice on average, 15 % at worst):
 //   * a k-block takes 270 to 390 cycles at 64 tokens and 310 to 370 at 128, more with more SMs busy (the operands come
 //     out of L2 at about 45 bytes per SM and cycle when all SMs ask), and 530 at 256, where the MMAs bound it; int8
-//     weights are delivery-bound at every width;
-//   * finishing a tile takes 33 cycles per token, 1500 at least (90 with SwiGLU, which changes no choice); two accumulators hide it behind the next
-//     tile's MMAs up to 128 tokens, at 256 there is room for one and nothing is hidden;
+//     weights are delivery-bound (52 bytes per cycle).  At 192 tokens two accumulators leave two buffers of unpacked
+//     weights: 560, and 780 with int8 weights;
+//   * finishing a tile takes 33 cycles per token, 1500 at least; 80 and 4800 with SwiGLU, which bounds the kernel at
+//     K = 4096 (192 tokens instead of 128 amortise it better: 4096 x 4096 -> 14336 450 -> 422 us); two accumulators hide
+//     it behind the next tile's MMAs up to 192 tokens, beyond there is room for one and nothing is hidden;
+//   * 224 tokens are for what 256 would cut worse (777 tokens, 14336 -> 4096 50 -> 46 us);
 //   * K in parts costs an exchange through L2: so much per part and pair, more for wide token tiles;
 //   * a launch on more than half of the SMs leaves the one behind it no room to set itself up meanwhile.
-PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, int sm_count)
+PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
 {
     PersistPlan best{256, 1};
     double best_time = 0;
     const int pairs = std::max(1, sm_count / 2);
-    for (const int tok : {64, 128, 256}) {
+    for (const int tok : {64, 128, 192, 224, 256}) {
         if (tok > 64 && M <= 64) break;                        // half of the tile would be padding
         const long long tiles = (long long)((columns + 255) / 256) * ((M + tok - 1) / tok);
         for (const int split : {1, 2, 3, 4, 6, 8}) {
-            if (split > 1 && (tok == 256 || tiles * split > pairs || KB < 4 * split)) break;
+            if (split > 1 && (tok > 128 || tiles * split > pairs || KB < 4 * split)) break;
             const long long clusters = std::min<long long>(tiles * split, pairs), rounds = (tiles + pairs - 1) / pairs;
             const double busy = double(clusters) / pairs;
-            double block = tok == 64 ? 270 + 120 * busy : tok == 128 ? 310 + 60 * busy : 530;
-            if (w8) block = std::max(block, (16384 + 64 * tok) / 45.0);
-            const double mma = KB * block / split, live = std::min(tok, M), finish = 1500 + 33 * live;
-            double time = tok == 256 ? rounds * (mma + finish) : rounds * std::max(mma, finish) + finish;
+            double block = tok == 64 ? 270 + 120 * busy : tok == 128 ? 310 + 60 * busy : tok == 192 ? 480 + 80 * busy : tok == 224 ? 470 : 530;
+            if (swiglu) block += 20;
+            if (w8) block = tok == 192 ? 780 : std::max(block, (16384 + 64 * tok) / 52.0);
+            const double mma = KB * block / split, live = std::min(tok, M), finish = swiglu ? 4800 + 80 * live : 1500 + 33 * live;
+            double time = tok > 192 ? rounds * (mma + finish) : mma + (rounds - 1) * std::max(mma, finish) + finish;
             if (split > 1) time += (1500 + 1000 * (split - 1) + 30 * clusters) * (1 + 1.5 * std::max(0.0, live - 64) / 64);
             if (2 * clusters > pairs) time += 3000;
             if (best_time == 0 || time < best_time) { best_time = time; best = {tok, split}; }
@@ -748,10 +761,12 @@ size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan)
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
     if (!gemm_tc_persist_supported(p)) return cudaErrorInvalidValue;
-    switch (p.T) {
-    case 32: return p.w8 ? launch_persist_inst<true, 64>(p, stream, pdl) : launch_persist_inst<false, 64>(p, stream, pdl);
-    case 64: return p.w8 ? launch_persist_inst<true, 128>(p, stream, pdl) : launch_persist_inst<false, 128>(p, stream, pdl);
-    default: return p.w8 ? launch_persist_inst<true, 256>(p, stream, pdl) : launch_persist_inst<false, 256>(p, stream, pdl);
+    switch (2 * p.T) {
+    case 64: return launch_persist_tok<64>(p, stream, pdl);
+    case 128: return launch_persist_tok<128>(p, stream, pdl);
+    case 192: return launch_persist_tok<192>(p, stream, pdl);
+    case 224: return launch_persist_tok<224>(p, stream, pdl);
+    default: return launch_persist_tok<256>(p, stream, pdl);
     }
 }
 

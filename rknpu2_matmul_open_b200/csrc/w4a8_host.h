@@ -133,7 +133,7 @@ struct rk_npu_w4a8_workspace {
     float* scales = nullptr;
     float* inverse = nullptr;
     uint32_t* rowmax = nullptr;
-    int parts = 1;                    // variant 2: parts a tile's K is cut into
+    rkb200::PersistPlan plan[2]{};    // variant 2: how a linear and a SwiGLU launch are cut
     int* partials = nullptr;          // variants 2, 4: partial sums of tiles and progress counters
     unsigned int* counts = nullptr;
     size_t partials_bytes = 0, counts_bytes = 0;

@@ -101,7 +101,7 @@ Sizes sizes_of(int M, int N, int K, int kind, int sm_count)
 {
     Sizes z{};
     z.KB = (K + KBLOCK - 1) / KBLOCK;
-    const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, sm_count);
+    const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, false, sm_count);
     z.T = plan.tok / 2;
     z.parts = plan.split;
     z.NG = align_up((N + GROUP - 1) / GROUP, 8) + 8;   // zero groups behind the last tile, as for the int4 weights
