@@ -86,9 +86,25 @@ __device__ __forceinline__ bool epilogue_all(bool ok)
     return all != 0;
 }
 
+// The same barrier; true: `here` holds in one of them.
+__device__ __forceinline__ bool epilogue_any(bool here)
+{
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %1, 0;\n\t"
+        "bar.red.or.pred p, 1, %2, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(any)
+        : "r"(here ? 1u : 0u), "n"(32 * PS_EPI_WARPS)
+        : "memory");
+    return any != 0;
+}
+
+// (Linear and SwiGLU launches have kernels of their own: less to fetch, and neither finishing pays for the other's registers.)
 // W8: the weights are int8 codes in the W8 layout (w8a8_kernels.cu): "unpacking" is a copy into tensor memory and the sums
 // are not scaled by 16.
-template <bool W8, int TOK>
+template <bool W8, bool SWIGLU, int TOK>
 __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const GemmParams p, int num_clusters)
 {
     using S = PsShape<W8, TOK>;
@@ -115,7 +131,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();
     const int cluster_id = blockIdx.x >> 1;
-    const bool swiglu = p.epi == EPI_SWIGLU;
+    constexpr bool swiglu = SWIGLU;
     const int KB = p.KB;
     const int nst = (KB + 1) / 2;                                      // stage iterations per tile
     const int tiles_n = swiglu ? (p.F + 63) / 64 : (p.N + TILE_N - 1) / TILE_N;
@@ -393,7 +409,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         // ---------------------------------------------------------------- epilogue warps
         // A warp finishes sixteen tokens (of its 32 accumulator rows) per turn of a rolled loop.  What bounds it is the
         // number of instructions: eight warps share the issue slots with the unpack warps, so the arithmetic works on pairs
-        // of tokens (one instruction per two operations).
+        // of tokens (one instruction per two operations), the int4 records' 1/16 is in the token scales, one look at the
+        // magnitudes of four gate values settles that none needs the slow division, and maxima are taken of floats, whose
+        // signs the instruction drops (4096 tokens, 4096 -> 2 x 14336: 424 -> 405 us; 300 tokens 54.4 -> 49.6).
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes 32-token chunks eset, eset + PS_EPI_SETS, ...
         const int sid = (warp - PS_EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
@@ -419,11 +437,23 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
             const float sw = n_ok ? p.sw[(up_lane ? p.F : 0) + n] : 0.f;
             // 32-token chunks of this warp that hold live tokens: those at 32 eset + STEP c, c < chunks
             const int chunks = max(0, (min(TOK, p.M - tok_base) - 32 * eset + STEP - 1) / STEP);
+            // Token scales, staged with the int4 records' 1/16 in them: (float)(16 s) * (sx / 16) is (float)s * sx, exactly,
+            // unless sx / 16 is subnormal.  (The barrier at the end of a tile keeps stragglers out.)
+            float sx_here = 0.f;
+            bool tiny = false;
             if (sid < TOK) {
                 const int m = tok_base + sid;
-                s_sx[sid] = m < p.M ? p.sx[m] : 0.f;
+                if (m < p.M) {
+                    sx_here = p.sx[m];
+                    tiny = !W8 && sx_here < 7.8886e-31f;
+                }
+                s_sx[sid] = W8 ? sx_here : sx_here * 0.0625f;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");   // scales staged (the barrier at the end of a tile keeps stragglers out)
+            tiny = epilogue_any(tiny);
+            if (tiny) {
+                if (sid < TOK) s_sx[sid] = sx_here;
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
+            }
             ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // one verdict for all eight warps
             if (!ok) { *s_error = 1; break; }
             if (sid == 0) PS_STAMP(j, 3);
@@ -503,7 +533,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                     if (k + 1 < turns) fetch_part(ahead, other, k + 1);
                 }
                 if (m0 >= p.M) continue;
-                if (p.epi == EPI_I32) {
+                if (!SWIGLU && p.epi == EPI_I32) {
                     int* const row0 = reinterpret_cast<int*>(p.out) + (size_t)m0 * out_cols + n;
                     if (n_ok) {
 #pragma unroll
@@ -522,12 +552,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                         const ulonglong2 sx = sx2[i];
                         y[2 * i] = f2_pack(__int2float_rn((int)r[4 * i]), __int2float_rn((int)r[4 * i + 1]));
                         y[2 * i + 1] = f2_pack(__int2float_rn((int)r[4 * i + 2]), __int2float_rn((int)r[4 * i + 3]));
-                        if constexpr (!W8) { y[2 * i] = f2_mul(y[2 * i], f2_all(0.0625f)); y[2 * i + 1] = f2_mul(y[2 * i + 1], f2_all(0.0625f)); }
+                        if (tiny) { y[2 * i] = f2_mul(y[2 * i], f2_all(0.0625f)); y[2 * i + 1] = f2_mul(y[2 * i + 1], f2_all(0.0625f)); }
                         y[2 * i] = f2_mul(f2_mul(y[2 * i], sx.x), sw2);
                         y[2 * i + 1] = f2_mul(f2_mul(y[2 * i + 1], sx.y), sw2);
                     }
                 }
-                if (p.epi == EPI_F16) {
+                if (!SWIGLU && p.epi == EPI_F16) {
                     // a lane holds one channel of sixteen tokens; two exchange rounds turn that into four neighbouring
                     // channels of four tokens: lanes 4g..4g+3 end up with tokens 4i + (lane & 3)
                     uint32_t word[8];
@@ -563,7 +593,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                                     if (n4 + e < out_cols) dst[e] = __ushort_as_half((unsigned short)((ww[e >> 1] >> (16 * (e & 1))) & 0xffffu));
                             }
                         }
-                } else if (p.epi == EPI_F32) {
+                } else if (!SWIGLU) {
                     float* dst = reinterpret_cast<float*>(p.out) + (size_t)m0 * out_cols + n;
                     if (n_ok) {
 #pragma unroll
@@ -578,46 +608,60 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                     // Lanes 0-15 hold the gate rows g, lanes 16-31 the matching up rows u of 16 features.  The gate lanes
                     // finish the even token of every pair and the up lanes the odd one: each sends the half of the pair
                     // that the other finishes and evaluates eight SiLUs.
-                    uint32_t mx[8];
+                    float v[8];
                     const int mine_row = m0 + (up_lane ? 1 : 0);
+                    const int left = n_ok ? p.M - mine_row : 0;         // rows from here on that are stored
                     float* dst = reinterpret_cast<float*>(p.out) + (size_t)mine_row * out_cols + n;
 #pragma unroll
-                    for (int i = 0; i < 8; i += 2) {
-                        float g[2], u[2], v[2];
+                    for (int h = 0; h < 8; h += 4) {           // (four at a time: one look at the magnitudes, few values waiting)
+                        float g[4];
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
+                        for (int i = 0; i < 4; ++i) {
                             float even_token, odd_token;
-                            f2_unpack(y[i + e], even_token, odd_token);
+                            f2_unpack(y[h + i], even_token, odd_token);
                             const float recv = __shfl_xor_sync(0xffffffffu, up_lane ? even_token : odd_token, 16);
-                            g[e] = up_lane ? recv : even_token;
-                            u[e] = up_lane ? odd_token : recv;
+                            g[i] = up_lane ? recv : even_token;
+                            v[h + i] = up_lane ? odd_token : recv;
                         }
-                        silu_poly2(g[0], g[1], v[0], v[1]);
+                        if (left < 16) {                        // what does not exist has zeros: keep it off the slow path below
 #pragma unroll
-                        for (int e = 0; e < 2; ++e, dst += 2 * (size_t)out_cols) {
-                            v[e] = __fmul_rn(v[e], u[e]);
-                            const bool live = n_ok && mine_row + 2 * (i + e) < p.M;
-                            if (live) *dst = v[e];
-                            mx[i + e] = live ? (__float_as_uint(v[e]) & 0x7fffffffu) : 0u;
+                            for (int i = 0; i < 4; ++i)
+                                if (2 * (h + i) >= left) g[i] = 1.f;
                         }
+                        if (silu_plain(min_abs(min_abs(g[0], g[1]), min_abs(g[2], g[3])), max_abs(max_abs(g[0], g[1]), max_abs(g[2], g[3])))) {
+#pragma unroll
+                            for (int i = 0; i < 4; i += 2) {
+                                float a, b;
+                                minus_silu_poly2(g[i], g[i + 1], a, b);
+                                v[h + i] = __fmul_rn(-a, v[h + i]);
+                                v[h + i + 1] = __fmul_rn(-b, v[h + i + 1]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) v[h + i] = __fmul_rn(silu_poly(g[i]), v[h + i]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i, dst += 2 * (size_t)out_cols)
+                            if (2 * (h + i) < left) *dst = v[h + i];
                     }
                     if (p.rowmax) {
                         // Maxima over the 16 lanes of each half, one token per value: three folding steps that halve the
                         // values a lane holds and a plain one; lanes 2i of a half end up with the maximum of their token.
+                        // (Tokens and channels that do not exist have zero scales, and zeros here.)
 #pragma unroll
                         for (int width = 8; width > 1; width >>= 1) {
                             const bool upper = (lane & width) != 0;
 #pragma unroll
                             for (int i = 0; i < width / 2; ++i) {
-                                const uint32_t keep = upper ? mx[i + width / 2] : mx[i];
-                                const uint32_t give = upper ? mx[i] : mx[i + width / 2];
-                                mx[i] = max(keep, __shfl_xor_sync(0xffffffffu, give, width));
+                                const float keep = upper ? v[i + width / 2] : v[i];
+                                const float give = upper ? v[i] : v[i + width / 2];
+                                v[i] = max_abs(keep, __shfl_xor_sync(0xffffffffu, give, width));
                             }
                         }
-                        mx[0] = max(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], 1));
+                        const uint32_t most = __float_as_uint(max_abs(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1)));
                         // collected per CTA and tile in shared memory first: one global atomic per token and tile
                         // instead of one per token, tile and 16 features
-                        if (!odd && mx[0]) atomicMax(&s_tilemax[t0 + (up_lane ? 1 : 0) + 2 * ((lane >> 1) & 7)], mx[0]);
+                        if (!odd && most) atomicMax(&s_tilemax[t0 + (up_lane ? 1 : 0) + 2 * ((lane >> 1) & 7)], most);
                     }
                 }
             }
@@ -651,11 +695,11 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
 namespace {
 constexpr long long PS_MAX_K = 131072;
 
-template <bool W8, int TOK>
+template <bool W8, bool SWIGLU, int TOK>
 cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
     using S = PsShape<W8, TOK>;
-    auto kernel = gemm_tc_persist_kernel<W8, TOK>;
+    auto kernel = gemm_tc_persist_kernel<W8, SWIGLU, TOK>;
     static PerDeviceOnce configured;
     static int clusters_of_device[64] = {};   // resident CTA pairs, per CUDA ordinal
     int device = -1;
@@ -701,7 +745,8 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
 template <int TOK>
 cudaError_t launch_persist_tok(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
-    return p.w8 ? launch_persist_inst<true, TOK>(p, stream, pdl) : launch_persist_inst<false, TOK>(p, stream, pdl);
+    if (p.w8) return p.epi == EPI_SWIGLU ? cudaErrorInvalidValue : launch_persist_inst<true, false, TOK>(p, stream, pdl);
+    return p.epi == EPI_SWIGLU ? launch_persist_inst<false, true, TOK>(p, stream, pdl) : launch_persist_inst<false, false, TOK>(p, stream, pdl);
 }
 } // namespace
 

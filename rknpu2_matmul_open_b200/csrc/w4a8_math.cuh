@@ -130,18 +130,19 @@ __device__ __forceinline__ float silu_poly(float g)
     const float d = __fadd_rn(1.f, __fmul_rn(q, power));
     return g < -80.f ? -0.f : __fdiv_rn(g, d);
 }
-// The same function, two arguments at a time, for the kernels that evaluate it over and over.
+// The same function, two arguments at a time, for the kernels that evaluate it over and over; for arguments with |g| in
+// [2^-40, 80] only (silu_plain), where no step leaves the normal range: d < 2^116.
 //   * floor(y) for |y| < 2^22: adding 1.5 * 2^23 with rounding towards minus infinity leaves floor(y) in the low bits,
 //     from where the subtraction brings it back as a float and a shift puts it into the exponent of 2^n.
 //   * g / d, correctly rounded: a reciprocal within an ulp refined by one Newton step, a quotient from it, its remainder
 //     by fused multiply-add (exact) and one correction (P. Markstein, "Computation of elementary functions on the IBM
-//     RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  Magnitudes for which a step could leave the normal range
-//     take the division instruction sequence.
-// Equal bit for bit to silu_poly for every one of the 2^32 arguments (checked).
-__device__ __forceinline__ void silu_poly2(float g0, float g1, float& y0, float& y1)
+//     RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), all of it negated: the reciprocal of a negated argument
+//     costs nothing, the negation of a pair two instructions.  Returns the negated values.
+// With silu_poly for every other argument equal bit for bit to silu_poly for every one of the 2^32 arguments (checked).
+__device__ __forceinline__ void minus_silu_poly2(float g0, float g1, float& y0, float& y1)
 {
     const F2 g = f2_pack(g0, g1);
-    const F2 x = f2_pack(fminf(fmaxf(-g0, -80.f), 80.f), fminf(fmaxf(-g1, -80.f), 80.f));
+    const F2 x = f2_pack(-g0, -g1);
     const F2 shifted = f2_add_rm(f2_fma(x, f2_all(1.4426950408889634f), f2_all(0.5f)), f2_all(12582912.f));
     const F2 n = f2_add(shifted, f2_all(-12582912.f));
     F2 r = f2_fma(n, f2_all(-0.693145751953125f), x);
@@ -159,17 +160,18 @@ __device__ __forceinline__ void silu_poly2(float g0, float g1, float& y0, float&
     const F2 d = f2_add(f2_all(1.f), f2_mul(q, power));
     float d0, d1, r0, r1;
     f2_unpack(d, d0, d1);
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
-    const F2 minus_d = f2_pack(-d0, -d1), rough = f2_pack(r0, r1);
-    const F2 inv = f2_fma(rough, f2_fma(minus_d, rough, f2_all(1.f)), rough);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-d0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-d1));
+    const F2 rough = f2_pack(r0, r1);                        // about -1 / d
+    const F2 inv = f2_fma(rough, f2_fma(d, rough, f2_all(1.f)), rough);
     const F2 quo = f2_mul(g, inv);
-    f2_unpack(f2_fma(f2_fma(minus_d, quo, g), inv, quo), y0, y1);
-    // |g| in [2^-40, 80]: d < 2^116, so quotient and remainder are normal numbers (or the remainder is zero)
-    const bool plain0 = fabsf(g0) >= 9.094947017729282e-13f && fabsf(g0) <= 80.f, plain1 = fabsf(g1) >= 9.094947017729282e-13f && fabsf(g1) <= 80.f;
-    if (!plain0) y0 = g0 < -80.f ? -0.f : __fdiv_rn(g0, d0);
-    if (!plain1) y1 = g1 < -80.f ? -0.f : __fdiv_rn(g1, d1);
+    f2_unpack(f2_fma(f2_fma(d, quo, g), inv, quo), y0, y1);
 }
+// Larger and smaller magnitude of two values; a NaN stays one.
+__device__ __forceinline__ float max_abs(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b))); return d; }
+__device__ __forceinline__ float min_abs(float a, float b) { float d; asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b))); return d; }
+__device__ __forceinline__ bool silu_plain(float smallest, float largest) { return smallest >= 9.094947017729282e-13f && largest <= 80.f; }
+
 __device__ __forceinline__ float dequant(int acc, float sx, float sw)
 {
     return __fmul_rn(__fmul_rn(__int2float_rn(acc), sx), sw);
