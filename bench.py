@@ -1129,9 +1129,12 @@ def _print_stamps(rk, case, calls, stream, torch):
         lib.rk_npu_b200_w4a8_trace_read(calls[0][1].handle, raw.ctypes.data, 32)
         print(f"clusters in the grid: {int(raw[200])}; per tile of cluster 0 (cycles since kernel start): MMA issuer begins,"
               " first MMA issued, last commit, epilogue sees the accumulator, tensor memory handed back, tile stored,"
-              " cycles the issuer waited for operands | unpack warp: waited for weights, for a free buffer, for activations")
-        for j in range(7):
-            print(f"tile {j}: {[int(x) for x in raw[j * 8:j * 8 + 7]]} | {int(raw[128 + 2 * j])} {int(raw[129 + 2 * j])} {int(raw[160 + j])}")
+              " cycles the issuer waited for operands")
+        for j in range(16):
+            if raw[j * 8 + 2]:
+                print(f"tile {j}: {[int(x) for x in raw[j * 8:j * 8 + 7]]}")
+        print(f"cycles in the whole launch: an unpack warp waited for weights {int(raw[128])}, for a free buffer {int(raw[129])};"
+              f" activations were waited for {int(raw[160])}")
 
 
 def main():

@@ -154,7 +154,7 @@ int rk_npu_b200_w4a8_last_quant(rk_npu_w4a8_workspace *workspace, float *scales,
  * RK_NPU_B200_VARIANT overrides where the geometry allows).  The family is fixed with the activation-code layout at
  * creation, except that a workspace of up to eight tokens may move between 3 and 5, which share it.
  * split_k: 0 = automatic, else the number of CTAs that cooperate on a column tile: the split-K factor (1..8 for
- * family 3; 1, 2, 4, 8 for 1 and 2) or the decode kernel's cluster size (1, 2, 4, 8); ignored by family 4.
+ * family 3; 1, 2, 4, 8 for 1) or the decode kernel's cluster size (1, 2, 4, 8); ignored by families 2 and 4.
  * Returns RK_NPU_ERR_PARAM when the workspace geometry cannot run the request.
  * rk_npu_b200_w4a8_schedule reads both back (either pointer may be NULL). */
 int rk_npu_b200_w4a8_set_schedule(rk_npu_w4a8_workspace *workspace, int variant, int split_k);
@@ -165,11 +165,12 @@ int rk_npu_b200_w4a8_schedule(const rk_npu_w4a8_workspace *workspace, int *varia
  * since the CTA's start at: weights requested, dependency met, scales known, slice quantised,
  * contraction done, partials exchanged -- and the end (ns); trace_read copies stamps[ctas][8]
  * (CTA index = blockIdx.y * gridDim.x + blockIdx.x, at most 16384 CTAs).
- * Persistent large-batch GEMM: CTA pair 0 records per tile j < 16 at [8 j + 0..6] the cycles since
- * kernel start at which the MMA issuer begins, issues its first MMA, commits the last, the epilogue
- * sees the accumulator, hands tensor memory back, has stored the tile, and the cycles the issuer
- * waited for operands; [128 + 2 j], [129 + 2 j], [160 + j] the cycles one unpack warp waited for
- * weights, for a free tensor-memory buffer and for activations; [200] the CTA pairs in the grid.
+ * Persistent large-batch GEMM: CTA pair 0 records per tile (or part of one) j < 16 at [8 j + 0..6] the
+ * cycles since kernel start at which the MMA issuer begins, issues its first MMA, commits the last,
+ * the epilogue sees the accumulator, hands tensor memory back, has stored the tile, and the cycles the
+ * issuer waited for operands; [128], [129] the cycles one unpack warp waited for weights and for a free
+ * tensor-memory buffer in the whole launch, [160] those until activations had landed; [200] the CTA
+ * pairs in the grid.
  * The caller synchronises first.  `bench.py --case decode|prefill --stamps` prints both. */
 int rk_npu_b200_w4a8_trace_enable(rk_npu_w4a8_workspace *workspace, int enable);
 int rk_npu_b200_w4a8_trace_read(rk_npu_w4a8_workspace *workspace, unsigned long long *stamps, int ctas);
