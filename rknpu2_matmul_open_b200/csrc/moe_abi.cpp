@@ -455,6 +455,8 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
         const int grid_rows = std::min(1 << level, c.max_rows);
         ok = ok && ((!timings && launch_kept(*ws, f32, pull, grid_rows, level)) || launch_run(*ws, f32, pull, grid_rows, true, timings ? ws->events : nullptr));
         at = Clock::now();
+        // int8 rows are not judged on the device, so a large result can follow its kernel at once
+        if (ok && !direct && !f32) ok = cudaMemcpyAsync(output, ws->out, values * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
         if (!ok) {      // a launch failed part-way: the row maxima may be left behind
             cudaGetLastError();
             cudaMemsetAsync(ws->row_max, 0, ws->row_max_bytes, s);
@@ -476,7 +478,7 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
         }
         if (ws->host_status->bad_input) return RK_NPU_ERR_PARAM;              // a rejected row: the output is not written
         if (!u.serial && direct) std::memcpy(output, ws->host_out.ptr, values * 4);
-        else if (!u.serial && cudaMemcpy(output, ws->out, values * 4, cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        else if (!u.serial && f32 && cudaMemcpy(output, ws->out, values * 4, cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
         t.sync_us = since_us(at);
         if (timings) {
             t.input_us = event_us(ws->events[0], ws->events[1]);

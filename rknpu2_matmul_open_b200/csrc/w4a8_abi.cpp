@@ -629,11 +629,14 @@ int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const vo
     // copies it out.  (The activations are still copied in: every CTA reads them.)  The single-kernel families write
     // every element once, in rows as long as a warp; the others in pieces of 64 bytes, which the bus takes more slowly, so
     // that from 128 KB on the copy engine is as fast.
+    // Rows that do not start on a sector leave it in pieces of sectors: beyond 40 KB of binary16 and 64 KB of
+    // words these are copied (13 x 4910 binary16 64 against 38 us, 13 x 4912 34; 3 x 4911 fp32 27 against 36).
     // (Not when the caller asks for stage timings: the device part of a call must not contain stores that cross the bus,
     // or the figures of different kernel families -- which the search tuner ranks -- stop being comparable.)
     const bool own_report = !grouped(*ws) && !metrics && ws->host_status_alias;
     const bool single_kernel = ws->variant == 3 || ws->variant == 5;
-    const bool bus_result = !c_dev && own_report && epi != EPI_SWIGLU && out_bytes <= (single_kernel ? size_t(512) << 10 : size_t(128) << 10);
+    const bool bus_result = !c_dev && own_report && epi != EPI_SWIGLU && out_bytes <= (single_kernel ? size_t(512) << 10 : size_t(128) << 10) &&
+                            (cfg.M == 1 || out_bytes / cfg.M % 32 == 0 || out_bytes <= (epi == EPI_F16 ? size_t(40) << 10 : size_t(64) << 10));
     void* c_alias = bus_result ? c_at.alias : nullptr;
     const bool bounce_out = bus_result && !c_alias && ws->bounce_out.alias && out_bytes <= ws->bounce_out.bytes;
     if (bounce_out) c_alias = ws->bounce_out.alias;
@@ -1136,9 +1139,10 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     const bool fused_mid = fused_ok && cfg->M > 8 && cfg->M <= 16 && (long long)cfg->K * local_N / 2 <= (8ll << 20);
     // From 17 tokens on the persistent tcgen05 kernel, whose time hardly depends on the batch up to 64 (4096 -> 4096 13 us,
     // 11008 -> 4096 19, 4096 -> 14336 14.5), unless its 256-channel tiles are so few that the ring's small CTAs cover more
-    // of the GPU (24 tokens: 2048 -> 2048 9.3 us, the ring's 16.4 / 24 / 17.1 us on the three shapes above).
+    // of the GPU (24 tokens: 2048 -> 2048 9.3 us, 3840 -> 3840 10.4 against 12.1, but 16.4 / 24 / 17.1 us on the three
+    // shapes above).
     const int channel_tiles = (local_N + 255) / 256;
-    const bool pair_best = tc_ok && (cfg->M > 96 || (cfg->M > 32 && channel_tiles > 4) || (cfg->M > 16 && channel_tiles > 12));
+    const bool pair_best = tc_ok && (cfg->M > 96 || (cfg->M > 32 && channel_tiles > 4) || (cfg->M > 16 && channel_tiles > 15));
     int variant = decode_best ? 5 : pair_best ? 2 : (fused_best || fused_mid) ? 3 : 1;
     if (forced == 1 || (forced == 2 && tc_ok) || (forced == 3 && fused_ok) || (forced == 4 && stream_ok) || (forced == 5 && decode_ok))
         variant = forced;
