@@ -10,6 +10,7 @@
 // Workspace::run (:582-595).
 #include "w4a8_host.h"
 #include "moe_device.h"
+#include "moe_rows.h"
 #include "../../include/rknpu_b200_moe.h"
 #include <algorithm>
 #if defined(__x86_64__)
@@ -28,10 +29,6 @@ using namespace rkb200;
 namespace {
 using Clock = std::chrono::steady_clock;
 double since_us(Clock::time_point t) { return std::chrono::duration<double, std::micro>(Clock::now() - t).count(); }
-// Rows up to this size are staged in page-locked memory and read from there by the intake kernel; larger ones are copied
-// from the caller's array by the driver (one token: the copy engine would cost another call and its own start, 4 + 2 us of
-// about 30; 512 KB: 40 us against 44; 2 MB: 148 against 136).
-constexpr size_t MOE_PULL_MOST = size_t(512) << 10;
 // Results up to this size are stored by the combine kernel straight into page-locked host memory.
 constexpr size_t MOE_DIRECT_MOST = size_t(512) << 10;
 constexpr int MOE_HIDDEN_MAX = 8192;   // 16 gathered rows of codes must fit one CTA's shared memory
@@ -160,7 +157,7 @@ struct rk_npu_moe_w8_workspace {
     size_t arrived_bytes = 0;
     uint32_t serial = 0;           // of the last run that raised flags
     // The launches of a run, kept as graphs: their parameters depend on the workspace, on the kind of rows, on how they
-    // arrive and on the grid's rows (a power of two, or max_rows) alone, so that any weights and routes can use them.  A
+    // arrive and on the grid's rows (moe_row_plan) alone, so that any weights and routes can use them.  A
     // graph is made at the second run of its kind: a state that runs once does not pay for it.
     struct Kept { bool seen = false, failed = false; cudaGraphExec_t exec = nullptr; };
     Kept kept[2][2][9];            // [fp32 rows][read from host memory][log2 of the grid's rows]
@@ -426,7 +423,8 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
             u.serial = ws->serial;
         }
         const size_t row_bytes = values * (f32 ? 4 : 1);
-        const bool pull = row_bytes <= MOE_PULL_MOST;
+        const MoeRowPlan plan = moe_row_plan(rows, c.max_rows, H, f32);
+        const bool pull = plan.pull;
         if (pull) stage_rows(ws->host_upload + ws->input_at, input, row_bytes);
         t.schedule_us = since_us(at);
         at = Clock::now();
@@ -450,10 +448,7 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
             if (timings) *timings = t;
             return RK_NPU_OK;
         }
-        int level = 0;
-        while ((1 << level) < rows) ++level;
-        const int grid_rows = std::min(1 << level, c.max_rows);
-        ok = ok && ((!timings && launch_kept(*ws, f32, pull, grid_rows, level)) || launch_run(*ws, f32, pull, grid_rows, true, timings ? ws->events : nullptr));
+        ok = ok && ((!timings && launch_kept(*ws, f32, pull, plan.grid_rows, plan.level)) || launch_run(*ws, f32, pull, plan.grid_rows, true, timings ? ws->events : nullptr));
         at = Clock::now();
         // int8 rows are not judged on the device, so a large result can follow its kernel at once
         if (ok && !direct && !f32) ok = cudaMemcpyAsync(output, ws->out, values * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
@@ -658,7 +653,7 @@ rk_npu_moe_w8_workspace* workspace_create(rk_npu_iommu_domain* domain, const rk_
          !device_alloc(domain, reinterpret_cast<void**>(&ws->upload), ws->upload_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->arrived), ws->arrived_bytes);
     ok = ok && cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess &&
-         cudaHostAlloc(reinterpret_cast<void**>(&ws->host_upload), ws->input_at + std::min(size_t(rows) * H * 4, std::max(MOE_PULL_MOST, size_t(H) * 4)), cudaHostAllocMapped) == cudaSuccess &&
+         cudaHostAlloc(reinterpret_cast<void**>(&ws->host_upload), ws->input_at + moe_piece_row_bytes(rows, H), cudaHostAllocMapped) == cudaSuccess &&
          cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws->host_upload_alias), ws->host_upload, 0) == cudaSuccess &&
          cudaHostAlloc(reinterpret_cast<void**>(&ws->host_status), sizeof(Status) + ws->arrived_bytes, cudaHostAllocMapped) == cudaSuccess &&
          cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws->host_status_alias), ws->host_status, 0) == cudaSuccess;

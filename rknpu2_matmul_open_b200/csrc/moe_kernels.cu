@@ -123,8 +123,9 @@ __global__ void __launch_bounds__(256) moe_pack_kernel(const MoePackParams p)
 
 // ------------------------------------------------------------------ intake (fp32 rows -> codes: src/rk_npu_moe_w8.cpp:317-343)
 // Blocks below row_blocks take a row each; the others carry the rest of a piece that is still in host memory (header and
-// schedule) to the device.  Nothing is asked of the header where that can be avoided: a row is requested before the header is known to name it (a piece always has room for every row
-// of the grid) and stays in registers between its maximum and its codes: one trip over the bus, not three.
+// schedule) to the device.  Nothing is asked of the header where that can be avoided: an fp32 row is requested before the
+// header is known to name it (moe_row_plan keeps every row of the grid inside the piece) and stays in registers between its
+// maximum and its codes: one trip over the bus, not three.
 constexpr int MOE_INTAKE_THREADS = 256, MOE_INTAKE_MOVERS = 8;
 constexpr int MOE_INTAKE_BLIND = MOE_INTAKE_MOVERS * MOE_INTAKE_THREADS * 16;    // moved without asking how much of it is in use
 __global__ void __launch_bounds__(MOE_INTAKE_THREADS) moe_intake_kernel(const MoeIntakeParams p)

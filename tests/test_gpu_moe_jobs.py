@@ -44,3 +44,34 @@ def test_jobs_items_and_stages(gpu, oracle, form, H, I, E):
             assert np.array_equal(bits(out), bits(ref)), rows
     ws.free()
     w.free()
+
+
+def test_fewer_rows_than_the_workspace_holds(gpu, oracle):
+    # a workspace for 256 rows: batches whose rows still fit the page-locked piece although a power of two of them would not
+    # (85 rows of 1536 floats do, 86 do not), and those on either side
+    _, dom, _ = gpu
+    H, I, E = 1536, 32, 4
+    rng = np.random.default_rng(7)
+    ex = dict(gate_up=rng.integers(-128, 128, size=(E, H, 2 * I), dtype=np.int8),
+              gate_up_scales=rng.uniform(2e-4, 6e-4, size=(E, 2 * I)).astype(np.float32),
+              down=rng.integers(-128, 128, size=(E, I, H), dtype=np.int8),
+              down_scales=rng.uniform(1e-3, 3e-3, size=(E, H)).astype(np.float32))
+    w = moe.MoeWeights(dom, shared_expert=0, form="w8", **ex)
+    ws = moe.MoeWorkspace(dom, moe.default_config(H, I, E, 0, 2, 256), form="w8")
+    for rows in (64, 65, 70, 85, 86, 128, 129, 256, 70):
+        x = rng.standard_normal((rows, H)).astype(np.float32)
+        ids = np.stack([np.arange(rows) % E, (np.arange(rows) + 1) % E], axis=1).astype(np.int32)
+        routes = rng.uniform(0.05, 0.95, size=(rows, 2)).astype(np.float32)
+        rc, q, s = oracle.moe_quantize_rows(x)
+        assert rc == 0
+        rc, ref = oracle.moe_run(ex, 0, 2, q, s, ids, routes, mode=1)
+        assert rc == 0
+        for _ in range(3):
+            out = np.full((rows, H), -1, np.float32)
+            assert ws.run_f32(w, x, ids, routes, out) == 0
+            assert np.array_equal(bits(out), bits(ref)), rows
+            out.fill(-1)
+            assert ws.run_quantized(w, q, s, ids, routes, out) == 0
+            assert np.array_equal(bits(out), bits(ref)), rows
+    ws.free()
+    w.free()

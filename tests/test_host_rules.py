@@ -1,0 +1,43 @@
+"""Rules that size and route launches, as host arithmetic: compiled from the library's own headers and checked over their
+whole range without a GPU."""
+import subprocess
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "rknpu2_matmul_open_b200" / "csrc"
+
+
+def _run(tmp_path, body):
+    (tmp_path / "rule.cpp").write_text(body)
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", "-Wall", f"-I{CSRC}", "-o", str(tmp_path / "rule"), str(tmp_path / "rule.cpp")], check=True)
+    out = subprocess.run([str(tmp_path / "rule")], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout
+
+
+def test_expert_rows_are_read_inside_the_piece_that_holds_them(tmp_path):
+    # the intake kernel requests an fp32 row for every block of its grid, whether the run has that row or not
+    _run(tmp_path, r"""
+#include "moe_rows.h"
+#include <initializer_list>
+#include <stdio.h>
+using namespace rkb200;
+#define CHECK(x) do { if (!(x)) { printf("%s: H %d max_rows %d rows %d f32 %d\n", #x, H, most, rows, f32); return 1; } } while (0)
+int main()
+{
+    for (int H : {64, 96, 512, 544, 1024, 1536, 1984, 2048, 2400, 4064, 4096, 7168, 8128, 8192})
+        for (int most = 1; most <= 256; ++most)
+            for (int f32 = 0; f32 < 2; ++f32) {
+                int grid[2][9] = {};
+                for (int rows = 1; rows <= most; ++rows) {
+                    const MoeRowPlan p = moe_row_plan(rows, most, H, f32);
+                    const size_t bytes = size_t(f32 ? 4 : 1) * H, piece = moe_piece_row_bytes(most, H);
+                    CHECK(p.grid_rows >= rows && p.grid_rows <= most && p.level >= 0 && p.level <= 8);
+                    CHECK(!p.pull || rows * bytes <= piece);                       // what the host stages
+                    CHECK(!p.pull || !f32 || p.grid_rows * bytes <= piece);       // what the kernel may request
+                    int& kept = grid[p.pull][p.level];                            // the launches of a kind are kept
+                    CHECK(kept == 0 || kept == p.grid_rows);
+                    kept = p.grid_rows;
+                }
+            }
+    return 0;
+}
+""")
