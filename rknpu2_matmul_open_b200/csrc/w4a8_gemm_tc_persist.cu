@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     } else if (warp == 3) {
         // ---------------------------------------------------------------- activation voucher
         // The leader's MMAs read both CTAs' activations: this warp passes on that this CTA's copy has landed.  It runs
-        // ahead of the MMAs by the depth of the ring.  (When the unpack warps vouched for it, with a release at cluster
-        // scope, that release bounded the whole loop: 730 cycles per k-block at K = 11008 against 525 now.)
+        // ahead of the MMAs by the depth of the ring.  (When the unpack warps vouched for it, with an arrival that released
+        // everything at cluster scope, that release bounded the whole loop: 730 cycles per k-block at K = 11008 against 525.)
         if (dependency_met() && lane == 0) {
             RingPos<S::XA> r;
             long long waited = 0;

@@ -42,6 +42,26 @@ def test_linear(gpu, oracle, monkeypatch, shape):
     w.free()
 
 
+@pytest.mark.parametrize("shape", [(50, 8192, 256), (190, 4096, 384), (250, 1152, 1024), (450, 640, 512), (1000, 2176, 256)], ids=lambda s: "x".join(map(str, s)))
+def test_new_activations_in_the_same_buffers(gpu, oracle, monkeypatch, shape):
+    # the leader's MMAs read both CTAs' activations: a launch that ran ahead of the peer's copy would multiply the rows of
+    # the launch before (other rows every time, the same buffers)
+    _, dom, _ = gpu
+    M, K, N = shape
+    monkeypatch.setenv("RK_NPU_B200_VARIANT", "2")
+    B, sw = make_weights(K, N, seed=K + N)
+    w, ws = rk.Weights(dom, B, sw), rk.Workspace(dom, rk.default_config(M, N, K))
+    rows = [make_activations(M, K, seed=s, dtype="f16") for s in range(4)]
+    refs = [oracle.linear(A, B, sw)[1] for A in rows]
+    out = np.zeros((M, N), np.uint16)
+    for turn in range(24):
+        out.fill(0x7C00)
+        assert ws.run_f16(w, rows[turn % 4], out) == 0
+        assert np.array_equal(out, refs[turn % 4]), turn
+    ws.free()
+    w.free()
+
+
 @pytest.mark.parametrize("shape", [(33, 512, 128, 300), (64, 8192, 192, 130), (128, 4096, 320, 512), (130, 1024, 2496, 257), (520, 640, 1280, 2048)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_ffn(gpu, oracle, monkeypatch, shape):
