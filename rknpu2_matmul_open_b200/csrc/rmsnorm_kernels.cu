@@ -36,10 +36,19 @@ constexpr int RN_CTAS = 2;      // CTAs per SM the register allocation is bounde
 constexpr int RN_MAX_DEVICES = 64;
 constexpr int RN_SMEM_SUMS = 64 * 1024;   // most bytes of sums one CTA keeps: TM * ceil(D/8/CS) * 16
 
+// (x and the residual of a kernel that starts behind the one in front, and is not launched before that has finished)
 __device__ __forceinline__ uint4 ld_stream(const uint4* p)
 {
     uint4 v;
     asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+// The same for a kernel that may start before the one in front has finished writing what it reads: a coherent load that the
+// compiler leaves behind the dependency wait.
+__device__ __forceinline__ uint4 ld_dependent(const uint4* p)
+{
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ void st_stream(uint4* p, const uint4& v)
@@ -206,8 +215,8 @@ __global__ void __launch_bounds__(RN_THREADS) add_rmsnorm_row_kernel(AddRmsNormP
             const int j = jl + u * JL;
             if (live && j < chunks) {
                 const size_t at = global_at(j);
-                sum[u] = ld_stream(p.x + at);
-                b[u] = ld_stream(p.residual + at);
+                sum[u] = ld_dependent(p.x + at);
+                b[u] = ld_dependent(p.residual + at);
             }
         }
 #pragma unroll
