@@ -7,6 +7,7 @@
 // order :83-94, BUSY guard :70-81, run :98-159, accounting :169-207, FFN :354-380) and
 // the backend geometry rules src/rk_npu_i4_plan.cpp:14-87.
 #include "../../include/rknpu_b200_quant.h"
+#include "w4a8_rules.h"
 #include "w4a8_tune.h"
 #include <algorithm>
 #include <cerrno>
@@ -626,17 +627,11 @@ int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const vo
     }
     // The verdict of a call lands in page-locked memory by itself (plain stores of the kernels), and so does a small
     // result: straight in the caller's tensor when that is page-locked, else in the workspace's piece, from where the host
-    // copies it out.  (The activations are still copied in: every CTA reads them.)  The single-kernel families write
-    // every element once, in rows as long as a warp; the others in pieces of 64 bytes, which the bus takes more slowly, so
-    // that from 128 KB on the copy engine is as fast.
-    // Rows that do not start on a sector leave it in pieces of sectors: beyond 40 KB of binary16 and 64 KB of
-    // words these are copied (13 x 4910 binary16 64 against 38 us, 13 x 4912 34; 3 x 4911 fp32 27 against 36).
+    // copies it out.  (The activations are still copied in: every CTA reads them.)
     // (Not when the caller asks for stage timings: the device part of a call must not contain stores that cross the bus,
     // or the figures of different kernel families -- which the search tuner ranks -- stop being comparable.)
     const bool own_report = !grouped(*ws) && !metrics && ws->host_status_alias;
-    const bool single_kernel = ws->variant == 3 || ws->variant == 5;
-    const bool bus_result = !c_dev && own_report && epi != EPI_SWIGLU && out_bytes <= (single_kernel ? size_t(512) << 10 : size_t(128) << 10) &&
-                            (cfg.M == 1 || out_bytes / cfg.M % 32 == 0 || out_bytes <= (epi == EPI_F16 ? size_t(40) << 10 : size_t(64) << 10));
+    const bool bus_result = !c_dev && own_report && epi != EPI_SWIGLU && result_over_bus(ws->variant, cfg.M, size_t(out_cols), epi == EPI_F16 ? 2 : 4);
     void* c_alias = bus_result ? c_at.alias : nullptr;
     const bool bounce_out = bus_result && !c_alias && ws->bounce_out.alias && out_bytes <= ws->bounce_out.bytes;
     if (bounce_out) c_alias = ws->bounce_out.alias;
@@ -1223,7 +1218,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
         const size_t in_most = size_t(cfg->M) * cfg->K * 4, out_most = size_t(cfg->M) * cfg->N * 4;
         if (cfg->M <= 128) {
             ws->bounce_in = host_piece_acquire(ctx, std::min(in_most, BOUNCE_IN));
-            ws->bounce_out = host_piece_acquire(ctx, std::min(out_most, BOUNCE_OUT));
+            ws->bounce_out = host_piece_acquire(ctx, std::min(out_most, variant == 3 || variant == 5 ? RESULT_OVER_BUS_MOST : BOUNCE_OUT));
         }
     }
     if (!ok) { cudaGetLastError(); workspace_destroy(ws); return nullptr; }

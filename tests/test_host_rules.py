@@ -41,3 +41,25 @@ int main()
     return 0;
 }
 """)
+
+
+def test_results_that_the_kernel_stores_over_the_bus(tmp_path):
+    # sizes at which copying and storing were both measured; the faster one is the rule's
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+struct Case { int family, M, cols, elem; bool store; };
+int main()
+{
+    const Case cases[] = {
+        {5, 4, 4911, 4, true}, {5, 3, 7001, 2, true}, {5, 4, 14330, 4, true}, {5, 8, 4911, 4, true}, {5, 8, 14331, 4, true}, {5, 1, 4911, 2, true},
+        {3, 8, 2900, 2, true}, {3, 8, 2900, 4, true}, {3, 8, 28672, 4, true}, {3, 8, 9984, 4, true},
+        {3, 8, 4911, 2, false}, {3, 8, 9998, 4, false}, {3, 5, 14330, 2, false}, {3, 8, 40000, 4, false},
+        {1, 13, 4912, 2, true}, {1, 13, 4910, 2, false}, {2, 64, 1024, 2, true}, {2, 64, 2048, 2, false},
+    };
+    for (const Case& c : cases)
+        if (result_over_bus(c.family, c.M, size_t(c.cols), size_t(c.elem)) != c.store) { printf("family %d %d x %d x %d\n", c.family, c.M, c.cols, c.elem); return 1; }
+    return 0;
+}
+""")
