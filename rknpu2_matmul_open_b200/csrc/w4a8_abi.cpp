@@ -315,6 +315,7 @@ struct Call {
     const int8_t* codes_in = nullptr;   // activations arrive as int8 codes [parts][M][K/parts]; scales from rowmax_in
     int parts = 1;
     Status* status = nullptr;   // page-locked block the call's verdict goes to (default: the workspace's device block)
+    bool over_bus = false;      // dOut is page-locked host memory
 };
 
 // Split-K factor (= cluster size) of the single-kernel path: the largest split whose CTAs
@@ -353,6 +354,13 @@ int fused_tiles_per_cta(const rk_npu_w4a8_workspace& ws, int tiles, int split, i
     const size_t all = size_t(tiles) * split * (gemm_fused_smem_bytes(ws.TC, stages, 1) + 1024);
     const size_t half_gpu = size_t(ws.domain->ctx->sm_count) * (220 * 1024) / 2;
     return all > half_gpu ? 2 : 1;
+}
+
+// The family that runs a call: the workspace's, or the ring where that is the faster for these rows (its code layout is the
+// same).  Results that go over the bus stay with the single launch, which stores them in whole rows.
+int family_of(const rk_npu_w4a8_workspace& ws, const Call& c)
+{
+    return ws.mid_batch && c.epi != EPI_SWIGLU && !c.rowmax_in && !c.over_bus && mid_batch_takes_ring(ws.config.M, ws.config.K, c.half) ? 1 : ws.variant;
 }
 
 // Launch parameters of the decode kernel for one call (its workspace runs that family).
@@ -395,7 +403,8 @@ int enqueue(const Call& c)
     const int F = c.epi == EPI_SWIGLU ? N / 2 : 0;
     const int tiles = c.epi == EPI_SWIGLU ? (F + 63) / 64 : (N + TILE_N - 1) / TILE_N;
     const unsigned long long timeout_ns = (unsigned long long)cfg.timeout_ms * 1000000ull;
-    if (ws.variant == 5 && !c.codes_in) {
+    const int family = family_of(ws, c);
+    if (family == 5 && !c.codes_in) {
         // One kernel, whole-K CTAs: scan + quantise (shared by a cluster) + GEMM + epilogue.
         DecodeParams d{};
         decode_params(c, d);
@@ -405,7 +414,7 @@ int enqueue(const Call& c)
         ws.launches.fetch_add(1, std::memory_order_relaxed);
         return RK_NPU_OK;
     }
-    if (ws.variant == 3 && !c.codes_in) {
+    if (family == 3 && !c.codes_in) {
         // One kernel: scan + quantise + GEMM + epilogue.
         FusedParams f{};
         f.Wp = c.w->packed;
@@ -494,7 +503,8 @@ int enqueue(const Call& c)
         g.counts = ws.counts;
         err = launch_gemm_stream(g, ws.domain->ctx->sm_count, c.stream, pdl);
     } else {
-        // (a single-kernel workspace given codes runs the ring GEMM; its split override may be odd, so it is not used here)
+        // (a single-kernel workspace runs the ring GEMM where it is given codes or family_of says so; its split override may
+        // be odd, so it is not used here)
         g.split = (ws.variant == 3 || ws.variant == 5) ? pick_split_auto(ws, tiles, (cfg.M + ws.TC - 1) / ws.TC)
                                   : pick_split(ws, tiles, (cfg.M + ws.TC - 1) / ws.TC);
         err = launch_gemm_mma(g, ws.TC, c.stream, pdl);
@@ -642,6 +652,7 @@ int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const vo
     t.sync_us += elapsed_us(copy_start);
     Call call{ws, w, dA, dC, half, epi, nullptr, nullptr, s, metrics ? ws->events : nullptr, epi == EPI_I32};
     call.status = status_alias;
+    call.over_bus = c_alias != nullptr;
     int rc = enqueue_linear(call, dC);
     if (rc) { cudaStreamSynchronize(s); return rc; }
     copy_start = Clock::now();
@@ -1130,7 +1141,8 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     const bool decode_ok = gemm_decode_supported(cfg->M, cfg->K);
     const bool decode_best = decode_ok && (cfg->M <= 4 || !fused_best);
     // 9..16 tokens: one launch (the split-K kernel) beats two (the ring) while the weights are small (16 tokens, 4096 ->
-    // 4096 9.6 against 10.0 us, 8192 -> 1024 8.5 against 10.6, 11008 -> 4096 17.2 against 14.1).
+    // 4096 9.6 against 10.0 us, 8192 -> 1024 8.5 against 10.6, 11008 -> 4096 17.2 against 14.1); not for all rows, see
+    // mid_batch_takes_ring.
     const bool fused_mid = fused_ok && cfg->M > 8 && cfg->M <= 16 && (long long)cfg->K * local_N / 2 <= (8ll << 20);
     // From 17 tokens on the persistent tcgen05 kernel, whose time hardly depends on the batch up to 64 (4096 -> 4096 13 us,
     // 11008 -> 4096 19, 4096 -> 14336 14.5), unless its 256-channel tiles are so few that the ring's small CTAs cover more
@@ -1142,6 +1154,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (forced == 1 || (forced == 2 && tc_ok) || (forced == 3 && fused_ok) || (forced == 4 && stream_ok) || (forced == 5 && decode_ok))
         variant = forced;
     ws->variant = variant;
+    ws->mid_batch = variant == 3 && forced != 3 && fused_mid;
     if (const char* e = std::getenv("RK_NPU_B200_TILES_PER_CTA")) {   // experiments and tests: 1 or 2, else automatic
         const int v = std::atoi(e);
         ws->tiles_per_cta_override = (v == 1 || v == 2) ? v : 0;
@@ -1583,6 +1596,7 @@ extern "C" int rk_npu_b200_w4a8_set_schedule(rk_npu_w4a8_workspace* ws, int vari
     if (!lock) return RK_NPU_ERR_BUSY;
     ws->variant = target;
     ws->split_override = split_k;
+    if (variant) ws->mid_batch = false;      // asked for by name
     return RK_NPU_OK;
 }
 extern "C" int rk_npu_b200_w4a8_schedule(const rk_npu_w4a8_workspace* ws, int* variant, int* split_k)

@@ -24,4 +24,18 @@ inline bool result_over_bus(int family, int M, size_t cols, size_t elem)
     return bytes <= (elem == 2 ? size_t(40) << 10 : size_t(64) << 10);
 }
 
+// 9..16 tokens of small weights: whether one launch (the split-K kernel, whose every cluster scans all of the rows) is left for
+// two (quantise, ring).  For binary16 rows that allow 16-byte loads one launch is the faster at every count (16 tokens, 4096 ->
+// 4096 10.2 us against 11.0, 4096 -> 1024 8.4 against 9.5, 1024 -> 14336 9.6 against 9.9; at worst 5504 -> 2112 10.7 against
+// 10.2).  fp32 rows are twice the scan: 13 tokens and more take two (13 tokens 2048 -> 2048 9.3 against 8.7, 4096 -> 4096 11.7
+// against 10.4, 16 tokens 2048 -> 8192 12.3 against 9.7; 12 tokens 8.8 against 8.7, 4096 -> 1024 8.4 against 9.3).  Rows that
+// are loaded element by element sooner still: binary16 from 11 tokens (10 tokens 1500 -> 2048 7.9 against 9.5, 2044 -> 4096
+// 11.6 against 11.0; 12 tokens 3070 -> 4911 13.1 against 11.5, 16 tokens 15.9 against 11.7), fp32 from 9 (3070 -> 4911 16.6
+// against 12.1, 1025 -> 1024 11.5 against 9.6).
+inline bool mid_batch_takes_ring(int M, int K, bool half)
+{
+    const bool wide = K % 8 == 0;
+    return half ? !wide && M > 10 : M > (wide ? 12 : 8);
+}
+
 } // namespace rkb200

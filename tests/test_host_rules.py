@@ -63,3 +63,24 @@ int main()
     return 0;
 }
 """)
+
+
+def test_rows_that_leave_the_single_launch_at_mid_batches(tmp_path):
+    # the faster of the two forms where both were measured and differ by more than 3 %
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+struct Case { int M, K; bool half, ring; };
+int main()
+{
+    const Case cases[] = {
+        {9, 4096, true, false}, {16, 4096, true, false}, {16, 1024, true, false}, {9, 1500, true, false}, {12, 2044, true, true}, {16, 3070, true, true},
+        {16, 1025, true, true}, {9, 4096, false, false}, {9, 1024, false, false}, {13, 4096, false, true}, {16, 2048, false, true}, {16, 8192, false, true},
+        {9, 2044, false, true}, {9, 3070, false, true}, {12, 1500, false, true}, {9, 1025, false, true},
+    };
+    for (const Case& c : cases)
+        if (mid_batch_takes_ring(c.M, c.K, c.half) != c.ring) { printf("%d x %d half %d\n", c.M, c.K, c.half); return 1; }
+    return 0;
+}
+""")
