@@ -121,7 +121,7 @@ struct RowQuant {
     }
 };
 template <bool HALF, int TG, bool SCAN, int BS, int UN>
-__global__ void __launch_bounds__(BS, (UN == 4 ? 2048 : 1024) / BS) quantize_rows_kernel(const QuantParams p)
+__global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) quantize_rows_kernel(const QuantParams p)
 {
     pdl_launch_dependents();   // the GEMM behind this kernel may start prefetching weights
     pdl_wait();                // A may be the output of the kernel in front of this one

@@ -1,7 +1,7 @@
 // w4a8_quantize.cuh -- activation rows -> int8 codes in the Xq layout, for rows that allow 16-byte loads.
 //
-// Byte work: every element is read once and a code is written for it.  A CTA owns TG tokens (neighbours in their token
-// tile) and keeps what it has read in registers between the maximum and the codes; only what exceeds a thread's UN loads is
+// Byte work: every element is read once and a code is written for it.  A CTA owns TG tokens (one or two, neighbours in their
+// token tile) and keeps what it has read in registers between the maximum and the codes; only what exceeds a thread's UN loads is
 // read a second time.  Lanes are dealt so that both sides move whole sectors: a warp's load covers 512 / TG contiguous bytes
 // of each token's row, and the store that follows puts the TG tokens' 16-byte units, which are neighbours in the layout,
 // side by side.  (One CTA per token with a thread per 16-element unit loaded every row twice, each load at a stride of 32 or
@@ -100,9 +100,18 @@ __device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int M,
 template <bool HALF>
 inline bool quantize_rows_ok(const void* A, int K, int T) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % QuantRows<HALF, 1>::EPW == 0 && T % 2 == 0; }
 // Calls f with the shape of the launch: <tokens per CTA, threads, loads a thread keeps>.
-// Two tokens per CTA once that leaves two CTAs per SM; below, a token per CTA spreads the rows over more SMs, and all the
-// threads that help with a row work on it.  There, four loads a thread and 32 registers where these hold the rows (or nothing
-// has to be held): twice the CTAs on an SM, in different phases (4096 x 14336 fp32 with known maxima 70 -> 60 us).
+// Rows that are scanned.  Up to 296 tokens (two CTAs of 512 threads an SM, all resident) a token per CTA, and all the
+// threads that help with a row work on it.  Up to 591 these CTAs would come in two waves: 256 threads (in front of 4096
+// channels 448 x 1024 binary16 13.8 -> 12.1 us, 448 x 4096 fp32 18.4 -> 16.9), but not for long fp32 rows, whose CTAs take
+// twice as long then (300 x 11008 -> 4096 28.0 us, 29.5 with 256; FFN of 400 x 8192 54.7 and 56.7). From 592 tokens on
+// binary16 rows of up to 4096 elements take 128 threads with two loads and 32 registers, sixteen CTAs an SM (in front of
+// 4096 channels 3000 x 1024 32.2 -> 28.8 us, 1024 x 4096 27.3 -> 25.8); the others two tokens per CTA, which make whole
+// sectors of codes (6144 and 8192 binary16 -6 to -10 % against a token per CTA).  (The two fp32 forms of eight loads and two
+// tokens spill six words.)
+// Rows whose maxima are known: two tokens per CTA, up to 591 tokens of 512 threads (FFN of 64 x 1024 -> 2 x 2048 24.2 ->
+// 21.6 us, of 591 x 4096 -> 2 x 14336 116 -> 103), beyond of 256 with 32 registers (4096 x 14336 fp32 60 us, 70 with twice
+// the registers).  Few long rows want a CTA each (20 x 11008 40.3 us against 42.3,
+// 20 x 4096 26.8 against 27.6).
 template <bool HALF, bool SCAN, class F>
 inline auto with_quantize_rows_shape(int M, int K, F f)
 {
@@ -112,11 +121,20 @@ inline auto with_quantize_rows_shape(int M, int K, F f)
     using I2 = integral_constant<int, 2>;
     using I4 = integral_constant<int, 4>;
     using I8 = integral_constant<int, 8>;
+    using B128 = integral_constant<int, 128>;
     using B256 = integral_constant<int, 256>;
     using B512 = integral_constant<int, 512>;
-    if (M < 4 * 148) return f(I1{}, B512{}, I8{});
-    if (!SCAN || K <= 256 * 4 * EPW / 2) return f(I2{}, B256{}, I4{});
-    return K <= 256 * 8 * EPW / 2 ? f(I2{}, B256{}, I8{}) : f(I2{}, B512{}, I8{});
+    if constexpr (!SCAN) {
+        if (M >= 592) return f(I2{}, B256{}, I4{});
+        return (M <= 296 && K > 8192) || (M < 24 && K >= 4096) ? f(I1{}, B512{}, I8{}) : f(I2{}, B512{}, I8{});
+    } else {
+        if (M <= 296) return f(I1{}, B512{}, I8{});
+        if (M < 592) return HALF || K < 8192 ? f(I1{}, B256{}, I8{}) : f(I1{}, B512{}, I8{});
+        if constexpr (HALF) {
+            if (K <= 4096) return f(I1{}, B128{}, I2{});
+        } else if (K <= 2048) return f(I2{}, B256{}, I4{});
+        return K <= 256 * 8 * EPW / 2 ? f(I2{}, B256{}, I8{}) : f(I2{}, B512{}, I8{});
+    }
 }
 
 } // namespace rkb200

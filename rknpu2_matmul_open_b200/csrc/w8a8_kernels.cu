@@ -95,7 +95,7 @@ struct W8RowQuant {
     }
 };
 template <bool HALF, int TG, bool SCAN, int BS, int UN>
-__global__ void __launch_bounds__(BS, (UN == 4 ? 2048 : 1024) / BS) w8_quantize_rows_kernel(const W8QuantParams p)
+__global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) w8_quantize_rows_kernel(const W8QuantParams p)
 {
     pdl_launch_dependents();   // the GEMM behind this kernel may set itself up and request its weights
     W8RowQuant<HALF> op{p};

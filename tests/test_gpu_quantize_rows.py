@@ -1,5 +1,5 @@
-"""Activation rows to int8 codes at the edges of the row kernel: one and two tokens per CTA and an odd last one, both block
-sizes, rows shorter than one step of a CTA, rows that just fill a thread's registers and rows beyond them, a ragged last
+"""Activation rows to int8 codes at the edges of the row kernel: one and two tokens per CTA and an odd last one, every block
+size on either side of its lines, rows shorter than one step of a CTA, rows that just fill a thread's registers and rows beyond them, a ragged last
 unit, rows that do not allow 16-byte loads; one non-finite element among many rows; collected row maxima against scanned
 ones.  Codes, scales and results bit for bit."""
 import numpy as np
@@ -22,7 +22,8 @@ def rows(M, K, seed):
     return a
 
 
-@pytest.mark.parametrize("M, K", [(17, 36), (17, 8200), (18, 16392), (33, 533), (129, 4096), (592, 128), (593, 4096), (593, 4100), (601, 8200)])
+@pytest.mark.parametrize("M, K", [(17, 36), (17, 8200), (18, 16392), (33, 533), (129, 4096), (592, 128), (593, 4096), (593, 4100), (601, 8200),
+                                  (296, 1032), (297, 1032), (297, 8184), (297, 8192), (297, 8200), (591, 2056), (592, 2048), (592, 2056), (592, 4096), (592, 4104)])
 def test_codes_and_scales(gpu, oracle, M, K):
     _, dom, _ = gpu
     rng = np.random.default_rng(K)
@@ -47,7 +48,7 @@ def test_codes_and_scales(gpu, oracle, M, K):
     w.free()
 
 
-@pytest.mark.parametrize("M, K, F", [(17, 64, 96), (594, 64, 4352)])
+@pytest.mark.parametrize("M, K, F", [(17, 64, 96), (594, 64, 4352), (296, 64, 8256), (297, 64, 8256), (591, 64, 160), (23, 64, 4096), (24, 64, 4096)])
 def test_collected_maxima_give_the_scanned_codes(gpu, M, K, F):
     _, dom, _ = gpu
     rng = np.random.default_rng(F)
