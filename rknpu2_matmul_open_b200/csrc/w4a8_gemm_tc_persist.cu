@@ -20,6 +20,7 @@
 // collected).
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
+#include "w4a8_rules.h"
 #include "w4a8_ptx.cuh"
 #include "w4a8_tc.cuh"
 #include <algorithm>
@@ -718,7 +719,7 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
     if (setup || !max_clusters) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
         if (e != cudaSuccess) return e;
-        // how many CTA pairs can be resident at once: the grid is at most that many
+        // how many CTA pairs can be resident at once
         cfg.gridDim = dim3(2, 1, 1);
         cfg.attrs = attr;
         cfg.numAttrs = 1;
@@ -729,8 +730,7 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
         if (device >= 0 && device < 64) { clusters_of_device[device] = n; configured.mark(device); }
     }
     const int tiles = gemm_tc_persist_tiles(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, TOK);
-    if (p.split > 1 && tiles * p.split > max_clusters) return cudaErrorInvalidValue;
-    const int clusters = p.split > 1 ? tiles * p.split : std::min(tiles, max_clusters);
+    const int clusters = persist_clusters(tiles, p.split, max_clusters);
     cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
     int n = 1;
     if (pdl) {

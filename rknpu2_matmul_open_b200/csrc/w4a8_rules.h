@@ -38,4 +38,13 @@ inline bool mid_batch_takes_ring(int M, int K, bool half)
     return half ? !wide && M > 10 : M > (wide ? 12 : 8);
 }
 
+// CTA pairs of a persistent launch: one per part where tiles are cut along K (no part waits for another, the last to arrive
+// finishes the tile, so more pairs than are resident at once run in turn), else at most as many as can be resident, each
+// with a run of whole tiles.
+inline int persist_clusters(int tiles, int split, int resident)
+{
+    if (split > 1) return tiles * split;
+    return tiles < resident ? tiles : resident;
+}
+
 } // namespace rkb200

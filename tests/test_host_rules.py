@@ -84,3 +84,25 @@ int main()
     return 0;
 }
 """)
+
+
+def test_tiles_in_parts_are_launched_whatever_can_be_resident(tmp_path):
+    # a plan is made for half of the SMs in pairs; where fewer pairs can be resident its parts still all run
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+int main()
+{
+    for (int resident = 1; resident <= 76; ++resident)
+        for (int tiles = 1; tiles <= 200; ++tiles)
+            for (int split = 1; split <= 8; ++split) {
+                const int clusters = persist_clusters(tiles, split, resident);
+                if (split > 1 ? clusters != tiles * split : clusters < 1 || clusters > resident || clusters > tiles || (clusters < resident && clusters != tiles)) {
+                    printf("%d tiles in %d parts, %d resident: %d\n", tiles, split, resident, clusters);
+                    return 1;
+                }
+            }
+    return 0;
+}
+""")
