@@ -20,7 +20,8 @@ using namespace rkb200;
 
 namespace {
 constexpr int W8_N_TILE_MAX = 3072, W8_CHANNEL_TILE = 32;   // src/rk_npu_quant_matmul.cpp:50, src/rk_npu_internal.h:123
-constexpr int QUERY_SMS = 148;                               // the memory query has no device to ask: this GPU's SM count
+// The SMs a plan is made for, whatever the device: the memory query has none to ask and has to agree with the workspace.
+constexpr int PLAN_SMS = 148;
 constexpr uint32_t W8_TIMEOUT_MS = 500;                      // the original's fixed plan timeout (src/rk_npu_quant_matmul.cpp:1709)
 
 struct W8Weights {
@@ -97,11 +98,11 @@ struct Sizes {
     int T, KB, NG, parts;
     size_t codes, partials, counts, scales, stage_in, stage_out, packed, wscales;
 };
-Sizes sizes_of(int M, int N, int K, int kind, int sm_count)
+Sizes sizes_of(int M, int N, int K, int kind)
 {
     Sizes z{};
     z.KB = (K + KBLOCK - 1) / KBLOCK;
-    const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, false, sm_count);
+    const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, false, PLAN_SMS);
     z.T = plan.tok / 2;
     z.parts = plan.split;
     z.NG = align_up((N + GROUP - 1) / GROUP, 8) + 8;   // zero groups behind the last tile, as for the int4 weights
@@ -143,7 +144,7 @@ int weights_prepare(W8Weights& w, rk_npu_iommu_domain* domain, const rk_npu_matm
     rk_npu_ctx* ctx = domain->ctx;
     if (ctx->world > 1 || !runnable_shape(1, config->N, config->K)) return RK_NPU_ERR_PARAM;
     if (cudaSetDevice(ctx->device) != cudaSuccess) return RK_NPU_ERR_SUBMIT;
-    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32, ctx->sm_count);
+    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32);
     w.config = *config;
     w.KB = z.KB;
     w.NG = z.NG;
@@ -296,7 +297,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
 int weights_memory_query(const rk_npu_matmul_weight_config* config, bool with_scale, rk_npu_matmul_weight_requirements* out)
 {
     if (!valid_weight_config(config) || !out || !runnable_shape(1, config->N, config->K)) return RK_NPU_ERR_PARAM;
-    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32, QUERY_SMS);
+    const Sizes z = sizes_of(1, config->N, config->K, RK_NPU_MATMUL_I8I8I32);
     std::memset(out, 0, sizeof(*out));
     out->packed_b_bytes = z.packed;
     out->scale_bytes = with_scale ? uint64_t(config->N) * sizeof(float) : 0;   // the logical payload, as the original counts it
@@ -322,7 +323,7 @@ extern "C" int rk_npu_matmul_k_partition_query(int M, int K, int k_tile)
 extern "C" int rk_npu_matmul_workspace_memory_query(const rk_npu_matmul_strategy* strategy, rk_npu_matmul_workspace_requirements* out)
 {
     if (!strategy || !out || !valid_strategy(strategy) || !runnable_shape(strategy->M, strategy->N, strategy->K)) return RK_NPU_ERR_PARAM;
-    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind), QUERY_SMS);
+    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind));
     std::memset(out, 0, sizeof(*out));
     out->input_bytes = z.codes + z.stage_in;
     out->output_bytes = z.stage_out;
@@ -345,7 +346,7 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     if (cudaSetDevice(ctx->device) != cudaSuccess) return nullptr;
     rk_npu_matmul_workspace* ws = new (std::nothrow) rk_npu_matmul_workspace();
     if (!ws) return nullptr;
-    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind), ctx->sm_count);
+    const Sizes z = sizes_of(strategy->M, strategy->N, strategy->K, int(strategy->op_kind));
     ws->strategy = *strategy;
     ws->domain = domain;
     ws->ctx_id = ctx->id;

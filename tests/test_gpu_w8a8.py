@@ -198,3 +198,17 @@ def test_memory_accounting_returns_to_the_baseline(gpu):
     w.free()
     after = dom.memory_stats()
     assert after.live_bytes == before.live_bytes and after.creates - after.destroys == before.creates - before.destroys
+
+
+@pytest.mark.parametrize("M, N, K", [(1, 96, 512), (64, 1024, 8192), (129, 4096, 1000), (777, 11008, 4096)])
+def test_the_memory_query_is_what_a_workspace_takes(gpu, M, N, K):
+    # parts of K included, which depend on the plan
+    _, dom, _ = gpu
+    lib = capi.load()
+    strategy = w8a8.default_strategy(w8a8.F16_DYNAMIC, M, N, K)
+    req = capi.MatmulWorkspaceRequirements()
+    assert lib.rk_npu_matmul_workspace_memory_query(C.byref(strategy), C.byref(req)) == 0
+    before = dom.memory_stats().live_bytes
+    ws = w8a8.MatmulWorkspace(dom, strategy)
+    assert dom.memory_stats().live_bytes - before == req.bytes == req.input_bytes + req.output_bytes + req.control_bytes
+    ws.free()
