@@ -473,7 +473,10 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
         }
         if (ws->host_status->bad_input) return RK_NPU_ERR_PARAM;              // a rejected row: the output is not written
         if (!u.serial && direct) std::memcpy(output, ws->host_out.ptr, values * 4);
-        else if (!u.serial && f32 && cudaMemcpy(output, ws->out, values * 4, cudaMemcpyDeviceToHost) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        else if (!u.serial && f32 && (cudaMemcpyAsync(output, ws->out, values * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)) {
+            cudaGetLastError();
+            return RK_NPU_ERR_SUBMIT;
+        }
         t.sync_us = since_us(at);
         if (timings) {
             t.input_us = event_us(ws->events[0], ws->events[1]);

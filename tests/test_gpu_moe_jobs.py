@@ -75,3 +75,39 @@ def test_fewer_rows_than_the_workspace_holds(gpu, oracle):
             assert np.array_equal(bits(out), bits(ref)), rows
     ws.free()
     w.free()
+
+
+@pytest.mark.parametrize("f32", [True, False])
+def test_large_results_do_not_wait_for_other_streams(gpu, oracle, f32):
+    # results beyond 512 KB are copied from the device; what the caller has running on the default stream is not waited for
+    import torch
+    _, dom, _ = gpu
+    H, I, E, rows = 1024, 32, 4, 200
+    rng = np.random.default_rng(3)
+    ex = dict(gate_up=rng.integers(-128, 128, size=(E, H, 2 * I), dtype=np.int8),
+              gate_up_scales=rng.uniform(2e-4, 6e-4, size=(E, 2 * I)).astype(np.float32),
+              down=rng.integers(-128, 128, size=(E, I, H), dtype=np.int8),
+              down_scales=rng.uniform(1e-3, 3e-3, size=(E, H)).astype(np.float32))
+    w = moe.MoeWeights(dom, shared_expert=0, form="w8", **ex)
+    ws = moe.MoeWorkspace(dom, moe.default_config(H, I, E, 0, 2, rows), form="w8")
+    x = rng.standard_normal((rows, H)).astype(np.float32)
+    ids = np.stack([np.arange(rows) % E, (np.arange(rows) + 1) % E], axis=1).astype(np.int32)
+    routes = rng.uniform(0.05, 0.95, size=(rows, 2)).astype(np.float32)
+    rc, q, s = oracle.moe_quantize_rows(x)
+    assert rc == 0
+    rc, ref = oracle.moe_run(ex, 0, 2, q, s, ids, routes, mode=1)
+    out = np.zeros((rows, H), np.float32)
+    run = (lambda: ws.run_f32(w, x, ids, routes, out)) if f32 else (lambda: ws.run_quantized(w, q, s, ids, routes, out))
+    for _ in range(3):                       # (the launches are kept from the second run on)
+        assert rc == 0 and run() == 0 and np.array_equal(bits(out), bits(ref))
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(600_000_000)           # a third of a second on the default stream
+    busy.record()
+    out.fill(0)
+    assert run() == 0
+    assert not busy.query(), "the call waited for the default stream"
+    assert np.array_equal(bits(out), bits(ref))
+    torch.cuda.synchronize()
+    ws.free()
+    w.free()
