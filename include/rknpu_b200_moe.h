@@ -95,7 +95,7 @@ uint64_t rk_npu_moe_w8_workspace_device_bytes(const rk_npu_moe_w8_workspace* wor
  * once with nearest-even rounding and scale max/127 (1 for a zero row).
  * RK_NPU_ERR_PARAM: NULL / rows out of range / overlapping arrays / bad id, coefficient, scale or non-finite input /
  * weights of another geometry; RK_NPU_ERR_DOMAIN: weights of another context or domain; RK_NPU_ERR_BUSY: workspace in
- * use.  A rejected call does not write the output. */
+ * use.  A rejected call does not write the output; after RK_NPU_ERR_SUBMIT it may hold anything. */
 int rk_npu_moe_w8_run_quantized(rk_npu_moe_w8_workspace* workspace, const rk_npu_moe_w8_weights* weights, int rows,
                                 const int8_t* input, const float* row_scales, const int32_t* expert_ids,
                                 const float* route_weights, float* output, rk_npu_moe_w8_timings* timings);

@@ -414,8 +414,8 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
         MoeRun& u = build_upload(*ws, *w, rows, input, f32, scales, ids, routes);
         const int assignments = u.assignments, jobs = u.jobs;
         // The combine kernel stores a small result straight into page-locked host memory, from where the host copies it to the
-        // caller's array; a larger one is copied by the driver.  Either once the verdict is known (a rejected call must not
-        // touch that array).
+        // caller's array; a larger one is copied by the driver.  Either once it is known whether the rows are accepted (a
+        // rejected call must not touch that array).
         const bool direct = ws->host_out.alias && values * 4 <= ws->host_out.bytes;
         u.out = direct ? static_cast<float*>(ws->host_out.alias) : ws->out;
         if (direct && !timings) {
@@ -450,7 +450,8 @@ int moe_run(rk_npu_moe_w8_workspace* ws, const rk_npu_moe_w8_weights* w, int row
         }
         ok = ok && ((!timings && launch_kept(*ws, f32, pull, plan.grid_rows, plan.level)) || launch_run(*ws, f32, pull, plan.grid_rows, true, timings ? ws->events : nullptr));
         at = Clock::now();
-        // int8 rows are not judged on the device, so a large result can follow its kernel at once
+        // int8 rows are not judged on the device, so a large result can follow its kernel at once (behind a device wait that
+        // ran out, RK_NPU_ERR_SUBMIT, the array then holds anything)
         if (ok && !direct && !f32) ok = cudaMemcpyAsync(output, ws->out, values * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
         if (!ok) {      // a launch failed part-way: the row maxima may be left behind
             cudaGetLastError();
