@@ -37,6 +37,7 @@ constexpr int PS_UNPACK_WARP0 = PS_ROLE_WARPS;
 constexpr int PS_EPI_WARP0 = PS_UNPACK_WARP0 + PS_UNPACK_WARPS;
 constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 640
 constexpr int PS_TMEM_COLS = 512;
+constexpr unsigned long long PS_DRAIN_NS = 50000;
 
 
 // One instantiation's resources.  TOK = tokens of the MMA tile (accumulator columns), half of them in each CTA.
@@ -684,6 +685,10 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     // ------------------------------------------------------------------------ teardown
     tc_fence_before();
     __syncthreads();
+    // A wait that ran out ends its role at once, and copies requested just before may still be on their way into this CTA's
+    // shared memory: they land within microseconds, so the CTA stays that long before it leaves.
+    if (*reinterpret_cast<volatile int*>(s_error))
+        for (const unsigned long long until = global_ns() + PS_DRAIN_NS; global_ns() < until;) __nanosleep(1000);
     cluster_arrive();
     cluster_wait();   // neither CTA frees tensor memory or leaves while the other may still use it
     if (tid == 0 && *s_error) report_device_error(p.status, p.report);
