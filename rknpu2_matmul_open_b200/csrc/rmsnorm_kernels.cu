@@ -6,13 +6,14 @@
 // the double-precision statement of the original's board test (tests/test_add_rmsnorm_f16.cpp:96-113), which is what
 // the original device's result is checked against.  Double-precision conversions run at a quarter of the fp32 rate and
 // would be the busiest pipe of this kernel, so the second pass proves per value that single precision
-// gives the same fp16 bits and falls back to the defining expression where it cannot (scale_one).
+// gives the same fp16 bits and falls back to the defining expression where it cannot (scale_pair).
 //
 // HBM-bound: 4 tensors of 2 M D bytes cross DRAM once each.  Two forms.  Rows that fit a CTA's registers take
-// add_rmsnorm_row_kernel; longer block-8 rows take add_rmsnorm_kernel, where a tile of TM tokens is shared by a CLUSTER of CS CTAs,
-// each taking a slice of D: the sums stay in that CTA's shared memory between the two passes (both outputs are stored
-// in the second one, so that no global store is in flight at the cluster barrier), the per-token sums of squares are exchanged through distributed shared memory and added in rank
-// order by every CTA, so that the result does not depend on the schedule.  Both tensor layouts move 16-byte chunks
+// add_rmsnorm_row_kernel; longer block-8 rows, and block-8 tensors across the bus, take add_rmsnorm_kernel, where a tile of TM
+// tokens is shared by a CLUSTER of CS CTAs, each taking a slice of D: the sums stay in that CTA's shared memory between the two
+// passes (both outputs are stored in the second one, so that no global store is in flight at the cluster barrier), the
+// per-token sums of squares are exchanged through distributed shared memory and added in rank order by every CTA, so that the
+// result does not depend on the schedule.  Both tensor layouts move 16-byte chunks
 // (8 elements): in the block-8 layout (D/8, M, 8) consecutive TOKENS of one chunk column are contiguous, in row-major
 // [M, D] consecutive CHUNKS of one token are; the thread index is split accordingly so that a warp touches 512
 // contiguous bytes either way.
@@ -97,8 +98,7 @@ __device__ __forceinline__ uint32_t scale_pair(uint32_t v, uint32_t g, double in
     return o;
 }
 
-// ROWS: row-major [M, D]; else block-8 (D/8, M, 8).  grid = tiles * CS CTAs in clusters of CS.
-template <bool ROWS>
+// Block-8 (D/8, M, 8).  grid = tiles * CS CTAs in clusters of CS.
 __global__ void __launch_bounds__(RN_THREADS, RN_CTAS) add_rmsnorm_kernel(AddRmsNormParams p)
 {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(RN_THREADS, RN_CTAS) add_rmsnorm_kernel(AddRms
     const int CS = int(cluster.num_blocks()), rank = int(cluster.block_rank());
     const int TM = p.tile_tokens, JL = RN_THREADS / TM;       // tokens of the tile x chunk lanes
     const int tid = threadIdx.x;
-    const int dm = ROWS ? tid / JL : tid % TM, jl = ROWS ? tid % JL : tid / TM;
+    const int dm = tid % TM, jl = tid / TM;
     const int m = int(blockIdx.x / CS) * TM + dm;
     const int chunks = p.D / 8, per = (chunks + CS - 1) / CS;
     const int j0 = min(chunks, rank * per), j1 = min(chunks, j0 + per);
@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(RN_THREADS, RN_CTAS) add_rmsnorm_kernel(AddRms
     uint4* s_sum = reinterpret_cast<uint4*>(smem);                               // this CTA's slice of the tile's sums
     double* s_part = reinterpret_cast<double*>(smem + size_t(TM) * per * 16);    // [RN_THREADS]
     double* s_token = s_part + RN_THREADS;                                       // [TM] this CTA's sum of squares per token
-    auto lane_of = [&](int token, int lane) { return ROWS ? token * JL + lane : lane * TM + token; };
-    auto global_at = [&](int j) { return ROWS ? size_t(m) * chunks + j : size_t(j) * p.M + m; };
-    auto shared_at = [&](int j) { return ROWS ? dm * per + (j - j0) : (j - j0) * TM + dm; };
+    auto lane_of = [&](int token, int lane) { return lane * TM + token; };
+    auto global_at = [&](int j) { return size_t(j) * p.M + m; };
+    auto shared_at = [&](int j) { return (j - j0) * TM + dm; };
 
     double acc = 0.0;
     if (live) {
@@ -260,17 +260,17 @@ __global__ void __launch_bounds__(RN_THREADS) add_rmsnorm_row_kernel(AddRmsNormP
 
 } // namespace
 
-// Tile and cluster.  Candidates: tokens per tile a power of two up to 32 and up to the batch (in the block-8 layout
-// at least 8 where the batch has them, so that a tile's chunks of one column are 128 contiguous bytes); clusters of
+// Tile and cluster.  Candidates: tokens per tile a power of two up to 32 and up to the batch (at least 8 where the
+// batch has them, so that a tile's chunks of one column are 128 contiguous bytes); clusters of
 // 1, 2, 4 or 8 CTAs over D; the CTA's slice of the sums within RN_SMEM_SUMS; every thread of a cluster member with at
 // least one chunk.  Taken: the candidate with the most CTAs up to 128 (small batches are spread over the GPU), then
 // the smallest cluster, then the most tokens per tile.  Measured on 4096 rows: time falls with the work per CTA (a
 // CTA's fixed cost -- start, load latency, two barriers, store drain -- is about 4 us) and rises with the cluster size.
-void add_rmsnorm_geometry(int M, int D, int row_major, int& tile_tokens, int& cluster)
+static void add_rmsnorm_geometry(int M, int D, int& tile_tokens, int& cluster)
 {
     int top = 1;
     while (top < 32 && top < M) top <<= 1;
-    const int floor_tokens = row_major ? 1 : (top < 8 ? top : 8);
+    const int floor_tokens = top < 8 ? top : 8;
     const int chunks = D / 8;
     if (const char* text = std::getenv("RK_NPU_B200_RMSNORM_TILE")) {      // experiments: "tokens,cluster"
         int tm = 0, cs = 0;
@@ -284,7 +284,7 @@ void add_rmsnorm_geometry(int M, int D, int row_major, int& tile_tokens, int& cl
     int best_score = -1;
     tile_tokens = 1;
     cluster = 8;        // D <= 32768: 512 chunks per CTA, one per thread
-    for (int pass = 0; pass < 2 && best_score < 0; ++pass)      // second pass: without the block-8 floor, if nothing fitted
+    for (int pass = 0; pass < 2 && best_score < 0; ++pass)      // second pass: without the floor, if nothing fitted
         for (int cs = 1; cs <= 8; cs <<= 1)
             for (int tm = top; tm >= (pass ? 1 : floor_tokens); tm >>= 1) {
                 const int per = (chunks + cs - 1) / cs;
@@ -359,20 +359,19 @@ cudaError_t launch_add_rmsnorm(const AddRmsNormParams& q, cudaStream_t stream)
     if (row_geometry(p, threads, p.tile_tokens, cpl))
         return p.row_major ? launch_rows<true>(p, threads, cpl, stream) : launch_rows<false>(p, threads, cpl, stream);
     int cs = 1;
-    add_rmsnorm_geometry(p.M, p.D, p.row_major, p.tile_tokens, cs);
+    add_rmsnorm_geometry(p.M, p.D, p.tile_tokens, cs);
     const int per = (p.D / 8 + cs - 1) / cs;
     const size_t shared = size_t(p.tile_tokens) * per * 16 + size_t(RN_THREADS + p.tile_tokens) * sizeof(double);
-    auto kernel = p.row_major ? add_rmsnorm_kernel<true> : add_rmsnorm_kernel<false>;
     // function attributes are per device: remember what this device's copy of the kernel already allows
-    static std::atomic<int> allowed[2][RN_MAX_DEVICES];
+    static std::atomic<int> allowed[RN_MAX_DEVICES];
     int device = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess) return err;
-    std::atomic<int>* known = device >= 0 && device < RN_MAX_DEVICES ? &allowed[p.row_major ? 1 : 0][device] : nullptr;
+    std::atomic<int>* known = device >= 0 && device < RN_MAX_DEVICES ? &allowed[device] : nullptr;
     if (!known || known->load(std::memory_order_relaxed) < int(shared)) {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(RN_SMEM_SUMS + (RN_THREADS + 32) * sizeof(double)));
+        err = cudaFuncSetAttribute(add_rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(RN_SMEM_SUMS + (RN_THREADS + 32) * sizeof(double)));
         if (err != cudaSuccess) return err;
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, int(cudaSharedmemCarveoutMaxShared));
+        err = cudaFuncSetAttribute(add_rmsnorm_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, int(cudaSharedmemCarveoutMaxShared));
         if (err != cudaSuccess) return err;
         if (known) known->store(int(RN_SMEM_SUMS + (RN_THREADS + 32) * sizeof(double)), std::memory_order_relaxed);
     }
@@ -389,7 +388,7 @@ cudaError_t launch_add_rmsnorm(const AddRmsNormParams& q, cudaStream_t stream)
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, p);
+    return cudaLaunchKernelEx(&cfg, add_rmsnorm_kernel, p);
 }
 
 } // namespace rkb200

@@ -62,7 +62,6 @@ struct QuantParams {
     uint8_t* Xq;            // activation codes, layout above
     float* scales;          // [M]
     float* inverse;         // [M]
-    uint32_t* rowmax_zero;  // [M] cleared before a SwiGLU epilogue maxes into it (nullable)
     uint32_t* rowmax;       // [M] non-null: scales come from these magnitude bits (no scan); cleared after use
     Status* status;
     int* host_flag;         // mapped host word mirroring status->bad_input (nullable)
@@ -250,7 +249,6 @@ cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, 
 // persistent two-CTA tcgen05 kernel (K <= 131072): p.T (tokens of one CTA's activation tile: 32, 64, 96, 112 or 128) and p.split
 // required, p.partials and p.counts where split > 1
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
-bool gemm_tc_persist_supported(const GemmParams& p);
 // How the persistent kernel cuts a problem (columns: all accumulator rows, i.e. gate and up together for SwiGLU)
 struct PersistPlan {
     int tok;      // tokens of the MMA tile (64, 128, 192, 224 or 256): p.T = tok / 2, the code buffer holds whole multiples of tok

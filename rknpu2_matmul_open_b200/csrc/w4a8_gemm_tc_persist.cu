@@ -755,11 +755,6 @@ cudaError_t launch_persist_tok(const GemmParams& p, cudaStream_t stream, bool pd
 }
 } // namespace
 
-bool gemm_tc_persist_supported(const GemmParams& p)
-{
-    return (p.T == 32 || p.T == 64 || p.T == 96 || p.T == 112 || p.T == 128) && (long long)p.KB * KBLOCK <= PS_MAX_K && p.split >= 1 && (p.split == 1 || (p.partials && p.counts));
-}
-
 int gemm_tc_persist_tiles(int columns, int M, int tok) { return (columns + 255) / 256 * ((M + tok - 1) / tok); }
 
 // The token tile and the number of parts a tile's K is cut into: the cheapest by a model of the kernel's time in cycles,
@@ -810,13 +805,14 @@ size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan)
 
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
-    if (!gemm_tc_persist_supported(p)) return cudaErrorInvalidValue;
+    if ((long long)p.KB * KBLOCK > PS_MAX_K || p.split < 1 || (p.split > 1 && !(p.partials && p.counts))) return cudaErrorInvalidValue;
     switch (2 * p.T) {
     case 64: return launch_persist_tok<64>(p, stream, pdl);
     case 128: return launch_persist_tok<128>(p, stream, pdl);
     case 192: return launch_persist_tok<192>(p, stream, pdl);
     case 224: return launch_persist_tok<224>(p, stream, pdl);
-    default: return launch_persist_tok<256>(p, stream, pdl);
+    case 256: return launch_persist_tok<256>(p, stream, pdl);
+    default: return cudaErrorInvalidValue;
     }
 }
 
