@@ -138,7 +138,8 @@ __device__ __forceinline__ float silu_poly(float g)
 //     by fused multiply-add (exact) and one correction (P. Markstein, "Computation of elementary functions on the IBM
 //     RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), all of it negated: the reciprocal of a negated argument
 //     costs nothing, the negation of a pair two instructions.  Returns the negated values.
-// With silu_poly for every other argument equal bit for bit to silu_poly for every one of the 2^32 arguments (checked).
+// With silu_poly for every other argument equal bit for bit to silu_poly for every one of the 2^32 arguments
+// (tests/test_gpu_silu_pairs.py tries them all).
 __device__ __forceinline__ void minus_silu_poly2(float g0, float g1, float& y0, float& y1)
 {
     const F2 g = f2_pack(g0, g1);
