@@ -737,7 +737,7 @@ void host_piece_release(rk_npu_ctx* ctx, rk_npu_ctx::HostPiece& piece)
     bool keep = false;
     {
         std::lock_guard<std::mutex> g(ctx->host_lock);
-        keep = ctx->host_free_bytes + piece.bytes <= HOST_PIECES_KEPT;
+        keep = !ctx->closed && ctx->host_free_bytes + piece.bytes <= HOST_PIECES_KEPT;
         if (keep) {
             try { ctx->host_free.push_back(piece); ctx->host_free_bytes += piece.bytes; } catch (...) { keep = false; }
         }
@@ -748,14 +748,22 @@ void host_piece_release(rk_npu_ctx* ctx, rk_npu_ctx::HostPiece& piece)
 void host_pieces_drop(rk_npu_ctx* ctx)
 {
     std::lock_guard<std::mutex> g(ctx->host_lock);
+    ctx->closed = true;
     for (auto& piece : ctx->host_free) cudaFreeHost(piece.ptr);
     ctx->host_free.clear();
     ctx->host_free_bytes = 0;
 }
+static void context_release(rk_npu_ctx* ctx)
+{
+    if (ctx->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) delete ctx;
+}
 void domain_retain(rk_npu_iommu_domain* d) { if (d) d->refs.fetch_add(1, std::memory_order_relaxed); }
 void domain_release(rk_npu_iommu_domain* d)
 {
-    if (d && d->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) delete d;
+    if (d && d->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) {
+        context_release(d->ctx);
+        delete d;
+    }
 }
 // Test hook: the allocation that brings this counter to zero fails as if the device were out of memory.
 static std::atomic<long long> g_allocations_until_failure{-1};
@@ -842,12 +850,12 @@ extern "C" rk_npu_ctx* rk_npu_b200_open_offline(uint32_t driver_version)
 extern "C" void rk_npu_close(rk_npu_ctx* ctx)
 {
     if (!ctx) return;
-    if (ctx->device < 0) { delete ctx; return; }
+    if (ctx->device < 0) { context_release(ctx); return; }
     cudaSetDevice(ctx->device);
     if (ctx->stream) { cudaStreamSynchronize(ctx->stream); cudaStreamDestroy(ctx->stream); }
     group_close(ctx);
     host_pieces_drop(ctx);
-    delete ctx;
+    context_release(ctx);
 }
 
 extern "C" int rk_npu_b200_device(const rk_npu_ctx* ctx) { return ctx ? ctx->device : -1; }
@@ -859,6 +867,7 @@ extern "C" rk_npu_iommu_domain* rk_npu_iommu_domain_create(rk_npu_ctx* ctx, uint
     auto* d = new (std::nothrow) rk_npu_iommu_domain;
     if (!d) { errno = ENOMEM; return nullptr; }
     d->ctx = ctx;
+    ctx->refs.fetch_add(1, std::memory_order_relaxed);
     d->id = domain_id;
     return d;
 }

@@ -20,6 +20,8 @@ struct rk_npu_ctx {
     std::mutex host_lock;
     std::vector<HostPiece> host_free;
     size_t host_free_bytes = 0;
+    bool closed = false;          // under host_lock: pieces that come back now go to the driver
+    std::atomic<int> refs{1};     // the caller's, until rk_npu_close, and one per domain: objects may be freed after the close
     // group of GPUs (rk_npu_b200_open_group): this context is `rank` of `world`; comm is the NCCL communicator
     int rank = 0, world = 1;
     void* comm = nullptr;

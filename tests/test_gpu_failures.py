@@ -109,3 +109,25 @@ def test_a_recorded_device_error_is_reported_once_and_cleared(gpu, oracle, M):
     assert np.array_equal(bits(out), bits(oracle.linear(A, B, sw)[1]))
     ws.free()
     w.free()
+
+
+def test_objects_freed_after_their_context_was_closed(oracle):
+    # workspaces give page-locked pieces back to the context they borrowed them from, also when it has been closed before
+    from rknpu2_matmul_open_b200 import moe
+    ctx = rk.Context("cuda:0")
+    dom = ctx.domain(0)
+    K, N = 512, 256
+    B, sw = make_weights(K, N, seed=5)
+    w = rk.Weights(dom, B, sw)
+    spaces = [rk.Workspace(dom, rk.default_config(M, N, K)) for M in (1, 8, 12, 64)]
+    experts = moe.MoeWorkspace(dom, moe.default_config(64, 32, 2, 0, 2, 8), form="w8")
+    A = make_activations(8, K, seed=6, dtype="f32")
+    out = np.zeros((8, N), np.float32)
+    assert spaces[1].run_f32(w, A, out) == 0 and np.array_equal(bits(out), bits(oracle.linear(A, B, sw)[1]))
+    spaces.pop(0).free()                     # one piece is back before the close, the others come back behind it
+    ctx.close()
+    for ws in spaces:
+        ws.free()
+    experts.free()
+    w.free()
+    dom.free()
