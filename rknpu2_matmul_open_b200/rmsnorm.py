@@ -8,6 +8,7 @@ buffers in its block-8 layout, ``enqueue`` the form on device tensors and the ca
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 
 import numpy as np
 
@@ -27,27 +28,57 @@ def from_block8(flat: np.ndarray, M: int, D: int) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(flat).reshape(D // 8, M, 8).transpose(1, 0, 2)).reshape(M, D)
 
 
-class Buffer:
-    """rk_npu_mem_alloc / rk_npu_mem_free."""
+class _Allocation:
+    """One rk_npu_mem_alloc; given back by release(), or with its last holder where that was asked for meanwhile."""
 
-    def __init__(self, domain, size: int, flags: int = 0):
+    def __init__(self, domain, size: int, flags: int):
         self.lib = capi.load()
         self.ctx = domain.ctx
         self.mem = Mem()
+        self.unwanted = False
         rc = self.lib.rk_npu_mem_alloc(domain.handle, size, flags, C.byref(self.mem))
         if rc != capi.RK_NPU_OK:
             raise W4A8Error(rc, "rk_npu_mem_alloc")
 
+    def release(self) -> int:
+        return self.lib.rk_npu_mem_free(self.ctx.handle, C.byref(self.mem)) if self.mem.handle else capi.RK_NPU_OK
+
+    def __del__(self):
+        if self.unwanted and self.ctx.handle:
+            self.release()
+
+
+class _Mapping:
+    """What an array of the host mapping is based on: keeps the allocation while the array lives."""
+
+    def __init__(self, allocation: _Allocation):
+        self.allocation = allocation
+        self.__array_interface__ = {"data": (allocation.mem.vaddr, False), "shape": (allocation.mem.size,), "typestr": "|u1", "version": 3}
+
+
+class Buffer:
+    """rk_npu_mem_alloc / rk_npu_mem_free."""
+
+    def __init__(self, domain, size: int, flags: int = 0):
+        self.allocation = _Allocation(domain, size, flags)
+        self.lib, self.ctx, self.mem = self.allocation.lib, self.allocation.ctx, self.allocation.mem
+        self.mappings = weakref.WeakSet()
+
     def array(self, dtype=np.uint16) -> np.ndarray:
-        """The host mapping as a numpy array (valid until free())."""
+        """The host mapping as a numpy array.  The memory stays while such an array lives, also after free()."""
+        mapping = _Mapping(self.allocation)
+        self.mappings.add(mapping)
         count = self.mem.size // np.dtype(dtype).itemsize
-        return np.ctypeslib.as_array(C.cast(self.mem.vaddr, C.POINTER(C.c_uint8)), (self.mem.size,)).view(dtype)[:count]
+        return np.asarray(mapping).view(dtype)[:count]
 
     def free(self) -> int:
-        rc = capi.RK_NPU_OK
-        if self.mem.handle:
-            rc = self.lib.rk_npu_mem_free(self.ctx.handle, C.byref(self.mem))
-        return rc
+        if self.allocation is None:
+            return capi.RK_NPU_OK
+        if not self.mappings:
+            return self.allocation.release()
+        self.allocation.unwanted = True            # the last of the arrays gives the memory back
+        self.allocation, self.mem = None, Mem()
+        return capi.RK_NPU_OK
 
 
 def default_config(M: int, D: int) -> AddRmsNormConfig:
