@@ -464,7 +464,7 @@ def run_cuda(args, rank, world, local_rank):
                              # traffic of a launch is its algorithmic bytes
                              "traffic": bytes_per_launch, "peak_kind": peak_kind,
                              "kernel": {3: "gemm_fused_kernel (split-K clusters)", 5: "gemm_decode_kernel (whole-K CTAs)"}.get(
-                                 linears[0]["ws"].schedule()[0], "quantize_kernel + gemm_mma_kernel") + ": scan + quantise + GEMM + dequantise",
+                                 linears[0]["ws"].schedule()[0], "quantize_rows_kernel + gemm_mma_kernel") + ": scan + quantise + GEMM + dequantise",
                              "frac_of_nominal": value / world / 8000.0, "nominal_peak": 8000.0,   # 8 TB/s data-sheet HBM3e
                              "bytes_per_launch": bytes_per_launch,
                              "us_per_launch": 1e3 * ms_step / len(linears)},
@@ -685,7 +685,7 @@ def _w8a8_prefill(rk, dom, dev, oracle, peak_tops):
     ws.free()
     w.free()
     return {"us": sec * 1e6, "tops": tops, "sampled_exact": exact, "frac_of_measured_int8_peak": tops / peak_tops if peak_tops else None,
-            "includes": "w8_quantize_kernel + persistent tcgen05 GEMM with int8 weights + the call's host synchronisation"}
+            "includes": "w8_quantize_rows_kernel + persistent tcgen05 GEMM with int8 weights + the call's host synchronisation"}
 
 
 def _check_ffn(oracle, A, Bg, sg, Bd, sd, middle, C):

@@ -758,8 +758,9 @@ cudaError_t launch_persist_tok(const GemmParams& p, cudaStream_t stream, bool pd
 int gemm_tc_persist_tiles(int columns, int M, int tok) { return (columns + 255) / 256 * ((M + tok - 1) / tok); }
 
 // The token tile and the number of parts a tile's K is cut into: the cheapest by a model of the kernel's time in cycles,
-// from what it measured on 80 shapes (M 33..4096, K 2048..14336, N 1024..28672, both epilogues; within 1 % of the best
-// choice on average, 15 % at worst):
+// fitted to 80 shapes (M 33..4096, K 2048..14336, N 1024..28672, both epilogues).  On 27 others, K 1024..11008, it is within
+// 2 % of the best choice but just above 64 tokens (a second tile of 64 would be nearly empty: 20 % at worst, 65 x 8192 -> 2048
+// 19.0 us where 64-token tiles take 15.8) and for 400 to 448 tokens of K = 1024 (23.9 against 22.0):
 //   * a k-block takes 270 to 390 cycles at 64 tokens and 310 to 370 at 128, more with more SMs busy (the operands come
 //     out of L2 at about 45 bytes per SM and cycle when all SMs ask), and 530 at 256, where the MMAs bound it; int8
 //     weights are delivery-bound (52 bytes per cycle).  At 192 tokens two accumulators leave two buffers of unpacked
