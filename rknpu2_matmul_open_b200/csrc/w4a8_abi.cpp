@@ -459,6 +459,7 @@ int enqueue(const Call& c)
     q.Xq = ws.codes;
     q.scales = ws.scales;
     q.inverse = ws.inverse;
+    q.rowmax_zero = nullptr;
     q.rowmax = c.rowmax_in;
     q.status = ws.status;
     q.host_flag = c.status ? &c.status->bad_input : nullptr;

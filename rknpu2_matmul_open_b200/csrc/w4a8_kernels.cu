@@ -98,6 +98,7 @@ struct RowQuant {
         const float inv = __fdiv_rn(1.0f, s);
         p.scales[m] = s;
         p.inverse[m] = inv;
+        if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
         // "any row bad" without a reset pass, see finish(): the ticket is drawn here, its answer is needed at the end
         if (bad) { atomicOr(&p.status->bad_accum, bad); __threadfence(); }
         ticket = atomicInc(&p.status->done, (unsigned)p.M - 1u);
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(256, 8) quantize_kernel(const QuantParams p)
     // Cross-CTA bookkeeping last, so that the other 255 threads of the CTA never wait for its
     // round trips to L2.
     if (tid == 0) {
+        if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
         // "Any row bad" across CTAs without a reset pass: the last CTA to arrive
         // publishes the accumulated flag and clears the scratch word; the counter
         // wraps to zero by itself (atomicInc with limit M-1).
