@@ -1,5 +1,5 @@
 """The paired SiLU of the large-batch epilogue against the scalar statement, for every one of the 2^32 arguments: the device
-functions themselves, compiled from the library's header into a small checker.  A value takes the paired form where it and
+functions themselves, compiled from the library's header into a small program.  A value takes the paired form where it and
 its neighbours are plain (silu_plain), in either half of a pair; every other value has to be recognised as not plain in any
 place of a group of four."""
 import ctypes as C
