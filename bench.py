@@ -1128,11 +1128,10 @@ def _print_stamps(rk, case, calls, stream, torch):
         raw = np.zeros(256, np.uint64)
         lib.rk_npu_b200_w4a8_trace_read(calls[0][1].handle, raw.ctypes.data, 32)
         print(f"clusters in the grid: {int(raw[200])}; per tile of cluster 0 (cycles since kernel start): MMA issuer begins,"
-              " first MMA issued, last commit, epilogue sees the accumulator, tensor memory handed back, tile stored,"
-              " cycles the issuer waited for operands")
+              " last commit, epilogue sees the accumulator, tensor memory handed back, tile stored")
         for j in range(16):
             if raw[j * 8 + 2]:
-                print(f"tile {j}: {[int(x) for x in raw[j * 8:j * 8 + 7]]}")
+                print(f"tile {j}: {[int(raw[j * 8 + k]) for k in (0, 2, 3, 4, 5)]}")
         print(f"cycles in the whole launch: an unpack warp waited for weights {int(raw[128])}, for a free buffer {int(raw[129])};"
               f" activations were waited for {int(raw[160])}")
 

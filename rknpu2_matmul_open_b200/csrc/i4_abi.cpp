@@ -42,7 +42,9 @@ struct rk_npu_i4_workspace {
     uint32_t domain_id = 0;
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
     cudaStream_t stream = nullptr;
-    int T = 0, KB = 0, parts = 1;
+    int KB = 0;
+    PersistPlan plan{};
+    PersistMaps maps{};
     uint8_t* codes = nullptr;
     int* partials = nullptr;         // partial sums of tiles whose K is cut between CTA pairs
     unsigned* counts = nullptr;      // and how far each such tile is
@@ -116,7 +118,7 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     q.A = dA;
     q.Xq = ws->codes;
     q.scales = ws->scales;
-    q.M = cfg.M; q.K = cfg.K; q.Kp = ws->KB * KBLOCK; q.T = ws->T;
+    q.M = cfg.M; q.K = cfg.K; q.Kp = ws->KB * KBLOCK; q.T = PERSIST_T;
     q.kind = 2;                                   // int8 codes as given
     GemmParams g{};
     g.Wp = w->packed;
@@ -126,9 +128,10 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     g.out = dC;
     g.status = ws->status;
     g.M = cfg.M; g.N = cfg.N; g.K = cfg.K;
-    g.KB = ws->KB; g.NG = w->NG; g.T = ws->T;
+    g.KB = ws->KB; g.NG = w->NG; g.T = PERSIST_T;
     g.epi = EPI_I32;
-    g.split = ws->parts;
+    set_plan(g, ws->plan);
+    g.maps = &ws->maps;
     g.partials = ws->partials;
     g.counts = ws->counts;
     g.timeout_ns = (unsigned long long)cfg.timeout_ms * 1000000ull;
@@ -241,9 +244,8 @@ extern "C" rk_npu_i4_workspace* rk_npu_i4_workspace_create(rk_npu_iommu_domain* 
         domain_retain(domain);
         ws->KB = (cfg->K + KBLOCK - 1) / KBLOCK;
         const PersistPlan plan = gemm_tc_persist_plan(cfg->N, cfg->M, ws->KB, false, false, ctx->sm_count);
-        ws->T = plan.tok / 2;
-        ws->parts = plan.split;
-        ws->codes_bytes = size_t(align_up(cfg->M, plan.tok)) * size_t(ws->KB) * KBLOCK;
+        ws->plan = plan;
+        ws->codes_bytes = size_t(align_up(cfg->M, PERSIST_TOKENS)) * size_t(ws->KB) * KBLOCK;
         ws->partials_bytes = gemm_tc_persist_slot_bytes(cfg->N, cfg->M, plan);
         ws->counts_bytes = gemm_tc_persist_count_bytes(cfg->N, cfg->M, plan);
         ws->stage_in_bytes = size_t(cfg->M) * cfg->K;
@@ -257,6 +259,7 @@ extern "C" rk_npu_i4_workspace* rk_npu_i4_workspace_create(rk_npu_iommu_domain* 
              !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status)) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->stage_in), ws->stage_in_bytes) &&
              !device_alloc(domain, reinterpret_cast<void**>(&ws->stage_out), ws->stage_out_bytes);
+        ok = ok && make_persist_maps(ws->maps, ws->codes, cfg->M, ws->KB);
         ok = ok && cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
              (!ws->counts || cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess) &&
              cudaMemsetAsync(ws->status, 0, sizeof(Status), ws->stream) == cudaSuccess && cudaStreamSynchronize(ws->stream) == cudaSuccess;

@@ -441,7 +441,6 @@ int enqueue(const Call& c)
         ws.launches.fetch_add(1, std::memory_order_relaxed);
         return RK_NPU_OK;
     }
-    if (ws.variant == 2) ws.T = ws.plan[c.epi == EPI_SWIGLU].tok / 2;      // the layout of the codes follows the launch that reads them
     if (c.codes_in) {
         CodesInParams ci{};
         ci.codes = c.codes_in;
@@ -495,7 +494,8 @@ int enqueue(const Call& c)
     if (ws.variant == 2) {
         g.partials = ws.partials;
         g.counts = ws.counts;
-        g.split = ws.plan[c.epi == EPI_SWIGLU].split;
+        set_plan(g, ws.plan[c.epi == EPI_SWIGLU]);
+        g.maps = &ws.maps;
         err = launch_gemm_tc_persist(g, c.stream, pdl);
     } else if (ws.variant == 4) {
         g.split = 1;
@@ -1171,7 +1171,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (variant == 2) {
         ws->TC = 0;
         for (int swiglu = 0; swiglu < 2; ++swiglu) ws->plan[swiglu] = gemm_tc_persist_plan(local_N, cfg->M, ws->KB, false, swiglu != 0, ctx->sm_count);
-        ws->T = ws->plan[0].tok / 2;
+        ws->T = PERSIST_T;
     } else if (variant == 4) {
         ws->TC = ws->T = cfg->M <= 16 ? 16 : cfg->M <= 32 ? 32 : cfg->M <= 64 ? 64 : 128;   // tcgen05 N
     } else {
@@ -1186,12 +1186,13 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (schedule.cluster && (variant == 1 || variant == 5 || (variant == 3 && (ws->KB + schedule.cluster - 1) / schedule.cluster <= FUSED_MAX_STAGES)) &&
         (variant == 5 || ws->KB >= schedule.cluster))
         ws->split_override = schedule.cluster;
-    const size_t Mp = variant == 2 ? size_t(std::max(align_up(cfg->M, ws->plan[0].tok), align_up(cfg->M, ws->plan[1].tok))) : size_t(align_up(cfg->M, ws->T));
+    const size_t Mp = size_t(align_up(cfg->M, variant == 2 ? PERSIST_TOKENS : ws->T));
     ws->codes_bytes = Mp * size_t(ws->KB) * KBLOCK;
     const int out_cols = cfg->N;
     ws->stage_in_bytes = size_t(cfg->M) * cfg->K * 4;
     ws->stage_out_bytes = size_t(cfg->M) * out_cols * 4;
     bool ok = !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes);
+    ok = ok && (variant != 2 || make_persist_maps(ws->maps, ws->codes, cfg->M, ws->KB));
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), sizeof(float) * 2 * cfg->M);
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->rowmax), sizeof(uint32_t) * cfg->M);
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status));

@@ -22,6 +22,7 @@
 //   (src/rk_npu_w4a8_quant.cpp:87-135): int8 MMA is native here so no split is needed.
 #pragma once
 #include <atomic>
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -99,6 +100,12 @@ __device__ __forceinline__ void report_device_error(Status* status, int* report)
     *reinterpret_cast<volatile int*>(report ? report : &status->device_error) = 1;
 }
 
+// Tensor maps of a persistent kernel's activation codes [groups of eight tokens][K bytes x 8]: boxes of two k-blocks of eight,
+// four and two groups.  Made once for a workspace's code buffer.
+struct PersistMaps {
+    CUtensorMap box[3];
+};
+
 struct GemmParams {
     const uint8_t* Wp;
     const uint8_t* Xq;
@@ -115,12 +122,14 @@ struct GemmParams {
     int F;                  // SwiGLU: N/2, else 0
     int epi;
     int split;              // split-K factor == cluster size along y (1, 2, 4, 8)
+    int unit, most, snap;   // persistent kernel: its PersistPlan
+    const PersistMaps* maps; // persistent kernel: in host memory, copied with the launch
     int w8;                 // persistent kernel: Wp holds int8 codes in the W8 layout (w8a8_kernels.cu), sums are not scaled by 16
     unsigned long long timeout_ns;
     unsigned long long* trace;  // optional cycle stamps of CTA (0,0): [role 0..2][k-block 0..63][2] (nullable)
     // streaming kernel: [2 x CTAs][T / 4][128][4] int32 partial sums (two slots per CTA, never cleared) and [tiles] stages
-    // accumulated so far, zero between launches; persistent kernel with split > 1: [tiles][split][2 CTAs][tokens of the
-    // tile / 4][128][4] and [tiles][2 CTAs] parts done
+    // accumulated so far, zero between launches; persistent kernel with split > 1: [tiles][split][2 CTAs][unit / 16][4]
+    // [128 threads][4] and [tiles][2 CTAs] parts done
     int* partials;
     unsigned int* counts;
 };
@@ -208,7 +217,7 @@ struct PackParams {
     int K, N, KC, NG;
 };
 
-// ---- W8A8 operators (w8a8_kernels.cu): int8 weights W8p[g][kb][c][r][16 B], activations in the same Xq layout
+// ---- W8A8 operators (w8a8_kernels.cu): int8 weights W8p[channel tile of 128][kb][c][r][16 B], activations in the same Xq layout
 struct W8PackParams {
     const int8_t* B;        // [K,N] int8 on the device
     uint8_t* Wp;
@@ -250,16 +259,29 @@ int gemm_decode_ctas(int items, int cluster, int cap);
 int gemm_decode_resident_ctas(int cluster, size_t smem, int sm_count);
 cudaError_t launch_gemm_decode(const DecodeParams& p, cudaStream_t stream, bool pdl);
 cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, bool pdl);
-// persistent two-CTA tcgen05 kernel (K <= 131072): p.T (tokens of one CTA's activation tile: 32, 64, 96, 112 or 128) and p.split
-// required, p.partials and p.counts where split > 1
+// Persistent two-CTA tcgen05 kernel (K <= 131072).  Its activation codes lie in groups of PERSIST_T tokens (p.T) up to a
+// multiple of 32 tokens; p.partials and p.counts where split > 1.
+constexpr int PERSIST_T = 8;
+constexpr int PERSIST_TOKENS = 32;
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
-// How the persistent kernel cuts a problem (columns: all accumulator rows, i.e. gate and up together for SwiGLU)
+bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB);
+// How the persistent kernel cuts a problem (columns: all accumulator rows, i.e. gate and up together for SwiGLU): pairs of
+// channel tiles x units of tokens, dealt to the CTA pairs in runs (w4a8_rules.h)
 struct PersistPlan {
-    int tok;      // tokens of the MMA tile (64, 128, 192, 224 or 256): p.T = tok / 2, the code buffer holds whole multiples of tok
-    int split;    // parts a tile's K is cut into (p.split)
+    int unit;     // tokens, a multiple of 32
+    int most;     // units of an item
+    int snap;     // see persist_bound
+    int split;    // parts K is cut into; one item per launch unit then, and most is 1
 };
+inline void set_plan(GemmParams& p, const PersistPlan& plan)
+{
+    p.unit = plan.unit;
+    p.most = plan.most;
+    p.snap = plan.snap;
+    p.split = plan.split;
+}
 PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count);
-int gemm_tc_persist_tiles(int columns, int M, int tok);
+int gemm_tc_persist_units(int columns, int M, int unit);
 // Bytes of GemmParams.partials and .counts (the latter zero before the first launch); 0 where nothing is split
 size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan);
 size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan);

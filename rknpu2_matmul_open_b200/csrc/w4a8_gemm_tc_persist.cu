@@ -1,23 +1,27 @@
 // w4a8_gemm_tc_persist.cu -- persistent two-CTA tcgen05 W4A8 GEMM from 17 tokens on (sm_100a).
 //
-// Packed int4 weights -> tensor memory as the A operand, int8 activation codes as shared-memory B operand, kind::i8
-// MMA over a CTA pair with cta_group::2, int32 accumulators in tensor memory, organised so that nothing but the
-// tensor pipe sits on the critical path:
-//   * one cluster of two CTAs per SM pair stays resident and walks a run of 256-channel x (64, 128, 192, 224 or
-//     256)-token tiles; barriers, tensor memory and descriptors are set up once.  Where the tiles are few, K is cut into parts;
-//   * weights and activations travel through SEPARATE rings of bulk copies.  A weight slot is
-//     free again as soon as the unpack warps have read it (the unpacked copy lives in tensor
-//     memory), an activation slot when the MMAs that read it retire.  Together the rings take all of shared memory,
-//     because the copies (L2 hits) take several MMA-stage times to arrive and the pipe starves on a
-//     shallower ring;
-//   * eight dedicated epilogue warps read the accumulator out of tensor memory, hand it back
-//     after the last read and store straight from registers: the 32 lanes of a warp hold 32
-//     neighbouring channels of one token, i.e. 64..128 contiguous bytes per store;
-//   * for SwiGLU the unpack warps place gate channels in lanes 0-15 and the matching up
-//     channels in lanes 16-31 of every tensor-memory lane quarter, so the epilogue pairs them
-//     with one warp shuffle.
-// Outputs: binary16 / fp32 / int32 [M,N], or the fused SwiGLU middle [M,F] fp32 (row maxima
-// collected).
+// Packed int4 weights -> tensor memory as the A operand (int8 weights stay in shared memory), int8 activation codes as
+// shared-memory B operand, kind::i8 MMA over a CTA pair with cta_group::2, int32 accumulators in tensor memory, organised so
+// that nothing but the tensor pipe sits on the critical path:
+//   * one cluster of two CTAs per SM pair stays resident and walks a run of items: 256 channels x up to 64 or 160 tokens (256
+//     with int8 weights), any multiple of 32 of them, so that equal runs leave no nearly empty last round (4096 -> 14336,
+//     2048 tokens: 13 rounds of 128-token tiles for 12.1 of work before).  Barriers, tensor memory and descriptors are set
+//     up once.  Where the tiles are few, K is cut into parts;
+//   * weights and activations travel through SEPARATE rings of bulk copies.  A weight slot is free again as soon as the unpack
+//     warps have read it (the unpacked copy lives in tensor memory), an activation slot when the MMAs that read it retire;
+//   * the MMA issuer is one warp whose every instruction counts: the tensor pipe queues about two MMAs, and what the issuer
+//     does between the last MMA of a stage and the first of the next has to fit under them.  So there is ONE barrier to wait
+//     for (activations and unpacked weights of a stage arrive on the same one) and ONE commit per stage.  (With a barrier and
+//     a commit per operand a stage of two k-blocks cost the issuer 610 cycles where the MMAs of 128 tokens take 512; leaving
+//     the copies, the unpacking or the finishing out changed that by less than 12 %, the waits for operands not at all);
+//   * 160 tokens: two accumulators and three unpacked stages fill tensor memory exactly, and per token the weights are
+//     unpacked, and shared memory is written and read, a quarter less often than with 128 (4096 -> 14336, MMA issue to MMA
+//     issue: 345 cycles per k-block at 128 tokens before, 300 at 128 and 336 of 320 at 160 now, without the finishing);
+//   * eight dedicated epilogue warps read the accumulator out of tensor memory, hand it back after the last read and store
+//     straight from registers.  They read it as fragments of sixteen lanes x 256 bits, and the unpack warps choose which
+//     channel goes to which lane: a thread then holds four neighbouring channels of a token (SwiGLU: two features' gate and up
+//     values), so that nothing has to be exchanged between lanes but row maxima.
+// Outputs: binary16 / fp32 / int32 [M,N], or the fused SwiGLU middle [M,F] fp32 (row maxima collected).
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
 #include "w4a8_rules.h"
@@ -27,42 +31,46 @@
 
 namespace rkb200 {
 
-constexpr int PS_ROLE_WARPS = 4;             // warp 0: activation producer, 1: MMA issuer, 2: weight producer, 3: activation voucher
-constexpr int PS_UNPACK_WARPS = 8;
+constexpr int PS_ROLE_WARPS = 4;             // warp 0: activation producer, 1: MMA issuer, 2: weight producer, 3: voucher
+constexpr int PS_UNPACK_SETS = 2;            // of four warps, taking stages in turn (three: the same time, unpacking no longer bounds it)
+constexpr int PS_UNPACK_WARPS = 4 * PS_UNPACK_SETS;
 // (With twelve or sixteen, at 80 and 72 registers a thread, the finishing gets the issue slots that the unpacking and the MMA
-// issuer need: SwiGLU at 192 tokens 426 -> 458 and 558 us.)
+// issuer need: 160 tokens 4096 -> 14336 80 -> 82 and 83 us, SwiGLU 181 -> 181 and 185.)
 constexpr int PS_EPI_WARPS = 8;
-constexpr int PS_EPI_SETS = PS_EPI_WARPS / 4;  // per tensor-memory lane quarter, taking 32-token chunks in turn
+constexpr int PS_EPI_SETS = PS_EPI_WARPS / 4;  // per tensor-memory lane quarter, taking pieces of sixteen tokens in turn
 constexpr int PS_UNPACK_WARP0 = PS_ROLE_WARPS;
 constexpr int PS_EPI_WARP0 = PS_UNPACK_WARP0 + PS_UNPACK_WARPS;
 constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 640
 constexpr int PS_TMEM_COLS = 512;
+constexpr int PS_SK = 2;                     // k-blocks of a stage
 constexpr unsigned long long PS_DRAIN_NS = 50000;
+constexpr float PS_LOW = 9.5367431640625e-7f;   // 2^-20: the product of two scales of at least that is at least 2^-40
 
-
-// One instantiation's resources.  TOK = tokens of the MMA tile (accumulator columns), half of them in each CTA.
-// Stages are 2 k-blocks.  Tensor memory holds the accumulator (two of them where they fit, so that the epilogue of a
-// segment overlaps the MMAs of the next) and the unpacked weights, 64 columns per stage.
+// One instantiation's resources.  TOK = the widest item (accumulator columns), half of its tokens in each CTA.
+// Tensor memory holds two accumulators, so that the epilogue of an item overlaps the MMAs of the next, and the unpacked int4
+// weights, 64 columns per stage.  (256 tokens leave room for one: for few, long items, whose finishing is not worth hiding.)
+// int8 weights are an operand as they lie in shared memory, in the slot of the activations they are multiplied with.
 template <bool W8, int TOK>
 struct PsShape {
-    static constexpr int T = TOK / 2;                                            // tokens of one CTA's activation tile
-    static constexpr int XA = TOK == 256 ? (W8 ? 3 : 5) : TOK == 224 ? (W8 ? 3 : 4) : TOK == 192 ? (W8 ? 4 : 5) : TOK == 128 && W8 ? 4 : 6;   // activation ring
-    static constexpr int XW = TOK == 256 || W8 ? 4 : TOK >= 128 ? 6 : 8;        // weight ring
-    static constexpr int ACC = TOK > 192 ? 1 : 2;                                // accumulators
-    static constexpr int ABUF = TOK == 64 ? 6 : TOK == 192 ? 2 : 4;              // unpacked weight stages
+    static constexpr int T = TOK / 2;                                            // tokens of one CTA's half
+    static constexpr int ACC = !W8 && TOK == 256 ? 1 : 2;                        // accumulators
+    static constexpr int XA = W8 ? (TOK == 64 ? 5 : 3) : TOK == 64 ? 8 : 4;      // activation ring, stages
+    static constexpr int XW = W8 ? XA : TOK == 64 ? 10 : TOK == 256 ? 6 : 8;     // weight ring
+    static constexpr int ABUF = W8 ? 0 : TOK == 64 ? 6 : TOK == 256 ? 4 : 3;     // unpacked weight stages
+    static constexpr int NR = XA > ABUF ? XA : ABUF;                             // barriers of stages ready for / done by the MMAs
     static constexpr int A_COL0 = ACC * TOK;
-    static constexpr size_t XA_BYTES = 2 * (size_t)T * 128;
+    static constexpr size_t XA_BYTES = PS_SK * (size_t)T * 128;
     static constexpr uint32_t GB = W8 ? 4096 : 2048;                             // one k-block of one 32-channel group
-    static constexpr size_t XW_BYTES = 2 * 4 * (size_t)GB;
-    static constexpr int BARRIERS = 3 * XA + 2 * XW + 2 * ABUF + 2 * ACC;
+    static constexpr size_t XW_BYTES = PS_SK * 4 * (size_t)GB;
+    static constexpr int BARRIERS = XA + 2 * XW + 2 * NR + 2 * ACC;
     static constexpr size_t SMEM = XA * XA_BYTES + XW * XW_BYTES + 2 * TOK * 4 + BARRIERS * 8 + 32;
-    static constexpr size_t SLOT_INTS = 128 * (size_t)TOK;                       // one CTA's partial sums of a segment
+    static_assert(TOK % 32 == 0 && TOK <= 256, "not the width of an MMA");
     static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
     static_assert(A_COL0 + 64 * ABUF <= PS_TMEM_COLS, "exceeds tensor memory");
-    // The two unpack sets take alternate stages, so with an even ring every slot belongs to one set, which sees all of its
-    // phases.  (With an odd one a set could ask for a slot's second phase while the first, the other set's, is still open;
-    // a parity wait takes that for completed.)
-    static_assert(XW % 2 == 0 && ABUF % 2 == 0, "a ring slot would change between the unpack sets");
+    // The two unpack sets take alternate stages, so with an even ring every weight slot belongs to one set, which sees all of
+    // its phases.  (With an odd one a set could ask for a slot's second phase while the first, the other set's, is still
+    // open; a parity wait takes that for completed.  The barriers of retired MMAs complete in order, whoever waits.)
+    static_assert(W8 || XW % PS_UNPACK_SETS == 0, "a ring slot would change between the unpack sets");
 };
 
 // A position in a ring of N barriers: slot and phase parity.
@@ -103,27 +111,41 @@ __device__ __forceinline__ bool epilogue_any(bool here)
     return any != 0;
 }
 
+// Four neighbouring channels of one token, held in the order (turn, turn + 1, ...) mod 4, in one store.
+__device__ __forceinline__ void store_four(uint32_t* dst, const uint32_t (&held)[4], int turn)
+{
+    uint32_t half[4], v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) half[i] = turn & 1 ? held[(i + 3) & 3] : held[i];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = turn & 2 ? half[(i + 2) & 3] : half[i];
+    *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void store_four_halves(__half* dst, uint32_t held01, uint32_t held23, int turn)
+{
+    // channel i is held at (i - turn) mod 4
+    const uint32_t a = (0u - turn) & 3u, b = (1u - turn) & 3u, c = (2u - turn) & 3u, d = (3u - turn) & 3u;
+    *reinterpret_cast<uint2*>(dst) = make_uint2(__byte_perm(held01, held23, 0x1010u + 0x22u * a + 0x2200u * b), __byte_perm(held01, held23, 0x1010u + 0x22u * c + 0x2200u * d));
+}
+
 // (Linear and SwiGLU launches have kernels of their own: less to fetch, and neither finishing pays for the other's registers.)
-// W8: the weights are int8 codes in the W8 layout (w8a8_kernels.cu): "unpacking" is a copy into tensor memory and the sums
-// are not scaled by 16.
+// W8: the weights are int8 codes in the W8 layout (w8a8_kernels.cu), and the sums are not scaled by 16.
 template <bool W8, bool SWIGLU, int TOK>
-__global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const GemmParams p, int num_clusters)
+__global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const GemmParams p, const __grid_constant__ PersistMaps maps, int num_clusters)
 {
     using S = PsShape<W8, TOK>;
     constexpr uint32_t GB = S::GB;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* const acts = smem;
     uint8_t* const wts = acts + S::XA * S::XA_BYTES;
-    float* const s_sx = reinterpret_cast<float*>(wts + S::XW * S::XW_BYTES);     // token scales of the tile being finished
-    uint32_t* const s_tilemax = reinterpret_cast<uint32_t*>(s_sx + TOK);         // SwiGLU: the CTA's row maxima of that tile
-    uint64_t* const xfull = reinterpret_cast<uint64_t*>(s_tilemax + TOK);
-    uint64_t* const xempty = xfull + S::XA;
-    uint64_t* const x_ready = xempty + S::XA;    // leader: both CTAs' activations of the stage have landed
-    uint64_t* const wfull = x_ready + S::XA;
+    float* const s_sx = reinterpret_cast<float*>(wts + S::XW * S::XW_BYTES);     // token scales of the item being finished
+    uint32_t* const s_tilemax = reinterpret_cast<uint32_t*>(s_sx + TOK);         // SwiGLU: the CTA's row maxima of that item
+    uint64_t* const xfull = reinterpret_cast<uint64_t*>(s_tilemax + TOK);        // W8: the weights of the stage as well
+    uint64_t* const wfull = xfull + S::XA;
     uint64_t* const wempty = wfull + S::XW;
-    uint64_t* const a_ready = wempty + S::XW;    // leader: both CTAs' weights of the stage are in tensor memory
-    uint64_t* const a_free = a_ready + S::ABUF;
-    uint64_t* const acc_full = a_free + S::ABUF;
+    uint64_t* const ready = wempty + S::XW;      // leader: both CTAs' operands of the stage are where the MMAs read them
+    uint64_t* const done = ready + S::NR;        // the stage's MMAs have retired: its operands may be overwritten
+    uint64_t* const acc_full = done + S::NR;
     uint64_t* const acc_empty = acc_full + S::ACC;
     uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(acc_empty + S::ACC);
     int* const s_error = reinterpret_cast<int*>(s_tmem + 1);
@@ -135,30 +157,40 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     const int cluster_id = blockIdx.x >> 1;
     constexpr bool swiglu = SWIGLU;
     const int KB = p.KB;
-    const int nst = (KB + 1) / 2;                                      // stage iterations per tile
+    const int nst = (KB + PS_SK - 1) / PS_SK;                          // stages of a tile
     const int tiles_n = swiglu ? (p.F + 63) / 64 : (p.N + TILE_N - 1) / TILE_N;
     const int pairs_n = (tiles_n + 1) / 2;
-    const int pairs_m = (p.M + TOK - 1) / TOK;
-    // Every cluster takes a run of whole tiles, or (split > 1) one of the `split` parts of one tile's stages.
-    const int tiles = pairs_n * pairs_m, split = p.split;
+    // Every cluster takes a run of items over all of K, or (split > 1) one of the `split` parts of one tile's stages.
+    const int per_tile = (p.M + p.unit - 1) / p.unit, split = p.split;
+    const unsigned units = (unsigned)pairs_n * (unsigned)per_tile;
     const int part = cluster_id % split;
-    const int tile0 = split > 1 ? cluster_id / split : (int)((long long)tiles * cluster_id / num_clusters);
-    const int it0 = nst * part / split;
-    const int n_items = split > 1 ? nst * (part + 1) / split - it0 : ((int)((long long)tiles * (cluster_id + 1) / num_clusters) - tile0) * nst;
+    const int it0 = nst * part / split, it1 = nst * (part + 1) / split;
+    const unsigned unit0 = split > 1 ? (unsigned)(cluster_id / split) : persist_bound(units, per_tile, p.snap, cluster_id, num_clusters);
+    const unsigned unit1 = split > 1 ? unit0 + 1 : persist_bound(units, per_tile, p.snap, cluster_id + 1, num_clusters);
+    // an item: pair of channel tiles, first token, tokens the MMAs take (a multiple of 32)
+    struct Item { int tile, tok0, width; };
+    PersistItems items(unit0, unit1, per_tile, p.most);
+    auto next_item = [&](Item& item) -> bool {
+        int first, n;
+        if (!items.next(item.tile, first, n)) return false;
+        item.tok0 = first * p.unit;
+        item.width = min(n * p.unit, (p.M - item.tok0 + 31) & ~31);
+        return true;
+    };
+    Item item;
     const unsigned long long deadline = global_ns() + p.timeout_ns;
-    // optional cycle stamps of cluster 0's leader: [segment j < 16][8] = MMA wait-begin, MMA first issue,
-    // MMA last commit, epilogue acc_full seen, tensor memory handed back, stored, [6] cycles the MMA
-    // issuer waited for operands; [128] / [129] cycles unpack warp 0 waited for weights / for a free
-    // tensor-memory buffer, [160] cycles for activations; [200] = clusters in the grid
+    // optional cycle stamps of cluster 0's leader: [item j < 16][8] = MMA issuer begins, [2] its last
+    // commit, [3] epilogue sees the accumulator, [4] tensor memory handed back, [5] stored; [128] / [129] cycles unpack warp 0 waited
+    // for weights / for a free tensor-memory buffer, [160] cycles for activations; [200] = clusters in the grid
     unsigned long long* const trace = (p.trace && blockIdx.x == 0) ? p.trace : nullptr;
     const long long c0 = clock64();
 #define PS_STAMP(j, slot) do { if (trace && (j) < 16) trace[(j) * 8 + (slot)] = (unsigned long long)(clock64() - c0); } while (0)
     if (trace && tid == 0) trace[200] = (unsigned long long)num_clusters;
 
     if (tid == 0) {
-        for (int s = 0; s < S::XA; ++s) { mbar_init(&xfull[s], 1); mbar_init(&xempty[s], 1); mbar_init(&x_ready[s], 2); }
+        for (int s = 0; s < S::XA; ++s) mbar_init(&xfull[s], W8 ? 2 : 1);
         for (int s = 0; s < S::XW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 4); }
-        for (int b = 0; b < S::ABUF; ++b) { mbar_init(&a_ready[b], 8); mbar_init(&a_free[b], 1); }
+        for (int b = 0; b < S::NR; ++b) { mbar_init(&ready[b], (W8 ? 0 : 8) + 2); mbar_init(&done[b], 1); }
         for (int b = 0; b < S::ACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * PS_EPI_WARPS); }   // every epilogue warp of both CTAs
         mbar_fence_init();
         *s_error = 0;
@@ -188,195 +220,224 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         // (the whole warp walks the loop and one elected lane issues, as in the MMA issuer below: copy requests take their
         // operands from uniform registers, and four lanes issuing one request each took 1000 cycles per stage)
         RingPos<S::XW> r;
-        int it = it0;
-        bool ok = true, live = true;
-        const uint8_t* src = nullptr;                              // group 0 of this CTA's channel tile, stage `it`
+        bool ok = true, live = true, asked = false;
+        int g = 0;
         const size_t group_bytes = (size_t)KB * GB;
         const size_t upper = swiglu ? (size_t)(p.F / GROUP) * group_bytes : 2 * group_bytes;   // groups 2, 3 behind groups 0, 1
-        for (int gi = 0, tile = tile0; gi < n_items; ++gi, r.next()) {
-            if (gi == S::XW) {
-                live = dependency_met();
-                if (!live) break;
+        while (live && ok && next_item(item)) {
+            const int ct = 2 * item.tile + (int)rank;
+            const uint8_t* src = p.Wp + (size_t)(swiglu ? ct * 2 : ct * 4) * group_bytes + (size_t)it0 * (W8 ? 4 : 1) * PS_SK * GB;
+            for (int it = it0; it < it1; ++it, ++g, r.next()) {
+                if (g == S::XW) {
+                    live = dependency_met();
+                    asked = true;
+                    if (!live) break;
+                }
+                const uint32_t bytes = (uint32_t)min(PS_SK, KB - PS_SK * it) * GB;
+                if (g >= S::XW) ok = __all_sync(0xffffffffu, W8 ? mbar_wait_cluster(&done[r.slot], r.phase ^ 1u, deadline) : mbar_wait(&wempty[r.slot], r.phase ^ 1u, deadline));
+                if (!ok) { *s_error = 1; break; }
+                uint8_t* const dst = wts + (size_t)r.slot * S::XW_BYTES;
+                if (elect_one()) {
+                    if constexpr (W8) {                        // a k-block of a channel tile is contiguous
+                        mbar_arrive_expect_tx(&xfull[r.slot], 4u * bytes);
+                        bulk_g2s(dst, src, 4u * bytes, &xfull[r.slot]);
+                    } else {
+                        mbar_arrive_expect_tx(&wfull[r.slot], 4u * bytes);
+                        bulk_g2s(dst, src, bytes, &wfull[r.slot]);
+                        bulk_g2s(dst + PS_SK * GB, src + group_bytes, bytes, &wfull[r.slot]);
+                        bulk_g2s(dst + 2 * PS_SK * GB, src + upper, bytes, &wfull[r.slot]);
+                        bulk_g2s(dst + 3 * PS_SK * GB, src + upper + group_bytes, bytes, &wfull[r.slot]);
+                    }
+                }
+                __syncwarp();
+                src += (W8 ? 4 : 1) * PS_SK * GB;
             }
-            if (src == nullptr) {
-                const int ct = 2 * (tile % pairs_n) + (int)rank;
-                src = p.Wp + (size_t)(swiglu ? ct * 2 : ct * 4) * group_bytes + (size_t)it * 2 * GB;
-            }
-            const uint32_t bytes = (uint32_t)min(2, KB - 2 * it) * GB;
-            if (gi >= S::XW) ok = __all_sync(0xffffffffu, mbar_wait(&wempty[r.slot], r.phase ^ 1u, deadline));
-            if (!ok) { *s_error = 1; break; }
-            uint8_t* const dst = wts + (size_t)r.slot * S::XW_BYTES;
-            if (elect_one()) {
-                mbar_arrive_expect_tx(&wfull[r.slot], 4u * bytes);
-                bulk_g2s(dst, src, bytes, &wfull[r.slot]);
-                bulk_g2s(dst + 2 * GB, src + group_bytes, bytes, &wfull[r.slot]);
-                bulk_g2s(dst + 4 * GB, src + upper, bytes, &wfull[r.slot]);
-                bulk_g2s(dst + 6 * GB, src + upper + group_bytes, bytes, &wfull[r.slot]);
-            }
-            __syncwarp();
-            src += 2 * GB;
-            if (++it == nst) { it = 0; ++tile; src = nullptr; }
         }
-        if (n_items <= S::XW) live = dependency_met();
-        if (!live && lane == 0)   // nobody will consume: let the copies already requested land before leaving
-            for (int s = 0; s < min(n_items, S::XW); ++s)
+        if (!asked) live = dependency_met();
+        if (!live && !W8 && lane == 0)   // nobody will consume: let the copies already requested land before leaving
+            for (int s = 0; s < min(g, S::XW); ++s)
                 if (!mbar_wait(&wfull[s], 0, deadline)) { *s_error = 1; break; }
+        if (!live && W8) {               // (their barriers wait for the activations' half as well, which does not come)
+            if (lane == 0)
+                for (int s = 0; s < min(g, S::XW); ++s) {
+                    mbar_arrive(&xfull[s]);
+                    if (!mbar_wait(&xfull[s], 0, deadline)) { *s_error = 1; break; }
+                }
+        }
     } else if (warp == 0) {
         // ---------------------------------------------------------------- activation producer
         if (dependency_met()) {
             RingPos<S::XA> r;
-            int it = it0;
-            const uint8_t* src = nullptr;
-            for (int gi = 0, tile = tile0; gi < n_items; ++gi, r.next()) {
-                if (src == nullptr) src = p.Xq + ((size_t)(2 * (tile / pairs_n) + (int)rank) * KB + (size_t)it * 2) * (S::T * 128);
-                const uint32_t bytes = (uint32_t)min(2, KB - 2 * it) * S::T * 128u;
-                bool ok = true;
-                if (gi >= S::XA) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&xempty[r.slot], r.phase ^ 1u, deadline));
-                if (!ok) { *s_error = 1; break; }
-                if (elect_one()) {
-                    mbar_arrive_expect_tx(&xfull[r.slot], bytes);
-                    bulk_g2s(acts + (size_t)r.slot * S::XA_BYTES, src, bytes, &xfull[r.slot]);
+            bool ok = true;
+            int g = 0;
+            while (ok && next_item(item)) {
+                const int groups = item.width / 16;            // of this CTA's half
+                const int row0 = item.tok0 / 8 + (int)rank * groups;
+                for (int it = it0; it < it1; ++it, ++g, r.next()) {
+                    if (g >= S::XA) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&done[(g - S::XA) % S::NR], (g - S::XA) / S::NR & 1, deadline));
+                    if (!ok) { *s_error = 1; break; }
+                    if (elect_one()) {
+                        // (a stage's second k-block that does not exist is filled with zeros)
+                        mbar_arrive_expect_tx(&xfull[r.slot], (uint32_t)groups * (PS_SK * 1024u));
+                        uint8_t* dst = acts + (size_t)r.slot * S::XA_BYTES;
+                        int row = row0, left = groups;
+                        for (; left >= 8; left -= 8, row += 8, dst += 8 * PS_SK * 1024) tensor_g2s(dst, &maps.box[0], it * PS_SK * 128, row, &xfull[r.slot]);
+                        if (left & 4) { tensor_g2s(dst, &maps.box[1], it * PS_SK * 128, row, &xfull[r.slot]); row += 4; dst += 4 * PS_SK * 1024; }
+                        if (left & 2) tensor_g2s(dst, &maps.box[2], it * PS_SK * 128, row, &xfull[r.slot]);
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
-                src += S::XA_BYTES;
-                if (++it == nst) { it = 0; ++tile; src = nullptr; }
             }
             // The MMAs' commits arrive on this CTA's barriers asynchronously, the peer's among them: the CTA may not leave
             // (and its shared memory change hands) before the last of them is here.
-            for (int gi = n_items; gi < n_items + S::XA && !*reinterpret_cast<volatile int*>(s_error); ++gi, r.next())
-                if (gi >= S::XA && !mbar_wait_cluster(&xempty[r.slot], r.phase ^ 1u, deadline)) *s_error = 1;
+            for (int k = max(0, g - S::XA); k < g && !*reinterpret_cast<volatile int*>(s_error); ++k)
+                if (!mbar_wait_cluster(&done[k % S::NR], k / S::NR & 1, deadline)) *s_error = 1;
         }
     } else if (warp == 3) {
-        // ---------------------------------------------------------------- activation voucher
-        // The leader's MMAs read both CTAs' activations: this warp passes on that this CTA's copy has landed.  It runs
+        // ---------------------------------------------------------------- voucher
+        // The leader's MMAs read both CTAs' shared memory: this warp passes on that this CTA's copies have landed.  It runs
         // ahead of the MMAs by the depth of the ring.  (When the unpack warps vouched for it, with an arrival that released
         // everything at cluster scope, that release bounded the whole loop: 730 cycles per k-block at K = 11008 against 525.)
         if (dependency_met() && lane == 0) {
             RingPos<S::XA> r;
+            RingPos<S::NR> to;
             long long waited = 0;
-            for (int gi = 0; gi < n_items; ++gi, r.next()) {
-                const long long w0 = trace ? clock64() : 0;
-                if (!mbar_wait(&xfull[r.slot], r.phase, deadline)) { *s_error = 1; break; }
-                if (trace) waited += clock64() - w0;
-                if (rank != 0) mbar_arrive_remote(&x_ready[r.slot], 0); else mbar_arrive(&x_ready[r.slot]);
-            }
+            bool ok = true;
+            while (ok && next_item(item))
+                for (int it = it0; it < it1; ++it, r.next(), to.next()) {
+                    const long long w0 = trace ? clock64() : 0;
+                    ok = mbar_wait(&xfull[r.slot], r.phase, deadline);
+                    if (!ok) { *s_error = 1; break; }
+                    if (trace) waited += clock64() - w0;
+                    if (rank != 0) mbar_arrive_remote(&ready[to.slot], 0); else mbar_arrive(&ready[to.slot]);
+                }
             if (trace) trace[160] = (unsigned long long)waited;
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (leader CTA)
         // The whole warp walks the loop, so that descriptors and addresses are warp-uniform values, and one elected lane
         // issues.  (A loop that only lane 0 enters moves every operand of every MMA into uniform registers first: 85
-        // cycles per MMA, which bounded a stage at 1190 cycles whatever the token tile; 1050 now at 256 tokens, of 1024.)
+        // cycles per MMA.)  Everything a stage needs is known before the one in front is issued; what stands between two
+        // stages' MMAs is one wait, one commit and a few additions.
         if (dependency_met() && rank == 0) {
-            const uint32_t idesc = tc_idesc_s8(256, TOK);
-            bool ok = true;
-            RingPos<S::XA> rx;
-            RingPos<S::ABUF> ra;
+            bool dead = false;                                     // (the elected lane's, always the same one)
             RingPos<S::ACC> rc;
-            int it = it0;
-            for (int gi = 0, j = 0; gi < n_items && ok; ++j, rc.next()) {
-                const int n = min(nst - it, n_items - gi);
+            const uint32_t ready0 = smem_u32(ready), done0 = smem_u32(done);
+            const uint64_t b_first = tc_smem_desc(smem_u32(acts), 128u, PS_SK * 1024u);
+            const uint64_t a_first = tc_smem_desc(smem_u32(wts), 2048u, 128u);        // W8
+            const uint32_t b_hi = (uint32_t)(b_first >> 32), a_hi = (uint32_t)(a_first >> 32);
+            const uint32_t b_lo0 = (uint32_t)b_first, a_lo0 = (uint32_t)a_first;
+            const uint32_t b_lo_end = b_lo0 + (uint32_t)(S::XA * S::XA_BYTES / 16);
+            const uint32_t a_tmem0 = tmem_base + S::A_COL0;
+            uint32_t b_lo = b_lo0, a_lo = a_lo0, a_tmem = a_tmem0, bar = 0, phase = 0;
+            for (int j = 0; next_item(item); ++j, rc.next()) {
+                const uint32_t idesc = tc_idesc_s8(256, item.width);
                 if (lane == 0) PS_STAMP(j, 0);
-                if (j >= S::ACC) {   // the epilogue warps of both CTAs have read this accumulator's previous segment
-                    ok = __all_sync(0xffffffffu, mbar_wait_cluster(&acc_empty[rc.slot], rc.phase ^ 1u, deadline));
-                    if (!ok) { *s_error = 1; break; }
+                if (j >= S::ACC) {   // the epilogue warps of both CTAs have read this accumulator's previous item
+                    if (!__all_sync(0xffffffffu, mbar_wait_cluster(&acc_empty[rc.slot], rc.phase ^ 1u, deadline))) { *s_error = 1; break; }
                     tc_fence_after();
                 }
                 const uint32_t d_tmem = tmem_base + rc.slot * TOK;
-                long long waited = 0;
-                for (int i = 0; i < n; ++i, ++it, rx.next(), ra.next()) {
-                    const int kbs = min(2, KB - 2 * it);
-                    const long long w0 = trace ? clock64() : 0;
-                    ok = mbar_wait_cluster(&x_ready[rx.slot], rx.phase, deadline) && mbar_wait_cluster(&a_ready[ra.slot], ra.phase, deadline);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (trace) waited += clock64() - w0;
-                    if (!ok) { *s_error = 1; break; }
-                    if (i == 0 && lane == 0) PS_STAMP(j, 1);
-                    tc_fence_after();
-                    const uint32_t xaddr = smem_u32(acts + (size_t)rx.slot * S::XA_BYTES);
-                    const uint32_t a_tmem = tmem_base + S::A_COL0 + ra.slot * 64;
-                    // k-step q: k-block q / 4 of the stage, 32 k = two 16-byte chunks per token: the descriptor's
-                    // address field advances by 2 * T (16-byte units) per step
-                    const uint64_t desc0 = tc_smem_desc(xaddr, S::T * 16u, 128u);
+                const bool odd_end = (KB & 1) && it1 == nst;       // the last stage has one k-block
+                for (int it = it0; it < it1; ++it) {
+                    // k-step q: 32 k = two 16-byte chunks per row: the descriptors' address fields advance by two core
+                    // matrices of the activations, by two 128-channel columns of int8 weights
+                    const uint64_t b_desc = (uint64_t)b_hi << 32 | b_lo, a_desc = (uint64_t)a_hi << 32 | a_lo;
+                    const uint32_t a_now = a_tmem;
+                    const bool whole = !(odd_end && it == nst - 1);
                     if (elect_one()) {
-                        tc_mma_i8_ts_pair(d_tmem, a_tmem, desc0, idesc, i > 0 ? 1u : 0u);
+                        if (!dead && !mbar_wait_cluster_at(ready0 + bar, phase, deadline)) { *s_error = 1; dead = true; }
+                        if (!dead) {
+                            tc_fence_after();
+                            if constexpr (W8) {
+                                tc_mma_i8_ss_pair(d_tmem, a_desc, b_desc, idesc, it != it0 ? 1u : 0u);
 #pragma unroll
-                        for (int q = 1; q < 4; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_tmem + q * 8, desc0 + (uint64_t)(q * 2 * S::T), idesc);
-                        if (kbs == 2) {
+                                for (int q = 1; q < 4; ++q) tc_mma_i8_ss_pair(d_tmem, a_desc + 256u * q, b_desc + 16u * q, idesc, 1u);
+                                if (whole) {
 #pragma unroll
-                            for (int q = 4; q < 8; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_tmem + q * 8, desc0 + (uint64_t)(q * 2 * S::T), idesc);
+                                    for (int q = 4; q < 8; ++q) tc_mma_i8_ss_pair(d_tmem, a_desc + 256u * q, b_desc + 16u * q, idesc, 1u);
+                                }
+                            } else {
+                                tc_mma_i8_ts_pair(d_tmem, a_now, b_desc, idesc, it != it0 ? 1u : 0u);
+#pragma unroll
+                                for (int q = 1; q < 4; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_now + 8 * q, b_desc + 16u * q, idesc);
+                                if (whole) {
+#pragma unroll
+                                    for (int q = 4; q < 8; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_now + 8 * q, b_desc + 16u * q, idesc);
+                                }
+                            }
+                            tc_commit_pair_at(done0 + bar);   // in both CTAs: the stage's operands may be overwritten once these MMAs retire
+                            if (it == it1 - 1) tc_commit_pair(&acc_full[rc.slot]);
                         }
-                        tc_commit_pair(&xempty[rx.slot]);   // the activation stage may be refilled once these MMAs retire
-                        tc_commit_pair(&a_free[ra.slot]);   // and the weight buffer rewritten, in both CTAs
-                        if (i == n - 1) tc_commit_pair(&acc_full[rc.slot]);
                     }
-                    __syncwarp();
+                    bar = bar == (S::NR - 1) * 8 ? 0 : bar + 8;
+                    phase ^= bar == 0 ? 1u : 0u;
+                    b_lo += (uint32_t)(S::XA_BYTES / 16);
+                    if (W8) a_lo += (uint32_t)(S::XW_BYTES / 16);
+                    if (b_lo == b_lo_end) { b_lo = b_lo0; a_lo = a_lo0; }
+                    if constexpr (!W8) a_tmem = a_tmem == a_tmem0 + (S::ABUF - 1) * 64 ? a_tmem0 : a_tmem + 64;
                 }
-                if (!ok) break;
-                if (lane == 0) {
-                    PS_STAMP(j, 2);
-                    if (trace && j < 16) trace[j * 8 + 6] = (unsigned long long)waited;
-                }
-                gi += n;
-                if (it == nst) it = 0;
+                __syncwarp();
+                if (lane == 0) PS_STAMP(j, 2);
             }
         }
     } else if (warp < PS_EPI_WARP0) {
         // ---------------------------------------------------------------- weight unpack -> TMEM
+        if constexpr (!W8) {
         const int q = warp & 3;
         const int set = (warp - PS_UNPACK_WARP0) >> 2;
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-        // which rows of the staged weight groups feed this thread's tensor-memory lane:
-        // plain: group q, row lane.  SwiGLU: lanes 0-15 gate rows, lanes 16-31 the matching
-        // up rows (staged groups 0,1 = gate, 2,3 = up of the same 64 features).
+        // Which row of the staged weight groups feeds this thread's tensor-memory lane.  The epilogue's thread t reads lanes
+        // t / 4 + 8 c; they hold channels 4 (t / 4) .. + 3 of the warp's group, or (SwiGLU) features 2 (t / 4), + 1 of sixteen,
+        // gate values in lanes 0-15 and up values in lanes 16-31 (staged groups 0, 1 = gate, 2, 3 = up of the same 64
+        // features).  The order inside those four (two) turns with t, so that eight neighbouring lanes read rows that are
+        // different modulo eight: no bank conflicts.
+        const int i8 = lane & 7;
         const int src_group = swiglu ? (q >> 1) + (lane >= 16 ? 2 : 0) : q;
-        const int src_row = swiglu ? (q & 1) * 16 + (lane & 15) : lane;
+        const int src_row = swiglu ? (q & 1) * 16 + 2 * i8 + (((lane >> 3) + (i8 >> 2)) & 1) : 4 * i8 + (((lane >> 3) + (i8 >> 1)) & 3);
         const bool tr = trace && warp == PS_UNPACK_WARP0 && lane == 0;
         long long wait_full = 0, wait_free = 0;
         RingPos<S::XW> rw;
-        RingPos<S::ABUF> ra;
         // The two sets take alternate stages.  A stage's packed words are read from shared memory while the previous
         // stage's stores to tensor memory are still on their way, so that the two latencies overlap.
-        constexpr int NV = W8 ? 16 : 8;                        // 16-byte pieces a lane takes from a stage
-        uint4 w[NV];
+        uint4 w[4 * PS_SK];                                    // 16-byte pieces of this lane's row
         bool ok = true;
-        auto fetch = [&](int it) {
-            const int kbs = min(2, KB - 2 * it);
+        int n_stages = (int)(unit1 - unit0);                   // one item a unit, or fewer
+        if (p.most != 1)
+            for (n_stages = 0; next_item(item);) ++n_stages;
+        n_stages *= it1 - it0;
+        int it = it0;
+        auto advance = [&]() { rw.next(); if (++it == it1) it = it0; };
+        auto fetch = [&]() {
+            const int kbs = min(PS_SK, KB - PS_SK * it);
             const long long w0 = tr ? clock64() : 0;
             ok = __all_sync(0xffffffffu, mbar_wait(&wfull[rw.slot], rw.phase, deadline));
             if (tr) wait_full += clock64() - w0;
-            const uint4* src = reinterpret_cast<const uint4*>(wts + (size_t)rw.slot * S::XW_BYTES + src_group * 2 * GB) + src_row;
+            const uint4* src = reinterpret_cast<const uint4*>(wts + (size_t)rw.slot * S::XW_BYTES + src_group * PS_SK * GB) + src_row;
 #pragma unroll
-            for (int c = 0; c < NV; ++c) w[c] = (c < NV / 2 * kbs) ? src[c * 32] : make_uint4(0u, 0u, 0u, 0u);
+            for (int c = 0; c < 4 * PS_SK; ++c) w[c] = (c < 4 * kbs) ? src[c * 32] : make_uint4(0u, 0u, 0u, 0u);
         };
-        int it = it0;
-        auto advance = [&]() { rw.next(); ra.next(); if (++it == nst) it = 0; };
-        if (set == 1) advance();
-        if (set < n_items) fetch(it);
-        for (int g = set; g < n_items && ok; g += 2) {
-            const int kbs = min(2, KB - 2 * it), b = ra.slot;
+        for (int k = 0; k < set; ++k) advance();
+        if (set < n_stages) fetch();
+        for (int g = set; g < n_stages && ok; g += PS_UNPACK_SETS) {
+            const int kbs = min(PS_SK, KB - PS_SK * it), b = g % S::ABUF;
+            const bool reuse = g >= S::ABUF;
             // (before the first buffer comes back from the MMAs, which need the activations)
-            if ((g == S::ABUF || g == S::ABUF + 1) && !dependency_met()) break;
+            if (reuse && g - PS_UNPACK_SETS < S::ABUF && !dependency_met()) break;
             const long long w0 = tr ? clock64() : 0;
-            if (g >= S::ABUF) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&a_free[b], ra.phase ^ 1u, deadline));
+            if (reuse) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&done[(g - S::ABUF) % S::NR], (g - S::ABUF) / S::NR & 1, deadline));
             if (tr) wait_free += clock64() - w0;
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < PS_SK; ++h)
                 if (h < kbs) {
-                    uint32_t r[32];
-                    if constexpr (W8) {
-                        // int8 codes: a lane's sixteen 16-byte pieces of the stage are the words of its tensor-memory row in order
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            const uint4 v = w[8 * h + c];
-                            r[4 * c] = v.x; r[4 * c + 1] = v.y; r[4 * c + 2] = v.z; r[4 * c + 3] = v.w;
-                        }
-                    } else {
+                    for (int e = 0; e < 2; ++e) {              // (sixteen columns at a time: fewer registers)
+                        uint32_t r[16];
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const uint4 v = w[4 * h + c];
+                        for (int c = 0; c < 2; ++c) {
+                            const uint4 v = w[4 * h + 2 * e + c];
                             const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                             for (int jj = 0; jj < 4; ++jj) {
@@ -384,137 +445,152 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                                 r[c * 8 + 4 + jj] = ww[jj] & 0xF0F0F0F0u;
                             }
                         }
+                        tc_st16(lane_addr + S::A_COL0 + b * 64 + h * 32 + e * 16, r);
                     }
-                    tc_st32(lane_addr + S::A_COL0 + b * 64 + h * 32, r);
                 }
-            }
             __syncwarp();
             if (lane == 0) mbar_arrive(&wempty[rw.slot]);      // the packed copy has been read
-            advance();
-            advance();
-            if (g + 2 < n_items) fetch(it);
+#pragma unroll
+            for (int k = 0; k < PS_UNPACK_SETS; ++k) advance();
+            if (g + PS_UNPACK_SETS < n_stages) fetch();
             tc_wait_st();
             tc_fence_before();
             // Tensor-memory writes are ordered by the wait and the fences; the arrival itself carries nothing, so it is
             // relaxed (see mbar_arrive_remote for what a release at cluster scope costs).
             __syncwarp();
-            if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(&a_ready[b], 0); else mbar_arrive_relaxed(&a_ready[b]); }
+            if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(&ready[g % S::NR], 0); else mbar_arrive_relaxed(&ready[g % S::NR]); }
         }
         if (!ok) *s_error = 1;
-        // (the commits on the buffers have to be here before the CTA leaves, as for the activation ring; none come where
-        // the input was rejected)
-        if (ok && dependency_met())
-            for (int g = n_items + ((n_items ^ set) & 1); g < n_items + S::ABUF; g += 2, ra.next(), ra.next())
-                if (g >= S::ABUF && !mbar_wait_cluster(&a_free[ra.slot], ra.phase ^ 1u, deadline)) { *s_error = 1; break; }
         if (tr) { trace[128] = (unsigned long long)wait_full; trace[129] = (unsigned long long)wait_free; }
+        }
     } else {
         // ---------------------------------------------------------------- epilogue warps
-        // A warp finishes sixteen tokens (of its 32 accumulator rows) per turn of a rolled loop.  What bounds it is the
-        // number of instructions: eight warps share the issue slots with the unpack warps, so the arithmetic works on pairs
-        // of tokens (one instruction per two operations), the int4 records' 1/16 is in the token scales, one look at the
-        // magnitudes of four gate values settles that none needs the slow division, and maxima are taken of floats, whose
-        // signs the instruction drops (4096 tokens, 4096 -> 2 x 14336: 424 -> 405 us; 300 tokens 54.4 -> 49.6).
+        // A warp finishes sixteen tokens of its 32 accumulator rows per turn of a rolled loop.  What bounds it is the
+        // number of instructions: eight warps share the issue slots with the unpack warps and the MMA issuer, so nothing is
+        // exchanged between lanes but row maxima, the arithmetic works on pairs of tokens (one instruction per two
+        // operations), the int4 records' 1/16 is in the token scales, one look at the largest magnitude of eight gate values
+        // settles that none needs the slow division, and maxima are taken of floats, whose signs the instruction drops.
+        // (Small ones are settled by the scales: a sum is zero, where the fast form is exact, or at least one.  Looking for
+        // the smallest magnitude as well sent every fourth turn to the slow form, one sum in eight hundred being zero.)
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
-        const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes 32-token chunks eset, eset + PS_EPI_SETS, ...
+        const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes pieces eset, eset + PS_EPI_SETS, ...
         const int sid = (warp - PS_EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const int out_cols = swiglu ? p.F : p.N;
-        // output column (inside the CTA's tile) this thread's accumulator row belongs to
-        const int col = swiglu ? (q >> 1) * 32 + (q & 1) * 16 + (lane & 15) : q * 32 + lane;
-        const bool up_lane = swiglu && lane >= 16;
-        const int odd = lane & 1;
-        const bool quad_ok = (out_cols % 4 == 0) && (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
-        constexpr int STEP = 32 * PS_EPI_SETS;
-        constexpr int SHIFT = W8 ? 0 : 4;             // int4 records enter the MMA times 16
+        // This thread's fragment: channels 4 i8 .. + 3 of its group (features 2 i8, + 1 of sixteen), the one in its c-th
+        // tensor-memory lane is number (c + turn) of them; tokens 2 tq, 2 tq + 1 and eight further of a piece.
+        const int i8 = lane >> 2, tq = lane & 3;
+        const int turn = W8 ? 0 : swiglu ? i8 >> 2 : i8 >> 1;
+        const int col = swiglu ? q * 16 + 2 * i8 : q * 32 + 4 * i8;      // its first channel inside the CTA's tile
+        const int holder = 8 * (((lane & 3) - (W8 ? 0 : lane >> 3)) & 3) + (lane >> 2);       // the tensor-memory lane of the group's channel `lane`
+        constexpr int CH = swiglu ? 2 : 4;
+        const size_t elem = swiglu || p.epi != EPI_F16 ? 4 : 2;
+        // All of them in one store; where the rows do not allow it a thread takes sixteen tokens of one channel instead, and a
+        // warp's store covers 32 neighbouring channels of a token, in order (224 tokens of fp32 3070 -> 4911 20 us; 28 with
+        // four scattered stores a token, and with the channels in the order of the tensor-memory lanes).
+        const bool wide_ok = out_cols % CH == 0 && reinterpret_cast<uintptr_t>(p.out) % (CH * elem) == 0;
+        const bool fragments = swiglu || wide_ok;
+        constexpr int STEP = 16 * PS_EPI_SETS;
+        constexpr int SHIFT = W8 ? 0 : 4;              // int4 records enter the MMA times 16
         bool ok = dependency_met();
         RingPos<S::ACC> rc;
-        int tile = tile0, it = it0;
-        for (int gi = 0, j = 0; gi < n_items && ok; ++j, rc.next()) {
-            const int n_seg = min(nst - it, n_items - gi);
-            const int ct = 2 * (tile % pairs_n) + (int)rank;
-            const int tok_base = (tile / pairs_n) * TOK;
-            const int col0 = swiglu ? ct * 64 : ct * TILE_N;
-            const int n = col0 + col;
-            const bool n_ok = n < out_cols;
-            const float sw = n_ok ? p.sw[(up_lane ? p.F : 0) + n] : 0.f;
-            // 32-token chunks of this warp that hold live tokens: those at 32 eset + STEP c, c < chunks
-            const int chunks = max(0, (min(TOK, p.M - tok_base) - 32 * eset + STEP - 1) / STEP);
+        for (int j = 0; ok && next_item(item); ++j, rc.next()) {
+            const int ct = 2 * item.tile + (int)rank;
+            const int tok_base = item.tok0;
+            const int n0 = (swiglu ? ct * 64 : ct * TILE_N) + col;
+            float sw[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int n = n0 + ((c + turn) & (CH - 1));
+                sw[c] = n < out_cols ? p.sw[(swiglu && c >= 2 ? p.F : 0) + n] : 0.f;
+                if (swiglu && c >= 2) sw[c] = -sw[c];  // (the SiLU comes negated)
+            }
+            // pieces of sixteen tokens of this warp that hold live tokens: those at 16 eset + STEP k, k < pieces
+            const int live = min(item.width, p.M - tok_base);
+            const int pieces = max(0, (live - 16 * eset + STEP - 1) / STEP);
             // Token scales, staged with the int4 records' 1/16 in them: (float)(16 s) * (sx / 16) is (float)s * sx, exactly,
-            // unless sx / 16 is subnormal.  (The barrier at the end of a tile keeps stragglers out.)
+            // unless sx / 16 is subnormal.  (The barrier at the end of an item keeps stragglers out.)
             float sx_here = 0.f;
+            const bool mine = sid < live && sid < TOK;
+            if (mine) sx_here = p.sx[tok_base + sid];
+            if (sid < TOK) s_sx[sid] = W8 ? sx_here : sx_here * 0.0625f;
+            const bool low = epilogue_any(mine && sx_here < PS_LOW);      // any scale that small: the careful ways below
             bool tiny = false;
-            if (sid < TOK) {
-                const int m = tok_base + sid;
-                if (m < p.M) {
-                    sx_here = p.sx[m];
-                    tiny = !W8 && sx_here < 7.8886e-31f;
+            if (!W8 && low) {
+                tiny = epilogue_any(mine && sx_here < 7.8886e-31f);
+                if (tiny) {
+                    if (sid < TOK) s_sx[sid] = sx_here;
+                    asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
                 }
-                s_sx[sid] = W8 ? sx_here : sx_here * 0.0625f;
             }
-            tiny = epilogue_any(tiny);
-            if (tiny) {
-                if (sid < TOK) s_sx[sid] = sx_here;
-                asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
-            }
+            // SwiGLU: no gate value of this thread is too small for the fast SiLU, whatever the sums are (zero is not)
+            const bool gates_ok = swiglu && !low && (n0 >= out_cols || (sw[0] >= PS_LOW && sw[1] >= PS_LOW));
             ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // one verdict for all eight warps
             if (!ok) { *s_error = 1; break; }
             if (sid == 0) PS_STAMP(j, 3);
             tc_fence_after();
-            const uint32_t acc_addr = lane_addr + rc.slot * TOK + 32 * eset;
-            const int row = q * 32 + lane;
-            auto hand_back = [&]() {   // this warp is done with the accumulator: another segment's MMAs may overwrite it
+            const uint32_t acc_addr = lane_addr + rc.slot * TOK + 16 * eset;
+            auto hand_back = [&]() {   // this warp is done with the accumulator: another item's MMAs may overwrite it
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) { if (rank != 0) mbar_arrive_remote_relaxed(&acc_empty[rc.slot], 0); else mbar_arrive_relaxed(&acc_empty[rc.slot]); }
                 if (sid == 0) PS_STAMP(j, 4);
             };
+            auto read_sums = [&](int k, uint32_t (&r)[16]) {
+                if (fragments) {
+                    tc_ld_16x256b_x2(acc_addr + STEP * k, r);
+                    tc_ld_16x256b_x2(acc_addr + (16u << 16) + STEP * k, r + 8);
+                } else tc_ld16(acc_addr + STEP * k, r);
+                tc_wait_ld();
+            };
             // ---- a part of a tile's K: the raw sums go to this CTA's slot, the tile's part counter is advanced, and the CTA
             // that completes it adds the other parts' slots to its own sums, which are still in tensor memory (integer
             // addition: exact in any order), and finishes the tile.  Nobody waits for anybody, and no slot needs clearing.
-            const size_t part_stride = 2 * (S::SLOT_INTS / 4);            // from one part's slot to the next one's
-            const int4* const slots = reinterpret_cast<const int4*>(p.partials) + (size_t)(2 * split * tile + (int)rank) * (S::SLOT_INTS / 4) + (size_t)(8 * eset) * 128 + row;   // [token / 4][row][4 tokens]
+            // A slot holds what a thread reads in one turn, four sums at a time: [piece][4][thread of the lane quarters].
+            const size_t tile_index = (size_t)unit0;
+            const size_t slot_quads = 32 * (size_t)p.unit, part_stride = 2 * slot_quads;
+            const int4* const slots = reinterpret_cast<const int4*>(p.partials) + (2 * split * tile_index + rank) * slot_quads + (size_t)(4 * eset) * 128 + q * 32 + lane;
             bool finish = true;
             if (split > 1) {
                 int4* const slot = const_cast<int4*>(slots) + part * part_stride;
 #pragma unroll 1
-                for (int c = 0; c < chunks; ++c) {
-                    uint32_t r[32];
-                    tc_ld32(acc_addr + STEP * c, r);
-                    tc_wait_ld();
+                for (int k = 0; k < pieces; ++k) {
+                    uint32_t r[16];
+                    read_sums(k, r);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        __stcg(slot + (size_t)(STEP / 4 * c + i) * 128, make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]));
+                    for (int i = 0; i < 4; ++i)
+                        __stcg(slot + (size_t)(STEP / 4 * k + i) * 128, make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]));
                 }
                 __threadfence();
                 asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
                 if (sid == 0) {
                     // (a tile with a part whose wait ran out is never completed; the launch reports the error and the host
                     // clears the counters)
-                    unsigned* const count = p.counts + 2 * tile + (int)rank;
-                    const bool done = atomicAdd(count, 1u) == (unsigned)split - 1u;
-                    if (done) *count = 0u;
-                    *s_finish = done ? 1 : 0;
+                    unsigned* const count = p.counts + 2 * tile_index + rank;
+                    const bool last = atomicAdd(count, 1u) == (unsigned)split - 1u;
+                    if (last) *count = 0u;
+                    *s_finish = last ? 1 : 0;
                     __threadfence();
                 }
                 asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
                 finish = *reinterpret_cast<volatile int*>(s_finish) != 0;
             }
-            const int turns = finish ? 2 * chunks : 0;
+            const int turns = finish ? pieces : 0;
             const int other = part == 0 ? 1 : 0;                          // the first of the other parts
             int4 ahead[4];                                                // its sums of the next turn, on their way
             auto fetch_part = [&](int4 (&v)[4], int which, int k) {
-                const int4* const src = slots + which * part_stride + (size_t)(STEP / 4 * (k >> 1) + 4 * (k & 1)) * 128;
+                const int4* const src = slots + which * part_stride + (size_t)(STEP / 4 * k) * 128;
 #pragma unroll
                 for (int h = 0; h < 4; ++h) v[h] = __ldcg(src + (size_t)h * 128);
             };
             if (split > 1 && turns) fetch_part(ahead, other, 0);
-            if (split == 1 && chunks == 0) hand_back();
+            if (split == 1 && pieces == 0) hand_back();
 #pragma unroll 1
             for (int k = 0; k < turns; ++k) {
-                const int t0 = 32 * eset + STEP * (k >> 1) + 16 * (k & 1), m0 = tok_base + t0;
+                const int t0 = 16 * eset + STEP * k + 2 * tq;             // this thread's first token of the turn
+                const int left = live - t0;                              // its tokens t0 + {0, 1, 8, 9} below t0 + left exist
                 uint32_t r[16];
-                tc_ld16(lane_addr + rc.slot * TOK + t0, r);
-                tc_wait_ld();
+                read_sums(k, r);
                 if (split == 1) {
                     if (k + 1 == turns) hand_back();
                 } else {
@@ -534,141 +610,153 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                         }
                     if (k + 1 < turns) fetch_part(ahead, other, k + 1);
                 }
-                if (m0 >= p.M) continue;
-                if (!SWIGLU && p.epi == EPI_I32) {
-                    int* const row0 = reinterpret_cast<int*>(p.out) + (size_t)m0 * out_cols + n;
-                    if (n_ok) {
+                if (!SWIGLU && !fragments) {
+                    const int first = 16 * eset + STEP * k, rows = live - first;
+                    const int n = ct * TILE_N + q * 32 + lane;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (m0 + i < p.M) row0[(size_t)i * out_cols] = (int)r[i] >> SHIFT;
+                    for (int i = 0; i < 16; ++i) r[i] = __shfl_sync(0xffffffffu, r[i], holder);
+                    if (n < out_cols) {
+                        const size_t at = (size_t)(tok_base + first) * out_cols + n;
+                        auto store_rows = [&](auto* dst, auto value) {
+                            if (rows >= 16) {
+#pragma unroll
+                                for (int i = 0; i < 16; ++i, dst += out_cols) *dst = value(i);
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < 16; ++i, dst += out_cols)
+                                    if (i < rows) *dst = value(i);
+                            }
+                        };
+                        if (p.epi == EPI_I32) store_rows(reinterpret_cast<int*>(p.out) + at, [&](int i) { return (int)r[i] >> SHIFT; });
+                        else {
+                            const F2 sw_own = f2_all(p.sw[n]);
+#pragma unroll
+                            for (int i = 0; i < 16; i += 2) {
+                                F2 v = f2_pack(__int2float_rn((int)r[i]), __int2float_rn((int)r[i + 1]));
+                                if (tiny) v = f2_mul(v, f2_all(0.0625f));
+                                float lo, hi;
+                                f2_unpack(f2_mul(f2_mul(v, *reinterpret_cast<const F2*>(s_sx + first + i)), sw_own), lo, hi);
+                                r[i] = __float_as_uint(lo);
+                                r[i + 1] = __float_as_uint(hi);
+                            }
+                            if (p.epi == EPI_F16) store_rows(reinterpret_cast<__half*>(p.out) + at, [&](int i) { return __float2half_rn(__uint_as_float(r[i])); });
+                            else store_rows(reinterpret_cast<float*>(p.out) + at, [&](int i) { return __uint_as_float(r[i]); });
+                        }
                     }
                     continue;
                 }
-                // y[i]: tokens m0 + 2i and m0 + 2i + 1.  (float)(16 s) / 16 is (float)s, exactly.
-                F2 y[8];
-                {
-                    const ulonglong2* const sx2 = reinterpret_cast<const ulonglong2*>(s_sx + t0);
-                    const F2 sw2 = f2_all(sw);
+                // r[8 (c / 2) + 4 h + 2 (c % 2) + e]: tensor-memory lane c, token t0 + 8 h + e
+                if (!SWIGLU && p.epi == EPI_I32) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const ulonglong2 sx = sx2[i];
-                        y[2 * i] = f2_pack(__int2float_rn((int)r[4 * i]), __int2float_rn((int)r[4 * i + 1]));
-                        y[2 * i + 1] = f2_pack(__int2float_rn((int)r[4 * i + 2]), __int2float_rn((int)r[4 * i + 3]));
-                        if (tiny) { y[2 * i] = f2_mul(y[2 * i], f2_all(0.0625f)); y[2 * i + 1] = f2_mul(y[2 * i + 1], f2_all(0.0625f)); }
-                        y[2 * i] = f2_mul(f2_mul(y[2 * i], sx.x), sw2);
-                        y[2 * i + 1] = f2_mul(f2_mul(y[2 * i + 1], sx.y), sw2);
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+                            if (8 * h + e < left && n0 < out_cols) {
+                                uint32_t v[4];
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) v[c] = (uint32_t)((int)r[8 * (c >> 1) + 4 * h + 2 * (c & 1) + e] >> SHIFT);
+                                store_four(reinterpret_cast<uint32_t*>(p.out) + (size_t)(tok_base + t0 + 8 * h + e) * out_cols + n0, v, turn);
+                            }
+                    continue;
+                }
+                F2 y[4][2];                                               // [lane c][h]: tokens t0 + 8 h, + 1
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const F2 sx = *reinterpret_cast<const F2*>(s_sx + t0 + 8 * h);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const uint32_t* const pair = r + 8 * (c >> 1) + 4 * h + 2 * (c & 1);
+                        y[c][h] = f2_pack(__int2float_rn((int)pair[0]), __int2float_rn((int)pair[1]));
+                        if (tiny) y[c][h] = f2_mul(y[c][h], f2_all(0.0625f));   // (float)(16 s) / 16 is (float)s, exactly
+                        y[c][h] = f2_mul(f2_mul(y[c][h], sx), f2_all(sw[c]));
                     }
                 }
-                if (!SWIGLU && p.epi == EPI_F16) {
-                    // a lane holds one channel of sixteen tokens; two exchange rounds turn that into four neighbouring
-                    // channels of four tokens: lanes 4g..4g+3 end up with tokens 4i + (lane & 3)
-                    uint32_t word[8];
+                if (!SWIGLU) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        float lo, hi;
-                        f2_unpack(y[i], lo, hi);
-                        const __half2 h = __floats2half2_rn(lo, hi);
-                        word[i] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                    const uint32_t selector = odd ? 0x3276u : 0x5410u;     // even lanes: low halves (own, peer's); odd lanes: high halves (peer's, own)
+                    for (int h = 0; h < 2; ++h) {
+                        float v[4][2];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) word[i] = __byte_perm(word[i], __shfl_xor_sync(0xffffffffu, word[i], 1), selector);
-                    const bool upper = (lane & 2) != 0;
+                        for (int c = 0; c < 4; ++c) f2_unpack(y[c][h], v[c][0], v[c][1]);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint32_t recv = __shfl_xor_sync(0xffffffffu, upper ? word[2 * i] : word[2 * i + 1], 2);
-                        if (upper) word[2 * i] = recv; else word[2 * i + 1] = recv;
-                        // now (word[2i], word[2i+1]) = channels n4 .. n4+3 of token m0 + 4i + (lane & 3)
-                    }
-                    const int n4 = n - (lane & 3);
-                    const int mrow = m0 + (lane & 3);
-                    __half* dst = reinterpret_cast<__half*>(p.out) + (size_t)mrow * out_cols + n4;
-                    const size_t step = 4 * (size_t)out_cols;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i, dst += step)
-                        if (mrow + 4 * i < p.M) {
-                            if (quad_ok && n4 + 3 < out_cols) *reinterpret_cast<uint2*>(dst) = make_uint2(word[2 * i], word[2 * i + 1]);
-                            else {
-                                const uint32_t ww[2] = {word[2 * i], word[2 * i + 1]};
-#pragma unroll
-                                for (int e = 0; e < 4; ++e)
-                                    if (n4 + e < out_cols) dst[e] = __ushort_as_half((unsigned short)((ww[e >> 1] >> (16 * (e & 1))) & 0xffffu));
+                        for (int e = 0; e < 2; ++e) {
+                            const size_t at = (size_t)(tok_base + t0 + 8 * h + e) * out_cols + n0;
+                            if (8 * h + e >= left || n0 >= out_cols) continue;
+                            if (p.epi == EPI_F16) {
+                                const __half2 lo = __floats2half2_rn(v[0][e], v[1][e]), hi = __floats2half2_rn(v[2][e], v[3][e]);
+                                store_four_halves(reinterpret_cast<__half*>(p.out) + at, *reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi), turn);
+                            } else {
+                                const uint32_t four[4] = {__float_as_uint(v[0][e]), __float_as_uint(v[1][e]), __float_as_uint(v[2][e]), __float_as_uint(v[3][e])};
+                                store_four(reinterpret_cast<uint32_t*>(p.out) + at, four, turn);
                             }
-                        }
-                } else if (!SWIGLU) {
-                    float* dst = reinterpret_cast<float*>(p.out) + (size_t)m0 * out_cols + n;
-                    if (n_ok) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i, dst += 2 * (size_t)out_cols) {
-                            float lo, hi;
-                            f2_unpack(y[i], lo, hi);
-                            if (m0 + 2 * i < p.M) dst[0] = lo;
-                            if (m0 + 2 * i + 1 < p.M) dst[out_cols] = hi;
                         }
                     }
                 } else {
-                    // Lanes 0-15 hold the gate rows g, lanes 16-31 the matching up rows u of 16 features.  The gate lanes
-                    // finish the even token of every pair and the up lanes the odd one: each sends the half of the pair
-                    // that the other finishes and evaluates eight SiLUs.
-                    float v[8];
-                    const int mine_row = m0 + (up_lane ? 1 : 0);
-                    const int left = n_ok ? p.M - mine_row : 0;         // rows from here on that are stored
-                    float* dst = reinterpret_cast<float*>(p.out) + (size_t)mine_row * out_cols + n;
+                    // lanes 0, 1: gate values of two features, lanes 2, 3: their up values, negated
+                    const bool n_ok = n0 < out_cols;                      // (features come in whole groups of 32)
+                    F2 v[2][2];
+                    float most = 0.f;
 #pragma unroll
-                    for (int h = 0; h < 8; h += 4) {           // (four at a time: one look at the magnitudes, few values waiting)
-                        float g[4];
+                    for (int h = 0; h < 2; ++h)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            float even_token, odd_token;
-                            f2_unpack(y[h + i], even_token, odd_token);
-                            const float recv = __shfl_xor_sync(0xffffffffu, up_lane ? even_token : odd_token, 16);
-                            g[i] = up_lane ? recv : even_token;
-                            v[h + i] = up_lane ? odd_token : recv;
+                        for (int c = 0; c < 2; ++c) {
+                            float a, b;
+                            f2_unpack(y[c][h], a, b);
+                            most = max_abs(most, max_abs(a, b));
                         }
-                        if (left < 16) {                        // what does not exist has zeros: keep it off the slow path below
+                    if (gates_ok && silu_plain(1.f, most)) {
 #pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                if (2 * (h + i) >= left) g[i] = 1.f;
-                        }
-                        if (silu_plain(min_abs(min_abs(g[0], g[1]), min_abs(g[2], g[3])), max_abs(max_abs(g[0], g[1]), max_abs(g[2], g[3])))) {
+                        for (int h = 0; h < 2; ++h)
 #pragma unroll
-                            for (int i = 0; i < 4; i += 2) {
-                                float a, b;
-                                minus_silu_poly2(g[i], g[i + 1], a, b);
-                                v[h + i] = __fmul_rn(-a, v[h + i]);
-                                v[h + i + 1] = __fmul_rn(-b, v[h + i + 1]);
+                            for (int c = 0; c < 2; ++c) {
+                                float a, b, ya, yb;
+                                f2_unpack(y[c][h], a, b);
+                                minus_silu_poly2(a, b, ya, yb);
+                                v[c][h] = f2_mul(f2_pack(ya, yb), y[c + 2][h]);
                             }
-                        } else {
+                    } else {
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) v[h + i] = __fmul_rn(silu_poly(g[i]), v[h + i]);
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int c = 0; c < 2; ++c) {
+                                float a, b, ua, ub;
+                                f2_unpack(y[c][h], a, b);
+                                f2_unpack(y[c + 2][h], ua, ub);
+                                v[c][h] = f2_pack(__fmul_rn(silu_poly(a), -ua), __fmul_rn(silu_poly(b), -ub));
+                            }
+                    }
+                    float top[4];                                         // [2 h + e]: the larger of the two features
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float a[2], b[2];
+                        f2_unpack(v[0][h], a[0], a[1]);
+                        f2_unpack(v[1][h], b[0], b[1]);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            top[2 * h + e] = max_abs(a[e], b[e]);
+                            if (n_ok && 8 * h + e < left) {
+                                float* const dst = reinterpret_cast<float*>(p.out) + (size_t)(tok_base + t0 + 8 * h + e) * out_cols + n0;
+                                const float first = turn ? b[e] : a[e], second = turn ? a[e] : b[e];
+                                if (wide_ok) *reinterpret_cast<float2*>(dst) = make_float2(first, second);
+                                else { dst[0] = first; dst[1] = second; }
+                            }
                         }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i, dst += 2 * (size_t)out_cols)
-                            if (2 * (h + i) < left) *dst = v[h + i];
                     }
                     if (p.rowmax) {
-                        // Maxima over the 16 lanes of each half, one token per value: three folding steps that halve the
-                        // values a lane holds and a plain one; lanes 2i of a half end up with the maximum of their token.
-                        // (Tokens and channels that do not exist have zero scales, and zeros here.)
+                        // Maxima over the sixteen features, one token per value: two folding steps that halve the values a
+                        // lane holds and a plain one.  (Tokens and features that do not exist have zero scales, and zeros here.)
+                        const bool far = (lane & 16) != 0, near = (lane & 8) != 0;
 #pragma unroll
-                        for (int width = 8; width > 1; width >>= 1) {
-                            const bool upper = (lane & width) != 0;
-#pragma unroll
-                            for (int i = 0; i < width / 2; ++i) {
-                                const float keep = upper ? v[i + width / 2] : v[i];
-                                const float give = upper ? v[i] : v[i + width / 2];
-                                v[i] = max_abs(keep, __shfl_xor_sync(0xffffffffu, give, width));
-                            }
-                        }
-                        const uint32_t most = __float_as_uint(max_abs(v[0], __shfl_xor_sync(0xffffffffu, v[0], 1)));
-                        // collected per CTA and tile in shared memory first: one global atomic per token and tile
-                        // instead of one per token, tile and 16 features
-                        if (!odd && most) atomicMax(&s_tilemax[t0 + (up_lane ? 1 : 0) + 2 * ((lane >> 1) & 7)], most);
+                        for (int e = 0; e < 2; ++e) top[e] = max_abs(far ? top[2 + e] : top[e], __shfl_xor_sync(0xffffffffu, far ? top[e] : top[2 + e], 16));
+                        top[0] = max_abs(near ? top[1] : top[0], __shfl_xor_sync(0xffffffffu, near ? top[0] : top[1], 8));
+                        const uint32_t bits = __float_as_uint(max_abs(top[0], __shfl_xor_sync(0xffffffffu, top[0], 4)));
+                        // collected per CTA and item in shared memory first: one global atomic per token and item
+                        // instead of one per token, item and sixteen features
+                        if (!(lane & 4) && bits) atomicMax(&s_tilemax[t0 + (far ? 8 : 0) + (near ? 1 : 0)], bits);
                     }
                 }
             }
             if (sid == 0) PS_STAMP(j, 5);
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");   // every epilogue warp is done with this tile's scales and maxima
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");   // every epilogue warp is done with this item's scales and maxima
             if (swiglu && p.rowmax && sid < TOK) {
                 const uint32_t m = s_tilemax[sid];
                 if (m) {
@@ -676,9 +764,6 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                     s_tilemax[sid] = 0u;
                 }
             }
-            gi += n_seg;
-            it += n_seg;
-            if (it == nst) { it = 0; ++tile; }
         }
     }
 
@@ -700,6 +785,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
 
 namespace {
 constexpr long long PS_MAX_K = 131072;
+
+// The widest item of a kernel that takes the plan's.
+constexpr int PS_NARROW = 64, PS_WIDE = 160, PS_WIDEST = 256;   // (int8 weights: narrow and widest)
 
 template <bool W8, bool SWIGLU, int TOK>
 cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool pdl)
@@ -734,8 +822,7 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
         max_clusters = n;
         if (device >= 0 && device < 64) { clusters_of_device[device] = n; configured.mark(device); }
     }
-    const int tiles = gemm_tc_persist_tiles(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, TOK);
-    const int clusters = persist_clusters(tiles, p.split, max_clusters);
+    const int clusters = persist_clusters(gemm_tc_persist_units(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, p.unit), p.split, max_clusters);
     cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
     int n = 1;
     if (pdl) {
@@ -745,76 +832,128 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kernel, p, clusters);
-}
-template <int TOK>
-cudaError_t launch_persist_tok(const GemmParams& p, cudaStream_t stream, bool pdl)
-{
-    if (p.w8) return p.epi == EPI_SWIGLU ? cudaErrorInvalidValue : launch_persist_inst<true, false, TOK>(p, stream, pdl);
-    return p.epi == EPI_SWIGLU ? launch_persist_inst<false, true, TOK>(p, stream, pdl) : launch_persist_inst<false, false, TOK>(p, stream, pdl);
+    return cudaLaunchKernelEx(&cfg, kernel, p, *p.maps, clusters);
 }
 } // namespace
 
-int gemm_tc_persist_tiles(int columns, int M, int tok) { return (columns + 255) / 256 * ((M + tok - 1) / tok); }
+int gemm_tc_persist_units(int columns, int M, int unit) { return (columns + 255) / 256 * ((M + unit - 1) / unit); }
 
-// The token tile and the number of parts a tile's K is cut into: the cheapest by a model of the kernel's time in cycles,
-// fitted to 80 shapes (M 33..4096, K 2048..14336, N 1024..28672, both epilogues).  On 27 others, K 1024..11008, it is within
-// 2 % of the best choice but just above 64 tokens (a second tile of 64 would be nearly empty: 20 % at worst, 65 x 8192 -> 2048
-// 19.0 us where 64-token tiles take 15.8) and for 400 to 448 tokens of K = 1024 (23.9 against 22.0):
-//   * a k-block takes 270 to 390 cycles at 64 tokens and 310 to 370 at 128, more with more SMs busy (the operands come
-//     out of L2 at about 45 bytes per SM and cycle when all SMs ask), and 530 at 256, where the MMAs bound it; int8
-//     weights are delivery-bound (52 bytes per cycle).  At 192 tokens two accumulators leave two buffers of unpacked
-//     weights: 560, and 780 with int8 weights;
-//   * finishing a tile takes 33 cycles per token, 1500 at least; 80 and 4800 with SwiGLU, which bounds the kernel at
-//     K = 4096 (192 tokens instead of 128 amortise it better: 4096 x 4096 -> 14336 450 -> 422 us); two accumulators hide
-//     it behind the next tile's MMAs up to 192 tokens, beyond there is room for one and nothing is hidden;
-//   * 224 tokens are for what 256 would cut worse (777 tokens, 14336 -> 4096 50 -> 46 us);
-//   * K in parts costs an exchange through L2: so much per part and pair, more for wide token tiles;
+// How a problem is cut: the cheapest by a model of the kernel's time in cycles, fitted to every cut of 350 shapes (1 to 3000
+// tokens, K 1024 .. 11008, 2048 .. 28672 channels; linear, SwiGLU and int8-weight launches).  What it takes is within 0.6, 0.6
+// and 2.5 % of the best cut in the mean and within 9, 6 and 15 % at worst (64 x 8192 -> 2048 15.5 us where three parts of
+// 32-token tiles take 14.3):
+//   * a k-block of an item costs a constant (the issuer's and the unpack warps' chains) and something per token: 305 + 0.6 per
+//     token with four-byte-packed weights, of which the MMAs need two per token, so wide items pay; less where SMs are idle;
+//   * finishing an item is hidden behind the next one's MMAs (two accumulators) unless it takes longer;
+//   * K in parts costs an exchange through L2: so much per part and pair, more for wide items;
 //   * a launch on more than half of the SMs leaves the one behind it no room to set itself up meanwhile.
+struct PersistCosts {
+    double narrow, narrow_token, wide, wide_token, widest, widest_token;   // cycles of a k-block in each kernel
+    double finish, finish_token, item;               // of finishing an item, and between two items
+    double part0, part, pair, part_wide;             // the exchange of parts
+    double crowded, idle;
+};
 PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
 {
-    PersistPlan best{256, 1};
+    static const PersistCosts linear{270, 1.15, 305, 0.6, 339, 0.845, 2200, 31, 195, 870, 1590, 23, 0.65, 1530, 0.17};
+    static const PersistCosts gated{366, 0.79, 420, 0.37, 326, 1.0, 5060, 60, 670, 1500, 1380, 30, 0.7, 2030, 0.15};
+    static const PersistCosts bytes{323, 0.63, 380, 1.2, 380, 1.2, 2430, 32, 725, 1490, 1000, 21, 1.12, 720, 0.18};
+    const PersistCosts& cost = w8 ? bytes : swiglu ? gated : linear;
+    PersistPlan best{PERSIST_TOKENS, 1, 0, 1};
     double best_time = 0;
-    const int pairs = std::max(1, sm_count / 2);
-    for (const int tok : {64, 128, 192, 224, 256}) {
-        if (tok > 64 && M <= 64) break;                        // half of the tile would be padding
-        const long long tiles = (long long)((columns + 255) / 256) * ((M + tok - 1) / tok);
+    const int pairs = std::max(1, sm_count / 2), channel_tiles = (columns + 255) / 256, widest = PS_WIDEST;
+    const int tokens = (M + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS;
+    auto consider = [&](int unit, int most, int snap, int split) {
+        const int per_tile = (M + unit - 1) / unit;
+        const unsigned units = unsigned(channel_tiles) * unsigned(per_tile);
+        const int clusters = persist_clusters(int(units), split, pairs);
+        const double share = 1 - cost.idle * (1 - std::min(1.0, double(clusters) / pairs));
+        const bool narrow = unit * most <= PS_NARROW, wide = unit * most <= PS_WIDE, hidden = w8 || wide;
+        auto block = [&](int width) {
+            return share * (narrow ? cost.narrow + cost.narrow_token * width : wide ? cost.wide + cost.wide_token * width : cost.widest + cost.widest_token * width);
+        };
+        auto finish = [&](int width) { return cost.finish + cost.finish_token * (columns % 4 ? 2.5 : 1) * width; };   // (narrower stores)
+        double longest = 0;
+        if (split > 1) {
+            const int width = std::min(unit, tokens);
+            longest = KB * block(width) / split + finish(width) +
+                      (cost.part0 + cost.part * (split - 1) + cost.pair * clusters) * (1 + cost.part_wide * std::max(0, width - 64) / 64.0);
+        } else
+            for (int i = 0; i < clusters; ++i) {
+                PersistItems items(persist_bound(units, per_tile, snap, i, clusters), persist_bound(units, per_tile, snap, i + 1, clusters), per_tile, most);
+                int tile, first, n;
+                double time = 0, last = 0;
+                while (items.next(tile, first, n)) {
+                    const int width = std::min(n * unit, tokens - first * unit);
+                    time += std::max(KB * block(width) + cost.item, hidden ? last : 0) + (hidden ? 0 : last);
+                    last = finish(width);
+                }
+                longest = std::max(longest, time + last);
+            }
+        if (2 * clusters > pairs) longest += cost.crowded;
+        if (best_time == 0 || longest < best_time) { best_time = longest; best = {unit, most, snap, split}; }
+    };
+    for (int unit = PERSIST_TOKENS; unit <= std::min(widest, tokens); unit += PERSIST_TOKENS)       // items of one width, K in parts or not
         for (const int split : {1, 2, 3, 4, 6, 8}) {
-            if (split > 1 && (tok > 128 || tiles * split > pairs || KB < 4 * split)) break;
-            const long long clusters = std::min<long long>(tiles * split, pairs), rounds = (tiles + pairs - 1) / pairs;
-            const double busy = double(clusters) / pairs;
-            double block = tok == 64 ? 270 + 120 * busy : tok == 128 ? 310 + 60 * busy : tok == 192 ? 480 + 80 * busy : tok == 224 ? 470 : 530;
-            if (swiglu) block += 20;
-            if (w8) block = tok == 192 ? 780 : std::max(block, (16384 + 64 * tok) / 52.0);
-            const double mma = KB * block / split, live = std::min(tok, M), finish = swiglu ? 4800 + 80 * live : 1500 + 33 * live;
-            double time = tok > 192 ? rounds * (mma + finish) : mma + (rounds - 1) * std::max(mma, finish) + finish;
-            if (split > 1) time += (1500 + 1000 * (split - 1) + 30 * clusters) * (1 + 1.5 * std::max(0.0, live - 64) / 64);
-            if (2 * clusters > pairs) time += 3000;
-            if (best_time == 0 || time < best_time) { best_time = time; best = {tok, split}; }
+            if (split > 1 && (unit > PS_WIDE || (long long)channel_tiles * ((M + unit - 1) / unit) * split > pairs || KB < 4 * split)) break;
+            consider(unit, 1, 0, split);
         }
-    }
+    for (int most = 2; most <= std::min(widest, tokens) / PERSIST_TOKENS; ++most)                  // equal runs
+        for (const int snap : {0, 2, 3}) consider(PERSIST_TOKENS, most, snap, 1);
     return best;
 }
 size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan)
 {
-    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_tiles(columns, M, plan.tok)) * size_t(plan.split) * 128 * size_t(plan.tok) * sizeof(int) : 0;
+    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_units(columns, M, plan.unit)) * size_t(plan.split) * 128 * size_t(plan.unit) * sizeof(int) : 0;
 }
 size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan)
 {
-    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_tiles(columns, M, plan.tok)) * sizeof(unsigned) : 0;
+    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_units(columns, M, plan.unit)) * sizeof(unsigned) : 0;
+}
+
+// Eight-byte elements: 256 of them, the most a box may have, are the two k-blocks of a stage.
+bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB)
+{
+    static const auto encode = []() {
+        void* entry = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &entry, 12000, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            entry = nullptr;
+        }
+        return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(entry);
+    }();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {cuuint64_t(KB) * 128, cuuint64_t((M + PERSIST_TOKENS - 1) / PERSIST_TOKENS * (PERSIST_TOKENS / PERSIST_T))};
+    const cuuint64_t strides[1] = {cuuint64_t(KB) * 1024};
+    const cuuint32_t steps[2] = {1, 1};
+    for (int i = 0; i < 3; ++i) {
+        const cuuint32_t box[2] = {PS_SK * 128, 8u >> i};
+        if (encode(&maps.box[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t*>(codes), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
+    return true;
 }
 
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl)
 {
-    if ((long long)p.KB * KBLOCK > PS_MAX_K || p.split < 1 || (p.split > 1 && !(p.partials && p.counts))) return cudaErrorInvalidValue;
-    switch (2 * p.T) {
-    case 64: return launch_persist_tok<64>(p, stream, pdl);
-    case 128: return launch_persist_tok<128>(p, stream, pdl);
-    case 192: return launch_persist_tok<192>(p, stream, pdl);
-    case 224: return launch_persist_tok<224>(p, stream, pdl);
-    case 256: return launch_persist_tok<256>(p, stream, pdl);
-    default: return cudaErrorInvalidValue;
+    if (!p.maps) return cudaErrorInvalidValue;
+    const int width = p.unit * p.most;   // picks the kernel
+    if ((long long)p.KB * KBLOCK > PS_MAX_K || p.T != PERSIST_T || p.unit < 32 || p.unit % 32 || p.most < 1 || width > PS_WIDEST || p.split < 1 ||
+        (p.split > 1 && !(p.most == 1 && p.partials && p.counts)))
+        return cudaErrorInvalidValue;
+    if (p.w8) {
+        if (p.epi == EPI_SWIGLU) return cudaErrorInvalidValue;
+        return width <= PS_NARROW ? launch_persist_inst<true, false, PS_NARROW>(p, stream, pdl) : launch_persist_inst<true, false, PS_WIDEST>(p, stream, pdl);
     }
+    if (p.epi == EPI_SWIGLU)
+        return width <= PS_NARROW ? launch_persist_inst<false, true, PS_NARROW>(p, stream, pdl)
+             : width <= PS_WIDE   ? launch_persist_inst<false, true, PS_WIDE>(p, stream, pdl)
+                                  : launch_persist_inst<false, true, PS_WIDEST>(p, stream, pdl);
+    return width <= PS_NARROW ? launch_persist_inst<false, false, PS_NARROW>(p, stream, pdl)
+         : width <= PS_WIDE   ? launch_persist_inst<false, false, PS_WIDE>(p, stream, pdl)
+                              : launch_persist_inst<false, false, PS_WIDEST>(p, stream, pdl);
 }
 
 } // namespace rkb200

@@ -137,6 +137,7 @@ struct rk_npu_w4a8_workspace {
     float* inverse = nullptr;
     uint32_t* rowmax = nullptr;
     rkb200::PersistPlan plan[2]{};    // variant 2: how a linear and a SwiGLU launch are cut
+    rkb200::PersistMaps maps{};       // and where its activation codes are
     int* partials = nullptr;          // variants 2, 4: partial sums of tiles and progress counters
     unsigned int* counts = nullptr;
     size_t partials_bytes = 0, counts_bytes = 0;

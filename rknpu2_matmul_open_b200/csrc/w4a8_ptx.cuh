@@ -86,6 +86,14 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_global,
                  : "memory");
 }
 
+// ---- tensor copy global -> shared of a box of a two-dimensional map (x in elements, a multiple of 16 bytes)
+__device__ __forceinline__ void tensor_g2s(void* dst_smem, const void* map, int x, int y, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                     smem_u32(dst_smem)),
+                 "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 // ---- distributed shared memory: a 32-bit store into a peer CTA's shared memory that also counts
 // four bytes on a barrier in that CTA.  Data and signal travel together, so the receiver needs no
 // cluster-wide barrier: it waits on its own mbarrier for the bytes it expects.

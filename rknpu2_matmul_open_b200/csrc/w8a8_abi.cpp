@@ -46,7 +46,9 @@ struct rk_npu_matmul_workspace {
     uint32_t domain_id = 0;
     std::atomic_flag busy = ATOMIC_FLAG_INIT;
     cudaStream_t stream = nullptr;
-    int T = 0, KB = 0, parts = 1;
+    int KB = 0;
+    PersistPlan plan{};
+    PersistMaps maps{};
     uint8_t* codes = nullptr;
     int* partials = nullptr;          // partial sums of tiles whose K is cut between CTA pairs
     unsigned* counts = nullptr;       // and how far each such tile is
@@ -95,7 +97,8 @@ bool valid_strategy(const rk_npu_matmul_strategy* s)
 // what the kernels need on top: K within the contraction kernel's range, sizes that fit
 bool runnable_shape(int M, int N, int K) { return K <= 131072 && (int64_t)M * K <= INT32_MAX && (int64_t)M * N <= INT32_MAX; }
 struct Sizes {
-    int T, KB, NG, parts;
+    int KB, NG;
+    PersistPlan plan;
     size_t codes, partials, counts, scales, stage_in, stage_out, packed, wscales;
 };
 Sizes sizes_of(int M, int N, int K, int kind)
@@ -103,10 +106,9 @@ Sizes sizes_of(int M, int N, int K, int kind)
     Sizes z{};
     z.KB = (K + KBLOCK - 1) / KBLOCK;
     const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, false, PLAN_SMS);
-    z.T = plan.tok / 2;
-    z.parts = plan.split;
+    z.plan = plan;
     z.NG = align_up((N + GROUP - 1) / GROUP, 8) + 8;   // zero groups behind the last tile, as for the int4 weights
-    z.codes = size_t(align_up(M, plan.tok)) * size_t(z.KB) * KBLOCK;
+    z.codes = size_t(align_up(M, PERSIST_TOKENS)) * size_t(z.KB) * KBLOCK;
     z.partials = gemm_tc_persist_slot_bytes(N, M, plan);
     z.counts = gemm_tc_persist_count_bytes(N, M, plan);
     z.scales = sizeof(float) * 2 * size_t(M);
@@ -259,7 +261,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     q.static_scale = static_dev;
     q.Xq = ws->codes;
     q.scales = ws->scales;
-    q.M = st.M; q.K = st.K; q.Kp = ws->KB * KBLOCK; q.T = ws->T;
+    q.M = st.M; q.K = st.K; q.Kp = ws->KB * KBLOCK; q.T = PERSIST_T;
     q.kind = kind == RK_NPU_MATMUL_I8I8I32 ? 2 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? 1 : 0);
     GemmParams g{};
     g.Wp = w->packed;
@@ -271,9 +273,10 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     g.report = &ws->host_status_alias->device_error;
     *ws->host_status = Status{};
     g.M = st.M; g.N = st.N; g.K = st.K;
-    g.KB = ws->KB; g.NG = w->NG; g.T = ws->T;
+    g.KB = ws->KB; g.NG = w->NG; g.T = PERSIST_T;
     g.epi = kind == RK_NPU_MATMUL_I8I8I32 ? EPI_I32 : (kind <= RK_NPU_MATMUL_F16I8F16_STATIC ? EPI_F16 : EPI_F32);
-    g.split = ws->parts;
+    set_plan(g, ws->plan);
+    g.maps = &ws->maps;
     g.w8 = 1;
     g.partials = ws->partials;
     g.counts = ws->counts;
@@ -351,8 +354,7 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
     ws->domain = domain;
     ws->ctx_id = ctx->id;
     ws->domain_id = domain->id;
-    ws->T = z.T;
-    ws->parts = z.parts;
+    ws->plan = z.plan;
     ws->KB = z.KB;
     ws->codes_bytes = z.codes;
     ws->partials_bytes = z.partials;
@@ -370,6 +372,7 @@ extern "C" rk_npu_matmul_workspace* rk_npu_matmul_workspace_create(rk_npu_iommu_
          !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), ws->scale_bytes) &&
          !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status)) &&
          !device_alloc(domain, &ws->stage_in, ws->stage_in_bytes) && !device_alloc(domain, &ws->stage_out, ws->stage_out_bytes);
+    ok = ok && make_persist_maps(ws->maps, ws->codes, strategy->M, ws->KB);
     // codes of the tokens that pad the last tile stay zero for the life of the workspace
     ok = ok && cudaMemsetAsync(ws->codes, 0, ws->codes_bytes, ws->stream) == cudaSuccess &&
          (!ws->counts || cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, ws->stream) == cudaSuccess) &&

@@ -9,10 +9,11 @@
 //   int8 A as given : include/rk_npu_quant_matmul.h:335-340 (no quantisation at all)
 // The contraction itself runs on the tcgen05 kernel of w4a8_gemm_tc_persist.cu with int8 weights (GemmParams::w8).
 //
-// Weight layout  W8p[g][kb][c][r][16 B]: g = group of 32 output channels, kb = 128-element k-block, c = 16-element
-// chunk of the k-block (8 of them), r = channel of the group; the 16 bytes are the int8 codes k = 128kb + 16c .. +15.
-// A lane of an unpack warp (lane = channel) reads its eight 16-byte pieces of a k-block 512 bytes apart, so a warp's
-// loads are conflict free, and the pieces are the words of that channel's tensor-memory row in order.
+// Weight layout  W8p[tile][kb][c][row][16 B]: tile of 128 output channels, kb = 128-element k-block, c = 16-element
+// chunk of the k-block (8 of them); the 16 bytes are the int8 codes k = 128kb + 16c .. +15 of one channel.  Eight rows are
+// a core matrix, so a k-block of a tile (16 KB, contiguous) is the MMA's K-major operand without swizzle as it lies: one
+// copy, no unpacking.  (When eight warps copied it on into tensor memory, 777 tokens 4096 -> 11008 took 43 us.)  Row
+// 32 g + 8 c + i holds channel 32 g + 4 i + c: a thread of the epilogue reads tensor-memory lanes i, i + 8, i + 16, i + 24.
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
 #include "w4a8_ptx.cuh"
@@ -41,7 +42,8 @@ __global__ void __launch_bounds__(256) w8_pack_weights_kernel(const W8PackParams
             if (k < p.K) word |= (uint32_t)(uint8_t)p.B[(size_t)k * p.N + n] << (8 * b);
         }
     }
-    reinterpret_cast<uint32_t*>(p.Wp)[(((size_t)g * p.KB * 8 + c) * GROUP + r) * 4 + j] = word;
+        const int row = 8 * (r & 3) + (r >> 2);
+    reinterpret_cast<uint32_t*>(p.Wp)[((((size_t)(g >> 2) * p.KB * 8 + c) * 4 + (g & 3)) * GROUP + row) * 4 + j] = word;
 }
 
 cudaError_t launch_w8_pack_weights(const W8PackParams& p, cudaStream_t stream)

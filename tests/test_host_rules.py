@@ -106,3 +106,38 @@ int main()
     return 0;
 }
 """)
+
+
+def test_runs_of_items_cover_every_token_of_every_channel_tile_once(tmp_path):
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+#include <vector>
+using namespace rkb200;
+int main()
+{
+    for (int tiles : {1, 2, 5, 16, 43, 56, 112, 300})
+        for (int per_tile : {1, 2, 3, 4, 5, 7, 24, 25, 64, 94, 128})
+            for (int most = 1; most <= 8; ++most)
+                for (int snap : {0, 2, 3})
+                    for (int pairs : {1, 2, 37, 73, 74}) {
+                        const int units = tiles * per_tile;
+                        const int n = persist_clusters(units, 1, pairs);
+                        std::vector<char> seen(units, 0);
+                        bool ok = true;
+                        for (int i = 0; i < n; ++i) {
+                            const unsigned from = persist_bound(units, per_tile, snap, i, n), to = persist_bound(units, per_tile, snap, i + 1, n);
+                            ok = ok && from <= to && (i || from == 0) && (i + 1 < n || to == (unsigned)units);
+                            PersistItems items(from, to, per_tile, most);
+                            int tile, first, len;
+                            while (items.next(tile, first, len)) {
+                                ok = ok && tile >= 0 && tile < tiles && first >= 0 && len >= 1 && len <= most && first + len <= per_tile;
+                                for (int k = 0; ok && k < len; ++k) ok = !seen[tile * per_tile + first + k]++;
+                            }
+                        }
+                        for (char c : seen) ok = ok && c == 1;
+                        if (!ok) { printf("%d tiles of %d, most %d, snap %d, %d pairs\n", tiles, per_tile, most, snap, pairs); return 1; }
+                    }
+    return 0;
+}
+""")
