@@ -130,9 +130,9 @@ __global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) quantize_row
     op.finish(threadIdx.x < TG && (int)(blockIdx.x * TG + threadIdx.x) < p.M);
 }
 
-// Any row: one CTA per token, a thread per 16-element unit, element by element where 16-byte loads are not possible.
+// Any row: one CTA per token.
 template <bool HALF>
-__global__ void __launch_bounds__(256, 8) quantize_kernel(const QuantParams p)
+__global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
 {
     constexpr int BS = 256;
     using T = typename ActType<HALF>::type;
@@ -140,8 +140,9 @@ __global__ void __launch_bounds__(256, 8) quantize_kernel(const QuantParams p)
     pdl_wait();                // A may be the output of the kernel in front of this one
     const int m = blockIdx.x, tid = threadIdx.x;
     const T* row = reinterpret_cast<const T*>(p.A) + (size_t)m * p.K;
-    const bool vec = ((reinterpret_cast<uintptr_t>(row) & 15u) == 0);
-    const int chunks = p.Kp / 16, live_chunks = (p.K + 15) / 16;
+    const int lane = tid & 31, first = tid & ~31;   // units of this warp: 32 from `first` on, and every BS further
+    const int chunks = p.Kp / 16;
+    __shared__ uint32_t s_words[BS / 32][PIECE_WORDS];
     __shared__ uint32_t s_part[BS / 32];
     __shared__ float s_inverse;
     __shared__ int s_bad;
@@ -149,8 +150,12 @@ __global__ void __launch_bounds__(256, 8) quantize_kernel(const QuantParams p)
     uint32_t maxbits = 0;
     int bad = 0;
     if (p.rowmax == nullptr) {
-        float v[16];
-        for (int kc = tid; kc < live_chunks; kc += BS) load16<HALF>(row, kc * 16, p.K, vec, v, maxbits);
+        for (int u = first; u * 16 < p.K; u += BS) {
+            uint32_t raw[16];
+            load_piece<HALF>(row, u * 16, p.K, lane, raw);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) maxbits = max(maxbits, raw[i] & (HALF ? 0x7fffu : 0x7fffffffu));
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) maxbits = max(maxbits, __shfl_xor_sync(0xffffffffu, maxbits, o));
         if ((tid & 31) == 0) s_part[tid >> 5] = maxbits;
@@ -190,15 +195,13 @@ __global__ void __launch_bounds__(256, 8) quantize_kernel(const QuantParams p)
     const float inv = s_inverse;
     const int mt = m / p.T, t = m - mt * p.T;
     uint4* dst = reinterpret_cast<uint4*>(p.Xq) + ((size_t)mt * chunks) * p.T + t;
-    for (int kc = tid; kc < chunks; kc += BS) {
-        uint4 q = make_uint4(0u, 0u, 0u, 0u);
-        if (kc < live_chunks) {
-            float v[16];
-            uint32_t unused = 0;
-            load16<HALF>(row, kc * 16, p.K, vec, v, unused);
-            q = quantize16(v, inv, kc * 16, p.K);
-        }
-        dst[(size_t)kc * p.T] = q;
+    for (int u = first; u < chunks; u += BS) {
+        uint32_t raw[16];
+        float v[16];
+        load_piece<HALF>(row, u * 16, p.K, lane, raw);
+        exchange_piece<HALF>(s_words[tid >> 5], lane, raw, v);
+        const int kc = u + lane;
+        if (kc < chunks) dst[(size_t)kc * p.T] = kc * 16 < p.K ? quantize16(v, inv, kc * 16, p.K) : make_uint4(0u, 0u, 0u, 0u);
     }
     // Cross-CTA bookkeeping last, so that the other 255 threads of the CTA never wait for its
     // round trips to L2.

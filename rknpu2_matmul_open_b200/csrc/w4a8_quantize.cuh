@@ -96,6 +96,35 @@ __device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int M,
     }
 }
 
+// Rows that do not allow 16-byte loads: a warp takes 512 elements at a time, a lane element 32 i + lane, so that every load
+// covers neighbouring elements, and hands them to the lane whose 16-element unit they belong to through shared memory, a word
+// per element, units seventeen words apart (no bank conflicts in either direction).  (A thread loading its unit element by
+// element touched 32 lines with every load: 193 rows of 3070 fp32 9 us where 3072 values take 5.5.)
+constexpr int PIECE_WORDS = 32 * 17;
+template <bool HALF>
+__device__ __forceinline__ void load_piece(const typename ActType<HALF>::type* row, int k0, int K, int lane, uint32_t (&raw)[16])
+{
+    using Bits = std::conditional_t<HALF, unsigned short, unsigned int>;
+    const Bits* const at = reinterpret_cast<const Bits*>(row) + k0 + lane;
+    const int left = K - k0 - lane;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) raw[i] = 32 * i < left ? (uint32_t)__ldcg(at + 32 * i) : 0u;
+}
+// The sixteen values of unit `lane` of a piece (between two barriers of the warp).
+template <bool HALF>
+__device__ __forceinline__ void exchange_piece(uint32_t* words, int lane, const uint32_t (&raw)[16], float (&v)[16])
+{
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) words[(2 * i + (lane >> 4)) * 17 + (lane & 15)] = raw[i];
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const uint32_t w = words[lane * 17 + i];
+        v[i] = HALF ? __half2float(__ushort_as_half((uint16_t)w)) : __uint_as_float(w);
+    }
+}
+
 // 16-byte loads are possible for every row.
 template <bool HALF>
 inline bool quantize_rows_ok(const void* A, int K, int T) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % QuantRows<HALF, 1>::EPW == 0 && T % 2 == 0; }

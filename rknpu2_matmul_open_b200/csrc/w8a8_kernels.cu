@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) w8_quantize_
     quantize_rows<HALF, TG, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, op);
 }
 
-// The same for any row: one CTA per token, a thread per 16-element unit.
+// The same for any row: one CTA per token.
 template <bool HALF>
 __global__ void __launch_bounds__(256) w8_quantize_kernel(const W8QuantParams p)
 {
@@ -112,30 +112,22 @@ __global__ void __launch_bounds__(256) w8_quantize_kernel(const W8QuantParams p)
     pdl_launch_dependents();   // the GEMM behind this kernel may set itself up and request its weights
     const int m = blockIdx.x, tid = threadIdx.x;
     const T* row = reinterpret_cast<const T*>(p.A) + (size_t)m * p.K;
-    const bool vec = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
-    const int chunks = p.Kp / 16, live_chunks = (p.K + 15) / 16;
+    const int lane = tid & 31, first = tid & ~31;   // units of this warp: 32 from `first` on, and every 256 further
+    const int chunks = p.Kp / 16;
+    __shared__ uint32_t s_words[8][PIECE_WORDS];
     __shared__ uint32_t s_part[8];
     __shared__ float s_scale;
     if (p.static_scale == nullptr) {
         // magnitude bits order like magnitudes; a NaN pattern (above infinity) never raises the maximum
         constexpr uint32_t INF = HALF ? 0x7c00u : 0x7f800000u;
         uint32_t best = 0;
-        for (int kc = tid; kc < live_chunks; kc += 256) {
-            Raw16<HALF> r;
-            load_raw<HALF>(row, kc * 16, p.K, vec, r);
-            if constexpr (HALF) {
+        for (int u = first; u * 16 < p.K; u += 256) {
+            uint32_t raw[16];
+            load_piece<HALF>(row, u * 16, p.K, lane, raw);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const uint32_t lo = r.w[i] & 0x7fffu, hi = (r.w[i] >> 16) & 0x7fffu;
-                    if (lo <= INF) best = max(best, lo);
-                    if (hi <= INF) best = max(best, hi);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const uint32_t a = r.w[i] & 0x7fffffffu;
-                    if (a <= INF) best = max(best, a);
-                }
+            for (int i = 0; i < 16; ++i) {
+                const uint32_t bits = raw[i] & (HALF ? 0x7fffu : 0x7fffffffu);
+                if (bits <= INF) best = max(best, bits);
             }
         }
         best = __reduce_max_sync(0xffffffffu, best);
@@ -163,13 +155,14 @@ __global__ void __launch_bounds__(256) w8_quantize_kernel(const W8QuantParams p)
     const float inv = live ? __fdiv_rn(1.0f, s) : 0.f;
     const int mt = m / p.T, t = m - mt * p.T;
     uint4* dst = reinterpret_cast<uint4*>(p.Xq) + ((size_t)mt * chunks) * p.T + t;
-    for (int kc = tid; kc < chunks; kc += 256) {
-        uint32_t w[4] = {0u, 0u, 0u, 0u};
-        if (live && kc < live_chunks) {
-            Raw16<HALF> r;
-            float v[16];
-            load_raw<HALF>(row, kc * 16, p.K, vec, r);
-            raw_to_float<HALF>(r, v);
+    for (int u = first; u < chunks; u += 256) {
+        uint32_t raw[16], w[4] = {0u, 0u, 0u, 0u};
+        float v[16];
+        load_piece<HALF>(row, u * 16, p.K, lane, raw);
+        exchange_piece<HALF>(s_words[tid >> 5], lane, raw, v);
+        const int kc = u + lane;
+        if (kc >= chunks) continue;                  // (some lanes of the row's last piece; every warp is at its last turn then)
+        if (live) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
 #pragma unroll
