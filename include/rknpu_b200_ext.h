@@ -165,12 +165,11 @@ int rk_npu_b200_w4a8_schedule(const rk_npu_w4a8_workspace *workspace, int *varia
  * since the CTA's start at: weights requested, dependency met, scales known, slice quantised,
  * contraction done, partials exchanged -- and the end (ns); trace_read copies stamps[ctas][8]
  * (CTA index = blockIdx.y * gridDim.x + blockIdx.x, at most 16384 CTAs).
- * Persistent large-batch GEMM: CTA pair 0 records per tile (or part of one) j < 16 at [8 j + 0..6] the
- * cycles since kernel start at which the MMA issuer begins, issues its first MMA, commits the last,
- * the epilogue sees the accumulator, hands tensor memory back, has stored the tile, and the cycles the
- * issuer waited for operands; [128], [129] the cycles one unpack warp waited for weights and for a free
- * tensor-memory buffer in the whole launch, [160] those until activations had landed; [200] the CTA
- * pairs in the grid.
+ * Persistent large-batch GEMM: CTA pair 0 records per item (or part of one) j < 16 the cycles since kernel
+ * start at which the MMA issuer begins [8 j], commits the last stage [8 j + 2], the epilogue sees the
+ * accumulator [8 j + 3], hands tensor memory back [8 j + 4] and has stored the item [8 j + 5]; [128], [129]
+ * the cycles one unpack warp waited for weights and for a free tensor-memory buffer in the whole launch,
+ * [160] those until activations had landed; [200] the CTA pairs in the grid.
  * The caller synchronises first.  `bench.py --case decode|prefill --stamps` prints both. */
 int rk_npu_b200_w4a8_trace_enable(rk_npu_w4a8_workspace *workspace, int enable);
 int rk_npu_b200_w4a8_trace_read(rk_npu_w4a8_workspace *workspace, unsigned long long *stamps, int ctas);
