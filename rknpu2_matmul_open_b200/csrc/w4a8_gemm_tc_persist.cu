@@ -879,7 +879,7 @@ PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swigl
             longest = KB * block(width) / split + finish(width) +
                       (cost.part0 + cost.part * (split - 1) + cost.pair * clusters) * (1 + cost.part_wide * std::max(0, width - 64) / 64.0);
         } else
-            for (int i = 0; i < clusters; ++i) {
+            for (int i = 0; i < clusters && (best_time == 0 || longest < best_time); ++i) {   // (no better than the best: given up)
                 PersistItems items(persist_bound(units, per_tile, snap, i, clusters), persist_bound(units, per_tile, snap, i + 1, clusters), per_tile, most);
                 int tile, first, n;
                 double time = 0, last = 0;
