@@ -47,7 +47,7 @@ inline bool mid_batch_takes_ring(int M, int K, bool half)
 
 // CTA pairs of a persistent launch: one per part where tiles are cut along K (no part waits for another, the last to arrive
 // finishes the tile, so more pairs than are resident at once run in turn), else at most as many as can be resident, each
-// with a run of whole tiles.
+// with a run of items.
 inline int persist_clusters(int tiles, int split, int resident)
 {
     if (split > 1) return tiles * split;
