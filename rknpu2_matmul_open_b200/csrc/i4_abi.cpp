@@ -245,7 +245,7 @@ extern "C" rk_npu_i4_workspace* rk_npu_i4_workspace_create(rk_npu_iommu_domain* 
         ws->KB = (cfg->K + KBLOCK - 1) / KBLOCK;
         const PersistPlan plan = gemm_tc_persist_plan(cfg->N, cfg->M, ws->KB, false, false, ctx->sm_count);
         ws->plan = plan;
-        ws->codes_bytes = size_t(align_up(cfg->M, PERSIST_TOKENS)) * size_t(ws->KB) * KBLOCK;
+        ws->codes_bytes = size_t(align_up64(cfg->M, PERSIST_TOKENS)) * size_t(ws->KB) * KBLOCK;
         ws->partials_bytes = gemm_tc_persist_slot_bytes(cfg->N, cfg->M, plan);
         ws->counts_bytes = gemm_tc_persist_count_bytes(cfg->N, cfg->M, plan);
         ws->stage_in_bytes = size_t(cfg->M) * cfg->K;

@@ -1,0 +1,196 @@
+// persist_plan.h -- how a launch of the persistent GEMM (w4a8_gemm_tc_persist.cu) is cut into items: the dealing, which every role
+// of the kernel walks on the GPU, and the plan, made on the host once for a workspace.  Arithmetic on sizes; needs no CUDA.
+#pragma once
+#include <algorithm>
+#include <stddef.h>
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define RKB200_HD __host__ __device__ __forceinline__
+#else
+#define RKB200_HD inline
+#endif
+
+namespace rkb200 {
+
+constexpr int PERSIST_T = 8;            // tokens of a group of activation codes (GemmParams::T)
+constexpr int PERSIST_TOKENS = 32;      // the code buffer holds a whole multiple of these, items are multiples of them
+
+// The widest item of a kernel that takes the plan's.  (int8 weights: the first and the last.)
+constexpr int PS_NARROW = 64, PS_WIDE = 160, PS_WIDEST = 256;
+
+// How a problem is cut (columns: all accumulator rows, i.e. gate and up together for SwiGLU): pairs of channel tiles x units of
+// tokens, dealt to the CTA pairs in runs.
+struct PersistPlan {
+    int unit;     // tokens, a multiple of 32
+    int most;     // units of an item
+    int snap;     // see persist_bound
+    int split;    // parts K is cut into; one item per launch unit then, and most is 1
+};
+
+// CTA pairs of a launch: one per part where tiles are cut along K (no part waits for another, the last to arrive finishes the
+// tile, so more pairs than are resident at once run in turn), else at most as many as can be resident, each with a run of items.
+inline int persist_clusters(int tiles, int split, int resident)
+{
+    if (split > 1) return tiles * split;
+    return tiles < resident ? tiles : resident;
+}
+
+// A channel tile's tokens are counted in units; all units of all channel tiles, one tile's behind the other's, are dealt to
+// the CTA pairs in equal runs: run i begins at units * i / pairs.  Where a run would begin or end less than `snap` units from the
+// edge of a channel tile, the edge is taken: a narrow item costs nearly as much as a wide one.  The host divides by the pairs,
+// before anything is multiplied: nothing here is larger than `units`, and the rounded-up inverse is exact for rest * i * pairs
+// below 2^32, i.e. up to 1600 pairs.  (64-bit divisions on the GPU cost a launch of K = 1024 a microsecond.)
+struct PersistShare {
+    unsigned whole, rest;       // units / pairs and what is left
+    unsigned inverse;           // 2^32 / pairs, rounded up (0 for one pair, which has no rest)
+};
+inline PersistShare persist_share(unsigned units, unsigned pairs)
+{
+    return {units / pairs, units % pairs, unsigned(((uint64_t(1) << 32) + pairs - 1) / pairs)};
+}
+RKB200_HD unsigned persist_bound(PersistShare share, unsigned per_tile, unsigned snap, unsigned i)
+{
+    const unsigned x = share.whole * i + (unsigned)(((uint64_t)(share.rest * i) * share.inverse) >> 32), in = x % per_tile;
+    if (in && in < snap) return x - in;
+    if (in && per_tile - in < snap) return x + per_tile - in;
+    return x;
+}
+inline unsigned persist_bound(unsigned units, unsigned per_tile, unsigned snap, unsigned i, unsigned pairs)
+{
+    return persist_bound(persist_share(units, pairs), per_tile, snap, i);
+}
+
+// The items of one run, in order: what lies in one channel tile is cut into as few items of at most `most` units as
+// possible, of nearly equal width.
+struct PersistItems {
+    unsigned tile, first;       // where the next item begins: channel tile, unit inside it
+    unsigned left_units;        // of the run
+    unsigned per_tile, most;
+    unsigned pieces, seg_end;   // items left in this channel tile, and their end inside it
+    RKB200_HD PersistItems(unsigned begin, unsigned end, unsigned units_per_tile, unsigned most_units)
+        : tile(begin / units_per_tile), first(begin - begin / units_per_tile * units_per_tile), left_units(end - begin), per_tile(units_per_tile), most(most_units), pieces(0), seg_end(0) {}
+    // channel tile, first unit inside it and units of the next item; false: there is none
+    RKB200_HD bool next(int& in_tile, int& at, int& units)
+    {
+        if (!left_units) return false;
+        if (!pieces) {
+            seg_end = first + left_units < per_tile ? first + left_units : per_tile;
+            pieces = most == 1 ? seg_end - first : (seg_end - first + most - 1) / most;
+        }
+        const unsigned n = most == 1 ? 1 : (seg_end - first + pieces - 1) / pieces;
+        in_tile = (int)tile;
+        at = (int)first;
+        units = (int)n;
+        first += n;
+        left_units -= n;
+        if (--pieces == 0 && first == per_tile) { first = 0; ++tile; }
+        return true;
+    }
+};
+
+// The same items without walking them: visit(units of an item, how many of them follow each other, whether the tile ends with
+// them) for `len` units of one channel tile, and for a run visit(first unit inside the tile, units, how many tiles alike).
+template <class Visit>
+inline void persist_widths(unsigned len, unsigned most, Visit visit)
+{
+    const unsigned pieces = (len + most - 1) / most, wider = pieces ? len % pieces : 0;
+    if (wider) visit(len / pieces + 1, wider);
+    if (pieces) visit(len / pieces, pieces - wider);
+}
+template <class Visit>
+inline void persist_stretches(unsigned begin, unsigned end, unsigned per_tile, Visit visit)
+{
+    if (const unsigned in = begin % per_tile; in && begin < end) {
+        const unsigned head = std::min(end - begin, per_tile - in);
+        visit(in, head, 1u);
+        begin += head;
+    }
+    if (const unsigned tiles = (end - begin) / per_tile) visit(0u, per_tile, tiles);
+    if (const unsigned tail = (end - begin) % per_tile) visit(0u, tail, 1u);
+}
+
+// The cheapest cut by a model of the kernel's time in cycles, fitted to every cut of 350 shapes (1 to 3000
+// tokens, K 1024 .. 11008, 2048 .. 28672 channels; linear, SwiGLU and int8-weight launches).  What it takes is within 0.6, 0.6
+// and 2.5 % of the best cut in the mean and within 9, 6 and 15 % at worst (64 x 8192 -> 2048 15.5 us where three parts of
+// 32-token tiles take 14.3):
+//   * a k-block of an item costs a constant (the issuer's and the unpack warps' chains) and something per token: 305 + 0.6 per
+//     token with four-byte-packed weights, of which the MMAs need two per token, so wide items pay; less where SMs are idle;
+//   * finishing an item is hidden behind the next one's MMAs (two accumulators) unless it takes longer;
+//   * K in parts costs an exchange through L2: so much per part and pair, more for wide items;
+//   * a launch on more than half of the SMs leaves the one behind it no room to set itself up meanwhile.
+// A run is priced by its stretches of equal items, so that a plan takes the same few microseconds whatever the token count.
+struct PersistCosts {
+    double narrow, narrow_token, wide, wide_token, widest, widest_token;   // cycles of a k-block in each kernel
+    double finish, finish_token, item;               // of finishing an item, and between two items
+    double part0, part, pair, part_wide;             // the exchange of parts
+    double crowded, idle;
+};
+inline PersistPlan persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
+{
+    static const PersistCosts linear{270, 1.15, 305, 0.6, 339, 0.845, 2200, 31, 195, 870, 1590, 23, 0.65, 1530, 0.17};
+    static const PersistCosts gated{366, 0.79, 420, 0.37, 326, 1.0, 5060, 60, 670, 1500, 1380, 30, 0.7, 2030, 0.15};
+    static const PersistCosts bytes{323, 0.63, 380, 1.2, 380, 1.2, 2430, 32, 725, 1490, 1000, 21, 1.12, 720, 0.18};
+    const PersistCosts& cost = w8 ? bytes : swiglu ? gated : linear;
+    PersistPlan best{PERSIST_TOKENS, 1, 0, 1};
+    const int64_t channel_tiles = (int64_t(columns) + 255) / 256, tokens = (int64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS;
+    if (channel_tiles * (tokens / PERSIST_TOKENS) > INT32_MAX) return best;      // (its activations or results fit no GPU)
+    double best_time = 0;
+    const int pairs = std::max(1, sm_count / 2);
+    auto consider = [&](int unit, int most, int snap, int split) {
+        const unsigned per_tile = unsigned((tokens + unit - 1) / unit), units = unsigned(channel_tiles) * per_tile;
+        const int clusters = persist_clusters(int(units), split, pairs);
+        const double load = 1 - cost.idle * (1 - std::min(1.0, double(clusters) / pairs));
+        const bool narrow = unit * most <= PS_NARROW, wide = unit * most <= PS_WIDE, hidden = w8 || wide;
+        auto block = [&](double width) {
+            return load * (narrow ? cost.narrow + cost.narrow_token * width : wide ? cost.wide + cost.wide_token * width : cost.widest + cost.widest_token * width);
+        };
+        auto finish = [&](double width) { return cost.finish + cost.finish_token * (columns % 4 ? 2.5 : 1) * width; };   // (narrower stores)
+        auto run = [&](unsigned begin, unsigned end) {
+            double time = 0, last = 0;                       // `last`: finishing the item in front, not paid for yet
+            auto alike = [&](double width, unsigned n) {
+                const double mmas = KB * block(width) + cost.item, then = finish(width);
+                time += hidden ? std::max(mmas, last) : mmas + last;
+                time += (n - 1) * (hidden ? std::max(mmas, then) : mmas + then);
+                last = then;
+            };
+            persist_stretches(begin, end, per_tile, [&](unsigned first, unsigned len, unsigned tiles) {
+                const bool cut = first + len == per_tile && int64_t(per_tile) * unit > tokens;    // (items of one unit then)
+                auto tile = [&] {
+                    persist_widths(len, most, [&](unsigned n_units, unsigned n) {
+                        if (n > cut) alike(double(n_units) * unit, n - cut);
+                        if (cut) alike(double(tokens - int64_t(per_tile - 1) * unit), 1);
+                    });
+                };
+                tile();
+                if (tiles == 1) return;
+                const double so_far = time;
+                tile();
+                time += (tiles - 2) * (time - so_far);
+            });
+            return time + last;
+        };
+        const PersistShare dealt = persist_share(units, unsigned(clusters));
+        double longest = 0;
+        if (split > 1) {
+            const double width = double(std::min<int64_t>(unit, tokens));
+            longest = KB * block(width) / split + finish(width) +
+                      (cost.part0 + cost.part * (split - 1) + cost.pair * clusters) * (1 + cost.part_wide * std::max(0.0, width - 64) / 64.0);
+        } else
+            for (int i = 0; i < clusters && (best_time == 0 || longest < best_time); ++i)   // (no better than the best: given up)
+                longest = std::max(longest, run(persist_bound(dealt, per_tile, snap, i), persist_bound(dealt, per_tile, snap, i + 1)));
+        if (2 * clusters > pairs) longest += cost.crowded;
+        if (best_time == 0 || longest < best_time) { best_time = longest; best = {unit, most, snap, split}; }
+    };
+    const int widest = int(std::min<int64_t>(PS_WIDEST, tokens));
+    for (int unit = PERSIST_TOKENS; unit <= widest; unit += PERSIST_TOKENS)       // items of one width, K in parts or not
+        for (const int split : {1, 2, 3, 4, 6, 8}) {
+            if (split > 1 && (unit > PS_WIDE || channel_tiles * ((tokens + unit - 1) / unit) * split > pairs || KB < 4 * split)) break;
+            consider(unit, 1, 0, split);
+        }
+    for (int most = 2; most <= widest / PERSIST_TOKENS; ++most)                  // equal runs
+        for (const int snap : {0, 2, 3}) consider(PERSIST_TOKENS, most, snap, 1);
+    return best;
+}
+
+} // namespace rkb200

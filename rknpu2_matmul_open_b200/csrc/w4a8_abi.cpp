@@ -1186,7 +1186,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     if (schedule.cluster && (variant == 1 || variant == 5 || (variant == 3 && (ws->KB + schedule.cluster - 1) / schedule.cluster <= FUSED_MAX_STAGES)) &&
         (variant == 5 || ws->KB >= schedule.cluster))
         ws->split_override = schedule.cluster;
-    const size_t Mp = size_t(align_up(cfg->M, variant == 2 ? PERSIST_TOKENS : ws->T));
+    const size_t Mp = size_t(align_up64(cfg->M, variant == 2 ? PERSIST_TOKENS : ws->T));
     ws->codes_bytes = Mp * size_t(ws->KB) * KBLOCK;
     const int out_cols = cfg->N;
     ws->stage_in_bytes = size_t(cfg->M) * cfg->K * 4;

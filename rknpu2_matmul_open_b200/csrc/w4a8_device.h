@@ -26,6 +26,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "persist_plan.h"
+
 namespace rkb200 {
 
 // A function attribute such as the dynamic shared-memory opt-in belongs to one device.  A process may
@@ -123,6 +125,7 @@ struct GemmParams {
     int epi;
     int split;              // split-K factor == cluster size along y (1, 2, 4, 8)
     int unit, most, snap;   // persistent kernel: its PersistPlan
+    PersistShare share;     // and what a run holds of its units (set by the launch)
     const PersistMaps* maps; // persistent kernel: in host memory, copied with the launch
     int w8;                 // persistent kernel: Wp holds int8 codes in the W8 layout (w8a8_kernels.cu), sums are not scaled by 16
     unsigned long long timeout_ns;
@@ -261,18 +264,8 @@ cudaError_t launch_gemm_decode(const DecodeParams& p, cudaStream_t stream, bool 
 cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, bool pdl);
 // Persistent two-CTA tcgen05 kernel (K <= 131072).  Its activation codes lie in groups of PERSIST_T tokens (p.T) up to a
 // multiple of 32 tokens; p.partials and p.counts where split > 1.
-constexpr int PERSIST_T = 8;
-constexpr int PERSIST_TOKENS = 32;
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
 bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB);
-// How the persistent kernel cuts a problem (columns: all accumulator rows, i.e. gate and up together for SwiGLU): pairs of
-// channel tiles x units of tokens, dealt to the CTA pairs in runs (w4a8_rules.h)
-struct PersistPlan {
-    int unit;     // tokens, a multiple of 32
-    int most;     // units of an item
-    int snap;     // see persist_bound
-    int split;    // parts K is cut into; one item per launch unit then, and most is 1
-};
 inline void set_plan(GemmParams& p, const PersistPlan& plan)
 {
     p.unit = plan.unit;
@@ -281,7 +274,6 @@ inline void set_plan(GemmParams& p, const PersistPlan& plan)
     p.split = plan.split;
 }
 PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count);
-int gemm_tc_persist_units(int columns, int M, int unit);
 // Bytes of GemmParams.partials and .counts (the latter zero before the first launch); 0 where nothing is split
 size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan);
 size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan);

@@ -24,10 +24,8 @@
 // Outputs: binary16 / fp32 / int32 [M,N], or the fused SwiGLU middle [M,F] fp32 (row maxima collected).
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
-#include "w4a8_rules.h"
 #include "w4a8_ptx.cuh"
 #include "w4a8_tc.cuh"
-#include <algorithm>
 
 namespace rkb200 {
 
@@ -158,15 +156,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     constexpr bool swiglu = SWIGLU;
     const int KB = p.KB;
     const int nst = (KB + PS_SK - 1) / PS_SK;                          // stages of a tile
-    const int tiles_n = swiglu ? (p.F + 63) / 64 : (p.N + TILE_N - 1) / TILE_N;
-    const int pairs_n = (tiles_n + 1) / 2;
     // Every cluster takes a run of items over all of K, or (split > 1) one of the `split` parts of one tile's stages.
     const int per_tile = (p.M + p.unit - 1) / p.unit, split = p.split;
-    const unsigned units = (unsigned)pairs_n * (unsigned)per_tile;
     const int part = cluster_id % split;
     const int it0 = nst * part / split, it1 = nst * (part + 1) / split;
-    const unsigned unit0 = split > 1 ? (unsigned)(cluster_id / split) : persist_bound(units, per_tile, p.snap, cluster_id, num_clusters);
-    const unsigned unit1 = split > 1 ? unit0 + 1 : persist_bound(units, per_tile, p.snap, cluster_id + 1, num_clusters);
+    const unsigned unit0 = split > 1 ? (unsigned)(cluster_id / split) : persist_bound(p.share, per_tile, p.snap, cluster_id);
+    const unsigned unit1 = split > 1 ? unit0 + 1 : persist_bound(p.share, per_tile, p.snap, cluster_id + 1);
     // an item: pair of channel tiles, first token, tokens the MMAs take (a multiple of 32)
     struct Item { int tile, tok0, width; };
     PersistItems items(unit0, unit1, per_tile, p.most);
@@ -786,8 +781,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
 namespace {
 constexpr long long PS_MAX_K = 131072;
 
-// The widest item of a kernel that takes the plan's.
-constexpr int PS_NARROW = 64, PS_WIDE = 160, PS_WIDEST = 256;   // (int8 weights: narrow and widest)
+int units_of(int columns, int M, int unit) { return ((columns - 1) / 256 + 1) * ((M - 1) / unit + 1); }
 
 template <bool W8, bool SWIGLU, int TOK>
 cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool pdl)
@@ -822,7 +816,9 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
         max_clusters = n;
         if (device >= 0 && device < 64) { clusters_of_device[device] = n; configured.mark(device); }
     }
-    const int clusters = persist_clusters(gemm_tc_persist_units(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, p.unit), p.split, max_clusters);
+    const int units = units_of(p.epi == EPI_SWIGLU ? 2 * p.F : p.N, p.M, p.unit), clusters = persist_clusters(units, p.split, max_clusters);
+    GemmParams q = p;
+    q.share = persist_share((unsigned)units, (unsigned)clusters);
     cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
     int n = 1;
     if (pdl) {
@@ -832,83 +828,19 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, kernel, p, *p.maps, clusters);
+    return cudaLaunchKernelEx(&cfg, kernel, q, *p.maps, clusters);
 }
 } // namespace
 
-int gemm_tc_persist_units(int columns, int M, int unit) { return (columns + 255) / 256 * ((M + unit - 1) / unit); }
 
-// How a problem is cut: the cheapest by a model of the kernel's time in cycles, fitted to every cut of 350 shapes (1 to 3000
-// tokens, K 1024 .. 11008, 2048 .. 28672 channels; linear, SwiGLU and int8-weight launches).  What it takes is within 0.6, 0.6
-// and 2.5 % of the best cut in the mean and within 9, 6 and 15 % at worst (64 x 8192 -> 2048 15.5 us where three parts of
-// 32-token tiles take 14.3):
-//   * a k-block of an item costs a constant (the issuer's and the unpack warps' chains) and something per token: 305 + 0.6 per
-//     token with four-byte-packed weights, of which the MMAs need two per token, so wide items pay; less where SMs are idle;
-//   * finishing an item is hidden behind the next one's MMAs (two accumulators) unless it takes longer;
-//   * K in parts costs an exchange through L2: so much per part and pair, more for wide items;
-//   * a launch on more than half of the SMs leaves the one behind it no room to set itself up meanwhile.
-struct PersistCosts {
-    double narrow, narrow_token, wide, wide_token, widest, widest_token;   // cycles of a k-block in each kernel
-    double finish, finish_token, item;               // of finishing an item, and between two items
-    double part0, part, pair, part_wide;             // the exchange of parts
-    double crowded, idle;
-};
-PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
-{
-    static const PersistCosts linear{270, 1.15, 305, 0.6, 339, 0.845, 2200, 31, 195, 870, 1590, 23, 0.65, 1530, 0.17};
-    static const PersistCosts gated{366, 0.79, 420, 0.37, 326, 1.0, 5060, 60, 670, 1500, 1380, 30, 0.7, 2030, 0.15};
-    static const PersistCosts bytes{323, 0.63, 380, 1.2, 380, 1.2, 2430, 32, 725, 1490, 1000, 21, 1.12, 720, 0.18};
-    const PersistCosts& cost = w8 ? bytes : swiglu ? gated : linear;
-    PersistPlan best{PERSIST_TOKENS, 1, 0, 1};
-    double best_time = 0;
-    const int pairs = std::max(1, sm_count / 2), channel_tiles = (columns + 255) / 256, widest = PS_WIDEST;
-    const int tokens = (M + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS;
-    auto consider = [&](int unit, int most, int snap, int split) {
-        const int per_tile = (M + unit - 1) / unit;
-        const unsigned units = unsigned(channel_tiles) * unsigned(per_tile);
-        const int clusters = persist_clusters(int(units), split, pairs);
-        const double share = 1 - cost.idle * (1 - std::min(1.0, double(clusters) / pairs));
-        const bool narrow = unit * most <= PS_NARROW, wide = unit * most <= PS_WIDE, hidden = w8 || wide;
-        auto block = [&](int width) {
-            return share * (narrow ? cost.narrow + cost.narrow_token * width : wide ? cost.wide + cost.wide_token * width : cost.widest + cost.widest_token * width);
-        };
-        auto finish = [&](int width) { return cost.finish + cost.finish_token * (columns % 4 ? 2.5 : 1) * width; };   // (narrower stores)
-        double longest = 0;
-        if (split > 1) {
-            const int width = std::min(unit, tokens);
-            longest = KB * block(width) / split + finish(width) +
-                      (cost.part0 + cost.part * (split - 1) + cost.pair * clusters) * (1 + cost.part_wide * std::max(0, width - 64) / 64.0);
-        } else
-            for (int i = 0; i < clusters && (best_time == 0 || longest < best_time); ++i) {   // (no better than the best: given up)
-                PersistItems items(persist_bound(units, per_tile, snap, i, clusters), persist_bound(units, per_tile, snap, i + 1, clusters), per_tile, most);
-                int tile, first, n;
-                double time = 0, last = 0;
-                while (items.next(tile, first, n)) {
-                    const int width = std::min(n * unit, tokens - first * unit);
-                    time += std::max(KB * block(width) + cost.item, hidden ? last : 0) + (hidden ? 0 : last);
-                    last = finish(width);
-                }
-                longest = std::max(longest, time + last);
-            }
-        if (2 * clusters > pairs) longest += cost.crowded;
-        if (best_time == 0 || longest < best_time) { best_time = longest; best = {unit, most, snap, split}; }
-    };
-    for (int unit = PERSIST_TOKENS; unit <= std::min(widest, tokens); unit += PERSIST_TOKENS)       // items of one width, K in parts or not
-        for (const int split : {1, 2, 3, 4, 6, 8}) {
-            if (split > 1 && (unit > PS_WIDE || (long long)channel_tiles * ((M + unit - 1) / unit) * split > pairs || KB < 4 * split)) break;
-            consider(unit, 1, 0, split);
-        }
-    for (int most = 2; most <= std::min(widest, tokens) / PERSIST_TOKENS; ++most)                  // equal runs
-        for (const int snap : {0, 2, 3}) consider(PERSIST_TOKENS, most, snap, 1);
-    return best;
-}
+PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count) { return persist_plan(columns, M, KB, w8, swiglu, sm_count); }
 size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan)
 {
-    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_units(columns, M, plan.unit)) * size_t(plan.split) * 128 * size_t(plan.unit) * sizeof(int) : 0;
+    return plan.split > 1 ? 2 * size_t(units_of(columns, M, plan.unit)) * size_t(plan.split) * 128 * size_t(plan.unit) * sizeof(int) : 0;
 }
 size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan)
 {
-    return plan.split > 1 ? 2 * size_t(gemm_tc_persist_units(columns, M, plan.unit)) * sizeof(unsigned) : 0;
+    return plan.split > 1 ? 2 * size_t(units_of(columns, M, plan.unit)) * sizeof(unsigned) : 0;
 }
 
 // Eight-byte elements: 256 of them, the most a box may have, are the two k-blocks of a stage.
@@ -924,7 +856,7 @@ bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB)
         return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(entry);
     }();
     if (!encode) return false;
-    const cuuint64_t dims[2] = {cuuint64_t(KB) * 128, cuuint64_t((M + PERSIST_TOKENS - 1) / PERSIST_TOKENS * (PERSIST_TOKENS / PERSIST_T))};
+    const cuuint64_t dims[2] = {cuuint64_t(KB) * 128, (cuuint64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * (PERSIST_TOKENS / PERSIST_T)};
     const cuuint64_t strides[1] = {cuuint64_t(KB) * 1024};
     const cuuint32_t steps[2] = {1, 1};
     for (int i = 0; i < 3; ++i) {

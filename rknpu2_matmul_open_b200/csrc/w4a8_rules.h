@@ -2,6 +2,8 @@
 #pragma once
 #include <stddef.h>
 
+#include "persist_plan.h"
+
 namespace rkb200 {
 
 // Whether a blocking call's kernel stores its [M][cols] result of `elem` bytes each straight into page-locked host memory
@@ -37,63 +39,5 @@ inline bool mid_batch_takes_ring(int M, int K, bool half)
     const bool wide = K % 8 == 0;
     return half ? !wide && M > 10 : M > (wide ? 12 : 8);
 }
-
-// ---- how a persistent launch is cut (used by its plan on the host and by every role of the kernel on the GPU)
-#ifdef __CUDACC__
-#define RKB200_HD __host__ __device__ __forceinline__
-#else
-#define RKB200_HD inline
-#endif
-
-// CTA pairs of a persistent launch: one per part where tiles are cut along K (no part waits for another, the last to arrive
-// finishes the tile, so more pairs than are resident at once run in turn), else at most as many as can be resident, each
-// with a run of items.
-inline int persist_clusters(int tiles, int split, int resident)
-{
-    if (split > 1) return tiles * split;
-    return tiles < resident ? tiles : resident;
-}
-
-// A channel tile's tokens are counted in units; all units of all channel tiles, one tile's behind the other's, are dealt to
-// the CTA pairs in equal runs.  Where a run would begin or end less than `snap` units from the edge of a channel tile, the
-// edge is taken: a narrow item costs nearly as much as a wide one.  (A result has fewer than 2^31 elements and an item takes at
-// least 256 channels x 32 tokens, so that units x pairs fits in 32 bits; wider divisions cost a launch of K = 1024 a
-// microsecond.)
-RKB200_HD unsigned persist_bound(unsigned units, unsigned per_tile, unsigned snap, unsigned i, unsigned pairs)
-{
-    const unsigned x = units * i / pairs, in = x % per_tile;
-    if (in && in < snap) return x - in;
-    if (in && per_tile - in < snap) return x + per_tile - in;
-    return x;
-}
-
-// The items of one run, in order: what lies in one channel tile is cut into as few items of at most `most` units as
-// possible, of nearly equal width.
-struct PersistItems {
-    unsigned tile, first;       // where the next item begins: channel tile, unit inside it
-    unsigned left_units;        // of the run
-    unsigned per_tile, most;
-    unsigned pieces, seg_end;   // items left in this channel tile, and their end inside it
-    RKB200_HD PersistItems(unsigned begin, unsigned end, unsigned units_per_tile, unsigned most_units)
-        : tile(begin / units_per_tile), first(begin - begin / units_per_tile * units_per_tile), left_units(end - begin), per_tile(units_per_tile), most(most_units), pieces(0), seg_end(0) {}
-    RKB200_HD bool more() const { return left_units != 0; }
-    // channel tile, first unit inside it and units of the next item; false: there is none
-    RKB200_HD bool next(int& in_tile, int& at, int& units)
-    {
-        if (!left_units) return false;
-        if (!pieces) {
-            seg_end = first + left_units < per_tile ? first + left_units : per_tile;
-            pieces = most == 1 ? seg_end - first : (seg_end - first + most - 1) / most;
-        }
-        const unsigned n = most == 1 ? 1 : (seg_end - first + pieces - 1) / pieces;
-        in_tile = (int)tile;
-        at = (int)first;
-        units = (int)n;
-        first += n;
-        left_units -= n;
-        if (--pieces == 0 && first == per_tile) { first = 0; ++tile; }
-        return true;
-    }
-};
 
 } // namespace rkb200

@@ -108,7 +108,7 @@ Sizes sizes_of(int M, int N, int K, int kind)
     const PersistPlan plan = gemm_tc_persist_plan(N, M, z.KB, true, false, PLAN_SMS);
     z.plan = plan;
     z.NG = align_up((N + GROUP - 1) / GROUP, 8) + 8;   // zero groups behind the last tile, as for the int4 weights
-    z.codes = size_t(align_up(M, PERSIST_TOKENS)) * size_t(z.KB) * KBLOCK;
+    z.codes = size_t(align_up64(M, PERSIST_TOKENS)) * size_t(z.KB) * KBLOCK;
     z.partials = gemm_tc_persist_slot_bytes(N, M, plan);
     z.counts = gemm_tc_persist_count_bytes(N, M, plan);
     z.scales = sizeof(float) * 2 * size_t(M);

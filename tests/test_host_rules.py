@@ -141,3 +141,57 @@ int main()
     return 0;
 }
 """)
+
+
+def test_runs_of_very_many_units(tmp_path):
+    # one channel tile of 2^31 tokens is 2^26 units: runs begin in order and cover all of them, and the plan, made for every
+    # memory query, does not take longer for it; its stretches of equal items are the items that the kernel walks
+    _run(tmp_path, r"""
+#include "persist_plan.h"
+#include <initializer_list>
+#include <stdio.h>
+#include <time.h>
+#include <vector>
+using namespace rkb200;
+int main()
+{
+    for (unsigned units : {57456230u, 58000000u, 67108864u, 2147483647u, 4294967295u})
+        for (unsigned per_tile : {1u, 7u, 57456230u, 67108864u, 4294967295u})
+            for (unsigned snap : {0u, 3u})
+                for (unsigned pairs : {1u, 2u, 66u, 74u, 75u, 1600u}) {
+                    unsigned from = 0;
+                    for (unsigned i = 0; i < pairs; ++i) {
+                        const unsigned exact = (unsigned)((unsigned long long)units * i / pairs), at = persist_bound(units, per_tile, snap, i, pairs);
+                        if (at < from || (snap == 0 && at != exact)) { printf("run %u of %u over %u: %u\n", i, pairs, units, at); return 1; }
+                        from = at;
+                    }
+                    if (persist_bound(units, 1, snap, pairs, pairs) != units) return 2;
+                }
+    for (int M : {4096, 100000000, 2000000000, 2147483647})
+        for (int columns : {1, 300, 2147483647}) {
+            const clock_t before = clock();
+            for (int kind = 0; kind < 3; ++kind) persist_plan(columns, M, 1, kind == 1, kind == 2, 148);
+            if (clock() - before > CLOCKS_PER_SEC / 20) { printf("a plan for %d tokens, %d columns took %g s\n", M, columns, double(clock() - before) / CLOCKS_PER_SEC); return 3; }
+        }
+    struct Walked { int first, units; };
+    for (unsigned per_tile : {1u, 2u, 5u, 13u, 24u})
+        for (unsigned most = 1; most <= 8; ++most)
+            for (unsigned begin = 0; begin <= 2 * per_tile; ++begin)
+                for (unsigned end = begin; end <= 4 * per_tile; ++end) {
+                    std::vector<Walked> walked, told;
+                    PersistItems items(begin, end, per_tile, most);
+                    for (int tile, first, n; items.next(tile, first, n);) walked.push_back({first, n});
+                    persist_stretches(begin, end, per_tile, [&](unsigned first, unsigned len, unsigned tiles) {
+                        while (tiles--) {
+                            unsigned at = first;
+                            persist_widths(len, most, [&](unsigned units, unsigned n) { for (; n--; at += units) told.push_back({(int)at, (int)units}); });
+                            if (at != first + len) told.clear();
+                        }
+                    });
+                    bool same = walked.size() == told.size();
+                    for (size_t i = 0; same && i < walked.size(); ++i) same = walked[i].first == told[i].first && walked[i].units == told[i].units;
+                    if (!same) { printf("units %u to %u, %u a tile, most %u\n", begin, end, per_tile, most); return 4; }
+                }
+    return 0;
+}
+""")

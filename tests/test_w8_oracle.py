@@ -1,6 +1,7 @@
 """The W8A8 part of the oracle against the reference's own CPU kernels (its scales, quantise + packing and fused
 dequantisation compiled from its sources), and the pure host functions of the typed W8A8 API."""
 import ctypes as C
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -123,3 +124,15 @@ def test_memory_queries_and_argument_errors():
     t = w8a8.default_strategy(w8a8.I8I8I32, 4, 64, 64)
     t.npu_core_mask, t.n_tile = 7, 64            # fewer column groups than device cores
     assert lib.rk_npu_matmul_workspace_memory_query(C.byref(t), C.byref(req)) == capi.RK_NPU_ERR_PARAM
+
+
+@pytest.mark.parametrize("M", [100_000_000, 2_000_000_000, 2_147_483_600, 2_147_483_647])
+def test_memory_query_of_very_many_tokens(M):
+    # codes padded to 32 tokens x 128 bytes; answered in a child process, which is ended where the answer does not come
+    import subprocess
+    import sys
+    child = ("import ctypes as C, time; from rknpu2_matmul_open_b200 import capi, w8a8; lib = capi.load(); req = capi.MatmulWorkspaceRequirements()\n"
+             f"s = w8a8.default_strategy(w8a8.I8I8I32, {M}, 1, 1); t = time.perf_counter()\n"
+             "rc = lib.rk_npu_matmul_workspace_memory_query(C.byref(s), C.byref(req)); print(rc, req.input_bytes, time.perf_counter() - t < 0.01)")
+    out = subprocess.run([sys.executable, "-c", child], capture_output=True, text=True, timeout=60, check=True, cwd=Path(__file__).resolve().parents[1]).stdout.split()
+    assert out == ["0", str((M + 31) // 32 * 32 * 128 + M), "True"]
