@@ -28,6 +28,14 @@ struct PersistPlan {
     int split;    // parts K is cut into; one item per launch unit then, and most is 1
 };
 
+// Whether the kernel runs a cut: one of those that persist_plan chooses from, whatever it would choose.
+inline bool persist_cut_ok(const PersistPlan& cut, int KB)
+{
+    const bool grid = cut.most == 1 && cut.snap == 0 && cut.unit % PERSIST_TOKENS == 0, runs = cut.unit == PERSIST_TOKENS && cut.most > 1 && cut.snap >= 0 && cut.snap <= 3;
+    if (!(grid || runs) || cut.unit < PERSIST_TOKENS || cut.most > PS_WIDEST / PERSIST_TOKENS || cut.unit > PS_WIDEST || cut.split < 1 || cut.split > 8) return false;
+    return cut.split == 1 || (grid && cut.unit <= PS_WIDE && KB >= 4 * cut.split);
+}
+
 // CTA pairs of a launch: one per part where tiles are cut along K (no part waits for another, the last to arrive finishes the
 // tile, so more pairs than are resident at once run in turn), else at most as many as can be resident, each with a run of items.
 inline int persist_clusters(int tiles, int split, int resident)

@@ -26,6 +26,8 @@
 #include "w4a8_math.cuh"
 #include "w4a8_ptx.cuh"
 #include "w4a8_tc.cuh"
+#include <cstdio>
+#include <cstdlib>
 
 namespace rkb200 {
 
@@ -833,7 +835,13 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
 } // namespace
 
 
-PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count) { return persist_plan(columns, M, KB, w8, swiglu, sm_count); }
+PersistPlan gemm_tc_persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
+{
+    PersistPlan cut{};
+    const char* const text = std::getenv("RK_NPU_B200_PERSIST_CUT");   // experiments and tests: "unit,most,snap,split"
+    if (text && std::sscanf(text, "%d,%d,%d,%d", &cut.unit, &cut.most, &cut.snap, &cut.split) == 4 && persist_cut_ok(cut, KB)) return cut;
+    return persist_plan(columns, M, KB, w8, swiglu, sm_count);
+}
 size_t gemm_tc_persist_slot_bytes(int columns, int M, const PersistPlan& plan)
 {
     return plan.split > 1 ? 2 * size_t(units_of(columns, M, plan.unit)) * size_t(plan.split) * 128 * size_t(plan.unit) * sizeof(int) : 0;

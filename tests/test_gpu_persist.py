@@ -1,6 +1,6 @@
-"""The persistent tcgen05 kernel at the edges of its tiles: token tiles of 64, 128 and 256, the last token of a tile and
-the first of the next, channel tiles that are cut, K of one stage, of an odd number of k-blocks and in parts (few channel
-tiles, long K).  Sums and outputs are exact, so every comparison is bit for bit."""
+"""The persistent tcgen05 kernel as the plan cuts a problem: a few tokens to many, cut channel tiles, K of one stage, of an odd
+number of k-blocks and in parts (few channel tiles, long K), part counters and buffers used again.  Sums and outputs are exact, so
+every comparison is bit for bit.  (test_gpu_persist_items.py forces the cuts.)"""
 import numpy as np
 import pytest
 
@@ -15,7 +15,7 @@ def bits(x):
     return x.view(np.uint32) if x.dtype == np.float32 else x
 
 
-# (tokens, K, N): 64-token tiles whole and in parts, 128 in parts and whole, 256, one k-block, cut channel tiles
+# (tokens, K, N): few channel tiles and many, long K and one k-block, cut channel tiles
 SHAPES = [(17, 640, 3400), (64, 8192, 260), (65, 4224, 1100), (96, 384, 1281), (128, 11008, 512), (129, 128, 257), (200, 6000, 300),
           (256, 1100, 2049), (257, 2048, 130), (1030, 4096, 1024)]
 

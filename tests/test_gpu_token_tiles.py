@@ -1,6 +1,6 @@
-"""The wider token tiles of the persistent tcgen05 kernel (192 and 224 tokens), on sizes that the plan gives to them: whole
-and cut last tiles, one k-block and an odd number of them, several tiles per CTA pair, and an FFN whose two launches cut the
-tokens differently.  Bit for bit."""
+"""Token counts around the widths of items, as the plan cuts them (test_gpu_persist_items.py forces cuts): whole and cut last items,
+one k-block and an odd number of them, several items per CTA pair, and an FFN whose two launches cut the tokens differently, its
+workspace used as a linear and as a SwiGLU launch in turn.  Bit for bit."""
 import numpy as np
 import pytest
 

@@ -195,3 +195,46 @@ int main()
     return 0;
 }
 """)
+
+
+def test_cuts_that_the_gpu_tests_force(tmp_path):
+    # accepted as they are; every width of an item is among them, some runs begin or end inside a channel tile, and some pair takes
+    # more items than there are accumulators
+    from persist_cuts import GRIDS, LONG, LONG_FFN, PARTS, RUNS, WHOLE, WHOLE_FFN
+    cuts = [f"{{{M}, {K}, {N}, {{{cut}}}}}" for shapes, names in (((WHOLE, WHOLE_FFN), GRIDS + RUNS), ((LONG, LONG_FFN), PARTS))
+            for M, K, N in shapes for cut in names]
+    _run(tmp_path, r"""
+#include "persist_plan.h"
+#include <stdio.h>
+#include <set>
+using namespace rkb200;
+struct Cut { int M, K, N; PersistPlan plan; };
+int main()
+{
+    const Cut cuts[] = {CUTS};
+    const PersistPlan refused[] = {{0, 1, 0, 1}, {48, 1, 0, 1}, {288, 1, 0, 1}, {64, 2, 0, 1}, {32, 9, 0, 1}, {32, 2, 4, 1}, {32, 1, 0, 0}, {32, 1, 0, 9},
+                                   {192, 1, 0, 2}, {32, 2, 0, 2}, {32, 1, 0, 8}, {-32, 1, 0, 1}, {32, -1, 0, 1}, {32, 0, 0, 1}};
+    for (const PersistPlan& p : refused)
+        if (persist_cut_ok(p, 31)) { printf("%d,%d,%d,%d accepted\n", p.unit, p.most, p.snap, p.split); return 1; }
+    std::set<int> of_one_width, of_runs;
+    int inside = 0;
+    for (const Cut& c : cuts) {
+        const PersistPlan& p = c.plan;
+        if (!persist_cut_ok(p, (c.K + 127) / 128)) { printf("%d,%d,%d,%d refused\n", p.unit, p.most, p.snap, p.split); return 2; }
+        if (p.split > 1) continue;
+        const unsigned per_tile = (c.M + p.unit - 1) / p.unit, units = (c.N + 255) / 256 * per_tile, pairs = persist_clusters(units, 1, 74);
+        const int accumulators = p.unit * p.most > PS_WIDE ? 1 : 2;
+        int longest = 0;
+        for (unsigned i = 0; i < pairs; ++i) {
+            const unsigned from = persist_bound(units, per_tile, p.snap, i, pairs);
+            PersistItems items(from, persist_bound(units, per_tile, p.snap, i + 1, pairs), per_tile, p.most);
+            inside += from % per_tile != 0;
+            int n_items = 0;
+            for (int tile, first, n; items.next(tile, first, n); ++n_items) (p.most > 1 ? of_runs : of_one_width).insert(n * p.unit);
+            if (n_items > longest) longest = n_items;
+        }
+        if (longest <= accumulators) { printf("%d,%d,%d,%d: %d items a pair\n", p.unit, p.most, p.snap, p.split, longest); return 3; }
+    }
+    return of_one_width.size() == 8 && of_runs.size() == 8 && inside ? 0 : 4;
+}
+""".replace("CUTS", ", ".join(cuts)))
