@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                             f2_unpack(y[c][h], a, b);
                             most = max_abs(most, max_abs(a, b));
                         }
-                    if (gates_ok && silu_plain(1.f, most)) {
+                    if (gates_ok && silu_fast(most)) {
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
 #pragma unroll

@@ -130,16 +130,16 @@ __device__ __forceinline__ float silu_poly(float g)
     const float d = __fadd_rn(1.f, __fmul_rn(q, power));
     return g < -80.f ? -0.f : __fdiv_rn(g, d);
 }
-// The same function, two arguments at a time, for the kernels that evaluate it over and over; for arguments with |g| in
-// [2^-40, 80] only (silu_plain), where no step leaves the normal range: d < 2^116.
+// The same function, two arguments at a time, for the kernels that evaluate it over and over; for +0 and for |g| in [2^-40, 80]
+// only, where no step leaves the normal range: d < 2^116.  The caller sees to the upper end with silu_fast and to the lower one by
+// what g is made of: an integer sum times two positive scales is +0 or, where both are at least 2^-20, at least 2^-40.
 //   * floor(y) for |y| < 2^22: adding 1.5 * 2^23 with rounding towards minus infinity leaves floor(y) in the low bits,
 //     from where the subtraction brings it back as a float and a shift puts it into the exponent of 2^n.
 //   * g / d, correctly rounded: a reciprocal within an ulp refined by one Newton step, a quotient from it, its remainder
 //     by fused multiply-add (exact) and one correction (P. Markstein, "Computation of elementary functions on the IBM
 //     RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), all of it negated: the reciprocal of a negated argument
 //     costs nothing, the negation of a pair two instructions.  Returns the negated values.
-// With silu_poly for every other argument equal bit for bit to silu_poly for every one of the 2^32 arguments
-// (tests/test_gpu_silu_pairs.py tries them all).
+// Equal bit for bit to silu_poly, negated, for every argument it is for (tests/test_gpu_silu_pairs.py tries them all).
 __device__ __forceinline__ void minus_silu_poly2(float g0, float g1, float& y0, float& y1)
 {
     const F2 g = f2_pack(g0, g1);
@@ -168,10 +168,10 @@ __device__ __forceinline__ void minus_silu_poly2(float g0, float g1, float& y0, 
     const F2 quo = f2_mul(g, inv);
     f2_unpack(f2_fma(f2_fma(d, quo, g), inv, quo), y0, y1);
 }
-// Larger and smaller magnitude of two values; a NaN stays one.
+// Larger magnitude of two values; a NaN stays one.
 __device__ __forceinline__ float max_abs(float a, float b) { float d; asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b))); return d; }
-__device__ __forceinline__ float min_abs(float a, float b) { float d; asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b))); return d; }
-__device__ __forceinline__ bool silu_plain(float smallest, float largest) { return smallest >= 9.094947017729282e-13f && largest <= 80.f; }
+// Whether none of several arguments, whose largest magnitude this is, lies beyond minus_silu_poly2's upper end.
+__device__ __forceinline__ bool silu_fast(float largest) { return largest <= 80.f; }
 
 __device__ __forceinline__ float dequant(int acc, float sx, float sw)
 {
