@@ -3,10 +3,10 @@
 // Packed int4 weights -> tensor memory as the A operand (int8 weights stay in shared memory), int8 activation codes as
 // shared-memory B operand, kind::i8 MMA over a CTA pair with cta_group::2, int32 accumulators in tensor memory, organised so
 // that nothing but the tensor pipe sits on the critical path:
-//   * one cluster of two CTAs per SM pair stays resident and walks a run of items: 256 channels x up to 64 or 160 tokens (256
-//     with int8 weights), any multiple of 32 of them, so that equal runs leave no nearly empty last round (4096 -> 14336,
-//     2048 tokens: 13 rounds of 128-token tiles for 12.1 of work before).  Barriers, tensor memory and descriptors are set
-//     up once.  Where the tiles are few, K is cut into parts;
+//   * one cluster of two CTAs per SM pair stays resident and walks a run of items: 256 channels x any multiple of 32 tokens up to
+//     the kernel's width (64, 160 or 256; int8 weights 64 or 256), so that equal runs leave no nearly empty last round
+//     (4096 -> 14336, 2048 tokens: 13 rounds of 128-token tiles for 12.1 of work before).  Barriers, tensor memory and
+//     descriptors are set up once.  Where the tiles are few, K is cut into parts (persist_plan.h);
 //   * weights and activations travel through SEPARATE rings of bulk copies.  A weight slot is free again as soon as the unpack
 //     warps have read it (the unpacked copy lives in tensor memory), an activation slot when the MMAs that read it retire;
 //   * the MMA issuer is one warp whose every instruction counts: the tensor pipe queues about two MMAs, and what the issuer
@@ -20,7 +20,8 @@
 //   * eight dedicated epilogue warps read the accumulator out of tensor memory, hand it back after the last read and store
 //     straight from registers.  They read it as fragments of sixteen lanes x 256 bits, and the unpack warps choose which
 //     channel goes to which lane: a thread then holds four neighbouring channels of a token (SwiGLU: two features' gate and up
-//     values), so that nothing has to be exchanged between lanes but row maxima.
+//     values), so that nothing has to be exchanged between lanes but row maxima (and the sums of rows whose length does not
+//     allow four channels in one store).
 // Outputs: binary16 / fp32 / int32 [M,N], or the fused SwiGLU middle [M,F] fp32 (row maxima collected).
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
@@ -39,8 +40,6 @@ constexpr int PS_UNPACK_WARPS = 4 * PS_UNPACK_SETS;
 constexpr int PS_EPI_WARPS = 8;
 constexpr int PS_EPI_SETS = PS_EPI_WARPS / 4;  // per tensor-memory lane quarter, taking pieces of sixteen tokens in turn
 constexpr int PS_UNPACK_WARP0 = PS_ROLE_WARPS;
-constexpr int PS_EPI_WARP0 = PS_UNPACK_WARP0 + PS_UNPACK_WARPS;
-constexpr int PS_THREADS = 32 * (PS_EPI_WARP0 + PS_EPI_WARPS);   // 640
 constexpr int PS_TMEM_COLS = 512;
 constexpr int PS_SK = 2;                     // k-blocks of a stage
 constexpr unsigned long long PS_DRAIN_NS = 50000;
@@ -58,11 +57,14 @@ struct PsShape {
     static constexpr int XW = W8 ? XA : TOK == 64 ? 10 : TOK == 256 ? 6 : 8;     // weight ring
     static constexpr int ABUF = W8 ? 0 : TOK == 64 ? 6 : TOK == 256 ? 4 : 3;     // unpacked weight stages
     static constexpr int NR = XA > ABUF ? XA : ABUF;                             // barriers of stages ready for / done by the MMAs
+    static constexpr int EPI_WARP0 = PS_UNPACK_WARP0 + (W8 ? 0 : PS_UNPACK_WARPS);
+    static constexpr int THREADS = 32 * (EPI_WARP0 + PS_EPI_WARPS);              // 640; 384 where nothing is unpacked (1 to 2 % of a call of 24 us)
+    static constexpr int WB = W8 ? 0 : XW;                                       // weight slots with barriers of their own
     static constexpr int A_COL0 = ACC * TOK;
     static constexpr size_t XA_BYTES = PS_SK * (size_t)T * 128;
     static constexpr uint32_t GB = W8 ? 4096 : 2048;                             // one k-block of one 32-channel group
     static constexpr size_t XW_BYTES = PS_SK * 4 * (size_t)GB;
-    static constexpr int BARRIERS = XA + 2 * XW + 2 * NR + 2 * ACC;
+    static constexpr int BARRIERS = XA + 2 * WB + 2 * NR + 2 * ACC;
     static constexpr size_t SMEM = XA * XA_BYTES + XW * XW_BYTES + 2 * TOK * 4 + BARRIERS * 8 + 32;
     static_assert(TOK % 32 == 0 && TOK <= 256, "not the width of an MMA");
     static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
@@ -131,7 +133,7 @@ __device__ __forceinline__ void store_four_halves(__half* dst, uint32_t held01, 
 // (Linear and SwiGLU launches have kernels of their own: less to fetch, and neither finishing pays for the other's registers.)
 // W8: the weights are int8 codes in the W8 layout (w8a8_kernels.cu), and the sums are not scaled by 16.
 template <bool W8, bool SWIGLU, int TOK>
-__global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const GemmParams p, const __grid_constant__ PersistMaps maps, int num_clusters)
+__global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_kernel(const GemmParams p, const __grid_constant__ PersistMaps maps, int num_clusters)
 {
     using S = PsShape<W8, TOK>;
     constexpr uint32_t GB = S::GB;
@@ -142,8 +144,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
     uint32_t* const s_tilemax = reinterpret_cast<uint32_t*>(s_sx + TOK);         // SwiGLU: the CTA's row maxima of that item
     uint64_t* const xfull = reinterpret_cast<uint64_t*>(s_tilemax + TOK);        // W8: the weights of the stage as well
     uint64_t* const wfull = xfull + S::XA;
-    uint64_t* const wempty = wfull + S::XW;
-    uint64_t* const ready = wempty + S::XW;      // leader: both CTAs' operands of the stage are where the MMAs read them
+    uint64_t* const wempty = wfull + S::WB;
+    uint64_t* const ready = wempty + S::WB;      // leader: both CTAs' operands of the stage are where the MMAs read them
     uint64_t* const done = ready + S::NR;        // the stage's MMAs have retired: its operands may be overwritten
     uint64_t* const acc_full = done + S::NR;
     uint64_t* const acc_empty = acc_full + S::ACC;
@@ -186,7 +188,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
 
     if (tid == 0) {
         for (int s = 0; s < S::XA; ++s) mbar_init(&xfull[s], W8 ? 2 : 1);
-        for (int s = 0; s < S::XW; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 4); }
+        for (int s = 0; s < S::WB; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 4); }
         for (int b = 0; b < S::NR; ++b) { mbar_init(&ready[b], (W8 ? 0 : 8) + 2); mbar_init(&done[b], 1); }
         for (int b = 0; b < S::ACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * PS_EPI_WARPS); }   // every epilogue warp of both CTAs
         mbar_fence_init();
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
                 if (lane == 0) PS_STAMP(j, 2);
             }
         }
-    } else if (warp < PS_EPI_WARP0) {
+    } else if (warp < S::EPI_WARP0) {
         // ---------------------------------------------------------------- weight unpack -> TMEM
         if constexpr (!W8) {
         const int q = warp & 3;
@@ -470,8 +472,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1) gemm_tc_persist_kernel(const Ge
         // (Small ones are settled by the scales: a sum is zero, where the fast form is exact, or at least one.  Looking for
         // the smallest magnitude as well sent every fourth turn to the slow form, one sum in eight hundred being zero.)
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
-        const int eset = (warp - PS_EPI_WARP0) >> 2;   // takes pieces eset, eset + PS_EPI_SETS, ...
-        const int sid = (warp - PS_EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
+        const int eset = (warp - S::EPI_WARP0) >> 2;   // takes pieces eset, eset + PS_EPI_SETS, ...
+        const int sid = (warp - S::EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const int out_cols = swiglu ? p.F : p.N;
         // This thread's fragment: channels 4 i8 .. + 3 of its group (features 2 i8, + 1 of sixteen), the one in its c-th
@@ -797,7 +799,7 @@ cudaError_t launch_persist_inst(const GemmParams& p, cudaStream_t stream, bool p
     const bool setup = configured.needed(device);
     if (!setup) max_clusters = clusters_of_device[device];
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(PS_THREADS);
+    cfg.blockDim = dim3(S::THREADS);
     cfg.dynamicSmemBytes = S::SMEM;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
