@@ -2,6 +2,7 @@
 // of the kernel walks on the GPU, and the plan, made on the host once for a workspace.  Arithmetic on sizes; needs no CUDA.
 #pragma once
 #include <algorithm>
+#include <math.h>
 #include <stddef.h>
 #include <stdint.h>
 
@@ -118,86 +119,108 @@ inline void persist_stretches(unsigned begin, unsigned end, unsigned per_tile, V
     if (const unsigned tail = (end - begin) % per_tile) visit(0u, tail, 1u);
 }
 
-// The cheapest cut by a model of the kernel's time in cycles, fitted to every cut of 350 shapes (1 to 3000
-// tokens, K 1024 .. 11008, 2048 .. 28672 channels; linear, SwiGLU and int8-weight launches).  What it takes is within 0.6, 0.6
-// and 2.5 % of the best cut in the mean and within 9, 6 and 15 % at worst (64 x 8192 -> 2048 15.5 us where three parts of
-// 32-token tiles take 14.3):
-//   * a k-block of an item costs a constant (the issuer's and the unpack warps' chains) and something per token: 305 + 0.6 per
-//     token with four-byte-packed weights, of which the MMAs need two per token, so wide items pay; less where SMs are idle;
-//   * finishing an item is hidden behind the next one's MMAs (two accumulators) unless it takes longer;
+// The cheapest cut by a model of a call's time, fitted to every cut of 709 linears and 244 int8-weight calls (1 to 3000 tokens,
+// K 1024 .. 11008, 1024 .. 14336 channels; SwiGLU launches: an earlier fit, which 319 shapes bear out).  Only what cuts of one
+// shape differ by was fitted, so the constants are the fit's cycles, not the kernel's.  What it takes costs 0.5 to 0.9 % against
+// the best cut in the mean:
+//   * a k-block of an item costs a constant (the issuer's and the unpack warps' chains) and something per token, so wide items
+//     pay; less where SMs are idle, a little more in runs, whose pairs do not share weights;
+//   * finishing an item is hidden behind the next one's MMAs (two accumulators) unless it takes longer.  Rows whose length does
+//     not allow four channels in one store cost 9 % more of it per token (2 to 3 % of a call at a fixed cut; when they were priced
+//     at two and a half times, 512 x 4096 -> 4911 took 22.4 us for 20.0 and 2266 x 4032 -> 1285 26.9 for 24.5);
 //   * K in parts costs an exchange through L2: so much per part and pair, more for wide items;
-//   * a launch on more than half of the SMs leaves the one behind it no room to set itself up meanwhile.
+//   * a launch that leaves too few SMs free has the next call's quantise kernel wait for it, and its own set-up for that kernel: no
+//     cost up to `knee` of the pairs, counting `rows` of them per thousand tokens to quantise, all of it `ramp` further
+//     (109 x 4352 -> 4547 14.7 us on 72 pairs, 13.4 on 36).
 // A run is priced by its stretches of equal items, so that a plan takes the same few microseconds whatever the token count.
 struct PersistCosts {
-    double narrow, narrow_token, wide, wide_token, widest, widest_token;   // cycles of a k-block in each kernel
-    double finish, finish_token, item;               // of finishing an item, and between two items
+    double narrow, narrow_token, wide, wide_token, widest, widest_token;   // a k-block in each kernel
+    double finish, finish_token, ragged, item;       // finishing an item (per token so many times as much for ragged rows), and between two
     double part0, part, pair, part_wide;             // the exchange of parts
-    double crowded, idle;
+    double crowded, knee, ramp, rows;                // see above
+    double idle, runs;                               // of a k-block: less with idle pairs, so many times as much in runs
 };
-inline PersistPlan persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
+// Cycles a cut takes; `enough`: more than that need not be told exactly.  (columns and tokens whose units fit 31 bits)
+inline double persist_cut_cycles(const PersistCosts& cost, const PersistPlan& cut, int columns, int M, int KB, bool w8, int pairs, double enough)
 {
-    static const PersistCosts linear{270, 1.15, 305, 0.6, 339, 0.845, 2200, 31, 195, 870, 1590, 23, 0.65, 1530, 0.17};
-    static const PersistCosts gated{366, 0.79, 420, 0.37, 326, 1.0, 5060, 60, 670, 1500, 1380, 30, 0.7, 2030, 0.15};
-    static const PersistCosts bytes{323, 0.63, 380, 1.2, 380, 1.2, 2430, 32, 725, 1490, 1000, 21, 1.12, 720, 0.18};
-    const PersistCosts& cost = w8 ? bytes : swiglu ? gated : linear;
-    PersistPlan best{PERSIST_TOKENS, 1, 0, 1};
-    const int64_t channel_tiles = (int64_t(columns) + 255) / 256, tokens = (int64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS;
-    if (channel_tiles * (tokens / PERSIST_TOKENS) > INT32_MAX) return best;      // (its activations or results fit no GPU)
-    double best_time = 0;
-    const int pairs = std::max(1, sm_count / 2);
-    auto consider = [&](int unit, int most, int snap, int split) {
-        const unsigned per_tile = unsigned((tokens + unit - 1) / unit), units = unsigned(channel_tiles) * per_tile;
-        const int clusters = persist_clusters(int(units), split, pairs);
-        const double load = 1 - cost.idle * (1 - std::min(1.0, double(clusters) / pairs));
-        const bool narrow = unit * most <= PS_NARROW, wide = unit * most <= PS_WIDE, hidden = w8 || wide;
-        auto block = [&](double width) {
-            return load * (narrow ? cost.narrow + cost.narrow_token * width : wide ? cost.wide + cost.wide_token * width : cost.widest + cost.widest_token * width);
-        };
-        auto finish = [&](double width) { return cost.finish + cost.finish_token * (columns % 4 ? 2.5 : 1) * width; };   // (narrower stores)
-        auto run = [&](unsigned begin, unsigned end) {
-            double time = 0, last = 0;                       // `last`: finishing the item in front, not paid for yet
-            auto alike = [&](double width, unsigned n) {
-                const double mmas = KB * block(width) + cost.item, then = finish(width);
-                time += hidden ? std::max(mmas, last) : mmas + last;
-                time += (n - 1) * (hidden ? std::max(mmas, then) : mmas + then);
-                last = then;
-            };
-            persist_stretches(begin, end, per_tile, [&](unsigned first, unsigned len, unsigned tiles) {
-                const bool cut = first + len == per_tile && int64_t(per_tile) * unit > tokens;    // (items of one unit then)
-                auto tile = [&] {
-                    persist_widths(len, most, [&](unsigned n_units, unsigned n) {
-                        if (n > cut) alike(double(n_units) * unit, n - cut);
-                        if (cut) alike(double(tokens - int64_t(per_tile - 1) * unit), 1);
-                    });
-                };
-                tile();
-                if (tiles == 1) return;
-                const double so_far = time;
-                tile();
-                time += (tiles - 2) * (time - so_far);
-            });
-            return time + last;
-        };
-        const PersistShare dealt = persist_share(units, unsigned(clusters));
-        double longest = 0;
-        if (split > 1) {
-            const double width = double(std::min<int64_t>(unit, tokens));
-            longest = KB * block(width) / split + finish(width) +
-                      (cost.part0 + cost.part * (split - 1) + cost.pair * clusters) * (1 + cost.part_wide * std::max(0.0, width - 64) / 64.0);
-        } else
-            for (int i = 0; i < clusters && (best_time == 0 || longest < best_time); ++i)   // (no better than the best: given up)
-                longest = std::max(longest, run(persist_bound(dealt, per_tile, snap, i), persist_bound(dealt, per_tile, snap, i + 1)));
-        if (2 * clusters > pairs) longest += cost.crowded;
-        if (best_time == 0 || longest < best_time) { best_time = longest; best = {unit, most, snap, split}; }
+    const int unit = cut.unit, most = cut.most, split = cut.split;
+    const int64_t tokens = (int64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS;
+    const unsigned per_tile = unsigned((tokens + unit - 1) / unit), units = unsigned((int64_t(columns) + 255) / 256) * per_tile;
+    const int clusters = persist_clusters(int(units), split, pairs);
+    const double busy = std::min(1.0, double(clusters) / pairs), load = (1 - cost.idle * (1 - busy)) * (most > 1 ? cost.runs : 1);
+    const bool narrow = unit * most <= PS_NARROW, wide = unit * most <= PS_WIDE, hidden = w8 || wide;
+    auto block = [&](double width) {
+        return load * (narrow ? cost.narrow + cost.narrow_token * width : wide ? cost.wide + cost.wide_token * width : cost.widest + cost.widest_token * width);
     };
+    auto finish = [&](double width) { return cost.finish + cost.finish_token * (columns % 4 ? cost.ragged : 1) * width; };
+    auto run = [&](unsigned begin, unsigned end) {
+        double time = 0, last = 0;                       // `last`: finishing the item in front, not paid for yet
+        auto alike = [&](double width, unsigned n) {
+            const double mmas = KB * block(width) + cost.item, then = finish(width);
+            time += hidden ? std::max(mmas, last) : mmas + last;
+            time += (n - 1) * (hidden ? std::max(mmas, then) : mmas + then);
+            last = then;
+        };
+        persist_stretches(begin, end, per_tile, [&](unsigned first, unsigned len, unsigned tiles) {
+            const bool short_end = first + len == per_tile && int64_t(per_tile) * unit > tokens;    // (items of one unit then)
+            auto tile = [&] {
+                persist_widths(len, most, [&](unsigned n_units, unsigned n) {
+                    if (n > short_end) alike(double(n_units) * unit, n - short_end);
+                    if (short_end) alike(double(tokens - int64_t(per_tile - 1) * unit), 1);
+                });
+            };
+            tile();
+            if (tiles == 1) return;
+            const double so_far = time;
+            tile();
+            time += (tiles - 2) * (time - so_far);
+        });
+        return time + last;
+    };
+    double longest = 0;
+    if (split > 1) {
+        const double width = double(std::min<int64_t>(unit, tokens));
+        longest = KB * block(width) / split + finish(width) +
+                  (cost.part0 + cost.part * (split - 1) + cost.pair * clusters) * (1 + cost.part_wide * std::max(0.0, width - 64) / 64.0);
+    } else {
+        const PersistShare dealt = persist_share(units, unsigned(clusters));
+        for (int i = 0; i < clusters && longest < enough; ++i)
+            longest = std::max(longest, run(persist_bound(dealt, per_tile, cut.snap, i), persist_bound(dealt, per_tile, cut.snap, i + 1)));
+    }
+    return longest + cost.crowded * std::min(1.0, std::max(0.0, (busy + cost.rows * M / 1000 - cost.knee) / cost.ramp));
+}
+inline const PersistCosts& persist_costs(bool w8, bool swiglu)
+{
+    static const PersistCosts linear{349, 2.48, 415, 1.53, 351, 2.15, 3000, 41.1, 1.09, 138, 1860, 1640, 8.33, 1.38, 2340, 0.569, 0.0642, 0.314, 0.316, 1.02};
+    static const PersistCosts gated{366, 0.79, 420, 0.37, 326, 1.0, 5060, 60, 2.5, 670, 1500, 1380, 30, 0.7, 2030, 0.5, 0.01, 0, 0.15, 1};
+    static const PersistCosts bytes{355, 2.58, 506, 1.75, 474, 2.08, 5070, 52, 1.75, 709, 4210, 1510, 16.3, 0.976, 989, 0.782, 0.121, 0.0751, 0.107, 1};
+    return w8 ? bytes : swiglu ? gated : linear;
+}
+// Every cut that is considered: visit(cut).
+template <class Visit>
+inline void persist_cuts(int columns, int M, int KB, int pairs, Visit visit)
+{
+    const int64_t channel_tiles = (int64_t(columns) + 255) / 256, tokens = (int64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS;
     const int widest = int(std::min<int64_t>(PS_WIDEST, tokens));
     for (int unit = PERSIST_TOKENS; unit <= widest; unit += PERSIST_TOKENS)       // items of one width, K in parts or not
         for (const int split : {1, 2, 3, 4, 6, 8}) {
             if (split > 1 && (unit > PS_WIDE || channel_tiles * ((tokens + unit - 1) / unit) * split > pairs || KB < 4 * split)) break;
-            consider(unit, 1, 0, split);
+            visit(PersistPlan{unit, 1, 0, split});
         }
     for (int most = 2; most <= widest / PERSIST_TOKENS; ++most)                  // equal runs
-        for (const int snap : {0, 2, 3}) consider(PERSIST_TOKENS, most, snap, 1);
+        for (const int snap : {0, 2, 3}) visit(PersistPlan{PERSIST_TOKENS, most, snap, 1});
+}
+inline PersistPlan persist_plan(int columns, int M, int KB, bool w8, bool swiglu, int sm_count)
+{
+    PersistPlan best{PERSIST_TOKENS, 1, 0, 1};
+    if ((int64_t(columns) + 255) / 256 * ((int64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS) > INT32_MAX) return best;   // (its activations or results fit no GPU)
+    const PersistCosts& cost = persist_costs(w8, swiglu);
+    const int pairs = std::max(1, sm_count / 2);
+    double best_cycles = HUGE_VAL;
+    persist_cuts(columns, M, KB, pairs, [&](const PersistPlan& cut) {
+        const double cycles = persist_cut_cycles(cost, cut, columns, M, KB, w8, pairs, best_cycles);
+        if (cycles < best_cycles) { best_cycles = cycles; best = cut; }
+    });
     return best;
 }
 
