@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(256) w8_pack_weights_kernel(const W8PackParams
             if (k < p.K) word |= (uint32_t)(uint8_t)p.B[(size_t)k * p.N + n] << (8 * b);
         }
     }
-        const int row = 8 * (r & 3) + (r >> 2);
+    const int row = 8 * (r & 3) + (r >> 2);
     reinterpret_cast<uint32_t*>(p.Wp)[((((size_t)(g >> 2) * p.KB * 8 + c) * 4 + (g & 3)) * GROUP + row) * 4 + j] = word;
 }
 
