@@ -126,7 +126,7 @@ int contract(rk_npu_i4_workspace* ws, const rk_npu_i4i4i32_weights* w, const int
     g.sx = ws->scales;
     g.sw = w->ones;
     g.out = dC;
-    g.status = ws->status;
+    g.status = g.report = ws->status;
     g.M = cfg.M; g.N = cfg.N; g.K = cfg.K;
     g.KB = ws->KB; g.NG = w->NG; g.T = PERSIST_T;
     g.epi = EPI_I32;

@@ -461,7 +461,6 @@ int enqueue(const Call& c)
     q.rowmax_zero = nullptr;
     q.rowmax = c.rowmax_in;
     q.status = ws.status;
-    q.host_flag = c.status ? &c.status->bad_input : nullptr;
     q.M = cfg.M;
     q.K = cfg.K;
     q.Kp = ws.KB * KBLOCK;
@@ -479,7 +478,7 @@ int enqueue(const Call& c)
     g.out = c.dOut;
     g.rowmax = c.rowmax_out;
     g.status = ws.status;
-    g.report = c.status ? &c.status->device_error : nullptr;
+    g.report = c.status ? c.status : ws.status;
     g.M = cfg.M;
     g.N = N;
     g.K = cfg.K;

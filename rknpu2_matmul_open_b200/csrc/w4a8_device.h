@@ -54,8 +54,8 @@ enum Epilogue : int { EPI_F32 = 0, EPI_F16 = 1, EPI_I32 = 2, EPI_SWIGLU = 3 };
 
 // Device-side status block of a workspace (all int32).
 struct Status {
-    int bad_input;      // set by the quantise kernel: 1 = NaN/Inf activation, 2 = non-finite middle
-    int bad_accum;      // scratch for the cross-CTA "any row bad" reduction
+    int bad_input;      // verdict of the last call: 1 = NaN/Inf activation, 2 = non-finite middle
+    int bad_accum;      // set by a quantise kernel, taken by the GEMM behind it (take_verdict); zero between calls
     unsigned done;      // scratch counter (wraps to 0 by itself)
     int device_error;   // 1 = a bounded wait inside a kernel ran out
 };
@@ -66,12 +66,11 @@ struct QuantParams {
     float* scales;          // [M]
     float* inverse;         // [M]
     // [M] cleared as well, for a SwiGLU epilogue that maxes into it; NULL: every caller's epilogue finds its maxima cleared by
-    // their consumer.  (Without this store the compiler spills 20 to 28 bytes in the fp32 forms that are held to 32 registers:
+    // their consumer.  (Without this store the compiler spills more bytes in the fp32 form that is held to 32 registers:
     // FFN of 1163 x 2816 -> 2 x 4096 72.2 -> 73.5 us, 1616 rows of 3735 115 -> 119.)
     uint32_t* rowmax_zero;
     uint32_t* rowmax;       // [M] non-null: scales come from these magnitude bits (no scan); cleared after use
     Status* status;
-    int* host_flag;         // mapped host word mirroring status->bad_input (nullable)
     int M, K, Kp, T;
     int half;
 };
@@ -97,10 +96,29 @@ struct CodesInParams {
 };
 
 // A bounded wait ran out (a plain store: the word may be page-locked host memory).
-__device__ __forceinline__ void report_device_error(Status* status, int* report)
+__device__ __forceinline__ void report_device_error(Status* report) { *reinterpret_cast<volatile int*>(&report->device_error) = 1; }
+
+#ifdef __CUDACC__
+// Verdict of the quantise launch in front, behind the dependency wait: called once by one thread of every CTA of the launch.
+// A quantise CTA that meets a bad row sets bad_accum and nothing else.  The last CTA to have seen it set publishes it and
+// clears the word for the next call; a good call publishes a zero.  (When the quantise CTA that drew the last ticket published
+// the verdict, the launch ended behind its ticket, a fence and an exchange, 1.5 to 4 us later than the other CTAs, and the GEMM
+// asked for its activations behind a look at the verdict: 24 x 4096 -> 4096 11.5 -> 10.2 us, 12 x 11008 -> 4096 13.0 -> 11.4,
+// 64 x 4096 -> 11008 fp32 13.2 -> 12.0.)
+__device__ __forceinline__ int take_verdict(Status* status, Status* report)
 {
-    *reinterpret_cast<volatile int*>(report ? report : &status->device_error) = 1;
+    const int bad = *reinterpret_cast<volatile const int*>(&status->bad_accum);
+    const unsigned ctas = gridDim.x * gridDim.y * gridDim.z;
+    if (bad) {
+        __threadfence();
+        if (atomicInc(&status->done, ctas - 1u) == ctas - 1u) {
+            *reinterpret_cast<volatile int*>(&status->bad_accum) = 0;
+            *reinterpret_cast<volatile int*>(&report->bad_input) = bad;
+        }
+    } else if (report == status && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) report->bad_input = 0;
+    return bad;
 }
+#endif
 
 // Tensor maps of a persistent kernel's activation codes [groups of eight tokens][K bytes x 8]: boxes of two k-blocks of eight,
 // four and two groups.  Made once for a workspace's code buffer.
@@ -116,7 +134,7 @@ struct GemmParams {
     void* out;              // [M,N] fp32 / fp16 / int32, or middle [M,F] fp32
     uint32_t* rowmax;       // SwiGLU: per-row max |middle| bit pattern (nullable)
     Status* status;
-    int* report;            // where a wait that ran out is recorded: a word of page-locked host memory, or NULL for status->device_error
+    Status* report;         // where the verdict and a wait that ran out are recorded: the same block, or one in page-locked host memory that the host has cleared
     int M, N, K;
     int KB;                 // k-blocks (Kp / 128)
     int NG;                 // weight groups (padded)

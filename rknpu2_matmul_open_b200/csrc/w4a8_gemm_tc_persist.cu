@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
     uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(acc_empty + S::ACC);
     int* const s_error = reinterpret_cast<int*>(s_tmem + 1);
     int* const s_finish = s_error + 1;           // this CTA completed the tile whose partial sums it just stored
+    int* const s_verdict = s_finish + 1;         // the quantiser rejected the input: nothing is to be written
 
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -208,30 +209,23 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
     const uint32_t tmem_base = *s_tmem;
 
     // What does not depend on the kernel in front -- requesting weights, unpacking the first of them into tensor
-    // memory -- starts before the dependency wait; every other warp waits here.
-    auto dependency_met = [&]() -> bool {   // false: the quantiser rejected the input, nothing is to be written
-        pdl_wait();
-        return *reinterpret_cast<volatile const int*>(&p.status->bad_input) == 0;
-    };
+    // memory -- starts before the dependency wait.  Where the quantiser rejected the input the contraction runs all the same
+    // and the epilogue drops its sums: whoever loads activations need not wait for the verdict (a trip to L2).
 
     if (warp == 2) {
         // ---------------------------------------------------------------- weight producer
         // (the whole warp walks the loop and one elected lane issues, as in the MMA issuer below: copy requests take their
         // operands from uniform registers, and four lanes issuing one request each took 1000 cycles per stage)
         RingPos<S::XW> r;
-        bool ok = true, live = true, asked = false;
+        bool ok = true;
         int g = 0;
         const size_t group_bytes = (size_t)KB * GB;
         const size_t upper = swiglu ? (size_t)(p.F / GROUP) * group_bytes : 2 * group_bytes;   // groups 2, 3 behind groups 0, 1
-        while (live && ok && next_item(item)) {
+        while (ok && next_item(item)) {
             const int ct = 2 * item.tile + (int)rank;
             const uint8_t* src = p.Wp + (size_t)(swiglu ? ct * 2 : ct * 4) * group_bytes + (size_t)it0 * (W8 ? 4 : 1) * PS_SK * GB;
             for (int it = it0; it < it1; ++it, ++g, r.next()) {
-                if (g == S::XW) {
-                    live = dependency_met();
-                    asked = true;
-                    if (!live) break;
-                }
+                if (g == S::XW) pdl_wait();                    // (slots come back once the MMAs have activations)
                 const uint32_t bytes = (uint32_t)min(PS_SK, KB - PS_SK * it) * GB;
                 if (g >= S::XW) ok = __all_sync(0xffffffffu, W8 ? mbar_wait_cluster(&done[r.slot], r.phase ^ 1u, deadline) : mbar_wait(&wempty[r.slot], r.phase ^ 1u, deadline));
                 if (!ok) { *s_error = 1; break; }
@@ -252,52 +246,41 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 src += (W8 ? 4 : 1) * PS_SK * GB;
             }
         }
-        if (!asked) live = dependency_met();
-        if (!live && !W8 && lane == 0)   // nobody will consume: let the copies already requested land before leaving
-            for (int s = 0; s < min(g, S::XW); ++s)
-                if (!mbar_wait(&wfull[s], 0, deadline)) { *s_error = 1; break; }
-        if (!live && W8) {               // (their barriers wait for the activations' half as well, which does not come)
-            if (lane == 0)
-                for (int s = 0; s < min(g, S::XW); ++s) {
-                    mbar_arrive(&xfull[s]);
-                    if (!mbar_wait(&xfull[s], 0, deadline)) { *s_error = 1; break; }
-                }
-        }
     } else if (warp == 0) {
         // ---------------------------------------------------------------- activation producer
-        if (dependency_met()) {
-            RingPos<S::XA> r;
-            bool ok = true;
-            int g = 0;
-            while (ok && next_item(item)) {
-                const int groups = item.width / 16;            // of this CTA's half
-                const int row0 = item.tok0 / 8 + (int)rank * groups;
-                for (int it = it0; it < it1; ++it, ++g, r.next()) {
-                    if (g >= S::XA) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&done[(g - S::XA) % S::NR], (g - S::XA) / S::NR & 1, deadline));
-                    if (!ok) { *s_error = 1; break; }
-                    if (elect_one()) {
-                        // (a stage's second k-block that does not exist is filled with zeros)
-                        mbar_arrive_expect_tx(&xfull[r.slot], (uint32_t)groups * (PS_SK * 1024u));
-                        uint8_t* dst = acts + (size_t)r.slot * S::XA_BYTES;
-                        int row = row0, left = groups;
-                        for (; left >= 8; left -= 8, row += 8, dst += 8 * PS_SK * 1024) tensor_g2s(dst, &maps.box[0], it * PS_SK * 128, row, &xfull[r.slot]);
-                        if (left & 4) { tensor_g2s(dst, &maps.box[1], it * PS_SK * 128, row, &xfull[r.slot]); row += 4; dst += 4 * PS_SK * 1024; }
-                        if (left & 2) tensor_g2s(dst, &maps.box[2], it * PS_SK * 128, row, &xfull[r.slot]);
-                    }
-                    __syncwarp();
+        pdl_wait();
+        RingPos<S::XA> r;
+        bool ok = true;
+        int g = 0;
+        while (ok && next_item(item)) {
+            const int groups = item.width / 16;            // of this CTA's half
+            const int row0 = item.tok0 / 8 + (int)rank * groups;
+            for (int it = it0; it < it1; ++it, ++g, r.next()) {
+                if (g >= S::XA) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&done[(g - S::XA) % S::NR], (g - S::XA) / S::NR & 1, deadline));
+                if (!ok) { *s_error = 1; break; }
+                if (elect_one()) {
+                    // (a stage's second k-block that does not exist is filled with zeros)
+                    mbar_arrive_expect_tx(&xfull[r.slot], (uint32_t)groups * (PS_SK * 1024u));
+                    uint8_t* dst = acts + (size_t)r.slot * S::XA_BYTES;
+                    int row = row0, left = groups;
+                    for (; left >= 8; left -= 8, row += 8, dst += 8 * PS_SK * 1024) tensor_g2s(dst, &maps.box[0], it * PS_SK * 128, row, &xfull[r.slot]);
+                    if (left & 4) { tensor_g2s(dst, &maps.box[1], it * PS_SK * 128, row, &xfull[r.slot]); row += 4; dst += 4 * PS_SK * 1024; }
+                    if (left & 2) tensor_g2s(dst, &maps.box[2], it * PS_SK * 128, row, &xfull[r.slot]);
                 }
+                __syncwarp();
             }
-            // The MMAs' commits arrive on this CTA's barriers asynchronously, the peer's among them: the CTA may not leave
-            // (and its shared memory change hands) before the last of them is here.
-            for (int k = max(0, g - S::XA); k < g && !*reinterpret_cast<volatile int*>(s_error); ++k)
-                if (!mbar_wait_cluster(&done[k % S::NR], k / S::NR & 1, deadline)) *s_error = 1;
         }
+        // The MMAs' commits arrive on this CTA's barriers asynchronously, the peer's among them: the CTA may not leave
+        // (and its shared memory change hands) before the last of them is here.
+        for (int k = max(0, g - S::XA); k < g && !*reinterpret_cast<volatile int*>(s_error); ++k)
+            if (!mbar_wait_cluster(&done[k % S::NR], k / S::NR & 1, deadline)) *s_error = 1;
     } else if (warp == 3) {
         // ---------------------------------------------------------------- voucher
         // The leader's MMAs read both CTAs' shared memory: this warp passes on that this CTA's copies have landed.  It runs
         // ahead of the MMAs by the depth of the ring.  (When the unpack warps vouched for it, with an arrival that released
         // everything at cluster scope, that release bounded the whole loop: 730 cycles per k-block at K = 11008 against 525.)
-        if (dependency_met() && lane == 0) {
+        pdl_wait();
+        if (lane == 0) {
             RingPos<S::XA> r;
             RingPos<S::NR> to;
             long long waited = 0;
@@ -318,7 +301,8 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         // issues.  (A loop that only lane 0 enters moves every operand of every MMA into uniform registers first: 85
         // cycles per MMA.)  Everything a stage needs is known before the one in front is issued; what stands between two
         // stages' MMAs is one wait, one commit and a few additions.
-        if (dependency_met() && rank == 0) {
+        pdl_wait();
+        if (rank == 0) {
             bool dead = false;                                     // (the elected lane's, always the same one)
             RingPos<S::ACC> rc;
             const uint32_t ready0 = smem_u32(ready), done0 = smem_u32(done);
@@ -422,7 +406,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             const int kbs = min(PS_SK, KB - PS_SK * it), b = g % S::ABUF;
             const bool reuse = g >= S::ABUF;
             // (before the first buffer comes back from the MMAs, which need the activations)
-            if (reuse && g - PS_UNPACK_SETS < S::ABUF && !dependency_met()) break;
+            if (reuse && g - PS_UNPACK_SETS < S::ABUF) pdl_wait();
             const long long w0 = tr ? clock64() : 0;
             if (reuse) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&done[(g - S::ABUF) % S::NR], (g - S::ABUF) / S::NR & 1, deadline));
             if (tr) wait_free += clock64() - w0;
@@ -491,7 +475,9 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         const bool fragments = swiglu || wide_ok;
         constexpr int STEP = 16 * PS_EPI_SETS;
         constexpr int SHIFT = W8 ? 0 : 4;              // int4 records enter the MMA times 16
-        bool ok = dependency_met();
+        pdl_wait();
+        if (!W8 && sid == 0) *s_verdict = take_verdict(p.status, p.report);
+        bool ok = true, good = true;
         RingPos<S::ACC> rc;
         for (int j = 0; ok && next_item(item); ++j, rc.next()) {
             const int ct = 2 * item.tile + (int)rank;
@@ -506,7 +492,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             }
             // pieces of sixteen tokens of this warp that hold live tokens: those at 16 eset + STEP k, k < pieces
             const int live = min(item.width, p.M - tok_base);
-            const int pieces = max(0, (live - 16 * eset + STEP - 1) / STEP);
+            int pieces = max(0, (live - 16 * eset + STEP - 1) / STEP);
             // Token scales, staged with the int4 records' 1/16 in them: (float)(16 s) * (sx / 16) is (float)s * sx, exactly,
             // unless sx / 16 is subnormal.  (The barrier at the end of an item keeps stragglers out.)
             float sx_here = 0.f;
@@ -524,8 +510,9 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             }
             // SwiGLU: no gate value of this thread is too small for the fast SiLU, whatever the sums are (zero is not)
             const bool gates_ok = swiglu && !low && (n0 >= out_cols || (sw[0] >= PS_LOW && sw[1] >= PS_LOW));
-            ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // one verdict for all eight warps
+            ok = epilogue_all(mbar_wait_cluster(&acc_full[rc.slot], rc.phase, deadline));   // all eight warps or none
             if (!ok) { *s_error = 1; break; }
+            if constexpr (!W8) good = *reinterpret_cast<volatile const int*>(s_verdict) == 0;
             if (sid == 0) PS_STAMP(j, 3);
             tc_fence_after();
             const uint32_t acc_addr = lane_addr + rc.slot * TOK + 16 * eset;
@@ -550,7 +537,8 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             const size_t slot_quads = 32 * (size_t)p.unit, part_stride = 2 * slot_quads;
             const int4* const slots = reinterpret_cast<const int4*>(p.partials) + (2 * split * tile_index + rank) * slot_quads + (size_t)(4 * eset) * 128 + q * 32 + lane;
             bool finish = true;
-            if (split > 1) {
+            if (!W8 && !good) pieces = 0;                  // a rejected input: the sums are dropped
+            else if (split > 1) {
                 int4* const slot = const_cast<int4*>(slots) + part * part_stride;
 #pragma unroll 1
                 for (int k = 0; k < pieces; ++k) {
@@ -583,7 +571,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 for (int h = 0; h < 4; ++h) v[h] = __ldcg(src + (size_t)h * 128);
             };
             if (split > 1 && turns) fetch_part(ahead, other, 0);
-            if (split == 1 && pieces == 0) hand_back();
+            if (pieces == 0 && (split == 1 || !good)) hand_back();
 #pragma unroll 1
             for (int k = 0; k < turns; ++k) {
                 const int t0 = 16 * eset + STEP * k + 2 * tq;             // this thread's first token of the turn
@@ -756,7 +744,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             }
             if (sid == 0) PS_STAMP(j, 5);
             asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");   // every epilogue warp is done with this item's scales and maxima
-            if (swiglu && p.rowmax && sid < TOK) {
+            if (swiglu && good && p.rowmax && sid < TOK) {
                 const uint32_t m = s_tilemax[sid];
                 if (m) {
                     atomicMax(&p.rowmax[tok_base + sid], m);
@@ -775,7 +763,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         for (const unsigned long long until = global_ns() + PS_DRAIN_NS; global_ns() < until;) __nanosleep(1000);
     cluster_arrive();
     cluster_wait();   // neither CTA frees tensor memory or leaves while the other may still use it
-    if (tid == 0 && *s_error) report_device_error(p.status, p.report);
+    if (tid == 0 && *s_error) report_device_error(p.report);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PS_TMEM_COLS) : "memory");

@@ -69,8 +69,6 @@ cudaError_t launch_pack_weights(const PackParams& p, cudaStream_t stream)
 template <bool HALF>
 struct RowQuant {
     const QuantParams& p;
-    int bad = 0;                 // of the tokens this thread began
-    unsigned ticket = 0;
     static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r)
     {
         if constexpr (HALF) {
@@ -87,6 +85,7 @@ struct RowQuant {
             p.rowmax[m] = 0u;    // consumed: the next SwiGLU epilogue maxes into a clean word
         }
         float maximum;
+        int bad;
         if (HALF && !p.rowmax) {
             bad = bits >= 0x7c00u ? 1 : 0;
             maximum = __half2float(__ushort_as_half((uint16_t)bits));
@@ -99,25 +98,12 @@ struct RowQuant {
         p.scales[m] = s;
         p.inverse[m] = inv;
         if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
-        // "any row bad" without a reset pass, see finish(): the ticket is drawn here, its answer is needed at the end
-        if (bad) { atomicOr(&p.status->bad_accum, bad); __threadfence(); }
-        ticket = atomicInc(&p.status->done, (unsigned)p.M - 1u);
+        if (bad) p.status->bad_accum = bad;     // (the same value from every bad row of a launch)
         return inv;
     }
     __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
     {
         return quantize4(__fmul_rn(a, inv), __fmul_rn(b, inv), __fmul_rn(c, inv), __fmul_rn(d, inv));
-    }
-    // the last token to have drawn its ticket publishes the accumulated verdict and clears the scratch word; the counter
-    // wraps to zero by itself (atomicInc with limit M - 1)
-    __device__ __forceinline__ void finish(bool began)
-    {
-        if (began && ticket == (unsigned)p.M - 1u) {
-            __threadfence();
-            const int any = atomicExch(&p.status->bad_accum, 0);
-            p.status->bad_input = any;
-            if (p.host_flag) *p.host_flag = any;
-        }
     }
 };
 template <bool HALF, int TG, bool SCAN, int BS, int UN>
@@ -127,7 +113,6 @@ __global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) quantize_row
     pdl_wait();                // A may be the output of the kernel in front of this one
     RowQuant<HALF> op{p};
     quantize_rows<HALF, TG, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, op);
-    op.finish(threadIdx.x < TG && (int)(blockIdx.x * TG + threadIdx.x) < p.M);
 }
 
 // Any row: one CTA per token.
@@ -145,7 +130,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
     __shared__ uint32_t s_words[BS / 32][PIECE_WORDS];
     __shared__ uint32_t s_part[BS / 32];
     __shared__ float s_inverse;
-    __shared__ int s_bad;
 
     uint32_t maxbits = 0;
     int bad = 0;
@@ -177,7 +161,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
             p.scales[m] = s;
             p.inverse[m] = inv;
             s_inverse = inv;
-            s_bad = bad;
         }
     } else if (tid == 0) {
         const uint32_t bits = p.rowmax[m];
@@ -189,7 +172,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
         p.scales[m] = s;
         p.inverse[m] = inv;
         s_inverse = inv;
-        s_bad = bad;
     }
     __syncthreads();
     const float inv = s_inverse;
@@ -203,28 +185,9 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
         const int kc = u + lane;
         if (kc < chunks) dst[(size_t)kc * p.T] = kc * 16 < p.K ? quantize16(v, inv, kc * 16, p.K) : make_uint4(0u, 0u, 0u, 0u);
     }
-    // Cross-CTA bookkeeping last, so that the other 255 threads of the CTA never wait for its
-    // round trips to L2.
     if (tid == 0) {
         if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
-        // "Any row bad" across CTAs without a reset pass: the last CTA to arrive
-        // publishes the accumulated flag and clears the scratch word; the counter
-        // wraps to zero by itself (atomicInc with limit M-1).
-        if (gridDim.x == 1) {
-            // a single row: its verdict is the verdict, no round trips through L2 before the kernel can end
-            p.status->bad_input = bad;
-            if (p.host_flag) *p.host_flag = bad;
-        } else {
-            if (bad) atomicOr(&p.status->bad_accum, bad);
-            __threadfence();
-            const unsigned prev = atomicInc(&p.status->done, (unsigned)p.M - 1u);
-            if (prev == (unsigned)p.M - 1u) {
-                __threadfence();
-                const int any = atomicExch(&p.status->bad_accum, 0);
-                p.status->bad_input = any;
-                if (p.host_flag) *p.host_flag = any;
-            }
-        }
+        if (bad) p.status->bad_accum = bad;     // (the same value from every bad row of a launch)
     }
 }
 
@@ -288,6 +251,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
     int32_t* const red = reinterpret_cast<int32_t*>(smem + MMA_STAGES * STAGE);
     uint64_t* const full = reinterpret_cast<uint64_t*>(smem + MMA_STAGES * STAGE + TC * RED_STRIDE * 4);
     uint64_t* const empty = full + MMA_STAGES;
+    __shared__ int s_verdict;
 
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -354,38 +318,32 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
             // for the kernel in front (which produces the activation codes).
             for (int it = 0; it < pre; ++it) { mbar_expect_tx(&full[it], 8192); copy_w(it, it); }
             pdl_wait();
-            const bool skip = *reinterpret_cast<volatile const int*>(&p.status->bad_input) != 0;
-            for (int it = 0; it < pre; ++it) {
-                if (skip) { mbar_arrive(&full[it]); }
-                else { mbar_arrive_expect_tx(&full[it], XB); copy_x(it, it); }
-            }
-            if (!skip) {
-                for (int it = pre; it < nkb; ++it) {
-                    const int s = it % MMA_STAGES;
-                    if (!mbar_wait(&empty[s], ((it / MMA_STAGES) - 1) & 1, deadline)) {
-                        report_device_error(p.status, p.report);
-                        break;
-                    }
-                    mbar_arrive_expect_tx(&full[s], STAGE);
-                    copy_w(it, s);
-                    copy_x(it, s);
+            for (int it = 0; it < pre; ++it) { mbar_arrive_expect_tx(&full[it], XB); copy_x(it, it); }
+            for (int it = pre; it < nkb; ++it) {
+                const int s = it % MMA_STAGES;
+                if (!mbar_wait(&empty[s], ((it / MMA_STAGES) - 1) & 1, deadline)) {
+                    report_device_error(p.report);
+                    break;
                 }
+                mbar_arrive_expect_tx(&full[s], STAGE);
+                copy_w(it, s);
+                copy_x(it, s);
             }
         }
         __syncwarp();
     } else {
         // ---------------- consumers: warp w owns weight group w (32 channels = two m16 tiles)
         pdl_wait();
-        const bool skip = *reinterpret_cast<volatile const int*>(&p.status->bad_input) != 0;
-        const int iters = skip ? (nkb < MMA_STAGES ? nkb : MMA_STAGES) : nkb;
+        // (the contraction does not wait for the verdict: only the results depend on it)
+        if (tid == 0) s_verdict = take_verdict(p.status, p.report);
         const int g8 = lane >> 2, t4 = lane & 3;
-        for (int it = 0; it < iters; ++it) {
+        for (int it = 0; it < nkb; ++it) {
             const int s = it % MMA_STAGES;
             if (!mbar_wait(&full[s], (it / MMA_STAGES) & 1, deadline)) {
-                if (lane == 0) report_device_error(p.status, p.report);
+                if (lane == 0) report_device_error(p.report);
                 break;
             }
-            if (!skip) {
+            {
                 const uint32_t wbase = smem_u32(stages + (size_t)s * STAGE + warp * 2048) + g8 * 16 + t4 * 4;
                 const uint32_t xbase = smem_u32(stages + (size_t)s * STAGE + 8192) + g8 * 16 + t4 * 4;
 #pragma unroll
@@ -441,8 +399,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
     cg::cluster_group cluster = cg::this_cluster();
     if (S > 1) cluster.sync();
 
-    const bool skip_out = *reinterpret_cast<volatile const int*>(&p.status->bad_input) != 0;
-    if (tid < 128 && !skip_out) {
+    if (tid < 128 && !s_verdict) {
         const int CH = (swiglu ? 64 : 128) / S;       // channels (gate channels) this rank finishes
         const int IPT = CH / 4;                       // 4-channel items per token
         const int items = TC * IPT;
@@ -693,7 +650,7 @@ extern "C" int rk_npu_b200_w4a8_enqueue_f16_static(const rk_npu_w4a8_weights* we
     g.sx = scales;
     g.sw = weights->scales;
     g.out = dC;
-    g.status = status;
+    g.status = g.report = status;
     g.M = M;
     g.N = N;
     g.K = K;

@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_tc_stream_kernel(const Gem
     uint64_t* const acc_empty = acc_full + 2;
     uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* const s_flag = reinterpret_cast<int*>(s_tmem + 1);   // [0] this CTA completed the tile, [1] a wait ran out
+    __shared__ int s_verdict;
 
     pdl_launch_dependents();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -126,7 +127,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_tc_stream_kernel(const Gem
         }
     }
     pdl_wait();       // activation codes, scales and the status word come from the kernel in front
-    const bool skip = *reinterpret_cast<volatile const int*>(&p.status->bad_input) != 0;
+    if (tid == 0) s_verdict = take_verdict(p.status, p.report);
+    __syncthreads();
+    const bool skip = s_verdict != 0;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer, part 2
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_tc_stream_kernel(const Gem
     // ------------------------------------------------------------------------ teardown
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && s_flag[1]) report_device_error(p.status, p.report);
+    if (tid == 0 && s_flag[1]) report_device_error(p.report);
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TS_TMEM_COLS) : "memory");

@@ -270,7 +270,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     g.sw = w->scales;
     g.out = dC;
     g.status = ws->status;
-    g.report = &ws->host_status_alias->device_error;
+    g.report = ws->host_status_alias;
     *ws->host_status = Status{};
     g.M = st.M; g.N = st.N; g.K = st.K;
     g.KB = ws->KB; g.NG = w->NG; g.T = PERSIST_T;
