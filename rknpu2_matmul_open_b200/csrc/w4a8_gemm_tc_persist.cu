@@ -65,6 +65,14 @@ struct PsShape {
     static constexpr uint32_t GB = W8 ? 4096 : 2048;                             // one k-block of one 32-channel group
     static constexpr size_t XW_BYTES = PS_SK * 4 * (size_t)GB;
     static constexpr int BARRIERS = XA + 2 * WB + 2 * NR + 2 * ACC;
+    // barriers in the order in which they lie: xfull, wfull, wempty, ready, done, acc_full, acc_empty
+    static __device__ __forceinline__ uint32_t arrivals(int i)
+    {
+        if (i < XA) return W8 ? 2 : 1;
+        if ((i -= XA) < 2 * WB) return i < WB ? 1 : 4;
+        if ((i -= 2 * WB) < 2 * NR) return i < NR ? (W8 ? 0 : 8) + 2 : 1;
+        return i - 2 * NR < ACC ? 1 : 2 * PS_EPI_WARPS;           // acc_empty: every epilogue warp of both CTAs
+    }
     static constexpr size_t SMEM = XA * XA_BYTES + XW * XW_BYTES + 2 * TOK * 4 + BARRIERS * 8 + 32;
     static_assert(TOK % 32 == 0 && TOK <= 256, "not the width of an MMA");
     static_assert(SMEM <= 232448, "exceeds the shared memory of one CTA");
@@ -187,26 +195,35 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
 #define PS_STAMP(j, slot) do { if (trace && (j) < 16) trace[(j) * 8 + (slot)] = (unsigned long long)(clock64() - c0); } while (0)
     if (trace && tid == 0) trace[200] = (unsigned long long)num_clusters;
 
-    if (tid == 0) {
-        for (int s = 0; s < S::XA; ++s) mbar_init(&xfull[s], W8 ? 2 : 1);
-        for (int s = 0; s < S::WB; ++s) { mbar_init(&wfull[s], 1); mbar_init(&wempty[s], 4); }
-        for (int b = 0; b < S::NR; ++b) { mbar_init(&ready[b], (W8 ? 0 : 8) + 2); mbar_init(&done[b], 1); }
-        for (int b = 0; b < S::ACC; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2 * PS_EPI_WARPS); }   // every epilogue warp of both CTAs
+    // Set-up: a CTA that could only start when one of the launch in front left is late with its weights and everything behind them,
+    // so nobody waits for more than it needs.  The weight producer makes the barriers (a lane each) and requests weights at once; it
+    // and the epilogue warps report here and settle later.
+    if (warp == 2) {
+        for (int i = lane; i < S::BARRIERS; i += 32) mbar_init(&xfull[i], S::arrivals(i));
         mbar_fence_init();
-        *s_error = 0;
-        *s_finish = 0;
-    }
-    if (tid < TOK) s_tilemax[tid] = 0u;
-    if (warp == 1) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (lane == 0) { *s_error = 0; *s_finish = 0; }
+        __syncwarp();
+    } else if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(PS_TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        tc_fence_before();
     }
-    tc_fence_before();
-    __syncthreads();
-    cluster_arrive();
-    cluster_wait();   // the peer's barriers and tensor memory exist from here on
-    tc_fence_after();
-    const uint32_t tmem_base = *s_tmem;
+    if (warp == 2 || warp >= S::EPI_WARP0) {
+        asm volatile("bar.arrive 2, %0;" ::"n"(S::THREADS) : "memory");
+        cluster_arrive();
+    } else {
+        asm volatile("bar.sync 2, %0;" ::"n"(S::THREADS) : "memory");
+        asm volatile("bar.arrive 3, %0;" ::"n"(S::THREADS) : "memory");
+        cluster_arrive();
+        cluster_wait();   // the peer's barriers and tensor memory exist from here on
+        tc_fence_after();
+    }
+    auto settle = [&]() {
+        asm volatile("bar.sync 3, %0;" ::"n"(S::THREADS) : "memory");
+        cluster_wait();
+        tc_fence_after();
+    };
 
     // What does not depend on the kernel in front -- requesting weights, unpacking the first of them into tensor
     // memory -- starts before the dependency wait.  Where the quantiser rejected the input the contraction runs all the same
@@ -217,7 +234,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         // (the whole warp walks the loop and one elected lane issues, as in the MMA issuer below: copy requests take their
         // operands from uniform registers, and four lanes issuing one request each took 1000 cycles per stage)
         RingPos<S::XW> r;
-        bool ok = true;
+        bool ok = true, settled = false;
         int g = 0;
         const size_t group_bytes = (size_t)KB * GB;
         const size_t upper = swiglu ? (size_t)(p.F / GROUP) * group_bytes : 2 * group_bytes;   // groups 2, 3 behind groups 0, 1
@@ -225,9 +242,13 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             const int ct = 2 * item.tile + (int)rank;
             const uint8_t* src = p.Wp + (size_t)(swiglu ? ct * 2 : ct * 4) * group_bytes + (size_t)it0 * (W8 ? 4 : 1) * PS_SK * GB;
             for (int it = it0; it < it1; ++it, ++g, r.next()) {
-                if (g == S::XW) pdl_wait();                    // (slots come back once the MMAs have activations)
+                if (g == S::XW) {                              // (slots come back once the MMAs have activations)
+                    settle();
+                    pdl_wait();
+                    settled = true;
+                }
                 const uint32_t bytes = (uint32_t)min(PS_SK, KB - PS_SK * it) * GB;
-                if (g >= S::XW) ok = __all_sync(0xffffffffu, W8 ? mbar_wait_cluster(&done[r.slot], r.phase ^ 1u, deadline) : mbar_wait(&wempty[r.slot], r.phase ^ 1u, deadline));
+                if (ok && g >= S::XW) ok = __all_sync(0xffffffffu, W8 ? mbar_wait_cluster(&done[r.slot], r.phase ^ 1u, deadline) : mbar_wait(&wempty[r.slot], r.phase ^ 1u, deadline));
                 if (!ok) { *s_error = 1; break; }
                 uint8_t* const dst = wts + (size_t)r.slot * S::XW_BYTES;
                 if (elect_one()) {
@@ -246,6 +267,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 src += (W8 ? 4 : 1) * PS_SK * GB;
             }
         }
+        if (!settled) settle();
     } else if (warp == 0) {
         // ---------------------------------------------------------------- activation producer
         pdl_wait();
@@ -306,12 +328,13 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             bool dead = false;                                     // (the elected lane's, always the same one)
             RingPos<S::ACC> rc;
             const uint32_t ready0 = smem_u32(ready), done0 = smem_u32(done);
+            int issued = 0;                                        // items
             const uint64_t b_first = tc_smem_desc(smem_u32(acts), 128u, PS_SK * 1024u);
             const uint64_t a_first = tc_smem_desc(smem_u32(wts), 2048u, 128u);        // W8
             const uint32_t b_hi = (uint32_t)(b_first >> 32), a_hi = (uint32_t)(a_first >> 32);
             const uint32_t b_lo0 = (uint32_t)b_first, a_lo0 = (uint32_t)a_first;
             const uint32_t b_lo_end = b_lo0 + (uint32_t)(S::XA * S::XA_BYTES / 16);
-            const uint32_t a_tmem0 = tmem_base + S::A_COL0;
+            const uint32_t tmem_base = *s_tmem, a_tmem0 = tmem_base + S::A_COL0;
             uint32_t b_lo = b_lo0, a_lo = a_lo0, a_tmem = a_tmem0, bar = 0, phase = 0;
             for (int j = 0; next_item(item); ++j, rc.next()) {
                 const uint32_t idesc = tc_idesc_s8(256, item.width);
@@ -364,12 +387,17 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 if (lane == 0) PS_STAMP(j, 2);
             }
         }
+                ++issued;
     } else if (warp < S::EPI_WARP0) {
+            // (the peer's last arrivals are waited for, so that none is on its way when this CTA leaves)
+            if (split == 1)
+                for (int j = max(0, issued - S::ACC); j < issued && !*reinterpret_cast<volatile int*>(s_error); ++j)
+                    if (!mbar_wait_cluster(&acc_empty[j % S::ACC], j / S::ACC & 1, deadline)) *s_error = 1;
         // ---------------------------------------------------------------- weight unpack -> TMEM
         if constexpr (!W8) {
         const int q = warp & 3;
         const int set = (warp - PS_UNPACK_WARP0) >> 2;
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+        const uint32_t lane_addr = *s_tmem + ((uint32_t)(q * 32) << 16);
         // Which row of the staged weight groups feeds this thread's tensor-memory lane.  The epilogue's thread t reads lanes
         // t / 4 + 8 c; they hold channels 4 (t / 4) .. + 3 of the warp's group, or (SwiGLU) features 2 (t / 4), + 1 of sixteen,
         // gate values in lanes 0-15 and up values in lanes 16-31 (staged groups 0, 1 = gate, 2, 3 = up of the same 64
@@ -458,7 +486,6 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         const int q = warp & 3;                        // TMEM lane quarter this warp may read
         const int eset = (warp - S::EPI_WARP0) >> 2;   // takes pieces eset, eset + PS_EPI_SETS, ...
         const int sid = (warp - S::EPI_WARP0) * 32 + lane;   // 0..255 among the epilogue threads
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
         const int out_cols = swiglu ? p.F : p.N;
         // This thread's fragment: channels 4 i8 .. + 3 of its group (features 2 i8, + 1 of sixteen), the one in its c-th
         // tensor-memory lane is number (c + turn) of them; tokens 2 tq, 2 tq + 1 and eight further of a piece.
@@ -475,7 +502,10 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         const bool fragments = swiglu || wide_ok;
         constexpr int STEP = 16 * PS_EPI_SETS;
         constexpr int SHIFT = W8 ? 0 : 4;              // int4 records enter the MMA times 16
+        if (sid < TOK) s_tilemax[sid] = 0u;            // (read behind barriers of the epilogue warps)
         pdl_wait();
+        settle();
+        const uint32_t lane_addr = *s_tmem + ((uint32_t)(q * 32) << 16);
         if (!W8 && sid == 0) *s_verdict = take_verdict(p.status, p.report);
         bool ok = true, good = true;
         RingPos<S::ACC> rc;
@@ -571,7 +601,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 for (int h = 0; h < 4; ++h) v[h] = __ldcg(src + (size_t)h * 128);
             };
             if (split > 1 && turns) fetch_part(ahead, other, 0);
-            if (pieces == 0 && (split == 1 || !good)) hand_back();
+            if (pieces == 0 && split == 1) hand_back();
 #pragma unroll 1
             for (int k = 0; k < turns; ++k) {
                 const int t0 = 16 * eset + STEP * k + 2 * tq;             // this thread's first token of the turn
@@ -761,12 +791,14 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
     // shared memory: they land within microseconds, so the CTA stays that long before it leaves.
     if (*reinterpret_cast<volatile int*>(s_error))
         for (const unsigned long long until = global_ns() + PS_DRAIN_NS; global_ns() < until;) __nanosleep(1000);
-    cluster_arrive();
-    cluster_wait();   // neither CTA frees tensor memory or leaves while the other may still use it
+    // Neither CTA frees tensor memory or leaves while the other may still use it.  (Every arrival from the other CTA has been
+    // waited for, so the barrier need not order memory: an arrival with a release waits for this CTA's results to be stored.)
+    cluster_arrive_relaxed();
+    cluster_wait();
     if (tid == 0 && *s_error) report_device_error(p.report);
     if (warp == 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(PS_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(*s_tmem), "r"(PS_TMEM_COLS) : "memory");
     }
 }
 
