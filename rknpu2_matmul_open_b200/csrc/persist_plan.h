@@ -14,7 +14,7 @@
 
 namespace rkb200 {
 
-constexpr int PERSIST_T = 8;            // tokens of a group of activation codes (GemmParams::T)
+constexpr int PERSIST_T = 1;            // tokens of a group of activation codes (GemmParams::T): every token's codes lie in one piece
 constexpr int PERSIST_TOKENS = 32;      // the code buffer holds a whole multiple of these, items are multiples of them
 
 // The widest item of a kernel that takes the plan's.  (int8 weights: the first and the last.)

@@ -18,7 +18,8 @@
 //   them), t : token inside the tile; the 16 bytes are the int8 codes k = 16kc .. 16kc+15.
 //   A k-block (128 k) of one token tile is contiguous, and a group of eight tokens x 16
 //   bytes is the 8x16-byte core matrix both mma.sync and tcgen05 (no-swizzle, K-major)
-//   consume.  Replaces the reference's MSD-split A[K/32, 2*rows, 32] int4 layout
+//   consume.  T = 1 (the persistent kernel): a token's codes are one row, no line of memory is written by two CTAs, and tensor
+//   copies bring boxes of rows x 128 bytes with the 128-byte swizzle that tcgen05 reads.  Replaces the reference's MSD-split A[K/32, 2*rows, 32] int4 layout
 //   (src/rk_npu_w4a8_quant.cpp:87-135): int8 MMA is native here so no split is needed.
 #pragma once
 #include <atomic>
@@ -120,10 +121,10 @@ __device__ __forceinline__ int take_verdict(Status* status, Status* report)
 }
 #endif
 
-// Tensor maps of a persistent kernel's activation codes [groups of eight tokens][K bytes x 8]: boxes of two k-blocks of eight,
-// four and two groups.  Made once for a workspace's code buffer.
+// Tensor maps of a persistent kernel's activation codes [k-blocks][tokens][128 bytes]: boxes of two k-blocks of 16, 32, ... 128 tokens
+// (the halves of an item's).  Made once for a workspace's code buffer.
 struct PersistMaps {
-    CUtensorMap box[3];
+    CUtensorMap box[8];
 };
 
 struct GemmParams {
@@ -280,7 +281,7 @@ int gemm_decode_ctas(int items, int cluster, int cap);
 int gemm_decode_resident_ctas(int cluster, size_t smem, int sm_count);
 cudaError_t launch_gemm_decode(const DecodeParams& p, cudaStream_t stream, bool pdl);
 cudaError_t launch_gemm_decode_batch(const DecodeBatch& b, cudaStream_t stream, bool pdl);
-// Persistent two-CTA tcgen05 kernel (K <= 131072).  Its activation codes lie in groups of PERSIST_T tokens (p.T) up to a
+// Persistent two-CTA tcgen05 kernel (K <= 131072).  Its activation codes are rows (p.T == PERSIST_T) up to a
 // multiple of 32 tokens; p.partials and p.counts where split > 1.
 cudaError_t launch_gemm_tc_persist(const GemmParams& p, cudaStream_t stream, bool pdl);
 bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB);

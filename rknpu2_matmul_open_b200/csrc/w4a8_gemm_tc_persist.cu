@@ -270,24 +270,26 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         if (!settled) settle();
     } else if (warp == 0) {
         // ---------------------------------------------------------------- activation producer
+        {
+            PersistItems first = items;
+            int tile, at, n;
+            if (lane == 0 && first.next(tile, at, n)) tensor_prefetch_map(&maps.box[min(n * p.unit, (p.M - at * p.unit + 31) & ~31) / 32 - 1]);
+        }
         pdl_wait();
         RingPos<S::XA> r;
         bool ok = true;
         int g = 0;
         while (ok && next_item(item)) {
-            const int groups = item.width / 16;            // of this CTA's half
-            const int row0 = item.tok0 / 8 + (int)rank * groups;
+            const int rows = item.width / 2;               // of this CTA's half
+            const int row0 = item.tok0 + (int)rank * rows;
+            const CUtensorMap* const box = &maps.box[rows / 16 - 1];
             for (int it = it0; it < it1; ++it, ++g, r.next()) {
                 if (g >= S::XA) ok = __all_sync(0xffffffffu, mbar_wait_cluster(&done[(g - S::XA) % S::NR], (g - S::XA) / S::NR & 1, deadline));
                 if (!ok) { *s_error = 1; break; }
                 if (elect_one()) {
                     // (a stage's second k-block that does not exist is filled with zeros)
-                    mbar_arrive_expect_tx(&xfull[r.slot], (uint32_t)groups * (PS_SK * 1024u));
-                    uint8_t* dst = acts + (size_t)r.slot * S::XA_BYTES;
-                    int row = row0, left = groups;
-                    for (; left >= 8; left -= 8, row += 8, dst += 8 * PS_SK * 1024) tensor_g2s(dst, &maps.box[0], it * PS_SK * 128, row, &xfull[r.slot]);
-                    if (left & 4) { tensor_g2s(dst, &maps.box[1], it * PS_SK * 128, row, &xfull[r.slot]); row += 4; dst += 4 * PS_SK * 1024; }
-                    if (left & 2) tensor_g2s(dst, &maps.box[2], it * PS_SK * 128, row, &xfull[r.slot]);
+                    mbar_arrive_expect_tx(&xfull[r.slot], (uint32_t)rows * (PS_SK * 128u));
+                    tensor_g2s(acts + (size_t)r.slot * S::XA_BYTES, box, row0, it * PS_SK, &xfull[r.slot]);
                 }
                 __syncwarp();
             }
@@ -326,10 +328,10 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         pdl_wait();
         if (rank == 0) {
             bool dead = false;                                     // (the elected lane's, always the same one)
+            int issued = 0;                                        // items
             RingPos<S::ACC> rc;
             const uint32_t ready0 = smem_u32(ready), done0 = smem_u32(done);
-            int issued = 0;                                        // items
-            const uint64_t b_first = tc_smem_desc(smem_u32(acts), 128u, PS_SK * 1024u);
+            const uint64_t b_first = tc_smem_desc_rows128(smem_u32(acts));
             const uint64_t a_first = tc_smem_desc(smem_u32(wts), 2048u, 128u);        // W8
             const uint32_t b_hi = (uint32_t)(b_first >> 32), a_hi = (uint32_t)(a_first >> 32);
             const uint32_t b_lo0 = (uint32_t)b_first, a_lo0 = (uint32_t)a_first;
@@ -338,6 +340,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
             uint32_t b_lo = b_lo0, a_lo = a_lo0, a_tmem = a_tmem0, bar = 0, phase = 0;
             for (int j = 0; next_item(item); ++j, rc.next()) {
                 const uint32_t idesc = tc_idesc_s8(256, item.width);
+                const uint32_t block = 4u * (uint32_t)item.width;  // of descriptor address between a stage's k-blocks
                 if (lane == 0) PS_STAMP(j, 0);
                 if (j >= S::ACC) {   // the epilogue warps of both CTAs have read this accumulator's previous item
                     if (!__all_sync(0xffffffffu, mbar_wait_cluster(&acc_empty[rc.slot], rc.phase ^ 1u, deadline))) { *s_error = 1; break; }
@@ -346,8 +349,7 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 const uint32_t d_tmem = tmem_base + rc.slot * TOK;
                 const bool odd_end = (KB & 1) && it1 == nst;       // the last stage has one k-block
                 for (int it = it0; it < it1; ++it) {
-                    // k-step q: 32 k = two 16-byte chunks per row: the descriptors' address fields advance by two core
-                    // matrices of the activations, by two 128-channel columns of int8 weights
+                    // k-step q: 32 k: 32 bytes of the activations' rows, two 128-channel columns of int8 weights
                     const uint64_t b_desc = (uint64_t)b_hi << 32 | b_lo, a_desc = (uint64_t)a_hi << 32 | a_lo;
                     const uint32_t a_now = a_tmem;
                     const bool whole = !(odd_end && it == nst - 1);
@@ -358,18 +360,18 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                             if constexpr (W8) {
                                 tc_mma_i8_ss_pair(d_tmem, a_desc, b_desc, idesc, it != it0 ? 1u : 0u);
 #pragma unroll
-                                for (int q = 1; q < 4; ++q) tc_mma_i8_ss_pair(d_tmem, a_desc + 256u * q, b_desc + 16u * q, idesc, 1u);
+                                for (int q = 1; q < 4; ++q) tc_mma_i8_ss_pair(d_tmem, a_desc + 256u * q, b_desc + 2u * q, idesc, 1u);
                                 if (whole) {
 #pragma unroll
-                                    for (int q = 4; q < 8; ++q) tc_mma_i8_ss_pair(d_tmem, a_desc + 256u * q, b_desc + 16u * q, idesc, 1u);
+                                    for (int q = 4; q < 8; ++q) tc_mma_i8_ss_pair(d_tmem, a_desc + 256u * q, b_desc + block + 2u * (q - 4), idesc, 1u);
                                 }
                             } else {
                                 tc_mma_i8_ts_pair(d_tmem, a_now, b_desc, idesc, it != it0 ? 1u : 0u);
 #pragma unroll
-                                for (int q = 1; q < 4; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_now + 8 * q, b_desc + 16u * q, idesc);
+                                for (int q = 1; q < 4; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_now + 8 * q, b_desc + 2u * q, idesc);
                                 if (whole) {
 #pragma unroll
-                                    for (int q = 4; q < 8; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_now + 8 * q, b_desc + 16u * q, idesc);
+                                    for (int q = 4; q < 8; ++q) tc_mma_i8_ts_pair_acc(d_tmem, a_now + 8 * q, b_desc + block + 2u * (q - 4), idesc);
                                 }
                             }
                             tc_commit_pair_at(done0 + bar);   // in both CTAs: the stage's operands may be overwritten once these MMAs retire
@@ -385,14 +387,14 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                 }
                 __syncwarp();
                 if (lane == 0) PS_STAMP(j, 2);
-            }
-        }
                 ++issued;
-    } else if (warp < S::EPI_WARP0) {
+            }
             // (the peer's last arrivals are waited for, so that none is on its way when this CTA leaves)
             if (split == 1)
                 for (int j = max(0, issued - S::ACC); j < issued && !*reinterpret_cast<volatile int*>(s_error); ++j)
                     if (!mbar_wait_cluster(&acc_empty[j % S::ACC], j / S::ACC & 1, deadline)) *s_error = 1;
+        }
+    } else if (warp < S::EPI_WARP0) {
         // ---------------------------------------------------------------- weight unpack -> TMEM
         if constexpr (!W8) {
         const int q = warp & 3;
@@ -506,8 +508,8 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         pdl_wait();
         settle();
         const uint32_t lane_addr = *s_tmem + ((uint32_t)(q * 32) << 16);
-        if (!W8 && sid == 0) *s_verdict = take_verdict(p.status, p.report);
         bool ok = true, good = true;
+        if (!W8 && sid == 0) *s_verdict = take_verdict(p.status, p.report);
         RingPos<S::ACC> rc;
         for (int j = 0; ok && next_item(item); ++j, rc.next()) {
             const int ct = 2 * item.tile + (int)rank;
@@ -873,7 +875,6 @@ size_t gemm_tc_persist_count_bytes(int columns, int M, const PersistPlan& plan)
     return plan.split > 1 ? 2 * size_t(units_of(columns, M, plan.unit)) * sizeof(unsigned) : 0;
 }
 
-// Eight-byte elements: 256 of them, the most a box may have, are the two k-blocks of a stage.
 bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB)
 {
     static const auto encode = []() {
@@ -886,12 +887,12 @@ bool make_persist_maps(PersistMaps& maps, const uint8_t* codes, int M, int KB)
         return reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(entry);
     }();
     if (!encode) return false;
-    const cuuint64_t dims[2] = {cuuint64_t(KB) * 128, (cuuint64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * (PERSIST_TOKENS / PERSIST_T)};
-    const cuuint64_t strides[1] = {cuuint64_t(KB) * 1024};
-    const cuuint32_t steps[2] = {1, 1};
-    for (int i = 0; i < 3; ++i) {
-        const cuuint32_t box[2] = {PS_SK * 128, 8u >> i};
-        if (encode(&maps.box[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t*>(codes), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    const cuuint64_t dims[3] = {128, (cuuint64_t(M) + PERSIST_TOKENS - 1) / PERSIST_TOKENS * PERSIST_TOKENS, cuuint64_t(KB)};
+    const cuuint64_t strides[2] = {cuuint64_t(KB) * 128, 128};
+    const cuuint32_t steps[3] = {1, 1, 1};
+    for (int i = 0; i < 8; ++i) {
+        const cuuint32_t box[3] = {128, 16u * (i + 1), PS_SK};
+        if (encode(&maps.box[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<uint8_t*>(codes), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return false;
     }

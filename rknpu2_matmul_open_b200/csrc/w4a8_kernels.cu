@@ -213,7 +213,7 @@ cudaError_t launch_quantize(const QuantParams& p, cudaStream_t stream, bool pdl)
     cfg.numAttrs = pdl ? 1 : 0;
     cfg.dynamicSmemBytes = 0;
     const bool scan = p.rowmax == nullptr;      // (collected maxima come with an fp32 middle)
-    if (!(p.half ? scan && quantize_rows_ok<true>(p.A, p.K, p.T) : quantize_rows_ok<false>(p.A, p.K, p.T))) {
+    if (!(p.half ? scan && quantize_rows_ok<true>(p.A, p.K) : quantize_rows_ok<false>(p.A, p.K))) {
         cfg.gridDim = dim3((unsigned)p.M);
         cfg.blockDim = dim3(256);
         return p.half ? cudaLaunchKernelEx(&cfg, quantize_kernel<true>, p) : cudaLaunchKernelEx(&cfg, quantize_kernel<false>, p);

@@ -86,13 +86,14 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_global,
                  : "memory");
 }
 
-// ---- tensor copy global -> shared of a box of a two-dimensional map (x in elements, a multiple of 16 bytes)
-__device__ __forceinline__ void tensor_g2s(void* dst_smem, const void* map, int x, int y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+// ---- tensor copy global -> shared of a box of a three-dimensional map that begins at x = 0
+__device__ __forceinline__ void tensor_g2s(void* dst_smem, const void* map, int y, int z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
                      smem_u32(dst_smem)),
-                 "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+                 "l"(map), "r"(0), "r"(y), "r"(z), "r"(smem_u32(bar))
                  : "memory");
 }
+__device__ __forceinline__ void tensor_prefetch_map(const void* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
 
 // ---- distributed shared memory: a 32-bit store into a peer CTA's shared memory that also counts
 // four bytes on a barrier in that CTA.  Data and signal travel together, so the receiver needs no
@@ -115,8 +116,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // ---- cluster barrier, split form: arrive early, wait right before the first access to a
 // peer's shared memory (all CTAs of the cluster have started once the wait returns)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;

@@ -127,7 +127,7 @@ __device__ __forceinline__ void exchange_piece(uint32_t* words, int lane, const 
 
 // 16-byte loads are possible for every row.
 template <bool HALF>
-inline bool quantize_rows_ok(const void* A, int K, int T) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % QuantRows<HALF, 1>::EPW == 0 && T % 2 == 0; }
+inline bool quantize_rows_ok(const void* A, int K) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % QuantRows<HALF, 1>::EPW == 0; }
 // Calls f with the shape of the launch: <tokens per CTA, threads, loads a thread keeps>.
 // Rows that are scanned.  Up to 296 tokens (two CTAs of 512 threads an SM, all resident) a token per CTA, and all the
 // threads that help with a row work on it.  Up to 591 these CTAs would come in two waves: 256 threads (in front of 4096

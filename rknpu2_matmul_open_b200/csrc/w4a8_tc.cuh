@@ -196,6 +196,14 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t smem_addr, uint32_t lb
     const uint32_t hi = (sbo >> 4) | (1u << 14);   // descriptor version 1 (sm_100); layout type 0 = no swizzle
     return ((uint64_t)hi << 32) | lo;
 }
+// K-major rows of 128 bytes, 128-byte swizzle, groups of eight rows behind each other: a tensor copy's box with the same swizzle, at
+// a multiple of 1024 bytes.  32 bytes further in K are 32 bytes further in the address field.
+__device__ __forceinline__ uint64_t tc_smem_desc_rows128(uint32_t smem_addr)
+{
+    const uint32_t lo = ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16);
+    const uint32_t hi = (1024u >> 4) | (1u << 14) | (2u << 29);   // stride of eight rows, descriptor version 1, layout type 2
+    return ((uint64_t)hi << 32) | lo;
+}
 // Instruction descriptor: int32 accumulators, signed 8-bit A and B, both K-major, M = 128.
 __device__ __forceinline__ uint32_t tc_idesc_s8(int m, int n)
 {

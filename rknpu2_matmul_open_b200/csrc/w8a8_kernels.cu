@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) w8_codes_kernel(const W8QuantParams p)
 template <bool HALF, bool SCAN>
 static void launch_w8_rows(const W8QuantParams& p, cudaStream_t stream)
 {
-    if (!quantize_rows_ok<HALF>(p.A, p.K, p.T)) {
+    if (!quantize_rows_ok<HALF>(p.A, p.K)) {
         w8_quantize_kernel<HALF><<<(unsigned)p.M, 256, 0, stream>>>(p);
         return;
     }
