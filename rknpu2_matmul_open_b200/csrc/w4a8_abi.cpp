@@ -477,6 +477,7 @@ int enqueue(const Call& c)
     g.sw = c.w->scales;
     g.out = c.dOut;
     g.rowmax = c.rowmax_out;
+    g.rowmax_in = c.codes_in ? nullptr : c.rowmax_in;    // (a launch that takes codes has cleared them)
     g.status = ws.status;
     g.report = c.status ? c.status : ws.status;
     g.M = cfg.M;

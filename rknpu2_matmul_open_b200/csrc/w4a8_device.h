@@ -70,7 +70,7 @@ struct QuantParams {
     // their consumer.  (Without this store the compiler spills more bytes in the fp32 form that is held to 32 registers:
     // FFN of 1163 x 2816 -> 2 x 4096 72.2 -> 73.5 us, 1616 rows of 3735 115 -> 119.)
     uint32_t* rowmax_zero;
-    uint32_t* rowmax;       // [M] non-null: scales come from these magnitude bits (no scan); cleared after use
+    const uint32_t* rowmax; // [M] non-null: scales come from these magnitude bits (no scan); cleared by the GEMM behind
     Status* status;
     int M, K, Kp, T;
     int half;
@@ -119,6 +119,13 @@ __device__ __forceinline__ int take_verdict(Status* status, Status* report)
     } else if (report == status && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) report->bad_input = 0;
     return bad;
 }
+// Collected maxima back to zero for the next SwiGLU epilogue, by one CTA behind everybody's reads.  (When whoever quantised a row
+// cleared its word, 32 CTAs took turns to read and write one line of L2, up to 8 us.)
+__device__ __forceinline__ void clear_maxima(uint32_t* rowmax, int M, int thread, int threads)
+{
+    if (rowmax)
+        for (int m = thread; m < M; m += threads) rowmax[m] = 0u;
+}
 #endif
 
 // Tensor maps of a persistent kernel's activation codes [k-blocks][tokens][128 bytes]: boxes of two k-blocks of 16, 32, ... 128 tokens
@@ -134,6 +141,7 @@ struct GemmParams {
     const float* sw;        // per-channel scales (padded to 32*NG)
     void* out;              // [M,N] fp32 / fp16 / int32, or middle [M,F] fp32
     uint32_t* rowmax;       // SwiGLU: per-row max |middle| bit pattern (nullable)
+    uint32_t* rowmax_in;    // maxima that the activations' scales came from, read by now: to be cleared (nullable)
     Status* status;
     Status* report;         // where the verdict and a wait that ran out are recorded: the same block, or one in page-locked host memory that the host has cleared
     int M, N, K;

@@ -509,7 +509,10 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
         settle();
         const uint32_t lane_addr = *s_tmem + ((uint32_t)(q * 32) << 16);
         bool ok = true, good = true;
-        if (!W8 && sid == 0) *s_verdict = take_verdict(p.status, p.report);
+        if constexpr (!W8) {
+            if (sid == 0) *s_verdict = take_verdict(p.status, p.report);
+            if (blockIdx.x == 0) clear_maxima(p.rowmax_in, p.M, sid, 32 * PS_EPI_WARPS);
+        }
         RingPos<S::ACC> rc;
         for (int j = 0; ok && next_item(item); ++j, rc.next()) {
             const int ct = 2 * item.tile + (int)rank;

@@ -82,7 +82,6 @@ struct RowQuant {
     {
         if (p.rowmax) {
             bits = p.rowmax[m];
-            p.rowmax[m] = 0u;    // consumed: the next SwiGLU epilogue maxes into a clean word
         }
         float maximum;
         int bad;
@@ -164,7 +163,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
         }
     } else if (tid == 0) {
         const uint32_t bits = p.rowmax[m];
-        p.rowmax[m] = 0u;   // consumed: the next SwiGLU epilogue maxes into a clean word
         bad = bits >= 0x7f800000u ? 2 : 0;
         const float maximum = __uint_as_float(bits);
         const float s = (maximum == 0.f || bad) ? 1.0f : fmaxf(__fdiv_rn(maximum, 127.0f), FLT_MIN);
@@ -336,6 +334,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
         pdl_wait();
         // (the contraction does not wait for the verdict: only the results depend on it)
         if (tid == 0) s_verdict = take_verdict(p.status, p.report);
+        if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) clear_maxima(p.rowmax_in, p.M, tid, 128);
         const int g8 = lane >> 2, t4 = lane & 3;
         for (int it = 0; it < nkb; ++it) {
             const int s = it % MMA_STAGES;

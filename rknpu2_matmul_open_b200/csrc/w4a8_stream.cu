@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1) gemm_tc_stream_kernel(const Gem
     }
     pdl_wait();       // activation codes, scales and the status word come from the kernel in front
     if (tid == 0) s_verdict = take_verdict(p.status, p.report);
+    if (blockIdx.x == 0) clear_maxima(p.rowmax_in, p.M, tid, (int)blockDim.x);
     __syncthreads();
     const bool skip = s_verdict != 0;
 
