@@ -446,7 +446,6 @@ int enqueue(const Call& c)
         ci.codes = c.codes_in;
         ci.Xq = ws.codes;
         ci.scales = ws.scales;
-        ci.inverse = ws.inverse;
         ci.rowmax = c.rowmax_in;
         ci.status = ws.status;
         ci.M = cfg.M; ci.K = cfg.K; ci.Kp = ws.KB * KBLOCK; ci.T = ws.T;
@@ -457,8 +456,6 @@ int enqueue(const Call& c)
     q.A = c.dA;
     q.Xq = ws.codes;
     q.scales = ws.scales;
-    q.inverse = ws.inverse;
-    q.rowmax_zero = nullptr;
     q.rowmax = c.rowmax_in;
     q.status = ws.status;
     q.M = cfg.M;
@@ -526,7 +523,7 @@ int status_to_rc(rk_npu_w4a8_workspace& ws, cudaStream_t stream)
 {
     const Status s = *ws.host_status;
     if (s.device_error) {
-        cudaMemsetAsync(&ws.status->device_error, 0, sizeof(int), stream);
+        cudaMemsetAsync(ws.status, 0, sizeof(Status), stream);
         // a launch that gave up may have left tiles unfinished
         if (ws.counts) cudaMemsetAsync(ws.counts, 0, ws.counts_bytes, stream);
         cudaStreamSynchronize(stream);
@@ -688,7 +685,7 @@ void workspace_destroy(rk_npu_w4a8_workspace* ws)
     if (d) cudaSetDevice(d->ctx->device);
     if (ws->stream) cudaStreamSynchronize(ws->stream);
     if (ws->codes) device_free(d, ws->codes, ws->codes_bytes);
-    if (ws->scales) device_free(d, ws->scales, sizeof(float) * 2 * ws->config.M);
+    if (ws->scales) device_free(d, ws->scales, sizeof(float) * ws->config.M);
     if (ws->rowmax) device_free(d, ws->rowmax, sizeof(uint32_t) * ws->config.M);
     if (ws->status) device_free(d, ws->status, sizeof(Status));
     if (ws->stage_in) device_free(d, ws->stage_in, ws->stage_in_bytes);
@@ -1193,7 +1190,7 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     ws->stage_out_bytes = size_t(cfg->M) * out_cols * 4;
     bool ok = !device_alloc(domain, reinterpret_cast<void**>(&ws->codes), ws->codes_bytes);
     ok = ok && (variant != 2 || make_persist_maps(ws->maps, ws->codes, cfg->M, ws->KB));
-    ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), sizeof(float) * 2 * cfg->M);
+    ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->scales), sizeof(float) * cfg->M);
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->rowmax), sizeof(uint32_t) * cfg->M);
     ok = ok && !device_alloc(domain, reinterpret_cast<void**>(&ws->status), sizeof(Status));
     if (variant == 4) {
@@ -1223,7 +1220,6 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     ok = ok && !device_alloc(domain, &ws->stage_in, ws->stage_in_bytes);
     ok = ok && !device_alloc(domain, &ws->stage_out, ws->stage_out_bytes);
     if (ok) {
-        ws->inverse = ws->scales + cfg->M;
         ok = cudaHostAlloc(reinterpret_cast<void**>(&ws->host_status), sizeof(Status), cudaHostAllocDefault) == cudaSuccess &&
              cudaStreamCreateWithFlags(&ws->stream, cudaStreamNonBlocking) == cudaSuccess;
     }

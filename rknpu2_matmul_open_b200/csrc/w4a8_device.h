@@ -65,11 +65,6 @@ struct QuantParams {
     const void* A;          // [M,K] fp32 or binary16
     uint8_t* Xq;            // activation codes, layout above
     float* scales;          // [M]
-    float* inverse;         // [M]
-    // [M] cleared as well, for a SwiGLU epilogue that maxes into it; NULL: every caller's epilogue finds its maxima cleared by
-    // their consumer.  (Without this store the compiler spills more bytes in the fp32 form that is held to 32 registers:
-    // FFN of 1163 x 2816 -> 2 x 4096 72.2 -> 73.5 us, 1616 rows of 3735 115 -> 119.)
-    uint32_t* rowmax_zero;
     const uint32_t* rowmax; // [M] non-null: scales come from these magnitude bits (no scan); cleared by the GEMM behind
     Status* status;
     int M, K, Kp, T;
@@ -89,7 +84,6 @@ struct CodesInParams {
     const int8_t* codes;    // [parts][M][K / parts] int8 (parts = 1: plain [M, K])
     uint8_t* Xq;
     float* scales;          // [M]
-    float* inverse;         // [M]
     uint32_t* rowmax;       // [M] magnitude bits the scales come from; cleared after use
     Status* status;
     int M, K, Kp, T;

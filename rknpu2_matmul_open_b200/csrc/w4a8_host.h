@@ -134,7 +134,6 @@ struct rk_npu_w4a8_workspace {
     // device buffers
     uint8_t* codes = nullptr;
     float* scales = nullptr;
-    float* inverse = nullptr;
     uint32_t* rowmax = nullptr;
     rkb200::PersistPlan plan[2]{};    // variant 2: how a linear and a SwiGLU launch are cut
     rkb200::PersistMaps maps{};       // and where its activation codes are

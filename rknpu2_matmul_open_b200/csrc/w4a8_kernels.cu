@@ -66,52 +66,12 @@ cudaError_t launch_pack_weights(const PackParams& p, cudaStream_t stream)
 // magnitude bits order like the magnitudes, and anything at or above the infinity pattern is
 // NaN/Inf).  Pass 2: q = clamp(round_half_away(x * inverse), -127, 127), written as 16-byte units of
 // the Xq layout.  Rows that allow 16-byte loads: quantize_rows (w4a8_quantize.cuh).
-template <bool HALF>
-struct RowQuant {
-    const QuantParams& p;
-    static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r)
-    {
-        if constexpr (HALF) {
-            // pairs of magnitudes in one word: both halves order like unsigned 16-bit numbers
-            uint32_t m = __vmaxu2(__vmaxu2(r.x & 0x7fff7fffu, r.y & 0x7fff7fffu), __vmaxu2(r.z & 0x7fff7fffu, r.w & 0x7fff7fffu));
-            return max(best, max(m & 0xffffu, m >> 16));
-        }
-        return max(max(best, max(r.x & 0x7fffffffu, r.y & 0x7fffffffu)), max(r.z & 0x7fffffffu, r.w & 0x7fffffffu));
-    }
-    __device__ __forceinline__ float begin(int m, uint32_t bits)
-    {
-        if (p.rowmax) {
-            bits = p.rowmax[m];
-        }
-        float maximum;
-        int bad;
-        if (HALF && !p.rowmax) {
-            bad = bits >= 0x7c00u ? 1 : 0;
-            maximum = __half2float(__ushort_as_half((uint16_t)bits));
-        } else {
-            bad = bits >= 0x7f800000u ? (p.rowmax ? 2 : 1) : 0;
-            maximum = __uint_as_float(bits);
-        }
-        const float s = (maximum == 0.f || bad) ? 1.0f : fmaxf(__fdiv_rn(maximum, 127.0f), FLT_MIN);
-        const float inv = __fdiv_rn(1.0f, s);
-        p.scales[m] = s;
-        p.inverse[m] = inv;
-        if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
-        if (bad) p.status->bad_accum = bad;     // (the same value from every bad row of a launch)
-        return inv;
-    }
-    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
-    {
-        return quantize4(__fmul_rn(a, inv), __fmul_rn(b, inv), __fmul_rn(c, inv), __fmul_rn(d, inv));
-    }
-};
-template <bool HALF, int TG, bool SCAN, int BS, int UN>
-__global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) quantize_rows_kernel(const QuantParams p)
+template <bool HALF, bool SCAN, int BS, int UN>
+__global__ void __launch_bounds__(BS, (UN <= 4 ? 1280 : 896) / BS) quantize_rows_kernel(const QuantParams p)
 {
     pdl_launch_dependents();   // the GEMM behind this kernel may start prefetching weights
     pdl_wait();                // A may be the output of the kernel in front of this one
-    RowQuant<HALF> op{p};
-    quantize_rows<HALF, TG, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, op);
+    quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, RowQuant<HALF>{p.scales, p.rowmax, &p.status->bad_accum});
 }
 
 // Any row: one CTA per token.
@@ -158,7 +118,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
             const float s = (maximum == 0.f || bad) ? 1.0f : fmaxf(__fdiv_rn(maximum, 127.0f), FLT_MIN);
             const float inv = __fdiv_rn(1.0f, s);
             p.scales[m] = s;
-            p.inverse[m] = inv;
             s_inverse = inv;
         }
     } else if (tid == 0) {
@@ -168,7 +127,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
         const float s = (maximum == 0.f || bad) ? 1.0f : fmaxf(__fdiv_rn(maximum, 127.0f), FLT_MIN);
         const float inv = __fdiv_rn(1.0f, s);
         p.scales[m] = s;
-        p.inverse[m] = inv;
         s_inverse = inv;
     }
     __syncthreads();
@@ -184,7 +142,6 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
         if (kc < chunks) dst[(size_t)kc * p.T] = kc * 16 < p.K ? quantize16(v, inv, kc * 16, p.K) : make_uint4(0u, 0u, 0u, 0u);
     }
     if (tid == 0) {
-        if (p.rowmax_zero) p.rowmax_zero[m] = 0u;
         if (bad) p.status->bad_accum = bad;     // (the same value from every bad row of a launch)
     }
 }
@@ -192,11 +149,11 @@ __global__ void __launch_bounds__(256, 6) quantize_kernel(const QuantParams p)
 template <bool HALF, bool SCAN>
 static cudaError_t launch_quantize_rows(const QuantParams& p, cudaLaunchConfig_t& cfg)
 {
-    return with_quantize_rows_shape<HALF, SCAN>(p.M, p.K, [&](auto tg, auto bs, auto un) {
-        constexpr int TG = decltype(tg)::value, BS = decltype(bs)::value, UN = decltype(un)::value;
-        cfg.gridDim = dim3((unsigned)((p.M + TG - 1) / TG));
+    return with_quantize_rows_shape<HALF, SCAN>(p.M, p.K, [&](auto bs, auto un) {
+        constexpr int BS = decltype(bs)::value, UN = decltype(un)::value;
+        cfg.gridDim = dim3((unsigned)p.M);
         cfg.blockDim = dim3((unsigned)BS);
-        return cudaLaunchKernelEx(&cfg, quantize_rows_kernel<HALF, TG, SCAN, BS, UN>, p);
+        return cudaLaunchKernelEx(&cfg, quantize_rows_kernel<HALF, SCAN, BS, UN>, p);
     });
 }
 
@@ -635,7 +592,6 @@ extern "C" int rk_npu_b200_w4a8_enqueue_f16_static(const rk_npu_w4a8_weights* we
     q.A = dA;
     q.Xq = codes;
     q.scales = scales;
-    q.inverse = scales + STATIC_MAX_TOKENS;
     q.status = status;
     q.M = M;
     q.K = K;

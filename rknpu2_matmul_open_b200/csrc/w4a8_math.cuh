@@ -229,11 +229,11 @@ __device__ __forceinline__ int round_clamp(float x)
     return (n ^ m) - m;
 }
 // Four products -> four int8 codes in one word (byte i = code of y[i]), ties away from zero.
-// Magnitudes: |y| + 0.5 added toward zero, then 1.5 * 2^23 added toward zero leaves floor(|y| + 0.5) in the low byte of
-// the float's bits (see round_clamp).  No clamp: every caller's scale is max(max|row| / 127, FLT_MIN) of the row the
+// Magnitudes: |y| + (1.5 * 2^15 + 0.5) added toward zero, in steps of 2^-8: the sum's floor is floor(|y| + 0.5) + 1.5 * 2^15, whose low
+// byte is the second one of the float's bits.  No clamp: every caller's scale is max(max|row| / 127, FLT_MIN) of the row the
 // product comes from, so |y| <= 127 (1 + 2^-22) and the floor never exceeds 127.  Signs: one byte of ones per negative
-// product (byte permutes that replicate the sign bit), then a bytewise two's-complement negation in five word
-// operations: x = n ^ s; low seven bits of x plus one where s is set cannot carry out of their byte.
+// product (byte permutes that replicate the sign bit), then a bytewise two's-complement negation: n ^ s; its low seven bits plus
+// one where s is set cannot carry out of their byte, and the eighth is that of s.
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t selector)
 {
     uint32_t d;
@@ -242,15 +242,20 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t select
 }
 __device__ __forceinline__ uint32_t quantize4(float y0, float y1, float y2, float y3)
 {
-    const uint32_t g0 = __float_as_uint(__fadd_rz(__fadd_rz(fabsf(y0), 0.5f), 12582912.0f));
-    const uint32_t g1 = __float_as_uint(__fadd_rz(__fadd_rz(fabsf(y1), 0.5f), 12582912.0f));
-    const uint32_t g2 = __float_as_uint(__fadd_rz(__fadd_rz(fabsf(y2), 0.5f), 12582912.0f));
-    const uint32_t g3 = __float_as_uint(__fadd_rz(__fadd_rz(fabsf(y3), 0.5f), 12582912.0f));
-    const uint32_t n = prmt(prmt(g0, g1, 0x0040u), prmt(g2, g3, 0x0040u), 0x5410u);
+    const uint32_t g0 = __float_as_uint(__fadd_rz(fabsf(y0), 49152.5f)), g1 = __float_as_uint(__fadd_rz(fabsf(y1), 49152.5f));
+    const uint32_t g2 = __float_as_uint(__fadd_rz(fabsf(y2), 49152.5f)), g3 = __float_as_uint(__fadd_rz(fabsf(y3), 49152.5f));
+    const uint32_t n = prmt(prmt(g0, g1, 0x0051u), prmt(g2, g3, 0x0051u), 0x5410u);
     // selector nibbles 0xB / 0xF: byte 3 of the first / second operand with its sign bit replicated
     const uint32_t sgn = prmt(prmt(__float_as_uint(y0), __float_as_uint(y1), 0x00FBu), prmt(__float_as_uint(y2), __float_as_uint(y3), 0x00FBu), 0x5410u);
-    const uint32_t x = n ^ sgn;
-    return (((x & 0x7F7F7F7Fu) + (sgn & 0x01010101u)) ^ (x & 0x80808080u));
+    return (((n ^ sgn) & 0x7F7F7F7Fu) + (sgn & 0x01010101u)) ^ (sgn & 0x80808080u);
+}
+// The products with a row's inverse scale, two at a time.
+__device__ __forceinline__ uint32_t quantize4_scaled(float a, float b, float c, float d, float inv)
+{
+    float y0, y1, y2, y3;
+    f2_unpack(f2_mul(f2_pack(a, b), f2_all(inv)), y0, y1);
+    f2_unpack(f2_mul(f2_pack(c, d), f2_all(inv)), y2, y3);
+    return quantize4(y0, y1, y2, y3);
 }
 // the unit that straddles K: elements at or beyond K are zero codes (out of line; the values travel as vector arguments
 // so that the caller's array stays in registers)
@@ -276,7 +281,7 @@ __device__ __forceinline__ uint4 quantize16(const float (&v)[16], float inv, int
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-        w[j] = quantize4(__fmul_rn(v[4 * j], inv), __fmul_rn(v[4 * j + 1], inv), __fmul_rn(v[4 * j + 2], inv), __fmul_rn(v[4 * j + 3], inv));
+        w[j] = quantize4_scaled(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], inv);
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 

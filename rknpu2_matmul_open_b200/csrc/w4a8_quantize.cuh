@@ -1,12 +1,11 @@
 // w4a8_quantize.cuh -- activation rows -> int8 codes in the Xq layout, for rows that allow 16-byte loads.
 //
-// Byte work: every element is read once and a code is written for it.  A CTA owns TG tokens (one or two, neighbours in their
-// token tile) and keeps what it has read in registers between the maximum and the codes; only what exceeds a thread's UN loads is
-// read a second time.  Lanes are dealt so that both sides move whole sectors: a warp's load covers 512 / TG contiguous bytes
-// of each token's row, and the store that follows puts the TG tokens' 16-byte units, which are neighbours in the layout,
-// side by side.  (One CTA per token with a thread per 16-element unit loaded every row twice, each load at a stride of 32 or
-// 64 bytes, and stored half sectors: 4096 x 14336 fp32 with known maxima 88-98 -> 60 us, 4096 x 4096 fp32 27 -> 21,
-// 128 x 11008 half 7.7 -> 5.8, 50 x 8192 fp32 6.8 -> 5.2, each with cold caches and a launch's own 2.5 us.)
+// Byte work: every element is read once and a code is written for it.  A CTA owns a token and keeps what it has read in registers
+// between the maximum and the codes; only what exceeds its threads' UN loads is read a second time.  A warp loads 512 neighbouring
+// bytes and stores the codes of the same elements, side by side where a token's codes are a row (T = 1).  What bounds a launch of
+// few tokens is latency: a trip to HBM, two barriers, and code that runs for the first time and is fetched from L2, so there is
+// little of it.  (With codes in groups of eight tokens two tokens a CTA were needed to store whole sectors, and eight CTAs wrote
+// into every line: 700 x 4096 binary16 -> 4096 22.7 -> 18.1 us with the GEMM behind it, 100 x 4096 13.4 -> 10.2.)
 #pragma once
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
@@ -15,86 +14,186 @@
 
 namespace rkb200 {
 
-template <bool HALF, int TG>
-struct QuantRows {
-    static constexpr int EPW = HALF ? 8 : 4;             // elements of a lane's 16 bytes
-    static constexpr int LPU = 16 / EPW;                 // lanes per 16-element unit
-    static constexpr int UPW = 32 / (LPU * TG);          // units of each token per warp and step
-};
+// Elements of a lane's 16 bytes.
+template <bool HALF> constexpr int PIECE = HALF ? 8 : 4;
 
-// UN: 16-byte loads a thread keeps.  Op: max_of(best, 16 bytes as loaded) -> best; begin(token, best) -> inverse scale, called by one thread per token, which
-// also writes the scales; word(y0..y3) -> four codes of products x * inverse.
-// SCAN false: the maxima are not needed (begin ignores its argument).
-template <bool HALF, int TG, bool SCAN, int UN, class Op>
-__device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int M, int K, int Kp, int T, Op& op)
+// Codes of eight binary16 values.
+template <class Word>
+__device__ __forceinline__ uint2 codes_of_halves(Word word, const uint4& r, float inv)
 {
-    using Q = QuantRows<HALF, TG>;
-    __shared__ uint32_t s_part[16][TG];
-    __shared__ float s_inverse[TG];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-    const int j = lane % Q::LPU, tg = lane / Q::LPU % TG, u = lane / (Q::LPU * TG);
-    const int m0 = blockIdx.x * TG, m = m0 + tg;
-    const bool mine = TG == 1 || m < M;
-    const uint4* const row = reinterpret_cast<const uint4*>(static_cast<const char*>(A) + (size_t)(mine ? m : m0) * K * (16 / Q::EPW));
-    const int pieces = K / Q::EPW;                       // 16-byte pieces of a row: K is a multiple of EPW
-    const int units = Kp / 16, step = warps * Q::UPW, first = warp * Q::UPW + u;
-    auto load = [&](int unit) {
-        const int piece = unit * Q::LPU + j;
-        return mine && piece < pieces ? __ldcg(row + piece) : make_uint4(0u, 0u, 0u, 0u);
-    };
+    float v[8];
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        v[2 * e] = __half2float(__ushort_as_half((uint16_t)(w[e] & 0xffffu)));
+        v[2 * e + 1] = __half2float(__ushort_as_half((uint16_t)(w[e] >> 16)));
+    }
+    return make_uint2(word(v[0], v[1], v[2], v[3], inv), word(v[4], v[5], v[6], v[7], inv));
+}
+
+// UN: 16-byte loads a thread keeps.  Op: max_of(best, 16 bytes as loaded) -> best; join(best, best) -> best, join_warp over a warp;
+// begin(token, best, one thread of the row's) -> inverse scale; the scales are written by that thread; word(x0..x3, inverse) -> four
+// codes.  SCAN false: the maxima are collected(token).
+template <bool HALF, bool SCAN, int UN, class Op>
+__device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int M, int K, int Kp, int T, Op op)
+{
+    constexpr int EPW = PIECE<HALF>, LPU = 16 / EPW;     // lanes per 16-element unit
+    __shared__ uint32_t s_part[16];
+    __shared__ float s_inverse;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x, m = blockIdx.x;
+    const uint4* const row = reinterpret_cast<const uint4*>(static_cast<const char*>(A) + (size_t)m * K * (16 / EPW));
+    const int pieces = K / EPW, padded = Kp / EPW;       // 16-byte pieces of a row: K is a multiple of EPW
+    auto load = [&](int piece) { return piece < pieces ? __ldcg(row + piece) : make_uint4(0u, 0u, 0u, 0u); };
     uint4 kept[UN];
     auto fill = [&](int from) {
 #pragma unroll
-        for (int i = 0; i < UN; ++i) kept[i] = load(from + i * step);
+        for (int i = 0; i < UN; ++i) kept[i] = load(from + i * threads);
     };
-    fill(first);
+    fill(tid);
     if (SCAN) {
         uint32_t best = 0;
 #pragma unroll
         for (int i = 0; i < UN; ++i) best = op.max_of(best, kept[i]);
-        for (int unit = first + UN * step; unit * Q::LPU < pieces; unit += step) best = op.max_of(best, load(unit));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            if (TG == 1 || (o != Q::LPU)) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-        if (lane % Q::LPU == 0 && lane < Q::LPU * TG) s_part[warp][tg] = best;
+        for (int piece = tid + UN * threads; piece < pieces; piece += threads) best = op.max_of(best, load(piece));
+        if constexpr (Op::CHECKS)
+            if (best >= Op::LEAST_BAD) {
+                best = 0;
+                for (int piece = tid; piece < pieces; piece += threads) best = op.max_checked(best, load(piece));
+            }
+        best = op.join_warp(best);
+        if (lane == 0) s_part[warp] = best;
         __syncthreads();
-        if (tid < TG && m0 + tid < M) {
+        if (tid == 0) {
             uint32_t all = 0;
-            for (int w = 0; w < warps; ++w) all = max(all, s_part[w][tid]);
-            s_inverse[tid] = op.begin(m0 + tid, all);
+            for (int w = 0; w < threads >> 5; ++w) all = op.join(all, s_part[w]);
+            s_inverse = op.begin(m, all, true);
         }
-    } else if (tid < TG && m0 + tid < M) s_inverse[tid] = op.begin(m0 + tid, 0u);
+    } else if (tid == 0) s_inverse = op.begin(m, op.collected(m), true);
     __syncthreads();
-    if (!mine) return;
-    const float inv = s_inverse[tg];
+    const float inv = s_inverse;
     const int mt = m / T, t = m - mt * T;
-    uint8_t* const dst = Xq + ((size_t)mt * units * T + t) * 16 + j * Q::EPW;
-    for (int from = first;;) {
+    uint8_t* const dst = Xq + ((size_t)mt * (Kp / 16) * T + t) * 16;
+    for (int from = tid;;) {
 #pragma unroll
         for (int i = 0; i < UN; ++i) {
-            const int unit = from + i * step;
-            if (unit < units) {
+            const int piece = from + i * threads;
+            if (piece < padded) {
                 const uint4 r = kept[i];
-                if constexpr (HALF) {
-                    float v[8];
-                    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        v[2 * e] = __half2float(__ushort_as_half((uint16_t)(w[e] & 0xffffu)));
-                        v[2 * e + 1] = __half2float(__ushort_as_half((uint16_t)(w[e] >> 16)));
-                    }
-                    *reinterpret_cast<uint2*>(dst + (size_t)unit * T * 16) = make_uint2(op.word(v[0], v[1], v[2], v[3], inv), op.word(v[4], v[5], v[6], v[7], inv));
-                } else {
-                    *reinterpret_cast<uint32_t*>(dst + (size_t)unit * T * 16) =
-                        op.word(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w), inv);
-                }
+                uint8_t* const to = dst + (uint32_t)(piece / LPU) * (T * 16u) + piece % LPU * EPW;
+                if constexpr (HALF) *reinterpret_cast<uint2*>(to) = codes_of_halves([&](float a, float b, float c, float d, float by) { return op.word(a, b, c, d, by); }, r, inv);
+                else *reinterpret_cast<uint32_t*>(to) = op.word(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w), inv);
             }
         }
-        from += UN * step;
-        if (from >= units) break;
+        from += UN * threads;
+        if (from >= padded) break;
         fill(from);
     }
 }
+
+// ---- what a row's maximum and its elements become: the W4A8 rule and the W8A8 one (the operators' definitions: w4a8_kernels.cu,
+// w8a8_kernels.cu)
+template <bool HALF>
+struct RowQuant {
+    float* scales;
+    const uint32_t* rowmax;      // collected maxima, or NULL: scanned
+    volatile int* bad_word;      // set where a row is rejected
+    static __device__ __forceinline__ uint32_t join(uint32_t a, uint32_t b) { return max(a, b); }
+    static __device__ __forceinline__ uint32_t join_warp(uint32_t a) { return __reduce_max_sync(0xffffffffu, a); }
+    static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r)
+    {
+        if constexpr (HALF) {
+            // pairs of magnitudes in one word: both halves order like unsigned 16-bit numbers
+            uint32_t m = __vmaxu2(__vmaxu2(r.x & 0x7fff7fffu, r.y & 0x7fff7fffu), __vmaxu2(r.z & 0x7fff7fffu, r.w & 0x7fff7fffu));
+            return max(best, max(m & 0xffffu, m >> 16));
+        }
+        return max(max(best, max(r.x & 0x7fffffffu, r.y & 0x7fffffffu)), max(r.z & 0x7fffffffu, r.w & 0x7fffffffu));
+    }
+    static constexpr bool CHECKS = false;
+    static constexpr uint32_t LEAST_BAD = 0xffffffffu;
+    // a row's maximum where it was collected and not scanned; the inverse of its scale (`store`: by one thread of the row's)
+    __device__ __forceinline__ uint32_t collected(int m) const { return __ldcg(rowmax + m); }
+    __device__ __forceinline__ float begin(int m, uint32_t bits, bool store = true) const
+    {
+        float maximum;
+        int bad;
+        if (HALF && !rowmax) {
+            bad = bits >= 0x7c00u ? 1 : 0;
+            maximum = __half2float(__ushort_as_half((uint16_t)bits));
+        } else {
+            bad = bits >= 0x7f800000u ? (rowmax ? 2 : 1) : 0;
+            maximum = __uint_as_float(bits);
+        }
+        float s, inv;
+        scale_from_max(maximum, bad != 0, s, inv);
+        if (store) {
+            scales[m] = s;
+            if (bad) *bad_word = bad;     // (the same value from every bad row of a launch)
+        }
+        return inv;
+    }
+    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
+    {
+        return quantize4_scaled(a, b, c, d, inv);
+    }
+};
+// round_half_away + clamp of one product; NaN gives +127 like the reference's min/max chain
+__device__ __forceinline__ int w8_code(float x, float inv)
+{
+    const float y = __fmul_rn(x, inv);
+    return (y != y) ? 127 : round_clamp(y);
+}
+
+// Scale (dynamic scan or the caller's), then codes in the Xq layout, for rows that allow 16-byte loads.
+template <bool HALF>
+struct W8RowQuant {
+    const float* static_scale;   // the caller's, or NULL: scanned
+    float* scales;
+    // Magnitude bits order like magnitudes; a NaN pattern (above infinity) never raises the maximum.  The top bit says that there is a
+    // NaN or an infinity among them.
+    static constexpr uint32_t CAREFUL = 0x80000000u, INF = HALF ? 0x7c00u : 0x7f800000u;
+    static __device__ __forceinline__ uint32_t join(uint32_t a, uint32_t b) { return max(a & ~CAREFUL, b & ~CAREFUL) | ((a | b) & CAREFUL); }
+    static __device__ __forceinline__ uint32_t join_warp(uint32_t a) { return __reduce_max_sync(0xffffffffu, a & ~CAREFUL) | (__any_sync(0xffffffffu, (a & CAREFUL) != 0) ? CAREFUL : 0u); }
+    static constexpr bool CHECKS = true;
+    static constexpr uint32_t LEAST_BAD = INF;
+    static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r) { return RowQuant<HALF>::max_of(best, r); }
+    // for a thread whose maximum is LEAST_BAD or more: its pieces once more
+    static __device__ __forceinline__ uint32_t max_checked(uint32_t best, const uint4& r)
+    {
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t a = w[i] & (HALF ? 0x7fffu : 0x7fffffffu), b = HALF ? (w[i] >> 16) & 0x7fffu : 0u;
+            if (a <= INF) best = join(best, a);
+            if (HALF && b <= INF) best = join(best, b);
+        }
+        return best | CAREFUL;
+    }
+    __device__ __forceinline__ uint32_t collected(int) const { return 0u; }
+    // The sign of the inverse says how its row is rounded: positive, no product is a NaN or rounds beyond 127 (the scale is that of
+    // the row, and normal), as in the W4A8 rule; negative, with the checks; a NaN: the scale is not positive (an underflowed maximum),
+    // the codes are zeros.
+    __device__ __forceinline__ float begin(int m, uint32_t bits, bool store = true) const
+    {
+        float s;
+        const uint32_t magnitude = bits & ~CAREFUL;
+        if (static_scale) s = static_scale[m];
+        else {
+            const float maximum = HALF ? __half2float(__ushort_as_half((uint16_t)magnitude)) : __uint_as_float(magnitude);
+            s = maximum > 0.f ? __fdiv_rn(maximum, 127.0f) : 1.0f;
+        }
+        if (store) scales[m] = s;
+        if (!(s > 0.f)) return __int_as_float(0x7fffffff);
+        const float inv = __frcp_rn(s);
+        return static_scale || (bits & CAREFUL) || s < FLT_MIN ? -inv : inv;
+    }
+    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
+    {
+        if (inv > 0.f) return quantize4_scaled(a, b, c, d, inv);
+        if (inv != inv) return 0u;
+        return __byte_perm(__byte_perm((uint32_t)w8_code(a, -inv), (uint32_t)w8_code(b, -inv), 0x0040),
+                           __byte_perm((uint32_t)w8_code(c, -inv), (uint32_t)w8_code(d, -inv), 0x0040), 0x5410);
+    }
+};
 
 // Rows that do not allow 16-byte loads: a warp takes 512 elements at a time, a lane element 32 i + lane, so that every load
 // covers neighbouring elements, and hands them to the lane whose 16-element unit they belong to through shared memory, a word
@@ -127,43 +226,27 @@ __device__ __forceinline__ void exchange_piece(uint32_t* words, int lane, const 
 
 // 16-byte loads are possible for every row.
 template <bool HALF>
-inline bool quantize_rows_ok(const void* A, int K) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % QuantRows<HALF, 1>::EPW == 0; }
-// Calls f with the shape of the launch: <tokens per CTA, threads, loads a thread keeps>.
-// Rows that are scanned.  Up to 296 tokens (two CTAs of 512 threads an SM, all resident) a token per CTA, and all the
-// threads that help with a row work on it.  Up to 591 these CTAs would come in two waves: 256 threads (in front of 4096
-// channels 448 x 1024 binary16 13.8 -> 12.1 us, 448 x 4096 fp32 18.4 -> 16.9), but not for long fp32 rows, whose CTAs take
-// twice as long then (300 x 11008 -> 4096 28.0 us, 29.5 with 256; FFN of 400 x 8192 54.7 and 56.7). From 592 tokens on
-// binary16 rows of up to 4096 elements take 128 threads with two loads and 32 registers, sixteen CTAs an SM (in front of
-// 4096 channels 3000 x 1024 32.2 -> 28.8 us, 1024 x 4096 27.3 -> 25.8); the others two tokens per CTA, which make whole
-// sectors of codes (6144 and 8192 binary16 -6 to -10 % against a token per CTA).  (The two fp32 forms of eight loads and two
-// tokens spill six words.)
-// Rows whose maxima are known: two tokens per CTA, up to 591 tokens of 512 threads (FFN of 64 x 1024 -> 2 x 2048 24.2 ->
-// 21.6 us, of 591 x 4096 -> 2 x 14336 116 -> 103), beyond of 256 with 32 registers (4096 x 14336 fp32 60 us, 70 with twice
-// the registers).  Few long rows want a CTA each (20 x 11008 40.3 us against 42.3,
-// 20 x 4096 26.8 against 27.6).
+inline bool quantize_rows_ok(const void* A, int K) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % PIECE<HALF> == 0; }
+// Calls f with the shape of the launch: <threads, loads a thread keeps>, a CTA for each token.  The threads' loads just hold the row,
+// as far as they go.  Up to 591 tokens (four a SM) all CTAs are resident anyway and half the loads on twice the threads are faster
+// (with the GEMM behind it, 256 x 8 loads against 512 x 4: 300 x 8192 fp32 21.7 -> 21.0 us; 512 x 8 against 128 x 4: 200 x 1024
+// binary16 11.6 -> 9.7, 400 x 2048 fp32 11.0 -> 9.7).  Beyond, CTAs in line behind each other: fewer threads a row, more of the row
+// each (2000 x 4096 fp32 256 x 4 23.1, 128 x 8 22.6; 3000 x 8192 fp32 512 x 4 50.9, 256 x 8 47.6, 128 x 8 54.1; 3000 x 11008
+// binary16 50.1, 47.9 and 50.5).  Short rows: 128 x 4 (2048 x 4096 binary16 18.1 us, 128 x 8 18.6; 700 x 2048 fp32 10.1 and 11.1),
+// but many with known maxima, which have less to wait for, 128 x 8 (FFN of 1000 x 2048 28.5 -> 27.6).
 template <bool HALF, bool SCAN, class F>
 inline auto with_quantize_rows_shape(int M, int K, F f)
 {
-    constexpr int EPW = QuantRows<HALF, 1>::EPW;
     using std::integral_constant;
-    using I1 = integral_constant<int, 1>;
-    using I2 = integral_constant<int, 2>;
     using I4 = integral_constant<int, 4>;
     using I8 = integral_constant<int, 8>;
     using B128 = integral_constant<int, 128>;
     using B256 = integral_constant<int, 256>;
     using B512 = integral_constant<int, 512>;
-    if constexpr (!SCAN) {
-        if (M >= 592) return f(I2{}, B256{}, I4{});
-        return (M <= 296 && K > 8192) || (M < 24 && K >= 4096) ? f(I1{}, B512{}, I8{}) : f(I2{}, B512{}, I8{});
-    } else {
-        if (M <= 296) return f(I1{}, B512{}, I8{});
-        if (M < 592) return HALF || K < 8192 ? f(I1{}, B256{}, I8{}) : f(I1{}, B512{}, I8{});
-        if constexpr (HALF) {
-            if (K <= 4096) return f(I1{}, B128{}, I2{});
-        } else if (K <= 2048) return f(I2{}, B256{}, I4{});
-        return K <= 256 * 8 * EPW / 2 ? f(I2{}, B256{}, I8{}) : f(I2{}, B512{}, I8{});
-    }
+    const int bytes = K * (16 / PIECE<HALF>);
+    if (bytes <= 8192 && (SCAN || M < 592)) return f(B128{}, I4{});
+    if (M < 592) return bytes <= 16384 ? f(B256{}, I4{}) : f(B512{}, I4{});
+    return bytes <= 16384 ? f(B128{}, I8{}) : f(B256{}, I8{});
 }
 
 } // namespace rkb200

@@ -85,7 +85,6 @@ __global__ void __launch_bounds__(256, 8) codes_in_kernel(const CodesInParams p)
         const float s = scale_from_bits(p.rowmax[m], bad);
         p.rowmax[m] = 0u;   // consumed: the next SwiGLU epilogue maxes into a clean word
         p.scales[m] = s;
-        p.inverse[m] = __fdiv_rn(1.0f, s);
         if (bad) p.status->bad_accum = bad;     // (the same value from every bad row of a launch)
     }
 }

@@ -290,6 +290,7 @@ int run(rk_npu_matmul_workspace* ws, const W8Weights* w, int kind, const void* A
     if (!c_dev) cudaMemcpyAsync(C, dC, ws->stage_out_bytes, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
     if (ws->host_status->device_error) {       // a bounded wait inside the kernel ran out: report, clear, stay usable
+        cudaMemsetAsync(ws->status, 0, sizeof(Status), s);
         if (ws->counts) cudaMemsetAsync(ws->counts, 0, ws->counts_bytes, s);
         cudaStreamSynchronize(s);
         return RK_NPU_ERR_SUBMIT;

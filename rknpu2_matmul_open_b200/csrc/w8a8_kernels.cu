@@ -53,55 +53,11 @@ cudaError_t launch_w8_pack_weights(const W8PackParams& p, cudaStream_t stream)
     return cudaGetLastError();
 }
 
-// round_half_away + clamp of one product; NaN gives +127 like the reference's min/max chain
-__device__ __forceinline__ int w8_code(float x, float inv)
-{
-    const float y = __fmul_rn(x, inv);
-    return (y != y) ? 127 : round_clamp(y);
-}
-
-// Scale (dynamic scan or the caller's), then codes in the Xq layout, for rows that allow 16-byte loads.
-template <bool HALF>
-struct W8RowQuant {
-    const W8QuantParams& p;
-    static __device__ __forceinline__ uint32_t max_of(uint32_t best, const uint4& r)
-    {
-        // magnitude bits order like magnitudes; a NaN pattern (above infinity) never raises the maximum
-        constexpr uint32_t INF = HALF ? 0x7c00u : 0x7f800000u;
-        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t a = w[i] & (HALF ? 0x7fffu : 0x7fffffffu), b = HALF ? (w[i] >> 16) & 0x7fffu : 0u;
-            if (a <= INF) best = max(best, a);
-            if (HALF && b <= INF) best = max(best, b);
-        }
-        return best;
-    }
-    // (a negative inverse marks a row whose scale is not positive -- an underflowed maximum: its codes are zeros)
-    __device__ __forceinline__ float begin(int m, uint32_t bits)
-    {
-        float s;
-        if (p.static_scale) s = p.static_scale[m];
-        else {
-            const float maximum = HALF ? __half2float(__ushort_as_half((uint16_t)bits)) : __uint_as_float(bits);
-            s = maximum > 0.f ? __fdiv_rn(maximum, 127.0f) : 1.0f;
-        }
-        p.scales[m] = s;
-        return s > 0.f ? __fdiv_rn(1.0f, s) : -1.f;
-    }
-    __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
-    {
-        if (inv < 0.f) return 0u;
-        return __byte_perm(__byte_perm((uint32_t)w8_code(a, inv), (uint32_t)w8_code(b, inv), 0x0040),
-                           __byte_perm((uint32_t)w8_code(c, inv), (uint32_t)w8_code(d, inv), 0x0040), 0x5410);
-    }
-};
-template <bool HALF, int TG, bool SCAN, int BS, int UN>
-__global__ void __launch_bounds__(BS, (UN <= 4 ? 2048 : 1024) / BS) w8_quantize_rows_kernel(const W8QuantParams p)
+template <bool HALF, bool SCAN, int BS, int UN>
+__global__ void __launch_bounds__(BS, (UN <= 4 ? 1280 : 896) / BS) w8_quantize_rows_kernel(const W8QuantParams p)
 {
     pdl_launch_dependents();   // the GEMM behind this kernel may set itself up and request its weights
-    W8RowQuant<HALF> op{p};
-    quantize_rows<HALF, TG, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, op);
+    quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, W8RowQuant<HALF>{p.static_scale, p.scales});
 }
 
 // The same for any row: one CTA per token.
@@ -208,9 +164,9 @@ static void launch_w8_rows(const W8QuantParams& p, cudaStream_t stream)
         w8_quantize_kernel<HALF><<<(unsigned)p.M, 256, 0, stream>>>(p);
         return;
     }
-    with_quantize_rows_shape<HALF, SCAN>(p.M, p.K, [&](auto tg, auto bs, auto un) {
-        constexpr int TG = decltype(tg)::value, BS = decltype(bs)::value, UN = decltype(un)::value;
-        w8_quantize_rows_kernel<HALF, TG, SCAN, BS, UN><<<(unsigned)((p.M + TG - 1) / TG), BS, 0, stream>>>(p);
+    with_quantize_rows_shape<HALF, SCAN>(p.M, p.K, [&](auto bs, auto un) {
+        constexpr int BS = decltype(bs)::value, UN = decltype(un)::value;
+        w8_quantize_rows_kernel<HALF, SCAN, BS, UN><<<(unsigned)p.M, BS, 0, stream>>>(p);
     });
 }
 

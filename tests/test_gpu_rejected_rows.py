@@ -1,0 +1,50 @@
+"""A row with NaN or Inf rejects its call and no other: good and bad calls back to back on one workspace, without a wait between
+them, for the kernels that run behind a quantise launch.  Good outputs bit for bit, outputs of bad calls untouched."""
+import numpy as np
+import pytest
+import torch
+
+import rknpu2_matmul_open_b200 as rk
+from conftest import bits
+from rknpu2_matmul_open_b200 import capi
+from rknpu2_matmul_open_b200.synthetic import make_activations, make_weights
+
+pytestmark = pytest.mark.gpu
+
+# kernel family, cut of the persistent kernel (items of one width, K in parts, runs of several items), tokens, K, N
+CASES = [(1, None, 12, 1032, 260), (1, None, 40, 2048, 200), (4, None, 24, 1024, 300), (2, "32,1,0,1", 40, 640, 700), (2, "64,1,0,3", 129, 2048, 512),
+         (2, "32,5,2,1", 700, 384, 1300), (2, None, 600, 4104, 256)]
+
+
+@pytest.mark.parametrize("family, cut, M, K, N", CASES)
+def test_good_and_bad_calls_in_turn(gpu, oracle, monkeypatch, family, cut, M, K, N):
+    _, dom, _ = gpu
+    monkeypatch.setenv("RK_NPU_B200_VARIANT", str(family))
+    if cut:
+        monkeypatch.setenv("RK_NPU_B200_PERSIST_CUT", cut)
+    B, sw = make_weights(K, N, seed=K)
+    w, ws = rk.Weights(dom, B, sw), rk.Workspace(dom, rk.default_config(M, N, K))
+    good = make_activations(M, K, seed=M, dtype="f32")
+    _, ref, _, _ = oracle.linear(good, B, sw)
+    one, every = good.copy(), good.copy()
+    one[M - 1, K - 1] = np.nan
+    every[:, 3] = np.inf
+    a = {"good": torch.from_numpy(good).cuda(), "one": torch.from_numpy(one).cuda(), "every": torch.from_numpy(every).cuda()}
+    turns = ["good", "one", "good", "good", "every", "one", "good", "every"]
+    outs = [torch.full((M, N), -7.0, device="cuda") for _ in turns]
+    stream = torch.cuda.current_stream().cuda_stream
+    for kind, out in zip(turns, outs):
+        assert ws.enqueue_f32(w, a[kind], out, stream) == 0
+    torch.cuda.synchronize()
+    for i, (kind, out) in enumerate(zip(turns, outs)):
+        got = out.cpu().numpy()
+        assert np.array_equal(bits(got), bits(ref)) if kind == "good" else np.all(got == -7.0), (i, kind)
+    assert ws.finish() == capi.RK_NPU_ERR_PARAM
+    host = np.full((M, N), -7.0, np.float32)
+    assert ws.run_f32(w, every, host) == capi.RK_NPU_ERR_PARAM
+    assert ws.run_f32(w, good, host) == 0 and np.array_equal(bits(host), bits(ref))
+    assert ws.enqueue_f32(w, a["good"], outs[1], stream) == 0
+    torch.cuda.synchronize()
+    assert ws.finish() == 0 and np.array_equal(bits(outs[1].cpu().numpy()), bits(ref))
+    ws.free()
+    w.free()
