@@ -583,9 +583,9 @@ __global__ void __launch_bounds__(PsShape<W8, TOK>::THREADS, 1) gemm_tc_persist_
                     for (int i = 0; i < 4; ++i)
                         __stcg(slot + (size_t)(STEP / 4 * k + i) * 128, make_int4((int)r[4 * i], (int)r[4 * i + 1], (int)r[4 * i + 2], (int)r[4 * i + 3]));
                 }
-                __threadfence();
                 asm volatile("bar.sync 1, %0;" ::"n"(32 * PS_EPI_WARPS) : "memory");
                 if (sid == 0) {
+                    __threadfence();                          // (for all of the warps' stores, behind the barrier)
                     // (a tile with a part whose wait ran out is never completed; the launch reports the error and the host
                     // clears the counters)
                     unsigned* const count = p.counts + 2 * tile_index + rank;

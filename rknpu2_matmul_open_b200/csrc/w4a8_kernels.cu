@@ -435,7 +435,11 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
             }
         }
     }
-    if (S > 1) cluster.sync();   // nobody leaves while a peer may still read its partials
+    if (S > 1) {                 // nobody leaves while a peer may still read its partials (what was read is here: no memory to order)
+        __syncwarp();
+        cluster_arrive_relaxed();
+        cluster_wait();
+    }
 }
 
 template <int NT, bool BIGK>
