@@ -356,11 +356,17 @@ int fused_tiles_per_cta(const rk_npu_w4a8_workspace& ws, int tiles, int split, i
     return all > half_gpu ? 2 : 1;
 }
 
-// The family that runs a call: the workspace's, or the ring where that is the faster for these rows (its code layout is the
-// same).  Results that go over the bus stay with the single launch, which stores them in whole rows.
+// The family that runs a call: the workspace's, or another with the same code layout where that is the faster for these rows.
+// Results that go over the bus stay with the workspace's, which stores them in whole rows.
 int family_of(const rk_npu_w4a8_workspace& ws, const Call& c)
 {
-    return ws.mid_batch && c.epi != EPI_SWIGLU && !c.rowmax_in && !c.over_bus && mid_batch_takes_ring(ws.config.M, ws.config.K, c.half) ? 1 : ws.variant;
+    const auto& cfg = ws.config;
+    if (!ws.by_rule || ws.split_override || c.over_bus || c.codes_in || c.keep_codes || (ws.variant != 3 && ws.variant != 5)) return ws.variant;
+    if (cfg.M > 8) return mid_batch_call_takes_ring(cfg.M, cfg.K, ws.shard_N, c.half, c.rowmax_in) ? 1 : 3;
+    const bool ffn = c.rowmax_in || c.epi == EPI_SWIGLU;
+    const int family = ffn ? few_tokens_ffn(ws.variant, cfg.M, cfg.K, ws.shard_N, c.rowmax_in) : few_tokens_linear(ws.variant, cfg.M, cfg.K, ws.shard_N, c.half);
+    if (family == 5 && ws.decode_cap[0] < 1) return ws.variant;
+    return family == 3 && ws.KB > 8 * FUSED_MAX_STAGES ? 1 : family;
 }
 
 // Launch parameters of the decode kernel for one call (its workspace runs that family).
@@ -384,7 +390,7 @@ void decode_params(const Call& c, DecodeParams& d, int cluster_override = 0)
     d.M = cfg.M; d.N = N; d.K = cfg.K;
     d.KB = ws.KB; d.NG = c.w->NG; d.F = F; d.epi = c.epi;
     d.half = c.half ? 1 : 0;
-    d.cluster = cluster_override ? cluster_override : ws.split_override ? ws.split_override : gemm_decode_cluster(cfg.M, ws.KB);
+    d.cluster = cluster_override ? cluster_override : ws.split_override ? ws.split_override : gemm_decode_cluster(cfg.M, ws.KB, c.half);
     d.ring = gemm_decode_ring(cfg.M, ws.KB, swiglu);
     const int slot = d.cluster == 1 ? 0 : d.cluster == 2 ? 1 : d.cluster == 4 ? 2 : 3;
     d.ctas = gemm_decode_ctas(swiglu ? F / GROUP : (N + GROUP - 1) / GROUP, d.cluster, ws.decode_cap[slot]);
@@ -1146,21 +1152,21 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     // and partial sums (8 tokens: 1479 against 1669 GB/s), so the split-K kernel keeps those where it applies.
     const bool decode_ok = gemm_decode_supported(cfg->M, cfg->K);
     const bool decode_best = decode_ok && (cfg->M <= 4 || !fused_best);
-    // 9..16 tokens: one launch (the split-K kernel) beats two (the ring) while the weights are small (16 tokens, 4096 ->
-    // 4096 9.6 against 10.0 us, 8192 -> 1024 8.5 against 10.6, 11008 -> 4096 17.2 against 14.1); not for all rows, see
-    // mid_batch_takes_ring.
+    // 9..16 tokens: the split-K kernel's single launch while the weights are small, where results go over the bus; which calls take
+    // the ring all the same: mid_batch_call_takes_ring.
     const bool fused_mid = fused_ok && cfg->M > 8 && cfg->M <= 16 && (long long)cfg->K * local_N / 2 <= (8ll << 20);
     // From 17 tokens on the persistent tcgen05 kernel, whose time hardly depends on the batch up to 64 (4096 -> 4096 13 us,
     // 11008 -> 4096 19, 4096 -> 14336 14.5), unless its 256-channel tiles are so few that the ring's small CTAs cover more
     // of the GPU (24 tokens: 2048 -> 2048 9.3 us, 3840 -> 3840 10.4 against 12.1, but 16.4 / 24 / 17.1 us on the three
-    // shapes above).
+    // shapes above).  From nine tokens where its tiles just fit the GPU's SM pairs: 12 x 2048 -> 2 x 5632 and back 15.8 us against
+    // 16.7, 12 x 4096 -> 11008 10.1 against 11.2; with more tiles a second round costs more than the ring's small CTAs.
     const int channel_tiles = (local_N + 255) / 256;
-    const bool pair_best = tc_ok && (cfg->M > 96 || (cfg->M > 32 && channel_tiles > 4) || (cfg->M > 16 && channel_tiles > 15));
+    const bool pair_best = tc_ok && (cfg->M > 96 || (cfg->M > 32 && channel_tiles > 4) || (cfg->M > 16 && channel_tiles > 15) || (cfg->M > 8 && channel_tiles > 40 && channel_tiles <= 64));
     int variant = decode_best ? 5 : pair_best ? 2 : (fused_best || fused_mid) ? 3 : 1;
     if (forced == 1 || (forced == 2 && tc_ok) || (forced == 3 && fused_ok) || (forced == 4 && stream_ok) || (forced == 5 && decode_ok))
         variant = forced;
     ws->variant = variant;
-    ws->mid_batch = variant == 3 && forced != 3 && fused_mid;
+    ws->by_rule = !forced;
     if (const char* e = std::getenv("RK_NPU_B200_TILES_PER_CTA")) {   // experiments and tests: 1 or 2, else automatic
         const int v = std::atoi(e);
         ws->tiles_per_cta_override = (v == 1 || v == 2) ? v : 0;
@@ -1396,7 +1402,7 @@ extern "C" int rk_npu_b200_w4a8_enqueue_batch_f16(int count, rk_npu_w4a8_workspa
     }
     // one cluster size for the launch: the one the longest reduction asks for
     int cluster = 1;
-    for (int i = 0; i < count; ++i) cluster = std::max(cluster, gemm_decode_cluster(workspaces[i]->config.M, workspaces[i]->KB));
+    for (int i = 0; i < count; ++i) cluster = std::max(cluster, gemm_decode_cluster(workspaces[i]->config.M, workspaces[i]->KB, true));
     std::unique_ptr<WorkspaceLock> locks[DEC_MAX_BATCH];
     for (int i = 0; i < count; ++i) {
         locks[i].reset(new WorkspaceLock(*workspaces[i]));
@@ -1602,7 +1608,7 @@ extern "C" int rk_npu_b200_w4a8_set_schedule(rk_npu_w4a8_workspace* ws, int vari
     if (!lock) return RK_NPU_ERR_BUSY;
     ws->variant = target;
     ws->split_override = split_k;
-    if (variant) ws->mid_batch = false;      // asked for by name
+    if (variant) ws->by_rule = false;        // asked for by name
     return RK_NPU_OK;
 }
 extern "C" int rk_npu_b200_w4a8_schedule(const rk_npu_w4a8_workspace* ws, int* variant, int* split_k)

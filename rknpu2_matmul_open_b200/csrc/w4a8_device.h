@@ -278,7 +278,7 @@ constexpr int DEC_MAX_RING = 12;
 bool gemm_decode_supported(int M, int K);
 size_t gemm_decode_smem_bytes(int M, int KB, bool swiglu, int ring);
 int gemm_decode_ring(int M, int KB, bool swiglu);
-int gemm_decode_cluster(int M, int KB);
+int gemm_decode_cluster(int M, int KB, bool half);
 int gemm_decode_ctas(int items, int cluster, int cap);
 int gemm_decode_resident_ctas(int cluster, size_t smem, int sm_count);
 cudaError_t launch_gemm_decode(const DecodeParams& p, cudaStream_t stream, bool pdl);

@@ -128,7 +128,7 @@ struct rk_npu_w4a8_workspace {
     int variant = 0, split_override = 0;   // variant: 1 quantise + mma.sync GEMM, 2 quantise + tcgen05 GEMM, 3 fused small batch
                                            // (split-K clusters), 4 quantise + persistent streaming GEMM (small batch, large
                                            // weights), 5 single-kernel decode (whole-K CTAs, up to eight tokens)
-    bool mid_batch = false;                // 9..16 tokens, family 3 by the library's own choice: linear calls may take 1 (mid_batch_takes_ring)
+    bool by_rule = false;                  // the variant is the library's own choice: a call may take another for its rows (family_of)
     int decode_cap[4] = {0, 0, 0, 0};      // variant 5: CTAs resident at once for cluster sizes 1, 2, 4, 8
     bool starve = false;                   // test hook (rk_npu_b200_w4a8_test_starve): first weight barrier never completes
     // device buffers

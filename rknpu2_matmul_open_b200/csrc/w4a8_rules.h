@@ -26,18 +26,73 @@ inline bool result_over_bus(int family, int M, size_t cols, size_t elem)
     return bytes <= (elem == 2 ? size_t(40) << 10 : size_t(64) << 10);
 }
 
-// 9..16 tokens of small weights: whether one launch (the split-K kernel, whose every cluster scans all of the rows) is left for
-// two (quantise, ring).  For binary16 rows that allow 16-byte loads one launch is the faster at every count (16 tokens, 4096 ->
-// 4096 10.2 us against 11.0, 4096 -> 1024 8.4 against 9.5, 1024 -> 14336 9.6 against 9.9; at worst 5504 -> 2112 10.7 against
-// 10.2).  fp32 rows are twice the scan: 13 tokens and more take two (13 tokens 2048 -> 2048 9.3 against 8.7, 4096 -> 4096 11.7
-// against 10.4, 16 tokens 2048 -> 8192 12.3 against 9.7; 12 tokens 8.8 against 8.7, 4096 -> 1024 8.4 against 9.3).  Rows that
-// are loaded element by element sooner still: binary16 from 11 tokens (10 tokens 1500 -> 2048 7.9 against 9.5, 2044 -> 4096
-// 11.6 against 11.0; 12 tokens 3070 -> 4911 13.1 against 11.5, 16 tokens 15.9 against 11.7), fp32 from 9 (3070 -> 4911 16.6
-// against 12.1, 1025 -> 1024 11.5 against 9.6).
+// Up to eight tokens: the family that runs a call of a workspace of family 3 (split-K clusters) or 5 (decode); the code layout is the
+// ring's (1) too.  Measured on 33 shapes of both types, the times are of one call of a back-to-back series in us, decode / clusters /
+// ring.  The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3
+// at least: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32 7.8 / 7.9 / 6.5,
+// 4 x 8192 -> 8192 13 / 12.6 / 10.6, 8 x 3070 -> 4911 10.3 / 13.2 / 7.6).  The decode kernel's CTAs take 32 channels over all of K:
+// best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2), poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.4 / 7.2) and
+// where some CTAs have two groups of channels (4 x 5120 -> 5120 9.0 / 7.0 / 7.9).
+inline int few_tokens_linear(int family, int M, int K, int columns, bool half)
+{
+    const double mb = double(K) * columns / 2 / (1 << 20);          // of weights
+    const bool ragged = K % (half ? 8 : 4) != 0;
+    const int groups = (columns + 31) / 32;
+    if (M > 4) {
+        if (K <= 3072 && mb <= 4.5) return 5;
+        if (ragged) return 1;
+        // 8 x 3072 -> 8192 9.0 / 7.1 / 7.0, 2048 -> 14336 8.8 / 9.7 / 7.3; 4096 -> 11008 is a tie alone, and in a chain of dependent
+        // calls the clusters' by 0.7
+        if (half) return mb <= 13.25 || (mb > 20 && K <= 4096) ? family : 1;
+        if (columns <= 1024 || (K >= 8192 && columns <= 2112 && M <= 6)) return 3;
+        return M <= 6 && groups > 144 && groups <= 192 ? 3 : 1;
+    }
+    if (columns <= 2112 && (K >= 8192 || (K >= 6144 && (M > 1 || !half)))) return 3;
+    if (groups > 144 && groups <= 240 && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
+    if (!half && groups > 144 && groups <= 296 && M > 2 && K >= 3072 && mb < 14) return 3;   // 4 x 3072 -> 8192 7.7 / 6.6 / 6.9
+    if (K <= 1024 && groups > 296) return 3;                         // 4 x 1024 -> 14336 6.1 / 5.6 / 6.3
+    if (ragged && M == 4 && mb > 4) return 1;
+    // (in a chain 4 x 4096 -> 11008 takes the decode kernel 0.9 less than the ring)
+    if (mb >= 14 && ((M > 2 && K <= 8192 && (mb >= 26 || K >= 6144)) || (M == 2 && K >= (half ? 8192 : 4096)) || (M < 3 && mb >= 40))) return 1;
+    return family;
+}
+
+// The same for the two projections of an FFN (times of the whole FFN).  The first's columns come in pairs and its quantising is fp32
+// (2048 -> 2 x 14336, 4 tokens: 22.9 / - / 17.9); the second finds its rows' maxima collected, so no kernel scans (14336 -> 1024
+// behind it 19.9 / 17.9 / 19.6, 5632 -> 2048 at 4 tokens 16.1 / 14.9 / 15.0).
+inline int few_tokens_ffn(int family, int M, int K, int columns, bool second)
+{
+    const double mb = double(K) * columns / 2 / (1 << 20);
+    if (second) {
+        if (M <= 4) return columns <= 2112 && K >= 5120 ? 3 : family;
+        if (mb <= 2) return 5;
+        return columns <= 2112 && K <= 6144 ? 1 : family;
+    }
+    if (K <= 2048 && columns > 2 * 148 * 32) return columns < 16384 && M <= 4 ? 3 : 1;
+    if (K % 4 && M >= 4) return 1;
+    if (M <= 2 && mb >= 50 && (M == 2 || K >= 8192)) return 1;       // 1 x 8192 -> 2 x 7168 27.6 / - / 25.1
+    if (M <= 4) return family;
+    return K >= 8192 && mb <= 26 ? 1 : 5;
+}
+
+// 9..16 tokens of very small weights: whether one launch (the split-K kernel, whose every cluster scans all of the rows) is left for
+// two (quantise, ring): fp32 rows are twice the scan, rows that are loaded element by element sooner still.
 inline bool mid_batch_takes_ring(int M, int K, bool half)
 {
     const bool wide = K % 8 == 0;
     return half ? !wide && M > 10 : M > (wide ? 12 : 8);
+}
+
+// 9..16 tokens of a workspace of family 3: whether a call takes two launches (quantise, ring) instead of the split-K kernel, whose
+// every cluster scans all of the rows.  Always but for weights of 256 KB, where a launch is most of the work, and unless the rows'
+// maxima are there already and the channels many (4096 -> 4096 behind a first projection: the FFN 19.4 us with one launch, 20.3 with
+// two; 4096 -> 2048 16.9 and 14.6).  16 tokens binary16, 1024 -> 1024 7.6 us with one and 6.5 with two, 4096 -> 4096 9.8 and 7.5;
+// fp32 2048 -> 8192 12.2 and 6.6.
+inline bool mid_batch_call_takes_ring(int M, int K, int columns, bool half, bool maxima_collected)
+{
+    const bool long_rows = columns <= 1024 && K > 8192 && M <= 12;   // 10 x 11008 -> 1024 fp32 9.3 us with one, 9.8 with two
+    if (maxima_collected) return columns <= 2112 && !long_rows;
+    return (!long_rows && (long long)K * columns / 2 > (256ll << 10)) || mid_batch_takes_ring(M, K, half);
 }
 
 } // namespace rkb200

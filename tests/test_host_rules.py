@@ -238,3 +238,39 @@ int main()
     return of_one_width.size() == 8 && of_runs.size() == 8 && inside ? 0 : 4;
 }
 """.replace("CUTS", ", ".join(cuts)))
+
+
+def test_families_for_few_tokens(tmp_path):
+    # sizes at which the three families were measured, within 7 % of the fastest; every answer is a family that shares the layout
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+struct Case { int M, K, cols; bool half; int family; };
+int main()
+{
+    const Case cases[] = {
+        {1, 4096, 4096, true, 5}, {1, 1024, 14336, true, 3}, {1, 11008, 2048, true, 3}, {2, 4096, 6144, true, 5}, {2, 5120, 5120, false, 3},
+        {2, 8192, 8192, false, 1}, {3, 11008, 8192, true, 5}, {4, 8192, 2048, false, 3}, {4, 4096, 6144, true, 3}, {4, 8192, 8192, true, 1},
+        {4, 3070, 4911, true, 1}, {4, 4096, 4096, false, 5}, {4, 5120, 13824, false, 1}, {5, 2048, 4096, true, 5}, {5, 5120, 5120, false, 3},
+        {8, 2048, 2048, false, 5}, {8, 4096, 4096, true, 3}, {8, 4096, 4096, false, 1}, {8, 2048, 14336, true, 1}, {8, 4096, 11008, true, 3}, {4, 4096, 11008, true, 5}, {4, 2048, 5632, true, 5}, {8, 3070, 4911, false, 1},
+        {8, 8192, 1024, false, 3}, {8, 8192, 2048, false, 1}, {6, 8192, 2048, false, 3}, {5, 1500, 2048, true, 5}, {8, 1500, 2048, true, 5}, {3, 3072, 8192, false, 3}, {4, 11008, 8192, false, 5},
+    };
+    for (const Case& c : cases) {
+        const int from = c.M <= 4 || (long long)c.K * c.cols / 2 > (24 << 20) ? 5 : 3;
+        if (few_tokens_linear(from, c.M, c.K, c.cols, c.half) != c.family) { printf("%d x %d -> %d half %d\n", c.M, c.K, c.cols, c.half); return 1; }
+    }
+    for (int M = 1; M <= 8; ++M)
+        for (int K = 1; K < 20000; K += 37)
+            for (int cols = 1; cols < 40000; cols += 401)
+                for (int bit = 0; bit < 2; ++bit)
+                    for (int from = 3; from <= 5; from += 2) {
+                        const int f[2] = {few_tokens_linear(from, M, K, cols, bit), few_tokens_ffn(from, M, K, cols, bit)};
+                        for (int x : f) if (x != 1 && x != 3 && x != 5) { printf("%d x %d -> %d: %d\n", M, K, cols, x); return 1; }
+                    }
+    for (int M = 9; M <= 16; ++M)
+        if (!mid_batch_call_takes_ring(M, 4096, 4096, true, false) || mid_batch_call_takes_ring(M, 4096, 4096, true, true) || !mid_batch_call_takes_ring(M, 4096, 2048, false, true) ||
+            mid_batch_call_takes_ring(9, 1024, 300, true, false)) { printf("%d\n", M); return 1; }
+    return 0;
+}
+""")
