@@ -319,6 +319,11 @@ __device__ __forceinline__ void decode_cta(const DecodeParams& p, const unsigned
     }
     bar_sync_contraction();
     stamp(66);
+    // This CTA has read its collected maxima; whoever takes the last ticket clears them for the next SwiGLU epilogue, at the end, when
+    // the ticket is here.  (The counter wraps by itself.  A ticket behind the results, with a fence in front of it, put two trips to L2
+    // at the end of every CTA: FFN of 1 x 1024 -> 2048 -> 1024 9.5 us, now 8.8.)
+    unsigned ticket = 0;
+    if (no_scan && tid == 0) ticket = atomicInc(&p.status->done, nctas - 1u);
     // ---- quantise this CTA's share into its own code rows
     auto keep_code = [&](int tok, int u, const uint4& q) {
         *reinterpret_cast<uint4*>(xs + (size_t)tok * row_bytes + (size_t)u * 16) = q;
@@ -486,13 +491,8 @@ __device__ __forceinline__ void decode_cta(const DecodeParams& p, const unsigned
     if (TRACE && trace) trace[7] = global_ns();
     if (tid == 0) {
         if (cta == 0) p.report->bad_input = verdict;
-        if (no_scan) {
-            // Every CTA has read the collected maxima by now; the last one to get here clears them
-            // for the next SwiGLU epilogue.  The ticket counter wraps by itself.
-            __threadfence();
-            if (atomicInc(&p.status->done, nctas - 1u) == nctas - 1u)
-                for (int t = 0; t < M; ++t) p.rowmax_in[t] = 0u;
-        }
+        if (no_scan && ticket == nctas - 1u)
+            for (int t = 0; t < M; ++t) p.rowmax_in[t] = 0u;
     }
 }
 

@@ -196,6 +196,10 @@ __global__ void __launch_bounds__(FUSED_THREADS) gemm_fused_kernel(const FusedPa
     __syncthreads();
     if (trace) trace[3] = (unsigned long long)(clock64() - c_start);
     const int verdict = s_flags[0];   // identical in every CTA: all of them saw the whole rows
+    // This CTA has read the row maxima; whoever takes the last ticket clears them for the next SwiGLU epilogue, at the end, when the
+    // ticket is here.  The counter wraps by itself.
+    unsigned ticket = 0;
+    if (tid == 0 && p.rowmax_in != nullptr) ticket = atomicInc(&p.status->done, gridDim.x * gridDim.y - 1u);
     // partial sums this rank will receive: its share of the channels, every token, from every rank
     const int Qq = p.epi == EPI_SWIGLU ? 16 : 32;
     const int my_quads = ((rank + 1) * Qq) / S - (rank * Qq) / S;
@@ -388,14 +392,8 @@ __global__ void __launch_bounds__(FUSED_THREADS) gemm_fused_kernel(const FusedPa
     if (tid == 0) {
         if (s_flags[1]) *reinterpret_cast<volatile int*>(&p.report->device_error) = 1;   // (plain store: may be page-locked host memory)
         if (blockIdx.x == 0 && rank == 0) p.report->bad_input = verdict;
-        if (p.rowmax_in != nullptr) {
-            // Every CTA has read the row maxima by now; the last one to get here clears
-            // them for the next SwiGLU epilogue.  The ticket counter wraps by itself.
-            __threadfence();
-            const unsigned total = gridDim.x * gridDim.y;
-            if (atomicInc(&p.status->done, total - 1u) == total - 1u)
-                for (int t = 0; t < p.M; ++t) p.rowmax_in[t] = 0u;
-        }
+        if (p.rowmax_in != nullptr && ticket == gridDim.x * gridDim.y - 1u)
+            for (int t = 0; t < p.M; ++t) p.rowmax_in[t] = 0u;
     }
 }
 

@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
             if (active) {
                 const uint32_t at = sums + (uint32_t)(tok * RED_STRIDE + rank * CH + c4) * 4u;
                 auto add = [&](uint32_t at, int (&to)[4]) {
-    int4 a[8];                               // all ranks' sums on their way at once
+                    int4 a[8];           // all ranks' sums on their way at once
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         if (q < S) a[q] = lds128_cluster(S > 1 ? map_to_cta(at, (uint32_t)q) : at);
