@@ -114,6 +114,13 @@ __device__ __forceinline__ void st_async_u32(uint32_t remote_addr, uint32_t valu
                  : "memory");
 }
 
+// Adds to a word of this GPU, releasing what this thread has seen and acquiring what others released there.
+__device__ __forceinline__ uint32_t atomic_add_acq_rel(unsigned* at, unsigned v) {
+    uint32_t before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(before) : "l"(at), "r"(v) : "memory");
+    return before;
+}
+
 // ---- programmatic dependent launch
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
