@@ -67,6 +67,7 @@ template <bool HALF, bool SCAN, int BS, int UN>
 __global__ void __launch_bounds__(BS, (UN <= 4 ? 1280 : 896) / BS) quantize_rows_kernel(const QuantParams p)
 {
     pdl_launch_dependents();   // the GEMM behind this kernel may start prefetching weights
+    if (SCAN) prefetch_row(p.A, (size_t)p.K * (HALF ? 2 : 4));
     pdl_wait();                // A may be the output of the kernel in front of this one
     quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, RowQuant<HALF>{p.scales, p.rowmax, &p.status->bad_accum});
 }
