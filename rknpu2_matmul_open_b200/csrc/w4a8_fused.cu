@@ -125,6 +125,10 @@ __global__ void __launch_bounds__(FUSED_THREADS) gemm_fused_kernel(const FusedPa
         const int idx = tid + FUSED_THREADS * it;
         pos_tok[it] = units > 0 ? idx / units : 0;
         pos_u[it] = idx - pos_tok[it] * units;
+        // (pulled towards L2 while the launch in front still runs: only a hint, L2 is the point of coherence; the projections of a
+        // layer of 4096 / 11008 with 8 tokens 60.0 us, 58.6)
+        if (p.rowmax_in == nullptr && idx < items && pos_tok[it] < p.M && k_begin + pos_u[it] * 16 < p.K)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(A + (size_t)pos_tok[it] * p.K + k_begin + pos_u[it] * 16));
     }
     if (trace) trace[1] = (unsigned long long)(clock64() - c_start);
     pdl_wait();   // the producer of A (and of the row maxima) has finished
