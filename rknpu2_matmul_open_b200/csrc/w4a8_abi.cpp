@@ -1149,7 +1149,8 @@ rk_npu_w4a8_workspace* rkb200::create_workspace_scheduled(rk_npu_iommu_domain* d
     // tokens (at most one 16-element unit to quantise per thread of a four-CTA cluster, or none to exchange at all)
     // it beats the split-K kernel (3) on 7B-class shapes (4 tokens: 1783 against 1718 GB/s on the decode ring);
     // from five tokens on its exchange of int8 codes costs more than the split-K kernel's exchange of row maxima
-    // and partial sums (8 tokens: 1479 against 1669 GB/s), so the split-K kernel keeps those where it applies.
+    // and partial sums (8 tokens: 1479 against 1669 GB/s), so the split-K kernel is those workspaces' where it applies.  A call may
+    // take another of the three families that share the code layout: few_tokens_linear, few_tokens_ffn.
     const bool decode_ok = gemm_decode_supported(cfg->M, cfg->K);
     const bool decode_best = decode_ok && (cfg->M <= 4 || !fused_best);
     // 9..16 tokens: the split-K kernel's single launch while the weights are small, where results go over the bus; which calls take

@@ -1,4 +1,4 @@
-// w4a8_gemm_tc_persist.cu -- persistent two-CTA tcgen05 W4A8 GEMM from 17 tokens on (sm_100a).
+// w4a8_gemm_tc_persist.cu -- persistent two-CTA tcgen05 W4A8 GEMM, from 9 or 17 tokens on by the width of the output (sm_100a).
 //
 // Packed int4 weights -> tensor memory as the A operand (int8 weights stay in shared memory), int8 activation codes as
 // shared-memory B operand, kind::i8 MMA over a CTA pair with cta_group::2, int32 accumulators in tensor memory, organised so
@@ -7,7 +7,7 @@
 //     the kernel's width (64, 160 or 256; int8 weights 64 or 256), so that equal runs leave no nearly empty last round
 //     (4096 -> 14336, 2048 tokens: 13 rounds of 128-token tiles for 12.1 of work before).  Barriers, tensor memory and
 //     descriptors are set up once.  Where the tiles are few, K is cut into parts (persist_plan.h);
-//   * weights and activations travel through SEPARATE rings of bulk copies.  A weight slot is free again as soon as the unpack
+//   * weights (bulk copies) and activations (tensor copies with the 128-byte swizzle) travel through SEPARATE rings.  A weight slot is free again as soon as the unpack
 //     warps have read it (the unpacked copy lives in tensor memory), an activation slot when the MMAs that read it retire;
 //   * the MMA issuer is one warp whose every instruction counts: the tensor pipe queues about two MMAs, and what the issuer
 //     does between the last MMA of a stage and the first of the next has to fit under them.  So there is ONE barrier to wait
