@@ -289,10 +289,12 @@ Placement placement(const void* p)
 int pick_split_auto(const rk_npu_w4a8_workspace& ws, int tiles, int token_chunks)
 {
     const int sms = ws.domain->ctx->sm_count;
-    // The smallest split that gives every SM a CTA: more only adds reduction traffic and shortens
-    // each CTA's stream (measured on 4096x11008: split 2 -> 13 us, split 4 -> 17 us).
+    // The smallest split that gives nearly every SM a CTA: more only adds reduction traffic and shortens each CTA's stream, and more
+    // than 33 clusters of eight or 66 of four need not be resident at once (two CTAs an SM, whole clusters in a GPC), which costs a
+    // second round.  (Until every SM had one: 34 tiles in eight parts, 12 x 4096 -> 4352 10.5 us, in four 7.4; 72 tiles in four parts,
+    // 8 x 4096 -> 9152 11.2, in two 8.5; 65 tiles, 8 x 4096 -> 8320, in four 7.0, in two 8.7.)
     int split = 1;
-    while (split < 8 && (long long)tiles * token_chunks * split < sms && ws.KB / (split * 2) >= 2) split *= 2;
+    while (split < 8 && (long long)tiles * token_chunks * split * 10 < sms * 9ll && ws.KB / (split * 2) >= 2) split *= 2;
     return split;
 }
 int pick_split(const rk_npu_w4a8_workspace& ws, int tiles, int token_chunks)
