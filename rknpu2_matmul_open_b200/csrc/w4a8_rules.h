@@ -48,7 +48,8 @@ inline int few_tokens_linear(int family, int M, int K, int columns, bool half)
         return M <= 6 && groups > 144 && groups <= 192 ? 3 : 1;
     }
     if (columns <= 2112 && (K >= 8192 || (K >= 6144 && (M > 1 || !half)))) return 3;
-    if (groups > 144 && groups <= 240 && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
+    // (in a chain of binary16 calls 3 x 3584 -> 7680, 240 groups, takes the decode kernel 1 less; 4 x 4096 -> 6144, 192 groups, the clusters 1.4)
+    if (groups > 144 && groups <= (half ? 192 : 240) && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
     if (!half && groups > 144 && groups <= 296 && M > 2 && K >= 3072 && mb < 14) return 3;   // 4 x 3072 -> 8192 7.7 / 6.6 / 6.9
     if (K <= 1024 && groups > 296) return 3;                         // 4 x 1024 -> 14336 6.1 / 5.6 / 6.3
     if (ragged && M == 4 && mb > 4) return 1;

@@ -253,7 +253,7 @@ int main()
         {1, 4096, 4096, true, 5}, {1, 1024, 14336, true, 3}, {1, 11008, 2048, true, 3}, {2, 4096, 6144, true, 5}, {2, 5120, 5120, false, 3},
         {2, 8192, 8192, false, 1}, {3, 11008, 8192, true, 5}, {4, 8192, 2048, false, 3}, {4, 4096, 6144, true, 3}, {4, 8192, 8192, true, 1},
         {4, 3070, 4911, true, 1}, {4, 4096, 4096, false, 5}, {4, 5120, 13824, false, 1}, {5, 2048, 4096, true, 5}, {5, 5120, 5120, false, 3},
-        {8, 2048, 2048, false, 5}, {8, 4096, 4096, true, 3}, {8, 4096, 4096, false, 1}, {8, 2048, 14336, true, 1}, {8, 4096, 11008, true, 3}, {4, 4096, 11008, true, 5}, {4, 2048, 5632, true, 5}, {8, 3070, 4911, false, 1},
+        {8, 2048, 2048, false, 5}, {8, 4096, 4096, true, 3}, {8, 4096, 4096, false, 1}, {8, 2048, 14336, true, 1}, {8, 4096, 11008, true, 3}, {4, 4096, 11008, true, 5}, {4, 2048, 5632, true, 5}, {3, 3584, 7680, true, 5}, {3, 5120, 5632, true, 3}, {8, 3070, 4911, false, 1},
         {8, 8192, 1024, false, 3}, {8, 8192, 2048, false, 1}, {6, 8192, 2048, false, 3}, {5, 1500, 2048, true, 5}, {8, 1500, 2048, true, 5}, {3, 3072, 8192, false, 3}, {4, 11008, 8192, false, 5},
     };
     for (const Case& c : cases) {
