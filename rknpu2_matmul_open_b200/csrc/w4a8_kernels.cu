@@ -230,12 +230,13 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
     // What a thread finishes: four channels of this rank's share (SwiGLU: of the gate, and the same of up), 128 / IPT tokens apart.
     const int CH = (swiglu ? 64 : TILE_N) / S;
     const int IPT = CH / 4, first_token = tid / IPT, c4 = (tid - first_token * IPT) * 4;
+    const int columns = swiglu ? p.F : p.N;
     const int n0 = swiglu ? tile * 64 + rank * CH + c4 : tile * TILE_N + rank * CH + c4;
     float sw[4], sw_up[4];
     if (warp < 4) {      // scales of channels never change
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            sw[e] = n0 + e < (swiglu ? p.F : p.N) ? p.sw[n0 + e] : 0.f;
+            sw[e] = n0 + e < columns ? p.sw[n0 + e] : 0.f;
             sw_up[e] = swiglu && n0 + e < p.F ? p.sw[p.F + n0 + e] : 0.f;
         }
     }
@@ -377,9 +378,9 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
 #pragma unroll 1
         for (int tok = first_token; tok - first_token < TC; tok += 128 / IPT) {      // (the same turns for all threads)
             const int m = tok0 + tok;
-            const bool active = tok < TC;
+            const bool finish = tok < TC && m < p.M && n0 < columns;      // only what is stored is asked for, see the end
             int v[4] = {}, u[4] = {};
-            if (active) {
+            if (finish) {
                 const uint32_t at = sums + (uint32_t)(tok * RED_STRIDE + rank * CH + c4) * 4u;
                 auto add = [&](uint32_t at, int (&to)[4]) {
                     int4 a[8];           // all ranks' sums on their way at once
@@ -393,10 +394,9 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
                 add(at, v);
                 if (swiglu) add(at + 256u, u);
             }
-            const float sx = active ? s_sx[tok] : 0.f;
-            const bool row_ok = active && m < p.M;
+            const float sx = finish ? s_sx[tok] : 0.f;
             if (!swiglu) {
-                if (row_ok && n0 < p.N) {
+                if (finish) {
                     if (p.epi == EPI_I32) {
                         int* out = reinterpret_cast<int*>(p.out) + (size_t)m * p.N + n0;
                         if (n0 + 3 < p.N && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) *reinterpret_cast<int4*>(out) = make_int4(v[0], v[1], v[2], v[3]);
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
                 }
             } else {
                 uint32_t mx = 0;
-                if (row_ok && n0 < p.F) {
+                if (finish) {
                     float y[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -441,12 +441,14 @@ __global__ void __launch_bounds__(160, 1) gemm_mma_kernel(const GemmParams p)
                 if (p.rowmax) {
                     // lanes of an aligned group of IPT share the token: one atomic per group
                     for (int o = 1; o < IPT && o < 32; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-                    if (row_ok && (lane & (IPT - 1) & 31) == 0 && mx) atomicMax(&p.rowmax[m], mx);
+                    if ((lane & (IPT - 1) & 31) == 0 && mx) atomicMax(&p.rowmax[m], mx);
                 }
             }
         }
     }
-    if (S > 1) {                 // nobody leaves while a peer may still read its partials (what was read is here: no memory to order)
+    // Nobody leaves while a peer may still read its sums.  A relaxed arrival does not wait for loads, so no load may be on its way here:
+    // each one's sums went into a store above, which needed them.
+    if (S > 1) {
         __syncwarp();
         cluster_arrive_relaxed();
         cluster_wait();

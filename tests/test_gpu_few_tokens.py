@@ -73,3 +73,34 @@ def test_ffn(gpu, oracle, M, K, F, N):
     assert np.array_equal(bits(outs[0][1]), bits(ref))
     wg.free()
     wd.free()
+
+
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+@pytest.mark.parametrize("M", [1, 9, 17, 31])
+def test_ring_parts_of_padded_tiles(gpu, oracle, monkeypatch, M, split):
+    # whole warps of a CTA have only tokens or channels that do not exist: launches back to back, nothing written beside the result
+    _, dom, _ = gpu
+    monkeypatch.setenv("RK_NPU_B200_VARIANT", "1")
+    K, N, F = 1100, 130, 96
+    (B, sw), (Bg, sg) = make_weights(K, N, seed=3), make_weights(K, 2 * F, seed=4)
+    w, wg = rk.Weights(dom, B, sw), rk.Weights(dom, Bg, sg)
+    ws, gu = rk.Workspace(dom, rk.default_config(M, N, K)), rk.Workspace(dom, rk.default_config(M, 2 * F, K))
+    assert ws.set_schedule(1, split) == 0 and gu.set_schedule(1, split) == 0
+    a = make_activations(M, K, seed=M, dtype="f32")
+    x = torch.from_numpy(a).cuda()
+    ref, (_, _, acc, scales) = oracle.linear(a, B, sw)[1], oracle.linear(a, Bg, sg)
+    middle, maxima = oracle.swiglu(acc, scales, sg)
+    stream = torch.cuda.current_stream().cuda_stream
+    outs, mids = ([torch.full((M + 1, n), -7.0, device="cuda") for _ in range(20)] for n in (N, F))
+    tops = torch.zeros((20, M + 1), dtype=torch.int32, device="cuda")
+    for out, mid, top in zip(outs, mids, tops):
+        assert ws.enqueue_f32(w, x, out, stream) == 0 and gu.enqueue_swiglu_collect_f32(wg, x, mid, top, stream) == 0
+    torch.cuda.synchronize()
+    assert ws.finish() == 0 and gu.finish() == 0
+    for out, mid, top in zip(outs, mids, tops):
+        out, mid, top = (t.cpu().numpy() for t in (out, mid, top))
+        assert np.array_equal(bits(out[:M]), bits(ref)) and np.all(out[M] == -7.0)
+        assert np.array_equal(bits(mid[:M]), bits(middle)) and np.all(mid[M] == -7.0)
+        assert np.array_equal(bits(top[:M]), maxima) and top[M] == 0
+    for o in (ws, gu, w, wg):
+        o.free()
