@@ -133,7 +133,8 @@ int rk_npu_b200_w4a8_enqueue_codes_f32(rk_npu_w4a8_workspace *down, const rk_npu
 
 /* After the caller has synchronised the stream: RK_NPU_OK, RK_NPU_ERR_PARAM (non-finite
  * activation or middle in the last queued call) or RK_NPU_ERR_SUBMIT (a bounded device
- * wait ran out).  Clears the recorded status. */
+ * wait ran out).  Clears the recorded status: asked again it says RK_NPU_OK.  A blocking
+ * call returns its own verdict and is not reported here. */
 int rk_npu_b200_w4a8_finish(rk_npu_w4a8_workspace *workspace);
 
 /* Diagnostic: the same linear as rk_npu_w4a8_run_f32 / _f16 (activation_is_f16 selects

@@ -527,7 +527,9 @@ float event_us(cudaEvent_t a, cudaEvent_t b)
     return ms * 1000.f;
 }
 
-int status_to_rc(rk_npu_w4a8_workspace& ws, cudaStream_t stream)
+// What *host_status says.  `copied` from the device block: a verdict is cleared there when it is reported.  (A call whose verdict goes
+// to page-locked memory leaves the block alone: it keeps that of the last queued call.)
+int status_to_rc(rk_npu_w4a8_workspace& ws, cudaStream_t stream, bool copied)
 {
     const Status s = *ws.host_status;
     if (s.device_error) {
@@ -537,7 +539,12 @@ int status_to_rc(rk_npu_w4a8_workspace& ws, cudaStream_t stream)
         cudaStreamSynchronize(stream);
         return RK_NPU_ERR_SUBMIT;
     }
-    return s.bad_input ? RK_NPU_ERR_PARAM : RK_NPU_OK;
+    if (!s.bad_input) return RK_NPU_OK;
+    if (copied) {
+        cudaMemsetAsync(&ws.status->bad_input, 0, sizeof(int), stream);
+        cudaStreamSynchronize(stream);
+    }
+    return RK_NPU_ERR_PARAM;
 }
 
 // Group of GPUs: the kernels have written this rank's compact [M][its columns] block into its slot of the
@@ -663,7 +670,7 @@ int run_locked(rk_npu_w4a8_workspace* ws, const rk_npu_w4a8_weights* w, const vo
     copy_start = Clock::now();
     if (!status_alias) cudaMemcpyAsync(ws->host_status, ws->status, sizeof(Status), cudaMemcpyDeviceToHost, s);
     const Download down[1] = {{C, dC, out_bytes, c_at.alias != nullptr}};
-    rc = download(*ws, down, !c_dev && !c_alias ? 1 : 0, s, [&] { return status_to_rc(*ws, s); });
+    rc = download(*ws, down, !c_dev && !c_alias ? 1 : 0, s, [&] { return status_to_rc(*ws, s, !status_alias); });
     if (bounce_out && rc == RK_NPU_OK) std::memcpy(C, ws->bounce_out.ptr, out_bytes);
     t.sync_us += elapsed_us(copy_start);
     if (metrics) {
@@ -1347,8 +1354,8 @@ extern "C" int rk_npu_w4a8_run_ffn_f32(rk_npu_w4a8_workspace* gate_up, const rk_
         if (!m_dev) results[count++] = {middle, dMiddle, size_t(M) * F * 4, m_at.alias != nullptr};
         int rc_down = RK_NPU_OK;
         rc = download(*gate_up, results, count, s, [&] {
-            const int rc_gate = status_to_rc(*gate_up, s);
-            rc_down = status_to_rc(*down, s);
+            const int rc_gate = status_to_rc(*gate_up, s, !own_report);
+            rc_down = status_to_rc(*down, s, !own_report);
             return rc_gate ? rc_gate : rc_down;
         });
         t.down.sync_us += elapsed_us(mark);
@@ -1571,7 +1578,7 @@ extern "C" int rk_npu_b200_w4a8_finish(rk_npu_w4a8_workspace* ws)
         cudaGetLastError();
         return RK_NPU_ERR_SUBMIT;
     }
-    return status_to_rc(*ws, ws->stream);
+    return status_to_rc(*ws, ws->stream, true);
 }
 
 extern "C" int rk_npu_b200_w4a8_last_quant(rk_npu_w4a8_workspace* ws, float* scales, int8_t* codes)

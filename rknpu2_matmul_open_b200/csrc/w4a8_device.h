@@ -55,7 +55,7 @@ enum Epilogue : int { EPI_F32 = 0, EPI_F16 = 1, EPI_I32 = 2, EPI_SWIGLU = 3 };
 
 // Device-side status block of a workspace (all int32).
 struct Status {
-    int bad_input;      // verdict of the last call: 1 = NaN/Inf activation, 2 = non-finite middle
+    int bad_input;      // verdict: 1 = NaN/Inf activation, 2 = non-finite middle; in the device block the last queued call's, until it is reported
     int bad_accum;      // set by a quantise kernel, taken by the GEMM behind it (take_verdict); zero between calls
     unsigned done;      // scratch counter (wraps to 0 by itself)
     int device_error;   // 1 = a bounded wait inside a kernel ran out

@@ -48,3 +48,39 @@ def test_good_and_bad_calls_in_turn(gpu, oracle, monkeypatch, family, cut, M, K,
     assert ws.finish() == 0 and np.array_equal(bits(outs[1].cpu().numpy()), bits(ref))
     ws.free()
     w.free()
+
+
+# kernel family, tokens, channels (41 tiles of 256 at twelve tokens)
+@pytest.mark.parametrize("family, M, N", [(1, 12, 260), (2, 40, 700), (3, 8, 260), (4, 24, 300), (5, 4, 260), (0, 8, 260), (0, 12, 10300)])
+def test_a_verdict_is_reported_once(gpu, oracle, monkeypatch, family, M, N):
+    _, dom, _ = gpu
+    if family:
+        monkeypatch.setenv("RK_NPU_B200_VARIANT", str(family))
+    K = 1032
+    B, sw = make_weights(K, N, seed=K)
+    w, ws = rk.Weights(dom, B, sw), rk.Workspace(dom, rk.default_config(M, N, K))
+    good = make_activations(M, K, seed=M, dtype="f32")
+    bad = good.copy()
+    bad[M - 1, 0] = np.nan
+    ref = oracle.linear(good, B, sw)[1]
+    stream = torch.cuda.current_stream().cuda_stream
+    dev, out, host = {"good": torch.from_numpy(good).cuda(), "bad": torch.from_numpy(bad).cuda()}, torch.zeros((M, N), device="cuda"), np.zeros((M, N), np.float32)
+
+    def queue(kind):
+        assert ws.enqueue_f32(w, dev[kind], out, stream) == 0
+        torch.cuda.synchronize()
+
+    assert ws.finish() == 0
+    queue("bad")
+    assert ws.finish() == capi.RK_NPU_ERR_PARAM and ws.finish() == 0
+    assert ws.run_f32(w, good, host) == 0 and np.array_equal(bits(host), bits(ref)) and ws.finish() == 0
+    assert ws.run_f32(w, bad, host) == capi.RK_NPU_ERR_PARAM and ws.finish() == 0
+    timings = capi.W4A8Timings()                                   # (the verdict of a timed call passes through the device's block)
+    assert ws.run_f32(w, bad, host, timings) == capi.RK_NPU_ERR_PARAM and ws.finish() == 0
+    queue("bad")
+    assert ws.run_f32(w, good, host) == 0 and ws.finish() == capi.RK_NPU_ERR_PARAM      # the queued call's
+    queue("bad")
+    queue("good")
+    assert ws.finish() == 0 and np.array_equal(bits(out.cpu().numpy()), bits(ref))
+    ws.free()
+    w.free()
