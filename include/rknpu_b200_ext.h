@@ -225,10 +225,13 @@ int rk_npu_b200_add_rmsnorm_f16_enqueue(rk_npu_add_rmsnorm_f16_plan *plan, int r
  *   every CTA expect 16 bytes that no copy brings, so the bounded wait on it runs out after the workspace's
  *   timeout_ms, the kernel records the error and returns (all real copies have landed), and the call reports
  *   RK_NPU_ERR_SUBMIT; (ws, 0) restores normal launches.  RK_NPU_ERR_PARAM for other kernel families.
+ * rk_npu_b200_w4a8_test_refuse(ws, 1): the workspace's GEMM launches are not made and count as refused by the
+ *   driver (a quantise launch in front of one is made), the calls report RK_NPU_ERR_SUBMIT; (ws, 0) ends it.
  * rk_npu_b200_w4a8_test_device_error(ws): sets the workspace's device-side error word from the host, as a kernel
  *   whose wait ran out would; the next status read reports RK_NPU_ERR_SUBMIT and clears it. */
 void rk_npu_b200_test_fail_allocation(long long after);
 int rk_npu_b200_w4a8_test_starve(rk_npu_w4a8_workspace *workspace, int on);
+int rk_npu_b200_w4a8_test_refuse(rk_npu_w4a8_workspace *workspace, int on);
 int rk_npu_b200_w4a8_test_device_error(rk_npu_w4a8_workspace *workspace);
 
 /* Kernels this workspace has launched since creation (for launch accounting). */

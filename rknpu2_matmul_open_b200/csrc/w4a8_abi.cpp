@@ -412,12 +412,20 @@ int enqueue(const Call& c)
     const int tiles = c.epi == EPI_SWIGLU ? (F + 63) / 64 : (N + TILE_N - 1) / TILE_N;
     const unsigned long long timeout_ns = (unsigned long long)cfg.timeout_ms * 1000000ull;
     const int family = family_of(ws, c);
+    // A refused launch must not leave behind what the launches in front of it handed on, or the next call would take it for its own: the
+    // mark of a rejected row, collected maxima.
+    auto refused = [&] {
+        cudaGetLastError();
+        cudaMemsetAsync(&ws.status->bad_accum, 0, sizeof(int), c.stream);
+        if (c.rowmax_in) cudaMemsetAsync(c.rowmax_in, 0, sizeof(uint32_t) * cfg.M, c.stream);
+        return RK_NPU_ERR_SUBMIT;
+    };
     if (family == 5 && !c.codes_in) {
         // One kernel, whole-K CTAs: scan + quantise (shared by a cluster) + GEMM + epilogue.
         DecodeParams d{};
         decode_params(c, d);
         if (c.events) cudaEventRecord(c.events[1], c.stream);
-        if (launch_gemm_decode(d, c.stream, pdl) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        if (ws.refuse || launch_gemm_decode(d, c.stream, pdl) != cudaSuccess) return refused();
         if (c.events) cudaEventRecord(c.events[2], c.stream);
         ws.launches.fetch_add(1, std::memory_order_relaxed);
         return RK_NPU_OK;
@@ -444,7 +452,7 @@ int enqueue(const Call& c)
         f.timeout_ns = timeout_ns;
         f.trace = ws.trace;
         if (c.events) cudaEventRecord(c.events[1], c.stream);
-        if (launch_gemm_fused(f, ws.TC, c.stream, pdl) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        if (ws.refuse || launch_gemm_fused(f, ws.TC, c.stream, pdl) != cudaSuccess) return refused();
         if (c.events) cudaEventRecord(c.events[2], c.stream);
         ws.launches.fetch_add(1, std::memory_order_relaxed);
         return RK_NPU_OK;
@@ -458,7 +466,7 @@ int enqueue(const Call& c)
         ci.status = ws.status;
         ci.M = cfg.M; ci.K = cfg.K; ci.Kp = ws.KB * KBLOCK; ci.T = ws.T;
         ci.parts = c.parts;
-        if (launch_codes_in(ci, c.stream) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+        if (launch_codes_in(ci, c.stream) != cudaSuccess) return refused();
     } else {
     QuantParams q{};
     q.A = c.dA;
@@ -471,7 +479,7 @@ int enqueue(const Call& c)
     q.Kp = ws.KB * KBLOCK;
     q.T = ws.T;
     q.half = c.half ? 1 : 0;
-    if (launch_quantize(q, c.stream, pdl) != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+    if (launch_quantize(q, c.stream, pdl) != cudaSuccess) return refused();
     }
     if (c.events) cudaEventRecord(c.events[1], c.stream);
 
@@ -496,7 +504,8 @@ int enqueue(const Call& c)
     g.timeout_ns = timeout_ns;
     g.trace = ws.trace;
     cudaError_t err;
-    if (ws.variant == 2) {
+    if (ws.refuse) err = cudaErrorLaunchFailure;
+    else if (ws.variant == 2) {
         g.partials = ws.partials;
         g.counts = ws.counts;
         set_plan(g, ws.plan[c.epi == EPI_SWIGLU]);
@@ -514,7 +523,7 @@ int enqueue(const Call& c)
                                   : pick_split(ws, tiles, (cfg.M + ws.TC - 1) / ws.TC);
         err = launch_gemm_mma(g, ws.TC, c.stream, pdl);
     }
-    if (err != cudaSuccess) { cudaGetLastError(); return RK_NPU_ERR_SUBMIT; }
+    if (err != cudaSuccess) return refused();
     if (c.events) cudaEventRecord(c.events[2], c.stream);
     ws.launches.fetch_add(2, std::memory_order_relaxed);
     return RK_NPU_OK;
@@ -1634,6 +1643,14 @@ extern "C" int rk_npu_b200_w4a8_test_starve(rk_npu_w4a8_workspace* ws, int on)
     WorkspaceLock lock(*ws);
     if (!lock) return RK_NPU_ERR_BUSY;
     ws->starve = on != 0;
+    return RK_NPU_OK;
+}
+extern "C" int rk_npu_b200_w4a8_test_refuse(rk_npu_w4a8_workspace* ws, int on)
+{
+    if (!ws) return RK_NPU_ERR_PARAM;
+    WorkspaceLock lock(*ws);
+    if (!lock) return RK_NPU_ERR_BUSY;
+    ws->refuse = on != 0;
     return RK_NPU_OK;
 }
 extern "C" int rk_npu_b200_w4a8_test_device_error(rk_npu_w4a8_workspace* ws)

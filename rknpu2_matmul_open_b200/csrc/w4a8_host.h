@@ -131,6 +131,7 @@ struct rk_npu_w4a8_workspace {
     bool by_rule = false;                  // the variant is the library's own choice: a call may take another for its rows (family_of)
     int decode_cap[4] = {0, 0, 0, 0};      // variant 5: CTAs resident at once for cluster sizes 1, 2, 4, 8
     bool starve = false;                   // test hook (rk_npu_b200_w4a8_test_starve): first weight barrier never completes
+    bool refuse = false;                   // test hook (rk_npu_b200_w4a8_test_refuse): GEMM launches count as refused
     // device buffers
     uint8_t* codes = nullptr;
     float* scales = nullptr;

@@ -131,3 +131,28 @@ def test_objects_freed_after_their_context_was_closed(oracle):
     experts.free()
     w.free()
     dom.free()
+
+
+@pytest.mark.parametrize("family, M", [(1, 12), (2, 40), (3, 8), (4, 24), (5, 4)])
+def test_a_refused_launch_leaves_nothing_to_the_next_call(gpu, oracle, monkeypatch, family, M):
+    # behind a quantise launch that marked a rejected row, and behind a first projection that collected large maxima
+    lib = capi.load()
+    _, dom, _ = gpu
+    monkeypatch.setenv("RK_NPU_B200_VARIANT", str(family))
+    K, F, N = 512, 256, 192
+    (Bg, sg), (Bd, sd) = make_weights(K, 2 * F, seed=1), make_weights(F, N, seed=2)
+    wg, wd = rk.Weights(dom, Bg, sg), rk.Weights(dom, Bd, sd)
+    gu, dn = (rk.Workspace(dom, rk.default_config(M, n, k)) for n, k in ((2 * F, K), (N, F)))
+    A = make_activations(M, K, seed=3, dtype="f32")
+    ref = oracle.ffn(A, Bg, sg, Bd, sd, mode=1)
+    bad = make_activations(M, F, seed=4, dtype="f32")
+    bad[0, 0] = np.inf
+    middle, out = np.zeros((M, F), np.float32), np.zeros((M, N), np.float32)
+    for call in (lambda: dn.run_f32(wd, bad, out), lambda: rk.run_ffn_f32(gu, wg, dn, wd, 50 * A, middle, out)):
+        assert lib.rk_npu_b200_w4a8_test_refuse(dn.handle, 1) == 0
+        assert call() == capi.RK_NPU_ERR_SUBMIT
+        assert lib.rk_npu_b200_w4a8_test_refuse(dn.handle, 0) == 0
+        assert rk.run_ffn_f32(gu, wg, dn, wd, A, middle, out) == 0
+        assert np.array_equal(bits(middle), bits(ref["middle"])) and np.array_equal(bits(out), bits(ref["C"]))
+    for o in (gu, dn, wg, wd):
+        o.free()
