@@ -463,7 +463,9 @@ def run_cuda(args, rank, world, local_rank):
                              # one read per weight byte (ncu: DRAM bytes read equal the algorithmic bytes to 0.1 %), so the
                              # traffic of a launch is its algorithmic bytes
                              "traffic": bytes_per_launch, "peak_kind": peak_kind,
-                             "kernel": {3: "gemm_fused_kernel (split-K clusters)", 5: "gemm_decode_kernel (whole-K CTAs)"}.get(
+                             # (a call may take the two launches of the ring where its workspace's own family has one)
+                             "kernel": ({} if launches_per_step > len(linears) else
+                                        {3: "gemm_fused_kernel (split-K clusters)", 5: "gemm_decode_kernel (whole-K CTAs)"}).get(
                                  linears[0]["ws"].schedule()[0], "quantize_rows_kernel + gemm_mma_kernel") + ": scan + quantise + GEMM + dequantise",
                              "frac_of_nominal": value / world / 8000.0, "nominal_peak": 8000.0,   # 8 TB/s data-sheet HBM3e
                              "bytes_per_launch": bytes_per_launch,

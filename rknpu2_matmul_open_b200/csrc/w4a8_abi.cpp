@@ -288,14 +288,7 @@ Placement placement(const void* p)
 // ------------------------------------------------------------------ kernel sequencing
 int pick_split_auto(const rk_npu_w4a8_workspace& ws, int tiles, int token_chunks)
 {
-    const int sms = ws.domain->ctx->sm_count;
-    // The smallest split that gives nearly every SM a CTA: more only adds reduction traffic and shortens each CTA's stream, and more
-    // than 33 clusters of eight or 66 of four need not be resident at once (two CTAs an SM, whole clusters in a GPC), which costs a
-    // second round.  (Until every SM had one: 34 tiles in eight parts, 12 x 4096 -> 4352 10.5 us, in four 7.4; 72 tiles in four parts,
-    // 8 x 4096 -> 9152 11.2, in two 8.5; 65 tiles, 8 x 4096 -> 8320, in four 7.0, in two 8.7.)
-    int split = 1;
-    while (split < 8 && (long long)tiles * token_chunks * split * 10 < sms * 9ll && ws.KB / (split * 2) >= 2) split *= 2;
-    return split;
+    return ring_parts((long long)tiles * token_chunks, ws.KB, ws.domain->ctx->sm_count);
 }
 int pick_split(const rk_npu_w4a8_workspace& ws, int tiles, int token_chunks)
 {
@@ -366,7 +359,7 @@ int family_of(const rk_npu_w4a8_workspace& ws, const Call& c)
     if (!ws.by_rule || ws.split_override || c.over_bus || c.codes_in || c.keep_codes || (ws.variant != 3 && ws.variant != 5)) return ws.variant;
     if (cfg.M > 8) return mid_batch_call_takes_ring(cfg.M, cfg.K, ws.shard_N, c.half, c.rowmax_in) ? 1 : 3;
     const bool ffn = c.rowmax_in || c.epi == EPI_SWIGLU;
-    const int family = ffn ? few_tokens_ffn(ws.variant, cfg.M, cfg.K, ws.shard_N, c.rowmax_in) : few_tokens_linear(ws.variant, cfg.M, cfg.K, ws.shard_N, c.half);
+    const int family = ffn ? few_tokens_ffn(ws.variant, cfg.M, cfg.K, ws.shard_N, c.rowmax_in) : few_tokens_linear(ws.variant, cfg.M, cfg.K, ws.shard_N, c.half, ws.domain->ctx->sm_count);
     if (family == 5 && ws.decode_cap[0] < 1) return ws.variant;
     return family == 3 && ws.KB > 8 * FUSED_MAX_STAGES ? 1 : family;
 }

@@ -26,36 +26,58 @@ inline bool result_over_bus(int family, int M, size_t cols, size_t elem)
     return bytes <= (elem == 2 ? size_t(40) << 10 : size_t(64) << 10);
 }
 
+// CTAs (of a cluster) that share a column tile of the ring: the smallest number that gives nearly every SM a CTA.  More only adds
+// reduction traffic and shortens each CTA's stream, and more than 33 clusters of eight or 66 of four need not be resident at once (two
+// CTAs an SM, whole clusters in a GPC), which costs a second round.  (Until every SM had one: 34 tiles in eight parts, 12 x 4096 ->
+// 4352 10.5 us, in four 7.4; 72 tiles in four parts, 8 x 4096 -> 9152 11.2, in two 8.5; 65 tiles, 8 x 4096 -> 8320, in four 7.0, in
+// two 8.7.)
+inline int ring_parts(long long tiles, int KB, int sms)
+{
+    int parts = 1;
+    while (parts < 8 && tiles * parts * 10 < sms * 9ll && KB / (parts * 2) >= 2) parts *= 2;
+    return parts;
+}
+
 // Up to eight tokens: the family that runs a call of a workspace of family 3 (split-K clusters) or 5 (decode); the code layout is the
-// ring's (1) too.  Measured on 33 shapes of both types, the times are of one call of a back-to-back series in us, decode / clusters /
-// ring.  The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3
-// at least: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32 7.8 / 7.9 / 6.5,
-// 4 x 8192 -> 8192 13 / 12.6 / 10.6, 8 x 3070 -> 4911 10.3 / 13.2 / 7.6).  The decode kernel's CTAs take 32 channels over all of K:
-// best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2), poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.4 / 7.2) and
-// where some CTAs have two groups of channels (4 x 5120 -> 5120 9.0 / 7.0 / 7.9).
-inline int few_tokens_linear(int family, int M, int K, int columns, bool half)
+// ring's (1) too.  Measured on 60 shapes of both types alone (times of one call of a back-to-back series in us, decode / clusters /
+// ring; with weights from HBM as with weights in L2) and in decoder layers, one call behind another.
+//   * The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3 at
+//     least, whatever the rows: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32
+//     7.8 / 7.9 / 6.3, 4 x 8192 -> 8192 13 / 12.7 / 10.1, 8 x 4096 -> 14336 13.9 / 13.8 / 9.5, 8 x 3070 -> 4911 10.3 / 13.3 / 7.5).
+//   * The clusters hold all of their weights in shared memory and are good while a CTA has one column tile, up to 12.5 MB of weights on
+//     148 SMs (fused_tiles_per_cta); of two the second's contraction, exchange and finish run behind the first's (8 x 4096 -> 6144
+//     9.8 / 7.1 / 6.9, -> 6784 9.4 / 9.7 / 7.0).
+//   * The decode kernel's CTAs take 32 channels over all of K: best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2) and few tokens,
+//     poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.5 / 6.9) and where some CTAs have two groups of channels
+//     (4 x 5120 -> 5120 9.1 / 7.0 / 7.3).
+constexpr int RULE_SMS = 148;
+inline int few_tokens_linear(int family, int M, int K, int columns, bool half, int sms = RULE_SMS)
 {
     const double mb = double(K) * columns / 2 / (1 << 20);          // of weights
     const bool ragged = K % (half ? 8 : 4) != 0;
+    const bool one_tile = mb * RULE_SMS <= 12.5 * sms;
     const int groups = (columns + 31) / 32;
     if (M > 4) {
-        if (K <= 3072 && mb <= 4.5) return 5;
+        if (K <= 2560 && mb <= 4.5) return 5;
         if (ragged) return 1;
-        // 8 x 3072 -> 8192 9.0 / 7.1 / 7.0, 2048 -> 14336 8.8 / 9.7 / 7.3; 4096 -> 11008 is a tie alone, and in a chain of dependent
-        // calls the clusters' by 0.7
-        if (half) return mb <= 13.25 || (mb > 20 && K <= 4096) ? family : 1;
-        if (columns <= 1024 || (K >= 8192 && columns <= 2112 && M <= 6)) return 3;
-        return M <= 6 && groups > 144 && groups <= 192 ? 3 : 1;
+        // few channels, where a launch less counts for more: 8 x 4096 -> 1024 5.7 / 5.5 / 6.3, 5 x 11008 -> 1024 fp32 12.8 / 7.3 / 8.5
+        if (half) return one_tile && (K <= 1024 || (columns <= 2112 && K >= 4096)) ? 3 : 1;
+        return M <= 6 && one_tile && (columns <= 1024 || (columns <= 2112 && K >= 8192)) ? 3 : 1;
     }
-    if (columns <= 2112 && (K >= 8192 || (K >= 6144 && (M > 1 || !half)))) return 3;
-    // (in a chain of binary16 calls 3 x 3584 -> 7680, 240 groups, takes the decode kernel 1 less; 4 x 4096 -> 6144, 192 groups, the clusters 1.4)
-    if (groups > 144 && groups <= (half ? 192 : 240) && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
-    if (!half && groups > 144 && groups <= 296 && M > 2 && K >= 3072 && mb < 14) return 3;   // 4 x 3072 -> 8192 7.7 / 6.6 / 6.9
+    if (columns <= 2112 && (K >= 8192 || (K >= 6144 && (M > 1 || !half))) && (M <= 2 || !half || one_tile)) return 3;
+    if (one_tile && groups > 144 && groups <= (half ? 192 : 240) && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
+    if (one_tile && !half && groups > 144 && groups <= 296 && M > 2 && K >= 3072) return 3;      // 4 x 3072 -> 8192 7.7 / 6.7 / 6.5
     if (K <= 1024 && groups > 296) return 3;                         // 4 x 1024 -> 14336 6.1 / 5.6 / 6.3
     if (ragged && M == 4 && mb > 4) return 1;
-    // (in a chain 4 x 4096 -> 11008 takes the decode kernel 0.9 less than the ring)
-    if (mb >= 14 && ((M > 2 && K <= 8192 && (mb >= 26 || K >= 6144)) || (M == 2 && K >= (half ? 8192 : 4096)) || (M < 3 && mb >= 40))) return 1;
-    return family;
+    // The ring's two CTAs an SM: with hardly more than one each it is no faster than the decode kernel (4 x 4096 -> 14336, 224 CTAs,
+    // 11.0 / 12.2 / 9.4, but -> 18944, 148 CTAs, 13.2 / 13.3 / 13.9; -> 11008, 172, 10.5 / 9.7 / 9.3 alone, in a layer 0.3 behind decode).
+    const long long tiles = (columns + 127) / 128;
+    const bool fills = tiles * ring_parts(tiles, (K + 127) / 128, sms) * 4 >= sms * 5ll;
+    // Long rows of 112 to 148 groups stay: 3 x 11008 -> 4096 9.1 / 10.9 / 9.1 alone, in a layer the ring is 4 behind.
+    if (M > 2) return !ragged && !one_tile && K < 10240 && (fills || K >= 5120) ? 1 : family;
+    // Two tokens cost the decode kernel less: fp32 4096 -> 11008 8.6 / 9.5 / 9.2, -> 14336 10.4 / 11.0 / 9.4, 5120 -> 6912 9.7 / 9.4 / 7.6
+    if (M == 2 && ((mb >= 14 && K >= (half ? 8192 : 5120)) || (!half && mb >= 28 && K >= 4096 && fills))) return 1;
+    return mb >= 40 ? 1 : family;
 }
 
 // The same for the two projections of an FFN (times of the whole FFN).  The first's columns come in pairs and its quantising is fp32

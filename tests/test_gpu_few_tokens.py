@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 # (M, K, N, launches of a call with fp32 rows, with binary16 rows)
 LINEAR = [(1, 8192, 512, 1, 1), (1, 1024, 9500, 1, 1), (3, 3200, 4640, 1, 1), (4, 2044, 4400, 1, 2), (5, 1500, 2048, 1, 1), (5, 3070, 3100, 2, 2),
-          (6, 4096, 1040, 2, 1), (8, 4096, 1024, 1, 1), (8, 2048, 1056, 1, 1), (8, 2048, 3200, 1, 1), (7, 1500, 2048, 1, 1), (8, 3104, 3104, 2, 1),
+          (6, 4096, 1040, 2, 1), (6, 4096, 1024, 1, 1), (8, 4096, 1024, 2, 1), (8, 2048, 1056, 1, 1), (8, 2048, 3200, 1, 1), (7, 1500, 2048, 1, 1), (8, 3104, 3104, 2, 2), (7, 2624, 3520, 2, 2), (4, 4096, 6464, 2, 2), (2, 4096, 7328, 1, 1),
           (9, 1024, 512, 1, 1), (9, 1024, 520, 2, 2), (16, 1030, 2050, 2, 2)]
 
 
