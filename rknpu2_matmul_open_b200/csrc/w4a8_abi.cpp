@@ -359,7 +359,8 @@ int family_of(const rk_npu_w4a8_workspace& ws, const Call& c)
     if (!ws.by_rule || ws.split_override || c.over_bus || c.codes_in || c.keep_codes || (ws.variant != 3 && ws.variant != 5)) return ws.variant;
     if (cfg.M > 8) return mid_batch_call_takes_ring(cfg.M, cfg.K, ws.shard_N, c.half, c.rowmax_in) ? 1 : 3;
     const bool ffn = c.rowmax_in || c.epi == EPI_SWIGLU;
-    const int family = ffn ? few_tokens_ffn(ws.variant, cfg.M, cfg.K, ws.shard_N, c.rowmax_in) : few_tokens_linear(ws.variant, cfg.M, cfg.K, ws.shard_N, c.half, ws.domain->ctx->sm_count);
+    const int sms = ws.domain->ctx->sm_count;
+    const int family = ffn ? few_tokens_ffn(ws.variant, cfg.M, cfg.K, ws.shard_N, c.rowmax_in, sms) : few_tokens_linear(ws.variant, cfg.M, cfg.K, ws.shard_N, c.half, sms);
     if (family == 5 && ws.decode_cap[0] < 1) return ws.variant;
     return family == 3 && ws.KB > 8 * FUSED_MAX_STAGES ? 1 : family;
 }

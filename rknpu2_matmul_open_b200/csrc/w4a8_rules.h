@@ -83,7 +83,7 @@ inline int few_tokens_linear(int family, int M, int K, int columns, bool half, i
 // The same for the two projections of an FFN (times of the whole FFN).  The first's columns come in pairs and its quantising is fp32
 // (2048 -> 2 x 14336, 4 tokens: 22.9 / - / 17.9); the second finds its rows' maxima collected, so no kernel scans (14336 -> 1024
 // behind it 19.9 / 17.9 / 19.6, 5632 -> 2048 at 4 tokens 16.1 / 14.9 / 15.0).
-inline int few_tokens_ffn(int family, int M, int K, int columns, bool second)
+inline int few_tokens_ffn(int family, int M, int K, int columns, bool second, int sms = RULE_SMS)
 {
     const double mb = double(K) * columns / 2 / (1 << 20);
     if (second) {
@@ -91,11 +91,13 @@ inline int few_tokens_ffn(int family, int M, int K, int columns, bool second)
         if (mb <= 2) return 5;
         return columns <= 2112 && K <= 6144 ? 1 : family;
     }
-    if (K <= 2048 && columns > 2 * 148 * 32) return columns < 16384 && M <= 4 ? 3 : 1;
+    if (K <= 2048 && columns > 2 * 32 * sms) return columns < 16384 && M <= 4 ? 3 : 1;
     if (K % 4 && M >= 4) return 1;
     if (M <= 2 && mb >= 50 && (M == 2 || K >= 8192)) return 1;       // 1 x 8192 -> 2 x 7168 27.6 / - / 25.1
     if (M <= 4) return family;
-    return K >= 8192 && mb <= 26 ? 1 : 5;
+    // 8 x 3840 -> 2 x 2496 -> 3840 with the decode kernel in front 18.0, with the ring 15.5 (clusters 16.6); 2560 -> 2 x 6912 18.7 and
+    // 15.9, 5120 -> 2 x 3456 17.7 and 16.3; but 2048 -> 2 x 5632 14.3 and 14.4, 4096 -> 2 x 5504 17.7 and 18.1, 4096 -> 2 x 11008 25.3 and 27.7
+    return K > 2048 && (K < 4096 || K >= 5120) ? 1 : 5;
 }
 
 // 9..16 tokens of very small weights: whether one launch (the split-K kernel, whose every cluster scans all of the rows) is left for

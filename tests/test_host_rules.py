@@ -266,6 +266,12 @@ int main()
         const int from = c.M <= 4 || (long long)c.K * c.cols / 2 > (24 << 20) ? 5 : 3;        // the workspace's
         if (few_tokens_linear(from, c.M, c.K, c.cols, c.half) != c.family) { printf("%d x %d -> %d half %d\n", c.M, c.K, c.cols, c.half); return 1; }
     }
+    const Case first[] = {       // columns: two a feature
+        {5, 1024, 4096, false, 5}, {8, 2048, 11264, false, 1}, {5, 2048, 8192, false, 5}, {5, 2560, 13824, false, 1}, {6, 3840, 4992, false, 1}, {8, 3840, 9984, false, 1}, {8, 4096, 4096, false, 5},
+        {8, 4096, 22016, false, 5}, {5, 5120, 6912, false, 1}, {8, 5120, 27648, false, 1}, {8, 6144, 8192, false, 1}, {5, 8192, 7168, false, 1}, {4, 4096, 22016, false, 5}, {4, 2048, 11264, false, 3},
+    };
+    for (const Case& c : first)
+        if (few_tokens_ffn(5, c.M, c.K, c.cols, false) != c.family) { printf("%d x %d -> %d first\n", c.M, c.K, c.cols); return 1; }
     for (int M = 1; M <= 8; ++M)
         for (int K = 1; K < 20000; K += 37)
             for (int cols = 1; cols < 40000; cols += 401)
