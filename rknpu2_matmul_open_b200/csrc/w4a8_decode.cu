@@ -29,6 +29,7 @@
 #include "w4a8_device.h"
 #include "w4a8_math.cuh"
 #include "w4a8_ptx.cuh"
+#include "w4a8_rules.h"
 
 namespace rkb200 {
 
@@ -538,16 +539,7 @@ int gemm_decode_ring(int M, int KB, bool swiglu)
     return ring < DEC_MAX_RING ? ring : DEC_MAX_RING;
 }
 
-// Cluster size (= how many CTAs share the quantisation).  Quantising a 16-element unit costs a thread about 500
-// cycles of issue slots and the exchange about as much as one and a half units, so up to three units per thread
-// stay local; beyond that four CTAs share (clusters of eight leave half of this GPU's SMs without a CTA).  fp32 rows are
-// twice the loads and the higher token slots more work per unit: two units (8 x 1536 -> 4096 fp32 6.4 us with 768, 5.3;
-// binary16 5.5 and 5.3; at 3072 -> 8192 with 4 tokens of binary16 the exchange costs more, 6.5 with 768 and 7.7).
-int gemm_decode_cluster(int M, int KB, bool half)
-{
-    const long long units = (long long)dec_token_slots(M) * KB * 8;
-    return units <= (half && M <= 4 ? 768 : 512) ? 1 : 4;
-}
+int gemm_decode_cluster(int M, int KB, bool half) { return decode_cluster(M, (long long)dec_token_slots(M) * KB * 8, half); }
 
 // CTAs: every resident CTA that has an item to work on (a multiple of the cluster size).  A launch lasts as long as
 // its busiest CTA, ceil(items / CTAs) items, which no smaller grid improves; more CTAs bring more copy engines.

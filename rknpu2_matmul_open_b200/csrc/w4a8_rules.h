@@ -26,6 +26,14 @@ inline bool result_over_bus(int family, int M, size_t cols, size_t elem)
     return bytes <= (elem == 2 ? size_t(40) << 10 : size_t(64) << 10);
 }
 
+// Cluster size of the decode kernel (= how many CTAs share the quantisation) for `units` of 16 elements, token slots included.
+// Quantising a unit costs a thread about 500 cycles of issue slots and the exchange about as much as one and a half units, so up to
+// three units per thread stay local; beyond that four CTAs share (clusters of eight leave half of this GPU's SMs without a CTA).  fp32
+// rows are twice the loads and the higher token slots more work per unit: two units (8 x 1536 -> 4096 fp32 6.4 us with 768, 5.3; binary16
+// 5.5 and 5.3; at 3072 -> 8192 with 4 tokens of binary16 the exchange costs more, 6.5 with 768 and 7.7).  A single row is little either
+// way, and CTAs with several groups of channels wait for each other: fp32 11008 -> 6144 14.4 with 768, 16.1 with 512, -> 11008 19.2 and 21.1.
+inline int decode_cluster(int M, long long units, bool half) { return units <= (M == 1 || (half && M <= 4) ? 768 : 512) ? 1 : 4; }
+
 // CTAs (of a cluster) that share a column tile of the ring: the smallest number that gives nearly every SM a CTA.  More only adds
 // reduction traffic and shortens each CTA's stream, and more than 33 clusters of eight or 66 of four need not be resident at once (two
 // CTAs an SM, whole clusters in a GPC), which costs a second round.  (Until every SM had one: 34 tiles in eight parts, 12 x 4096 ->

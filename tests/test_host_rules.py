@@ -286,3 +286,21 @@ int main()
     return 0;
 }
 """)
+
+
+def test_ctas_of_a_cluster_that_share_the_quantisation(tmp_path):
+    # units of 16 elements a token; fp32 rows of one token were measured up to 12288 elements, with and without a partner
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+struct Case { int M, units; bool half; int ctas; };
+int main()
+{
+    const Case cases[] = {{1, 576, false, 1}, {1, 688, false, 1}, {1, 768, false, 1}, {1, 776, false, 4}, {1, 768, true, 1}, {1, 896, true, 4}, {2, 512, false, 1}, {2, 768, false, 4},
+                          {2, 768, true, 1}, {4, 768, true, 1}, {4, 768, false, 4}, {8, 512, true, 1}, {8, 768, true, 4}, {8, 576, false, 4}};
+    for (const Case& c : cases)
+        if (decode_cluster(c.M, c.units, c.half) != c.ctas) { printf("%d tokens, %d units, half %d\n", c.M, c.units, c.half); return 1; }
+    return 0;
+}
+""")
