@@ -47,45 +47,88 @@ inline int ring_parts(long long tiles, int KB, int sms)
 }
 
 // Up to eight tokens: the family that runs a call of a workspace of family 3 (split-K clusters) or 5 (decode); the code layout is the
-// ring's (1) too.  Measured on 60 shapes of both types alone (times of one call of a back-to-back series in us, decode / clusters /
-// ring; with weights from HBM as with weights in L2) and in decoder layers, one call behind another.
-//   * The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3 at
-//     least, whatever the rows: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32
-//     7.8 / 7.9 / 6.3, 4 x 8192 -> 8192 13 / 12.7 / 10.1, 8 x 4096 -> 14336 13.9 / 13.8 / 9.5, 8 x 3070 -> 4911 10.3 / 13.3 / 7.5).
-//   * The clusters hold all of their weights in shared memory and are good while a CTA has one column tile, up to 12.5 MB of weights on
-//     148 SMs (fused_tiles_per_cta); of two the second's contraction, exchange and finish run behind the first's (8 x 4096 -> 6144
-//     9.8 / 7.1 / 6.9, -> 6784 9.4 / 9.7 / 7.0).
-//   * The decode kernel's CTAs take 32 channels over all of K: best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2) and few tokens,
-//     poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.5 / 6.9) and where some CTAs have two groups of channels
-//     (4 x 5120 -> 5120 9.1 / 7.0 / 7.3).
+// ring's (1) too.  Measured on 33 shapes of both types, the times are of one call of a back-to-back series in us, decode / clusters /
+// ring.  The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3
+// at least: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32 7.8 / 7.9 / 6.5,
+// 4 x 8192 -> 8192 13 / 12.6 / 10.6, 8 x 3070 -> 4911 10.3 / 13.2 / 7.6).  The decode kernel's CTAs take 32 channels over all of K:
+// best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2), poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.4 / 7.2) and
+// where some CTAs have two groups of channels (4 x 5120 -> 5120 9.0 / 7.0 / 7.9).
 constexpr int RULE_SMS = 148;
+
+// How much of its rounds a launch fills: `ctas` of equal work, `places` at once.
+inline double filled(long long ctas, long long places) { return double(ctas) / double((ctas + places - 1) / places * places); }
+
+// The ring's CTAs, `parts` of K for each column tile, two an SM.  Where the last round leaves more than three eighths of the places
+// empty, SMs with one CTA stream with half of their bandwidth: 4096 -> 14336, 224 CTAs, 9.5 us, -> 18944, 148 CTAs, 14.9.  In four
+// parts and more a CTA's stream is short and that costs little.
+struct RingFill {
+    int parts;
+    double used;
+    bool fills, thin;
+    RingFill(int K, int columns, int sms)
+    {
+        const long long tiles = (columns + 127) / 128;
+        parts = ring_parts(tiles, (K + 127) / 128, sms);
+        used = filled(tiles * parts, 2 * sms);
+        fills = used >= 0.625;
+        thin = !fills && parts <= 2;
+    }
+};
+
 inline int few_tokens_linear(int family, int M, int K, int columns, bool half, int sms = RULE_SMS)
 {
     const double mb = double(K) * columns / 2 / (1 << 20);          // of weights
     const bool ragged = K % (half ? 8 : 4) != 0;
-    const bool one_tile = mb * RULE_SMS <= 12.5 * sms;
     const int groups = (columns + 31) / 32;
+    const RingFill ring(K, columns, sms);
+    // The clusters hold their weights in shared memory: on 148 SMs a CTA has one column tile up to 12.5 MB (fused_tiles_per_cta) and
+    // two beyond, and from about 28 MB on they are not resident at once (3 x 11008 -> 6144 11.5 / 22.4 / -, 6 fp32 17.2 / 25.0 / -).
+    const bool one_tile = mb * RULE_SMS <= 12.5 * sms, one_round = mb * RULE_SMS <= 28. * sms;
     if (M > 4) {
-        if (K <= 2560 && mb <= 4.5) return 5;
-        if (ragged) return 1;
-        // few channels, where a launch less counts for more: 8 x 4096 -> 1024 5.7 / 5.5 / 6.3, 5 x 11008 -> 1024 fp32 12.8 / 7.3 / 8.5
-        if (half) return one_tile && (K <= 1024 || (columns <= 2112 && K >= 4096)) ? 3 : 1;
-        return M <= 6 && one_tile && (columns <= 1024 || (columns <= 2112 && K >= 8192)) ? 3 : 1;
+        if (K <= 3072 && mb <= 4.5) return 5;
+        if (ragged) return half && M <= 6 && K >= 4096 && mb <= 11.2 ? 3 : 1;       // 5 x 4405 -> 1792 8.4 / 7.4 / 8.3, -> 6000 12.7 / 10.6 / 9.7
+        if (half) {
+            // 8 x 3072 -> 8192 9.0 / 7.1 / 7.0, 2048 -> 14336 8.9 / 9.7 / 6.9, 4096 -> 8320 9.5 / 9.7 / 7.6.  Where the ring is thin:
+            //   * 5 x 6144 -> 9216 11.1 / 13.1 / 12.8, 8 x 8192 -> 11008 15.0 / 26.7 / 15.8, 4608 -> 11008 13.8 / 12.4 / 10.3;
+            //   * the clusters are near alone and in front in a chain (4096 -> 11008 11.7 / 10.1 / 9.3, layers of 4096 / 11008 with 8 tokens
+            //     65.9 / 61.3 / 62.7, of 4096 / 11776 65.5 / 61.4 / 63.3); beyond they are not (4096 -> 12288 11.8 / 12.6 / 9.4, -> 14336
+            //     13.8 / 13.8 / 9.7, layers of 4096 / 14336 70.7 / 73.4 / 65.2); short rows are quantised sooner (2048 -> 22528 11.8 / 10.2 / 9.0).
+            if (mb <= 13.25) return family;
+            if (ring.thin && K >= 5120) return 5;
+            return mb > 20 && family == 3 && (K <= 1280 || (K > 3072 && K <= 4096 && ring.thin)) ? 3 : 1;    // 8 x 1024 -> 49152 15.8 / 9.5 / 11.2
+        }
+        if (columns <= 1024 || (K >= 8192 && columns <= 2112 && M <= 6)) return 3;
+        return M <= 6 && one_tile && groups > 144 && groups <= 192 ? 3 : 1;
     }
-    if (columns <= 2112 && (K >= 8192 || (K >= 6144 && (M > 1 || !half))) && (M <= 2 || !half || one_tile)) return 3;
-    if (one_tile && groups > 144 && groups <= (half ? 192 : 240) && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
-    if (one_tile && !half && groups > 144 && groups <= 296 && M > 2 && K >= 3072) return 3;      // 4 x 3072 -> 8192 7.7 / 6.7 / 6.5
+    if (columns <= 2112 && (K >= 8192 || (K >= 6144 && (M > 1 || !half)))) return 3;
+    // (In a chain of binary16 calls 3 x 3584 -> 7680, 240 groups, takes the decode kernel 1 less; 4 x 4096 -> 6144, 192 groups, the clusters
+    // 1.4.)  fp32: 3 x 4096 -> 7168 8.3 / 9.4 / 6.9
+    if ((half && M > 2 ? one_round && K < 10240 : one_tile) && groups > 144 && groups <= (half ? 192 : 240) && !ragged && M > 1 && K > (M == 2 ? 4096 : 3072)) return 3;
+    if (!half && (one_tile || (ragged && M == 3 && mb < 14)) && groups > 144 && groups <= 296 && M > 2 && K >= 3072) return 3;      // 4 x 3072 -> 8192 7.7 / 6.7 / 6.5
     if (K <= 1024 && groups > 296) return 3;                         // 4 x 1024 -> 14336 6.1 / 5.6 / 6.3
     if (ragged && M == 4 && mb > 4) return 1;
-    // The ring's two CTAs an SM: with hardly more than one each it is no faster than the decode kernel (4 x 4096 -> 14336, 224 CTAs,
-    // 11.0 / 12.2 / 9.4, but -> 18944, 148 CTAs, 13.2 / 13.3 / 13.9; -> 11008, 172, 10.5 / 9.7 / 9.3 alone, in a layer 0.3 behind decode).
-    const long long tiles = (columns + 127) / 128;
-    const bool fills = tiles * ring_parts(tiles, (K + 127) / 128, sms) * 4 >= sms * 5ll;
-    // Long rows of 112 to 148 groups stay: 3 x 11008 -> 4096 9.1 / 10.9 / 9.1 alone, in a layer the ring is 4 behind.
-    if (M > 2) return !ragged && !one_tile && K < 10240 && (fills || K >= 5120) ? 1 : family;
-    // Two tokens cost the decode kernel less: fp32 4096 -> 11008 8.6 / 9.5 / 9.2, -> 14336 10.4 / 11.0 / 9.4, 5120 -> 6912 9.7 / 9.4 / 7.6
-    if (M == 2 && ((mb >= 14 && K >= (half ? 8192 : 5120)) || (!half && mb >= 28 && K >= 4096 && fills))) return 1;
-    return mb >= 40 ? 1 : family;
+    if (M > 2) {
+        // 4 x 6144 -> 11008 14.0 / 13.6 / 12.5, 4 x 8192 -> 9216 15.8 / 22.9 / 14.4; in one part 4 x 6144 -> 18944 17.9 / 24.8 / 21.1
+        const bool pays = ring.fills || (K >= 4608 && ring.parts > 1);
+        // (in a chain 4 x 4096 -> 11008 of binary16 takes the decode kernel 0.9 less than the ring)
+        if (half) return mb >= 14 && K <= 8192 && (mb >= 26 || K >= 6144) && pays ? 1 : family;
+        // long rows of 112 to 148 groups stay: 3 x 11008 -> 4096 9.1 / 10.9 / 9.1 alone, in a layer the ring is 4 behind
+        return !ragged && !one_tile && K < 10240 && pays ? 1 : family;
+    }
+    // Two tokens cost the decode kernel less: fp32 4096 -> 11008 8.6 / 9.5 / 9.2, -> 12544 8.8 / 10.8 / 9.3, -> 14336 10.5 / 11.2 / 9.4,
+    // 5120 -> 6912 9.8 / 9.4 / 7.6, binary16 5120 -> 6144 8.6 / 9.6 / 7.5; where the ring is thin it is behind unless the decode kernel's
+    // last round is as empty (fp32 5120 -> 9216, 288 groups, 10.5 / 9.8 / 10.9, -> 11008, 344 groups, 12.9 / 11.8 / 11.0).
+    const double decode_used = filled(groups, sms);
+    const bool better = ring.fills || decode_used < 0.85;
+    if (M == 2) {
+        if (half && mb >= 14 && K >= 8192 && !ring.thin && better) return 1;
+        if (half && !one_tile && groups > sms && groups <= 192 && !ragged && K > 4096) return 1;
+        if (!half && mb >= 14 && (K >= 5120 || (ragged && K >= 4096)) && better) return 1;
+        if (!half && mb >= 28 && K >= 4096 && ring.fills) return 1;
+        return mb >= 40 && !ring.thin ? 1 : family;
+    }
+    // One token: 8192 -> 11008 14.0 / 22.4 / 15.6, -> 12416 14.2 / - / 15.6, -> 14336 17.0 / - / 15.7, 11008 -> 8192 13.6 / - / 12.5
+    return mb >= 40 && ring.used > 0.9 * decode_used ? 1 : family;
 }
 
 // The same for the two projections of an FFN (times of the whole FFN).  The first's columns come in pairs and its quantising is fp32

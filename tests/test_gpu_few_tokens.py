@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 # (M, K, N, launches of a call with fp32 rows, with binary16 rows)
 LINEAR = [(1, 8192, 512, 1, 1), (1, 1024, 9500, 1, 1), (3, 3200, 4640, 1, 1), (4, 2044, 4400, 1, 2), (5, 1500, 2048, 1, 1), (5, 3070, 3100, 2, 2),
-          (6, 4096, 1040, 2, 1), (6, 4096, 1024, 1, 1), (8, 4096, 1024, 2, 1), (8, 2048, 1056, 1, 1), (8, 2048, 3200, 1, 1), (7, 1500, 2048, 1, 1), (8, 3104, 3104, 2, 2), (7, 2624, 3520, 2, 2), (4, 4096, 6464, 2, 2), (2, 4096, 7328, 1, 1),
+          (6, 4096, 1040, 2, 1), (8, 4096, 1024, 1, 1), (8, 2048, 1056, 1, 1), (8, 2048, 3200, 1, 1), (7, 1500, 2048, 1, 1), (8, 3104, 3104, 2, 1),
           (9, 1024, 512, 1, 1), (9, 1024, 520, 2, 2), (16, 1030, 2050, 2, 2)]
 
 
@@ -104,3 +104,28 @@ def test_ring_parts_of_padded_tiles(gpu, oracle, monkeypatch, M, split):
         assert np.array_equal(bits(top[:M]), maxima) and top[M] == 0
     for o in (ws, gu, w, wg):
         o.free()
+
+
+# sizes on the rule's lines by the rounds of the three kernels
+LINES = [(7, 4100, 1000, 1, 2), (5, 4100, 1000, 1, 1), (2, 5120, 5632, 1, 2), (4, 4096, 6464, 2, 1), (8, 5120, 9216, 2, 1), (3, 3584, 7680, 2, 1), (6, 5120, 5184, 2, 1),
+         (2, 4102, 7200, 2, 1), (8, 4096, 11776, 2, 1), (8, 4096, 12288, 2, 2), (1, 8320, 4768, 1, 1)]
+
+
+@pytest.mark.parametrize("M,K,N,fp32,binary16", LINES)
+def test_linear_where_the_ring_is_thin(gpu, oracle, M, K, N, fp32, binary16):
+    _, dom, _ = gpu
+    B, sw = make_weights(K, N, seed=K)
+    w, ws = rk.Weights(dom, B, sw), rk.Workspace(dom, rk.default_config(M, N, K))
+    stream = torch.cuda.current_stream().cuda_stream
+    for d, launches in (("f32", fp32), ("f16", binary16)):
+        a = make_activations(M, K, seed=M, dtype=d)
+        ref, half = oracle.linear(a, B, sw)[1], d == "f16"
+        da = torch.from_numpy(a.view(np.int16) if half else a).cuda()
+        do = torch.zeros((M, N), dtype=da.dtype, device="cuda")
+        before = ws.launch_count()
+        assert (ws.enqueue_f16 if half else ws.enqueue_f32)(w, da, do, stream) == 0
+        torch.cuda.synchronize()
+        assert ws.launch_count() - before == launches, d
+        assert ws.finish() == 0 and np.array_equal(bits(do.cpu().numpy().view(ref.dtype)), bits(ref)), d
+    ws.free()
+    w.free()
