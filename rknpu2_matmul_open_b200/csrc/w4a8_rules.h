@@ -144,11 +144,15 @@ inline int few_tokens_ffn(int family, int M, int K, int columns, bool second, in
     }
     if (K <= 2048 && columns > 2 * 32 * sms) return columns < 16384 && M <= 4 ? 3 : 1;
     if (K % 4 && M >= 4) return 1;
-    if (M <= 2 && mb >= 50 && (M == 2 || K >= 8192)) return 1;       // 1 x 8192 -> 2 x 7168 27.6 / - / 25.1
+    // The ring's one part is slow where it is thin, on longer rows above all: 5 x 3072 -> 2 x 11008 23.0 and 20.6, but 5120 -> 2 x 9472 23.7 and
+    // 26.9, 8192 -> 2 x 9472 29.5 and 36.3, 1 x 8192 -> 2 x 9472 27.1 and 35.1; in two parts 5 x 6144 -> 2 x 4608 19.6 and 19.5.
+    const RingFill ring(K, columns, sms);
+    const bool pays = ring.fills || ring.parts > 1;
+    if (M <= 2 && mb >= 50 && (M == 2 || K >= 8192) && (pays || K <= 5120)) return 1;       // 1 x 8192 -> 2 x 7168 27.6 / - / 25.1
     if (M <= 4) return family;
     // 8 x 3840 -> 2 x 2496 -> 3840 with the decode kernel in front 18.0, with the ring 15.5 (clusters 16.6); 2560 -> 2 x 6912 18.7 and
     // 15.9, 5120 -> 2 x 3456 17.7 and 16.3; but 2048 -> 2 x 5632 14.3 and 14.4, 4096 -> 2 x 5504 17.7 and 18.1, 4096 -> 2 x 11008 25.3 and 27.7
-    return K > 2048 && (K < 4096 || K >= 5120) ? 1 : 5;
+    return K > 2048 && (K < 4096 || K >= 5120) && (pays || K < 3328) ? 1 : 5;
 }
 
 // 9..16 tokens of very small weights: whether one launch (the split-K kernel, whose every cluster scans all of the rows) is left for

@@ -321,3 +321,24 @@ int main()
     return 0;
 }
 """)
+
+
+def test_first_projections_where_the_ring_is_thin(tmp_path):
+    # columns: two a feature; no slower than the decode kernel, which is the workspace's own, and no slower than the ring by more than 5 %
+    # where K is at least 5120 or up to 3328
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+struct Case { int M, K, cols, family; };
+int main()
+{
+    const Case cases[] = {
+        {1, 8192, 14336, 1}, {1, 8192, 18944, 5}, {2, 5120, 22016, 1}, {2, 6144, 18944, 5}, {4, 4096, 22016, 5}, {5, 3072, 22016, 1}, {5, 3584, 18944, 5}, {8, 4096, 22016, 5}, {5, 5120, 18944, 5},
+        {5, 6144, 9216, 1}, {8, 6144, 22016, 5}, {8, 8192, 11008, 1}, {5, 8192, 18944, 5}, {8, 8192, 22016, 5}, {8, 5120, 27648, 1}, {8, 3840, 4992, 1},
+    };
+    for (const Case& c : cases)
+        if (few_tokens_ffn(5, c.M, c.K, c.cols, false) != c.family) { printf("%d x %d -> %d\n", c.M, c.K, c.cols); return 1; }
+    return 0;
+}
+""")
