@@ -84,3 +84,45 @@ def test_a_verdict_is_reported_once(gpu, oracle, monkeypatch, family, M, N):
     assert ws.finish() == 0 and np.array_equal(bits(out.cpu().numpy()), bits(ref))
     ws.free()
     w.free()
+
+
+# kernel family, cut of the persistent kernel, tokens (families 3 and 5 have tickets of their own)
+@pytest.mark.parametrize("family, cut, M", [(1, None, 12), (1, None, 40), (2, "32,1,0,1", 40), (2, "64,1,0,3", 129), (2, "32,5,2,1", 200), (4, None, 24), (3, None, 8), (5, None, 4)])
+def test_ffn_calls_good_and_bad_in_turn(gpu, oracle, monkeypatch, family, cut, M):
+    # one pair of workspaces: NaN in the input, a middle that is not finite, in between good calls with small and large maxima
+    _, dom, _ = gpu
+    monkeypatch.setenv("RK_NPU_B200_VARIANT", str(family))
+    if cut:
+        monkeypatch.setenv("RK_NPU_B200_PERSIST_CUT", cut)
+    K, F, N = 1024, 1152, 260
+    (Bg, sg), (Bd, sd) = make_weights(K, 2 * F, seed=1), make_weights(F, N, seed=2)
+    huge = np.where(np.arange(2 * F) % 64 == 5, np.float32(1e30), sg).astype(np.float32)
+    wg, wh, wd = rk.Weights(dom, Bg, sg), rk.Weights(dom, Bg, huge), rk.Weights(dom, Bd, sd)
+    gu, dn = (rk.Workspace(dom, rk.default_config(M, n, k)) for n, k in ((2 * F, K), (N, F)))
+    good = make_activations(M, K, seed=M, dtype="f32")
+    nan = good.copy()
+    nan[M - 1, K - 1] = np.nan
+    rows = {"good": good, "large": 30 * good, "nan": nan, "overflow": good}
+    ref = {kind: oracle.ffn(rows[kind], Bg, sg, Bd, sd, mode=1) for kind in ("good", "large")}
+    dev = {kind: torch.from_numpy(np.ascontiguousarray(a)).cuda() for kind, a in rows.items()}
+    turns = ["large", "nan", "good", "overflow", "good", "nan", "overflow", "large", "good"]
+    mids, outs = ([torch.full((M, n), -7.0, device="cuda") for _ in turns] for n in (F, N))
+    stream = torch.cuda.current_stream().cuda_stream
+    for kind, mid, out in zip(turns, mids, outs):
+        assert rk.enqueue_ffn_f32(gu, wh if kind == "overflow" else wg, dn, wd, dev[kind], mid, out, stream) == 0
+    torch.cuda.synchronize()
+    assert gu.finish() == 0 and dn.finish() == 0
+    for i, (kind, mid, out) in enumerate(zip(turns, mids, outs)):
+        mid, out = mid.cpu().numpy(), out.cpu().numpy()
+        if kind in ref:
+            assert np.array_equal(bits(mid), bits(ref[kind]["middle"])) and np.array_equal(bits(out), bits(ref[kind]["C"])), (i, kind)
+        else:
+            assert np.all(mid == -7.0) if kind == "nan" else not np.isfinite(mid).all() and np.all(out == -7.0), (i, kind)
+    middle, result = np.zeros((M, F), np.float32), np.zeros((M, N), np.float32)
+    for kind, w in (("overflow", wh), ("good", wg), ("nan", wg), ("large", wg), ("good", wg)):
+        rc = rk.run_ffn_f32(gu, w, dn, wd, rows[kind], middle, result)
+        assert rc == (0 if kind in ref else capi.RK_NPU_ERR_PARAM), kind
+        if kind in ref:
+            assert np.array_equal(bits(middle), bits(ref[kind]["middle"])) and np.array_equal(bits(result), bits(ref[kind]["C"])), kind
+    for o in (gu, dn, wg, wh, wd):
+        o.free()
