@@ -152,12 +152,16 @@ int rk_npu_b200_w4a8_last_quant(rk_npu_w4a8_workspace *workspace, float *scales,
 /* Scheduling override for experiments and tuning.  variant: 0 = keep, else the workspace's kernel family
  * (1 quantise + mma.sync GEMM, 2 quantise + tcgen05 GEMM, 3 single-kernel split-K small batch, 4 quantise +
  * persistent tcgen05 streaming GEMM, 5 single-kernel decode with whole-K CTAs; chosen at creation,
- * RK_NPU_B200_VARIANT overrides where the geometry allows).  The family is fixed with the activation-code layout at
- * creation, except that a workspace of up to eight tokens may move between 3 and 5, which share it.
+ * RK_NPU_B200_VARIANT overrides where the geometry allows).  The activation-code layout is fixed at creation, so a
+ * family that is asked for has to be the workspace's own, or the other of 3 and 5 up to eight tokens, which share it.
+ * While the family is the library's choice and split_k is automatic, a workspace of family 3 or 5 may run single calls
+ * in another of 1, 3 and 5, by the call's rows, type and channels (results that go over the bus stay); a family that
+ * was named here or by RK_NPU_B200_VARIANT runs every call.
  * split_k: 0 = automatic, else the number of CTAs that cooperate on a column tile: the split-K factor (1..8 for
  * family 3; 1, 2, 4, 8 for 1) or the decode kernel's cluster size (1, 2, 4, 8); ignored by families 2 and 4.
  * Returns RK_NPU_ERR_PARAM when the workspace geometry cannot run the request.
- * rk_npu_b200_w4a8_schedule reads both back (either pointer may be NULL). */
+ * rk_npu_b200_w4a8_schedule reads both back (either pointer may be NULL): the workspace's family, not that of its last
+ * call; rk_npu_b200_w4a8_launch_count tells them apart (families 3 and 5 launch once a call, 1 twice). */
 int rk_npu_b200_w4a8_set_schedule(rk_npu_w4a8_workspace *workspace, int variant, int split_k);
 int rk_npu_b200_w4a8_schedule(const rk_npu_w4a8_workspace *workspace, int *variant, int *split_k);
 
