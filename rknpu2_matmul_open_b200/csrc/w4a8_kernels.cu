@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(BS, (UN <= 4 ? 1280 : 896) / BS) quantize_rows
     pdl_launch_dependents();   // the GEMM behind this kernel may start prefetching weights
     if (SCAN) prefetch_row(p.A, (size_t)p.K * (HALF ? 2 : 4));
     pdl_wait();                // A may be the output of the kernel in front of this one
-    quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, RowQuant<HALF>{p.scales, p.rowmax, &p.status->bad_accum});
+    quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.K, p.Kp, p.T, RowQuant<HALF>{p.scales, p.rowmax, &p.status->bad_accum});
 }
 
 // Any row: one CTA per token.
@@ -519,7 +519,7 @@ cudaError_t launch_gemm_mma(const GemmParams& p, int tokens_per_cta, cudaStream_
 namespace {
 constexpr int STATIC_MAX_TOKENS = 32;
 constexpr size_t STATIC_CODE_BYTES = size_t(2) << 20;               // activation codes: tokens_per_cta x padded K bytes
-constexpr size_t STATIC_SCRATCH_BYTES = STATIC_CODE_BYTES + 4096;   // + scales, inverse scales, status block
+constexpr size_t STATIC_SCRATCH_BYTES = STATIC_CODE_BYTES + 4096;   // + scales, status block
 }
 static __device__ __align__(256) unsigned char g_static_scratch[STATIC_SCRATCH_BYTES];
 

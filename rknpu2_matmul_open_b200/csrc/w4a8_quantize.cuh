@@ -41,10 +41,10 @@ __device__ __forceinline__ void prefetch_row(const void* A, size_t row_bytes)
 }
 
 // UN: 16-byte loads a thread keeps.  Op: max_of(best, 16 bytes as loaded) -> best; join(best, best) -> best, join_warp over a warp;
-// begin(token, best, one thread of the row's) -> inverse scale; the scales are written by that thread; word(x0..x3, inverse) -> four
+// begin(token, best) -> inverse scale, called by one thread of the row's, which writes the scale; word(x0..x3, inverse) -> four
 // codes.  SCAN false: the maxima are collected(token).
 template <bool HALF, bool SCAN, int UN, class Op>
-__device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int M, int K, int Kp, int T, Op op)
+__device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int K, int Kp, int T, Op op)
 {
     constexpr int EPW = PIECE<HALF>, LPU = 16 / EPW;     // lanes per 16-element unit
     __shared__ uint32_t s_part[16];
@@ -75,9 +75,9 @@ __device__ __forceinline__ void quantize_rows(const void* A, uint8_t* Xq, int M,
         if (tid == 0) {
             uint32_t all = 0;
             for (int w = 0; w < threads >> 5; ++w) all = op.join(all, s_part[w]);
-            s_inverse = op.begin(m, all, true);
+            s_inverse = op.begin(m, all);
         }
-    } else if (tid == 0) s_inverse = op.begin(m, op.collected(m), true);
+    } else if (tid == 0) s_inverse = op.begin(m, op.collected(m));
     __syncthreads();
     const float inv = s_inverse;
     const int mt = m / T, t = m - mt * T;
@@ -119,9 +119,9 @@ struct RowQuant {
     }
     static constexpr bool CHECKS = false;
     static constexpr uint32_t LEAST_BAD = 0xffffffffu;
-    // a row's maximum where it was collected and not scanned; the inverse of its scale (`store`: by one thread of the row's)
+    // a row's maximum where it was collected and not scanned; the inverse of its scale
     __device__ __forceinline__ uint32_t collected(int m) const { return __ldcg(rowmax + m); }
-    __device__ __forceinline__ float begin(int m, uint32_t bits, bool store = true) const
+    __device__ __forceinline__ float begin(int m, uint32_t bits) const
     {
         float maximum;
         int bad;
@@ -134,10 +134,8 @@ struct RowQuant {
         }
         float s, inv;
         scale_from_max(maximum, bad != 0, s, inv);
-        if (store) {
-            scales[m] = s;
-            if (bad) *bad_word = bad;     // (the same value from every bad row of a launch)
-        }
+        scales[m] = s;
+        if (bad) *bad_word = bad;         // (the same value from every bad row of a launch)
         return inv;
     }
     __device__ __forceinline__ uint32_t word(float a, float b, float c, float d, float inv) const
@@ -181,7 +179,7 @@ struct W8RowQuant {
     // The sign of the inverse says how its row is rounded: positive, no product is a NaN or rounds beyond 127 (the scale is that of
     // the row, and normal), as in the W4A8 rule; negative, with the checks; a NaN: the scale is not positive (an underflowed maximum),
     // the codes are zeros.
-    __device__ __forceinline__ float begin(int m, uint32_t bits, bool store = true) const
+    __device__ __forceinline__ float begin(int m, uint32_t bits) const
     {
         float s;
         const uint32_t magnitude = bits & ~CAREFUL;
@@ -190,7 +188,7 @@ struct W8RowQuant {
             const float maximum = HALF ? __half2float(__ushort_as_half((uint16_t)magnitude)) : __uint_as_float(magnitude);
             s = maximum > 0.f ? __fdiv_rn(maximum, 127.0f) : 1.0f;
         }
-        if (store) scales[m] = s;
+        scales[m] = s;
         if (!(s > 0.f)) return __int_as_float(0x7fffffff);
         const float inv = __frcp_rn(s);
         return static_scale || (bits & CAREFUL) || s < FLT_MIN ? -inv : inv;

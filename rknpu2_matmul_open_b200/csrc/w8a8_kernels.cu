@@ -57,7 +57,7 @@ template <bool HALF, bool SCAN, int BS, int UN>
 __global__ void __launch_bounds__(BS, (UN <= 4 ? 1280 : 896) / BS) w8_quantize_rows_kernel(const W8QuantParams p)
 {
     pdl_launch_dependents();   // the GEMM behind this kernel may set itself up and request its weights
-    quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.M, p.K, p.Kp, p.T, W8RowQuant<HALF>{p.static_scale, p.scales});
+    quantize_rows<HALF, SCAN, UN>(p.A, p.Xq, p.K, p.Kp, p.T, W8RowQuant<HALF>{p.static_scale, p.scales});
 }
 
 // The same for any row: one CTA per token.
