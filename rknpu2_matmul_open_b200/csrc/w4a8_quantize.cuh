@@ -235,9 +235,12 @@ __device__ __forceinline__ void exchange_piece(uint32_t* words, int lane, const 
 template <bool HALF>
 inline bool quantize_rows_ok(const void* A, int K) { return (reinterpret_cast<uintptr_t>(A) & 15u) == 0 && K % PIECE<HALF> == 0; }
 // Calls f with the shape of the launch: <threads, loads a thread keeps>, a CTA for each token.  The threads' loads just hold the row,
-// as far as they go.  Up to 591 tokens (four a SM) all CTAs are resident anyway and half the loads on twice the threads are faster
-// (with the GEMM behind it, 256 x 8 loads against 512 x 4: 300 x 8192 fp32 21.7 -> 21.0 us; 512 x 8 against 128 x 4: 200 x 1024
-// binary16 11.6 -> 9.7, 400 x 2048 fp32 11.0 -> 9.7).  Beyond, CTAs in line behind each other: fewer threads a row, more of the row
+// as far as they go.  Up to 591 tokens (four a SM) all CTAs of up to 256 threads are resident and half the loads on twice the threads
+// are faster (with the GEMM behind it, 512 x 8 loads against 128 x 4: 200 x 1024 binary16 11.6 -> 9.7 us, 400 x 2048 fp32 11.0 -> 9.7), but of
+// 512 threads only two an SM are, up to 296 tokens; from there on rows that 256 x 8 loads hold take these (512 x 4 against 256 x 8: 350 x
+// 5120 fp32 16.4 -> 15.8, 400 x 8192 22.3 -> 21.4, 591 x 8192 24.8 -> 24.6, 400 x 11008 binary16 25.9 -> 25.1).  Longer ones stay, read a second
+// time in part (300 x 14336 fp32 27.3 and 27.7, 400 x 14336 33.6 and 32.3), and rows with known maxima, where it hardly matters (FFN of 300 x
+// 6144 35.1 and 35.5, of 500 41.7 and 41.2).  Beyond, CTAs in line behind each other: fewer threads a row, more of the row
 // each (2000 x 4096 fp32 256 x 4 23.1, 128 x 8 22.6; 3000 x 8192 fp32 512 x 4 50.9, 256 x 8 47.6, 128 x 8 54.1; 3000 x 11008
 // binary16 50.1, 47.9 and 50.5).  Short rows: 128 x 4 (2048 x 4096 binary16 18.1 us, 128 x 8 18.6; 700 x 2048 fp32 10.1 and 11.1),
 // but many with known maxima, which have less to wait for, 128 x 8 (FFN of 1000 x 2048 28.5 -> 27.6).
@@ -252,7 +255,10 @@ inline auto with_quantize_rows_shape(int M, int K, F f)
     using B512 = integral_constant<int, 512>;
     const int bytes = K * (16 / PIECE<HALF>);
     if (bytes <= 8192 && (SCAN || M < 592)) return f(B128{}, I4{});
-    if (M < 592) return bytes <= 16384 ? f(B256{}, I4{}) : f(B512{}, I4{});
+    if (M < 592) {
+        if (bytes <= 16384) return f(B256{}, I4{});
+        return SCAN && M > 296 && bytes <= 32768 ? f(B256{}, I8{}) : f(B512{}, I4{});
+    }
     return bytes <= 16384 ? f(B128{}, I8{}) : f(B256{}, I8{});
 }
 

@@ -55,3 +55,8 @@ def test_careful_rows(gpu, oracle, M, K, dtype):
         assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(bits(out)[~np.isnan(want)], bits(ref)[~np.isnan(want)])
     for o in (dyn, sta, w):
         o.free()
+
+
+@pytest.mark.parametrize("M, K", [(296, 8200), (297, 8200), (298, 4104), (591, 4100), (300, 8192), (297, 16384), (299, 16392), (297, 8196)])
+def test_codes_and_scales_of_long_rows_in_more_than_a_round(gpu, oracle, M, K):
+    test_codes_and_scales(gpu, oracle, M, K)
