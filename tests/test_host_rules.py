@@ -342,3 +342,25 @@ int main()
     return 0;
 }
 """)
+
+
+def test_calls_of_nine_to_sixteen_tokens(tmp_path):
+    # both sides of the lines between one launch and two: 256 KB of weights, few channels of long rows, collected maxima with up to 2112 channels
+    _run(tmp_path, r"""
+#include "w4a8_rules.h"
+#include <stdio.h>
+using namespace rkb200;
+struct Case { int M, K, cols; bool half, collected, ring; };
+int main()
+{
+    const Case cases[] = {
+        {9, 1024, 512, true, false, false}, {9, 1024, 520, true, false, true}, {16, 1024, 512, true, false, false}, {13, 1024, 512, false, false, true}, {12, 1024, 512, false, false, false},
+        {12, 1500, 300, true, false, true}, {10, 1500, 300, true, false, false}, {9, 4096, 4096, true, false, true}, {16, 2048, 8192, false, false, true},
+        {12, 11008, 1024, true, false, false}, {12, 11008, 1024, false, false, false}, {13, 11008, 1024, true, false, true}, {12, 8192, 1024, true, false, true}, {12, 11008, 1056, true, false, true},
+        {9, 4096, 2112, false, true, true}, {16, 4096, 2113, false, true, false}, {12, 11008, 1024, false, true, false}, {16, 11008, 1024, false, true, true}, {9, 512, 64, false, true, true},
+    };
+    for (const Case& c : cases)
+        if (mid_batch_call_takes_ring(c.M, c.K, c.cols, c.half, c.collected) != c.ring) { printf("%d x %d -> %d half %d collected %d\n", c.M, c.K, c.cols, c.half, c.collected); return 1; }
+    return 0;
+}
+""")
