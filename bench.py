@@ -266,6 +266,14 @@ def measure_int8_peak():
             "how": "lib/int8_peak 60000: 128x256x32 kind::i8 MMAs back to back on every SM, best of the runs"}
 
 
+def kernel_names(family, linears, launches):
+    """The kernels of a step, by the launches that were counted: a call may take the ring's two where its workspace's own family has one."""
+    ring, single = "quantize_rows_kernel + gemm_mma_kernel", {3: "gemm_fused_kernel (split-K clusters)", 5: "gemm_decode_kernel (whole-K CTAs)"}.get(family)
+    if single is None or launches >= 2 * linears:
+        return ring
+    return single + (f", {ring} for {launches - linears} of {linears} linears" if launches > linears else "")
+
+
 def run_cuda(args, rank, world, local_rank):
     import torch
     import torch.distributed as dist
@@ -463,10 +471,7 @@ def run_cuda(args, rank, world, local_rank):
                              # one read per weight byte (ncu: DRAM bytes read equal the algorithmic bytes to 0.1 %), so the
                              # traffic of a launch is its algorithmic bytes
                              "traffic": bytes_per_launch, "peak_kind": peak_kind,
-                             # (a call may take the two launches of the ring where its workspace's own family has one)
-                             "kernel": ({} if launches_per_step > len(linears) else
-                                        {3: "gemm_fused_kernel (split-K clusters)", 5: "gemm_decode_kernel (whole-K CTAs)"}).get(
-                                 linears[0]["ws"].schedule()[0], "quantize_rows_kernel + gemm_mma_kernel") + ": scan + quantise + GEMM + dequantise",
+                             "kernel": kernel_names(linears[0]["ws"].schedule()[0], len(linears), launches_per_step) + ": scan + quantise + GEMM + dequantise",
                              "frac_of_nominal": value / world / 8000.0, "nominal_peak": 8000.0,   # 8 TB/s data-sheet HBM3e
                              "bytes_per_launch": bytes_per_launch,
                              "us_per_launch": 1e3 * ms_step / len(linears)},
