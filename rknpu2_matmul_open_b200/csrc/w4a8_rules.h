@@ -46,13 +46,6 @@ inline int ring_parts(long long tiles, int KB, int sms)
     return parts;
 }
 
-// Up to eight tokens: the family that runs a call of a workspace of family 3 (split-K clusters) or 5 (decode); the code layout is the
-// ring's (1) too.  Measured on 33 shapes of both types, the times are of one call of a back-to-back series in us, decode / clusters /
-// ring.  The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3
-// at least: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32 7.8 / 7.9 / 6.5,
-// 4 x 8192 -> 8192 13 / 12.6 / 10.6, 8 x 3070 -> 4911 10.3 / 13.2 / 7.6).  The decode kernel's CTAs take 32 channels over all of K:
-// best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2), poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.4 / 7.2) and
-// where some CTAs have two groups of channels (4 x 5120 -> 5120 9.0 / 7.0 / 7.9).
 constexpr int RULE_SMS = 148;
 
 // How much of its rounds a launch fills: `ctas` of equal work, `places` at once.
@@ -67,7 +60,7 @@ struct RingFill {
     bool fills, thin;
     RingFill(int K, int columns, int sms)
     {
-        const long long tiles = (columns + 127) / 128;
+        const long long tiles = (columns + 127ll) / 128;
         parts = ring_parts(tiles, (K + 127) / 128, sms);
         used = filled(tiles * parts, 2 * sms);
         fills = used >= 0.625;
@@ -75,11 +68,18 @@ struct RingFill {
     }
 };
 
+// Up to eight tokens: the family that runs a call of a workspace of family 3 (split-K clusters) or 5 (decode); the code layout is the
+// ring's (1) too.  Measured on 33 shapes of both types and again on 146, the times are of one call of a back-to-back series in us, decode / clusters /
+// ring.  The two single launches scan and quantise the rows in every cluster, the ring has a launch of its own for that and costs 6.3
+// at least: long rows, large weights and rows without 16-byte loads are the ring's (8 x 4096 -> 4096 fp32 7.8 / 7.9 / 6.5,
+// 4 x 8192 -> 8192 13 / 12.6 / 10.6, 8 x 3070 -> 4911 10.3 / 13.2 / 7.6).  The decode kernel's CTAs take 32 channels over all of K:
+// best on short rows (8 x 2048 -> 2048 5.2 / 5.7 / 6.2), poor on few channels of long rows (4 x 8192 -> 2048 8.5 / 6.4 / 7.2) and
+// where some CTAs have two groups of channels (4 x 5120 -> 5120 9.0 / 7.0 / 7.9).
 inline int few_tokens_linear(int family, int M, int K, int columns, bool half, int sms = RULE_SMS)
 {
     const double mb = double(K) * columns / 2 / (1 << 20);          // of weights
     const bool ragged = K % (half ? 8 : 4) != 0;
-    const int groups = (columns + 31) / 32;
+    const int groups = int((columns + 31ll) / 32);
     const RingFill ring(K, columns, sms);
     // The clusters hold their weights in shared memory: on 148 SMs a CTA has one column tile up to 12.5 MB (fused_tiles_per_cta) and
     // two beyond, and from about 28 MB on they are not resident at once (3 x 11008 -> 6144 11.5 / 22.4 / -, 6 fp32 17.2 / 25.0 / -).
@@ -93,7 +93,9 @@ inline int few_tokens_linear(int family, int M, int K, int columns, bool half, i
             //   * the clusters are near alone and in front in a chain (4096 -> 11008 11.7 / 10.1 / 9.3, layers of 4096 / 11008 with 8 tokens
             //     65.9 / 61.3 / 62.7, of 4096 / 11776 65.5 / 61.4 / 63.3); beyond they are not (4096 -> 12288 11.8 / 12.6 / 9.4, -> 14336
             //     13.8 / 13.8 / 9.7, layers of 4096 / 14336 70.7 / 73.4 / 65.2); short rows are quantised sooner (2048 -> 22528 11.8 / 10.2 / 9.0).
-            if (mb <= 13.25) return family;
+            // With a second round of channel groups the ring is in front alone and in a chain (5 x 1664 -> 7168 6.7 / 6.5 / 5.6, 8 x 3072 -> 8192
+            // 8.7 / 7.4 / 6.7, -> 4096 6.8 / 6.7 / 6.0; layers of 1664 / 7168 with 5 tokens 39.1 / 41.7 / 37.0, of 3072 / 8192 48.4 / 47.3 / 46.4).
+            if (mb <= 13.25) return groups > sms ? 1 : family;
             if (ring.thin && K >= 5120) return 5;
             return mb > 20 && family == 3 && (K <= 1280 || (K > 3072 && K <= 4096 && ring.thin)) ? 3 : 1;    // 8 x 1024 -> 49152 15.8 / 9.5 / 11.2
         }

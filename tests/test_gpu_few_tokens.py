@@ -107,7 +107,7 @@ def test_ring_parts_of_padded_tiles(gpu, oracle, monkeypatch, M, split):
 
 
 # sizes on the rule's lines by the rounds of the three kernels
-LINES = [(7, 4100, 1000, 1, 2), (5, 4100, 1000, 1, 1), (2, 5120, 5632, 1, 2), (4, 4096, 6464, 2, 1), (8, 5120, 9216, 2, 1), (3, 3584, 7680, 2, 1), (6, 5120, 5184, 2, 1),
+LINES = [(7, 4100, 1000, 1, 2), (5, 4100, 1000, 1, 1), (2, 5120, 5632, 1, 2), (4, 4096, 6464, 2, 1), (8, 5120, 9216, 2, 1), (3, 3584, 7680, 2, 1), (6, 5120, 5184, 2, 2), (5, 2048, 4800, 1, 2),
          (2, 4102, 7200, 2, 1), (8, 4096, 11776, 2, 1), (8, 4096, 12288, 2, 2), (1, 8320, 4768, 1, 1)]
 
 

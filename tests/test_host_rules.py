@@ -311,7 +311,7 @@ int main()
         {3, 4096, 7168, false, 1}, {3, 11008, 6144, true, 5}, {3, 10112, 5693, true, 3}, {3, 5120, 9984, false, 1}, {4, 4096, 12544, false, 1}, {4, 4096, 18944, false, 5}, {4, 4096, 18944, true, 5},
         {4, 2048, 40960, false, 5}, {4, 6144, 11008, true, 1}, {4, 6144, 18944, true, 5}, {5, 4405, 1792, true, 3}, {6, 4702, 1024, true, 3}, {5, 4405, 6000, true, 1}, {6, 11008, 6144, false, 1},
         {8, 4096, 8320, true, 1}, {8, 4096, 11776, true, 3}, {8, 4096, 12288, true, 1}, {8, 4096, 12544, true, 1}, {8, 4096, 14336, true, 1}, {8, 4096, 28672, true, 1},
-        {5, 4608, 11008, true, 1}, {5, 5120, 9984, true, 5}, {8, 6144, 9216, true, 5}, {8, 8192, 11008, true, 5}, {8, 8192, 14336, true, 1}, {8, 2048, 22528, true, 1}, {8, 1024, 28672, true, 1}, {8, 1024, 49152, true, 3},
+        {5, 4608, 11008, true, 1}, {5, 5120, 9984, true, 5}, {8, 6144, 9216, true, 5}, {8, 8192, 11008, true, 5}, {8, 8192, 14336, true, 1}, {5, 1664, 7168, true, 1}, {8, 1664, 4736, true, 5}, {8, 3072, 4736, true, 3}, {8, 3072, 4864, true, 1}, {6, 4224, 6272, true, 1}, {8, 2048, 22528, true, 1}, {8, 1024, 28672, true, 1}, {8, 1024, 49152, true, 3},
     };
     for (const Case& c : cases) {
         const int from = c.M <= 4 || (long long)c.K * c.cols / 2 > (24 << 20) ? 5 : 3;        // the workspace's
